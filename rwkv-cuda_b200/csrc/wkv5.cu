@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(NMAX) wkv5_backward_kernel(
 
 template <typename E>
 bool chunked_ok(int T, int N, std::initializer_list<const void*> ps) {
-    if (!std::is_same<E, bf16>::value || N != 64 || T % 16 != 0) return false;
+    if (!std::is_same<E, bf16>::value || N != 64 || (T % 16 != 0 && !wkv6_ragged_ok(T))) return false;
     for (const void* p : ps)
         if (p != nullptr && (reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
     return true;
@@ -241,8 +241,9 @@ int launch_fwd(int B, int T, int C, int H, const void* r, const void* k, const v
         int* flag = wkv6_chunked_flag(st);   // NULL: every slot is taken, the general-shape kernel runs alone
         if (flag != nullptr) {
             RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA, "wkv5_forward: clearing the device flag failed");
-            if (int e = wkv6_chunked_forward(B, T, H, r, k, v, w1, 2, u1, nullptr, 0, y, nullptr, nullptr, flag, st)) return e;
-            only_if = flag;
+            const int e = wkv6_chunked_forward(B, T, H, r, k, v, w1, 2, u1, nullptr, 0, y, nullptr, nullptr, flag, st);
+            if (e < 0) return e;
+            if (e == 0) only_if = flag;   // 1: no kernel for this T here, the general-shape kernel runs alone
         }
     }
 #define RWKV_GO(NM)                                                                                           \
@@ -275,17 +276,17 @@ int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const v
                void* scratch = nullptr, float* gw32 = nullptr, float* gu32 = nullptr) {
     const int N = C / H;
     const int* only_if = nullptr;
-    if (!DUAL && scratch != nullptr && chunked_ok<E>(T, N, {r, k, v, u1, gy, gr, gk, gv, gw1, gu1, scratch})) {
+    if (!DUAL && scratch != nullptr && (T % 16 == 0 || wkv6_states_fit(B, T, H)) && chunked_ok<E>(T, N, {r, k, v, u1, gy, gr, gk, gv, gw1, gu1, scratch})) {
         // chunked forward into the scratch buffer (chunk-start states), chunked reverse pass, then the
         // general-shape kernel only if the decay is too strong for the chunked form
         int* flag = wkv6_chunked_flag(st);   // NULL: every slot is taken, the general-shape kernel runs alone
         if (flag != nullptr) {
             RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA, "wkv5_backward: clearing the device flag failed");
             float* ck = static_cast<float*>(scratch);
-            if (int e = wkv6_backward_with_states(B, T, H, r, k, v, ww1, 3, u1, nullptr, 0, gy, nullptr, ck, gr, gk, gv, gw1, gu1,
-                                                  nullptr, 0, flag, st, gw32, gu32))
-                return e;
-            only_if = flag;
+            const int e = wkv6_backward_with_states(B, T, H, r, k, v, ww1, 3, u1, nullptr, 0, gy, nullptr, ck, gr, gk, gv, gw1, gu1,
+                                                    nullptr, 0, flag, st, gw32, gu32);
+            if (e < 0) return e;
+            if (e == 0) only_if = flag;
         }
     }
 #define RWKV_GO(NM)                                                                                              \
@@ -422,7 +423,7 @@ extern "C" int rwkvb200_wkv5_forward_saved(int dtype, int B, int T, int C, int H
     const int N = C / H;
     cudaStream_t st = as_stream(stream);
     int* flag = nullptr;
-    if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && chunked_ok<bf16>(T, N, {r, k, v, u, y, saved})) flag = wkv6_chunked_flag(st);
+    if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && wkv6_states_fit(B, T, H) && chunked_ok<bf16>(T, N, {r, k, v, u, y, saved})) flag = wkv6_chunked_flag(st);
     if (flag != nullptr) {
         RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA,
                      "wkv5_forward_saved: clearing the device flags failed");

@@ -245,9 +245,12 @@ __global__ void __launch_bounds__(NMAX) wkv6_backward_kernel(
 
 static int g_wkv6_chunked_enabled = 1;
 
+// fp32_state_out: the call returns a state or its gradient in fp32.  Such a call with a ragged T stays on the fp32
+// general-shape kernels: TF32 operands would cost that output three digits (bf16 outputs are rounded more coarsely than that).
 template <typename E>
-bool chunked_ok(int T, int N, std::initializer_list<const void*> ps) {
-    if (!g_wkv6_chunked_enabled || !std::is_same<E, bf16>::value || N != 64 || T % 16 != 0) return false;
+bool chunked_ok(int T, int N, bool fp32_state_out, std::initializer_list<const void*> ps) {
+    if (!g_wkv6_chunked_enabled || !std::is_same<E, bf16>::value || N != 64) return false;
+    if (T % 16 != 0 && (fp32_state_out || !wkv6_ragged_ok(T))) return false;
     for (const void* p : ps)
         if (p != nullptr && (reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
     return true;
@@ -258,14 +261,15 @@ int launch_fwd(int B, int T, int C, int H, const void* r, const void* k, const v
                const void* u, const void* s0, int s0_kind, void* y, float* sT, cudaStream_t st, const char* what) {
     const int N = C / H;
     const int* only_if = nullptr;
-    if (chunked_ok<E>(T, N, {r, k, v, w, u, s0, y, sT})) {
+    if (chunked_ok<E>(T, N, sT != nullptr, {r, k, v, w, u, s0, y, sT})) {
         // tensor-core kernel first; the general-shape kernel below then only runs if that one found a
         // chunk whose decay is too strong for the chunked form
         int* flag = wkv6_chunked_flag(st);   // NULL: every slot is taken, the general-shape kernel runs alone
         if (flag != nullptr) {
             RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA, "%s: clearing the device flag failed", what);
-            if (int e = wkv6_chunked_forward(B, T, H, r, k, v, w, w_raw, u, s0, s0_kind, y, sT, nullptr, flag, st)) return e;
-            only_if = flag;
+            const int e = wkv6_chunked_forward(B, T, H, r, k, v, w, w_raw, u, s0, s0_kind, y, sT, nullptr, flag, st);
+            if (e < 0) return e;
+            if (e == 0) only_if = flag;   // 1: no kernel for this T here, the general-shape kernel runs alone
         }
     }
 #define RWKV_GO(NM)                                                                                              \
@@ -287,7 +291,7 @@ int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const v
                const char* what, bool big_scratch = true) {
     const int N = C / H;
     const int* only_if = nullptr;
-    if (big_scratch && chunked_ok<E>(T, N, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, scratch})) {
+    if (big_scratch && T % 16 == 0 && chunked_ok<E>(T, N, true, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, scratch})) {
         // tensor-core kernels first: a forward pass that leaves the chunk-start states in the scratch
         // buffer, then the reverse pass; the general-shape kernel below then only runs if a chunk's decay
         // was too strong for the chunked form (it reuses the front of the same scratch buffer)
@@ -472,7 +476,7 @@ extern "C" int rwkvb200_wkv6state_forward_tsplit(int dtype, int B, int T, int C,
     const int K = segments, N = C / H;
     RWKV_REQUIRE(K >= 1 && T % K == 0 && (T / K) % 16 == 0, RWKVB200_EINVAL,
                  "wkv6state_forward_tsplit: T = %d is not %d segments of a multiple of 16 tokens", T, K);
-    RWKV_REQUIRE(dtype == RWKVB200_BF16 && chunked_ok<bf16>(T / K, N, {r, k, v, w, u, s0, y, sT, work}), RWKVB200_EINVAL,
+    RWKV_REQUIRE(dtype == RWKVB200_BF16 && (T / K) % 16 == 0 && chunked_ok<bf16>(T / K, N, true, {r, k, v, w, u, s0, y, sT, work}), RWKVB200_EINVAL,
                  "wkv6state_forward_tsplit: needs bf16 tensors, head size 64, 16-byte alignment");
     cudaStream_t st = as_stream(stream);
     int* flag = wkv6_chunked_flag(st);
@@ -506,7 +510,7 @@ extern "C" int rwkvb200_wkv6state_forward_saved(int dtype, int B, int T, int C, 
     const int N = C / H, sk = s0 ? kF32 : kNone;
     cudaStream_t st = as_stream(stream);
     int* flag = nullptr;
-    if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && chunked_ok<bf16>(T, N, {r, k, v, w, u, s0, y, sT, saved}))
+    if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && wkv6_states_fit(B, T, H) && chunked_ok<bf16>(T, N, sT != nullptr, {r, k, v, w, u, s0, y, sT, saved}))
         flag = wkv6_chunked_flag(st);
     if (flag != nullptr) {
         RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA,
@@ -540,7 +544,7 @@ extern "C" int rwkvb200_wkv6state_backward_saved(int dtype, int B, int T, int C,
     const int N = C / H, sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
     cudaStream_t st = as_stream(stream);
     int* flag = nullptr;
-    if (saved_valid && dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, N, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, saved}))
+    if (saved_valid && dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, N, ds0 != nullptr, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, saved}))
         flag = wkv6_chunked_flag(st);
     if (flag != nullptr) {
         const char* tail = static_cast<const char*>(saved) + rwkvb200_wkv6_scratch_bytes(B, T, C) - sizeof(int) * kChunkedFlagUnits;

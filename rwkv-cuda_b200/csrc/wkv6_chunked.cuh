@@ -1,4 +1,4 @@
-// Launchers of the chunked (tensor-core) RWKV-6 kernels: bf16, head size 64, T a multiple of 16.
+// Launchers of the chunked (tensor-core) RWKV-6 kernels: bf16, head size 64, T a multiple of 16 (mma.sync) or any T (tcgen05).
 #pragma once
 #include "common.cuh"
 
@@ -42,9 +42,21 @@ int wkv6_backward_with_states(int B, int T, int H, const void* r, const void* k,
                               void* gk, void* gv, void* gw, void* gu, void* ds0, int ds0_kind, int* unsafe, cudaStream_t st,
                               float* gw32 = nullptr, float* gu32 = nullptr);
 int wkv6_forward_choice();
+// wkv6_chunked_forward and wkv6_backward_with_states return 1, with nothing enqueued, when T is not a multiple of 16 and
+// the tcgen05 kernels cannot run here.
+
+// T that is not a multiple of 16: only the tcgen05 kernels mask the tokens of a partial chunk.  A partial chunk costs as
+// much as a whole one, about 2 us, the time in which the general-shape forward takes two or three tokens: from one chunk on
+// they win.
+inline bool wkv6_ragged_ok(int T) { return T >= 32 && wkv6_forward_choice() && !tensor_maps_disabled(); }
 
 // the "decay too strong" flags of the calling stream: kChunkedFlagUnits ints, one per (batch, head) unit modulo that
 constexpr int kChunkedFlagUnits = 1024;
+// whether a buffer of 16 bytes per element holds one fp32 N x N state per 32 tokens and head, and the flags behind them
+inline bool wkv6_states_fit(int B, int T, int H) {
+    const long long units = (long long)B * H;
+    return units * ((T + 31) / 32) * 64 * 64 * 4 + (long long)sizeof(int) * kChunkedFlagUnits <= units * T * 64 * 16;
+}
 int* wkv6_chunked_flag(cudaStream_t st);
 
 }  // namespace rwkvb200

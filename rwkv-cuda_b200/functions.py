@@ -122,27 +122,39 @@ class WKV_5A(torch.autograd.Function):
 
 
 class WKV_6(torch.autograd.Function):
-    """RWKV-6 (wkv6/run.py:128-170): the kernel receives ew = -exp(w) in fp32."""
+    """RWKV-6 (wkv6/run.py:128-170).  The harness hands its kernel ew = -exp(w) in fp32; here the kernels take w itself
+    (in the activation dtype) and keep the chunk-start states for the backward, as in WKV_6STATE_EX without a state.
+    Only a w of another dtype than the activations goes the harness's way."""
 
     @staticmethod
     def forward(ctx, B, T, C, H, r, k, v, w, u):
         with torch.no_grad():
             ctx.B, ctx.T, ctx.C, ctx.H = B, T, C, H
             r, k, v, w, u = (x.contiguous() for x in (r, k, v, w, u))
-            ew = (-torch.exp(w.float())).contiguous()
-            ctx.save_for_backward(r, k, v, ew, u)
             y = torch.empty((B, T, C), device=r.device, dtype=r.dtype)
-            ops.wkv6_forward(B, T, C, H, r, k, v, ew, u, y)
+            ctx.raw = w.dtype == r.dtype
+            if not ctx.raw:
+                ew = (-torch.exp(w.float())).contiguous()
+                ctx.save_for_backward(r, k, v, ew, u, None)
+                ops.wkv6_forward(B, T, C, H, r, k, v, ew, u, y)
+                return y
+            saved = torch.empty(ops.wkv6_saved_bytes(B, T, C), dtype=torch.uint8, device=r.device)
+            ctx.saved_valid = ops.wkv6state_forward_saved(B, T, C, H, r, k, v, w, u, None, y, None, saved)
+            ctx.save_for_backward(r, k, v, w, u, saved)
             return y
 
     @staticmethod
     def backward(ctx, gy):
         with torch.no_grad():
             B, T, C, H = ctx.B, ctx.T, ctx.C, ctx.H
-            r, k, v, ew, u = ctx.saved_tensors
+            r, k, v, w, u, saved = ctx.saved_tensors
             gr, gk, gv, gw = (torch.empty((B, T, C), device=gy.device, dtype=r.dtype) for _ in range(4))
             gu = torch.empty((B, C), device=gy.device, dtype=r.dtype)
-            ops.wkv6_backward(B, T, C, H, r, k, v, ew, u, gy.contiguous(), gr, gk, gv, gw, gu)
+            if ctx.raw:
+                ops.wkv6state_backward_saved(B, T, C, H, r, k, v, w, u, None, gy.contiguous(), None, gr, gk, gv, gw, gu,
+                                             None, saved, ctx.saved_valid)
+            else:
+                ops.wkv6_backward(B, T, C, H, r, k, v, w, u, gy.contiguous(), gr, gk, gv, gw, gu)
             return (None, None, None, None, gr, gk, gv, gw, torch.sum(gu, 0).view(H, C // H))
 
 
