@@ -197,8 +197,8 @@ extern "C" int rwkvb200_wkv7_state_update(int dtype, int B, int T, int H, int N,
     if (int e = wkv7_check("wkv7_state_update", dtype, B, T, H, N, 1)) return e;
     RWKV_NOTNULL(state); RWKV_NOTNULL(r); RWKV_NOTNULL(w); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(a); RWKV_NOTNULL(b);
     RWKV_NOTNULL(y);
-    // long aligned prompts in bf16 with head size 64 take the tensor-core forward, everything else
-    // (decoding steps, odd lengths, other head sizes, fp32) the general-shape kernel
+    // long aligned prompts in bf16 with head size 64 take the tensor-core forward, decoding steps, odd lengths and fp32
+    // the fp32 kernels of wkv7_update.cu, other head sizes the general-shape kernel
     const bool tensor = g_wkv7_path.load() != 1 && dtype == RWKVB200_BF16 && N == 64 && T % 16 == 0 && T >= 64 &&
                         aligned16({state, r, w, k, v, a, b, y});
     if (tensor) {
@@ -208,5 +208,7 @@ extern "C" int rwkvb200_wkv7_state_update(int dtype, int B, int T, int H, int N,
         }
         return wkv7_l32_forward(B, T, H, state, r, w, k, v, a, b, y, state, nullptr, 0, as_stream(stream));
     }
+    if (N == 64 && aligned16({state, r, w, k, v, a, b, y}))
+        return wkv7_update64(dtype, B, T, H, state, r, w, k, v, a, b, y, sm_count(), as_stream(stream));
     return wkv7_generic_forward(dtype, B, T, H, N, T, state, r, w, k, v, a, b, y, state, nullptr, nullptr, as_stream(stream));
 }

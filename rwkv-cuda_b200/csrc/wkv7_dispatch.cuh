@@ -12,6 +12,10 @@ int wkv7_generic_backward(int dtype, int B, int T, int H, int N, int chunk, cons
                           const float* dsT, const float* s, const float* sa, float* ds0, void* dr, void* dw, void* dk,
                           void* dv, void* da, void* db, cudaStream_t st);
 
+// Inference, head size 64 (16-byte aligned tensors): state (B,H,64,64) in place over T tokens (wkv7_update.cu).
+int wkv7_update64(int dtype, int B, int T, int H, float* state, const void* r, const void* w, const void* k, const void* v,
+                  const void* a, const void* b, void* y, int sms, cudaStream_t st);
+
 // Tensor-core path (bf16, head size 64, checkpoint stride 16, 16-byte aligned tensors): chunks of 32 tokens,
 // every product on tcgen05 with the dependent products chained through tensor memory.  Saved buffer: the
 // state at the start of every 32-token chunk in s[b][h][c] (c < ceil(T/32); the rest of `s` and all of `sa`
