@@ -62,6 +62,16 @@ int rwkvb200_wkv4_forward(int B, int T, int C, const float* w, const float* u, c
 int rwkvb200_wkv4_backward(int B, int T, int C, const float* w, const float* u, const float* k,
                            const float* v, const float* gy, float* gw, float* gu, float* gk,
                            float* gv, void* stream);
+/* Training flow: the harness's pre- and post-operations (wkv/run.py:89-117) inside the kernels.  w_raw = time_decay (C); the
+ * forward leaves the start states of its time segments in `saved` (rwkvb200_wkv4_saved_bytes(B,T,C) bytes) for the
+ * backward, which returns gwu (2,C): the gradients of w_raw and u, summed over the batch in a fixed order.
+ * partial: (B,2,C) floats of work space (may be NULL when B = 1). */
+size_t rwkvb200_wkv4_saved_bytes(int B, int T, int C);
+int rwkvb200_wkv4_train_forward(int B, int T, int C, const float* w_raw, const float* u, const float* k,
+                                const float* v, float* y, void* saved, void* stream);
+int rwkvb200_wkv4_train_backward(int B, int T, int C, const float* w_raw, const float* u, const float* k,
+                                 const float* v, const float* gy, const void* saved, float* gwu, float* partial,
+                                 float* gk, float* gv, void* stream);
 
 /* ---------------------------------------------------------------------------------
  * depthwise_conv1d ("TimeX"), fp32.  Replaces cuda_forward / cuda_backward of

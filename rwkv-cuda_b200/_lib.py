@@ -5,6 +5,8 @@ C ABI.  There is no fallback: if the shared library is missing or a call fails, 
 is raised.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import re
 
@@ -64,6 +66,25 @@ def lib():
 
 class RwkvB200Error(RuntimeError):
     pass
+
+
+_native = None
+
+
+def native():
+    """The extension module with the host side of the training classes (loads on first use)."""
+    global _native
+    if _native is None:
+        lib()
+        path = os.path.join(HERE, "_native.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} not found: it is not built (run `python rwkv-cuda_b200/build.py`)")
+        loader = importlib.machinery.ExtensionFileLoader("_native", path)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_native", loader))
+        loader.exec_module(mod)
+        mod.set_error_class(RwkvB200Error)
+        _native = mod
+    return _native
 
 
 def call(name, *args):

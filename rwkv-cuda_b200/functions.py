@@ -1,56 +1,28 @@
-"""torch.autograd.Function mirrors of the reference harnesses' operators, same class names,
-same forward/backward argument order and the same pre/post tensor ops around the kernels.
-Module-level globals of the reference (HEAD_SIZE, B, T, C ...) are taken from the tensors.
+"""torch.autograd.Function mirrors of the reference harnesses' operators: same class names, same arguments of `apply`,
+same results.  Module-level globals of the reference (HEAD_SIZE, B, T, C ...) are taken from the tensors.
+Where `apply` is given here, forward and backward are native code (csrc_py/native.cpp).
 """
 import torch
 
 from . import ops
+from ._lib import native
 
 
 class WKV(torch.autograd.Function):
-    """RWKV-4 (wkv/run.py:89-117): w -> -exp(w) before, per-batch gw/gu summed after."""
+    """RWKV-4 (wkv/run.py:89-117): w is time_decay; the harness's w -> -exp(w) before and its sums of the per-batch gw, gu
+    after are done by the kernels."""
 
     @staticmethod
-    def forward(ctx, B, T, C, w, u, k, v):
-        ctx.B, ctx.T, ctx.C = B, T, C
-        w = -torch.exp(w.contiguous())
-        u, k, v = u.contiguous(), k.contiguous(), v.contiguous()
-        ctx.save_for_backward(w, u, k, v)
-        y = torch.empty((B, T, C), device=k.device, dtype=torch.float32)
-        ops.wkv4_forward(B, T, C, w, u, k, v, y)
-        return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        B, T, C = ctx.B, ctx.T, ctx.C
-        w, u, k, v = ctx.saved_tensors
-        gw = torch.zeros((B, C), device=k.device)
-        gu = torch.zeros((B, C), device=k.device)
-        gk = torch.empty((B, T, C), device=k.device)
-        gv = torch.empty((B, T, C), device=k.device)
-        ops.wkv4_backward(B, T, C, w, u, k, v, gy.contiguous(), gw, gu, gk, gv)
-        return None, None, None, gw.sum(dim=0), gu.sum(dim=0), gk, gv
+    def apply(B, T, C, w, u, k, v):
+        return native().wkv4(B, T, C, w, u, k, v)
 
 
 class TimeX(torch.autograd.Function):
-    """depthwise_conv1d (depthwise_conv1d/run.py:76-102); gw is reduced over the batch inside the kernel."""
+    """depthwise_conv1d (depthwise_conv1d/run.py:76-102); gw is reduced over the batch inside the kernels."""
 
     @staticmethod
-    def forward(ctx, w, k, B, C, T, eps):
-        ctx.B, ctx.C, ctx.T = B, C, T
-        w, k = w.contiguous(), k.contiguous()
-        ctx.save_for_backward(w, k)
-        wk = torch.empty((B, C, T), device=k.device, dtype=torch.float32)
-        ops.timex_forward(w, k, wk, eps, B, C, T)
-        return wk
-
-    @staticmethod
-    def backward(ctx, gwk):
-        w, k = ctx.saved_tensors
-        gw = torch.empty((ctx.C, ctx.T), device=k.device, dtype=torch.float32)
-        gk = torch.empty((ctx.B, ctx.C, ctx.T), device=k.device, dtype=torch.float32)
-        ops.timex_backward_reduced(w, k, gwk.contiguous(), gw, gk, ctx.B, ctx.C, ctx.T)
-        return gw, gk, None, None, None, None
+    def apply(w, k, B, C, T, eps):
+        return native().timex(w, k, B, C, T, eps)
 
 
 class WKV_5(torch.autograd.Function):
@@ -214,89 +186,28 @@ class WKV_6STATE_EX(torch.autograd.Function):
             return gr, gk, gv, gw, torch.sum(gu.float(), 0).view(H, C // H).to(u.dtype), ds0
 
 
-CHUNK_LEN = 16
-
-
-def _v7_saved(r):
-    B, T, H, N = r.shape
-    s = torch.empty(B, H, T // CHUNK_LEN, N, N, dtype=torch.float32, device=r.device)
-    sa = torch.empty(B, T, H, N, dtype=torch.float32, device=r.device)
-    return s, sa
-
-
-def _v7_check(*xs):
-    r = xs[0]
-    assert r.shape[1] % CHUNK_LEN == 0
-    assert all(i.dtype == r.dtype for i in xs)
-    assert all(i.is_contiguous() for i in xs)
-
-
 class RWKV7_CLAMPW_CUDA_OP(torch.autograd.Function):
     """rwkv7_fast_fused/rwkv7_cuda_benchmark.py:76-96; inputs (B,T,H,N)."""
 
     @staticmethod
-    def forward(ctx, r, w, k, v, a, b):
-        _v7_check(r, w, k, v, a, b)
-        y = torch.empty_like(v)
-        s, sa = _v7_saved(r)
-        ops.wkv7_forward(None, r, w, k, v, a, b, y, None, s, sa)
-        ctx.save_for_backward(r, w, k, v, a, b, s, sa)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        r, w, k, v, a, b, s, sa = ctx.saved_tensors
-        dr, dw, dk, dv, da, db = (torch.empty_like(x) for x in (r, w, k, v, a, b))
-        ops.wkv7_backward(r, w, k, v, a, b, dy.contiguous(), None, s, sa, None, dr, dw, dk, dv, da, db)
-        return dr, dw, dk, dv, da, db
+    def apply(r, w, k, v, a, b):
+        return native().wkv7(r, w, k, v, a, b)
 
 
 class RWKV7_STATE_CLAMPW_CUDA_OP(torch.autograd.Function):
     """rwkv7_fast_fused/rwkv7_cuda_benchmark_state.py:75-99."""
 
     @staticmethod
-    def forward(ctx, s0, r, w, k, v, a, b):
-        _v7_check(r, w, k, v, a, b)
-        assert s0.dtype == torch.float and s0.is_contiguous()
-        y = torch.empty_like(v)
-        s, sa = _v7_saved(r)
-        ops.wkv7_forward(s0, r, w, k, v, a, b, y, None, s, sa)
-        ctx.save_for_backward(r, w, k, v, a, b, s, sa)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        r, w, k, v, a, b, s, sa = ctx.saved_tensors
-        B, T, H, N = r.shape
-        dr, dw, dk, dv, da, db = (torch.empty_like(x) for x in (r, w, k, v, a, b))
-        ds0 = torch.empty(B, H, N, N, dtype=torch.float32, device=r.device)
-        ops.wkv7_backward(r, w, k, v, a, b, dy.contiguous(), None, s, sa, ds0, dr, dw, dk, dv, da, db)
-        return ds0, dr, dw, dk, dv, da, db
+    def apply(s0, r, w, k, v, a, b):
+        return native().wkv7_state(s0, r, w, k, v, a, b)
 
 
 class RWKV7_STATE_PASSING_CLAMPW_CUDA_OP(torch.autograd.Function):
     """rwkv7_fast_fused/rwkv7_cuda_benchmark_state_passing.py:75-99: returns (y, sT)."""
 
     @staticmethod
-    def forward(ctx, s0, r, w, k, v, a, b):
-        B, T, H, N = r.shape
-        _v7_check(r, w, k, v, a, b)
-        assert s0.dtype == torch.float and s0.is_contiguous()
-        y = torch.empty_like(v)
-        sT = torch.empty_like(s0)
-        s, sa = _v7_saved(r)
-        ops.wkv7_forward(s0, r, w, k, v, a, b, y, sT, s, sa)
-        ctx.save_for_backward(r, w, k, v, a, b, s, sa)
-        return y.view(B, T, H * N), sT
-
-    @staticmethod
-    def backward(ctx, dy, dsT):
-        r, w, k, v, a, b, s, sa = ctx.saved_tensors
-        assert dsT.dtype == torch.float
-        ds0 = torch.empty_like(dsT)
-        dr, dw, dk, dv, da, db = (torch.empty_like(x) for x in (r, w, k, v, a, b))
-        ops.wkv7_backward(r, w, k, v, a, b, dy.contiguous(), dsT.contiguous(), s, sa, ds0, dr, dw, dk, dv, da, db)
-        return ds0, dr, dw, dk, dv, da, db
+    def apply(s0, r, w, k, v, a, b):
+        return native().wkv7_statepassing(s0, r, w, k, v, a, b)
 
 
 def _heads(x, head_size):
