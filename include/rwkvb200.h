@@ -104,7 +104,7 @@ int rwkvb200_wkv5_backward(int dtype, int B, int T, int C, int H, const void* r,
                            const void* gy, void* gr, void* gk, void* gv, void* gw, void* gu,
                            void* stream);
 /* Sum of the per-batch parameter-gradient partials the backward kernels emit, gw / gu (B,n) in `dtype`,
- * into fp32 out[n], accumulated in fp32 in batch order (deterministic).  Replaces the harnesses'
+ * into fp32 out[n], accumulated in fp32 in a fixed order (deterministic).  Replaces the harnesses'
  * `torch.sum(gw, 0)` on bf16 partials (wkv5_bf16/run.py:86-87, wkv6/run.py:169, wkv/run.py:115-116), whose
  * result is rounded to bf16; several partials can be reduced into one fp32 buffer, which is then what a
  * multi-GPU run all-reduces once. */
@@ -127,6 +127,18 @@ int rwkvb200_wkv5_backward_ws32(int dtype, int B, int T, int C, int H, const voi
                                 const void* v, const float* w, const float* ww, const void* u,
                                 const void* gy, void* gr, void* gk, void* gv, void* gw, void* gu,
                                 float* gw32, float* gu32, void* scratch, void* stream);
+
+/* Training flow: the harness's pre- and post-operations (wkv5_bf16/run.py:44-88) inside the kernels.  w_raw (H,N) in `dtype`;
+ * gwu (2,C) in `dtype`: the gradients of w_raw and u, summed over the batch in fp32 and in a fixed order.  The forward leaves
+ * in `saved` (rwkvb200_wkv5_train_saved_bytes) what the backward needs and returns the path that both take (0 or 1, or a
+ * negative code); `work`: rwkvb200_wkv5_train_work_bytes(..., path) bytes. */
+size_t rwkvb200_wkv5_train_saved_bytes(int B, int T, int C, int H);
+size_t rwkvb200_wkv5_train_work_bytes(int B, int T, int C, int H, int path);
+int rwkvb200_wkv5_train_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v,
+                                const void* w_raw, const void* u, void* y, void* saved, void* stream);
+int rwkvb200_wkv5_train_backward(int dtype, int B, int T, int C, int H, int path, const void* r, const void* k,
+                                 const void* v, const void* w_raw, const void* u, const void* gy, void* gr, void* gk,
+                                 void* gv, void* gwu, const void* saved, void* work, void* stream);
 
 /* ---------------------------------------------------------------------------------
  * RWKV-5a WKV (decay w1[j]*w2[i], bonus u1[j]+u2[i]), fp32 or bf16 activations.
@@ -226,6 +238,18 @@ int rwkvb200_wkv6state_backward_saved(int dtype, int B, int T, int C, int H, con
                                       const float* s0, const void* gy, const float* dsT, void* gr,
                                       void* gk, void* gv, void* gw, void* gu, float* ds0,
                                       void* saved, int saved_valid, void* stream);
+
+/* The same flow as the training classes use it, with or without a state (s0, sT, dsT, ds0 may be NULL): gu (C) in `dtype` is
+ * summed over the batch in fp32, `saved` and `work` have the sizes that the path (the forward's return value) needs. */
+size_t rwkvb200_wkv6_train_saved_bytes(int dtype, int B, int T, int C, int H);
+size_t rwkvb200_wkv6_train_work_bytes(int B, int T, int C, int path);
+int rwkvb200_wkv6_train_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v,
+                                const void* w, const void* u, const float* s0, void* y, float* sT, void* saved,
+                                void* stream);
+int rwkvb200_wkv6_train_backward(int dtype, int B, int T, int C, int H, int path, const void* r, const void* k,
+                                 const void* v, const void* w, const void* u, const float* s0, const void* gy,
+                                 const float* dsT, void* gr, void* gk, void* gv, void* gw, void* gu, float* ds0,
+                                 void* saved, void* work, void* stream);
 
 /* Kernels of the bf16 / head-size-64 forward and backward of RWKV-5 and RWKV-6: 1 (default) = tcgen05 (32-token
  * chunks; the forward as three warp groups with inputs by TMA), 0 = mma.sync (16-token chunks).  Results agree to rounding.

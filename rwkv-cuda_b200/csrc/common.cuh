@@ -51,6 +51,9 @@ void set_error(const char* fmt, ...);
 // Called after every launch: turns a launch-time CUDA error into a status code.
 int check_launch(const char* what);
 
+// out[n] (fp32 or bf16) <- sums over the rows of partial[rows][n] (wkv5.cu)
+int sum_rows(int out_dtype, long long rows, int n, const float* partial, void* out, cudaStream_t st);
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // test hook (rwkvb200_test_disable_tensor_maps): true makes every tensor-map maker report failure, so that the

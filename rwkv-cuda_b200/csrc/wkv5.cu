@@ -22,6 +22,7 @@
 #include "common.cuh"
 #include "wkv6_chunked.cuh"
 #include "wkv6_tsplit.cuh"
+#include "wkv5_seg.cuh"
 #include <initializer_list>
 #include <type_traits>
 
@@ -34,18 +35,21 @@ struct __align__(16) Stage {
 };
 
 // ------------------------------------------------------------------------------------
+// only_if_ / only_mask: when given, a unit runs only if its flag (unit index & only_mask) is set.  w_raw_: when given, the raw
+// decay input (decay exp(-exp(w))) in place of w1_.
 template <typename E, int NMAX, bool DUAL>
 __global__ void __launch_bounds__(NMAX) wkv5_forward_kernel(int T, int C, int H, int N, const E* __restrict__ r_,
                                                            const E* __restrict__ k_, const E* __restrict__ v_,
                                                            const float* __restrict__ w1_, const E* __restrict__ u1_,
                                                            const float* __restrict__ w2_, const E* __restrict__ u2_,
-                                                           E* __restrict__ y_, const int* __restrict__ only_if_) {
-    if (only_if_ != nullptr && only_if_[blockIdx.x & (kChunkedFlagUnits - 1)] == 0) return;   // fallback launch: the chunked kernel's result stands for this unit
+                                                           E* __restrict__ y_, const int* __restrict__ only_if_,
+                                                           int only_mask, const E* __restrict__ w_raw_) {
+    if (only_if_ != nullptr && only_if_[blockIdx.x & only_mask] == 0) return;   // fallback launch: the chunked kernel's result stands for this unit
     const int b = blockIdx.x / H, h = blockIdx.x - b * H, i = threadIdx.x;
     const bool live = i < N;
     __shared__ Stage<NMAX> rs, ks;
     __shared__ __align__(16) float ws[NMAX], us[NMAX];
-    ws[i] = live ? w1_[h * N + i] : 0.f;
+    ws[i] = !live ? 0.f : w_raw_ != nullptr ? expf(-expf(to_f(w_raw_[h * N + i]))) : w1_[h * N + i];
     us[i] = live ? to_f(u1_[h * N + i]) : 0.f;
     const float w2 = (DUAL && live) ? w2_[h * N + i] : 1.f;
     const float u2 = (DUAL && live) ? to_f(u2_[h * N + i]) : 0.f;
@@ -93,13 +97,14 @@ __global__ void __launch_bounds__(NMAX) wkv5_backward_kernel(
     const float* __restrict__ w1_, const float* __restrict__ ww1_, const E* __restrict__ u1_,
     const float* __restrict__ w2_, const float* __restrict__ ww2_, const E* __restrict__ u2_,
     const E* __restrict__ gy_, E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_, E* __restrict__ gw1_,
-    E* __restrict__ gu1_, E* __restrict__ gw2_, E* __restrict__ gu2_, const int* __restrict__ only_if_) {
-    if (only_if_ != nullptr && only_if_[blockIdx.x & (kChunkedFlagUnits - 1)] == 0) return;   // fallback launch: the chunked kernels' result stands for this unit
+    E* __restrict__ gu1_, E* __restrict__ gw2_, E* __restrict__ gu2_, const int* __restrict__ only_if_, int only_mask,
+    const E* __restrict__ w_raw_, float* __restrict__ gw32_, float* __restrict__ gu32_, i64 gstride) {
+    if (only_if_ != nullptr && only_if_[blockIdx.x & only_mask] == 0) return;   // fallback launch: the chunked kernels' result stands for this unit
     const int b = blockIdx.x / H, h = blockIdx.x - b * H, i = threadIdx.x;
     const bool live = i < N;
     __shared__ Stage<NMAX> rs, ks, vs, gs;
     __shared__ __align__(16) float w1s[NMAX], u1s[NMAX], w2s[NMAX], u2s[NMAX];
-    w1s[i] = live ? w1_[h * N + i] : 0.f;
+    w1s[i] = !live ? 0.f : w_raw_ != nullptr ? expf(-expf(to_f(w_raw_[h * N + i]))) : w1_[h * N + i];
     u1s[i] = live ? to_f(u1_[h * N + i]) : 0.f;
     w2s[i] = (DUAL && live) ? w2_[h * N + i] : (live ? 1.f : 0.f);
     u2s[i] = (DUAL && live) ? to_f(u2_[h * N + i]) : 0.f;
@@ -143,8 +148,9 @@ __global__ void __launch_bounds__(NMAX) wkv5_backward_kernel(
             gw = fmaf(r, zg, gw);
         }
         if (live) {
-            gu1_[pbase] = from_f<E>(gu);
-            gw1_[pbase] = from_f<E>(ww1_[h * N + i] * gw);
+            gw *= w_raw_ != nullptr ? -expf(to_f(w_raw_[h * N + i])) : ww1_[h * N + i];
+            if (gu1_ != nullptr) { gu1_[pbase] = from_f<E>(gu); gw1_[pbase] = from_f<E>(gw); }
+            if (gu32_ != nullptr) { gu32_[b * gstride + h * N + i] = gu; gw32_[b * gstride + h * N + i] = gw; }   // unrounded
         }
     }
 
@@ -248,7 +254,7 @@ int launch_fwd(int B, int T, int C, int H, const void* r, const void* k, const v
     }
 #define RWKV_GO(NM)                                                                                           \
     wkv5_forward_kernel<E, NM, DUAL><<<B * H, NM, 0, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, \
-                                                            w1, (const E*)u1, w2, (const E*)u2, (E*)y, only_if)
+                                                            w1, (const E*)u1, w2, (const E*)u2, (E*)y, only_if, kChunkedFlagUnits - 1, nullptr)
     switch (head_capacity(N)) {
         case 32: RWKV_GO(32); break;
         case 64: RWKV_GO(64); break;
@@ -256,17 +262,6 @@ int launch_fwd(int B, int T, int C, int H, const void* r, const void* k, const v
     }
 #undef RWKV_GO
     return check_launch(DUAL ? "wkv5a_forward" : "wkv5_forward");
-}
-
-// fp32 copies of the (B,C) partials; only_if: run only when that device flag is set (NULL: always)
-template <typename E>
-__global__ void widen_partials_kernel(int n, int C, int N, const E* __restrict__ gw, const E* __restrict__ gu,
-                                      float* __restrict__ gw32, float* __restrict__ gu32, const int* __restrict__ only_if) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int unit = (i / C) * (C / N) + (i % C) / N;   // (batch, head) of this element
-    if (only_if != nullptr && only_if[unit & (kChunkedFlagUnits - 1)] == 0) return;
-    gw32[i] = to_f(gw[i]); gu32[i] = to_f(gu[i]);
 }
 
 template <typename E, bool DUAL>
@@ -292,18 +287,13 @@ int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const v
 #define RWKV_GO(NM)                                                                                              \
     wkv5_backward_kernel<E, NM, DUAL><<<B * H, NM, 0, st>>>(                                                     \
         T, C, H, N, (const E*)r, (const E*)k, (const E*)v, w1, ww1, (const E*)u1, w2, ww2, (const E*)u2,         \
-        (const E*)gy, (E*)gr, (E*)gk, (E*)gv, (E*)gw1, (E*)gu1, (E*)gw2, (E*)gu2, only_if)
+        (const E*)gy, (E*)gr, (E*)gk, (E*)gv, (E*)gw1, (E*)gu1, (E*)gw2, (E*)gu2, only_if, kChunkedFlagUnits - 1, nullptr, gw32, gu32, C)
     switch (head_capacity(N)) {
         case 32: RWKV_GO(32); break;
         case 64: RWKV_GO(64); break;
         default: RWKV_GO(128); break;
     }
 #undef RWKV_GO
-    if (gw32 != nullptr && gu32 != nullptr) {
-        // the general-shape kernel has the (B,C) partials in the activation type only: where it ran (it was the
-        // only kernel, or the chunked one raised its flag) the fp32 copies are made from those
-        widen_partials_kernel<E><<<(B * C + 255) / 256, 256, 0, st>>>(B * C, C, N, (const E*)gw1, (const E*)gu1, gw32, gu32, only_if);
-    }
     return check_launch(DUAL ? "wkv5a_backward" : "wkv5_backward");
 }
 
@@ -357,7 +347,7 @@ extern "C" int rwkvb200_wkv5_forward_tsplit(int dtype, int B, int T, int C, int 
     if (int e = wkv6_chunked_forward(B * K, T / K, H, r, k, v, w, 2, u, start, 2, y, nullptr, nullptr, flag, st, K)) return e;
     // a decay too strong for the chunked form: the general-shape kernel redoes the call
     wkv5_forward_kernel<bf16, 64, false><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w,
-                                                              (const bf16*)u, nullptr, nullptr, (bf16*)y, flag);
+                                                              (const bf16*)u, nullptr, nullptr, (bf16*)y, flag, kChunkedFlagUnits - 1, nullptr);
     return check_launch("wkv5_forward_tsplit");
 }
 
@@ -422,21 +412,14 @@ extern "C" int rwkvb200_wkv5_forward_saved(int dtype, int B, int T, int C, int H
     RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w); RWKV_NOTNULL(u); RWKV_NOTNULL(y); RWKV_NOTNULL(saved);
     const int N = C / H;
     cudaStream_t st = as_stream(stream);
-    int* flag = nullptr;
-    if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && wkv6_states_fit(B, T, H) && chunked_ok<bf16>(T, N, {r, k, v, u, y, saved})) flag = wkv6_chunked_flag(st);
-    if (flag != nullptr) {
-        RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA,
-                     "wkv5_forward_saved: clearing the device flags failed");
-        const int rc = wkv6_l32_forward(B, T, H, r, k, v, w, 2, u, nullptr, 0, y, nullptr, static_cast<float*>(saved), flag, st, 1);
+    if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && wkv6_states_fit(B, T, H) && chunked_ok<bf16>(T, N, {r, k, v, u, y, saved})) {
+        int* flags = wkv6_saved_flags(saved, B, T, H);
+        const int rc = wkv6_l32_forward(B, T, H, r, k, v, w, 2, u, nullptr, 0, y, nullptr, static_cast<float*>(saved), flags, st, 0);
         if (rc < 0) return rc;
         if (rc == 0) {
             wkv5_forward_kernel<bf16, 64, false><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w,
-                                                                      (const bf16*)u, nullptr, nullptr, (bf16*)y, flag);
-            if (int e = check_launch("wkv5_forward_saved")) return e;
-            char* tail = static_cast<char*>(saved) + rwkvb200_wkv5_scratch_bytes(B, T, C) - sizeof(int) * kChunkedFlagUnits;
-            RWKV_REQUIRE(cudaMemcpyAsync(tail, flag, sizeof(int) * kChunkedFlagUnits, cudaMemcpyDeviceToDevice, st) == cudaSuccess,
-                         RWKVB200_ECUDA, "wkv5_forward_saved: saving the device flags failed");
-            return RWKVB200_OK;
+                                                                      (const bf16*)u, nullptr, nullptr, (bf16*)y, flags, -1, nullptr);
+            return check_launch("wkv5_forward_saved");
         }
     }
     const int e = dtype == RWKVB200_F32 ? launch_fwd<float, false>(B, T, C, H, r, k, v, w, u, nullptr, nullptr, y, st)
@@ -454,21 +437,15 @@ extern "C" int rwkvb200_wkv5_backward_saved(int dtype, int B, int T, int C, int 
     RWKV_REQUIRE((gw32 == nullptr) == (gu32 == nullptr), RWKVB200_EINVAL, "wkv5_backward_saved: gw32 and gu32 go together");
     const int N = C / H;
     cudaStream_t st = as_stream(stream);
-    int* flag = nullptr;
-    if (saved_valid && dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, N, {r, k, v, u, gy, gr, gk, gv, gw, gu, saved})) flag = wkv6_chunked_flag(st);
-    if (flag != nullptr) {
-        const char* tail = static_cast<const char*>(saved) + rwkvb200_wkv5_scratch_bytes(B, T, C) - sizeof(int) * kChunkedFlagUnits;
-        RWKV_REQUIRE(cudaMemcpyAsync(flag, tail, sizeof(int) * kChunkedFlagUnits, cudaMemcpyDeviceToDevice, st) == cudaSuccess,
-                     RWKVB200_ECUDA, "wkv5_backward_saved: restoring the device flags failed");
+    if (saved_valid && dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, N, {r, k, v, u, gy, gr, gk, gv, gw, gu, saved})) {
+        const int* flags = wkv6_saved_flags(saved, B, T, H);
         if (int e = wkv6_l32_backward(B, T, H, r, k, v, ww, 3, u, gy, nullptr, static_cast<const float*>(saved), gr, gk, gv, gw, gu,
-                                      nullptr, 0, st, gw32, gu32))
+                                      nullptr, 0, st, gw32, gu32, 0, flags))
             return e;
         wkv5_backward_kernel<bf16, 64, false><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w, ww,
                                                                    (const bf16*)u, nullptr, nullptr, nullptr, (const bf16*)gy,
                                                                    (bf16*)gr, (bf16*)gk, (bf16*)gv, (bf16*)gw, (bf16*)gu, nullptr,
-                                                                   nullptr, flag);
-        if (gw32 != nullptr)
-            widen_partials_kernel<bf16><<<(B * C + 255) / 256, 256, 0, st>>>(B * C, C, N, (const bf16*)gw, (const bf16*)gu, gw32, gu32, flag);
+                                                                   nullptr, flags, -1, nullptr, gw32, gu32, C);
         return check_launch("wkv5_backward_saved");
     }
     return dtype == RWKVB200_F32
@@ -476,6 +453,67 @@ extern "C" int rwkvb200_wkv5_backward_saved(int dtype, int B, int T, int C, int 
                                           nullptr, st, saved, gw32, gu32)
                : launch_bwd<bf16, false>(B, T, C, H, r, k, v, w, ww, u, nullptr, nullptr, nullptr, gy, gr, gk, gv, gw, gu, nullptr,
                                          nullptr, st, saved, gw32, gu32);
+}
+
+// ---- training flow: the harness's pre- and post-operations inside the kernels -------------------------------------------
+// bf16 / head size 64 on the tcgen05 kernels (as rwkvb200_wkv5_forward_saved), everything else on the segments of wkv5_seg.cu.
+extern "C" size_t rwkvb200_wkv5_train_saved_bytes(int B, int T, int C, int H) {
+    if (B <= 0 || T <= 0 || C <= 0 || H <= 0) return 0;
+    return (size_t)B * H * (wkv5_seg_count(T) * (C / H) * (C / H) + 1) * sizeof(float);   // a state per 32 tokens and a flag per unit
+}
+
+extern "C" int rwkvb200_wkv5_train_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v,
+                                           const void* w_raw, const void* u, void* y, void* saved, void* stream) {
+    if (int e = check_dims("wkv5_train_forward", dtype, B, T, C, H)) return e;
+    RWKV_REQUIRE(B * (i64)H <= 65535, RWKVB200_EINVAL, "wkv5_train_forward: B*H=%lld exceeds 65535", B * (i64)H);
+    RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w_raw); RWKV_NOTNULL(u); RWKV_NOTNULL(y); RWKV_NOTNULL(saved);
+    cudaStream_t st = as_stream(stream);
+    if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && chunked_ok<bf16>(T, C / H, {r, k, v, y, saved})) {
+        int* flags = wkv6_saved_flags(saved, B, T, H);
+        const int rc = wkv6_l32_forward(B, T, H, r, k, v, w_raw, 4, u, nullptr, 0, y, nullptr, static_cast<float*>(saved), flags, st, 0);
+        if (rc < 0) return rc;
+        if (rc == 0) {
+            wkv5_forward_kernel<bf16, 64, false><<<B * H, 64, 0, st>>>(T, C, H, C / H, (const bf16*)r, (const bf16*)k, (const bf16*)v, nullptr,
+                                                                      (const bf16*)u, nullptr, nullptr, (bf16*)y, flags, -1, (const bf16*)w_raw);
+            return check_launch("wkv5_train_forward");
+        }
+    }
+    const int e = wkv5_seg_forward(dtype, B, T, C, H, r, k, v, w_raw, u, y, static_cast<float*>(saved), st);
+    return e ? e : 1;
+}
+
+extern "C" size_t rwkvb200_wkv5_train_work_bytes(int B, int T, int C, int H, int path) {
+    if (B <= 0 || T <= 0 || C <= 0 || H <= 0) return 0;
+    if (path == 0) return (size_t)B * 2 * C * sizeof(float);
+    return wkv5_seg_count(T) * ((size_t)B * H * (C / H) * (C / H) + (size_t)B * 2 * C) * sizeof(float);
+}
+
+extern "C" int rwkvb200_wkv5_train_backward(int dtype, int B, int T, int C, int H, int path, const void* r, const void* k, const void* v,
+                                            const void* w_raw, const void* u, const void* gy, void* gr, void* gk, void* gv, void* gwu,
+                                            const void* saved, void* work, void* stream) {
+    if (int e = check_dims("wkv5_train_backward", dtype, B, T, C, H)) return e;
+    RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w_raw); RWKV_NOTNULL(u); RWKV_NOTNULL(gy);
+    RWKV_NOTNULL(gr); RWKV_NOTNULL(gk); RWKV_NOTNULL(gv); RWKV_NOTNULL(gwu); RWKV_NOTNULL(saved); RWKV_NOTNULL(work);
+    cudaStream_t st = as_stream(stream);
+    float* partial = static_cast<float*>(work);
+    i64 rows = B;
+    if (path == 0) {
+        RWKV_REQUIRE(dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, C / H, {r, k, v, gy, gr, gk, gv, saved}), RWKVB200_EALIGN,
+                     "wkv5_train_backward: the bf16 N=64 path needs 16-byte aligned tensors");
+        const int* flags = wkv6_saved_flags(const_cast<void*>(saved), B, T, H);
+        if (int e = wkv6_l32_backward(B, T, H, r, k, v, w_raw, 4, u, gy, nullptr, static_cast<const float*>(saved), gr, gk, gv, nullptr, nullptr,
+                                      nullptr, 0, st, partial, partial + C, 2 * (i64)C, flags))
+            return e;
+        wkv5_backward_kernel<bf16, 64, false><<<B * H, 64, 0, st>>>(
+            T, C, H, C / H, (const bf16*)r, (const bf16*)k, (const bf16*)v, nullptr, nullptr, (const bf16*)u, nullptr, nullptr, nullptr, (const bf16*)gy,
+            (bf16*)gr, (bf16*)gk, (bf16*)gv, nullptr, nullptr, nullptr, nullptr, flags, -1, (const bf16*)w_raw, partial, partial + C, 2 * (i64)C);
+        if (int e = check_launch("wkv5_train_backward")) return e;
+    } else {
+        float* D = partial + (size_t)B * wkv5_seg_count(T) * 2 * C;
+        if (int e = wkv5_seg_backward(dtype, B, T, C, H, r, k, v, w_raw, u, gy, gr, gk, gv, static_cast<const float*>(saved), D, partial, st)) return e;
+        rows = (i64)B * wkv5_seg_count(T);
+    }
+    return sum_rows(dtype, rows, 2 * C, partial, gwu, st);
 }
 
 extern "C" int rwkvb200_wkv5a_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k,
@@ -503,29 +541,44 @@ extern "C" int rwkvb200_wkv5a_backward(int dtype, int B, int T, int C, int H, co
                                         gw2, gu2, as_stream(stream));
 }
 
-// ---- parameter gradients: per-batch partials -> one fp32 vector ------------------------------------------
+// ---- parameter gradients: sums of partials over rows (batch rows, time segments) ---------------------------------------
 namespace rwkvb200 {
 namespace {
-// out[off + j] = sum_b partial[b][j], fp32 accumulation in batch order (deterministic); one thread per column
-template <typename E>
-__global__ void reduce_batch_partials_kernel(int B, int n, const E* __restrict__ partial, float* __restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
+// out[j] = sum over rows of partial[row][j], in fp32 and in an order that depends on the shape only: 8 threads take every
+// 8th row of a column, their sums are added in order.  A row is read as 32 consecutive columns per warp.
+template <typename E, typename O>
+__global__ void __launch_bounds__(256) sum_rows_kernel(i64 rows, int n, const E* __restrict__ partial, O* __restrict__ out) {
+    __shared__ float part[8][32];
+    const int j = blockIdx.x * 32 + threadIdx.x;
     float acc = 0.f;
-    for (int b = 0; b < B; ++b) acc += to_f(partial[(i64)b * n + j]);
-    out[j] = acc;
+    if (j < n) {
+#pragma unroll 4
+        for (i64 b = threadIdx.y; b < rows; b += 8) acc += to_f(partial[b * n + j]);
+    }
+    part[threadIdx.y][threadIdx.x] = acc;
+    __syncthreads();
+    if (threadIdx.y == 0 && j < n) {
+        acc = 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc += part[q][threadIdx.x];
+        out[j] = from_f<O>(acc);
+    }
 }
 }  // namespace
+
+int sum_rows(int out_dtype, long long rows, int n, const float* partial, void* out, cudaStream_t st) {
+    const dim3 block(32, 8);
+    if (out_dtype == RWKVB200_F32) sum_rows_kernel<float, float><<<(n + 31) / 32, block, 0, st>>>(rows, n, partial, (float*)out);
+    else sum_rows_kernel<float, bf16><<<(n + 31) / 32, block, 0, st>>>(rows, n, partial, (bf16*)out);
+    return check_launch("sum_rows");
+}
 }  // namespace rwkvb200
 
 extern "C" int rwkvb200_reduce_batch_partials(int dtype, int B, int n, const void* partial, float* out, void* stream) {
     RWKV_REQUIRE(dtype == RWKVB200_F32 || dtype == RWKVB200_BF16, RWKVB200_EINVAL, "reduce_batch_partials: unknown dtype %d", dtype);
     RWKV_REQUIRE(B > 0 && n > 0, RWKVB200_EINVAL, "reduce_batch_partials: B=%d n=%d must be positive", B, n);
     RWKV_NOTNULL(partial); RWKV_NOTNULL(out);
-    const int threads = 128, blocks = (n + threads - 1) / threads;
-    if (dtype == RWKVB200_F32)
-        reduce_batch_partials_kernel<float><<<blocks, threads, 0, as_stream(stream)>>>(B, n, (const float*)partial, out);
-    else
-        reduce_batch_partials_kernel<bf16><<<blocks, threads, 0, as_stream(stream)>>>(B, n, (const bf16*)partial, out);
+    if (dtype == RWKVB200_F32) return sum_rows(RWKVB200_F32, B, n, static_cast<const float*>(partial), out, as_stream(stream));
+    sum_rows_kernel<bf16, float><<<(n + 31) / 32, dim3(32, 8), 0, as_stream(stream)>>>(B, n, (const bf16*)partial, out);
     return check_launch("reduce_batch_partials");
 }

@@ -69,8 +69,8 @@ __global__ void __launch_bounds__(NMAX) wkv6_forward_kernel(int T, int C, int H,
                                                            const void* __restrict__ w_, int w_raw,
                                                            const E* __restrict__ u_, const void* __restrict__ s0_,
                                                            int s0_kind, E* __restrict__ y_, float* __restrict__ sT_,
-                                                           const int* __restrict__ only_if_) {
-    if (only_if_ != nullptr && only_if_[blockIdx.x & (kChunkedFlagUnits - 1)] == 0) return;   // fallback launch: the chunked kernel's result stands for this unit
+                                                           const int* __restrict__ only_if_, int only_mask) {
+    if (only_if_ != nullptr && only_if_[blockIdx.x & only_mask] == 0) return;   // fallback launch: the chunked kernel's result stands for this unit
     const int b = blockIdx.x / H, h = blockIdx.x - b * H, i = threadIdx.x;
     const bool live = i < N;
     __shared__ Stage<NMAX> rs, ks, ds;
@@ -130,8 +130,8 @@ __global__ void __launch_bounds__(NMAX) wkv6_backward_kernel(
     const void* __restrict__ w_, int w_raw, const E* __restrict__ u_, const void* __restrict__ s0_, int s0_kind,
     const E* __restrict__ gy_, const float* __restrict__ dsT_, E* __restrict__ gr_, E* __restrict__ gk_,
     E* __restrict__ gv_, E* __restrict__ gw_, E* __restrict__ gu_, void* __restrict__ ds0_, int ds0_kind,
-    float* __restrict__ scratch_, const int* __restrict__ only_if_) {
-    if (only_if_ != nullptr && only_if_[blockIdx.x & (kChunkedFlagUnits - 1)] == 0) return;   // fallback launch: the chunked kernels' result stands for this unit
+    float* __restrict__ scratch_, const int* __restrict__ only_if_, int only_mask, float* __restrict__ gu32_) {
+    if (only_if_ != nullptr && only_if_[blockIdx.x & only_mask] == 0) return;   // fallback launch: the chunked kernels' result stands for this unit
     const int b = blockIdx.x / H, h = blockIdx.x - b * H, i = threadIdx.x;
     const bool live = i < N;
     __shared__ Stage<NMAX> rs, ks, vs, gs, ds;
@@ -180,7 +180,8 @@ __global__ void __launch_bounds__(NMAX) wkv6_backward_kernel(
             }
             gu = fmaf(r * k, vg, gu);
         }
-        if (live) gu_[(i64)b * C + h * N + i] = from_f<E>(gu);
+        if (live && gu_ != nullptr) gu_[(i64)b * C + h * N + i] = from_f<E>(gu);
+        if (live && gu32_ != nullptr) gu32_[(i64)b * C + h * N + i] = gu;   // unrounded
         if (dsT_ != nullptr && live) {
 #pragma unroll
             for (int j = 0; j < NMAX; ++j)
@@ -274,7 +275,7 @@ int launch_fwd(int B, int T, int C, int H, const void* r, const void* k, const v
     }
 #define RWKV_GO(NM)                                                                                              \
     wkv6_forward_kernel<E, NM><<<B * H, NM, 0, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, w, w_raw, \
-                                                      (const E*)u, s0, s0_kind, (E*)y, sT, only_if)
+                                                      (const E*)u, s0, s0_kind, (E*)y, sT, only_if, kChunkedFlagUnits - 1)
     switch (head_capacity(N)) {
         case 32: RWKV_GO(32); break;
         case 64: RWKV_GO(64); break;
@@ -288,7 +289,7 @@ template <typename E>
 int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, int w_raw,
                const void* u, const void* s0, int s0_kind, const void* gy, const float* dsT, void* gr, void* gk,
                void* gv, void* gw, void* gu, void* ds0, int ds0_kind, void* scratch, cudaStream_t st,
-               const char* what, bool big_scratch = true) {
+               const char* what, bool big_scratch = true, float* gu32 = nullptr) {
     const int N = C / H;
     const int* only_if = nullptr;
     if (big_scratch && T % 16 == 0 && chunked_ok<E>(T, N, true, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, scratch})) {
@@ -300,7 +301,7 @@ int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const v
             RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA, "%s: clearing the device flag failed", what);
             float* ck = static_cast<float*>(scratch);
             if (int e = wkv6_backward_with_states(B, T, H, r, k, v, w, w_raw, u, s0, s0_kind, gy, dsT, ck, gr, gk, gv, gw, gu, ds0,
-                                                  ds0_kind, flag, st))
+                                                  ds0_kind, flag, st, nullptr, gu32))
                 return e;
             only_if = flag;
         }
@@ -309,13 +310,42 @@ int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const v
     wkv6_backward_kernel<E, NM><<<B * H, NM, 0, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, w, w_raw, \
                                                        (const E*)u, s0, s0_kind, (const E*)gy, dsT, (E*)gr,       \
                                                        (E*)gk, (E*)gv, (E*)gw, (E*)gu, ds0, ds0_kind,             \
-                                                       (float*)scratch, only_if)
+                                                       (float*)scratch, only_if, kChunkedFlagUnits - 1, gu32)
     switch (head_capacity(N)) {
         case 32: RWKV_GO(32); break;
         case 64: RWKV_GO(64); break;
         default: RWKV_GO(128); break;
     }
 #undef RWKV_GO
+    return check_launch(what);
+}
+
+// Forward on the tcgen05 kernel that leaves the chunk-start states and the flags of its units in `saved`, and the general-shape
+// kernel for the flagged units.  1: not for this call (nothing is enqueued).
+int tensor_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
+                   const float* s0, void* y, float* sT, void* saved, cudaStream_t st, const char* what) {
+    const int N = C / H, sk = s0 ? kF32 : kNone;
+    if (dtype != RWKVB200_BF16 || !wkv6_forward_choice() || !chunked_ok<bf16>(T, N, sT != nullptr, {r, k, v, w, u, s0, y, sT, saved})) return 1;
+    int* flags = wkv6_saved_flags(saved, B, T, H);
+    const int rc = wkv6_l32_forward(B, T, H, r, k, v, w, 1, u, s0, sk, y, sT, static_cast<float*>(saved), flags, st, 0);
+    if (rc != 0) return rc;
+    wkv6_forward_kernel<bf16, 64><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w, 1, (const bf16*)u, s0,
+                                                       sk, (bf16*)y, sT, flags, -1);
+    return check_launch(what);
+}
+
+// The backward that goes with it; scratch: (B,T,C) floats for the flagged units (may be `saved`).
+int tensor_backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, const float* s0,
+                    const void* gy, const float* dsT, void* gr, void* gk, void* gv, void* gw, void* gu, float* ds0, float* gu32, void* saved,
+                    float* scratch, cudaStream_t st, const char* what) {
+    const int N = C / H, sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
+    const int* flags = wkv6_saved_flags(saved, B, T, H);
+    if (int e = wkv6_l32_backward(B, T, H, r, k, v, w, 1, u, gy, dsT, static_cast<const float*>(saved), gr, gk, gv, gw, gu, ds0, dk, st, nullptr,
+                                  gu32, 0, flags))
+        return e;
+    wkv6_backward_kernel<bf16, 64><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w, 1, (const bf16*)u, s0,
+                                                        sk, (const bf16*)gy, dsT, (bf16*)gr, (bf16*)gk, (bf16*)gv, (bf16*)gw, (bf16*)gu,
+                                                        ds0, dk, scratch, flags, -1, gu32);
     return check_launch(what);
 }
 
@@ -492,7 +522,7 @@ extern "C" int rwkvb200_wkv6state_forward_tsplit(int dtype, int B, int T, int C,
     if (int e = wkv6_chunked_forward(B * K, T / K, H, r, k, v, w, 1, u, start, kF32, y, nullptr, nullptr, flag, st, K)) return e;
     // a chunk whose decay is too strong for the chunked form: the general-shape kernel redoes the call
     wkv6_forward_kernel<bf16, 64><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w, 1,
-                                                       (const bf16*)u, s0, s0 ? kF32 : kNone, (bf16*)y, sT, flag);
+                                                       (const bf16*)u, s0, s0 ? kF32 : kNone, (bf16*)y, sT, flag, kChunkedFlagUnits - 1);
     return check_launch("wkv6state_forward_tsplit");
 }
 
@@ -507,26 +537,11 @@ extern "C" int rwkvb200_wkv6state_forward_saved(int dtype, int B, int T, int C, 
                                                 float* sT, void* saved, void* stream) {
     if (int e = check_dims("wkv6state_forward_saved", dtype, B, T, C, H)) return e;
     RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w); RWKV_NOTNULL(u); RWKV_NOTNULL(y); RWKV_NOTNULL(saved);
-    const int N = C / H, sk = s0 ? kF32 : kNone;
+    const int sk = s0 ? kF32 : kNone;
     cudaStream_t st = as_stream(stream);
-    int* flag = nullptr;
-    if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && wkv6_states_fit(B, T, H) && chunked_ok<bf16>(T, N, sT != nullptr, {r, k, v, w, u, s0, y, sT, saved}))
-        flag = wkv6_chunked_flag(st);
-    if (flag != nullptr) {
-        RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA,
-                     "wkv6state_forward_saved: clearing the device flags failed");
-        const int rc = wkv6_l32_forward(B, T, H, r, k, v, w, 1, u, s0, sk, y, sT, static_cast<float*>(saved), flag, st, 1);
-        if (rc < 0) return rc;
-        if (rc == 0) {
-            // flagged units: the general-shape kernel redoes them; the flags travel with the saved states
-            wkv6_forward_kernel<bf16, 64><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w, 1,
-                                                               (const bf16*)u, s0, sk, (bf16*)y, sT, flag);
-            if (int e = check_launch("wkv6state_forward_saved")) return e;
-            char* tail = static_cast<char*>(saved) + rwkvb200_wkv6_scratch_bytes(B, T, C) - sizeof(int) * kChunkedFlagUnits;
-            RWKV_REQUIRE(cudaMemcpyAsync(tail, flag, sizeof(int) * kChunkedFlagUnits, cudaMemcpyDeviceToDevice, st) == cudaSuccess,
-                         RWKVB200_ECUDA, "wkv6state_forward_saved: saving the device flags failed");
-            return RWKVB200_OK;
-        }
+    if (wkv6_states_fit(B, T, H)) {
+        const int rc = tensor_forward(dtype, B, T, C, H, r, k, v, w, u, s0, y, sT, saved, st, "wkv6state_forward_saved");
+        if (rc != 1) return rc;
     }
     const int e = dtype == RWKVB200_F32
                       ? launch_fwd<float>(B, T, C, H, r, k, v, w, 1, u, s0, sk, y, sT, st, "wkv6state_forward_saved")
@@ -541,27 +556,64 @@ extern "C" int rwkvb200_wkv6state_backward_saved(int dtype, int B, int T, int C,
     if (int e = check_dims("wkv6state_backward_saved", dtype, B, T, C, H)) return e;
     RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w); RWKV_NOTNULL(u); RWKV_NOTNULL(gy);
     RWKV_NOTNULL(gr); RWKV_NOTNULL(gk); RWKV_NOTNULL(gv); RWKV_NOTNULL(gw); RWKV_NOTNULL(gu); RWKV_NOTNULL(saved);
-    const int N = C / H, sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
+    const int sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
     cudaStream_t st = as_stream(stream);
-    int* flag = nullptr;
-    if (saved_valid && dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, N, ds0 != nullptr, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, saved}))
-        flag = wkv6_chunked_flag(st);
-    if (flag != nullptr) {
-        const char* tail = static_cast<const char*>(saved) + rwkvb200_wkv6_scratch_bytes(B, T, C) - sizeof(int) * kChunkedFlagUnits;
-        RWKV_REQUIRE(cudaMemcpyAsync(flag, tail, sizeof(int) * kChunkedFlagUnits, cudaMemcpyDeviceToDevice, st) == cudaSuccess,
-                     RWKVB200_ECUDA, "wkv6state_backward_saved: restoring the device flags failed");
-        if (int e = wkv6_l32_backward(B, T, H, r, k, v, w, 1, u, gy, dsT, static_cast<const float*>(saved), gr, gk, gv, gw, gu, ds0, dk, st))
-            return e;
-        // flagged units: the general-shape kernel redoes them (it uses the front of `saved` as its scratch, after
-        // the kernel above has read the states)
-        wkv6_backward_kernel<bf16, 64><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w, 1,
-                                                            (const bf16*)u, s0, sk, (const bf16*)gy, dsT, (bf16*)gr, (bf16*)gk,
-                                                            (bf16*)gv, (bf16*)gw, (bf16*)gu, ds0, dk, static_cast<float*>(saved), flag);
-        return check_launch("wkv6state_backward_saved");
-    }
+    if (saved_valid && dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, C / H, ds0 != nullptr, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, saved}))
+        // (flagged units: the general-shape kernel uses the front of `saved` as its scratch, after the states have been read)
+        return tensor_backward(B, T, C, H, r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, nullptr, saved, static_cast<float*>(saved), st, "wkv6state_backward_saved");
     return dtype == RWKVB200_F32
                ? launch_bwd<float>(B, T, C, H, r, k, v, w, 1, u, s0, sk, gy, dsT, gr, gk, gv, gw, gu, ds0, dk, saved, st, "wkv6state_backward_saved")
                : launch_bwd<bf16>(B, T, C, H, r, k, v, w, 1, u, s0, sk, gy, dsT, gr, gk, gv, gw, gu, ds0, dk, saved, st, "wkv6state_backward_saved");
+}
+
+// ---- training flow: gu summed over the batch inside the library, buffers of the size that the path needs -----------------
+// (the flagged units of the tcgen05 backward use the states in `saved` as scratch, as in rwkvb200_wkv6state_backward_saved:
+// they hold 2 floats per element and the scratch takes one)
+extern "C" size_t rwkvb200_wkv6_train_saved_bytes(int dtype, int B, int T, int C, int H) {
+    if (B <= 0 || T <= 0 || C <= 0 || H <= 0 || dtype != RWKVB200_BF16 || C / H != 64) return 16;
+    return (size_t)B * H * ((size_t)((T + 31) / 32) * 64 * 64 + 1) * sizeof(float);
+}
+
+extern "C" int rwkvb200_wkv6_train_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w,
+                                           const void* u, const float* s0, void* y, float* sT, void* saved, void* stream) {
+    if (int e = check_dims("wkv6_train_forward", dtype, B, T, C, H)) return e;
+    RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w); RWKV_NOTNULL(u); RWKV_NOTNULL(y); RWKV_NOTNULL(saved);
+    cudaStream_t st = as_stream(stream);
+    const int rc = tensor_forward(dtype, B, T, C, H, r, k, v, w, u, s0, y, sT, saved, st, "wkv6_train_forward");
+    if (rc != 1) return rc;
+    const int sk = s0 ? kF32 : kNone;
+    const int e = dtype == RWKVB200_F32 ? launch_fwd<float>(B, T, C, H, r, k, v, w, 1, u, s0, sk, y, sT, st, "wkv6_train_forward")
+                                        : launch_fwd<bf16>(B, T, C, H, r, k, v, w, 1, u, s0, sk, y, sT, st, "wkv6_train_forward");
+    return e ? e : 1;
+}
+
+extern "C" size_t rwkvb200_wkv6_train_work_bytes(int B, int T, int C, int path) {
+    if (B <= 0 || T <= 0 || C <= 0) return 0;
+    return (size_t)B * C * sizeof(float) + (path == 0 ? 0 : rwkvb200_wkv6_scratch_bytes(B, T, C));
+}
+
+extern "C" int rwkvb200_wkv6_train_backward(int dtype, int B, int T, int C, int H, int path, const void* r, const void* k, const void* v,
+                                            const void* w, const void* u, const float* s0, const void* gy, const float* dsT, void* gr,
+                                            void* gk, void* gv, void* gw, void* gu, float* ds0, void* saved, void* work, void* stream) {
+    if (int e = check_dims("wkv6_train_backward", dtype, B, T, C, H)) return e;
+    RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w); RWKV_NOTNULL(u); RWKV_NOTNULL(gy);
+    RWKV_NOTNULL(gr); RWKV_NOTNULL(gk); RWKV_NOTNULL(gv); RWKV_NOTNULL(gw); RWKV_NOTNULL(gu); RWKV_NOTNULL(saved); RWKV_NOTNULL(work);
+    cudaStream_t st = as_stream(stream);
+    const int sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
+    float* scratch = static_cast<float*>(work);   // (path 1; the partials of gu come behind it)
+    float* gu32 = path == 0 ? scratch : scratch + rwkvb200_wkv6_scratch_bytes(B, T, C) / sizeof(float);
+    int e;
+    if (path == 0) {
+        RWKV_REQUIRE(dtype == RWKVB200_BF16 && C / H == 64, RWKVB200_EINVAL, "wkv6_train_backward: path 0 is bf16, head size 64");
+        for (const void* p : std::initializer_list<const void*>{r, k, v, w, gy, dsT, gr, gk, gv, gw, ds0, saved})
+            RWKV_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15) == 0, RWKVB200_EALIGN, "wkv6_train_backward: the bf16 N=64 path needs 16-byte aligned tensors");
+        e = tensor_backward(B, T, C, H, r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, nullptr, ds0, gu32, saved, static_cast<float*>(saved), st, "wkv6_train_backward");
+    } else {
+        e = dtype == RWKVB200_F32
+                ? launch_bwd<float>(B, T, C, H, r, k, v, w, 1, u, s0, sk, gy, dsT, gr, gk, gv, gw, nullptr, ds0, dk, scratch, st, "wkv6_train_backward", true, gu32)
+                : launch_bwd<bf16>(B, T, C, H, r, k, v, w, 1, u, s0, sk, gy, dsT, gr, gk, gv, gw, nullptr, ds0, dk, scratch, st, "wkv6_train_backward", true, gu32);
+    }
+    return e ? e : sum_rows(dtype, B, C, gu32, gu, st);
 }
 
 extern "C" int rwkvb200_wkv6state_backward_ex(int dtype, int B, int T, int C, int H, const void* r, const void* k,

@@ -595,7 +595,7 @@ wkv6c_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     for (int h2 = 0; h2 < 2; ++h2) {
         gu_acc[h2] += __shfl_xor_sync(0xffffffffu, gu_acc[h2], 1);
         gu_acc[h2] += __shfl_xor_sync(0xffffffffu, gu_acc[h2], 2);
-        if (t == 0) gu_[(i64)bb * C + hh * N + row0 + 2 * g + h2] = __float2bfloat16_rn(gu_acc[h2]);
+        if (t == 0 && gu_ != nullptr) gu_[(i64)bb * C + hh * N + row0 + 2 * g + h2] = __float2bfloat16_rn(gu_acc[h2]);
         if (t == 0 && gu32_ != nullptr) gu32_[(i64)bb * C + hh * N + row0 + 2 * g + h2] = gu_acc[h2];   // unrounded
         if (gw_reduce) {
             gw_acc[h2] += __shfl_xor_sync(0xffffffffu, gw_acc[h2], 1);

@@ -63,15 +63,16 @@ __device__ __forceinline__ void store_state(void* p, int kind, i64 idx, float x)
 }
 
 // WMODE as in wkv6_l32_fwd.cu: 0 = fp32 log-decay (B,T,C), 1 = bf16 raw input (B,T,C), 2 = fp32 decay value (C),
-// 3 = fp32 log-decay (C)
+// 3 = fp32 log-decay (C), 4 = bf16 raw input (C).  flags_: units whose flag is set are left to the general-shape kernel.
+// gu_ (and gw_ of a static decay): (B,C) bf16 or NULL; gw32_, gu32_: the same unrounded or NULL, rows gstride apart
 template <int WMODE>
 __global__ void __launch_bounds__(BNT, 2)
 wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __restrict__ k_, const bf16* __restrict__ v_,
                       const void* __restrict__ w_, const bf16* __restrict__ u_, const bf16* __restrict__ gy_,
                       const float* __restrict__ dsT_, const float* __restrict__ ck_, bf16* __restrict__ gr_,
                       bf16* __restrict__ gk_, bf16* __restrict__ gv_, bf16* __restrict__ gw_, bf16* __restrict__ gu_,
-                      void* __restrict__ ds0_, int ds0_kind, float* __restrict__ gw32_, float* __restrict__ gu32_,
-                      const __grid_constant__ TileMaps<5> maps) {
+                      void* __restrict__ ds0_, int ds0_kind, float* __restrict__ gw32_, float* __restrict__ gu32_, i64 gstride,
+                      const int* __restrict__ flags_, const __grid_constant__ TileMaps<5> maps) {
     constexpr bool kStatic = WMODE >= 2;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -88,6 +89,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     unsigned char* Raw = smem + Smem::kRaw;
 
     const int hh = blockIdx.x, bb = blockIdx.y;
+    if (flags_ != nullptr && flags_[bb * H + hh] != 0) return;
     const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int quarter = warp & 3, hs = warp >> 2;
@@ -143,6 +145,9 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     } else if (WMODE == 3) {
         ls0 = reinterpret_cast<const float*>(w_)[hh * 64 + j0] * 1.4426950408889634f;
         ls1 = reinterpret_cast<const float*>(w_)[hh * 64 + j0 + 1] * 1.4426950408889634f;
+    } else if (WMODE == 4) {
+        ls0 = -expf(__bfloat162float(reinterpret_cast<const bf16*>(w_)[hh * 64 + j0])) * 1.4426950408889634f;
+        ls1 = -expf(__bfloat162float(reinterpret_cast<const bf16*>(w_)[hh * 64 + j0 + 1])) * 1.4426950408889634f;
     }
 
     RawChunk<4, BTPW> raw;
@@ -514,11 +519,11 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             for (int h = 0; h < 2; ++h) {
                 const int j = row0 + g + 8 * h;
                 const float gu = gu_acc[h] + A0p[j], gw = gw_acc[h] + A0p[64 + j];
-                gu_[(i64)bb * C + hh * 64 + j] = __float2bfloat16_rn(gu);
-                if (gu32_ != nullptr) gu32_[(i64)bb * C + hh * 64 + j] = gu;
+                if (gu_ != nullptr) gu_[(i64)bb * C + hh * 64 + j] = __float2bfloat16_rn(gu);
+                if (gu32_ != nullptr) gu32_[bb * gstride + hh * 64 + j] = gu;
                 if (kStatic) {
-                    gw_[(i64)bb * C + hh * 64 + j] = __float2bfloat16_rn(gw);
-                    if (gw32_ != nullptr) gw32_[(i64)bb * C + hh * 64 + j] = gw;
+                    if (gw_ != nullptr) gw_[(i64)bb * C + hh * 64 + j] = __float2bfloat16_rn(gw);
+                    if (gw32_ != nullptr) gw32_[bb * gstride + hh * 64 + j] = gw;
                 }
             }
         }
@@ -544,8 +549,9 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 // by wkv6_l32_forward with its `ck` argument).
 int wkv6_l32_backward(int B, int T, int H, const void* r, const void* k, const void* v, const void* w, int w_mode, const void* u,
                       const void* gy, const float* dsT, const float* ck, void* gr, void* gk, void* gv, void* gw, void* gu,
-                      void* ds0, int ds0_kind, cudaStream_t st, float* gw32, float* gu32) {
+                      void* ds0, int ds0_kind, cudaStream_t st, float* gw32, float* gu32, long long gstride, const int* flags) {
     using namespace v6b;
+    if (gstride == 0) gstride = (i64)H * 64;
     TileMaps<5> maps;
     const void* in[5] = {r, k, v, gy, w_mode <= 1 ? w : r};
     maps.valid = 1;
@@ -559,13 +565,14 @@ int wkv6_l32_backward(int B, int T, int H, const void* r, const void* k, const v
         wkv6b_backward_kernel<M><<<grid, BNT, Smem::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)k, (const bf16*)v, w,  \
                                                                  (const bf16*)u, (const bf16*)gy, dsT, ck, (bf16*)gr,    \
                                                                  (bf16*)gk, (bf16*)gv, (bf16*)gw, (bf16*)gu, ds0,        \
-                                                                 ds0_kind, gw32, gu32, maps);                            \
+                                                                 ds0_kind, gw32, gu32, gstride, flags, maps);            \
     } while (0)
     switch (w_mode) {
         case 0: RWKV_GO(0); break;
         case 1: RWKV_GO(1); break;
         case 2: RWKV_GO(2); break;
-        default: RWKV_GO(3); break;
+        case 3: RWKV_GO(3); break;
+        default: RWKV_GO(4); break;
     }
 #undef RWKV_GO
     return check_launch("wkv6_backward(tcgen05, 32-token chunks)");

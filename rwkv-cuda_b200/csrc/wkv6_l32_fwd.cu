@@ -74,7 +74,7 @@ enum { kFullA = 0, kEmptyA = kFullA + NA, kFullU = kEmptyA + NA, kEmptyU = kFull
        kRawFull, kNBar = kRawFull + NS };
 
 // WMODE: 0 = fp32 log-decay (B,T,C), 1 = bf16 raw input (B,T,C) with log-decay = -exp(w), 2 = fp32 decay value (C),
-// 3 = fp32 log-decay (C)   (the forms of wkv6_chunked.cu)
+// 3 = fp32 log-decay (C)   (the forms of wkv6_chunked.cu), 4 = bf16 raw input (C) with log-decay = -exp(w)
 template <int WMODE>
 __global__ void __launch_bounds__(PNT, 1)
 wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void* __restrict__ wstat_, const bf16* __restrict__ u_,
@@ -135,8 +135,12 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
         } else if (WMODE == 3) {
             ls0 = reinterpret_cast<const float*>(wstat_)[hh * 64 + j0] * 1.4426950408889634f;
             ls1 = reinterpret_cast<const float*>(wstat_)[hh * 64 + j0 + 1] * 1.4426950408889634f;
+        } else if (WMODE == 4) {
+            ls0 = -expf(__bfloat162float(reinterpret_cast<const bf16*>(wstat_)[hh * 64 + j0])) * 1.4426950408889634f;
+            ls1 = -expf(__bfloat162float(reinterpret_cast<const bf16*>(wstat_)[hh * 64 + j0 + 1])) * 1.4426950408889634f;
         }
         int issued = 0;
+        bool too_strong = false;
         auto issue_raw = [&](int c) {   // every warp's lane 0 issues its share of the tiles
             const int st = c & 1;
             uint64_t* fb = bar + kRawFull + st;
@@ -202,8 +206,7 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             }
             if (wg == 0) {
                 *reinterpret_cast<float2*>(We + j0) = make_float2(fex2(tot0), fex2(tot1));
-                if (-tot0 > kMaxChunkLog2Decay || -tot1 > kMaxChunkLog2Decay)   // this unit must be redone by the general-shape kernel
-                    atomicOr(unsafe_ + (((bb / flag_div) * H + hh) & (kChunkedFlagUnits - 1)), 1);
+                too_strong |= -tot0 > kMaxChunkLog2Decay || -tot1 > kMaxChunkLog2Decay;
             }
             float lp0 = base0, lp1 = base1;   // log2 P_{t-1}
 #pragma unroll
@@ -224,6 +227,11 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             group_sync(gbar, GNT);
             if (gtid == 0) mbar_arrive(bar + kFullA + sa);
             if (++sa == NA) { sa = 0; ++ua; }
+        }
+        if (wg == 0) {   // a unit with a decay too strong for the chunked form is redone by the general-shape kernel
+            const int any = __any_sync(0xffffffffu, too_strong);
+            if (lane == 0 && flag_div == 0) unsafe_[bb * H + hh] = any;
+            else if (lane == 0 && any) atomicOr(unsafe_ + (((bb / flag_div) * H + hh) & (kChunkedFlagUnits - 1)), 1);
         }
         if (fail) atomicMax(const_cast<int*>(abort_word), fail);
         for (int cc = c; cc < issued; ++cc) mbar_wait(bar + kRawFull + (cc & 1), (cc >> 1) & 1);
@@ -466,7 +474,8 @@ int wkv6_l32_forward(int B, int T, int H, const void* r, const void* k, const vo
         case 0: RWKV_GO(0); break;
         case 1: RWKV_GO(1); break;
         case 2: RWKV_GO(2); break;
-        default: RWKV_GO(3); break;
+        case 3: RWKV_GO(3); break;
+        default: RWKV_GO(4); break;
     }
 #undef RWKV_GO
     return check_launch("wkv6_forward(tcgen05, 32-token chunks, three stages)");

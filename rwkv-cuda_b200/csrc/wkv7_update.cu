@@ -20,6 +20,7 @@
 // One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 212 us here (106 ns per token); 256 units
 // 2045 -> 870 us.
 #include "common.cuh"
+#include "packed.cuh"
 #include "wkv7_dispatch.cuh"
 
 namespace rwkvb200 {
@@ -85,27 +86,6 @@ __global__ void __launch_bounds__(128) wkv7_decode_kernel(float* __restrict__ st
 }
 
 // ---- prompts ----------------------------------------------------------------------------------------------
-using f2 = unsigned long long;   // two packed fp32
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-    f2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ float sum2(f2 a) {
-    float lo, hi;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
-    return lo + hi;
-}
 // The 64 / LG keys of lane x of a row (LG = 8 or 16 lanes).  In shared memory the first four of every eight keys come
 // first, then the other four, so that eight lanes read and write 128 consecutive bytes: staged_at(key) is the place.
 __device__ __forceinline__ int staged_at(int ch) { return ((ch & 4) << 3) + ((ch >> 3) << 2) + (ch & 3); }

@@ -145,12 +145,95 @@ struct TimeX : torch::autograd::Function<TimeX> {
     }
 };
 
+// ---- RWKV-5 ---------------------------------------------------------------------------------------------------
+static Tensor bytes(size_t n, const Tensor& like) { return empty({(int64_t)n}, at::kByte, like); }
+
+struct Wkv5 : torch::autograd::Function<Wkv5> {
+    static Tensor forward(AutogradContext* ctx, int64_t B, int64_t T, int64_t C, int64_t H, Tensor r, Tensor k, Tensor v, Tensor w, Tensor u) {
+        for (const Tensor* x : {&k, &v, &w, &u}) assert_py(x->scalar_type() == r.scalar_type(), "r, k, v, w, u must have one dtype");
+        on_device(r, "r");
+        const c10::cuda::CUDAGuard guard(r.device());
+        const auto d = r.scalar_type();
+        const int dtype = dt(r, "r");
+        r = r.contiguous(); k = k.contiguous(); v = v.contiguous(); w = w.contiguous(); u = u.contiguous();
+        numel(r, B * T * C, "r"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v"); numel(w, C, "w"); numel(u, C, "u");
+        Tensor y = empty({B, T, C}, d, r), saved = bytes(rwkvb200_wkv5_train_saved_bytes(B, T, C, H), r);
+        const int path = rwkvb200_wkv5_train_forward(dtype, B, T, C, H, ptr(r, "r", d), ptr(k, "k", d), ptr(v, "v", d), ptr(w, "w", d),
+                                                     ptr(u, "u", d), y.data_ptr(), saved.data_ptr(), stream());
+        check_rc(path, "rwkvb200_wkv5_train_forward");
+        ctx->save_for_backward({r, k, v, w, u, saved});
+        ctx->saved_data["dims"] = std::vector<int64_t>{B, T, C, H, path};
+        return y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const auto s = ctx->get_saved_variables();
+        const auto dims = ctx->saved_data["dims"].toIntVector();
+        const int64_t B = dims[0], T = dims[1], C = dims[2], H = dims[3], path = dims[4];
+        const c10::cuda::CUDAGuard guard(s[0].device());
+        const auto d = s[0].scalar_type();
+        const Tensor gy = g[0].contiguous();
+        numel(gy, B * T * C, "gy");
+        Tensor gr = empty({B, T, C}, d, gy), gk = empty({B, T, C}, d, gy), gv = empty({B, T, C}, d, gy), gwu = empty({2, C}, d, gy);
+        Tensor work = bytes(rwkvb200_wkv5_train_work_bytes(B, T, C, H, path), gy);
+        check_rc(rwkvb200_wkv5_train_backward(dt(s[0], "r"), B, T, C, H, path, s[0].data_ptr(), s[1].data_ptr(), s[2].data_ptr(), s[3].data_ptr(),
+                                              s[4].data_ptr(), ptr(gy, "gy", d), gr.data_ptr(), gk.data_ptr(), gv.data_ptr(), gwu.data_ptr(),
+                                              s[5].data_ptr(), work.data_ptr(), stream()),
+                 "rwkvb200_wkv5_train_backward", true);
+        return {Tensor(), Tensor(), Tensor(), Tensor(), gr, gk, gv, gwu.select(0, 0).view_as(s[3]), gwu.select(0, 1).view_as(s[4])};
+    }
+};
+
+// ---- RWKV-6, without a state (kState = false) or with an fp32 state in and out ----------------------------------------
+template <bool kState>
+struct Wkv6 : torch::autograd::Function<Wkv6<kState>> {
+    static variable_list forward(AutogradContext* ctx, int64_t B, int64_t T, int64_t C, int64_t H, Tensor r, Tensor k, Tensor v, Tensor w,
+                                 Tensor u, std::optional<Tensor> state) {
+        on_device(r, "r");
+        Tensor s0 = kState ? state->contiguous() : Tensor();
+        const c10::cuda::CUDAGuard guard(r.device());
+        const auto d = r.scalar_type(), f = at::kFloat;
+        const int dtype = dt(r, "r");
+        r = r.contiguous(); k = k.contiguous(); v = v.contiguous(); w = w.contiguous(); u = u.contiguous();
+        numel(r, B * T * C, "r"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v"); numel(w, B * T * C, "w"); numel(u, C, "u");
+        if (kState) numel(s0, B * H * (C / H) * (C / H), "s0");
+        Tensor y = empty({B, T, C}, d, r), sT = kState ? same(s0) : Tensor();
+        Tensor saved = bytes(rwkvb200_wkv6_train_saved_bytes(dtype, B, T, C, H), r);
+        const int path = rwkvb200_wkv6_train_forward(dtype, B, T, C, H, ptr(r, "r", d), ptr(k, "k", d), ptr(v, "v", d), ptr(w, "w", d), ptr(u, "u", d),
+                                                     kState ? f32(ptr(s0, "s0", f)) : nullptr, y.data_ptr(), kState ? f32(sT.data_ptr()) : nullptr,
+                                                     saved.data_ptr(), stream());
+        check_rc(path, "rwkvb200_wkv6_train_forward");
+        ctx->save_for_backward({r, k, v, w, u, saved, kState ? s0 : saved});
+        ctx->saved_data["dims"] = std::vector<int64_t>{B, T, C, H, path};
+        if (kState) return {y, sT};
+        return {y};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list g) {
+        const auto s = ctx->get_saved_variables();
+        const auto dims = ctx->saved_data["dims"].toIntVector();
+        const int64_t B = dims[0], T = dims[1], C = dims[2], H = dims[3], path = dims[4];
+        const c10::cuda::CUDAGuard guard(s[0].device());
+        const auto d = s[0].scalar_type(), f = at::kFloat;
+        const Tensor gy = g[0].contiguous(), dsT = kState ? g[1].contiguous() : Tensor();
+        numel(gy, B * T * C, "gy");
+        Tensor gr = empty({B, T, C}, d, gy), gk = empty({B, T, C}, d, gy), gv = empty({B, T, C}, d, gy), gw = empty({B, T, C}, d, gy);
+        Tensor gu = empty(s[4].sizes(), d, gy), ds0 = kState ? same(s[6]) : Tensor();
+        Tensor work = bytes(rwkvb200_wkv6_train_work_bytes(B, T, C, path), gy);
+        check_rc(rwkvb200_wkv6_train_backward(dt(s[0], "r"), B, T, C, H, path, s[0].data_ptr(), s[1].data_ptr(), s[2].data_ptr(), s[3].data_ptr(),
+                                              s[4].data_ptr(), kState ? f32(s[6].data_ptr()) : nullptr, ptr(gy, "gy", d),
+                                              kState ? f32(ptr(dsT, "dsT", f)) : nullptr, gr.data_ptr(), gk.data_ptr(), gv.data_ptr(), gw.data_ptr(),
+                                              gu.data_ptr(), kState ? f32(ds0.data_ptr()) : nullptr, s[5].data_ptr(), work.data_ptr(), stream()),
+                 "rwkvb200_wkv6_train_backward", true);
+        return {Tensor(), Tensor(), Tensor(), Tensor(), gr, gk, gv, gw, gu, ds0};
+    }
+};
+
 // ---- RWKV-7, the three operators: state in (s0) and out (sT) or not ---------------------------------------------
 constexpr int64_t kChunkLen = 16;
 
 template <bool kS0, bool kST>
 struct Wkv7 : torch::autograd::Function<Wkv7<kS0, kST>> {
-    static variable_list forward(AutogradContext* ctx, Tensor s0, Tensor r, Tensor w, Tensor k, Tensor v, Tensor a, Tensor b) {
+    static variable_list forward(AutogradContext* ctx, std::optional<Tensor> state, Tensor r, Tensor w, Tensor k, Tensor v, Tensor a, Tensor b) {
+        const Tensor s0 = kS0 ? *state : Tensor();
         assert_py(r.dim() == 4 && r.size(1) % kChunkLen == 0, "T must be a multiple of 16");
         for (const Tensor* x : {&w, &k, &v, &a, &b}) assert_py(x->scalar_type() == r.scalar_type(), "r, w, k, v, a, b must have one dtype");
         for (const Tensor* x : {&r, &w, &k, &v, &a, &b}) assert_py(x->is_contiguous(), "r, w, k, v, a, b must be contiguous");
@@ -196,14 +279,25 @@ PYBIND11_MODULE(_native, m) {
         return Wkv4::apply(B, T, C, w, u, k, v);
     });
     m.def("timex", [](const Tensor& w, const Tensor& k, int64_t B, int64_t C, int64_t T, double eps) { return TimeX::apply(w, k, B, C, T, eps); });
+    m.def("wkv5", [](int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
+        return Wkv5::apply(B, T, C, H, r, k, v, w, u);
+    });
+    m.def("wkv6", [](int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
+        return Wkv6<false>::apply(B, T, C, H, r, k, v, w, u, std::optional<Tensor>())[0];
+    });
+    m.def("wkv6_state", [](const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u, const Tensor& s0) {
+        TORCH_CHECK_VALUE(r.dim() == 3, "r: expected (B,T,C), got ", r.sizes());
+        const auto out = Wkv6<true>::apply(r.size(0), r.size(1), r.size(2), u.size(0), r, k, v, w, u, std::optional<Tensor>(s0));
+        return std::make_tuple(out[0], out[1]);
+    });
     m.def("wkv7", [](const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        return Wkv7<false, false>::apply(Tensor(), r, w, k, v, a, b)[0];
+        return Wkv7<false, false>::apply(std::optional<Tensor>(), r, w, k, v, a, b)[0];
     });
     m.def("wkv7_state", [](const Tensor& s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        return Wkv7<true, false>::apply(s0, r, w, k, v, a, b)[0];
+        return Wkv7<true, false>::apply(std::optional<Tensor>(s0), r, w, k, v, a, b)[0];
     });
     m.def("wkv7_statepassing", [](const Tensor& s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        const auto out = Wkv7<true, true>::apply(s0, r, w, k, v, a, b);
+        const auto out = Wkv7<true, true>::apply(std::optional<Tensor>(s0), r, w, k, v, a, b);
         return std::make_tuple(out[0], out[1]);
     });
 }

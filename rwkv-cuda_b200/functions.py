@@ -26,40 +26,12 @@ class TimeX(torch.autograd.Function):
 
 
 class WKV_5(torch.autograd.Function):
-    """RWKV-5, bf16 or fp32 (wkv5_bf16/run.py:44-88, wkv5/run.py:469-504)."""
+    """RWKV-5, bf16 or fp32 (wkv5_bf16/run.py:44-88, wkv5/run.py:469-504): w is the raw decay input.  The harness sums bf16
+    (B,C) partials of gw, gu in bf16 (wkv5_bf16/run.py:83-87); here they are summed in fp32 and rounded once."""
 
     @staticmethod
-    def forward(ctx, B, T, C, H, r, k, v, w, u):
-        with torch.no_grad():
-            assert r.dtype == k.dtype == v.dtype == w.dtype == u.dtype
-            ctx.B, ctx.T, ctx.C, ctx.H = B, T, C, H
-            r, k, v, w, u = (x.contiguous() for x in (r, k, v, w, u))
-            ew = (-torch.exp(w.float())).contiguous()
-            eew = torch.exp(ew).contiguous()
-            y = torch.empty((B, T, C), device=r.device, dtype=r.dtype)
-            # the chunk-start states are kept for the backward (no second pass over the sequence there)
-            saved = torch.empty(ops.wkv5_saved_bytes(B, T, C), dtype=torch.uint8, device=r.device)
-            ctx.saved_valid = ops.wkv5_forward_saved(B, T, C, H, r, k, v, eew, u, y, saved)
-            ctx.save_for_backward(r, k, v, eew, ew, u, saved)
-            return y
-
-    @staticmethod
-    def backward(ctx, gy):
-        with torch.no_grad():
-            B, T, C, H = ctx.B, ctx.T, ctx.C, ctx.H
-            r, k, v, eew, ew, u, saved = ctx.saved_tensors
-            gr, gk, gv = (torch.empty((B, T, C), device=gy.device, dtype=r.dtype) for _ in range(3))
-            gw, gu = (torch.empty((B, C), device=gy.device, dtype=r.dtype) for _ in range(2))
-            # the harness sums bf16 (B,C) partials in bf16 (wkv5_bf16/run.py:83-87); here the unrounded fp32
-            # partials are summed in fp32 on the device and rounded once
-            gw32, gu32 = (torch.empty((B, C), device=gy.device, dtype=torch.float32) for _ in range(2))
-            ops.wkv5_backward_saved(B, T, C, H, r, k, v, eew, ew, u, gy.contiguous(), gr, gk, gv, gw, gu, saved,
-                                    ctx.saved_valid, gw32, gu32)
-            sums = torch.empty((2, C), device=gy.device, dtype=torch.float32)
-            ops.reduce_batch_partials(gw32, sums[0])
-            ops.reduce_batch_partials(gu32, sums[1])
-            shape = u.shape
-            return (None, None, None, None, gr, gk, gv, sums[0].to(u.dtype).view(shape), sums[1].to(u.dtype).view(shape))
+    def apply(B, T, C, H, r, k, v, w, u):
+        return native().wkv5(B, T, C, H, r, k, v, w, u)
 
 
 class WKV_5A(torch.autograd.Function):
@@ -96,37 +68,33 @@ class WKV_5A(torch.autograd.Function):
 class WKV_6(torch.autograd.Function):
     """RWKV-6 (wkv6/run.py:128-170).  The harness hands its kernel ew = -exp(w) in fp32; here the kernels take w itself
     (in the activation dtype) and keep the chunk-start states for the backward, as in WKV_6STATE_EX without a state.
-    Only a w of another dtype than the activations goes the harness's way."""
+    Only a w of another dtype than the activations goes the harness's way, through forward and backward below."""
+
+    @classmethod
+    def apply(cls, B, T, C, H, r, k, v, w, u):
+        if w.dtype == r.dtype:
+            return native().wkv6(B, T, C, H, r, k, v, w, u)
+        return super().apply(B, T, C, H, r, k, v, w, u)
 
     @staticmethod
     def forward(ctx, B, T, C, H, r, k, v, w, u):
         with torch.no_grad():
             ctx.B, ctx.T, ctx.C, ctx.H = B, T, C, H
             r, k, v, w, u = (x.contiguous() for x in (r, k, v, w, u))
+            ew = (-torch.exp(w.float())).contiguous()
+            ctx.save_for_backward(r, k, v, ew, u)
             y = torch.empty((B, T, C), device=r.device, dtype=r.dtype)
-            ctx.raw = w.dtype == r.dtype
-            if not ctx.raw:
-                ew = (-torch.exp(w.float())).contiguous()
-                ctx.save_for_backward(r, k, v, ew, u, None)
-                ops.wkv6_forward(B, T, C, H, r, k, v, ew, u, y)
-                return y
-            saved = torch.empty(ops.wkv6_saved_bytes(B, T, C), dtype=torch.uint8, device=r.device)
-            ctx.saved_valid = ops.wkv6state_forward_saved(B, T, C, H, r, k, v, w, u, None, y, None, saved)
-            ctx.save_for_backward(r, k, v, w, u, saved)
+            ops.wkv6_forward(B, T, C, H, r, k, v, ew, u, y)
             return y
 
     @staticmethod
     def backward(ctx, gy):
         with torch.no_grad():
             B, T, C, H = ctx.B, ctx.T, ctx.C, ctx.H
-            r, k, v, w, u, saved = ctx.saved_tensors
+            r, k, v, ew, u = ctx.saved_tensors
             gr, gk, gv, gw = (torch.empty((B, T, C), device=gy.device, dtype=r.dtype) for _ in range(4))
             gu = torch.empty((B, C), device=gy.device, dtype=r.dtype)
-            if ctx.raw:
-                ops.wkv6state_backward_saved(B, T, C, H, r, k, v, w, u, None, gy.contiguous(), None, gr, gk, gv, gw, gu,
-                                             None, saved, ctx.saved_valid)
-            else:
-                ops.wkv6_backward(B, T, C, H, r, k, v, w, u, gy.contiguous(), gr, gk, gv, gw, gu)
+            ops.wkv6_backward(B, T, C, H, r, k, v, ew, u, gy.contiguous(), gr, gk, gv, gw, gu)
             return (None, None, None, None, gr, gk, gv, gw, torch.sum(gu, 0).view(H, C // H))
 
 
@@ -156,34 +124,11 @@ class WKV_6STATE(torch.autograd.Function):
 
 
 class WKV_6STATE_EX(torch.autograd.Function):
-    """RWKV-6 with fp32 state in and out (state passing); no counterpart class in the reference."""
+    """RWKV-6 with fp32 state in and out (state passing), (r, k, v, w, u, s0) -> (y, sT); no counterpart class in the reference."""
 
     @staticmethod
-    def forward(ctx, r, k, v, w, u, s0):
-        with torch.no_grad():
-            B, T, C = r.shape
-            H = u.shape[0]
-            ctx.dims = (B, T, C, H)
-            r, k, v, w, u, s0 = (x.contiguous() for x in (r, k, v, w, u, s0))
-            y = torch.empty((B, T, C), device=r.device, dtype=r.dtype)
-            sT = torch.empty_like(s0)
-            # the chunk-start states are kept for the backward (half the size of its scratch buffer is used)
-            saved = torch.empty(ops.wkv6_saved_bytes(B, T, C), dtype=torch.uint8, device=r.device)
-            ctx.saved_valid = ops.wkv6state_forward_saved(B, T, C, H, r, k, v, w, u, s0, y, sT, saved)
-            ctx.save_for_backward(r, k, v, w, u, s0, saved)
-            return y, sT
-
-    @staticmethod
-    def backward(ctx, gy, dsT):
-        with torch.no_grad():
-            B, T, C, H = ctx.dims
-            r, k, v, w, u, s0, saved = ctx.saved_tensors
-            gr, gk, gv, gw = (torch.empty((B, T, C), device=gy.device, dtype=r.dtype) for _ in range(4))
-            gu = torch.empty((B, C), device=gy.device, dtype=r.dtype)
-            ds0 = torch.empty_like(s0)
-            ops.wkv6state_backward_saved(B, T, C, H, r, k, v, w, u, s0, gy.contiguous(), dsT.contiguous(), gr, gk, gv,
-                                         gw, gu, ds0, saved, ctx.saved_valid)
-            return gr, gk, gv, gw, torch.sum(gu.float(), 0).view(H, C // H).to(u.dtype), ds0
+    def apply(r, k, v, w, u, s0):
+        return native().wkv6_state(r, k, v, w, u, s0)
 
 
 class RWKV7_CLAMPW_CUDA_OP(torch.autograd.Function):

@@ -34,3 +34,20 @@ def test_training_at_any_length(op, B, T, H):
     want = grads(lambda *xs: oracle(*xs, H), (r, k, v, w, u), gy)
     for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
         Hh.assert_close(a, b, Hh.TOL_BF16, f"{op} {name}")
+
+
+@pytest.mark.parametrize("use_s0", [False, True])
+def test_rwkv7_training_classes(use_s0):
+    import rwkv_cuda_b200 as R
+    B, T, H, N = 2, 48, 2, 64
+    inp = Hh.v7_inputs(B, T, H, N, seed=3)
+    names = ("r", "w", "k", "v", "a", "b")
+    x64 = {n: (x.double() if n in ("s0", "dsT") else x.to(BF).double()) for n, x in inp.items()}
+    want = Hh.v7_oracle(x64, H, use_s0=use_s0, use_dsT=False)
+    xs = [inp[n].to(BF).cuda().requires_grad_(True) for n in names]
+    s0 = inp["s0"].cuda().requires_grad_(True)
+    y = R.functions.RWKV7_STATE_CLAMPW_CUDA(s0, *xs) if use_s0 else R.functions.RWKV7_CLAMPW_CUDA(*xs)
+    g = torch.autograd.grad(y, xs + ([s0] if use_s0 else []), inp["dy"].to(BF).cuda())
+    Hh.assert_close(y, want["y"], Hh.TOL_BF16, "y")
+    for a, n in zip(g, names + ("s0",)):
+        Hh.assert_close(a, want["d" + n], Hh.TOL_BF16, "d" + n)
