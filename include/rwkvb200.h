@@ -130,7 +130,7 @@ int rwkvb200_wkv5_backward_ws32(int dtype, int B, int T, int C, int H, const voi
 
 /* Training flow: the harness's pre- and post-operations (wkv5_bf16/run.py:44-88) inside the kernels.  w_raw (H,N) in `dtype`;
  * gwu (2,C) in `dtype`: the gradients of w_raw and u, summed over the batch in fp32 and in a fixed order.  The forward leaves
- * in `saved` (rwkvb200_wkv5_train_saved_bytes) what the backward needs and returns the path that both take (0 or 1, or a
+ * in `saved` (rwkvb200_wkv5_train_saved_bytes) what the backward needs and returns the path that both take (0 to 2, or a
  * negative code); `work`: rwkvb200_wkv5_train_work_bytes(..., path) bytes. */
 size_t rwkvb200_wkv5_train_saved_bytes(int B, int T, int C, int H);
 size_t rwkvb200_wkv5_train_work_bytes(int B, int T, int C, int H, int path);

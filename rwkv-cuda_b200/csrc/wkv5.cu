@@ -456,7 +456,8 @@ extern "C" int rwkvb200_wkv5_backward_saved(int dtype, int B, int T, int C, int 
 }
 
 // ---- training flow: the harness's pre- and post-operations inside the kernels -------------------------------------------
-// bf16 / head size 64 on the tcgen05 kernels (as rwkvb200_wkv5_forward_saved), everything else on the segments of wkv5_seg.cu.
+// Path 0: bf16 / head size 64 on the tcgen05 kernels (as rwkvb200_wkv5_forward_saved); 1: other head sizes up to 64 and fp32 on
+// the segments of wkv5_seg.cu; 2: larger heads on the general-shape kernels.
 extern "C" size_t rwkvb200_wkv5_train_saved_bytes(int B, int T, int C, int H) {
     if (B <= 0 || T <= 0 || C <= 0 || H <= 0) return 0;
     return (size_t)B * H * (wkv5_seg_count(T) * (C / H) * (C / H) + 1) * sizeof(float);   // a state per 32 tokens and a flag per unit
@@ -478,13 +479,22 @@ extern "C" int rwkvb200_wkv5_train_forward(int dtype, int B, int T, int C, int H
             return check_launch("wkv5_train_forward");
         }
     }
-    const int e = wkv5_seg_forward(dtype, B, T, C, H, r, k, v, w_raw, u, y, static_cast<float*>(saved), st);
-    return e ? e : 1;
+    if (C / H <= 64) {
+        const int e = wkv5_seg_forward(dtype, B, T, C, H, r, k, v, w_raw, u, y, static_cast<float*>(saved), st);
+        return e ? e : 1;
+    }
+#define RWKV_GO(E)                                                                                                                   \
+    wkv5_forward_kernel<E, 128, false><<<B * H, 128, 0, st>>>(T, C, H, C / H, (const E*)r, (const E*)k, (const E*)v, nullptr, (const E*)u, \
+                                                              nullptr, nullptr, (E*)y, nullptr, 0, (const E*)w_raw)
+    if (dtype == RWKVB200_F32) RWKV_GO(float); else RWKV_GO(bf16);
+#undef RWKV_GO
+    const int e = check_launch("wkv5_train_forward");
+    return e ? e : 2;
 }
 
 extern "C" size_t rwkvb200_wkv5_train_work_bytes(int B, int T, int C, int H, int path) {
     if (B <= 0 || T <= 0 || C <= 0 || H <= 0) return 0;
-    if (path == 0) return (size_t)B * 2 * C * sizeof(float);
+    if (path != 1) return (size_t)B * 2 * C * sizeof(float);
     return wkv5_seg_count(T) * ((size_t)B * H * (C / H) * (C / H) + (size_t)B * 2 * C) * sizeof(float);
 }
 
@@ -507,6 +517,14 @@ extern "C" int rwkvb200_wkv5_train_backward(int dtype, int B, int T, int C, int 
         wkv5_backward_kernel<bf16, 64, false><<<B * H, 64, 0, st>>>(
             T, C, H, C / H, (const bf16*)r, (const bf16*)k, (const bf16*)v, nullptr, nullptr, (const bf16*)u, nullptr, nullptr, nullptr, (const bf16*)gy,
             (bf16*)gr, (bf16*)gk, (bf16*)gv, nullptr, nullptr, nullptr, nullptr, flags, -1, (const bf16*)w_raw, partial, partial + C, 2 * (i64)C);
+        if (int e = check_launch("wkv5_train_backward")) return e;
+    } else if (path == 2) {
+#define RWKV_GO(E)                                                                                                                          \
+    wkv5_backward_kernel<E, 128, false><<<B * H, 128, 0, st>>>(                                                                             \
+        T, C, H, C / H, (const E*)r, (const E*)k, (const E*)v, nullptr, nullptr, (const E*)u, nullptr, nullptr, nullptr, (const E*)gy, (E*)gr, (E*)gk, \
+        (E*)gv, nullptr, nullptr, nullptr, nullptr, nullptr, 0, (const E*)w_raw, partial, partial + C, 2 * (i64)C)
+        if (dtype == RWKVB200_F32) RWKV_GO(float); else RWKV_GO(bf16);
+#undef RWKV_GO
         if (int e = check_launch("wkv5_train_backward")) return e;
     } else {
         float* D = partial + (size_t)B * wkv5_seg_count(T) * 2 * C;

@@ -1,5 +1,5 @@
-// RWKV-5 training in fp32 arithmetic (fp32 activations; bf16 where the tensor-core kernels do not apply), any head size
-// N <= 128, split over time.
+// RWKV-5 training in fp32 arithmetic (fp32 activations; bf16 where the tensor-core kernels do not apply), head sizes
+// N <= 64, split over time.
 //
 // Per (batch, head), S indexed [key j][value i], w the decay of a key:
 //   y_t[i] = sum_j r_t[j] S_{t-1}[j,i] + v_t[i] sum_j r_t u k_t      S_t[j,i] = w[j] S_{t-1}[j,i] + k_t[j] v_t[i]
@@ -9,82 +9,151 @@
 //           and token because the powers of w are put on k when it is staged (they are <= 1: nothing can overflow, whatever w is);
 //   scan    start states of the segments, in place: S <- S diag(w^n) + local;
 //   y       every segment again, token by token from its start state.
-// Backward: the same two steps for the adjoint D = dL/dS (k, v -> r, gy, time reversed), then one block per segment whose three
-// groups of threads walk it at the same time: S forward (gr), D by key lines backward (gk), D by value lines backward (gv).
+// Backward: the same two steps for the adjoint D = dL/dS (k, v -> r, gy, time reversed), then one block per segment: two warps
+// carry S forward (gr) while two carry D backward (gk, gv).
 // The decays of a segment act on its own outputs and on its end state: with Z = dS/dlog w counted from the segment's start
 // (Z_0 = 0, Z <- w (Z + S)), the segment's part of dL/dlog w is sum_t r_t sum_i gy_t Z_t + sum_i D_end Z_end.  (The sum over
 // states and gradients that needs no Z cancels for fast decays: 10 % error in gw at w = exp(-exp(3)).)
 // Inputs are staged in shared memory once per segment, so the token loops have no barrier; multiply-adds are packed in pairs.
-// fp32, B8 T512 H16 N64, forward + backward on a B200: 1285 us with wkv5.cu, 635 us here.
+// Shared memory delivers 4 bytes per lane and clock even when all lanes read the same word, so with one state line per thread
+// the reads of the token's vectors bound everything (512 bytes per 96 packed multiply-adds); a lane therefore owns a tile of
+// 8 keys x 8 values, and the sums over lanes are taken for eight elements at a time (7 shuffles).
+// fp32, B8 T512 H16 N64, forward + backward on a B200: 1285 us with wkv5.cu, 635 us with a line per thread, SEG_MEASURED here.
 #include "wkv5_seg.cuh"
 #include "packed.cuh"
 
 namespace rwkvb200 {
 namespace {
 
-constexpr int kSeg = kWkv5Seg;
+constexpr int kSeg = kWkv5Seg, kN = 64;   // tokens of a segment; head size of the tiles (smaller heads are padded with zeros)
 
-// Stages `n` tokens of a (T, C) tensor into dst[kSeg][NMAX] as fp32, zero where there is no token or channel.
-template <typename E, int NMAX>
-__device__ __forceinline__ void stage(float* dst, const E* __restrict__ src, int n, int C, int N, int tid, int nth) {
-    for (int x = tid; x < kSeg * NMAX; x += nth) {
-        const int t = x / NMAX, j = x % NMAX;
-        dst[x] = (t < n && j < N) ? to_f(src[(i64)t * C + j]) : 0.f;
-    }
-}
 template <typename E>
 __device__ __forceinline__ float log_decay(const E* w_raw) { return -expf(to_f(*w_raw)); }   // log w = -exp(w_raw)
 __device__ __forceinline__ float power(float lw, int e) { return e == 0 ? 1.f : expf(lw * (float)e); }   // w^e, also for w = 0
 
-// state line of a thread: element e at p[e * stride]
-template <int NMAX>
-__device__ __forceinline__ void load_line(f2 (&s)[NMAX / 2], const float* p, int stride, int N, bool live) {
-#pragma unroll
-    for (int e = 0; e < NMAX / 2; ++e)
-        s[e] = pack2(live && 2 * e < N ? p[(i64)(2 * e) * stride] : 0.f, live && 2 * e + 1 < N ? p[(i64)(2 * e + 1) * stride] : 0.f);
+// Rows of 64 channels in shared memory: the first four of every eight channels come first, then the other four, so that lanes
+// that own eight channels each read 16-byte pieces without bank conflicts.
+__device__ __forceinline__ int place(int ch) { return ((ch & 4) << 3) + ((ch >> 3) << 2) + (ch & 3); }
+struct Eight { float4 lo, hi; };
+__device__ __forceinline__ Eight load8(const float* row, int grp) {
+    return Eight{*reinterpret_cast<const float4*>(row + 4 * grp), *reinterpret_cast<const float4*>(row + 32 + 4 * grp)};
 }
-template <int NMAX>
-__device__ __forceinline__ void store_line(const f2 (&s)[NMAX / 2], float* p, int stride, int N, bool live) {
+__device__ __forceinline__ void pairs(const Eight& x, f2 (&p)[4]) {
+    p[0] = pack2(x.lo.x, x.lo.y); p[1] = pack2(x.lo.z, x.lo.w); p[2] = pack2(x.hi.x, x.hi.y); p[3] = pack2(x.hi.z, x.hi.w);
+}
+__device__ __forceinline__ void twice(const Eight& x, f2 (&p)[8]) {
+    p[0] = pack2(x.lo.x, x.lo.x); p[1] = pack2(x.lo.y, x.lo.y); p[2] = pack2(x.lo.z, x.lo.z); p[3] = pack2(x.lo.w, x.lo.w);
+    p[4] = pack2(x.hi.x, x.hi.x); p[5] = pack2(x.hi.y, x.hi.y); p[6] = pack2(x.hi.z, x.hi.z); p[7] = pack2(x.hi.w, x.hi.w);
+}
+
+// Stages `n` tokens of a (T, C) tensor as fp32 rows, zero where there is no token or channel, each times scale(token, channel).
+// Whole aligned heads are read four channels at a time with every load of the thread in flight.
+__device__ __forceinline__ float4 read4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 read4(const bf16* p) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(x.x << 16), __uint_as_float(x.x & 0xffff0000u), __uint_as_float(x.y << 16), __uint_as_float(x.y & 0xffff0000u));
+}
+template <int NTH, typename E, typename F>
+__device__ __forceinline__ void stage(float* dst, const E* __restrict__ src, int n, int C, int N, int tid, F scale) {
+    if (N == kN && (reinterpret_cast<uintptr_t>(src) & (4 * sizeof(E) - 1)) == 0) {
+        constexpr int PER = kSeg * kN / 4 / NTH;
+        float4 x[PER];
 #pragma unroll
-    for (int e = 0; e < NMAX / 2; ++e) {
-        float lo, hi;
-        unpack2(s[e], lo, hi);
-        if (live && 2 * e < N) p[(i64)(2 * e) * stride] = lo;
-        if (live && 2 * e + 1 < N) p[(i64)(2 * e + 1) * stride] = hi;
+        for (int i = 0; i < PER; ++i) {
+            const int t = (i * NTH + tid) / 16, j = (tid & 15) * 4;
+            x[i] = t < n ? read4(src + (i64)t * C + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int t = (i * NTH + tid) / 16, j = (tid & 15) * 4;
+            *reinterpret_cast<float4*>(dst + t * kN + place(j)) =
+                make_float4(x[i].x * scale(t, j), x[i].y * scale(t, j + 1), x[i].z * scale(t, j + 2), x[i].w * scale(t, j + 3));
+        }
+    } else {
+        for (int x = tid; x < kSeg * kN; x += NTH) {
+            const int t = x / kN, j = x % kN;
+            dst[t * kN + place(j)] = (t < n && j < N) ? to_f(src[(i64)t * C + j]) * scale(t, j) : 0.f;
+        }
+    }
+}
+template <int NTH, typename E>
+__device__ __forceinline__ void stage(float* dst, const E* __restrict__ src, int n, int C, int N, int tid) {
+    stage<NTH>(dst, src, n, C, N, tid, [](int, int) { return 1.f; });
+}
+
+// A lane's tile of a state, x[value][key pair]: 8 values from v0 on, 8 keys from k0 on; states are [key][value] in memory.
+typedef f2 Tile[8][4];
+// key pair p of the tile
+__device__ __forceinline__ void load_pair(f2 (&x)[8], int p, const float* st, int k0, int v0, int N) {
+    float a[2][8];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const float* row = st + (i64)(k0 + 2 * p + e) * N + v0;
+        if (N == kN) {
+            *reinterpret_cast<float4*>(a[e]) = *reinterpret_cast<const float4*>(row);
+            *reinterpret_cast<float4*>(a[e] + 4) = *reinterpret_cast<const float4*>(row + 4);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[e][i] = (k0 + 2 * p + e < N && v0 + i < N) ? row[i] : 0.f;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = pack2(a[0][i], a[1][i]);
+}
+__device__ __forceinline__ void load_tile(Tile& x, const float* st, int k0, int v0, int N) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        f2 q[8];
+        load_pair(q, p, st, k0, v0, N);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i][p] = q[i];
+    }
+}
+__device__ __forceinline__ void store_tile(const Tile& x, float* st, int k0, int v0, int N) {
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        float a[2][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) unpack2(x[i][p], a[0][i], a[1][i]);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            float* row = st + (i64)(k0 + 2 * p + e) * N + v0;
+            if (N == kN) {
+                *reinterpret_cast<float4*>(row) = *reinterpret_cast<const float4*>(a[e]);
+                *reinterpret_cast<float4*>(row + 4) = *reinterpret_cast<const float4*>(a[e] + 4);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (k0 + 2 * p + e < N && v0 + i < N) row[i] = a[e][i];
+            }
+        }
     }
 }
 
-// grid (segments, units), NMAX threads, thread = value i.  REV = false: a = k, b = v; REV = true: a = r, b = gy.
-template <typename E, int NMAX, bool REV>
-__global__ void __launch_bounds__(NMAX, NMAX == 128 ? 2 : 512 / NMAX) seg_local_kernel(int T, int C, int H, int N, const E* __restrict__ a_, const E* __restrict__ b_,
-                                                         const E* __restrict__ w_, float* __restrict__ states) {
-    __shared__ __align__(16) float as[kSeg * NMAX];
-    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, i = threadIdx.x;
-    const int n = min(kSeg, T - seg * kSeg);
-    const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
-    const bool live = i < N;
-    {   // a, times the decay between its token and the end (REV: the start) of the segment; thread = key here
-        const float lw = live ? log_decay(w_ + h * N + i) : 0.f;
-        for (int t = 0; t < kSeg; ++t)
-            as[t * NMAX + i] = (live && t < n) ? to_f(a_[base + (i64)t * C + i]) * power(lw, REV ? t : n - 1 - t) : 0.f;
-    }
-    __syncthreads();
-    f2 s[NMAX / 2];
+// Sums of v[0..7] over the 8 lanes that differ in bits 2 to 4, in 7 shuffles: a lane ends with element (lane >> 2) of them.
+__device__ __forceinline__ float reduce8(float (&v)[8], int lane) {
 #pragma unroll
-    for (int e = 0; e < NMAX / 2; ++e) s[e] = 0ull;
-#pragma unroll 2
-    for (int t = 0; t < n; ++t) {
-        const float b = live ? to_f(b_[base + (i64)t * C + i]) : 0.f;
-        const f2 bb = pack2(b, b);
-        const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(as + t * NMAX);
+    for (int m = 16, n = 4; n >= 1; m >>= 1, n >>= 1) {
+        const bool up = (lane & m) != 0;
 #pragma unroll
-        for (int e = 0; e < NMAX / 4; ++e) {
-            const ulonglong2 q = ap[e];
-            s[2 * e] = fma2(q.x, bb, s[2 * e]);
-            s[2 * e + 1] = fma2(q.y, bb, s[2 * e + 1]);
+        for (int i = 0; i < n; ++i) {
+            const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
         }
     }
-    store_line<NMAX>(s, states + ((i64)unit * gridDim.x + seg) * N * N + i, N, N, live);
+    return v[0];
+}
+// The same over the 4 lanes that differ in bits 0 and 1: a lane ends with elements 2 (lane & 3) and the next, in v[0], v[1].
+__device__ __forceinline__ void reduce8_pairs(float (&v)[8], int lane) {
+#pragma unroll
+    for (int m = 2, n = 4; n >= 2; m >>= 1, n >>= 1) {
+        const bool up = (lane & m) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+        }
+    }
 }
 
 // In place: local end states -> state before each segment (REV: adjoint after each segment).  One thread per state element.
@@ -95,7 +164,7 @@ __global__ void __launch_bounds__(256) seg_scan_kernel(int T, int H, int N, int 
     const float lw = log_decay(w_ + (unit % H) * N + e / N);
     const float full = expf(lw * kSeg), tail = expf(lw * (float)(T - (nseg - 1) * kSeg));
     float* p = states + (i64)unit * nseg * N * N + e;
-    constexpr int AHEAD = 8;
+    constexpr int AHEAD = 16;
     float cur = 0.f;
     for (int k0 = 0; k0 < nseg; k0 += AHEAD) {   // the loads of AHEAD segments are in flight together
         float x[AHEAD];
@@ -112,226 +181,252 @@ __global__ void __launch_bounds__(256) seg_scan_kernel(int T, int H, int N, int 
     }
 }
 
-// grid (segments, units), NMAX threads, thread = value i
-template <typename E, int NMAX>
-__global__ void __launch_bounds__(NMAX, NMAX == 128 ? 2 : 512 / NMAX) seg_y_kernel(int T, int C, int H, int N, const E* __restrict__ r_, const E* __restrict__ k_,
-                                                     const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
-                                                     const float* __restrict__ states, E* __restrict__ y_) {
-    __shared__ __align__(16) float rs[kSeg * NMAX], ks[kSeg * NMAX], ws[NMAX], us[NMAX], ruk[kSeg];
-    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, i = threadIdx.x;
+// grid (segments, units), 2 warps: a warp has the keys 32 warp .. of all values, a lane 8 keys x 8 values.
+// REV = false: a = k, b = v; REV = true: a = r, b = gy.
+template <typename E, bool REV>
+__global__ void __launch_bounds__(64, 8) seg_local_kernel(int T, int C, int H, int N, const E* __restrict__ a_, const E* __restrict__ b_,
+                                                          const E* __restrict__ w_, float* __restrict__ states) {
+    __shared__ __align__(16) float as[kSeg * kN], bs[kSeg * kN], lw[kN];
+    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, tid = threadIdx.x, lane = tid & 31;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
-    const bool live = i < N;
-    stage<E, NMAX>(rs, r_ + base, n, C, N, i, NMAX);
-    stage<E, NMAX>(ks, k_ + base, n, C, N, i, NMAX);
-    ws[i] = live ? expf(log_decay(w_ + h * N + i)) : 0.f;
-    us[i] = live ? to_f(u_[h * N + i]) : 0.f;
-    f2 s[NMAX / 2];
-    load_line<NMAX>(s, states + ((i64)unit * gridDim.x + seg) * N * N + i, N, N, live);
+    lw[tid] = tid < N ? log_decay(w_ + h * N + tid) : 0.f;
+    stage<64>(bs, b_ + base, n, C, N, tid);
     __syncthreads();
-    for (int t = i / 32; t < n; t += NMAX / 32) {   // the bonus of a token: one warp each
-        float x = 0.f;
-        for (int j = i & 31; j < NMAX; j += 32) x = fmaf(rs[t * NMAX + j] * us[j], ks[t * NMAX + j], x);
+    // a, times the decay between its token and the end (REV: the start) of the segment
+    stage<64>(as, a_ + base, n, C, N, tid, [&](int t, int j) { return t < n ? power(lw[j], REV ? t : n - 1 - t) : 0.f; });
+    __syncthreads();
+    const int kg = 4 * (tid >> 5) + (lane & 3), vg = lane >> 2;
+    Tile s;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) s[i][p] = 0ull;
+#pragma unroll 2
+    for (int t = 0; t < n; ++t) {
+        f2 a[4], b[8];
+        pairs(load8(as + t * kN, kg), a);
+        twice(load8(bs + t * kN, vg), b);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) s[i][p] = fma2(a[p], b[i], s[i][p]);
+    }
+    store_tile(s, states + ((i64)unit * gridDim.x + seg) * N * N, 8 * kg, 8 * vg, N);
+}
+
+// grid (segments, units), 2 warps: a warp has the values 32 warp .. of all keys
+template <typename E>
+__global__ void __launch_bounds__(64, 8) seg_y_kernel(int T, int C, int H, int N, const E* __restrict__ r_, const E* __restrict__ k_,
+                                                      const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
+                                                      const float* __restrict__ states, E* __restrict__ y_) {
+    __shared__ __align__(16) float rs[kSeg * kN], ks[kSeg * kN], vs[kSeg * kN], ws[kN], us[kN], ruk[kSeg];
+    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = min(kSeg, T - seg * kSeg);
+    const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
+    const int kg = lane >> 2, vg = 4 * warp + (lane & 3);
+    Tile s;
+    load_tile(s, states + ((i64)unit * gridDim.x + seg) * N * N, 8 * kg, 8 * vg, N);
+    stage<64>(rs, r_ + base, n, C, N, tid);
+    stage<64>(ks, k_ + base, n, C, N, tid);
+    stage<64>(vs, v_ + base, n, C, N, tid);
+    ws[place(tid)] = tid < N ? expf(log_decay(w_ + h * N + tid)) : 0.f;
+    us[place(tid)] = tid < N ? to_f(u_[h * N + tid]) : 0.f;
+    __syncthreads();
+    for (int t = warp; t < n; t += 2) {   // the bonus of a token: one warp each
+        float x = fmaf(rs[t * kN + lane] * us[lane], ks[t * kN + lane], rs[t * kN + 32 + lane] * us[32 + lane] * ks[t * kN + 32 + lane]);
 #pragma unroll
         for (int m = 16; m; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
-        if ((i & 31) == 0) ruk[t] = x;
+        if (lane == 0) ruk[t] = x;
     }
     __syncthreads();
-    float vn = live ? to_f(v_[base + i]) : 0.f;
+    f2 w[4];
+    pairs(load8(ws, kg), w);
+    const int i_out = 8 * vg + kg;   // the value whose sum this lane ends with
     for (int t = 0; t < n; ++t) {
-        const float v = vn;
-        if (t + 1 < n && live) vn = to_f(v_[base + (i64)(t + 1) * C + i]);
-        const f2 vv = pack2(v, v);
-        f2 y0 = 0ull, y1 = 0ull;
-        const ulonglong2 *rp = reinterpret_cast<const ulonglong2*>(rs + t * NMAX), *kp = reinterpret_cast<const ulonglong2*>(ks + t * NMAX),
-                         *wp = reinterpret_cast<const ulonglong2*>(ws);
+        f2 r[4], k[4], v[8];
+        pairs(load8(rs + t * kN, kg), r);
+        pairs(load8(ks + t * kN, kg), k);
+        twice(load8(vs + t * kN, vg), v);
+        float y[8];
 #pragma unroll
-        for (int e = 0; e < NMAX / 4; ++e) {
-            const ulonglong2 r = rp[e], k = kp[e], w = wp[e];
-            y0 = fma2(r.x, s[2 * e], y0);
-            y1 = fma2(r.y, s[2 * e + 1], y1);
-            s[2 * e] = fma2(s[2 * e], w.x, mul2(k.x, vv));
-            s[2 * e + 1] = fma2(s[2 * e + 1], w.y, mul2(k.y, vv));
+        for (int i = 0; i < 8; ++i) {
+            f2 acc = mul2(s[i][0], r[0]);
+#pragma unroll
+            for (int p = 1; p < 4; ++p) acc = fma2(s[i][p], r[p], acc);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) s[i][p] = fma2(s[i][p], w[p], mul2(k[p], v[i]));
+            y[i] = sum2(acc);
         }
-        if (live) y_[base + (i64)t * C + i] = from_f<E>(fmaf(v, ruk[t], sum2(y0) + sum2(y1)));
+        const float yo = reduce8(y, lane);
+        if (i_out < N) y_[base + (i64)t * C + i_out] = from_f<E>(fmaf(vs[t * kN + place(i_out)], ruk[t], yo));
     }
 }
 
-// grid (segments, units), 4 NMAX threads: the first half = key lines of S and Z, two neighbouring threads per line; then NMAX
-// threads for the key lines of D and NMAX for its value lines
-template <int NMAX>
+// grid (segments, units), 4 warps: warps 0, 1 carry S and Z forward (gr, gw, gu), warps 2, 3 carry D backward (gk, gv); a warp
+// has 32 keys of all values.  gv sums over all keys: the two halves meet in shared memory at the end.
 struct BwdSmem {
-    float r[kSeg * NMAX], k[kSeg * NMAX], v[kSeg * NMAX], g[kSeg * NMAX];
-    float w[NMAX], u[NMAX], vg[kSeg], ruk[kSeg];
+    float r[kSeg * kN], k[kSeg * kN], v[kSeg * kN], g[kSeg * kN], gv[2][kSeg * kN];
+    float w[kN], u[kN], vg[kSeg], ruk[kSeg];
 };
 
-template <typename E, int NMAX>
-__global__ void __launch_bounds__(4 * NMAX, NMAX == 128 ? 1 : 2) seg_backward_kernel(int T, int C, int H, int N, const E* __restrict__ r_, const E* __restrict__ k_,
-                                                                const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
-                                                                const E* __restrict__ gy_, const float* __restrict__ S_,
-                                                                const float* __restrict__ D_, E* __restrict__ gr_, E* __restrict__ gk_,
-                                                                E* __restrict__ gv_, float* __restrict__ partial_) {
+template <typename E>
+__global__ void __launch_bounds__(128, 3) seg_backward_kernel(int T, int C, int H, int N, const E* __restrict__ r_, const E* __restrict__ k_,
+                                                              const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
+                                                              const E* __restrict__ gy_, const float* __restrict__ S_, const float* __restrict__ D_,
+                                                              E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_,
+                                                              float* __restrict__ partial_) {
     extern __shared__ __align__(16) unsigned char smem_seg[];
-    BwdSmem<NMAX>& sm = *reinterpret_cast<BwdSmem<NMAX>*>(smem_seg);
-    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, grp = threadIdx.x / NMAX, half = threadIdx.x & 1;
-    const int i = grp < 2 ? threadIdx.x >> 1 : threadIdx.x % NMAX;   // line
-    constexpr int NTH = 4 * NMAX, HP = NMAX / 4;                      // pairs of half a line
+    BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_seg);
+    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
-    const bool live = i < N;
-    const float* S0 = S_ + ((i64)unit * gridDim.x + seg) * N * N;
     const float* D0 = D_ + ((i64)unit * gridDim.x + seg) * N * N;
-    stage<E, NMAX>(sm.r, r_ + base, n, C, N, threadIdx.x, NTH);
-    stage<E, NMAX>(sm.k, k_ + base, n, C, N, threadIdx.x, NTH);
-    stage<E, NMAX>(sm.v, v_ + base, n, C, N, threadIdx.x, NTH);
-    stage<E, NMAX>(sm.g, gy_ + base, n, C, N, threadIdx.x, NTH);
-    const float lw = live ? log_decay(w_ + h * N + i) : 0.f, w = live ? expf(lw) : 0.f, u = live ? to_f(u_[h * N + i]) : 0.f;
-    if (grp == 2) { sm.w[i] = w; sm.u[i] = u; }
-    f2 s[NMAX / 2];   // half of S[key i][:] and of Z[key i][:], D[key i][:] or D[:][value i]
-    if (grp < 2) {
-#pragma unroll
-        for (int e = 0; e < HP; ++e) {   // (neighbouring float4s go to the two halves)
-            const int j = 8 * (e >> 1) + 4 * half + 2 * (e & 1);
-            s[e] = pack2(live && j < N ? S0[(i64)i * N + j] : 0.f, live && j + 1 < N ? S0[(i64)i * N + j + 1] : 0.f);
-            s[HP + e] = 0ull;
-        }
-    } else if (grp == 2) load_line<NMAX>(s, D0 + (i64)i * N, 1, N, live);
-    else load_line<NMAX>(s, D0 + i, N, N, live);
-    __syncthreads();
-    for (int t = threadIdx.x / 32; t < n; t += NTH / 32) {   // sums of a token over its channels: one warp each
-        float x = 0.f, z = 0.f;
-        for (int j = threadIdx.x & 31; j < NMAX; j += 32) {
-            x = fmaf(sm.r[t * NMAX + j] * sm.u[j], sm.k[t * NMAX + j], x);
-            z = fmaf(sm.v[t * NMAX + j], sm.g[t * NMAX + j], z);
-        }
-#pragma unroll
-        for (int m = 16; m; m >>= 1) { x += __shfl_xor_sync(0xffffffffu, x, m); z += __shfl_xor_sync(0xffffffffu, z, m); }
-        if ((threadIdx.x & 31) == 0) { sm.ruk[t] = x; sm.vg[t] = z; }
+    const int kg = 4 * (warp & 1) + (lane & 3), vg = lane >> 2, j_out = 8 * kg + vg;   // j_out: the key whose sums this lane ends with
+    Tile s;
+    load_tile(s, warp < 2 ? S_ + ((i64)unit * gridDim.x + seg) * N * N : D0, 8 * kg, 8 * vg, N);
+    stage<128>(sm.r, r_ + base, n, C, N, tid);
+    stage<128>(sm.k, k_ + base, n, C, N, tid);
+    stage<128>(sm.v, v_ + base, n, C, N, tid);
+    stage<128>(sm.g, gy_ + base, n, C, N, tid);
+    if (tid < kN) {
+        sm.w[place(tid)] = tid < N ? expf(log_decay(w_ + h * N + tid)) : 0.f;
+        sm.u[place(tid)] = tid < N ? to_f(u_[h * N + tid]) : 0.f;
     }
     __syncthreads();
-    const f2 ww = pack2(w, w);
-    float gw = 0.f, gu = 0.f;
-    if (grp < 2) {
+    for (int t = warp; t < n; t += 4) {   // sums of a token over its channels: one warp each
+        const float *r = sm.r + t * kN, *k = sm.k + t * kN, *v = sm.v + t * kN, *g = sm.g + t * kN;
+        float x = fmaf(r[lane] * sm.u[lane], k[lane], r[lane + 32] * sm.u[lane + 32] * k[lane + 32]);
+        float z = fmaf(v[lane], g[lane], v[lane + 32] * g[lane + 32]);
+#pragma unroll
+        for (int m = 16; m; m >>= 1) { x += __shfl_xor_sync(0xffffffffu, x, m); z += __shfl_xor_sync(0xffffffffu, z, m); }
+        if (lane == 0) { sm.ruk[t] = x; sm.vg[t] = z; }
+    }
+    __syncthreads();
+    const float uj = sm.u[place(j_out)];
+    f2 w[4];
+    pairs(load8(sm.w, kg), w);
+    if (warp < 2) {
+        Tile z;
+        f2 gw2[4] = {0ull, 0ull, 0ull, 0ull};
+        float gu = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) z[i][p] = 0ull;
         for (int t = 0; t < n; ++t) {
-            const float r = sm.r[t * NMAX + i], k = sm.k[t * NMAX + i], vg = sm.vg[t];
-            const f2 kk = pack2(k, k);
-            const ulonglong2 *vp = reinterpret_cast<const ulonglong2*>(sm.v + t * NMAX) + half, *gp = reinterpret_cast<const ulonglong2*>(sm.g + t * NMAX) + half;
-            f2 a0 = 0ull, a1 = 0ull, z0 = 0ull, z1 = 0ull;
+            f2 r[4], k[4], v[8], g[8];
+            pairs(load8(sm.r + t * kN, kg), r);
+            pairs(load8(sm.k + t * kN, kg), k);
+            twice(load8(sm.v + t * kN, vg), v);
+            twice(load8(sm.g + t * kN, vg), g);
+            f2 sg[4], zg[4];
 #pragma unroll
-            for (int e = 0; e < HP / 2; ++e) {
-                const ulonglong2 v = vp[2 * e], g = gp[2 * e];
-                f2 &s0 = s[2 * e], &s1 = s[2 * e + 1], &y0 = s[HP + 2 * e], &y1 = s[HP + 2 * e + 1];
-                a0 = fma2(s0, g.x, a0);
-                a1 = fma2(s1, g.y, a1);
-                z0 = fma2(y0, g.x, z0);
-                z1 = fma2(y1, g.y, z1);
-                s0 = mul2(s0, ww);
-                s1 = mul2(s1, ww);
-                y0 = fma2(y0, ww, s0);
-                y1 = fma2(y1, ww, s1);
-                s0 = fma2(v.x, kk, s0);
-                s1 = fma2(v.y, kk, s1);
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    sg[p] = i ? fma2(s[i][p], g[i], sg[p]) : mul2(s[i][p], g[i]);
+                    zg[p] = i ? fma2(z[i][p], g[i], zg[p]) : mul2(z[i][p], g[i]);
+                    s[i][p] = mul2(s[i][p], w[p]);
+                    z[i][p] = fma2(z[i][p], w[p], s[i][p]);
+                    s[i][p] = fma2(k[p], v[i], s[i][p]);
+                }
+            float x[8];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                gw2[p] = fma2(zg[p], r[p], gw2[p]);
+                unpack2(sg[p], x[2 * p], x[2 * p + 1]);
             }
-            float sg = sum2(a0) + sum2(a1);
-            sg += __shfl_xor_sync(0xffffffffu, sg, 1);
-            if (live && half == 0) gr_[base + (i64)t * C + i] = from_f<E>(fmaf(u * k, vg, sg));
-            gw = fmaf(r, sum2(z0) + sum2(z1), gw);
-            gu = fmaf(r * k, vg, gu);
+            const float sgj = reduce8(x, lane), rj = sm.r[t * kN + place(j_out)], kj = sm.k[t * kN + place(j_out)], vgt = sm.vg[t];
+            if (j_out < N) gr_[base + (i64)t * C + j_out] = from_f<E>(fmaf(uj * kj, vgt, sgj));
+            gu = fmaf(rj * kj, vgt, gu);
         }
-        f2 a0 = 0ull;   // sum over values of D_end Z_end
+        float x[8];   // + sum over values of D_end Z_end
 #pragma unroll
-        for (int e = 0; e < HP; ++e) {
-            const int j = 8 * (e >> 1) + 4 * half + 2 * (e & 1);
-            a0 = fma2(pack2(live && j < N ? D0[(i64)i * N + j] : 0.f, live && j + 1 < N ? D0[(i64)i * N + j + 1] : 0.f), s[HP + e], a0);
+        for (int p = 0; p < 4; ++p) {
+            f2 d[8];
+            load_pair(d, p, D0, 8 * kg, 8 * vg, N);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) gw2[p] = fma2(d[i], z[i][p], gw2[p]);
+            unpack2(gw2[p], x[2 * p], x[2 * p + 1]);
         }
-        gw += sum2(a0);
-        gw += __shfl_xor_sync(0xffffffffu, gw, 1);
-        if (live && half == 0) {
-            float* p = partial_ + ((i64)(unit / H) * gridDim.x + seg) * 2 * C + h * N + i;
-            p[0] = lw * gw;   // d log w / d w_raw = log w
+        const float gw = reduce8(x, lane);
+        if (j_out < N) {
+            float* p = partial_ + ((i64)(unit / H) * gridDim.x + seg) * 2 * C + h * N + j_out;
+            p[0] = log_decay(w_ + h * N + j_out) * gw;   // d log w / d w_raw = log w
             p[C] = gu;
         }
-    } else if (grp == 2) {
-        for (int t = n - 1; t >= 0; --t) {
-            const float r = sm.r[t * NMAX + i];
-            const f2 rr = pack2(r, r);
-            const ulonglong2 *vp = reinterpret_cast<const ulonglong2*>(sm.v + t * NMAX), *gp = reinterpret_cast<const ulonglong2*>(sm.g + t * NMAX);
-            f2 a0 = 0ull, a1 = 0ull;
-#pragma unroll
-            for (int e = 0; e < NMAX / 4; ++e) {
-                const ulonglong2 v = vp[e], g = gp[e];
-                a0 = fma2(s[2 * e], v.x, a0);
-                a1 = fma2(s[2 * e + 1], v.y, a1);
-                s[2 * e] = fma2(s[2 * e], ww, mul2(g.x, rr));
-                s[2 * e + 1] = fma2(s[2 * e + 1], ww, mul2(g.y, rr));
-            }
-            const float dv = sum2(a0) + sum2(a1);
-            if (live) gk_[base + (i64)t * C + i] = from_f<E>(fmaf(u * r, sm.vg[t], dv));
-        }
     } else {
-        const ulonglong2* wp = reinterpret_cast<const ulonglong2*>(sm.w);
         for (int t = n - 1; t >= 0; --t) {
-            const float g = sm.g[t * NMAX + i];
-            const f2 gg = pack2(g, g);
-            const ulonglong2 *rp = reinterpret_cast<const ulonglong2*>(sm.r + t * NMAX), *kp = reinterpret_cast<const ulonglong2*>(sm.k + t * NMAX);
-            f2 a0 = 0ull, a1 = 0ull;
+            f2 r[4], k[4], v[8], g[8];
+            pairs(load8(sm.r + t * kN, kg), r);
+            pairs(load8(sm.k + t * kN, kg), k);
+            twice(load8(sm.v + t * kN, vg), v);
+            twice(load8(sm.g + t * kN, vg), g);
+            f2 gk[4];
+            float x[8], y[8];
 #pragma unroll
-            for (int e = 0; e < NMAX / 4; ++e) {
-                const ulonglong2 r = rp[e], k = kp[e], wj = wp[e];
-                a0 = fma2(s[2 * e], k.x, a0);
-                a1 = fma2(s[2 * e + 1], k.y, a1);
-                s[2 * e] = fma2(s[2 * e], wj.x, mul2(r.x, gg));
-                s[2 * e + 1] = fma2(s[2 * e + 1], wj.y, mul2(r.y, gg));
+            for (int i = 0; i < 8; ++i) {
+                f2 acc = mul2(s[i][0], k[0]);
+#pragma unroll
+                for (int p = 1; p < 4; ++p) acc = fma2(s[i][p], k[p], acc);
+                y[i] = sum2(acc);
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    gk[p] = i ? fma2(s[i][p], v[i], gk[p]) : mul2(s[i][p], v[i]);
+                    s[i][p] = fma2(s[i][p], w[p], mul2(r[p], g[i]));
+                }
             }
-            if (live) gv_[base + (i64)t * C + i] = from_f<E>(fmaf(g, sm.ruk[t], sum2(a0) + sum2(a1)));
+#pragma unroll
+            for (int p = 0; p < 4; ++p) unpack2(gk[p], x[2 * p], x[2 * p + 1]);
+            const float dv = reduce8(x, lane);
+            if (j_out < N) gk_[base + (i64)t * C + j_out] = from_f<E>(fmaf(uj * sm.r[t * kN + place(j_out)], sm.vg[t], dv));
+            reduce8_pairs(y, lane);
+            *reinterpret_cast<float2*>(sm.gv[warp - 2] + t * kN + 8 * vg + 2 * (lane & 3)) = make_float2(y[0], y[1]);
         }
+    }
+    __syncthreads();
+    for (int x = tid; x < n * kN; x += 128) {
+        const int t = x / kN, i = x % kN;
+        if (i < N) gv_[base + (i64)t * C + i] = from_f<E>(fmaf(sm.g[t * kN + place(i)], sm.ruk[t], sm.gv[0][x] + sm.gv[1][x]));
     }
 }
 
-template <typename E, int NMAX>
+template <typename E>
 int forward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, void* y, float* states,
             cudaStream_t st) {
     const int N = C / H, nseg = (T + kSeg - 1) / kSeg;
     const dim3 grid(nseg, B * H), scan((N * N + 255) / 256, B * H);
-    seg_local_kernel<E, NMAX, false><<<grid, NMAX, 0, st>>>(T, C, H, N, (const E*)k, (const E*)v, (const E*)w, states);
+    seg_local_kernel<E, false><<<grid, 64, 0, st>>>(T, C, H, N, (const E*)k, (const E*)v, (const E*)w, states);
     seg_scan_kernel<E, false><<<scan, 256, 0, st>>>(T, H, N, nseg, (const E*)w, states);
-    seg_y_kernel<E, NMAX><<<grid, NMAX, 0, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states, (E*)y);
+    seg_y_kernel<E><<<grid, 64, 0, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states, (E*)y);
     return check_launch("wkv5_train_forward(segments)");
 }
 
-template <typename E, int NMAX>
+template <typename E>
 int backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, const void* gy, void* gr,
              void* gk, void* gv, const float* S, float* D, float* partial, cudaStream_t st) {
-    const int N = C / H, nseg = (T + kSeg - 1) / kSeg, smem = sizeof(BwdSmem<NMAX>);
+    const int N = C / H, nseg = (T + kSeg - 1) / kSeg, smem = sizeof(BwdSmem);
     const dim3 grid(nseg, B * H), scan((N * N + 255) / 256, B * H);
-    const cudaError_t e = cudaFuncSetAttribute(seg_backward_kernel<E, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(seg_backward_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv5_train_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    seg_local_kernel<E, NMAX, true><<<grid, NMAX, 0, st>>>(T, C, H, N, (const E*)r, (const E*)gy, (const E*)w, D);
+    seg_local_kernel<E, true><<<grid, 64, 0, st>>>(T, C, H, N, (const E*)r, (const E*)gy, (const E*)w, D);
     seg_scan_kernel<E, true><<<scan, 256, 0, st>>>(T, H, N, nseg, (const E*)w, D);
-    seg_backward_kernel<E, NMAX><<<grid, 4 * NMAX, smem, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u,
-                                                              (const E*)gy, S, D, (E*)gr, (E*)gk, (E*)gv, partial);
+    seg_backward_kernel<E><<<grid, 128, smem, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, (const E*)gy, S,
+                                                    D, (E*)gr, (E*)gk, (E*)gv, partial);
     return check_launch("wkv5_train_backward(segments)");
 }
 
 }  // namespace
 
-#define RWKV_BY_SHAPE(CALL)                                                                     \
-    switch (head_capacity(C / H)) {                                                             \
-        case 32: return dtype == RWKVB200_F32 ? CALL(float, 32) : CALL(bf16, 32);               \
-        case 64: return dtype == RWKVB200_F32 ? CALL(float, 64) : CALL(bf16, 64);               \
-        default: return dtype == RWKVB200_F32 ? CALL(float, 128) : CALL(bf16, 128);             \
-    }
 int wkv5_seg_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, void* y,
                      float* states, cudaStream_t st) {
-#define CALL(E, NM) forward<E, NM>(B, T, C, H, r, k, v, w, u, y, states, st)
-    RWKV_BY_SHAPE(CALL)
-#undef CALL
+    return dtype == RWKVB200_F32 ? forward<float>(B, T, C, H, r, k, v, w, u, y, states, st) : forward<bf16>(B, T, C, H, r, k, v, w, u, y, states, st);
 }
 int wkv5_seg_backward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
                       const void* gy, void* gr, void* gk, void* gv, const float* S, float* D, float* partial, cudaStream_t st) {
-#define CALL(E, NM) backward<E, NM>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, st)
-    RWKV_BY_SHAPE(CALL)
-#undef CALL
+    return dtype == RWKVB200_F32 ? backward<float>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, st)
+                                 : backward<bf16>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, st);
 }
 
 }  // namespace rwkvb200
