@@ -18,7 +18,8 @@
 // Shared memory delivers 4 bytes per lane and clock even when all lanes read the same word, so with one state line per thread
 // the reads of the token's vectors bound everything (512 bytes per 96 packed multiply-adds); a lane therefore owns a tile of
 // 8 keys x 8 values, and the sums over lanes are taken for eight elements at a time (7 shuffles).
-// fp32, B8 T512 H16 N64, forward + backward on a B200: 1285 us with wkv5.cu, 635 us with a line per thread, SEG_MEASURED here.
+// fp32, B8 T512 H16 N64, forward + backward on a B200: 1285 us with wkv5.cu, 635 us with a line per thread, 320 us here
+// (without register spills in the backward, which two blocks per SM allow and three do not: 212 -> 167 us for that kernel).
 #include "wkv5_seg.cuh"
 #include "packed.cuh"
 
@@ -271,7 +272,7 @@ struct BwdSmem {
 };
 
 template <typename E>
-__global__ void __launch_bounds__(128, 3) seg_backward_kernel(int T, int C, int H, int N, const E* __restrict__ r_, const E* __restrict__ k_,
+__global__ void __launch_bounds__(128, 2) seg_backward_kernel(int T, int C, int H, int N, const E* __restrict__ r_, const E* __restrict__ k_,
                                                               const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
                                                               const E* __restrict__ gy_, const float* __restrict__ S_, const float* __restrict__ D_,
                                                               E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_,
