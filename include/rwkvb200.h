@@ -88,6 +88,11 @@ int rwkvb200_timex_backward(const float* w, const float* k, const float* gwk, fl
                             float* gk, int B, int C, int T, void* stream);
 int rwkvb200_timex_backward_reduced(const float* w, const float* k, const float* gwk,
                                     float* gw_sum, float* gk, int B, int C, int T, void* stream);
+/* The same with `work` (rwkvb200_timex_work_bytes(B,C,T) bytes, may be NULL when that is 0), which lets parts of the batch be
+ * worked on at the same time. */
+size_t rwkvb200_timex_work_bytes(int B, int C, int T);
+int rwkvb200_timex_train_backward(const float* w, const float* k, const float* gwk, float* gw_sum, float* gk, float* work,
+                                  int B, int C, int T, void* stream);
 
 /* ---------------------------------------------------------------------------------
  * RWKV-5 WKV, fp32 or bf16 activations.  Replaces cuda_forward / cuda_backward of

@@ -9,7 +9,8 @@
 //   forward: F = w[c] (shared by the batch), G = k[b,c]
 //   gw     : F = g[b,c] (one per batch),     G = k[b,c]
 //   gk     : F = w[c], G = g[b,c] read back to front, and the output written back to front.
-// so one kernel template serves them.
+// so one kernel template serves them.  (Lengths of 65 to 1024 go through timex_fft.cu; the gradient per batch row and other
+// lengths are done here.)
 //
 // Mapping: one CTA per (channel, group of BG batch rows).  The filter row(s) and the BG
 // signal rows are staged once in shared memory (zero padded to a multiple of 4 plus a 4-float
@@ -20,7 +21,7 @@
 // tile grows linearly with t, so every thread takes tile p and its mirror image P-1-p: all
 // threads do the same amount of work.  The binding roof of this operator is the FP32 pipe
 // (T/2 FMAs per loaded element), not HBM.
-#include "common.cuh"
+#include "timex_fft.cuh"
 
 namespace rwkvb200 {
 namespace {
@@ -180,6 +181,7 @@ extern "C" int rwkvb200_timex_forward(const float* w, const float* k, float* x, 
                                       void* stream) {
     if (int e = check_dims(B, C, T, "timex_forward")) return e;
     RWKV_NOTNULL(w); RWKV_NOTNULL(k); RWKV_NOTNULL(x);
+    if (timex_fft_applies(T)) return timex_fft_forward(w, k, x, eps, B, C, T, as_stream(stream));
     return launch_any<kFwd>(w, k, x, eps, B, C, T, as_stream(stream), "timex_forward");
 }
 
@@ -195,10 +197,23 @@ extern "C" int rwkvb200_timex_backward_reduced(const float* w, const float* k, c
                                                float* gk, int B, int C, int T, void* stream) {
     if (int e = check_dims(B, C, T, "timex_backward_reduced")) return e;
     RWKV_NOTNULL(w); RWKV_NOTNULL(k); RWKV_NOTNULL(gwk); RWKV_NOTNULL(gw_sum); RWKV_NOTNULL(gk);
+    if (timex_fft_applies(T)) return timex_fft_backward(w, k, gwk, gw_sum, gk, nullptr, B, C, T, as_stream(stream));
     // The per-row filter gradients go into the gk buffer (same shape, written afterwards), are summed over the
     // batch in a fixed order, and only then gk is computed: no extra memory, and the sum does not depend on the
     // order in which thread blocks run (an atomic sum over the batch groups was 3 % faster and did).
     if (int e = launch_any<kGw>(gwk, k, gk, 0.f, B, C, T, as_stream(stream), "timex_backward_reduced(gw)")) return e;
     if (int e = rwkvb200_reduce_batch_partials(RWKVB200_F32, B, C * T, gk, gw_sum, stream)) return e;
     return launch_any<kGk>(w, gwk, gk, 0.f, B, C, T, as_stream(stream), "timex_backward_reduced(gk)");
+}
+
+extern "C" size_t rwkvb200_timex_work_bytes(int B, int C, int T) {
+    return B > 0 && C > 0 && T > 0 && timex_fft_applies(T) ? (size_t)kTimexSplits * C * T * sizeof(float) : 0;
+}
+
+extern "C" int rwkvb200_timex_train_backward(const float* w, const float* k, const float* gwk, float* gw_sum, float* gk, float* work,
+                                             int B, int C, int T, void* stream) {
+    if (!timex_fft_applies(T)) return rwkvb200_timex_backward_reduced(w, k, gwk, gw_sum, gk, B, C, T, stream);
+    if (int e = check_dims(B, C, T, "timex_train_backward")) return e;
+    RWKV_NOTNULL(w); RWKV_NOTNULL(k); RWKV_NOTNULL(gwk); RWKV_NOTNULL(gw_sum); RWKV_NOTNULL(gk); RWKV_NOTNULL(work);
+    return timex_fft_backward(w, k, gwk, gw_sum, gk, work, B, C, T, as_stream(stream));
 }

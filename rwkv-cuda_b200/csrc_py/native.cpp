@@ -61,6 +61,7 @@ void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 Tensor empty(at::IntArrayRef sizes, at::ScalarType d, const Tensor& like) {
     return Tensor(at::detail::empty_cuda(sizes, d, like.device(), std::nullopt));
 }
+Tensor bytes(size_t n, const Tensor& like) { return empty({(int64_t)n}, at::kByte, like); }
 Tensor same(const Tensor& like) { return empty(like.sizes(), like.scalar_type(), like); }
 const float* f32(const void* p) { return static_cast<const float*>(p); }
 float* f32(void* p) { return static_cast<float*>(p); }
@@ -138,16 +139,16 @@ struct TimeX : torch::autograd::Function<TimeX> {
         const Tensor gx = g[0].contiguous();
         numel(gx, B * C * T, "gwk");
         Tensor gw = empty({C, T}, f, gx), gk = empty({B, C, T}, f, gx);
-        check_rc(rwkvb200_timex_backward_reduced(f32(s[0].data_ptr()), f32(s[1].data_ptr()), f32(ptr(gx, "gwk", f)), f32(gw.data_ptr()),
-                                                 f32(gk.data_ptr()), B, C, T, stream()),
-                 "rwkvb200_timex_backward_reduced", true);
+        const size_t nbytes = rwkvb200_timex_work_bytes(B, C, T);
+        Tensor work = nbytes ? bytes(nbytes, gx) : Tensor();
+        check_rc(rwkvb200_timex_train_backward(f32(s[0].data_ptr()), f32(s[1].data_ptr()), f32(ptr(gx, "gwk", f)), f32(gw.data_ptr()),
+                                               f32(gk.data_ptr()), nbytes ? f32(work.data_ptr()) : nullptr, B, C, T, stream()),
+                 "rwkvb200_timex_train_backward", true);
         return {gw, gk, Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
 // ---- RWKV-5 ---------------------------------------------------------------------------------------------------
-static Tensor bytes(size_t n, const Tensor& like) { return empty({(int64_t)n}, at::kByte, like); }
-
 struct Wkv5 : torch::autograd::Function<Wkv5> {
     static Tensor forward(AutogradContext* ctx, int64_t B, int64_t T, int64_t C, int64_t H, Tensor r, Tensor k, Tensor v, Tensor w, Tensor u) {
         for (const Tensor* x : {&k, &v, &w, &u}) assert_py(x->scalar_type() == r.scalar_type(), "r, k, v, w, u must have one dtype");
