@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <stdarg.h>
+#include <atomic>
 
 #include "../../include/rwkvb200.h"
 
@@ -50,6 +51,20 @@ void set_error(const char* fmt, ...);
 
 // Called after every launch: turns a launch-time CUDA error into a status code.
 int check_launch(const char* what);
+
+// Allows a kernel its dynamic shared memory (always the same amount), once per device: the runtime call costs as much as a
+// third of a launch.
+template <auto Kernel>
+inline cudaError_t allow_smem(int bytes) {
+    static std::atomic<unsigned long long> done{0};   // a bit per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 64 && (done.load(std::memory_order_relaxed) >> dev & 1)) return cudaSuccess;
+    e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64) done.fetch_or(1ull << dev, std::memory_order_relaxed);
+    return e;
+}
 
 // out[n] (fp32 or bf16) <- sums over the rows of partial[rows][n] (wkv5.cu)
 int sum_rows(int out_dtype, long long rows, int n, const float* partial, void* out, cudaStream_t st);

@@ -325,7 +325,7 @@ int splits(int B, int C, int G, int most) {
 
 template <int R>
 int forward(const float* w, const float* k, float* x, float eps, int B, int C, int T, cudaStream_t st) {
-    const cudaError_t e = cudaFuncSetAttribute(timex_fft_forward_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan<R>::kSmem);
+    const cudaError_t e = allow_smem<timex_fft_forward_kernel<R>>(Plan<R>::kSmem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "timex_forward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     timex_fft_forward_kernel<R><<<dim3(C, splits(B, C, Plan<R>::G, 1 << 20)), kThreads, Plan<R>::kSmem, st>>>(w, k, x, eps, B, C, T);
     return check_launch("timex_forward(transforms)");
@@ -333,7 +333,7 @@ int forward(const float* w, const float* k, float* x, float eps, int B, int C, i
 
 template <int R>
 int backward(const float* w, const float* k, const float* g, float* gw, float* gk, float* work, int most, int B, int C, int T, cudaStream_t st) {
-    const cudaError_t e = cudaFuncSetAttribute(timex_fft_backward_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan<R>::kSmem);
+    const cudaError_t e = allow_smem<timex_fft_backward_kernel<R>>(Plan<R>::kSmem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "timex_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     const int s = splits(B, C, Plan<R>::G, work != nullptr ? most : 1);
     timex_fft_backward_kernel<R><<<dim3(C, s), kThreads, Plan<R>::kSmem, st>>>(w, k, g, s > 1 ? work : gw, gk, B, C, T);

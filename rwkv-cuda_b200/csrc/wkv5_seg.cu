@@ -409,7 +409,7 @@ int backward(int B, int T, int C, int H, const void* r, const void* k, const voi
              void* gk, void* gv, const float* S, float* D, float* partial, cudaStream_t st) {
     const int N = C / H, nseg = (T + kSeg - 1) / kSeg, smem = sizeof(BwdSmem);
     const dim3 grid(nseg, B * H), scan((N * N + 255) / 256, B * H);
-    const cudaError_t e = cudaFuncSetAttribute(seg_backward_kernel<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem<seg_backward_kernel<E>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv5_train_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     seg_local_kernel<E, true><<<grid, 64, 0, st>>>(T, C, H, N, (const E*)r, (const E*)gy, (const E*)w, D);
     seg_scan_kernel<E, true><<<scan, 256, 0, st>>>(T, H, N, nseg, (const E*)w, D);

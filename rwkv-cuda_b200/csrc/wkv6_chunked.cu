@@ -665,7 +665,7 @@ int wkv6_chunked_forward(int B, int T, int H, const void* r, const void* k, cons
     dim3 grid(H, B);
 #define RWKV_GO1(M, SO)                                                                                                \
     do {                                                                                                               \
-        cudaError_t e = cudaFuncSetAttribute(wkv6c_forward_kernel<M, SO>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+        cudaError_t e = allow_smem<wkv6c_forward_kernel<M, SO>>(\
                                              FSmem::kBytes);                                                           \
         RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv6_forward: cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
         wkv6c_forward_kernel<M, SO><<<grid, NT, FSmem::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)k, (const bf16*)v, \
@@ -715,7 +715,7 @@ int wkv6_chunked_backward(int B, int T, int H, const void* r, const void* k, con
     dim3 grid(H, B);
 #define RWKV_GO(M)                                                                                                      \
     do {                                                                                                                \
-        cudaError_t e = cudaFuncSetAttribute(wkv6c_backward_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
+        cudaError_t e = allow_smem<wkv6c_backward_kernel<M>>(\
                                              BSmem::kBytes);                                                            \
         RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv6_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
         wkv6c_backward_kernel<M><<<grid, NT, BSmem::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)k, (const bf16*)v, w, \

@@ -560,7 +560,7 @@ int wkv6_l32_backward(int B, int T, int H, const void* r, const void* k, const v
     dim3 grid(H, B);
 #define RWKV_GO(M)                                                                                                        \
     do {                                                                                                                  \
-        cudaError_t e = cudaFuncSetAttribute(wkv6b_backward_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kBytes); \
+        cudaError_t e = allow_smem<wkv6b_backward_kernel<M>>(Smem::kBytes); \
         RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv6_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));  \
         wkv6b_backward_kernel<M><<<grid, BNT, Smem::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)k, (const bf16*)v, w,  \
                                                                  (const bf16*)u, (const bf16*)gy, dsT, ck, (bf16*)gr,    \

@@ -465,7 +465,7 @@ int wkv6_l32_forward(int B, int T, int H, const void* r, const void* k, const vo
     dim3 grid(H, B);
 #define RWKV_GO(M)                                                                                                       \
     do {                                                                                                                 \
-        cudaError_t e = cudaFuncSetAttribute(wkv6q_forward_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kBytes); \
+        cudaError_t e = allow_smem<wkv6q_forward_kernel<M>>(Smem::kBytes); \
         RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv6_forward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));  \
         wkv6q_forward_kernel<M><<<grid, PNT, Smem::kBytes, st>>>(T, H, maps, w, (const bf16*)u, s0, s0_kind, (bf16*)y, sT, \
                                                                 ck, unsafe, flag_div);                                       \

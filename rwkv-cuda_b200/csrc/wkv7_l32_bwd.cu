@@ -558,7 +558,7 @@ int wkv7_l32_backward(int B, int T, int H, const void* r, const void* w, const v
                       const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
                       void* dk, void* dv, void* da, void* db, cudaStream_t st) {
     using namespace v7x;
-    cudaError_t e = cudaFuncSetAttribute(wkv7x_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdSmemX::kBytes);
+    cudaError_t e = allow_smem<wkv7x_backward_kernel>(BwdSmemX::kBytes);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv7_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     TileMaps<7> maps;
     const void* in[7] = {r, w, k, v, a, b, dy};

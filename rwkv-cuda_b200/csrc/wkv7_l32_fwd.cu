@@ -263,7 +263,7 @@ WKV7_PHASE_READER(rwkvb200_phase_clocks_l32_fwd)
 int wkv7_l32_forward(int B, int T, int H, const float* s0, const void* r, const void* w, const void* k, const void* v,
                      const void* a, const void* b, void* y, float* sT, float* s, int test_expire, cudaStream_t st) {
     using namespace v7x;
-    cudaError_t e = cudaFuncSetAttribute(wkv7x_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem::kBytes);
+    cudaError_t e = allow_smem<wkv7x_forward_kernel>(FwdSmem::kBytes);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv7_forward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     dim3 grid(H, B);
     wkv7x_forward_kernel<<<grid, FNT, FwdSmem::kBytes, st>>>(T, H, s0, (const bf16*)r, (const bf16*)w, (const bf16*)k,

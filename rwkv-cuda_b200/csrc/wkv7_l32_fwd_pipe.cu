@@ -429,7 +429,7 @@ int wkv7_l32_forward_pipelined(int B, int T, int H, const float* s0, const void*
     const void* in[6] = {r, w, k, v, a, b};
     for (int x = 0; x < 6; ++x)
         if (!make_map(&maps.m[x], in[x], (uint64_t)B * T, (uint64_t)H * 64)) return 1;
-    cudaError_t e = cudaFuncSetAttribute(wkv7q_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PipeSmem::kBytes);
+    cudaError_t e = allow_smem<wkv7q_forward_kernel>(PipeSmem::kBytes);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv7_forward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     dim3 grid(H, B);
     wkv7q_forward_kernel<<<grid, PNT, PipeSmem::kBytes, st>>>(T, H, s0, maps, (bf16*)y, sT, s);

@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(32 * (NCW + 4)) wkv7_rows_kernel(int T, int H,
 template <typename E, int LG, int NCW, int RPT>
 int launch_rows(int B, int T, int H, float* state, const void* r, const void* w, const void* k, const void* v, const void* a,
                 const void* b, void* y, cudaStream_t st) {
-    const cudaError_t e = cudaFuncSetAttribute(wkv7_rows_kernel<E, LG, NCW, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmem);
+    const cudaError_t e = allow_smem<wkv7_rows_kernel<E, LG, NCW, RPT>>(kRowsSmem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv7_state_update: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     wkv7_rows_kernel<E, LG, NCW, RPT><<<dim3(B * H, kN * LG / (32 * NCW * RPT)), 32 * (NCW + 4), kRowsSmem, st>>>(
         T, H, state, (const E*)r, (const E*)w, (const E*)k, (const E*)v, (const E*)a, (const E*)b, (E*)y);

@@ -8,6 +8,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
 #include "../../include/rwkvb200.h"
@@ -15,7 +17,7 @@
 namespace {
 
 using at::Tensor;
-using torch::autograd::AutogradContext;
+using torch::autograd::SavedVariable;
 using torch::autograd::variable_list;
 namespace py = pybind11;
 
@@ -65,6 +67,84 @@ Tensor bytes(size_t n, const Tensor& like) { return empty({(int64_t)n}, at::kByt
 Tensor same(const Tensor& like) { return empty(like.sizes(), like.scalar_type(), like); }
 const float* f32(const void* p) { return static_cast<const float*>(p); }
 float* f32(void* p) { return static_cast<float*>(p); }
+// a tensor of the shape of `like` on the storage of `whole`, from element `offset` on (without a trip through the dispatcher)
+Tensor part(const Tensor& whole, int64_t offset, const Tensor& like) {
+    Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(whole.storage()), whole.key_set(), whole.dtype());
+    t.unsafeGetTensorImpl()->set_storage_offset(offset);
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(like.sizes());
+    return t;
+}
+
+// ---- autograd -------------------------------------------------------------------------------------------------
+// One node type for all operators (a node of its own instead of torch::autograd::Function, whose context, argument unpacking
+// and dictionary cost as much as the launches): the inputs as saved variables, plain tensors that the forward made, a few
+// integers, and the operator's backward, which returns the gradients in the order of `inputs`.
+struct Saved {
+    std::array<Tensor, 8> in;       // contiguous inputs
+    std::array<Tensor, 2> own;      // buffers of the forward
+    std::array<int64_t, 6> dims{};
+};
+using BackwardFn = variable_list (*)(const Saved&, const variable_list& grads);
+
+struct OpNode : torch::autograd::Node {
+    BackwardFn fn = nullptr;
+    const char* op = "";
+    int n = 0;
+    std::array<SavedVariable, 8> in;
+    std::array<Tensor, 8> copy;      // where a contiguous copy of the input had to be made
+    Saved own;
+    bool released = false;
+
+    std::string name() const override { return op; }
+    void release_variables() override {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (auto& x : in) x.reset_data();
+        for (auto& x : copy) x.reset();
+        for (auto& x : own.own) x.reset();
+        released = true;
+    }
+    variable_list apply(variable_list&& grads) override {
+        Saved s;
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+            for (int i = 0; i < n; ++i) s.in[i] = copy[i].defined() ? copy[i] : in[i].unpack();
+            s.own = own.own;
+            s.dims = own.dims;
+        }
+        at::AutoDispatchBelowAutograd no_graph;
+        for (size_t i = 0; i < grads.size(); ++i)
+            grads[i] = grads[i].defined() ? grads[i].contiguous() : input_metadata(i).zeros_like();
+        return fn(s, grads);
+    }
+};
+
+// Ties `outputs` to a node that keeps `inputs` (as given) and what `s` holds; s.in are their contiguous forms.
+void record(const char* op, BackwardFn fn, at::ArrayRef<Tensor> inputs, Saved&& s, at::ArrayRef<Tensor> outputs) {
+    bool any = false;
+    for (const Tensor& x : inputs) any |= x.requires_grad();
+    if (!any || !at::GradMode::is_enabled()) return;
+    auto node = std::shared_ptr<OpNode>(new OpNode(), torch::autograd::deleteNode);
+    torch::autograd::edge_list edges;
+    edges.reserve(inputs.size());
+    for (const Tensor& x : inputs) edges.push_back(torch::autograd::impl::gradient_edge(x));
+    node->set_next_edges(std::move(edges));
+    node->fn = fn;
+    node->op = op;
+    node->n = inputs.size();
+    for (int i = 0; i < node->n; ++i) {
+        if (s.in[i].is_same(inputs[i])) node->in[i] = SavedVariable(inputs[i], false);
+        else node->copy[i] = s.in[i];
+    }
+    node->own.own = std::move(s.own);
+    node->own.dims = s.dims;
+    for (const Tensor& y : outputs) torch::autograd::set_history(y, node);
+}
+Tensor dense(const Tensor& x) {   // contiguous form, outside of the graph
+    if (x.is_contiguous()) return x;
+    at::NoGradGuard guard;
+    return x.contiguous();
+}
 
 }  // namespace
 
@@ -82,223 +162,206 @@ static void wkv7_state_update(const Tensor& state, const Tensor& r, const Tensor
 }
 
 // ---- RWKV-4 -------------------------------------------------------------------------------------------------
-struct Wkv4 : torch::autograd::Function<Wkv4> {
-    static Tensor forward(AutogradContext* ctx, int64_t B, int64_t T, int64_t C, Tensor w, Tensor u, Tensor k, Tensor v) {
-        on_device(k, "k");
-        const c10::cuda::CUDAGuard guard(k.device());
-        const auto f = at::kFloat;
-        w = w.contiguous(); u = u.contiguous(); k = k.contiguous(); v = v.contiguous();
-        numel(w, C, "w"); numel(u, C, "u"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v");
-        Tensor y = empty({B, T, C}, f, k);
-        Tensor saved = empty({(int64_t)rwkvb200_wkv4_saved_bytes(B, T, C)}, at::kByte, k);
-        check_rc(rwkvb200_wkv4_train_forward(B, T, C, f32(ptr(w, "w", f)), f32(ptr(u, "u", f)), f32(ptr(k, "k", f)), f32(ptr(v, "v", f)),
-                                             f32(y.data_ptr()), saved.data_ptr(), stream()),
-                 "rwkvb200_wkv4_train_forward");
-        ctx->save_for_backward({w, u, k, v, saved});
-        ctx->saved_data["dims"] = std::vector<int64_t>{B, T, C};
-        return y;
-    }
-    static variable_list backward(AutogradContext* ctx, variable_list g) {
-        const auto s = ctx->get_saved_variables();
-        const auto dims = ctx->saved_data["dims"].toIntVector();
-        const int64_t B = dims[0], T = dims[1], C = dims[2];
-        const c10::cuda::CUDAGuard guard(s[2].device());
-        const auto f = at::kFloat;
-        const Tensor gy = g[0].contiguous();
-        numel(gy, B * T * C, "gy");
-        Tensor gwu = empty({2, C}, f, gy), gk = empty({B, T, C}, f, gy), gv = empty({B, T, C}, f, gy);
-        Tensor partial = B > 1 ? empty({B, 2, C}, f, gy) : Tensor();
-        check_rc(rwkvb200_wkv4_train_backward(B, T, C, f32(s[0].data_ptr()), f32(s[1].data_ptr()), f32(s[2].data_ptr()), f32(s[3].data_ptr()),
-                                              f32(ptr(gy, "gy", f)), s[4].data_ptr(), f32(gwu.data_ptr()),
-                                              partial.defined() ? f32(partial.data_ptr()) : nullptr, f32(gk.data_ptr()), f32(gv.data_ptr()), stream()),
-                 "rwkvb200_wkv4_train_backward", true);
-        return {Tensor(), Tensor(), Tensor(), gwu.select(0, 0).view_as(s[0]), gwu.select(0, 1).view_as(s[1]), gk, gv};
-    }
-};
+static variable_list wkv4_backward(const Saved& s, const variable_list& g) {
+    const auto [B, T, C, d3, d4, d5] = s.dims;
+    const c10::cuda::CUDAGuard guard(s.in[2].device());
+    const auto f = at::kFloat;
+    const Tensor& gy = g[0];
+    numel(gy, B * T * C, "gy");
+    Tensor gwu = empty({2, C}, f, gy), gk = empty({B, T, C}, f, gy), gv = empty({B, T, C}, f, gy);
+    const Tensor partial = B > 1 ? empty({B, 2, C}, f, gy) : Tensor();
+    check_rc(rwkvb200_wkv4_train_backward(B, T, C, f32(s.in[0].data_ptr()), f32(s.in[1].data_ptr()), f32(s.in[2].data_ptr()),
+                                          f32(s.in[3].data_ptr()), f32(ptr(gy, "gy", f)), s.own[0].data_ptr(), f32(gwu.data_ptr()),
+                                          partial.defined() ? f32(partial.data_ptr()) : nullptr, f32(gk.data_ptr()), f32(gv.data_ptr()), stream()),
+             "rwkvb200_wkv4_train_backward", true);
+    return {part(gwu, 0, s.in[0]), part(gwu, C, s.in[1]), std::move(gk), std::move(gv)};
+}
+static Tensor wkv4(int64_t B, int64_t T, int64_t C, const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+    on_device(k, "k");
+    const c10::cuda::CUDAGuard guard(k.device());
+    const auto f = at::kFloat;
+    Saved s{{dense(w), dense(u), dense(k), dense(v)}, {}, {B, T, C}};
+    numel(w, C, "w"); numel(u, C, "u"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v");
+    Tensor y = empty({B, T, C}, f, k);
+    s.own[0] = bytes(rwkvb200_wkv4_saved_bytes(B, T, C), k);
+    check_rc(rwkvb200_wkv4_train_forward(B, T, C, f32(ptr(s.in[0], "w", f)), f32(ptr(s.in[1], "u", f)), f32(ptr(s.in[2], "k", f)),
+                                         f32(ptr(s.in[3], "v", f)), f32(y.data_ptr()), s.own[0].data_ptr(), stream()),
+             "rwkvb200_wkv4_train_forward");
+    record("WKV", wkv4_backward, {w, u, k, v}, std::move(s), {y});
+    return y;
+}
 
 // ---- depthwise_conv1d -----------------------------------------------------------------------------------------
-struct TimeX : torch::autograd::Function<TimeX> {
-    static Tensor forward(AutogradContext* ctx, Tensor w, Tensor k, int64_t B, int64_t C, int64_t T, double eps) {
-        on_device(k, "k");
-        const c10::cuda::CUDAGuard guard(k.device());
-        const auto f = at::kFloat;
-        w = w.contiguous(); k = k.contiguous();
-        numel(w, C * T, "w"); numel(k, B * C * T, "k");
-        Tensor x = empty({B, C, T}, f, k);
-        check_rc(rwkvb200_timex_forward(f32(ptr(w, "w", f)), f32(ptr(k, "k", f)), f32(x.data_ptr()), (float)eps, B, C, T, stream()), "rwkvb200_timex_forward");
-        ctx->save_for_backward({w, k});
-        ctx->saved_data["dims"] = std::vector<int64_t>{B, C, T};
-        return x;
-    }
-    static variable_list backward(AutogradContext* ctx, variable_list g) {
-        const auto s = ctx->get_saved_variables();
-        const auto dims = ctx->saved_data["dims"].toIntVector();
-        const int64_t B = dims[0], C = dims[1], T = dims[2];
-        const c10::cuda::CUDAGuard guard(s[1].device());
-        const auto f = at::kFloat;
-        const Tensor gx = g[0].contiguous();
-        numel(gx, B * C * T, "gwk");
-        Tensor gw = empty({C, T}, f, gx), gk = empty({B, C, T}, f, gx);
-        const size_t nbytes = rwkvb200_timex_work_bytes(B, C, T);
-        Tensor work = nbytes ? bytes(nbytes, gx) : Tensor();
-        check_rc(rwkvb200_timex_train_backward(f32(s[0].data_ptr()), f32(s[1].data_ptr()), f32(ptr(gx, "gwk", f)), f32(gw.data_ptr()),
-                                               f32(gk.data_ptr()), nbytes ? f32(work.data_ptr()) : nullptr, B, C, T, stream()),
-                 "rwkvb200_timex_train_backward", true);
-        return {gw, gk, Tensor(), Tensor(), Tensor(), Tensor()};
-    }
-};
+static variable_list timex_backward(const Saved& s, const variable_list& g) {
+    const auto [B, C, T, d3, d4, d5] = s.dims;
+    const c10::cuda::CUDAGuard guard(s.in[1].device());
+    const auto f = at::kFloat;
+    const Tensor& gx = g[0];
+    numel(gx, B * C * T, "gwk");
+    Tensor gw = empty({C, T}, f, gx), gk = empty({B, C, T}, f, gx);
+    const size_t nbytes = rwkvb200_timex_work_bytes(B, C, T);
+    const Tensor work = nbytes ? bytes(nbytes, gx) : Tensor();
+    check_rc(rwkvb200_timex_train_backward(f32(s.in[0].data_ptr()), f32(s.in[1].data_ptr()), f32(ptr(gx, "gwk", f)), f32(gw.data_ptr()),
+                                           f32(gk.data_ptr()), nbytes ? f32(work.data_ptr()) : nullptr, B, C, T, stream()),
+             "rwkvb200_timex_train_backward", true);
+    return {std::move(gw), std::move(gk)};
+}
+static Tensor timex(const Tensor& w, const Tensor& k, int64_t B, int64_t C, int64_t T, double eps) {
+    on_device(k, "k");
+    const c10::cuda::CUDAGuard guard(k.device());
+    const auto f = at::kFloat;
+    Saved s{{dense(w), dense(k)}, {}, {B, C, T}};
+    numel(w, C * T, "w"); numel(k, B * C * T, "k");
+    Tensor x = empty({B, C, T}, f, k);
+    check_rc(rwkvb200_timex_forward(f32(ptr(s.in[0], "w", f)), f32(ptr(s.in[1], "k", f)), f32(x.data_ptr()), (float)eps, B, C, T, stream()),
+             "rwkvb200_timex_forward");
+    record("TimeX", timex_backward, {w, k}, std::move(s), {x});
+    return x;
+}
 
 // ---- RWKV-5 ---------------------------------------------------------------------------------------------------
-struct Wkv5 : torch::autograd::Function<Wkv5> {
-    static Tensor forward(AutogradContext* ctx, int64_t B, int64_t T, int64_t C, int64_t H, Tensor r, Tensor k, Tensor v, Tensor w, Tensor u) {
-        for (const Tensor* x : {&k, &v, &w, &u}) assert_py(x->scalar_type() == r.scalar_type(), "r, k, v, w, u must have one dtype");
-        on_device(r, "r");
-        const c10::cuda::CUDAGuard guard(r.device());
-        const auto d = r.scalar_type();
-        const int dtype = dt(r, "r");
-        r = r.contiguous(); k = k.contiguous(); v = v.contiguous(); w = w.contiguous(); u = u.contiguous();
-        numel(r, B * T * C, "r"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v"); numel(w, C, "w"); numel(u, C, "u");
-        Tensor y = empty({B, T, C}, d, r), saved = bytes(rwkvb200_wkv5_train_saved_bytes(B, T, C, H), r);
-        const int path = rwkvb200_wkv5_train_forward(dtype, B, T, C, H, ptr(r, "r", d), ptr(k, "k", d), ptr(v, "v", d), ptr(w, "w", d),
-                                                     ptr(u, "u", d), y.data_ptr(), saved.data_ptr(), stream());
-        check_rc(path, "rwkvb200_wkv5_train_forward");
-        ctx->save_for_backward({r, k, v, w, u, saved});
-        ctx->saved_data["dims"] = std::vector<int64_t>{B, T, C, H, path};
-        return y;
-    }
-    static variable_list backward(AutogradContext* ctx, variable_list g) {
-        const auto s = ctx->get_saved_variables();
-        const auto dims = ctx->saved_data["dims"].toIntVector();
-        const int64_t B = dims[0], T = dims[1], C = dims[2], H = dims[3], path = dims[4];
-        const c10::cuda::CUDAGuard guard(s[0].device());
-        const auto d = s[0].scalar_type();
-        const Tensor gy = g[0].contiguous();
-        numel(gy, B * T * C, "gy");
-        Tensor gr = empty({B, T, C}, d, gy), gk = empty({B, T, C}, d, gy), gv = empty({B, T, C}, d, gy), gwu = empty({2, C}, d, gy);
-        Tensor work = bytes(rwkvb200_wkv5_train_work_bytes(B, T, C, H, path), gy);
-        check_rc(rwkvb200_wkv5_train_backward(dt(s[0], "r"), B, T, C, H, path, s[0].data_ptr(), s[1].data_ptr(), s[2].data_ptr(), s[3].data_ptr(),
-                                              s[4].data_ptr(), ptr(gy, "gy", d), gr.data_ptr(), gk.data_ptr(), gv.data_ptr(), gwu.data_ptr(),
-                                              s[5].data_ptr(), work.data_ptr(), stream()),
-                 "rwkvb200_wkv5_train_backward", true);
-        return {Tensor(), Tensor(), Tensor(), Tensor(), gr, gk, gv, gwu.select(0, 0).view_as(s[3]), gwu.select(0, 1).view_as(s[4])};
-    }
-};
+static variable_list wkv5_backward(const Saved& s, const variable_list& g) {
+    const auto [B, T, C, H, path, d5] = s.dims;
+    const c10::cuda::CUDAGuard guard(s.in[0].device());
+    const auto d = s.in[0].scalar_type();
+    const Tensor& gy = g[0];
+    numel(gy, B * T * C, "gy");
+    Tensor gr = empty({B, T, C}, d, gy), gk = empty({B, T, C}, d, gy), gv = empty({B, T, C}, d, gy), gwu = empty({2, C}, d, gy);
+    const Tensor work = bytes(rwkvb200_wkv5_train_work_bytes(B, T, C, H, path), gy);
+    check_rc(rwkvb200_wkv5_train_backward(dt(s.in[0], "r"), B, T, C, H, path, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
+                                          s.in[3].data_ptr(), s.in[4].data_ptr(), ptr(gy, "gy", d), gr.data_ptr(), gk.data_ptr(), gv.data_ptr(),
+                                          gwu.data_ptr(), s.own[0].data_ptr(), work.data_ptr(), stream()),
+             "rwkvb200_wkv5_train_backward", true);
+    return {std::move(gr), std::move(gk), std::move(gv), part(gwu, 0, s.in[3]), part(gwu, C, s.in[4])};
+}
+static Tensor wkv5(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
+    for (const Tensor* x : {&k, &v, &w, &u}) assert_py(x->scalar_type() == r.scalar_type(), "r, k, v, w, u must have one dtype");
+    on_device(r, "r");
+    const c10::cuda::CUDAGuard guard(r.device());
+    const auto d = r.scalar_type();
+    const int dtype = dt(r, "r");
+    Saved s{{dense(r), dense(k), dense(v), dense(w), dense(u)}, {}, {B, T, C, H}};
+    numel(r, B * T * C, "r"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v"); numel(w, C, "w"); numel(u, C, "u");
+    Tensor y = empty({B, T, C}, d, r);
+    s.own[0] = bytes(rwkvb200_wkv5_train_saved_bytes(B, T, C, H), r);
+    const int path = rwkvb200_wkv5_train_forward(dtype, B, T, C, H, ptr(s.in[0], "r", d), ptr(s.in[1], "k", d), ptr(s.in[2], "v", d),
+                                                 ptr(s.in[3], "w", d), ptr(s.in[4], "u", d), y.data_ptr(), s.own[0].data_ptr(), stream());
+    check_rc(path, "rwkvb200_wkv5_train_forward");
+    s.dims[4] = path;
+    record("WKV_5", wkv5_backward, {r, k, v, w, u}, std::move(s), {y});
+    return y;
+}
 
-// ---- RWKV-6, without a state (kState = false) or with an fp32 state in and out ----------------------------------------
-template <bool kState>
-struct Wkv6 : torch::autograd::Function<Wkv6<kState>> {
-    static variable_list forward(AutogradContext* ctx, int64_t B, int64_t T, int64_t C, int64_t H, Tensor r, Tensor k, Tensor v, Tensor w,
-                                 Tensor u, std::optional<Tensor> state) {
-        on_device(r, "r");
-        Tensor s0 = kState ? state->contiguous() : Tensor();
-        const c10::cuda::CUDAGuard guard(r.device());
-        const auto d = r.scalar_type(), f = at::kFloat;
-        const int dtype = dt(r, "r");
-        r = r.contiguous(); k = k.contiguous(); v = v.contiguous(); w = w.contiguous(); u = u.contiguous();
-        numel(r, B * T * C, "r"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v"); numel(w, B * T * C, "w"); numel(u, C, "u");
-        if (kState) numel(s0, B * H * (C / H) * (C / H), "s0");
-        Tensor y = empty({B, T, C}, d, r), sT = kState ? same(s0) : Tensor();
-        Tensor saved = bytes(rwkvb200_wkv6_train_saved_bytes(dtype, B, T, C, H), r);
-        const int path = rwkvb200_wkv6_train_forward(dtype, B, T, C, H, ptr(r, "r", d), ptr(k, "k", d), ptr(v, "v", d), ptr(w, "w", d), ptr(u, "u", d),
-                                                     kState ? f32(ptr(s0, "s0", f)) : nullptr, y.data_ptr(), kState ? f32(sT.data_ptr()) : nullptr,
-                                                     saved.data_ptr(), stream());
-        check_rc(path, "rwkvb200_wkv6_train_forward");
-        ctx->save_for_backward({r, k, v, w, u, saved, kState ? s0 : saved});
-        ctx->saved_data["dims"] = std::vector<int64_t>{B, T, C, H, path};
-        if (kState) return {y, sT};
-        return {y};
+// ---- RWKV-6, without a state or with an fp32 state in and out (s0, sT, dsT, ds0) ------------------------------------------
+static variable_list wkv6_backward(const Saved& s, const variable_list& g) {
+    const auto [B, T, C, H, path, state] = s.dims;
+    const c10::cuda::CUDAGuard guard(s.in[0].device());
+    const auto d = s.in[0].scalar_type(), f = at::kFloat;
+    const Tensor& gy = g[0];
+    numel(gy, B * T * C, "gy");
+    Tensor gr = empty({B, T, C}, d, gy), gk = empty({B, T, C}, d, gy), gv = empty({B, T, C}, d, gy), gw = empty({B, T, C}, d, gy);
+    Tensor gu = empty(s.in[4].sizes(), d, gy), ds0 = state ? same(s.in[5]) : Tensor();
+    const Tensor work = bytes(rwkvb200_wkv6_train_work_bytes(B, T, C, path), gy);
+    check_rc(rwkvb200_wkv6_train_backward(dt(s.in[0], "r"), B, T, C, H, path, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
+                                          s.in[3].data_ptr(), s.in[4].data_ptr(), state ? f32(s.in[5].data_ptr()) : nullptr, ptr(gy, "gy", d),
+                                          state ? f32(ptr(g[1], "dsT", f)) : nullptr, gr.data_ptr(), gk.data_ptr(), gv.data_ptr(), gw.data_ptr(),
+                                          gu.data_ptr(), state ? f32(ds0.data_ptr()) : nullptr, s.own[0].data_ptr(), work.data_ptr(), stream()),
+             "rwkvb200_wkv6_train_backward", true);
+    variable_list out{std::move(gr), std::move(gk), std::move(gv), std::move(gw), std::move(gu)};
+    if (state) out.push_back(std::move(ds0));
+    return out;
+}
+static std::tuple<Tensor, Tensor> wkv6_forward(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v,
+                                               const Tensor& w, const Tensor& u, const Tensor* s0) {
+    on_device(r, "r");
+    const c10::cuda::CUDAGuard guard(r.device());
+    const auto d = r.scalar_type(), f = at::kFloat;
+    const int dtype = dt(r, "r");
+    Saved s{{dense(r), dense(k), dense(v), dense(w), dense(u)}, {}, {B, T, C, H, 0, s0 != nullptr}};
+    numel(r, B * T * C, "r"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v"); numel(w, B * T * C, "w"); numel(u, C, "u");
+    Tensor y = empty({B, T, C}, d, r), sT;
+    if (s0) {
+        numel(*s0, B * H * (C / H) * (C / H), "s0");
+        s.in[5] = dense(*s0);
+        sT = same(*s0);
     }
-    static variable_list backward(AutogradContext* ctx, variable_list g) {
-        const auto s = ctx->get_saved_variables();
-        const auto dims = ctx->saved_data["dims"].toIntVector();
-        const int64_t B = dims[0], T = dims[1], C = dims[2], H = dims[3], path = dims[4];
-        const c10::cuda::CUDAGuard guard(s[0].device());
-        const auto d = s[0].scalar_type(), f = at::kFloat;
-        const Tensor gy = g[0].contiguous(), dsT = kState ? g[1].contiguous() : Tensor();
-        numel(gy, B * T * C, "gy");
-        Tensor gr = empty({B, T, C}, d, gy), gk = empty({B, T, C}, d, gy), gv = empty({B, T, C}, d, gy), gw = empty({B, T, C}, d, gy);
-        Tensor gu = empty(s[4].sizes(), d, gy), ds0 = kState ? same(s[6]) : Tensor();
-        Tensor work = bytes(rwkvb200_wkv6_train_work_bytes(B, T, C, path), gy);
-        check_rc(rwkvb200_wkv6_train_backward(dt(s[0], "r"), B, T, C, H, path, s[0].data_ptr(), s[1].data_ptr(), s[2].data_ptr(), s[3].data_ptr(),
-                                              s[4].data_ptr(), kState ? f32(s[6].data_ptr()) : nullptr, ptr(gy, "gy", d),
-                                              kState ? f32(ptr(dsT, "dsT", f)) : nullptr, gr.data_ptr(), gk.data_ptr(), gv.data_ptr(), gw.data_ptr(),
-                                              gu.data_ptr(), kState ? f32(ds0.data_ptr()) : nullptr, s[5].data_ptr(), work.data_ptr(), stream()),
-                 "rwkvb200_wkv6_train_backward", true);
-        return {Tensor(), Tensor(), Tensor(), Tensor(), gr, gk, gv, gw, gu, ds0};
-    }
-};
+    s.own[0] = bytes(rwkvb200_wkv6_train_saved_bytes(dtype, B, T, C, H), r);
+    const int path = rwkvb200_wkv6_train_forward(dtype, B, T, C, H, ptr(s.in[0], "r", d), ptr(s.in[1], "k", d), ptr(s.in[2], "v", d),
+                                                 ptr(s.in[3], "w", d), ptr(s.in[4], "u", d), s0 ? f32(ptr(s.in[5], "s0", f)) : nullptr,
+                                                 y.data_ptr(), s0 ? f32(sT.data_ptr()) : nullptr, s.own[0].data_ptr(), stream());
+    check_rc(path, "rwkvb200_wkv6_train_forward");
+    s.dims[4] = path;
+    if (s0) record("WKV_6STATE_EX", wkv6_backward, {r, k, v, w, u, *s0}, std::move(s), {y, sT});
+    else record("WKV_6", wkv6_backward, {r, k, v, w, u}, std::move(s), {y});
+    return {y, sT};
+}
 
 // ---- RWKV-7, the three operators: state in (s0) and out (sT) or not ---------------------------------------------
 constexpr int64_t kChunkLen = 16;
 
-template <bool kS0, bool kST>
-struct Wkv7 : torch::autograd::Function<Wkv7<kS0, kST>> {
-    static variable_list forward(AutogradContext* ctx, std::optional<Tensor> state, Tensor r, Tensor w, Tensor k, Tensor v, Tensor a, Tensor b) {
-        const Tensor s0 = kS0 ? *state : Tensor();
-        assert_py(r.dim() == 4 && r.size(1) % kChunkLen == 0, "T must be a multiple of 16");
-        for (const Tensor* x : {&w, &k, &v, &a, &b}) assert_py(x->scalar_type() == r.scalar_type(), "r, w, k, v, a, b must have one dtype");
-        for (const Tensor* x : {&r, &w, &k, &v, &a, &b}) assert_py(x->is_contiguous(), "r, w, k, v, a, b must be contiguous");
-        if (kS0) assert_py(s0.scalar_type() == at::kFloat && s0.is_contiguous(), "s0 must be contiguous float32");
-        on_device(r, "r");
-        const c10::cuda::CUDAGuard guard(r.device());
-        const auto d = r.scalar_type(), f = at::kFloat;
-        const int dtype = dt(r, "r");
-        const int64_t B = r.size(0), T = r.size(1), H = r.size(2), N = r.size(3);
-        Tensor y = same(v), sT = kST ? same(s0) : Tensor();
-        Tensor s = empty({B, H, T / kChunkLen, N, N}, f, r), sa = empty({B, T, H, N}, f, r);
-        check_rc(rwkvb200_wkv7_forward(dtype, B, T, H, N, kChunkLen, kS0 ? f32(ptr(s0, "s0", f)) : nullptr, ptr(r, "r", d), ptr(w, "w", d),
-                                       ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
-                                       kST ? f32(sT.data_ptr()) : nullptr, f32(s.data_ptr()), f32(sa.data_ptr()), stream()),
-                 "rwkvb200_wkv7_forward");
-        ctx->save_for_backward({r, w, k, v, a, b, s, sa});
-        if (kST) return {y.view({B, T, H * N}), sT};
-        return {y};
-    }
-    static variable_list backward(AutogradContext* ctx, variable_list g) {
-        const auto x = ctx->get_saved_variables();
-        const c10::cuda::CUDAGuard guard(x[0].device());
-        const auto d = x[0].scalar_type(), f = at::kFloat;
-        const int64_t B = x[0].size(0), T = x[0].size(1), H = x[0].size(2), N = x[0].size(3);
-        const Tensor dy = g[0].contiguous(), dsT = kST ? g[1].contiguous() : Tensor();
-        if (kST && dsT.scalar_type() != f) raise(PyExc_AssertionError, "dsT must be float32", true);
-        Tensor ds0 = kS0 ? empty({B, H, N, N}, f, dy) : Tensor();
-        variable_list out{ds0};
-        for (int i = 0; i < 6; ++i) out.push_back(same(x[i]));
-        check_rc(rwkvb200_wkv7_backward(dt(x[0], "r"), B, T, H, N, kChunkLen, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), x[3].data_ptr(),
-                                        x[4].data_ptr(), x[5].data_ptr(), ptr(dy, "dy", d), kST ? f32(ptr(dsT, "dsT", f)) : nullptr,
-                                        f32(x[6].data_ptr()), f32(x[7].data_ptr()), kS0 ? f32(ds0.data_ptr()) : nullptr, out[1].data_ptr(),
-                                        out[2].data_ptr(), out[3].data_ptr(), out[4].data_ptr(), out[5].data_ptr(), out[6].data_ptr(), stream()),
-                 "rwkvb200_wkv7_backward", true);
-        return out;
-    }
-};
+static variable_list wkv7_backward(const Saved& s, const variable_list& g) {
+    const auto [B, T, H, N, s0, sT] = s.dims;
+    const c10::cuda::CUDAGuard guard(s.in[0].device());
+    const auto d = s.in[0].scalar_type(), f = at::kFloat;
+    if (sT && g[1].scalar_type() != f) raise(PyExc_AssertionError, "dsT must be float32", true);
+    std::array<Tensor, 6> x;
+    for (auto& t : x) t = empty({B, T, H, N}, d, g[0]);
+    Tensor ds0 = s0 ? empty({B, H, N, N}, f, g[0]) : Tensor();
+    check_rc(rwkvb200_wkv7_backward(dt(s.in[0], "r"), B, T, H, N, kChunkLen, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
+                                    s.in[3].data_ptr(), s.in[4].data_ptr(), s.in[5].data_ptr(), ptr(g[0], "dy", d),
+                                    sT ? f32(ptr(g[1], "dsT", f)) : nullptr, f32(s.own[0].data_ptr()), f32(s.own[1].data_ptr()),
+                                    s0 ? f32(ds0.data_ptr()) : nullptr, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), x[3].data_ptr(),
+                                    x[4].data_ptr(), x[5].data_ptr(), stream()),
+             "rwkvb200_wkv7_backward", true);
+    variable_list out{std::move(x[0]), std::move(x[1]), std::move(x[2]), std::move(x[3]), std::move(x[4]), std::move(x[5])};
+    if (s0) out.push_back(std::move(ds0));
+    return out;
+}
+static std::tuple<Tensor, Tensor> wkv7_forward(const Tensor* s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v,
+                                               const Tensor& a, const Tensor& b, bool passing) {
+    assert_py(r.dim() == 4 && r.size(1) % kChunkLen == 0, "T must be a multiple of 16");
+    for (const Tensor* x : {&w, &k, &v, &a, &b}) assert_py(x->scalar_type() == r.scalar_type(), "r, w, k, v, a, b must have one dtype");
+    for (const Tensor* x : {&r, &w, &k, &v, &a, &b}) assert_py(x->is_contiguous(), "r, w, k, v, a, b must be contiguous");
+    if (s0) assert_py(s0->scalar_type() == at::kFloat && s0->is_contiguous(), "s0 must be contiguous float32");
+    on_device(r, "r");
+    const c10::cuda::CUDAGuard guard(r.device());
+    const auto d = r.scalar_type(), f = at::kFloat;
+    const int dtype = dt(r, "r");
+    const int64_t B = r.size(0), T = r.size(1), H = r.size(2), N = r.size(3);
+    Tensor y = passing ? empty({B, T, H * N}, d, r) : same(v), sT = passing ? same(*s0) : Tensor();
+    Saved s{{r, w, k, v, a, b}, {empty({B, H, T / kChunkLen, N, N}, f, r), empty({B, T, H, N}, f, r)}, {B, T, H, N, s0 != nullptr, passing}};
+    check_rc(rwkvb200_wkv7_forward(dtype, B, T, H, N, kChunkLen, s0 ? f32(ptr(*s0, "s0", f)) : nullptr, ptr(r, "r", d), ptr(w, "w", d),
+                                   ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
+                                   passing ? f32(sT.data_ptr()) : nullptr, f32(s.own[0].data_ptr()), f32(s.own[1].data_ptr()), stream()),
+             "rwkvb200_wkv7_forward");
+    if (s0) s.in[6] = *s0;
+    const char* op = passing ? "RWKV7_STATE_PASSING_CLAMPW_CUDA_OP" : s0 ? "RWKV7_STATE_CLAMPW_CUDA_OP" : "RWKV7_CLAMPW_CUDA_OP";
+    if (passing) record(op, wkv7_backward, {r, w, k, v, a, b, *s0}, std::move(s), {y, sT});
+    else if (s0) record(op, wkv7_backward, {r, w, k, v, a, b, *s0}, std::move(s), {y});
+    else record(op, wkv7_backward, {r, w, k, v, a, b}, std::move(s), {y});
+    return {y, sT};
+}
 
 PYBIND11_MODULE(_native, m) {
     m.def("set_error_class", [](py::object cls) { g_error_class = cls.inc_ref().ptr(); });
     m.def("wkv7_state_update", &wkv7_state_update);
-    m.def("wkv4", [](int64_t B, int64_t T, int64_t C, const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
-        return Wkv4::apply(B, T, C, w, u, k, v);
-    });
-    m.def("timex", [](const Tensor& w, const Tensor& k, int64_t B, int64_t C, int64_t T, double eps) { return TimeX::apply(w, k, B, C, T, eps); });
-    m.def("wkv5", [](int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
-        return Wkv5::apply(B, T, C, H, r, k, v, w, u);
-    });
+    m.def("wkv4", &wkv4);
+    m.def("timex", &timex);
+    m.def("wkv5", &wkv5);
     m.def("wkv6", [](int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
-        return Wkv6<false>::apply(B, T, C, H, r, k, v, w, u, std::optional<Tensor>())[0];
+        return std::get<0>(wkv6_forward(B, T, C, H, r, k, v, w, u, nullptr));
     });
     m.def("wkv6_state", [](const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u, const Tensor& s0) {
         TORCH_CHECK_VALUE(r.dim() == 3, "r: expected (B,T,C), got ", r.sizes());
-        const auto out = Wkv6<true>::apply(r.size(0), r.size(1), r.size(2), u.size(0), r, k, v, w, u, std::optional<Tensor>(s0));
-        return std::make_tuple(out[0], out[1]);
+        return wkv6_forward(r.size(0), r.size(1), r.size(2), u.size(0), r, k, v, w, u, &s0);
     });
     m.def("wkv7", [](const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        return Wkv7<false, false>::apply(std::optional<Tensor>(), r, w, k, v, a, b)[0];
+        return std::get<0>(wkv7_forward(nullptr, r, w, k, v, a, b, false));
     });
     m.def("wkv7_state", [](const Tensor& s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        return Wkv7<true, false>::apply(std::optional<Tensor>(s0), r, w, k, v, a, b)[0];
+        return std::get<0>(wkv7_forward(&s0, r, w, k, v, a, b, false));
     });
     m.def("wkv7_statepassing", [](const Tensor& s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        const auto out = Wkv7<true, true>::apply(std::optional<Tensor>(s0), r, w, k, v, a, b);
-        return std::make_tuple(out[0], out[1]);
+        return wkv7_forward(&s0, r, w, k, v, a, b, true);
     });
 }
