@@ -107,12 +107,13 @@ __device__ __forceinline__ Place place(int C, int lane) {
 template <int S, bool Y>
 __global__ void __launch_bounds__(32 * S) wkv4_forward_kernel(int T, int C, const float* __restrict__ w_, int w_raw, const float* __restrict__ u_,
                                                               const float* __restrict__ k_, const float* __restrict__ v_,
-                                                              float* __restrict__ y_, States st) {
+                                                              float* __restrict__ y_, States st, unsigned* counters) {
     __shared__ ScanBuf<S> buf;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Place at = place(C, lane);
     const i64 off = (i64)at.b * T * C + at.c;
     const float w = w_raw ? -expf(w_[at.c]) : w_[at.c], u = u_[at.c];
+    if (counters != nullptr && threadIdx.x == 0 && at.b == 0) counters[blockIdx.x] = 0;   // for the backward
     if (warp == 0) { buf.w[lane] = w; buf.carry[0][lane] = 0.f; buf.carry[1][lane] = 0.f; buf.carry[2][lane] = kNegInf; }
     float kn[L], vn[L];
     auto fetch = [&](int t0) {
@@ -151,13 +152,15 @@ __global__ void __launch_bounds__(32 * S) wkv4_forward_kernel(int T, int C, cons
     }
 }
 
-// gw, gu: per batch row (row stride gstride), added to when `accumulate`
+// gw, gu: per batch row (row stride gstride), added to when `accumulate`.  With `sum_` (2,C) the last block of a channel group to
+// finish adds the rows up in order (counters[group] counts the others and is left at zero): no launch for it.
 template <int S>
 __global__ void __launch_bounds__(32 * S, 16 / S) wkv4_backward_kernel(int T, int C, const float* __restrict__ w_, int w_raw,
                                                                        const float* __restrict__ u_, const float* __restrict__ k_,
                                                                        const float* __restrict__ v_, const float* __restrict__ gy_,
                                                                        States st, float* __restrict__ gw_, float* __restrict__ gu_,
-                                                                       i64 gstride, int accumulate, float* gk_, float* gv_) {
+                                                                       i64 gstride, int accumulate, float* gk_, float* gv_, int B,
+                                                                       float* sum_, unsigned* counters) {
     __shared__ ScanBuf<S> buf;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Place at = place(C, lane);
@@ -224,6 +227,20 @@ __global__ void __launch_bounds__(32 * S, 16 / S) wkv4_backward_kernel(int T, in
         if (accumulate) { gw += *pw; gu += *pu; }
         *pw = gw; *pu = gu;
     }
+    if (sum_ == nullptr || warp != 0) return;
+    const int group = blockIdx.x % ((C + 31) / 32);
+    __threadfence();
+    __syncwarp();
+    unsigned before = 0;
+    if (lane == 0) before = atomicAdd(counters + group, 1u);
+    if (__shfl_sync(0xffffffffu, before, 0) != (unsigned)(B - 1)) return;
+    __threadfence();
+    if (lane == 0) counters[group] = 0;
+    if (!at.live) return;
+    gw = 0.f; gu = 0.f;
+#pragma unroll 4
+    for (int b = 0; b < B; ++b) { gw += __ldcg(gw_ + b * gstride + at.c); gu += __ldcg(gu_ + b * gstride + at.c); }
+    sum_[at.c] = gw; sum_[C + at.c] = gu;
 }
 
 // S: the fewest blocks get the most warps (32 channel groups are a fifth of the SMs); with more groups than SMs short tiles,
@@ -237,12 +254,12 @@ int pick_segments(int B, int T, int C, int most) {
 i64 group_count(int B, int C) { return (i64)B * ((C + 31) / 32); }
 
 int forward(int B, int T, int C, const float* w, int w_raw, const float* u, const float* k, const float* v, float* y, States st,
-            cudaStream_t s) {
+            unsigned* counters, cudaStream_t s) {
     const unsigned grid = (unsigned)group_count(B, C);
 #define RWKV_GO(SEG)                                                                                                    \
     do {                                                                                                                \
-        if (y != nullptr) wkv4_forward_kernel<SEG, true><<<grid, 32 * SEG, 0, s>>>(T, C, w, w_raw, u, k, v, y, st);     \
-        else wkv4_forward_kernel<SEG, false><<<grid, 32 * SEG, 0, s>>>(T, C, w, w_raw, u, k, v, y, st);                 \
+        if (y != nullptr) wkv4_forward_kernel<SEG, true><<<grid, 32 * SEG, 0, s>>>(T, C, w, w_raw, u, k, v, y, st, counters); \
+        else wkv4_forward_kernel<SEG, false><<<grid, 32 * SEG, 0, s>>>(T, C, w, w_raw, u, k, v, y, st, counters); \
     } while (0)
     switch (pick_segments(B, T, C, 32)) {
         case 32: RWKV_GO(32); break;
@@ -254,18 +271,22 @@ int forward(int B, int T, int C, const float* w, int w_raw, const float* u, cons
 }
 
 int backward(int B, int T, int C, const float* w, int w_raw, const float* u, const float* k, const float* v, const float* gy, States st,
-             float* gw, float* gu, i64 gstride, int accumulate, float* gk, float* gv, cudaStream_t s) {
+             float* gw, float* gu, i64 gstride, int accumulate, float* gk, float* gv, float* sum, unsigned* counters, cudaStream_t s) {
     const unsigned grid = (unsigned)group_count(B, C);
     if (pick_segments(B, T, C, 16) == 16)
-        wkv4_backward_kernel<16><<<grid, 512, 0, s>>>(T, C, w, w_raw, u, k, v, gy, st, gw, gu, gstride, accumulate, gk, gv);
+        wkv4_backward_kernel<16><<<grid, 512, 0, s>>>(T, C, w, w_raw, u, k, v, gy, st, gw, gu, gstride, accumulate, gk, gv, B, sum, counters);
     else
-        wkv4_backward_kernel<8><<<grid, 256, 0, s>>>(T, C, w, w_raw, u, k, v, gy, st, gw, gu, gstride, accumulate, gk, gv);
+        wkv4_backward_kernel<8><<<grid, 256, 0, s>>>(T, C, w, w_raw, u, k, v, gy, st, gw, gu, gstride, accumulate, gk, gv, B, sum, counters);
     return check_launch("wkv4_backward");
 }
 
 States saved_states(float* p, int T, int C) {
     const i64 nseg = (T + L - 1) / L;
     return States{p, (nseg - 1) * 3 * C, 3 * (i64)C};
+}
+
+unsigned* saved_counters(void* p, int B, int T, int C) {   // behind the states
+    return static_cast<unsigned*>(p) + (size_t)B * ((T + L - 1) / L - 1) * 3 * C;
 }
 
 }  // namespace
@@ -284,7 +305,7 @@ extern "C" int rwkvb200_wkv4_forward(int B, int T, int C, const float* w, const 
                                      const float* v, float* y, void* stream) {
     if (int e = check_wkv4("wkv4_forward", B, T, C)) return e;
     RWKV_NOTNULL(w); RWKV_NOTNULL(u); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(y);
-    return forward(B, T, C, w, 0, u, k, v, y, States{nullptr, 0, 0}, as_stream(stream));
+    return forward(B, T, C, w, 0, u, k, v, y, States{nullptr, 0, 0}, nullptr, as_stream(stream));
 }
 
 extern "C" int rwkvb200_wkv4_backward(int B, int T, int C, const float* w, const float* u, const float* k,
@@ -297,20 +318,20 @@ extern "C" int rwkvb200_wkv4_backward(int B, int T, int C, const float* w, const
     // reverse pass reads a segment's state before it writes the gk of the one before.
     const States st = {gk, (i64)T * C, (i64)L * C};
     if (T > L)
-        if (int e = forward(B, T, C, w, 0, u, k, v, nullptr, st, as_stream(stream))) return e;
-    return backward(B, T, C, w, 0, u, k, v, gy, st, gw, gu, C, 1, gk, gv, as_stream(stream));
+        if (int e = forward(B, T, C, w, 0, u, k, v, nullptr, st, nullptr, as_stream(stream))) return e;
+    return backward(B, T, C, w, 0, u, k, v, gy, st, gw, gu, C, 1, gk, gv, nullptr, nullptr, as_stream(stream));
 }
 
 extern "C" size_t rwkvb200_wkv4_saved_bytes(int B, int T, int C) {
     if (B <= 0 || T <= 0 || C <= 0) return 0;
-    return ((size_t)B * ((T + L - 1) / L - 1) * 3 * C + 1) * sizeof(float);
+    return ((size_t)B * ((T + L - 1) / L - 1) * 3 * C + (C + 31) / 32) * sizeof(float);   // states, and a counter per channel group
 }
 
 extern "C" int rwkvb200_wkv4_train_forward(int B, int T, int C, const float* w_raw, const float* u, const float* k, const float* v,
                                            float* y, void* saved, void* stream) {
     if (int e = check_wkv4("wkv4_train_forward", B, T, C)) return e;
     RWKV_NOTNULL(w_raw); RWKV_NOTNULL(u); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(y); RWKV_NOTNULL(saved);
-    return forward(B, T, C, w_raw, 1, u, k, v, y, saved_states(static_cast<float*>(saved), T, C), as_stream(stream));
+    return forward(B, T, C, w_raw, 1, u, k, v, y, saved_states(static_cast<float*>(saved), T, C), saved_counters(saved, B, T, C), as_stream(stream));
 }
 
 extern "C" int rwkvb200_wkv4_train_backward(int B, int T, int C, const float* w_raw, const float* u, const float* k, const float* v,
@@ -322,6 +343,6 @@ extern "C" int rwkvb200_wkv4_train_backward(int B, int T, int C, const float* w_
     RWKV_REQUIRE(B == 1 || partial != nullptr, RWKVB200_ENULL, "wkv4_train_backward: partial is NULL");
     float* p = B == 1 ? gwu : partial;
     const States st = saved_states(static_cast<float*>(const_cast<void*>(saved)), T, C);
-    if (int e = backward(B, T, C, w_raw, 1, u, k, v, gy, st, p, p + C, 2 * (i64)C, 0, gk, gv, as_stream(stream))) return e;
-    return B == 1 ? RWKVB200_OK : rwkvb200_reduce_batch_partials(RWKVB200_F32, B, 2 * C, partial, gwu, stream);
+    return backward(B, T, C, w_raw, 1, u, k, v, gy, st, p, p + C, 2 * (i64)C, 0, gk, gv, B == 1 ? nullptr : gwu,
+                    saved_counters(const_cast<void*>(saved), B, T, C), as_stream(stream));
 }

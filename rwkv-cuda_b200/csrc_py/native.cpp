@@ -70,10 +70,29 @@ float* f32(void* p) { return static_cast<float*>(p); }
 // a tensor of the shape of `like` on the storage of `whole`, from element `offset` on (without a trip through the dispatcher)
 Tensor part(const Tensor& whole, int64_t offset, const Tensor& like) {
     Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(whole.storage()), whole.key_set(), whole.dtype());
-    t.unsafeGetTensorImpl()->set_storage_offset(offset);
+    t.unsafeGetTensorImpl()->set_storage_offset(whole.storage_offset() + offset);
     t.unsafeGetTensorImpl()->set_sizes_contiguous(like.sizes());
     return t;
 }
+
+// Several outputs at once: one allocation when they are small (an allocation costs about 1 us, as much as a tenth of a small
+// step), one each when keeping one of them alive would keep much memory alive.
+struct Outputs {
+    Tensor whole;
+    int64_t at = 0;
+    at::ScalarType d;
+    Outputs(int64_t elems, int count, at::ScalarType type, const Tensor& like) : d(type) {
+        if (elems * (int64_t)c10::elementSize(type) <= (1 << 20)) whole = empty({elems + 16 * count}, type, like);
+    }
+    Tensor next(at::IntArrayRef sizes, const Tensor& like) {
+        if (!whole.defined()) return empty(sizes, d, like);
+        Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(whole.storage()), whole.key_set(), whole.dtype());
+        t.unsafeGetTensorImpl()->set_storage_offset(at);
+        t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+        at += (t.numel() + 15) / 16 * 16;   // 32-byte aligned
+        return t;
+    }
+};
 
 // ---- autograd -------------------------------------------------------------------------------------------------
 // One node type for all operators (a node of its own instead of torch::autograd::Function, whose context, argument unpacking
@@ -168,8 +187,10 @@ static variable_list wkv4_backward(const Saved& s, const variable_list& g) {
     const auto f = at::kFloat;
     const Tensor& gy = g[0];
     numel(gy, B * T * C, "gy");
-    Tensor gwu = empty({2, C}, f, gy), gk = empty({B, T, C}, f, gy), gv = empty({B, T, C}, f, gy);
-    const Tensor partial = B > 1 ? empty({B, 2, C}, f, gy) : Tensor();
+    const int64_t n = B * T * C;
+    Outputs o(2 * n + 2 * C + 2 * B * C, 4, f, gy);
+    Tensor gk = o.next({B, T, C}, gy), gv = o.next({B, T, C}, gy), gwu = o.next({2, C}, gy);
+    const Tensor partial = B > 1 ? o.next({B, 2, C}, gy) : Tensor();
     check_rc(rwkvb200_wkv4_train_backward(B, T, C, f32(s.in[0].data_ptr()), f32(s.in[1].data_ptr()), f32(s.in[2].data_ptr()),
                                           f32(s.in[3].data_ptr()), f32(ptr(gy, "gy", f)), s.own[0].data_ptr(), f32(gwu.data_ptr()),
                                           partial.defined() ? f32(partial.data_ptr()) : nullptr, f32(gk.data_ptr()), f32(gv.data_ptr()), stream()),
@@ -198,7 +219,8 @@ static variable_list timex_backward(const Saved& s, const variable_list& g) {
     const auto f = at::kFloat;
     const Tensor& gx = g[0];
     numel(gx, B * C * T, "gwk");
-    Tensor gw = empty({C, T}, f, gx), gk = empty({B, C, T}, f, gx);
+    Outputs o(C * T + B * C * T, 2, f, gx);
+    Tensor gw = o.next({C, T}, gx), gk = o.next({B, C, T}, gx);
     const size_t nbytes = rwkvb200_timex_work_bytes(B, C, T);
     const Tensor work = nbytes ? bytes(nbytes, gx) : Tensor();
     check_rc(rwkvb200_timex_train_backward(f32(s.in[0].data_ptr()), f32(s.in[1].data_ptr()), f32(ptr(gx, "gwk", f)), f32(gw.data_ptr()),
@@ -226,7 +248,8 @@ static variable_list wkv5_backward(const Saved& s, const variable_list& g) {
     const auto d = s.in[0].scalar_type();
     const Tensor& gy = g[0];
     numel(gy, B * T * C, "gy");
-    Tensor gr = empty({B, T, C}, d, gy), gk = empty({B, T, C}, d, gy), gv = empty({B, T, C}, d, gy), gwu = empty({2, C}, d, gy);
+    Outputs o(3 * B * T * C + 2 * C, 4, d, gy);
+    Tensor gr = o.next({B, T, C}, gy), gk = o.next({B, T, C}, gy), gv = o.next({B, T, C}, gy), gwu = o.next({2, C}, gy);
     const Tensor work = bytes(rwkvb200_wkv5_train_work_bytes(B, T, C, H, path), gy);
     check_rc(rwkvb200_wkv5_train_backward(dt(s.in[0], "r"), B, T, C, H, path, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
                                           s.in[3].data_ptr(), s.in[4].data_ptr(), ptr(gy, "gy", d), gr.data_ptr(), gk.data_ptr(), gv.data_ptr(),
@@ -259,8 +282,9 @@ static variable_list wkv6_backward(const Saved& s, const variable_list& g) {
     const auto d = s.in[0].scalar_type(), f = at::kFloat;
     const Tensor& gy = g[0];
     numel(gy, B * T * C, "gy");
-    Tensor gr = empty({B, T, C}, d, gy), gk = empty({B, T, C}, d, gy), gv = empty({B, T, C}, d, gy), gw = empty({B, T, C}, d, gy);
-    Tensor gu = empty(s.in[4].sizes(), d, gy), ds0 = state ? same(s.in[5]) : Tensor();
+    Outputs o(4 * B * T * C + C, 5, d, gy);
+    Tensor gr = o.next({B, T, C}, gy), gk = o.next({B, T, C}, gy), gv = o.next({B, T, C}, gy), gw = o.next({B, T, C}, gy);
+    Tensor gu = o.next(s.in[4].sizes(), gy), ds0 = state ? same(s.in[5]) : Tensor();
     const Tensor work = bytes(rwkvb200_wkv6_train_work_bytes(B, T, C, path), gy);
     check_rc(rwkvb200_wkv6_train_backward(dt(s.in[0], "r"), B, T, C, H, path, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
                                           s.in[3].data_ptr(), s.in[4].data_ptr(), state ? f32(s.in[5].data_ptr()) : nullptr, ptr(gy, "gy", d),
@@ -305,7 +329,8 @@ static variable_list wkv7_backward(const Saved& s, const variable_list& g) {
     const auto d = s.in[0].scalar_type(), f = at::kFloat;
     if (sT && g[1].scalar_type() != f) raise(PyExc_AssertionError, "dsT must be float32", true);
     std::array<Tensor, 6> x;
-    for (auto& t : x) t = empty({B, T, H, N}, d, g[0]);
+    Outputs o(6 * B * T * H * N, 6, d, g[0]);
+    for (auto& t : x) t = o.next({B, T, H, N}, g[0]);
     Tensor ds0 = s0 ? empty({B, H, N, N}, f, g[0]) : Tensor();
     check_rc(rwkvb200_wkv7_backward(dt(s.in[0], "r"), B, T, H, N, kChunkLen, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
                                     s.in[3].data_ptr(), s.in[4].data_ptr(), s.in[5].data_ptr(), ptr(g[0], "dy", d),
@@ -329,7 +354,10 @@ static std::tuple<Tensor, Tensor> wkv7_forward(const Tensor* s0, const Tensor& r
     const int dtype = dt(r, "r");
     const int64_t B = r.size(0), T = r.size(1), H = r.size(2), N = r.size(3);
     Tensor y = passing ? empty({B, T, H * N}, d, r) : same(v), sT = passing ? same(*s0) : Tensor();
-    Saved s{{r, w, k, v, a, b}, {empty({B, H, T / kChunkLen, N, N}, f, r), empty({B, T, H, N}, f, r)}, {B, T, H, N, s0 != nullptr, passing}};
+    Saved s{{r, w, k, v, a, b}, {}, {B, T, H, N, s0 != nullptr, passing}};
+    Outputs o(B * H * (T / kChunkLen) * N * N + B * T * H * N, 2, f, r);
+    s.own[0] = o.next({B, H, T / kChunkLen, N, N}, r);
+    s.own[1] = o.next({B, T, H, N}, r);
     check_rc(rwkvb200_wkv7_forward(dtype, B, T, H, N, kChunkLen, s0 ? f32(ptr(*s0, "s0", f)) : nullptr, ptr(r, "r", d), ptr(w, "w", d),
                                    ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
                                    passing ? f32(sT.data_ptr()) : nullptr, f32(s.own[0].data_ptr()), f32(s.own[1].data_ptr()), stream()),
