@@ -300,6 +300,21 @@ int rwkvb200_wkv7_backward(int dtype, int B, int T, int H, int N, int chunk_len,
                            const float* sa, float* ds0, void* dr, void* dw, void* dk, void* dv,
                            void* da, void* db, void* stream);
 
+/* Training flow with buffers of the library's own: rwkvb200_wkv7_train_path picks the kernels for a shape (0: those of
+ * rwkvb200_wkv7_forward / _backward; 1: the chunks of a sequence in parallel, for launches with few (batch, head) units) and
+ * the other calls are told it; `saved` is kept from the forward to the backward, `work` (may be NULL when its size is 0) is
+ * free after each call.  s0, sT, dsT, ds0 may be NULL as above. */
+int rwkvb200_wkv7_train_path(int dtype, int B, int T, int H, int N);
+size_t rwkvb200_wkv7_train_saved_bytes(int B, int T, int H, int N, int path);
+size_t rwkvb200_wkv7_train_work_bytes(int B, int T, int H, int path, int backward);
+int rwkvb200_wkv7_train_forward(int dtype, int B, int T, int H, int N, int path, const float* s0, const void* r,
+                                const void* w, const void* k, const void* v, const void* a, const void* b, void* y,
+                                float* sT, void* saved, void* work, void* stream);
+int rwkvb200_wkv7_train_backward(int dtype, int B, int T, int H, int N, int path, const void* r, const void* w,
+                                 const void* k, const void* v, const void* a, const void* b, const void* dy,
+                                 const float* dsT, const void* saved, void* work, float* ds0, void* dr, void* dw,
+                                 void* dk, void* dv, void* da, void* db, void* stream);
+
 /* Inference-shaped RWKV-7 entry point: advances `state` (B,H,N,N) fp32, indexed [value i][key j] as the
  * reference's s0 / sT (rwkv7_fast_fused/cuda/rwkv7_statepassing_clampw.cu:26-32, 78-80), by T >= 1 tokens
  * IN PLACE and writes y (B,T,H,N).  Nothing is saved for a backward pass and T needs no alignment: T = 1
@@ -327,7 +342,8 @@ int rwkvb200_wkv7_select_form(int form);
 /* Synchronous read of the current device's sticky status word: 0, or 10 + n / 20 + n when the n-th
  * bounded wait of the tensor-core forward / backward ran out in some thread block (30.. / 40..: the
  * front / back warp group of the two-stage backward, 50.. / 55.. / 60..: loader / matrix / chain group of the
- * staged forward; 70.. / 75.. / 80..: the same groups of the staged RWKV-6 / RWKV-5 forward; 91..: their tcgen05 backward) (the outputs of
+ * staged forward; 70.. / 75.. / 80..: the same groups of the staged RWKV-6 / RWKV-5 forward; 91..: their tcgen05 backward;
+ * 101..: the RWKV-7 kernels with the chunks in parallel) (the outputs of
  * that call are then invalid); negative on a CUDA error.  Per device; stays set until cleared. */
 int rwkvb200_device_status(void);
 /* Resets the current device's status word.  No counterpart in the reference. */

@@ -4,6 +4,7 @@
 #include "wkv7_dispatch.cuh"
 #include "wkv6_chunked.cuh"
 #include <atomic>
+#include <stdlib.h>
 #include <initializer_list>
 
 namespace rwkvb200 {
@@ -123,7 +124,8 @@ extern "C" int rwkvb200_device_status(void) {
         return RWKVB200_ECUDA;
     }
     const int p = wkv7_l32_bwdp_error(0), q = wkv7_l32_fwdp_error(0), r6 = wkv6_l32_error(0), b6 = wkv6_l32_bwd_error(0);
-    if (p < 0 || q < 0 || r6 < 0 || b6 < 0) {
+    const int v7s = wkv7_scan_error(0);
+    if (p < 0 || q < 0 || r6 < 0 || b6 < 0 || v7s < 0) {
         set_error("device_status: reading the status words failed");
         return RWKVB200_ECUDA;
     }
@@ -132,11 +134,12 @@ extern "C" int rwkvb200_device_status(void) {
     if (p) return p;            // the two-stage backward records 30.. (front group) or 40.. (back group)
     if (q) return q + 20;       // the staged RWKV-7 forward 50.. / 55.. / 60..
     if (r6) return r6 + 40;     // the staged RWKV-6 / RWKV-5 forward 70.. / 75.. / 80..
-    return b6 ? b6 + 90 : 0;    // the tcgen05 RWKV-6 / RWKV-5 backward 91..
+    if (b6) return b6 + 90;     // the tcgen05 RWKV-6 / RWKV-5 backward 91..
+    return v7s ? v7s + 100 : 0; // the RWKV-7 kernels with the chunks in parallel 101..
 }
 
 extern "C" int rwkvb200_device_status_clear(void) {
-    RWKV_REQUIRE(wkv7_l32_clear_errors() == 0 && wkv7_l32_bwdp_error(1) == 0 && wkv7_l32_fwdp_error(1) == 0 && wkv6_l32_error(1) == 0 && wkv6_l32_bwd_error(1) == 0, RWKVB200_ECUDA, "device_status_clear: writing the status words failed");
+    RWKV_REQUIRE(wkv7_l32_clear_errors() == 0 && wkv7_l32_bwdp_error(1) == 0 && wkv7_l32_fwdp_error(1) == 0 && wkv6_l32_error(1) == 0 && wkv6_l32_bwd_error(1) == 0 && wkv7_scan_error(1) == 0, RWKVB200_ECUDA, "device_status_clear: writing the status words failed");
     return RWKVB200_OK;
 }
 
@@ -211,4 +214,54 @@ extern "C" int rwkvb200_wkv7_state_update(int dtype, int B, int T, int H, int N,
     if (N == 64 && aligned16({state, r, w, k, v, a, b, y}))
         return wkv7_update64(dtype, B, T, H, state, r, w, k, v, a, b, y, sm_count(), as_stream(stream));
     return wkv7_generic_forward(dtype, B, T, H, N, T, state, r, w, k, v, a, b, y, state, nullptr, nullptr, as_stream(stream));
+}
+
+// ---- training flow ------------------------------------------------------------------------------------------------------
+// Path 1: the chunks in parallel (wkv7_scan.cu), for tensor-core shapes with few units.  Path 0: rwkvb200_wkv7_forward /
+// _backward, `saved` = s then sa.
+extern "C" int rwkvb200_wkv7_train_path(int dtype, int B, int T, int H, int N) {
+    static const int lim = getenv("V7_SCAN") ? atoi(getenv("V7_SCAN")) : 64;
+    const bool tensor = dtype == RWKVB200_BF16 && N == 64 && g_wkv7_path.load() != 1 && g_wkv7_bwd_form.load() == 0 && !g_no_tensor_maps.load();
+    return tensor && T > 64 && (long long)B * H <= lim && B <= 65535 ? 1 : 0;
+}
+extern "C" size_t rwkvb200_wkv7_train_saved_bytes(int B, int T, int H, int N, int path) {
+    if (B <= 0 || T <= 0 || H <= 0 || N <= 0) return 0;
+    if (path == 1) return wkv7_scan_saved_bytes(B, T, H);
+    return ((size_t)B * H * (T / 16) * N * N + (size_t)B * T * H * N) * sizeof(float);
+}
+extern "C" size_t rwkvb200_wkv7_train_work_bytes(int B, int T, int H, int path, int backward) {
+    return path == 1 && B > 0 && T > 0 && H > 0 ? wkv7_scan_work_bytes(B, T, H, backward != 0) : 0;
+}
+extern "C" int rwkvb200_wkv7_train_forward(int dtype, int B, int T, int H, int N, int path, const float* s0, const void* r, const void* w,
+                                           const void* k, const void* v, const void* a, const void* b, void* y, float* sT, void* saved,
+                                           void* work, void* stream) {
+    if (int e = wkv7_check("wkv7_train_forward", dtype, B, T, H, N, 16)) return e;
+    RWKV_NOTNULL(saved);
+    if (path == 0) {
+        float* s = static_cast<float*>(saved);
+        return rwkvb200_wkv7_forward(dtype, B, T, H, N, 16, s0, r, w, k, v, a, b, y, sT, s, s + (size_t)B * H * (T / 16) * N * N, stream);
+    }
+    RWKV_NOTNULL(r); RWKV_NOTNULL(w); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(a); RWKV_NOTNULL(b); RWKV_NOTNULL(y); RWKV_NOTNULL(work);
+    RWKV_REQUIRE(dtype == RWKVB200_BF16 && N == 64, RWKVB200_EINVAL, "wkv7_train_forward: path 1 is bf16, head size 64");
+    RWKV_REQUIRE(aligned16({s0, r, w, k, v, a, b, y, sT, saved, work}), RWKVB200_EALIGN, "wkv7_train_forward: the bf16 N=64 path needs 16-byte aligned tensors");
+    const int rc = wkv7_scan_forward(B, T, H, s0, r, w, k, v, a, b, y, sT, saved, work, as_stream(stream));
+    RWKV_REQUIRE(rc != 1, RWKVB200_EUNSUPPORTED, "wkv7_train_forward: tensor maps cannot be made here");
+    return rc;
+}
+extern "C" int rwkvb200_wkv7_train_backward(int dtype, int B, int T, int H, int N, int path, const void* r, const void* w, const void* k,
+                                            const void* v, const void* a, const void* b, const void* dy, const float* dsT, const void* saved,
+                                            void* work, float* ds0, void* dr, void* dw, void* dk, void* dv, void* da, void* db, void* stream) {
+    if (int e = wkv7_check("wkv7_train_backward", dtype, B, T, H, N, 16)) return e;
+    RWKV_NOTNULL(saved);
+    if (path == 0) {
+        const float* s = static_cast<const float*>(saved);
+        return rwkvb200_wkv7_backward(dtype, B, T, H, N, 16, r, w, k, v, a, b, dy, dsT, s, s + (size_t)B * H * (T / 16) * N * N, ds0, dr, dw, dk,
+                                      dv, da, db, stream);
+    }
+    RWKV_NOTNULL(r); RWKV_NOTNULL(w); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(a); RWKV_NOTNULL(b); RWKV_NOTNULL(dy); RWKV_NOTNULL(work);
+    RWKV_NOTNULL(dr); RWKV_NOTNULL(dw); RWKV_NOTNULL(dk); RWKV_NOTNULL(dv); RWKV_NOTNULL(da); RWKV_NOTNULL(db);
+    RWKV_REQUIRE(dtype == RWKVB200_BF16 && N == 64, RWKVB200_EINVAL, "wkv7_train_backward: path 1 is bf16, head size 64");
+    RWKV_REQUIRE(aligned16({r, w, k, v, a, b, dy, dsT, saved, work, ds0, dr, dw, dk, dv, da, db}), RWKVB200_EALIGN,
+                 "wkv7_train_backward: the bf16 N=64 path needs 16-byte aligned tensors");
+    return wkv7_scan_backward(B, T, H, r, w, k, v, a, b, dy, dsT, saved, work, ds0, dr, dw, dk, dv, da, db, as_stream(stream));
 }

@@ -26,6 +26,21 @@ int wkv7_l32_forward(int B, int T, int H, const float* s0, const void* r, const 
 int wkv7_l32_backward(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
                       const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
                       void* dk, void* dv, void* da, void* db, cudaStream_t st);
+// The same kernel with one block per chunk: adj = the adjoint at the end, states = the state at the start of every chunk,
+// both (B,H,ceil(T/32),64,64) fp32 (wkv7_scan.cu).
+int wkv7_l32_backward_chunks(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
+                             const void* b, const void* dy, const float* adj, const float* states, void* dr, void* dw,
+                             void* dk, void* dv, void* da, void* db, cudaStream_t st);
+// Training with the chunks in parallel (wkv7_scan.cu), for launches with few units.  The forward returns 1 when tensor maps
+// cannot be made.  saved / work: the sizes below.
+size_t wkv7_scan_saved_bytes(int B, int T, int H);
+size_t wkv7_scan_work_bytes(int B, int T, int H, bool backward);
+int wkv7_scan_forward(int B, int T, int H, const float* s0, const void* r, const void* w, const void* k, const void* v, const void* a,
+                      const void* b, void* y, float* sT, void* saved, void* work, cudaStream_t st);
+int wkv7_scan_backward(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                       const void* dy, const float* dsT, const void* saved, void* work, float* ds0, void* dr, void* dw, void* dk, void* dv,
+                       void* da, void* db, cudaStream_t st);
+int wkv7_scan_error(int clear);
 // The backward as two warp groups working on consecutive chunks (one thread block per SM; same
 // products, results equal to rounding); for launches with at most one unit per SM.  Error word: read (clear = 0) or reset (clear = 1).
 int wkv7_l32_backward_pipelined(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,

@@ -16,6 +16,9 @@
 //   dL/dlog d_t = A0 - sum_{tau<t} c_tau - a~_t dA'_t
 // anchored afresh at every chunk so rounding does not accumulate along the sequence.
 //
+// With `adj_` (the adjoint at the end of every chunk, from wkv7_scan.cu) a block does the one chunk blockIdx.z, and the states in
+// ck_ follow each other chunk by chunk.
+//
 // One CTA of 8 warps per (batch, head), two CTAs per SM.  Warp w works on quarter w%4 of tensor memory
 // (16 rows) and, where a region is split, on token half w/4.  Shared memory: six [64][64] operand
 // arrays (each read K-major and MN-major as needed), P reusing the space of the U matrices.
@@ -96,7 +99,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                       const bf16* __restrict__ b_, const bf16* __restrict__ dy_, const float* __restrict__ dsT_,
                       const float* __restrict__ ck_, float* __restrict__ ds0_, bf16* __restrict__ dr_,
                       bf16* __restrict__ dw_, bf16* __restrict__ dk_, bf16* __restrict__ dv_, bf16* __restrict__ da_,
-                      bf16* __restrict__ db_, const __grid_constant__ TileMaps<7> maps) {
+                      bf16* __restrict__ db_, const float* __restrict__ adj_, const __grid_constant__ TileMaps<7> maps) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // the swizzle acts on address bits
     unsigned char *AR = smem + BwdSmemX::kAR, *BK = smem + BwdSmemX::kBK, *SV = smem + BwdSmemX::kSV, *EY = smem + BwdSmemX::kEY;
@@ -121,7 +124,9 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     const i64 tok0 = (i64)bb * T * C + hh * 64;
     const i64 sbase = (i64)(bb * H + hh) * 64 * 64;
     const int nchunks = (T + LC - 1) / LC;
-    const float* ck = ck_ + (i64)(bb * H + hh) * (T / 16) * 64 * 64;   // block [b][h] of the caller's (B,H,T/16,N,N) buffer
+    const int c_hi = adj_ ? blockIdx.z : nchunks - 1, c_lo = adj_ ? blockIdx.z : 0;
+    const float* ck = ck_ + (i64)(bb * H + hh) * (adj_ ? nchunks : T / 16) * 64 * 64;   // block [b][h] of the caller's (B,H,T/16,N,N) buffer
+    const float* E0 = adj_ ? adj_ + ((i64)(bb * H + hh) * nchunks + c_hi) * 64 * 64 : dsT_ ? dsT_ + sbase : nullptr;
     const bf16* src[7] = {r_, w_, k_, v_, a_, b_, dy_};
 
     if (tid == 0) {
@@ -143,7 +148,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     const uint32_t arA = smem_u32(AR), bkA = smem_u32(BK), svA = smem_u32(SV), eyA = smem_u32(EY), s0A = smem_u32(S0);
     const uint32_t uakA = smem_u32(Uak), ubrA = smem_u32(Ubr), ukrA = smem_u32(Ukr), d0A = smem_u32(D0), n1A = smem_u32(N1), pA = smem_u32(Pm);
 
-    // E, ET <- dsT (or zero); this warp: its 16 rows, columns 32*hs .. 32*hs+31
+    // E, ET <- the adjoint at the end (or zero); this warp: its 16 rows, columns 32*hs .. 32*hs+31
     {
         float Ed[4][4], Td[4][4];
 #pragma unroll
@@ -151,8 +156,8 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int row = row0 + g + ((e & 2) ? 8 : 0), col = 32 * hs + nt * 8 + 2 * t + (e & 1);
-                Ed[nt][e] = dsT_ ? dsT_[sbase + row * 64 + col] : 0.f;
-                Td[nt][e] = dsT_ ? dsT_[sbase + col * 64 + row] : 0.f;
+                Ed[nt][e] = E0 ? E0[row * 64 + col] : 0.f;
+                Td[nt][e] = E0 ? E0[col * 64 + row] : 0.f;
             }
         tmem_st_tiles<4>(tmE + 32 * hs + lane_off, Ed);
         tmem_st_tiles<4>(tmET + 32 * hs + lane_off, Td);
@@ -199,15 +204,15 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             for (int q = 0; q < BTPW; ++q)
                 raw.x[x][q] = (t0 + q < T) ? *reinterpret_cast<const uint32_t*>(Raw + x * 4096 + (BTPW * warp + q) * 128 + lane * 4) : 0u;
     };
-    if (staged) { request(nchunks - 1); pending = true; }
-    else fetch_chunk<7, BTPW>(raw, src, tok0, C, nchunks - 1, T, warp, lane);
-    if (nchunks > 1) ask_l2(nchunks - 2);
+    if (staged) { request(c_hi); pending = true; }
+    else fetch_chunk<7, BTPW>(raw, src, tok0, C, c_hi, T, warp, lane);
+    if (c_hi > c_lo) ask_l2(c_hi - 1);
     int fail = 0;
     uint32_t par = 0;
     ChainSync cs{bar + 6, 0, 0};   // used by warp 0 only
 
     WKV7_PHASE_BEGIN();
-    for (int c = nchunks - 1; c >= 0; --c, par ^= 1) {
+    for (int c = c_hi; c >= c_lo; --c, par ^= 1) {
         const int valid = min(LC, T - c * LC);
         tc_fence_before();
         if (__syncthreads_or(fail)) break;
@@ -289,8 +294,8 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             tmem_st_tiles<4>(tmET + 32 * hs + lane_off, Td);
             tmem_wait_st();
         }
-        if (c > 0 && !staged) fetch_chunk<7, BTPW>(raw, src, tok0, C, c - 1, T, warp, lane);   // under the chain
-        if (c > 1) ask_l2(c - 2);
+        if (c > c_lo && !staged) fetch_chunk<7, BTPW>(raw, src, tok0, C, c - 1, T, warp, lane);   // under the chain
+        if (c > c_lo + 1) ask_l2(c - 2);
         WKV7_PHASE(5);   // issue of the forward part, decay scaling of E, request of the next chunk
         if (!mbar_wait(bar + 1, par)) fail = 2;
         tc_fence_after();
@@ -493,7 +498,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
         }
         __syncthreads();
         // every product that reads EY or S0 has completed and every thread has taken its anchor from S0
-        if (staged && c > 0) { request(c - 1); pending = true; }
+        if (staged && c > c_lo) { request(c - 1); pending = true; }
         WKV7_PHASE(13);  // epilogue part 1
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -530,7 +535,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     if (pending) mbar_wait(bar + 7, par);   // leaving early: the requested tiles must have landed before the block may end
     if (fail && tid == 0) {   // a wait ran out: record it and poison this unit's outputs so that they cannot pass as results
         atomicMax(&g_l32_bwd_error, fail);
-        dr_[tok0] = __ushort_as_bfloat16((unsigned short)0x7fc0);
+        dr_[tok0 + (i64)c_lo * LC * C] = __ushort_as_bfloat16((unsigned short)0x7fc0);
     }
     tc_fence_before();
     __syncthreads();
@@ -554,21 +559,32 @@ WKV7_PHASE_READER(rwkvb200_phase_clocks_l32_bwd)
 
 }  // namespace v7x
 
-int wkv7_l32_backward(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
-                      const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
-                      void* dk, void* dv, void* da, void* db, cudaStream_t st) {
+static int launch_l32_backward(int B, int T, int H, int chunks, const void* r, const void* w, const void* k, const void* v, const void* a,
+                               const void* b, const void* dy, const float* dsT, const float* adj, const float* s, float* ds0, void* dr,
+                               void* dw, void* dk, void* dv, void* da, void* db, cudaStream_t st) {
     using namespace v7x;
     cudaError_t e = allow_smem<wkv7x_backward_kernel>(BwdSmemX::kBytes);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv7_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     TileMaps<7> maps;
     const void* in[7] = {r, w, k, v, a, b, dy};
     make_tile_maps<7>(maps, in, B, T, H);
-    dim3 grid(H, B);
-    wkv7x_backward_kernel<<<grid, BNT, BwdSmemX::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)w, (const bf16*)k,
-                                                               (const bf16*)v, (const bf16*)a, (const bf16*)b, (const bf16*)dy,
-                                                               dsT, s, ds0, (bf16*)dr, (bf16*)dw, (bf16*)dk, (bf16*)dv,
-                                                               (bf16*)da, (bf16*)db, maps);
+    wkv7x_backward_kernel<<<dim3(H, B, chunks), BNT, BwdSmemX::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)w, (const bf16*)k,
+                                                                             (const bf16*)v, (const bf16*)a, (const bf16*)b,
+                                                                             (const bf16*)dy, dsT, s, ds0, (bf16*)dr, (bf16*)dw, (bf16*)dk,
+                                                                             (bf16*)dv, (bf16*)da, (bf16*)db, adj, maps);
     return check_launch("wkv7_backward(tcgen05, 32-token chunks)");
+}
+
+int wkv7_l32_backward(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
+                      const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
+                      void* dk, void* dv, void* da, void* db, cudaStream_t st) {
+    return launch_l32_backward(B, T, H, 1, r, w, k, v, a, b, dy, dsT, nullptr, s, ds0, dr, dw, dk, dv, da, db, st);
+}
+
+int wkv7_l32_backward_chunks(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
+                             const void* b, const void* dy, const float* adj, const float* states, void* dr, void* dw,
+                             void* dk, void* dv, void* da, void* db, cudaStream_t st) {
+    return launch_l32_backward(B, T, H, (T + v7x::LC - 1) / v7x::LC, r, w, k, v, a, b, dy, nullptr, adj, states, nullptr, dr, dw, dk, dv, da, db, st);
 }
 
 int wkv7_l32_bwd_error_clear() {

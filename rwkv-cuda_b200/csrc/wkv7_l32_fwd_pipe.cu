@@ -409,9 +409,13 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols) {
     const cuuint64_t strides[1] = {cols * 2};
     const cuuint32_t box[2] = {64, 32};
     const cuuint32_t elem[2] = {1, 1};
-    return encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    auto encode = [&] {
+        return encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    // (a thread that has made no runtime call yet has no context, which this driver call wants)
+    return encode() || (cudaFree(nullptr) == cudaSuccess && encode());
 }
 }  // namespace
 

@@ -324,7 +324,8 @@ static std::tuple<Tensor, Tensor> wkv6_forward(int64_t B, int64_t T, int64_t C, 
 constexpr int64_t kChunkLen = 16;
 
 static variable_list wkv7_backward(const Saved& s, const variable_list& g) {
-    const auto [B, T, H, N, s0, sT] = s.dims;
+    const auto [B, T, H, N, form, path] = s.dims;
+    const bool s0 = form & 1, sT = form & 2;
     const c10::cuda::CUDAGuard guard(s.in[0].device());
     const auto d = s.in[0].scalar_type(), f = at::kFloat;
     if (sT && g[1].scalar_type() != f) raise(PyExc_AssertionError, "dsT must be float32", true);
@@ -332,12 +333,14 @@ static variable_list wkv7_backward(const Saved& s, const variable_list& g) {
     Outputs o(6 * B * T * H * N, 6, d, g[0]);
     for (auto& t : x) t = o.next({B, T, H, N}, g[0]);
     Tensor ds0 = s0 ? empty({B, H, N, N}, f, g[0]) : Tensor();
-    check_rc(rwkvb200_wkv7_backward(dt(s.in[0], "r"), B, T, H, N, kChunkLen, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
-                                    s.in[3].data_ptr(), s.in[4].data_ptr(), s.in[5].data_ptr(), ptr(g[0], "dy", d),
-                                    sT ? f32(ptr(g[1], "dsT", f)) : nullptr, f32(s.own[0].data_ptr()), f32(s.own[1].data_ptr()),
-                                    s0 ? f32(ds0.data_ptr()) : nullptr, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), x[3].data_ptr(),
-                                    x[4].data_ptr(), x[5].data_ptr(), stream()),
-             "rwkvb200_wkv7_backward", true);
+    const size_t nwork = rwkvb200_wkv7_train_work_bytes(B, T, H, path, 1);
+    const Tensor work = nwork ? bytes(nwork, g[0]) : Tensor();
+    check_rc(rwkvb200_wkv7_train_backward(dt(s.in[0], "r"), B, T, H, N, path, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
+                                          s.in[3].data_ptr(), s.in[4].data_ptr(), s.in[5].data_ptr(), ptr(g[0], "dy", d),
+                                          sT ? f32(ptr(g[1], "dsT", f)) : nullptr, s.own[0].data_ptr(), nwork ? work.data_ptr() : nullptr,
+                                          s0 ? f32(ds0.data_ptr()) : nullptr, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), x[3].data_ptr(),
+                                          x[4].data_ptr(), x[5].data_ptr(), stream()),
+             "rwkvb200_wkv7_train_backward", true);
     variable_list out{std::move(x[0]), std::move(x[1]), std::move(x[2]), std::move(x[3]), std::move(x[4]), std::move(x[5])};
     if (s0) out.push_back(std::move(ds0));
     return out;
@@ -353,15 +356,15 @@ static std::tuple<Tensor, Tensor> wkv7_forward(const Tensor* s0, const Tensor& r
     const auto d = r.scalar_type(), f = at::kFloat;
     const int dtype = dt(r, "r");
     const int64_t B = r.size(0), T = r.size(1), H = r.size(2), N = r.size(3);
+    const int path = rwkvb200_wkv7_train_path(dtype, B, T, H, N);
     Tensor y = passing ? empty({B, T, H * N}, d, r) : same(v), sT = passing ? same(*s0) : Tensor();
-    Saved s{{r, w, k, v, a, b}, {}, {B, T, H, N, s0 != nullptr, passing}};
-    Outputs o(B * H * (T / kChunkLen) * N * N + B * T * H * N, 2, f, r);
-    s.own[0] = o.next({B, H, T / kChunkLen, N, N}, r);
-    s.own[1] = o.next({B, T, H, N}, r);
-    check_rc(rwkvb200_wkv7_forward(dtype, B, T, H, N, kChunkLen, s0 ? f32(ptr(*s0, "s0", f)) : nullptr, ptr(r, "r", d), ptr(w, "w", d),
-                                   ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
-                                   passing ? f32(sT.data_ptr()) : nullptr, f32(s.own[0].data_ptr()), f32(s.own[1].data_ptr()), stream()),
-             "rwkvb200_wkv7_forward");
+    Saved s{{r, w, k, v, a, b}, {bytes(rwkvb200_wkv7_train_saved_bytes(B, T, H, N, path), r)}, {B, T, H, N, (s0 ? 1 : 0) + (passing ? 2 : 0), path}};
+    const size_t nwork = rwkvb200_wkv7_train_work_bytes(B, T, H, path, 0);
+    const Tensor work = nwork ? bytes(nwork, r) : Tensor();
+    check_rc(rwkvb200_wkv7_train_forward(dtype, B, T, H, N, path, s0 ? f32(ptr(*s0, "s0", f)) : nullptr, ptr(r, "r", d), ptr(w, "w", d),
+                                         ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
+                                         passing ? f32(sT.data_ptr()) : nullptr, s.own[0].data_ptr(), nwork ? work.data_ptr() : nullptr, stream()),
+             "rwkvb200_wkv7_train_forward");
     if (s0) s.in[6] = *s0;
     const char* op = passing ? "RWKV7_STATE_PASSING_CLAMPW_CUDA_OP" : s0 ? "RWKV7_STATE_CLAMPW_CUDA_OP" : "RWKV7_CLAMPW_CUDA_OP";
     if (passing) record(op, wkv7_backward, {r, w, k, v, a, b, *s0}, std::move(s), {y, sT});
