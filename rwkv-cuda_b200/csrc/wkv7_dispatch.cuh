@@ -26,7 +26,7 @@ int wkv7_l32_forward(int B, int T, int H, const float* s0, const void* r, const 
 int wkv7_l32_backward(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
                       const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
                       void* dk, void* dv, void* da, void* db, cudaStream_t st);
-// The same kernel with one block per chunk: adj = the adjoint at the end, states = the state at the start of every chunk,
+// The same kernel with a block per few chunks: adj = the adjoint at the end, states = the state at the start of every chunk,
 // both (B,H,ceil(T/32),64,64) fp32 (wkv7_scan.cu).
 int wkv7_l32_backward_chunks(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
                              const void* b, const void* dy, const float* adj, const float* states, void* dr, void* dw,

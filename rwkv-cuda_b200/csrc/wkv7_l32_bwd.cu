@@ -16,8 +16,8 @@
 //   dL/dlog d_t = A0 - sum_{tau<t} c_tau - a~_t dA'_t
 // anchored afresh at every chunk so rounding does not accumulate along the sequence.
 //
-// With `adj_` (the adjoint at the end of every chunk, from wkv7_scan.cu) a block does the one chunk blockIdx.z, and the states in
-// ck_ follow each other chunk by chunk.
+// With `adj_` (the adjoint at the end of every chunk, from wkv7_scan.cu) a block does `group` chunks, the blockIdx.z-th such group,
+// and the states in ck_ follow each other chunk by chunk.
 //
 // One CTA of 8 warps per (batch, head), two CTAs per SM.  Warp w works on quarter w%4 of tensor memory
 // (16 rows) and, where a region is split, on token half w/4.  Shared memory: six [64][64] operand
@@ -99,7 +99,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                       const bf16* __restrict__ b_, const bf16* __restrict__ dy_, const float* __restrict__ dsT_,
                       const float* __restrict__ ck_, float* __restrict__ ds0_, bf16* __restrict__ dr_,
                       bf16* __restrict__ dw_, bf16* __restrict__ dk_, bf16* __restrict__ dv_, bf16* __restrict__ da_,
-                      bf16* __restrict__ db_, const float* __restrict__ adj_, const __grid_constant__ TileMaps<7> maps) {
+                      bf16* __restrict__ db_, const float* __restrict__ adj_, int group, const __grid_constant__ TileMaps<7> maps) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // the swizzle acts on address bits
     unsigned char *AR = smem + BwdSmemX::kAR, *BK = smem + BwdSmemX::kBK, *SV = smem + BwdSmemX::kSV, *EY = smem + BwdSmemX::kEY;
@@ -124,7 +124,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     const i64 tok0 = (i64)bb * T * C + hh * 64;
     const i64 sbase = (i64)(bb * H + hh) * 64 * 64;
     const int nchunks = (T + LC - 1) / LC;
-    const int c_hi = adj_ ? blockIdx.z : nchunks - 1, c_lo = adj_ ? blockIdx.z : 0;
+    const int c_lo = adj_ ? blockIdx.z * group : 0, c_hi = adj_ ? min(nchunks, c_lo + group) - 1 : nchunks - 1;
     const float* ck = ck_ + (i64)(bb * H + hh) * (adj_ ? nchunks : T / 16) * 64 * 64;   // block [b][h] of the caller's (B,H,T/16,N,N) buffer
     const float* E0 = adj_ ? adj_ + ((i64)(bb * H + hh) * nchunks + c_hi) * 64 * 64 : dsT_ ? dsT_ + sbase : nullptr;
     const bf16* src[7] = {r_, w_, k_, v_, a_, b_, dy_};
@@ -559,7 +559,7 @@ WKV7_PHASE_READER(rwkvb200_phase_clocks_l32_bwd)
 
 }  // namespace v7x
 
-static int launch_l32_backward(int B, int T, int H, int chunks, const void* r, const void* w, const void* k, const void* v, const void* a,
+static int launch_l32_backward(int B, int T, int H, int group, const void* r, const void* w, const void* k, const void* v, const void* a,
                                const void* b, const void* dy, const float* dsT, const float* adj, const float* s, float* ds0, void* dr,
                                void* dw, void* dk, void* dv, void* da, void* db, cudaStream_t st) {
     using namespace v7x;
@@ -568,23 +568,34 @@ static int launch_l32_backward(int B, int T, int H, int chunks, const void* r, c
     TileMaps<7> maps;
     const void* in[7] = {r, w, k, v, a, b, dy};
     make_tile_maps<7>(maps, in, B, T, H);
-    wkv7x_backward_kernel<<<dim3(H, B, chunks), BNT, BwdSmemX::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)w, (const bf16*)k,
+    const int groups = ((T + LC - 1) / LC + group - 1) / group;
+    wkv7x_backward_kernel<<<dim3(H, B, groups), BNT, BwdSmemX::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)w, (const bf16*)k,
                                                                              (const bf16*)v, (const bf16*)a, (const bf16*)b,
                                                                              (const bf16*)dy, dsT, s, ds0, (bf16*)dr, (bf16*)dw, (bf16*)dk,
-                                                                             (bf16*)dv, (bf16*)da, (bf16*)db, adj, maps);
+                                                                             (bf16*)dv, (bf16*)da, (bf16*)db, adj, group, maps);
     return check_launch("wkv7_backward(tcgen05, 32-token chunks)");
 }
 
 int wkv7_l32_backward(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
                       const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
                       void* dk, void* dv, void* da, void* db, cudaStream_t st) {
-    return launch_l32_backward(B, T, H, 1, r, w, k, v, a, b, dy, dsT, nullptr, s, ds0, dr, dw, dk, dv, da, db, st);
+    return launch_l32_backward(B, T, H, (T + v7x::LC - 1) / v7x::LC, r, w, k, v, a, b, dy, dsT, nullptr, s, ds0, dr, dw, dk, dv, da, db, st);
 }
 
 int wkv7_l32_backward_chunks(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
                              const void* b, const void* dy, const float* adj, const float* states, void* dr, void* dw,
                              void* dk, void* dv, void* da, void* db, cudaStream_t st) {
-    return launch_l32_backward(B, T, H, (T + v7x::LC - 1) / v7x::LC, r, w, k, v, a, b, dy, nullptr, adj, states, nullptr, dr, dw, dk, dv, da, db, st);
+    // Chunks per block: the fewest waves of blocks, two per SM, where starting a block costs about half a chunk (its first tiles
+    // and the adjoint arrive with nothing to hide them).
+    const int nch = (T + v7x::LC - 1) / v7x::LC;
+    int group = 1;
+    double best = 1e30;
+    for (int g = 1; g <= nch; ++g) {
+        const long long blocks = (long long)B * H * ((nch + g - 1) / g);
+        const double cost = (double)((blocks + 295) / 296) * (g + 0.5);
+        if (cost < best) { best = cost; group = g; }
+    }
+    return launch_l32_backward(B, T, H, group, r, w, k, v, a, b, dy, nullptr, adj, states, nullptr, dr, dw, dk, dv, da, db, st);
 }
 
 int wkv7_l32_bwd_error_clear() {

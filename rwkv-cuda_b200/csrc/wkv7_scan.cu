@@ -14,6 +14,7 @@
 //
 // Record of a chunk, A (kept for the backward): Delta and Yop as the swizzled shared-memory images that the products read, We;
 // B (dropped after the forward): G and Y0 in the order of the threads that add them.  Bulk copies bring records in whole.
+#include <algorithm>
 #include "wkv7_l32.cuh"
 #include "wkv7_dispatch.cuh"
 
@@ -53,6 +54,8 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes,
 }
 
 // ---- (1) the operators of a chunk ------------------------------------------------------------------------------
+// Blocks walk over the chunks of all units (two blocks per SM); the tiles of a block's next chunk are on their way while it
+// works on this one.
 struct OpsSmem {
     static constexpr int kAR = 0, kBK = kAR + ARR64, kV = kBK + ARR64, kUak = kV + ARR32;
     static constexpr int kUbr = kUak + HALF32, kUkr = kUbr + HALF32, kD0 = kUkr + HALF32, kN1 = kD0 + HALF32;
@@ -63,7 +66,7 @@ struct OpsSmem {
 };
 static_assert(OpsSmem::kBytes <= 115712, "two blocks per SM");
 
-__global__ void __launch_bounds__(128, 2) wkv7_ops_kernel(int T, int H, const __grid_constant__ TileMaps<6> maps, unsigned char* __restrict__ recA,
+__global__ void __launch_bounds__(128, 2) wkv7_ops_kernel(int T, int H, int nch, int total, const __grid_constant__ TileMaps<6> maps, unsigned char* __restrict__ recA,
                                                           unsigned char* __restrict__ recB) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -73,19 +76,21 @@ __global__ void __launch_bounds__(128, 2) wkv7_ops_kernel(int T, int H, const __
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + OpsSmem::kBar);   // tiles landed, U done, outputs done, the chain's own
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 4);
 
-    const int c = blockIdx.x, hh = blockIdx.y, bb = blockIdx.z, nch = gridDim.x;
     const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int row0 = warp * 16, valid = min(LC, T - c * LC);
-    const i64 rec = ((i64)(bb * H + hh) * nch + c);
+    const int row0 = warp * 16;
+    auto request = [&](int rec) {   // one thread: the six tiles of a chunk
+        const int unit = rec / nch, c = rec - unit * nch, bb = unit / H, hh = unit - bb * H;
+        mbar_expect_bytes(bar, 6 * 4096);
+#pragma unroll
+        for (int x = 0; x < 6; ++x) tma_tile_load(Raw + x * 4096, &maps.m[x], hh * 64, bb * T + c * LC, bar);
+    };
 
     if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) mbar_init(bar + i);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        mbar_expect_bytes(bar, 6 * 4096);
-#pragma unroll
-        for (int x = 0; x < 6; ++x) tma_tile_load(Raw + x * 4096, &maps.m[x], hh * 64, bb * T + c * LC, bar);
+        request(blockIdx.x);
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(tmem_slot)) : "memory");
@@ -101,116 +106,128 @@ __global__ void __launch_bounds__(128, 2) wkv7_ops_kernel(int T, int H, const __
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16, lead = elect_one();
     const uint32_t arA = smem_u32(AR), bkA = smem_u32(BK), vA = smem_u32(Vs), uakA = smem_u32(Uak), ubrA = smem_u32(Ubr), ukrA = smem_u32(Ukr);
     const uint32_t d0A = smem_u32(D0), n1A = smem_u32(N1);
+    ChainSync cs{bar + 3, 0, 0};   // used by warp 0 only
     int fail = 0;
+    uint32_t par = 0;
+    bool pending = true;           // tiles on their way that nobody has waited for
 
-    if (!mbar_wait(bar, 0)) fail = 1;
-    RawChunk<6, 8> raw;
+    for (int rec = blockIdx.x; rec < total; rec += gridDim.x, par ^= 1) {
+        const int unit = rec / nch, valid = min(LC, T - (rec - unit * nch) * LC);
+        if (!mbar_wait(bar, par)) fail = 1;
+        pending = false;
+        RawChunk<6, 8> raw;
 #pragma unroll
-    for (int x = 0; x < 6; ++x)
+        for (int x = 0; x < 6; ++x)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int tt = 8 * warp + q;
-            raw.x[x][q] = tt < valid ? *reinterpret_cast<const uint32_t*>(Raw + x * 4096 + tt * 128 + 4 * lane) : 0u;
-        }
-    prepare_operands<6, 8, 4>(raw, valid, AR, BK, Vs, HALF32, nullptr, 0, We, Hs, nullptr, warp, lane);
-    proxy_fence();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (warp == 0) {
-        issue_u(tmG, arA, bkA, lead);
-        mma_commit(bar + 1, lead);
-    }
-    if (!mbar_wait(bar + 1, 0)) fail = 2;
-    tc_fence_after();
-    {
-        float u[8][4];
-        tmem_ld_tiles<8>(u, tmG + lane_off);
-        tmem_wait_ld();
-        scatter_u(u, warp, lane, Uab, N1, Uak, Ubr, Ukr);
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp < 2) tri_inverse16<UPITCH>(Uab + 16 * warp * (UPITCH + 1), D0, 16 * warp, lane);
-    proxy_fence();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (warp == 0) {
-        ChainSync cs{bar + 3, 0, 0};
-        const uint32_t id32s = idesc64(32, 1, 1), id32t = idesc64(32, 0, 1), id64s = idesc64(64, 1, 1), id64t = idesc64(64, 0, 1);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ss(tmZ, desc_mn(vA, ks * 8, HALF32), desc_mn(uakA, ks * 8, HALF32), id32s, ks > 0, lead);    // Z = V U_ak
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ss(tmS1, desc_mn(arA, ks * 8, HALF64), desc_mn(d0A, ks * 8, HALF32), id32s, ks > 0, lead);   // A~^T D0
-        cs.commit(lead);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ss(tmG, desc_mn(vA, ks * 8, HALF32), desc_mn(bkA + 32 * 128, ks * 8, HALF64), id64s, ks > 0, lead);   // G = V K~
-        cs.wait();
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ts(tmS2, tmZ + ks * 8, desc_mn(d0A, ks * 8, HALF32), id32t, ks > 0, lead);   // Z D0
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) mma_ts(tmR, tmS1 + ks * 8, desc_mn(n1A, ks * 8, HALF32), id32t, ks > 0, lead);   // (A~^T D0) N1
-        cs.sync(lead);
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) mma_ts(tmZ, tmS2 + ks * 8, desc_mn(n1A, ks * 8, HALF32), id32t, ks > 0, lead);   // (Z D0) N1
-#pragma unroll
-        for (int ks = 2; ks < 4; ++ks) mma_ts(tmS1, tmR + ks * 8, desc_mn(d0A, ks * 8, HALF32), id32t, 1, lead);        // A~^T T
-        cs.sync(lead);
-#pragma unroll
-        for (int ks = 2; ks < 4; ++ks) mma_ts(tmS2, tmZ + ks * 8, desc_mn(d0A, ks * 8, HALF32), id32t, 1, lead);        // V U_ak T
-        cs.commit(lead);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ts(tmD, tmS1 + ks * 8, desc_mn(bkA, ks * 8, HALF64), id64t, ks > 0, lead);   // Delta
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ts(tmR, tmS1 + ks * 8, desc_mn(ubrA, ks * 8, HALF32), id32t, ks > 0, lead);  // Yop (R~^T is added below)
-        cs.wait();
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ts(tmG, tmS2 + ks * 8, desc_mn(bkA, ks * 8, HALF64), id64t, 1, lead);        // G += V U_ak T B~
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ss(tmZ, desc_mn(vA, ks * 8, HALF32), desc_mn(ukrA, ks * 8, HALF32), id32s, ks > 0, lead);    // Y0 = V U_kr
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) mma_ts(tmZ, tmS2 + ks * 8, desc_mn(ubrA, ks * 8, HALF32), id32t, 1, lead);       //    + V U_ak T U_br
-        mma_commit(bar + 2, lead);
-        if (cs.fail) fail = 3;
-    }
-    if (!mbar_wait(bar + 2, 0)) fail = 4;
-    tc_fence_after();
-    {
-        unsigned char* A = recA + rec * kRecA;
-        float4* Bo = reinterpret_cast<float4*>(recB + rec * kRecB);
-        float d[8][4];
-        tmem_ld_tiles<8>(d, tmD + lane_off);
-        tmem_wait_ld();
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *reinterpret_cast<float2*>(A + sw(row0 + g + 8 * h, nt * 8 + 2 * t, HALF64)) = make_float2(tf32rf(d[nt][2 * h]), tf32rf(d[nt][2 * h + 1]));
-        float y[4][4];
-        tmem_ld_tiles<4>(y, tmR + lane_off);
-        tmem_wait_ld();
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = row0 + g + 8 * h, tt = nt * 8 + 2 * t;
-                const float r0 = unrounded(AR + sw(32 + tt, j, HALF64)), r1 = unrounded(AR + sw(33 + tt, j, HALF64));
-                *reinterpret_cast<float2*>(A + ARR64 + sw32(j, tt)) = make_float2(tf32rf(y[nt][2 * h] + r0), tf32rf(y[nt][2 * h + 1] + r1));
+            for (int q = 0; q < 8; ++q) {
+                const int tt = 8 * warp + q;
+                raw.x[x][q] = tt < valid ? *reinterpret_cast<const uint32_t*>(Raw + x * 4096 + tt * 128 + 4 * lane) : 0u;
             }
-        if (tid < 64) reinterpret_cast<float*>(A + ARR64 + HALF64)[tid] = We[tid];
-        tmem_ld_tiles<8>(d, tmG + lane_off);
-        tmem_ld_tiles<4>(y, tmZ + lane_off);
-        tmem_wait_ld();
+        prepare_operands<6, 8, 4>(raw, valid, AR, BK, Vs, HALF32, nullptr, 0, We, Hs, nullptr, warp, lane);
+        proxy_fence();
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        pending = rec + (int)gridDim.x < total;
+        if (pending && tid == 0) request(rec + gridDim.x);   // every thread has taken its part of the tiles
+        if (warp == 0) {
+            issue_u(tmG, arA, bkA, lead);
+            mma_commit(bar + 1, lead);
+        }
+        if (!mbar_wait(bar + 1, par)) fail = 2;
+        tc_fence_after();
+        {
+            float u[8][4];
+            tmem_ld_tiles<8>(u, tmG + lane_off);
+            tmem_wait_ld();
+            scatter_u(u, warp, lane, Uab, N1, Uak, Ubr, Ukr);
+        }
+        tc_fence_before();
+        __syncthreads();
+        if (warp < 2) tri_inverse16<UPITCH>(Uab + 16 * warp * (UPITCH + 1), D0, 16 * warp, lane);
+        proxy_fence();
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        if (warp == 0) {
+            const uint32_t id32s = idesc64(32, 1, 1), id32t = idesc64(32, 0, 1), id64s = idesc64(64, 1, 1), id64t = idesc64(64, 0, 1);
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) Bo[nt * 128 + tid] = make_float4(d[nt][0], d[nt][1], d[nt][2], d[nt][3]);
+            for (int ks = 0; ks < 4; ++ks) mma_ss(tmZ, desc_mn(vA, ks * 8, HALF32), desc_mn(uakA, ks * 8, HALF32), id32s, ks > 0, lead);    // Z = V U_ak
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) Bo[8 * 128 + nt * 128 + tid] = make_float4(y[nt][0], y[nt][1], y[nt][2], y[nt][3]);
+            for (int ks = 0; ks < 4; ++ks) mma_ss(tmS1, desc_mn(arA, ks * 8, HALF64), desc_mn(d0A, ks * 8, HALF32), id32s, ks > 0, lead);   // A~^T D0
+            cs.commit(lead);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) mma_ss(tmG, desc_mn(vA, ks * 8, HALF32), desc_mn(bkA + 32 * 128, ks * 8, HALF64), id64s, ks > 0, lead);   // G = V K~
+            cs.wait();
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) mma_ts(tmS2, tmZ + ks * 8, desc_mn(d0A, ks * 8, HALF32), id32t, ks > 0, lead);   // Z D0
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) mma_ts(tmR, tmS1 + ks * 8, desc_mn(n1A, ks * 8, HALF32), id32t, ks > 0, lead);   // (A~^T D0) N1
+            cs.sync(lead);
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) mma_ts(tmZ, tmS2 + ks * 8, desc_mn(n1A, ks * 8, HALF32), id32t, ks > 0, lead);   // (Z D0) N1
+#pragma unroll
+            for (int ks = 2; ks < 4; ++ks) mma_ts(tmS1, tmR + ks * 8, desc_mn(d0A, ks * 8, HALF32), id32t, 1, lead);        // A~^T T
+            cs.sync(lead);
+#pragma unroll
+            for (int ks = 2; ks < 4; ++ks) mma_ts(tmS2, tmZ + ks * 8, desc_mn(d0A, ks * 8, HALF32), id32t, 1, lead);        // V U_ak T
+            cs.commit(lead);
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) mma_ts(tmD, tmS1 + ks * 8, desc_mn(bkA, ks * 8, HALF64), id64t, ks > 0, lead);   // Delta
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) mma_ts(tmR, tmS1 + ks * 8, desc_mn(ubrA, ks * 8, HALF32), id32t, ks > 0, lead);  // Yop (R~^T is added below)
+            cs.wait();
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) mma_ts(tmG, tmS2 + ks * 8, desc_mn(bkA, ks * 8, HALF64), id64t, 1, lead);        // G += V U_ak T B~
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) mma_ss(tmZ, desc_mn(vA, ks * 8, HALF32), desc_mn(ukrA, ks * 8, HALF32), id32s, ks > 0, lead);    // Y0 = V U_kr
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks) mma_ts(tmZ, tmS2 + ks * 8, desc_mn(ubrA, ks * 8, HALF32), id32t, 1, lead);       //    + V U_ak T U_br
+            mma_commit(bar + 2, lead);
+            if (cs.fail) fail = 3;
+        }
+        if (!mbar_wait(bar + 2, par)) fail = 4;
+        tc_fence_after();
+        {
+            unsigned char* A = recA + (i64)rec * kRecA;
+            float4* Bo = reinterpret_cast<float4*>(recB + (i64)rec * kRecB);
+            float d[8][4];
+            tmem_ld_tiles<8>(d, tmD + lane_off);
+            tmem_wait_ld();
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    *reinterpret_cast<float2*>(A + sw(row0 + g + 8 * h, nt * 8 + 2 * t, HALF64)) = make_float2(tf32rf(d[nt][2 * h]), tf32rf(d[nt][2 * h + 1]));
+            float y[4][4];
+            tmem_ld_tiles<4>(y, tmR + lane_off);
+            tmem_wait_ld();
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int j = row0 + g + 8 * h, tt = nt * 8 + 2 * t;
+                    const float r0 = unrounded(AR + sw(32 + tt, j, HALF64)), r1 = unrounded(AR + sw(33 + tt, j, HALF64));
+                    *reinterpret_cast<float2*>(A + ARR64 + sw32(j, tt)) = make_float2(tf32rf(y[nt][2 * h] + r0), tf32rf(y[nt][2 * h + 1] + r1));
+                }
+            if (tid < 64) reinterpret_cast<float*>(A + ARR64 + HALF64)[tid] = We[tid];
+            tmem_ld_tiles<8>(d, tmG + lane_off);
+            tmem_ld_tiles<4>(y, tmZ + lane_off);
+            tmem_wait_ld();
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt) Bo[nt * 128 + tid] = make_float4(d[nt][0], d[nt][1], d[nt][2], d[nt][3]);
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) Bo[8 * 128 + nt * 128 + tid] = make_float4(y[nt][0], y[nt][1], y[nt][2], y[nt][3]);
+        }
+        if (fail) reinterpret_cast<float*>(recA + (i64)rec * kRecA)[0] = __int_as_float(0x7fc00000);   // the chain carries it into the outputs
+        tc_fence_before();
+        if (__syncthreads_or(fail)) { par ^= 1; break; }   // (and: the operand arrays may be written again)
+        tc_fence_after();
     }
+    if (pending && fail) mbar_wait(bar, par);   // leaving early: the requested tiles must have landed before the block may end
     if (fail) atomicMax(&g_v7s_error, fail);
     tc_fence_before();
     __syncthreads();
-    if (fail) reinterpret_cast<float*>(recA + rec * kRecA)[0] = __int_as_float(0x7fc00000);   // the chain carries it into the outputs
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tm) : "memory");
 }
 
@@ -225,11 +242,18 @@ struct ChainSmem {
     static constexpr int kBytes = kBar + 256 + 1024;
 };
 static_assert(ChainSmem::kStage % 1024 == 0 && ChainSmem::kBytes <= 232448, "layout");
-enum { kFull = 0, kEmpty = kFull + NSTG, kOper = kEmpty + NSTG, kState = kOper + NSTG, kProdD, kProdY, kNBarC };
+enum { kFull = 0, kEmpty = kFull + NSTG, kOper = kEmpty + NSTG, kState = kOper + NSTG, kProdD, kProdY, kYTaken = kProdY + 2, kNBarC = kYTaken + 2 };
 
-// Forward: warps 0-3 carry S in fp32 registers (16 value rows each) and write y, the states and sT; warp 4 issues the products;
-// warp 5 asks for the records.  grid (H, B).  states: S at the start of every chunk.
-__global__ void __launch_bounds__(192, 1) wkv7_chain_forward_kernel(int T, int H, int nch, const float* __restrict__ s0_, const unsigned char* __restrict__ recA,
+// Arrival of a warp (after what its lanes have done): one lane arrives, 32 arrivals on one word would queue up.
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+
+// Forward: warps 0-3 carry S in fp32 registers (16 value rows each) and write the states and sT; warps 4-7 write y; warp 8 issues
+// the products; warp 9 asks for the records.  A waiter may be one phase of an mbarrier behind, not two: the Y product and its
+// release have an mbarrier for even and one for odd chunks.  grid (H, B).  states: S at the start of every chunk.
+__global__ void __launch_bounds__(320, 1) wkv7_chain_forward_kernel(int T, int H, int nch, const float* __restrict__ s0_, const unsigned char* __restrict__ recA,
                                                                     const unsigned char* __restrict__ recB, bf16* __restrict__ y_,
                                                                     float* __restrict__ sT_, float* __restrict__ states) {
     extern __shared__ unsigned char smem_raw[];
@@ -244,7 +268,7 @@ __global__ void __launch_bounds__(192, 1) wkv7_chain_forward_kernel(int T, int H
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < kNBarC; ++i) mbar_init_count(bar + i, i == kState ? 128 : 1);
+        for (int i = 0; i < kNBarC; ++i) mbar_init_count(bar + i, i == kState || i == kYTaken || i == kYTaken + 1 ? 4 : i >= kEmpty && i < kEmpty + NSTG ? 8 : 1);
         *abort_word = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -259,7 +283,7 @@ __global__ void __launch_bounds__(192, 1) wkv7_chain_forward_kernel(int T, int H
     const uint32_t tmD = tm + 128, tmY = tm + 192;
     int fail = 0;
 
-    if (warp == 5) {
+    if (warp == 9) {
         if (lane == 0) {
             int c = 0;
             for (; c < nch; ++c) {
@@ -277,27 +301,68 @@ __global__ void __launch_bounds__(192, 1) wkv7_chain_forward_kernel(int T, int H
             if (*abort_word)   // leaving early: the copies in flight must have landed before the block may end
                 for (int cc = max(0, c - NSTG); cc < c; ++cc) mbar_wait(bar + kFull + cc % NSTG, (cc / NSTG) & 1);
         }
-    } else if (warp == 4) {
+    } else if (warp == 8) {
         const uint32_t lead = elect_one(), idD = idesc64(64, 0, 1), idY = idesc64(32, 0, 1);
         for (int c = 0; c < nch; ++c) {
             const int st = c % NSTG;
             if (!mbar_wait(bar + kFull + st, (c / NSTG) & 1)) fail = 2;
             if (!mbar_wait(bar + kState, c & 1)) fail = 3;
-            if (__any_sync(0xffffffffu, fail != 0 || *abort_word != 0)) break;
+            if (__any_sync(0xffffffffu, fail)) break;
             tc_fence_after();
             const uint32_t dA = smem_u32(smem + st * ChainSmem::kStage), yA = dA + ARR64, tmS = tm + (c & 1) * 64;
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) mma_ts(tmD, tmS + ks * 8, desc_mn(dA, ks * 8, HALF64), idD, ks > 0, lead);   // S Delta
             mma_commit(bar + kProdD, lead);
+            if (c > 1 && !mbar_wait(bar + kYTaken + (c & 1), ((c >> 1) - 1) & 1)) fail = 7;   // the Y of two chunks ago has been read
+            if (__any_sync(0xffffffffu, fail)) break;
+            tc_fence_after();
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) mma_ts(tmY + (c & 1) * 32, tmS + ks * 8, desc_mn(yA, ks * 8, HALF64), idY, ks > 0, lead);   // S Yop
-            mma_commit(bar + kProdY, lead);
+            mma_commit(bar + kProdY + (c & 1), lead);
         }
         if (fail && lane == 0) atomicMax(const_cast<int*>(abort_word), fail);
+    } else if (warp >= 4) {
+        // y: the product and Y0, out as rows of bf16
+        const int quarter = warp & 3, gtid = tid & 127, row0 = quarter * 16;
+        const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+        const i64 tok0 = (i64)bb * T * C + hh * 64;
+        for (int c = 0; c < nch; ++c) {
+            const int st = c % NSTG, valid = min(LC, T - c * LC);
+            const float4* Y0 = reinterpret_cast<const float4*>(smem + st * ChainSmem::kStage + 2 * ARR64 + HALF64);
+            if (!mbar_wait(bar + kFull + st, (c / NSTG) & 1)) fail = 8;
+            if (!mbar_wait(bar + kProdY + (c & 1), (c >> 1) & 1)) fail = 6;
+            tc_fence_after();
+            float y[4][4];
+            tmem_ld_tiles<4>(y, tmY + (c & 1) * 32 + lane_off);
+            tmem_wait_ld();
+            tc_fence_before();
+            warp_arrive(bar + kYTaken + (c & 1), lane);
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const float4 q = Y0[nt * 128 + gtid];
+                const float add[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    ystage[(nt * 8 + 2 * t + (e & 1)) * 72 + row0 + g + ((e & 2) ? 8 : 0)] = __float2bfloat16_rn(y[nt][e] + add[e]);
+            }
+            warp_arrive(bar + kEmpty + st, lane);   // (the product has read the record: it is complete)
+            if (fail) atomicMax(const_cast<int*>(abort_word), fail);
+            if (gtid == 0) *gabort = *abort_word;
+            group_sync(1, 128);
+            const int stop = *gabort, tt = gtid >> 2, q = gtid & 3;
+            if (tt < valid) {
+                const uint4* sp = reinterpret_cast<const uint4*>(ystage + tt * 72 + q * 16);
+                uint4* dp = reinterpret_cast<uint4*>(y_ + tok0 + (i64)(c * LC + tt) * C + q * 16);
+                dp[0] = sp[0];
+                dp[1] = sp[1];
+            }
+            if (stop) break;
+            group_sync(2, 128);                     // the staging rows may be written again
+        }
     } else {
         const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
         const int row0 = warp * 16;
-        const i64 tok0 = (i64)bb * T * C + hh * 64, sbase = (i64)unit * 4096;
+        const i64 sbase = (i64)unit * 4096;
         float* st_out = states + (i64)unit * nch * 4096;
         auto put_state = [&](float* dst, const float (&S)[8][4]) {
 #pragma unroll
@@ -318,12 +383,12 @@ __global__ void __launch_bounds__(192, 1) wkv7_chain_forward_kernel(int T, int H
         }
         put_operand(tm + lane_off, S);
         tc_fence_before();
-        mbar_arrive(bar + kState);
+        warp_arrive(bar + kState, lane);
         put_state(st_out, S);
         for (int c = 0; c < nch; ++c) {
-            const int st = c % NSTG, valid = min(LC, T - c * LC);
+            const int st = c % NSTG;
             const unsigned char* s = smem + st * ChainSmem::kStage;
-            const float4 *G = reinterpret_cast<const float4*>(s + ARR64 + HALF64), *Y0 = G + 8 * 128;
+            const float4 *G = reinterpret_cast<const float4*>(s + ARR64 + HALF64);
             const float* We = reinterpret_cast<const float*>(s + ChainSmem::kWe);
             if (!mbar_wait(bar + kFull + st, (c / NSTG) & 1)) fail = 4;
             // (S + G) diag(We) is ready before the product is
@@ -350,43 +415,15 @@ __global__ void __launch_bounds__(192, 1) wkv7_chain_forward_kernel(int T, int H
             if (c + 1 < nch) {
                 put_operand(tm + ((c + 1) & 1) * 64 + lane_off, S);
                 tc_fence_before();
-                mbar_arrive(bar + kState);   // the next chunk's products may start
+                warp_arrive(bar + kState, lane);   // the next chunk's products may start
                 put_state(st_out + (i64)(c + 1) * 4096, S);
             } else if (sT_ != nullptr) {
                 put_state(sT_ + sbase, S);
             }
-            if (!mbar_wait(bar + kProdY, c & 1)) fail = 6;
-            tc_fence_after();
-            {
-                float y[4][4];
-                tmem_ld_tiles<4>(y, tmY + (c & 1) * 32 + lane_off);
-                tmem_wait_ld();
-#pragma unroll
-                for (int nt = 0; nt < 4; ++nt) {
-                    const float4 q = Y0[nt * 128 + tid];
-                    const float add[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        ystage[(nt * 8 + 2 * t + (e & 1)) * 72 + row0 + g + ((e & 2) ? 8 : 0)] = __float2bfloat16_rn(y[nt][e] + add[e]);
-                }
-            }
-            if (fail) atomicMax(const_cast<int*>(abort_word), fail);
-            if (tid == 0) *gabort = *abort_word;
-            group_sync(1, 128);
-            if (tid == 0) mbar_arrive(bar + kEmpty + st);   // both products have read the record, every thread its part of G and Y0
-            const int stop = *gabort;
-            {
-                const int tt = tid >> 2, q = tid & 3;
-                if (tt < valid) {
-                    const uint4* sp = reinterpret_cast<const uint4*>(ystage + tt * 72 + q * 16);
-                    uint4* dp = reinterpret_cast<uint4*>(y_ + tok0 + (i64)(c * LC + tt) * C + q * 16);
-                    dp[0] = sp[0];
-                    dp[1] = sp[1];
-                }
-            }
-            if (stop) break;
-            group_sync(2, 128);                              // the staging rows may be written again
+            warp_arrive(bar + kEmpty + st, lane);
+            if (__any_sync(0xffffffffu, fail)) break;
         }
+        if (fail) atomicMax(const_cast<int*>(abort_word), fail);
     }
     tc_fence_before();
     __syncthreads();
@@ -414,7 +451,7 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
     if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < kNBarC; ++i)
-            mbar_init_count(bar + i, i == kState || (i >= kEmpty && i < kEmpty + NSTG) ? 128 : i >= kOper && i < kOper + NSTG ? 64 : 1);
+            mbar_init_count(bar + i, i == kState || (i >= kEmpty && i < kEmpty + NSTG) ? 4 : i >= kOper && i < kOper + NSTG ? 2 : 1);
         *abort_word = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -450,7 +487,7 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
         for (int n = 0; n < nch; ++n) {
             const int st = n % NSTG, valid = min(LC, T - (nch - 1 - n) * LC);
             if (!mbar_wait(bar + kFull + st, (n / NSTG) & 1)) fail = 12;
-            if (__any_sync(0xffffffffu, fail != 0 || *abort_word != 0)) break;
+            if (__any_sync(0xffffffffu, fail)) break;
             unsigned char* s = smem + st * ChainSmem::kStage;
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
@@ -459,7 +496,7 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
                 *reinterpret_cast<float2*>(s + kOperand + sw(tt, 2 * lane, HALF32)) = bf16x2_to_f2(x);
             }
             proxy_fence();
-            mbar_arrive(bar + kOper + st);
+            warp_arrive(bar + kOper + st, lane);
         }
         if (fail && lane == 0) atomicMax(const_cast<int*>(abort_word), fail);
     } else if (warp == 4) {
@@ -467,7 +504,7 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
         for (int n = 0; n <= nch; ++n) {
             if (n > 0) {   // Ew Delta^T of step n - 1
                 if (!mbar_wait(bar + kState, (n - 1) & 1)) fail = 13;
-                if (__any_sync(0xffffffffu, fail != 0 || *abort_word != 0)) break;
+                if (__any_sync(0xffffffffu, fail)) break;
                 tc_fence_after();
                 const uint32_t dA = smem_u32(smem + ((n - 1) % NSTG) * ChainSmem::kStage);
 #pragma unroll
@@ -477,7 +514,7 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
             if (n == nch) break;
             const int st = n % NSTG;   // dY Yop^T of step n needs no state: it is under way before the state arrives
             if (!mbar_wait(bar + kOper + st, (n / NSTG) & 1)) fail = 14;
-            if (__any_sync(0xffffffffu, fail != 0 || *abort_word != 0)) break;
+            if (__any_sync(0xffffffffu, fail)) break;
             tc_fence_after();
             const uint32_t yA = smem_u32(smem + st * ChainSmem::kStage + ARR64), oA = smem_u32(smem + st * ChainSmem::kStage + kOperand);
 #pragma unroll
@@ -517,7 +554,7 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
             }
             put_operand(tm + lane_off, Ew);
             tc_fence_before();
-            mbar_arrive(bar + kState);
+            warp_arrive(bar + kState, lane);
             put(adjoints + ((i64)unit * nch + c) * 4096, E);
             if (!mbar_wait(bar + kProdD, n & 1)) fail = 16;
             tc_fence_after();
@@ -528,10 +565,10 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
             for (int nt = 0; nt < 8; ++nt)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) E[nt][e] += Ew[nt][e];
-            mbar_arrive(bar + kEmpty + st);
-            if (fail) atomicMax(const_cast<int*>(abort_word), fail);
-            if (__any_sync(0xffffffffu, fail != 0 || *abort_word != 0)) break;
+            warp_arrive(bar + kEmpty + st, lane);
+            if (__any_sync(0xffffffffu, fail)) break;
         }
+        if (fail) atomicMax(const_cast<int*>(abort_word), fail);
         if (ds0_ != nullptr) put(ds0_ + sbase, E);
     }
     tc_fence_before();
@@ -563,8 +600,10 @@ int wkv7_scan_forward(int B, int T, int H, const float* s0, const void* r, const
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv7_train_forward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     float* states = static_cast<float*>(saved);
     unsigned char* recA = static_cast<unsigned char*>(saved) + (size_t)B * H * nch * 64 * 64 * sizeof(float);
-    wkv7_ops_kernel<<<dim3(nch, H, B), 128, OpsSmem::kBytes, st>>>(T, H, maps, recA, static_cast<unsigned char*>(work));
-    wkv7_chain_forward_kernel<<<dim3(H, B), 192, ChainSmem::kBytes, st>>>(T, H, nch, s0, recA, static_cast<unsigned char*>(work), (bf16*)y, sT, states);
+    const long long total = (long long)B * H * nch;
+    RWKV_REQUIRE(total < (1ll << 31), RWKVB200_EINVAL, "wkv7_train_forward: too many chunks");
+    wkv7_ops_kernel<<<(int)std::min<long long>(total, 2 * 148), 128, OpsSmem::kBytes, st>>>(T, H, nch, (int)total, maps, recA, static_cast<unsigned char*>(work));
+    wkv7_chain_forward_kernel<<<dim3(H, B), 320, ChainSmem::kBytes, st>>>(T, H, nch, s0, recA, static_cast<unsigned char*>(work), (bf16*)y, sT, states);
     return check_launch("wkv7_train_forward(chunks in parallel)");
 }
 
