@@ -17,7 +17,7 @@
 // anchored afresh at every chunk so rounding does not accumulate along the sequence.
 //
 // With `adj_` (the adjoint at the end of every chunk, from wkv7_scan.cu) a block does `group` chunks, the blockIdx.z-th such group,
-// and the states in ck_ follow each other chunk by chunk.
+// and the states in ck_ follow each other chunk by chunk; both are images in the layout of the operand arrays.
 //
 // One CTA of 8 warps per (batch, head), two CTAs per SM.  Warp w works on quarter w%4 of tensor memory
 // (16 rows) and, where a region is split, on token half w/4.  Shared memory: six [64][64] operand
@@ -156,8 +156,8 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const int row = row0 + g + ((e & 2) ? 8 : 0), col = 32 * hs + nt * 8 + 2 * t + (e & 1);
-                Ed[nt][e] = E0 ? E0[row * 64 + col] : 0.f;
-                Td[nt][e] = E0 ? E0[col * 64 + row] : 0.f;
+                Ed[nt][e] = E0 ? E0[adj_ ? sw(row, col, HALF64) / 4 : row * 64 + col] : 0.f;
+                Td[nt][e] = E0 ? E0[adj_ ? sw(col, row, HALF64) / 4 : col * 64 + row] : 0.f;
             }
         tmem_st_tiles<4>(tmE + 32 * hs + lane_off, Ed);
         tmem_st_tiles<4>(tmET + 32 * hs + lane_off, Td);
@@ -169,7 +169,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
             const int idx = q4 * BNT + tid, i = idx >> 4, col = (idx & 15) * 4;
-            cp_async16(S0 + sw(i, col, HALF64), s0g + i * 64 + col);
+            cp_async16(S0 + (adj_ ? idx * 16 : sw(i, col, HALF64)), s0g + idx * 4);
         }
         cp_async_commit();
     };

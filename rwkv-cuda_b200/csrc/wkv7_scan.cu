@@ -238,7 +238,8 @@ struct ChainSmem {
     static constexpr int kStage = ARR64 + HALF64 + ARR64 + HALF64 + 1024;   // Delta, Yop, then G and Y0 (backward: dY as operand, its raw tile), We
     static constexpr int kWe = ARR64 + HALF64 + ARR64 + HALF64;
     static constexpr int kY = NSTG * kStage;                                // bf16 [32][72]
-    static constexpr int kBar = kY + (32 * 72 * 2 + 127) / 128 * 128;
+    static constexpr int kOut = (kY + 32 * 72 * 2 + 1023) / 1024 * 1024;    // two images of S (or E) on their way out
+    static constexpr int kBar = kOut + 2 * ARR64;
     static constexpr int kBytes = kBar + 256 + 1024;
 };
 static_assert(ChainSmem::kStage % 1024 == 0 && ChainSmem::kBytes <= 232448, "layout");
@@ -250,9 +251,39 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
     if (lane == 0) mbar_arrive(bar);
 }
 
+// A warp's 16 rows of S (or E) -> image `n` of a chunk in device memory, in the swizzled layout of an operand array: 16 stores of 8
+// bytes straight to device memory took longer than the products they ran beside, so the rows go through shared memory (two
+// buffers in turn) and leave as two bulk copies of 2 KB.
+__device__ __forceinline__ void send_rows(unsigned char* smem_out, int n, unsigned char* image, const float (&x)[8][4], int row0, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    unsigned char* buf = smem_out + (n & 1) * ARR64;
+    if (n >= 2) {   // the copies that left this buffer before have read it
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+    }
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+        *reinterpret_cast<float2*>(buf + sw(row0 + g, nt * 8 + 2 * t, HALF64)) = make_float2(x[nt][0], x[nt][1]);
+        *reinterpret_cast<float2*>(buf + sw(row0 + g + 8, nt * 8 + 2 * t, HALF64)) = make_float2(x[nt][2], x[nt][3]);
+    }
+    proxy_fence();
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(__cvta_generic_to_global(image + h * HALF64 + row0 * 128)),
+                         "r"(smem_u32(buf + h * HALF64 + row0 * 128)), "r"(16 * 128) : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+}
+__device__ __forceinline__ void sent_all(int lane) {   // before the block ends
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 // Forward: warps 0-3 carry S in fp32 registers (16 value rows each) and write the states and sT; warps 4-7 write y; warp 8 issues
 // the products; warp 9 asks for the records.  A waiter may be one phase of an mbarrier behind, not two: the Y product and its
-// release have an mbarrier for even and one for odd chunks.  grid (H, B).  states: S at the start of every chunk.
+// release have an mbarrier for even and one for odd chunks.  grid (H, B).  states: S at the start of
+// every chunk, as images of the operand array that the backward makes of it.
 __global__ void __launch_bounds__(320, 1) wkv7_chain_forward_kernel(int T, int H, int nch, const float* __restrict__ s0_, const unsigned char* __restrict__ recA,
                                                                     const unsigned char* __restrict__ recB, bf16* __restrict__ y_,
                                                                     float* __restrict__ sT_, float* __restrict__ states) {
@@ -363,7 +394,7 @@ __global__ void __launch_bounds__(320, 1) wkv7_chain_forward_kernel(int T, int H
         const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
         const int row0 = warp * 16;
         const i64 sbase = (i64)unit * 4096;
-        float* st_out = states + (i64)unit * nch * 4096;
+        unsigned char* st_out = reinterpret_cast<unsigned char*>(states) + (i64)unit * nch * ARR64;
         auto put_state = [&](float* dst, const float (&S)[8][4]) {
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt) {
@@ -384,7 +415,7 @@ __global__ void __launch_bounds__(320, 1) wkv7_chain_forward_kernel(int T, int H
         put_operand(tm + lane_off, S);
         tc_fence_before();
         warp_arrive(bar + kState, lane);
-        put_state(st_out, S);
+        send_rows(smem + ChainSmem::kOut, 0, st_out, S, row0, lane);
         for (int c = 0; c < nch; ++c) {
             const int st = c % NSTG;
             const unsigned char* s = smem + st * ChainSmem::kStage;
@@ -416,13 +447,14 @@ __global__ void __launch_bounds__(320, 1) wkv7_chain_forward_kernel(int T, int H
                 put_operand(tm + ((c + 1) & 1) * 64 + lane_off, S);
                 tc_fence_before();
                 warp_arrive(bar + kState, lane);   // the next chunk's products may start
-                put_state(st_out + (i64)(c + 1) * 4096, S);
+                send_rows(smem + ChainSmem::kOut, c + 1, st_out + (i64)(c + 1) * ARR64, S, row0, lane);
             } else if (sT_ != nullptr) {
                 put_state(sT_ + sbase, S);
             }
             warp_arrive(bar + kEmpty + st, lane);
             if (__any_sync(0xffffffffu, fail)) break;
         }
+        sent_all(lane);
         if (fail) atomicMax(const_cast<int*>(abort_word), fail);
     }
     tc_fence_before();
@@ -435,7 +467,7 @@ __global__ void __launch_bounds__(320, 1) wkv7_chain_forward_kernel(int T, int H
 }
 
 // Backward: the same roles with E; warps 6 and 7 turn the tile of dY into an operand.  E at the end of every chunk is written to
-// `adjoints`, the adjoint of the initial state to ds0.
+// `adjoints` (images like the states), the adjoint of the initial state to ds0.
 __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int H, int nch, const float* __restrict__ dsT_,
                                                                      const __grid_constant__ CUtensorMap dymap, const unsigned char* __restrict__ recA,
                                                                      float* __restrict__ adjoints, float* __restrict__ ds0_) {
@@ -555,7 +587,7 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
             put_operand(tm + lane_off, Ew);
             tc_fence_before();
             warp_arrive(bar + kState, lane);
-            put(adjoints + ((i64)unit * nch + c) * 4096, E);
+            send_rows(smem + ChainSmem::kOut, n, reinterpret_cast<unsigned char*>(adjoints) + ((i64)unit * nch + c) * ARR64, E, row0, lane);
             if (!mbar_wait(bar + kProdD, n & 1)) fail = 16;
             tc_fence_after();
             tmem_ld_tiles<8>(E, tmD + (n & 1) * 64 + lane_off);
@@ -568,6 +600,7 @@ __global__ void __launch_bounds__(256, 1) wkv7_chain_backward_kernel(int T, int 
             warp_arrive(bar + kEmpty + st, lane);
             if (__any_sync(0xffffffffu, fail)) break;
         }
+        sent_all(lane);
         if (fail) atomicMax(const_cast<int*>(abort_word), fail);
         if (ds0_ != nullptr) put(ds0_ + sbase, E);
     }
