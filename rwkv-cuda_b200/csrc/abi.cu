@@ -4,7 +4,6 @@
 #include "wkv7_dispatch.cuh"
 #include "wkv6_chunked.cuh"
 #include <atomic>
-#include <stdlib.h>
 #include <initializer_list>
 
 namespace rwkvb200 {
@@ -217,12 +216,13 @@ extern "C" int rwkvb200_wkv7_state_update(int dtype, int B, int T, int H, int N,
 }
 
 // ---- training flow ------------------------------------------------------------------------------------------------------
-// Path 1: the chunks in parallel (wkv7_scan.cu), for tensor-core shapes with few units.  Path 0: rwkvb200_wkv7_forward /
-// _backward, `saved` = s then sa.
+// Path 1: the chunks in parallel (wkv7_scan.cu), for tensor-core shapes with at most a unit per two SMs: beyond that the extra
+// products cost more than the short chain saves (T 2048, forward + backward: 32 units 408 -> 226 us, 64 units 410 -> 345 us,
+// 80 units 413 -> 399 us, 128 units 421 -> 586 us), and up to 64 tokens there is next to nothing to walk in parallel.
+// Path 0: rwkvb200_wkv7_forward / _backward, `saved` = s then sa.
 extern "C" int rwkvb200_wkv7_train_path(int dtype, int B, int T, int H, int N) {
-    static const int lim = getenv("V7_SCAN") ? atoi(getenv("V7_SCAN")) : 64;
     const bool tensor = dtype == RWKVB200_BF16 && N == 64 && g_wkv7_path.load() != 1 && g_wkv7_bwd_form.load() == 0 && !g_no_tensor_maps.load();
-    return tensor && T > 64 && (long long)B * H <= lim && B <= 65535 ? 1 : 0;
+    return tensor && T > 64 && 2ll * B * H <= sm_count() ? 1 : 0;
 }
 extern "C" size_t rwkvb200_wkv7_train_saved_bytes(int B, int T, int H, int N, int path) {
     if (B <= 0 || T <= 0 || H <= 0 || N <= 0) return 0;

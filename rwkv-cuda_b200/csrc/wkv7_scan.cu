@@ -10,7 +10,13 @@
 // So: (1) one block per chunk makes Delta, Yop, G, Y0 (nothing of it depends on the state); (2) one block per unit walks the
 // chunks with two products each, S in fp32 registers and, rounded to TF32, in tensor memory; (3) backward: one block per unit
 // walks the adjoint the same way and leaves it at the end of every chunk; (4) wkv7_l32_bwd.cu runs with one block per chunk.
-// The products of the chain are read as TF32 like every other operand; S, E and all sums stay fp32.
+// The products of the chain are read as TF32 like every other operand; S, E and all sums stay fp32 (errors against fp64 as in the
+// chunk-by-chunk kernels: sT 2.2e-4, ds0 2.1e-4).
+//
+// Measured on a B200, B2 T1040 H12 (24 units, 792 chunks): operators 19 us, chain 27 us (0.7 us per chunk against 2 us), adjoint
+// chain 26 us (against 4.5 us per chunk), gradients 35 us; forward + backward 219 -> 113 us.  The chain of a chunk is one 64x64x64
+// product and its way through registers; 16 stores of the state per thread beside it made it 1.0 us (see send_rows), y written
+// by the same warps as long again.
 //
 // Record of a chunk, A (kept for the backward): Delta and Yop as the swizzled shared-memory images that the products read, We;
 // B (dropped after the forward): G and Y0 in the order of the threads that add them.  Bulk copies bring records in whole.
