@@ -47,6 +47,28 @@ __device__ __forceinline__ Sum after(Sum first, float dw, Sum second) {
     return Sum{s.a * first.p + s.b * second.p, s.a * first.q + s.b * second.q, s.m};
 }
 
+// Plain weights.  While the exponents of a segment lie within kSpan of each other (and the start state's with them) they are taken
+// relative to the largest once, e_i = e^{k_i - M}, and the recurrences inside the segment are multiply-adds with the constant
+// e^w: one exponential per token instead of three forward and six backward.  What such a weight loses by underflow (below
+// e^{-87}) is less than 1e-11 of any term that it is added to, because every token's own weight is at least e^{-kSpan - kBonus}.
+// A warp with a lane outside the bounds takes the running-maximum form for that segment.  The scan over segments is the same.
+constexpr float kSpan = 40.f, kBonus = 20.f;
+struct Range {
+    float lo, hi;
+};
+__device__ __forceinline__ Range range_of(const float (&k)[L], int n) {
+    Range r = {k[0], k[0]};
+#pragma unroll
+    for (int i = 1; i < L; ++i)
+        if (i < n) { r.lo = fminf(r.lo, k[i]); r.hi = fmaxf(r.hi, k[i]); }
+    return r;
+}
+// the start state joins the range (an empty one has no exponent): true if plain weights relative to r.hi serve
+__device__ __forceinline__ bool join(Range& r, const Sum& s) {
+    if (s.q != 0.f) { r.lo = fminf(r.lo, s.o); r.hi = fmaxf(r.hi, s.o); }
+    return r.hi - r.lo <= kSpan;
+}
+
 template <int S>
 struct ScanBuf {
     float x[3][S][33];
@@ -54,10 +76,21 @@ struct ScanBuf {
     float carry[3][32];
 };
 
+// e^{8 w}, e^{16 w}, ... of the channel that a thread scans (constant for the kernel)
+struct SegmentDecay {
+    float d[5];
+    template <int S>
+    __device__ __forceinline__ void set(const ScanBuf<S>& buf, int warp, int lane) {
+        const float lw = L * buf.w[warp * (32 / S) + lane / S];
+#pragma unroll
+        for (int j = 0; (1 << j) < S; ++j) d[j] = expf(lw * (float)(1 << j));
+    }
+};
+
 // Start states of the S segments of a tile from their local sums and the state carried in from the tile before (in walking
 // order: REV walks the segments from S-1 down).  Called by all warps; leaves the carried state after the tile in `buf`.
 template <int S, bool REV>
-__device__ __forceinline__ Sum scan_segments(ScanBuf<S>& buf, Sum local, int warp, int lane) {
+__device__ __forceinline__ Sum scan_segments(ScanBuf<S>& buf, const SegmentDecay& decay, Sum local, int warp, int lane) {
     buf.x[0][warp][lane] = local.p; buf.x[1][warp][lane] = local.q; buf.x[2][warp][lane] = local.o;
     __syncthreads();
     {   // this thread: channel ch, segment number i in walking order
@@ -65,21 +98,48 @@ __device__ __forceinline__ Sum scan_segments(ScanBuf<S>& buf, Sum local, int war
         const float lw = L * buf.w[ch];
         Sum s = {buf.x[0][seg][ch], buf.x[1][seg][ch], buf.x[2][seg][ch]};
         const Sum c = {buf.carry[0][ch], buf.carry[1][ch], buf.carry[2][ch]};
-        if (i == 0) s = after(c, lw, s);
+        // plain form: everything in units of the largest exponent of the tile, constant decays; empty sums have no exponent
+        constexpr int LOG = S == 8 ? 3 : S == 16 ? 4 : 5;
+        const bool none = s.o <= 0.5f * kNegInf, c_none = c.o <= 0.5f * kNegInf;
+        float hi = none ? kNegInf : s.o, lo = none ? -kNegInf : s.o;
+        if (!c_none) { hi = fmaxf(hi, c.o); lo = fminf(lo, c.o); }
 #pragma unroll
-        for (int m = 1; m < S; m <<= 1) {   // inclusive: s covers up to 2 m segments after the step
-            Sum f;
-            f.p = __shfl_up_sync(0xffffffffu, s.p, m, S);
-            f.q = __shfl_up_sync(0xffffffffu, s.q, m, S);
-            f.o = __shfl_up_sync(0xffffffffu, s.o, m, S);
-            const Sum t = after(f, m * lw, s);
-            if (i >= m) s = t;
+        for (int m = 1; m < S; m <<= 1) {
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, m));
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, m));
         }
-        Sum e;                               // exclusive: the state before this segment
-        e.p = __shfl_up_sync(0xffffffffu, s.p, 1, S);
-        e.q = __shfl_up_sync(0xffffffffu, s.q, 1, S);
-        e.o = __shfl_up_sync(0xffffffffu, s.o, 1, S);
-        if (i == 0) e = c;
+        Sum e;                                   // the state before this segment
+        if (__all_sync(0xffffffffu, hi - lo <= kSpan)) {
+            const float f = none ? 0.f : expf(s.o - hi), fc = c_none ? 0.f : expf(c.o - hi);
+            const Sum c1 = {c.p * fc, c.q * fc, hi};
+            s.p *= f; s.q *= f;
+            if (i == 0) { s.p = fmaf(c1.p, decay.d[0], s.p); s.q = fmaf(c1.q, decay.d[0], s.q); }
+#pragma unroll
+            for (int j = 0; j < LOG; ++j) {      // inclusive: s covers up to 2^(j+1) segments after the step
+                const float fp = __shfl_up_sync(0xffffffffu, s.p, 1 << j, S), fq = __shfl_up_sync(0xffffffffu, s.q, 1 << j, S);
+                if (i >= (1 << j)) { s.p = fmaf(fp, decay.d[j], s.p); s.q = fmaf(fq, decay.d[j], s.q); }
+            }
+            s.o = hi;
+            e.p = __shfl_up_sync(0xffffffffu, s.p, 1, S);
+            e.q = __shfl_up_sync(0xffffffffu, s.q, 1, S);
+            e.o = hi;
+            if (i == 0) e = c1;
+        } else {
+            if (i == 0) s = after(c, lw, s);
+#pragma unroll
+            for (int m = 1; m < S; m <<= 1) {
+                Sum f;
+                f.p = __shfl_up_sync(0xffffffffu, s.p, m, S);
+                f.q = __shfl_up_sync(0xffffffffu, s.q, m, S);
+                f.o = __shfl_up_sync(0xffffffffu, s.o, m, S);
+                const Sum t = after(f, m * lw, s);
+                if (i >= m) s = t;
+            }
+            e.p = __shfl_up_sync(0xffffffffu, s.p, 1, S);
+            e.q = __shfl_up_sync(0xffffffffu, s.q, 1, S);
+            e.o = __shfl_up_sync(0xffffffffu, s.o, 1, S);
+            if (i == 0) e = c;
+        }
         __syncwarp();
         buf.x[0][seg][ch] = e.p; buf.x[1][seg][ch] = e.q; buf.x[2][seg][ch] = e.o;
         if (i == S - 1) { buf.carry[0][ch] = s.p; buf.carry[1][ch] = s.q; buf.carry[2][ch] = s.o; }
@@ -104,17 +164,34 @@ __device__ __forceinline__ Place place(int C, int lane) {
     return Place{b, min(c, C - 1), c < C};
 }
 
+// A segment of n tokens from state s in the running-maximum form: y (if y_ is given) and the state behind it.
+__device__ __noinline__ Sum forward_running_max(Sum s, int n, float w, float u, const float* k_, const float* v_, float* y_, int C) {
+    for (int i = 0; i < n; ++i) {
+        const float k = k_[(i64)i * C], v = v_[(i64)i * C];
+        if (y_ != nullptr) {
+            const Pair e = softpair(s.o, u + k);
+            y_[(i64)i * C] = (e.a * s.p + e.b * v) / (e.a * s.q + e.b);
+        }
+        s = after(s, w, Sum{v, 1.f, k});
+    }
+    return s;
+}
+
 template <int S, bool Y>
-__global__ void __launch_bounds__(32 * S) wkv4_forward_kernel(int T, int C, const float* __restrict__ w_, int w_raw, const float* __restrict__ u_,
+__global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_forward_kernel(int T, int C, const float* __restrict__ w_, int w_raw, const float* __restrict__ u_,
                                                               const float* __restrict__ k_, const float* __restrict__ v_,
                                                               float* __restrict__ y_, States st, unsigned* counters) {
     __shared__ ScanBuf<S> buf;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Place at = place(C, lane);
     const i64 off = (i64)at.b * T * C + at.c;
-    const float w = w_raw ? -expf(w_[at.c]) : w_[at.c], u = u_[at.c];
+    const float w = w_raw ? -expf(w_[at.c]) : w_[at.c], u = u_[at.c], ew = expf(w), eu = expf(u);
+    const bool bonus_ok = fabsf(u) <= kBonus;
     if (counters != nullptr && threadIdx.x == 0 && at.b == 0) counters[blockIdx.x] = 0;   // for the backward
     if (warp == 0) { buf.w[lane] = w; buf.carry[0][lane] = 0.f; buf.carry[1][lane] = 0.f; buf.carry[2][lane] = kNegInf; }
+    __syncthreads();
+    SegmentDecay decay;
+    decay.set<S>(buf, warp, lane);
     float kn[L], vn[L];
     auto fetch = [&](int t0) {
 #pragma unroll
@@ -131,31 +208,74 @@ __global__ void __launch_bounds__(32 * S) wkv4_forward_kernel(int T, int C, cons
         for (int i = 0; i < L; ++i) { k[i] = kn[i]; v[i] = vn[i]; }
         fetch(t0 + S * L);   // the next tile's loads are in flight during this tile's math
         const int n = T - t0;
+        Range rg = range_of(k, n);
         Sum s = {0.f, 0.f, kNegInf};
+        float e[L], base = rg.hi;
+        const bool plain = __all_sync(0xffffffffu, bonus_ok && rg.hi - rg.lo <= kSpan);
+        if (plain) {
 #pragma unroll
-        for (int i = 0; i < L; ++i)
-            if (i < n) s = after(s, w, Sum{v[i], 1.f, k[i]});
-        s = scan_segments<S, false>(buf, s, warp, lane);
+            for (int i = 0; i < L; ++i) {
+                e[i] = expf(k[i] - rg.hi);
+                if (i < n) { s.p = fmaf(s.p, ew, e[i] * v[i]); s.q = fmaf(s.q, ew, e[i]); }
+            }
+            if (n > 0) s.o = rg.hi;
+        } else {
+            s = forward_running_max(s, min(n, L), w, u, k_ + off + (i64)t0 * C, v_ + off + (i64)t0 * C, nullptr, C);
+        }
+        s = scan_segments<S, false>(buf, decay, s, warp, lane);
         if (st.p != nullptr && t0 > 0 && n > 0 && at.live) {
             float* p = st.p + at.b * st.row + (t0 / L - 1) * st.seg + at.c;
             p[0] = s.p; p[C] = s.q; p[2 * (i64)C] = s.o;
         }
-        if (Y) {
+        if (Y && plain && __all_sync(0xffffffffu, join(rg, s))) {
+            const float fs = s.q != 0.f ? expf(s.o - rg.hi) : 0.f, fk = expf(base - rg.hi);
+            float p = s.p * fs, q = s.q * fs;
 #pragma unroll
             for (int i = 0; i < L; ++i)
                 if (i < n) {
-                    const Pair e = softpair(s.o, u + k[i]);
-                    if (at.live) y_[off + (i64)(t0 + i) * C] = (e.a * s.p + e.b * v[i]) / (e.a * s.q + e.b);
-                    s = after(s, w, Sum{v[i], 1.f, k[i]});
+                    const float x = e[i] * fk, xu = x * eu;
+                    if (at.live) y_[off + (i64)(t0 + i) * C] = fmaf(xu, v[i], p) / (q + xu);
+                    p = fmaf(p, ew, x * v[i]);
+                    q = fmaf(q, ew, x);
                 }
+        } else if (Y && at.live) {
+            forward_running_max(s, min(n, L), w, u, k_ + off + (i64)t0 * C, v_ + off + (i64)t0 * C, y_ + off + (i64)t0 * C, C);
         }
     }
+}
+
+// A segment of n tokens in reverse in the running-maximum form: gk, gv from its start state and the adjoint G behind it; returns
+// its part of dL/dw.
+__device__ __noinline__ float reverse_running_max(Sum start, Sum G, int n, float w, float u, const float* k_, const float* v_, const float* g_,
+                                                  float* gk_, float* gv_, int C, bool live) {
+    Sum before[L];
+    float ld[L], y[L], A[L], gw = 0.f;
+    for (int i = 0; i < n; ++i) {
+        const float k = k_[(i64)i * C], v = v_[(i64)i * C];
+        before[i] = start;
+        const Pair x = softpair(start.o, u + k);
+        const float den = x.a * start.q + x.b, iden = 1.f / den;
+        y[i] = (x.a * start.p + x.b * v) * iden;
+        ld[i] = x.m + logf(den);
+        A[i] = g_[(i64)i * C] * x.b * iden;
+        start = after(start, w, Sum{v, 1.f, k});
+    }
+    for (int i = n - 1; i >= 0; --i) {
+        const float k = k_[(i64)i * C], v = v_[(i64)i * C], g = g_[(i64)i * C], Bk = expf(k + G.o);
+        gw = fmaf(expf(w + G.o + before[i].o), fmaf(G.p, before[i].p, G.q * before[i].q), gw);
+        if (live) {
+            gk_[(i64)i * C] = A[i] * (v - y[i]) + Bk * fmaf(G.p, v, G.q);
+            gv_[(i64)i * C] = fmaf(Bk, G.p, A[i]);
+        }
+        G = after(G, w, Sum{g, -g * y[i], -ld[i]});
+    }
+    return gw;
 }
 
 // gw, gu: per batch row (row stride gstride), added to when `accumulate`.  With `sum_` (2,C) the last block of a channel group to
 // finish adds the rows up in order (counters[group] counts the others and is left at zero): no launch for it.
 template <int S>
-__global__ void __launch_bounds__(32 * S, 16 / S) wkv4_backward_kernel(int T, int C, const float* __restrict__ w_, int w_raw,
+__global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(int T, int C, const float* __restrict__ w_, int w_raw,
                                                                        const float* __restrict__ u_, const float* __restrict__ k_,
                                                                        const float* __restrict__ v_, const float* __restrict__ gy_,
                                                                        States st, float* __restrict__ gw_, float* __restrict__ gu_,
@@ -165,9 +285,13 @@ __global__ void __launch_bounds__(32 * S, 16 / S) wkv4_backward_kernel(int T, in
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const Place at = place(C, lane);
     const i64 off = (i64)at.b * T * C + at.c;
-    const float w = w_raw ? -expf(w_[at.c]) : w_[at.c], u = u_[at.c];
+    const float w = w_raw ? -expf(w_[at.c]) : w_[at.c], u = u_[at.c], ew = expf(w), eu = expf(u);
+    const bool bonus_ok = fabsf(u) <= kBonus;
     if (warp == 0) { buf.w[lane] = w; buf.carry[0][lane] = 0.f; buf.carry[1][lane] = 0.f; buf.carry[2][lane] = kNegInf; }
-    float gw = 0.f, gu = 0.f;
+    __syncthreads();
+    SegmentDecay decay;
+    decay.set<S>(buf, warp, lane);
+    float gw = 0.f, gw_plain = 0.f, gu = 0.f;   // gw_plain: without the factor e^w
     for (int t0 = (T - 1) / (S * L) * (S * L) + warp * L; t0 >= 0; t0 -= S * L) {
         const int n = T - t0;
         float k[L], v[L], g[L];
@@ -182,39 +306,70 @@ __global__ void __launch_bounds__(32 * S, 16 / S) wkv4_backward_kernel(int T, in
             const float* p = st.p + at.b * st.row + (t0 / L - 1) * st.seg + at.c;
             s = Sum{p[0], p[C], p[2 * (i64)C]};
         }
-        // forward inside the segment: the running sums before each token, y, log den and A
-        Sum before[L];
-        float y[L], A[L], ld[L];
-#pragma unroll
-        for (int i = 0; i < L; ++i) {
-            before[i] = s;
-            const Pair e = softpair(s.o, u + k[i]);
-            const float den = e.a * s.q + e.b, iden = 1.f / den;
-            y[i] = (e.a * s.p + e.b * v[i]) * iden;
-            ld[i] = e.m + logf(den);
-            A[i] = g[i] * e.b * iden;
-            gu = fmaf(A[i], v[i] - y[i], gu);
-            s = after(s, w, Sum{v[i], 1.f, k[i]});
-        }
-        // the adjoint: what the segment adds by itself, then its state from the segments behind it
+        const Sum start = s;
+        Range rg = range_of(k, n);
+        const bool plain = __all_sync(0xffffffffu, bonus_ok && join(rg, s));
+        // forward inside the segment: the running sums before each token, y, and the token's term h (1, -y) of the adjoint (all in
+        // units of the largest weight); then the adjoint that the segment adds by itself
+        float bp[L], bq[L], y[L], h[L], e[L];
         Sum G = {0.f, 0.f, kNegInf};
+        if (plain) {
+            const float fs = s.q != 0.f ? expf(s.o - rg.hi) : 0.f;
+            s.p *= fs; s.q *= fs;
 #pragma unroll
-        for (int i = L - 1; i >= 0; --i)
-            if (i < n) G = after(G, w, Sum{g[i], -g[i] * y[i], -ld[i]});
-        G = scan_segments<S, true>(buf, G, warp, lane);
-#pragma unroll
-        for (int i = L - 1; i >= 0; --i)
-            if (i < n) {
-                const float Bk = expf(k[i] + G.o);
-                gw = fmaf(expf(w + G.o + before[i].o), fmaf(G.p, before[i].p, G.q * before[i].q), gw);
-                if (at.live) {
-                    const i64 o = off + (i64)(t0 + i) * C;
-                    gk_[o] = A[i] * (v[i] - y[i]) + Bk * fmaf(G.p, v[i], G.q);
-                    gv_[o] = fmaf(Bk, G.p, A[i]);
-                }
-                G = after(G, w, Sum{g[i], -g[i] * y[i], -ld[i]});
+            for (int i = 0; i < L; ++i) {
+                e[i] = expf(k[i] - rg.hi);
+                const float xu = e[i] * eu, iden = 1.f / (s.q + xu);
+                bp[i] = s.p; bq[i] = s.q;
+                y[i] = fmaf(xu, v[i], s.p) * iden;
+                h[i] = g[i] * iden;                    // (g is zero where there is no token)
+                gu = fmaf(h[i] * xu, v[i] - y[i], gu);
+                s.p = fmaf(s.p, ew, e[i] * v[i]);
+                s.q = fmaf(s.q, ew, e[i]);
             }
+#pragma unroll
+            for (int i = L - 1; i >= 0; --i)
+                if (i < n) { G.p = fmaf(G.p, ew, h[i]); G.q = fmaf(G.q, ew, -h[i] * y[i]); }
+            if (n > 0) G.o = -rg.hi;
+        } else {
+            // running-maximum form; y and log den are rebuilt by the reverse walk
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+                const Pair x = softpair(s.o, u + k[i]);
+                const float den = x.a * s.q + x.b, iden = 1.f / den;
+                y[i] = (x.a * s.p + x.b * v[i]) * iden;
+                gu = fmaf(g[i] * x.b * iden, v[i] - y[i], gu);
+                h[i] = x.m + logf(den);
+                s = after(s, w, Sum{v[i], 1.f, k[i]});
+            }
+#pragma unroll
+            for (int i = L - 1; i >= 0; --i)
+                if (i < n) G = after(G, w, Sum{g[i], -g[i] * y[i], -h[i]});
+        }
+        G = scan_segments<S, true>(buf, decay, G, warp, lane);
+        const bool empty = G.p == 0.f && G.q == 0.f;
+        if (plain && __all_sync(0xffffffffu, empty || fabsf(G.o + rg.hi) <= kSpan)) {
+            const float f = empty ? 0.f : expf(G.o + rg.hi);
+            float gp = G.p * f, gq = G.q * f;
+#pragma unroll
+            for (int i = L - 1; i >= 0; --i)
+                if (i < n) {
+                    const float A = h[i] * e[i] * eu;
+                    gw_plain = fmaf(gp, bp[i], fmaf(gq, bq[i], gw_plain));
+                    if (at.live) {
+                        const i64 o = off + (i64)(t0 + i) * C;
+                        gk_[o] = fmaf(A, v[i] - y[i], e[i] * fmaf(gp, v[i], gq));
+                        gv_[o] = fmaf(e[i], gp, A);
+                    }
+                    gp = fmaf(gp, ew, h[i]);
+                    gq = fmaf(gq, ew, -h[i] * y[i]);
+                }
+        } else {
+            gw += reverse_running_max(start, G, min(n, L), w, u, k_ + off + (i64)t0 * C, v_ + off + (i64)t0 * C, gy_ + off + (i64)t0 * C,
+                                      gk_ + off + (i64)t0 * C, gv_ + off + (i64)t0 * C, C, at.live);
+        }
     }
+    gw = fmaf(ew, gw_plain, gw);
     __syncthreads();
     buf.x[0][warp][lane] = gw; buf.x[1][warp][lane] = gu;
     __syncthreads();
