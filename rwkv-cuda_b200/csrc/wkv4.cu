@@ -16,7 +16,7 @@
 // are rebuilt inside a segment from its start state, which the forward pass leaves once per segment:
 //   G_{t-1} = e^w G_t + (1, -y_t) gy_t / den_t      gv_t = A_t + e^{k_t} Gp_t     gk_t = A_t (v_t - y_t) + e^{k_t} (Gp_t v_t + Gq_t)
 //   A_t = gy_t e^{u+k_t} / den_t    gu = sum_t A_t (v_t - y_t)    dL/dw = sum_t e^w (Gp_t p_{t-1} + Gq_t q_{t-1})
-// Forward + backward of a training step, B32 T768 C768 on a B200: 1111 us token by token, 294 us here; B4 T256 C256: the two
+// Forward + backward of a training step, B32 T768 C768 on a B200: 1111 us token by token, 294 us with a running maximum in every token, 223 us here; B4 T256 C256: the two
 // kernels took 143 us, the whole step is 75 us now, host side included.
 //
 // Compiled without fast-math: the fp32 tolerance of this operator (1e-5) needs accurate expf.
@@ -51,7 +51,8 @@ __device__ __forceinline__ Sum after(Sum first, float dw, Sum second) {
 // relative to the largest once, e_i = e^{k_i - M}, and the recurrences inside the segment are multiply-adds with the constant
 // e^w: one exponential per token instead of three forward and six backward.  What such a weight loses by underflow (below
 // e^{-87}) is less than 1e-11 of any term that it is added to, because every token's own weight is at least e^{-kSpan - kBonus}.
-// A warp with a lane outside the bounds takes the running-maximum form for that segment.  The scan over segments is the same.
+// A warp with a lane outside the bounds takes the running-maximum form for that segment.
+// (The scan over segments in this form measured no faster: it saves exponentials and needs two more rounds of shuffles.)
 constexpr float kSpan = 40.f, kBonus = 20.f;
 struct Range {
     float lo, hi;
@@ -76,21 +77,10 @@ struct ScanBuf {
     float carry[3][32];
 };
 
-// e^{8 w}, e^{16 w}, ... of the channel that a thread scans (constant for the kernel)
-struct SegmentDecay {
-    float d[5];
-    template <int S>
-    __device__ __forceinline__ void set(const ScanBuf<S>& buf, int warp, int lane) {
-        const float lw = L * buf.w[warp * (32 / S) + lane / S];
-#pragma unroll
-        for (int j = 0; (1 << j) < S; ++j) d[j] = expf(lw * (float)(1 << j));
-    }
-};
-
 // Start states of the S segments of a tile from their local sums and the state carried in from the tile before (in walking
 // order: REV walks the segments from S-1 down).  Called by all warps; leaves the carried state after the tile in `buf`.
 template <int S, bool REV>
-__device__ __forceinline__ Sum scan_segments(ScanBuf<S>& buf, const SegmentDecay& decay, Sum local, int warp, int lane) {
+__device__ __forceinline__ Sum scan_segments(ScanBuf<S>& buf, Sum local, int warp, int lane) {
     buf.x[0][warp][lane] = local.p; buf.x[1][warp][lane] = local.q; buf.x[2][warp][lane] = local.o;
     __syncthreads();
     {   // this thread: channel ch, segment number i in walking order
@@ -98,48 +88,21 @@ __device__ __forceinline__ Sum scan_segments(ScanBuf<S>& buf, const SegmentDecay
         const float lw = L * buf.w[ch];
         Sum s = {buf.x[0][seg][ch], buf.x[1][seg][ch], buf.x[2][seg][ch]};
         const Sum c = {buf.carry[0][ch], buf.carry[1][ch], buf.carry[2][ch]};
-        // plain form: everything in units of the largest exponent of the tile, constant decays; empty sums have no exponent
-        constexpr int LOG = S == 8 ? 3 : S == 16 ? 4 : 5;
-        const bool none = s.o <= 0.5f * kNegInf, c_none = c.o <= 0.5f * kNegInf;
-        float hi = none ? kNegInf : s.o, lo = none ? -kNegInf : s.o;
-        if (!c_none) { hi = fmaxf(hi, c.o); lo = fminf(lo, c.o); }
+        if (i == 0) s = after(c, lw, s);
 #pragma unroll
-        for (int m = 1; m < S; m <<= 1) {
-            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, m));
-            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, m));
+        for (int m = 1; m < S; m <<= 1) {   // inclusive: s covers up to 2 m segments after the step
+            Sum f;
+            f.p = __shfl_up_sync(0xffffffffu, s.p, m, S);
+            f.q = __shfl_up_sync(0xffffffffu, s.q, m, S);
+            f.o = __shfl_up_sync(0xffffffffu, s.o, m, S);
+            const Sum t = after(f, m * lw, s);
+            if (i >= m) s = t;
         }
-        Sum e;                                   // the state before this segment
-        if (__all_sync(0xffffffffu, hi - lo <= kSpan)) {
-            const float f = none ? 0.f : expf(s.o - hi), fc = c_none ? 0.f : expf(c.o - hi);
-            const Sum c1 = {c.p * fc, c.q * fc, hi};
-            s.p *= f; s.q *= f;
-            if (i == 0) { s.p = fmaf(c1.p, decay.d[0], s.p); s.q = fmaf(c1.q, decay.d[0], s.q); }
-#pragma unroll
-            for (int j = 0; j < LOG; ++j) {      // inclusive: s covers up to 2^(j+1) segments after the step
-                const float fp = __shfl_up_sync(0xffffffffu, s.p, 1 << j, S), fq = __shfl_up_sync(0xffffffffu, s.q, 1 << j, S);
-                if (i >= (1 << j)) { s.p = fmaf(fp, decay.d[j], s.p); s.q = fmaf(fq, decay.d[j], s.q); }
-            }
-            s.o = hi;
-            e.p = __shfl_up_sync(0xffffffffu, s.p, 1, S);
-            e.q = __shfl_up_sync(0xffffffffu, s.q, 1, S);
-            e.o = hi;
-            if (i == 0) e = c1;
-        } else {
-            if (i == 0) s = after(c, lw, s);
-#pragma unroll
-            for (int m = 1; m < S; m <<= 1) {
-                Sum f;
-                f.p = __shfl_up_sync(0xffffffffu, s.p, m, S);
-                f.q = __shfl_up_sync(0xffffffffu, s.q, m, S);
-                f.o = __shfl_up_sync(0xffffffffu, s.o, m, S);
-                const Sum t = after(f, m * lw, s);
-                if (i >= m) s = t;
-            }
-            e.p = __shfl_up_sync(0xffffffffu, s.p, 1, S);
-            e.q = __shfl_up_sync(0xffffffffu, s.q, 1, S);
-            e.o = __shfl_up_sync(0xffffffffu, s.o, 1, S);
-            if (i == 0) e = c;
-        }
+        Sum e;                               // exclusive: the state before this segment
+        e.p = __shfl_up_sync(0xffffffffu, s.p, 1, S);
+        e.q = __shfl_up_sync(0xffffffffu, s.q, 1, S);
+        e.o = __shfl_up_sync(0xffffffffu, s.o, 1, S);
+        if (i == 0) e = c;
         __syncwarp();
         buf.x[0][seg][ch] = e.p; buf.x[1][seg][ch] = e.q; buf.x[2][seg][ch] = e.o;
         if (i == S - 1) { buf.carry[0][ch] = s.p; buf.carry[1][ch] = s.q; buf.carry[2][ch] = s.o; }
@@ -178,7 +141,7 @@ __device__ __noinline__ Sum forward_running_max(Sum s, int n, float w, float u, 
 }
 
 template <int S, bool Y>
-__global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_forward_kernel(int T, int C, const float* __restrict__ w_, int w_raw, const float* __restrict__ u_,
+__global__ void __launch_bounds__(32 * S) wkv4_forward_kernel(int T, int C, const float* __restrict__ w_, int w_raw, const float* __restrict__ u_,
                                                               const float* __restrict__ k_, const float* __restrict__ v_,
                                                               float* __restrict__ y_, States st, unsigned* counters) {
     __shared__ ScanBuf<S> buf;
@@ -189,9 +152,6 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_forward_kernel(in
     const bool bonus_ok = fabsf(u) <= kBonus;
     if (counters != nullptr && threadIdx.x == 0 && at.b == 0) counters[blockIdx.x] = 0;   // for the backward
     if (warp == 0) { buf.w[lane] = w; buf.carry[0][lane] = 0.f; buf.carry[1][lane] = 0.f; buf.carry[2][lane] = kNegInf; }
-    __syncthreads();
-    SegmentDecay decay;
-    decay.set<S>(buf, warp, lane);
     float kn[L], vn[L];
     auto fetch = [&](int t0) {
 #pragma unroll
@@ -222,7 +182,7 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_forward_kernel(in
         } else {
             s = forward_running_max(s, min(n, L), w, u, k_ + off + (i64)t0 * C, v_ + off + (i64)t0 * C, nullptr, C);
         }
-        s = scan_segments<S, false>(buf, decay, s, warp, lane);
+        s = scan_segments<S, false>(buf, s, warp, lane);
         if (st.p != nullptr && t0 > 0 && n > 0 && at.live) {
             float* p = st.p + at.b * st.row + (t0 / L - 1) * st.seg + at.c;
             p[0] = s.p; p[C] = s.q; p[2 * (i64)C] = s.o;
@@ -288,9 +248,6 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(i
     const float w = w_raw ? -expf(w_[at.c]) : w_[at.c], u = u_[at.c], ew = expf(w), eu = expf(u);
     const bool bonus_ok = fabsf(u) <= kBonus;
     if (warp == 0) { buf.w[lane] = w; buf.carry[0][lane] = 0.f; buf.carry[1][lane] = 0.f; buf.carry[2][lane] = kNegInf; }
-    __syncthreads();
-    SegmentDecay decay;
-    decay.set<S>(buf, warp, lane);
     float gw = 0.f, gw_plain = 0.f, gu = 0.f;   // gw_plain: without the factor e^w
     for (int t0 = (T - 1) / (S * L) * (S * L) + warp * L; t0 >= 0; t0 -= S * L) {
         const int n = T - t0;
@@ -346,7 +303,7 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(i
             for (int i = L - 1; i >= 0; --i)
                 if (i < n) G = after(G, w, Sum{g[i], -g[i] * y[i], -h[i]});
         }
-        G = scan_segments<S, true>(buf, decay, G, warp, lane);
+        G = scan_segments<S, true>(buf, G, warp, lane);
         const bool empty = G.p == 0.f && G.q == 0.f;
         if (plain && __all_sync(0xffffffffu, empty || fabsf(G.o + rg.hi) <= kSpan)) {
             const float f = empty ? 0.f : expf(G.o + rg.hi);

@@ -526,3 +526,22 @@ def test_wkv7_state_update_decoding_and_prompt(R, dtype, N):
     tol = Hh.tol_for(dtype)
     Hh.assert_close(torch.cat(ys, 1).view(B, T, H * N), y64, tol, "y")
     Hh.assert_close(state, sT64, tol, "state")
+
+
+@pytest.mark.parametrize("spread,mix", [(8.0, False), (30.0, False), (100.0, False), (30.0, True)])
+def test_wkv4_exponents_on_both_sides_of_the_plain_form(R, spread, mix):
+    """Segments whose exponents are close together, far apart, and (mix) both in one sequence; T with a partial segment."""
+    g = Hh.gen(int(spread))
+    B, T, C = 2, 203, 40
+    w_raw, u = Hh.rand(g, C, lo=-4, hi=2), Hh.rand(g, C, lo=-2, hi=2)
+    k, v, gy = Hh.rand(g, B, T, C, lo=-spread, hi=spread), Hh.randn(g, B, T, C), Hh.randn(g, B, T, C)
+    if mix:
+        k[:, ::2] *= 0.02
+        k[:, 64:128] *= 0.02
+    xs = [x.double().requires_grad_(True) for x in (w_raw, u, k, v)]
+    yo = O.wkv4(*xs)
+    yo.backward(gy.double())
+    y, gw, gu, gk, gv = run_wkv4(R, w_raw, u, k, v, gy)
+    for got, want, name in ((y, yo.detach(), "y"), (gw, xs[0].grad, "gw"), (gu, xs[1].grad, "gu"),
+                            (gk, xs[2].grad, "gk"), (gv, xs[3].grad, "gv")):
+        Hh.assert_close(got, want, 2e-5, f"wkv4 {name}")
