@@ -15,7 +15,7 @@
 // the summed |log d| of a chunk stays below 80; beyond that the kernel raises the flag of its (batch, head)
 // unit and the general-shape kernel redoes that unit.
 //
-//   two loader groups, chunks c+2 and c+3:  raw rows by TMA (r, k, v and a per-token decay input), operand preparation;
+//   loader group, chunk c+2:  raw rows by TMA (r, k, v and a per-token decay input), operand preparation;
 //   matrix group, chunk c+1:  [K~;K^] R~^T on the tensor core, A masked into shared memory;
 //   chain group, chunk c:     X = S R~^T, Y = X + V A, S += V K~, y out, S scaled by We.
 #include <cuda.h>
@@ -29,10 +29,10 @@ namespace v6q {
 using namespace v7x;
 
 constexpr int GNT = 128;          // threads per group
-constexpr int PNT = 4 * GNT;
-constexpr int NA = 4;             // operand sets in flight
+constexpr int PNT = 3 * GNT;
+constexpr int NA = 3;             // operand sets in flight
 constexpr int NU = 2;             // A matrices in flight
-constexpr int NS = 2;             // chunks of raw input rows in flight (one per loader group)
+constexpr int NS = 2;             // chunks of raw input rows in flight
 constexpr int kRawStage = 3 * 4096 + 8192;   // r, k, v tiles (bf16) and the decay tile (bf16 or fp32)
 constexpr float kMaxChunkLog2Decay = 80.f * 1.4426950408889634f;
 
@@ -41,7 +41,7 @@ struct Smem {
     static constexpr int kU = NA * kASet;                 // A matrices, swizzled [32][32]
     static constexpr int kWe = kU + NU * HALF32;
     static constexpr int kHs = kWe + NA * 256;
-    static constexpr int kY = kHs + 2 * 1024;                 // bf16 [32][72]
+    static constexpr int kY = kHs + 1024;                 // bf16 [32][72]
     static constexpr int kRaw = (kY + 32 * 72 * 2 + 127) / 128 * 128;
     static constexpr int kOut = (kRaw + NS * kRawStage + 1023) / 1024 * 1024;   // two images of the state on their way out
     static constexpr int kBar = kOut + 2 * ARR64;
@@ -88,7 +88,6 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + kNBar);
     volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* gabort = abort_word + 1;
-    int* strong = const_cast<int*>(abort_word) + 5;   // a chunk's decay was too strong
 
     const int hh = blockIdx.x, bb = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -107,7 +106,7 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
     if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < kNBar; ++i) mbar_init_count(bar + i, (i >= kEmptyA && i < kEmptyA + NA) ? 2 : 1);
-        *abort_word = 0; gabort[0] = 0; gabort[1] = 0; gabort[2] = 0; gabort[3] = 0; *strong = 0;
+        *abort_word = 0; gabort[0] = 0; gabort[1] = 0; gabort[2] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -124,10 +123,9 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
     const int gbar = 1 + grp;
     int fail = 0;
 
-    if (grp == 0 || grp == 3) {
-        // ================================ loader groups: even and odd chunks =================================
-        const int lg = grp == 3;
-        float* Hs = reinterpret_cast<float*>(smem + Smem::kHs + lg * 1024);
+    if (grp == 0) {
+        // ================================ loader group =====================================================
+        float* Hs = reinterpret_cast<float*>(smem + Smem::kHs);
         unsigned char* stg = smem + Smem::kRaw;
         const int j0 = 2 * lane;
         const float u0 = __bfloat162float(u_[hh * 64 + j0]), u1 = __bfloat162float(u_[hh * 64 + j0 + 1]);
@@ -154,10 +152,12 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             }
             issued = c + 1;
         };
-        if (lg < nchunks) issue_raw(lg);
-        int c = lg;
-        for (; c < nchunks; c += 2) {
-            const int valid = min(LC, T - c * LC), st = lg, sa = c % NA, ua = c / NA;
+        issue_raw(0);
+        if (nchunks > 1) issue_raw(1);
+        int sa = 0, ua = 0;
+        int c = 0;
+        for (; c < nchunks; ++c) {
+            const int valid = min(LC, T - c * LC), st = c & 1;
             unsigned char* A = smem + sa * Smem::kASet;
             unsigned char *RT = A, *KK = A + ARR32, *Vs = A + ARR32 + ARR64;
             float* We = reinterpret_cast<float*>(smem + Smem::kWe + sa * 256);
@@ -188,10 +188,10 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
                 }
             }
             if (fail) atomicMax(const_cast<int*>(abort_word), fail);
-            if (gtid == 0) gabort[grp] = *abort_word;
+            if (gtid == 0) gabort[0] = *abort_word;
             group_sync(gbar, GNT);   // (every thread has taken its part of the rows: the stage may be refilled)
-            if (gabort[grp]) break;
-            if (c + 2 < nchunks) issue_raw(c + 2);
+            if (gabort[0]) break;
+            if (c + NS < nchunks) issue_raw(c + NS);
             // cumulative log2 decays: within the warp's 8 tokens, then across the warps
             float cs0[8], cs1[8], run0 = 0.f, run1 = 0.f;
 #pragma unroll
@@ -227,10 +227,15 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             proxy_fence();
             group_sync(gbar, GNT);
             if (gtid == 0) mbar_arrive(bar + kFullA + sa);
+            if (++sa == NA) { sa = 0; ++ua; }
         }
-        if (too_strong) atomicOr(strong, 1);
+        if (wg == 0) {   // a unit with a decay too strong for the chunked form is redone by the general-shape kernel
+            const int any = __any_sync(0xffffffffu, too_strong);
+            if (lane == 0 && flag_div == 0) unsafe_[bb * H + hh] = any;
+            else if (lane == 0 && any) atomicOr(unsafe_ + (((bb / flag_div) * H + hh) & (kChunkedFlagUnits - 1)), 1);
+        }
         if (fail) atomicMax(const_cast<int*>(abort_word), fail);
-        if (c < issued) mbar_wait(bar + kRawFull + lg, (c >> 1) & 1);   // left early: the requested rows must have landed
+        for (int cc = c; cc < issued; ++cc) mbar_wait(bar + kRawFull + (cc & 1), (cc >> 1) & 1);
     } else if (grp == 1) {
         // ================================ matrix group =====================================================
         int sa = 0, ua = 0;
@@ -399,10 +404,6 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
 
     tc_fence_before();
     __syncthreads();
-    if (tid == 0) {   // a unit with a decay too strong for the chunked form is redone by the general-shape kernel
-        if (flag_div == 0) unsafe_[bb * H + hh] = *strong;
-        else if (*strong) atomicOr(unsafe_ + (((bb / flag_div) * H + hh) & (kChunkedFlagUnits - 1)), 1);
-    }
     const int ab = *abort_word;
     if (ab && tid == 0) {   // a wait ran out: record it and poison this unit's outputs
         atomicMax(&g_v6q_error, ab);
