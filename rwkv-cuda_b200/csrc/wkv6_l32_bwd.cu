@@ -228,12 +228,12 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
         tc_fence_before();
         if (__syncthreads_or(fail)) break;
         tc_fence_after();
-        {   // chunk-start state -> S0: the forward has left it in the array's layout
+        {   // chunk-start state -> S0 (swizzled), 16-byte pieces
             const float* s0g = ck + (i64)c * 64 * 64;
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
-                const int idx = q4 * BNT + tid;
-                cp_async16(S0 + idx * 16, s0g + idx * 4);
+                const int idx = q4 * BNT + tid, i = idx >> 4, col = (idx & 15) * 4;
+                cp_async16(S0 + sw(i, col, HALF64), s0g + i * 64 + col);
             }
             cp_async_commit();
         }

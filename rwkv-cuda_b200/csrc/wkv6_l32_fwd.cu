@@ -43,8 +43,7 @@ struct Smem {
     static constexpr int kHs = kWe + NA * 256;
     static constexpr int kY = kHs + 1024;                 // bf16 [32][72]
     static constexpr int kRaw = (kY + 32 * 72 * 2 + 127) / 128 * 128;
-    static constexpr int kOut = (kRaw + NS * kRawStage + 1023) / 1024 * 1024;   // two images of the state on their way out
-    static constexpr int kBar = kOut + 2 * ARR64;
+    static constexpr int kBar = kRaw + NS * kRawStage;
     static constexpr int kBytes = kBar + 256 + 1024;
 };
 static_assert(Smem::kASet % 1024 == 0 && Smem::kU % 1024 == 0 && Smem::kRaw % 128 == 0 && Smem::kBytes <= 232448, "layout");
@@ -99,7 +98,7 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
     const i64 sbase = (i64)(bb * H + hh) * 64 * 64;
     const int nchunks = (T + LC - 1) / LC;
     constexpr bool kPerToken = WMODE < 2;
-    float* ck = ck_ ? ck_ + (i64)(bb * H + hh) * nchunks * 64 * 64 : nullptr;   // chunk-start states for a backward pass, as images of its operand array
+    float* ck = ck_ ? ck_ + (i64)(bb * H + hh) * nchunks * 64 * 64 : nullptr;   // chunk-start states for a backward pass
     const bool states_only = y_ == nullptr;                                  // no y: the pass that only saves the states
     constexpr int kWTile = WMODE == 0 ? 8192 : 4096;
 
@@ -307,7 +306,13 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
                     Sd[nt][e] = s0_kind == 2 ? reinterpret_cast<const float*>(s0_)[idx]
                               : s0_kind == 1 ? __bfloat162float(reinterpret_cast<const bf16*>(s0_)[idx]) : 0.f;
                 }
-            if (ck != nullptr) send_rows(smem + Smem::kOut, 0, reinterpret_cast<unsigned char*>(ck), Sd, row0, lane);
+            if (ck != nullptr) {
+#pragma unroll
+                for (int nt = 0; nt < 8; ++nt) {
+                    *reinterpret_cast<float2*>(ck + (row0 + g) * 64 + nt * 8 + 2 * t) = make_float2(Sd[nt][0], Sd[nt][1]);
+                    *reinterpret_cast<float2*>(ck + (row0 + g + 8) * 64 + nt * 8 + 2 * t) = make_float2(Sd[nt][2], Sd[nt][3]);
+                }
+            }
             tmem_st_tiles<8>(tmS + lane_off, Sd);
             tmem_wait_st();
         }
@@ -372,7 +377,7 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             if (!mbar_wait(bar + kBS, par)) fail = 43;
             tc_fence_after();
             {
-                float* dst = (c + 1 == nchunks && sT_) ? sT_ + sbase : nullptr;
+                float* dst = (c + 1 < nchunks) ? (ck ? ck + (i64)(c + 1) * 64 * 64 : nullptr) : (sT_ ? sT_ + sbase : nullptr);
                 float Sd[8][4];
                 tmem_ld_tiles<8>(Sd, tmS + lane_off);
                 tmem_wait_ld();
@@ -386,8 +391,6 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
                     }
                 }
                 tmem_st_tiles<8>(tmS + lane_off, Sd);
-                if (ck != nullptr && c + 1 < nchunks)
-                    send_rows(smem + Smem::kOut, c + 1, reinterpret_cast<unsigned char*>(ck) + (i64)(c + 1) * ARR64, Sd, row0, lane);
                 tmem_wait_st();
             }
             tc_fence_before();
@@ -398,7 +401,6 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             }
             if (++sa == NA) sa = 0;
         }
-        sent_all(lane);
         if (fail) atomicMax(const_cast<int*>(abort_word), fail);
     }
 
