@@ -49,14 +49,12 @@ struct Smem {
     static constexpr int kBar = kGam + 128;              // 7 mbarriers + tmem slot
     static constexpr int kRaw = kBar + 128;              // the next chunk's inputs as the copy engine delivers them:
                                                          // r, k, v, gy [32][64] bf16 each, then the decay input (bf16 or fp32)
-    static constexpr int kBytes = kRaw + 4 * 4096 + 8192 + 1024;
+    static constexpr int kDv = kRaw + 4 * 4096 + 8192;   // staging rows of gv
+    static constexpr int kBytes = kDv + 4096 + 1024;
     static constexpr int kHs = kAm;                      // [8][64] exchange buffer of the preparation (A, G not yet written)
 };
 static_assert(Smem::kBytes <= 115712 && 8 * 64 * 4 <= 2 * HALF32, "two CTAs per SM");
 
-__device__ __forceinline__ float tf32_seen(const unsigned char* p) {
-    return __uint_as_float(*reinterpret_cast<const uint32_t*>(p) & 0xffffe000u);
-}
 __device__ __forceinline__ void store_state(void* p, int kind, i64 idx, float x) {
     if (kind == 2) reinterpret_cast<float*>(p)[idx] = x;
     else if (kind == 1) reinterpret_cast<bf16*>(p)[idx] = __float2bfloat16_rn(x);
@@ -86,7 +84,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     float* Hs = reinterpret_cast<float*>(smem + Smem::kHs);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + Smem::kBar);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 7);
-    unsigned char* Raw = smem + Smem::kRaw;
+    unsigned char *Raw = smem + Smem::kRaw, *Dv = smem + Smem::kDv;
 
     const int hh = blockIdx.x, bb = blockIdx.y;
     if (flags_ != nullptr && flags_[bb * H + hh] != 0) return;
@@ -325,18 +323,27 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int s = sb + 8 * h, tc = 16 * hs + nt * 8 + 2 * t + e, x = 2 * h + e;
-                        if (quarter < 2) {   // rows k~_s / v_s
-                            if (s != tc) *reinterpret_cast<float*>(Am + sw32(s, tc)) = s < tc ? tf32rf(ua[nt][x]) : 0.f;
-                            *reinterpret_cast<float*>(Gm + sw32(s, tc)) = s < tc ? tf32rf(gg[nt][x]) : 0.f;
-                            if (s == tc) Gam[s] = gg[nt][x];
-                        } else {             // rows k^_s: the diagonal of A
-                            if (s == tc) *reinterpret_cast<float*>(Am + sw32(s, tc)) = tf32rf(ua[nt][x]);
+                for (int h = 0; h < 2; ++h) {
+                    const int s = sb + 8 * h, c0 = 16 * hs + nt * 8 + 2 * t;   // columns c0, c0 + 1
+                    const bool diag = nt == h && hs == (quarter & 1);         // the tile with the diagonal in it
+                    const float a0 = ua[nt][2 * h], a1 = ua[nt][2 * h + 1], g0 = gg[nt][2 * h], g1 = gg[nt][2 * h + 1];
+                    float* am = reinterpret_cast<float*>(Am + sw32(s, c0));
+                    if (quarter < 2) {   // rows k~_s / v_s; the diagonal of A comes from the rows k^_s
+                        const float2 as = make_float2(s < c0 ? tf32rf(a0) : 0.f, s < c0 + 1 ? tf32rf(a1) : 0.f);
+                        if (!diag) {
+                            *reinterpret_cast<float2*>(am) = as;
+                        } else {
+                            if (s != c0) am[0] = as.x;
+                            if (s != c0 + 1) am[1] = as.y;
+                            if (s == c0) Gam[s] = g0;
+                            if (s == c0 + 1) Gam[s] = g1;
                         }
+                        *reinterpret_cast<float2*>(Gm + sw32(s, c0)) = make_float2(s < c0 ? tf32rf(g0) : 0.f, s < c0 + 1 ? tf32rf(g1) : 0.f);
+                    } else if (diag) {
+                        if (s == c0) am[0] = tf32rf(a0);
+                        if (s == c0 + 1) am[1] = tf32rf(a1);
                     }
+                }
         }
         proxy_fence();
         tc_fence_before();
@@ -372,7 +379,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                 mma_ss(tmET, desc_mn(rtA, ks * 8, HALF32), desc_mn(vyA + 32 * 128, ks * 8, HALF64), idesc64(64, 1, 1), 1, lead);
             mma_commit(bar + 3, lead);
         }
-        // ---- 5. dv out: this warp's rows i, tokens 16*hs .. 16*hs+15 -----------------------------------------
+        // ---- 5. dv: this warp's rows i, tokens 16*hs .. 16*hs+15 -----------------------------------------
         if (!mbar_wait(bar + 1, par)) fail = 2;
         tc_fence_after();
         {
@@ -384,7 +391,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int i = row0 + g + ((e & 2) ? 8 : 0), tt = 16 * hs + nt * 8 + 2 * t + (e & 1);
-                    if (tt < valid) gv_[tok0 + (i64)(c * LC + tt) * C + i] = __float2bfloat16_rn(dv[nt][e]);
+                    *reinterpret_cast<bf16*>(Dv + stage_off(tt, i)) = __float2bfloat16_rn(dv[nt][e]);   // staged, sent with gr and gk
                 }
         }
         // ---- 6. the anchor A0[j] = sum_i ET_new[j][i] S0[i][j]; this warp: value columns 32*hs .. 32*hs+31 -----
@@ -396,13 +403,12 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             tmem_wait_ld();
             float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int i = 32 * hs + nt * 8 + 2 * t + e;
-                    acc0 = fmaf(Td[nt][e], *reinterpret_cast<const float*>(S0 + sw(i, row0 + g, HALF64)), acc0);
-                    acc1 = fmaf(Td[nt][2 + e], *reinterpret_cast<const float*>(S0 + sw(i, row0 + g + 8, HALF64)), acc1);
-                }
+            for (int nt = 0; nt < 4; ++nt) {
+                const int i = 32 * hs + nt * 8 + 2 * t;
+                const float2 s0 = f32_pair(S0, i, row0 + g, HALF64, t >> 1), s1 = f32_pair(S0, i, row0 + g + 8, HALF64, t >> 1);
+                acc0 = fmaf(Td[nt][1], s0.y, fmaf(Td[nt][0], s0.x, acc0));
+                acc1 = fmaf(Td[nt][3], s1.y, fmaf(Td[nt][2], s1.x, acc1));
+            }
             acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1); acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
             acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1); acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
             if (t == 0) { A0p[hs * 64 + row0 + g] = acc0; A0p[hs * 64 + row0 + g + 8] = acc1; }
@@ -425,25 +431,31 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
                 float ct[2][2];
+                const int t0 = 16 * hs + nt * 8 + 2 * t;   // this lane's two tokens: t0, t0 + 1
+                const float2 gam = *reinterpret_cast<const float2*>(Gam + t0);
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                for (int h = 0; h < 2; ++h) {
+                    const int j = row0 + g + 8 * h;
+                    const float2 rt2 = tf32_pair(RT, t0, j, HALF32, t >> 1), kt2 = tf32_pair(KK, t0, j, HALF64, t >> 1);
+                    // log2 P of tokens t0 - 1, t0, t0 + 1, and both powers of each
+                    const float lm[3] = {t0 > 0 ? Lam[(t0 - 1) * LAMP + j] : 0.f, Lam[t0 * LAMP + j], Lam[(t0 + 1) * LAMP + j]};
+                    const float wp[3] = {fex2(lm[0]), fex2(lm[1]), fex2(lm[2])}, iw[3] = {fex2(-lm[0]), fex2(-lm[1]), fex2(-lm[2])};
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const int j = row0 + g + 8 * h, tt = 16 * hs + nt * 8 + 2 * t + e, x = 2 * h + e;
-                        const float rt = tf32_seen(RT + sw(tt, j, HALF32)), kt = tf32_seen(KK + sw(tt, j, HALF64));
-                        const float lam = Lam[tt * LAMP + j], lamp = tt > 0 ? Lam[(tt - 1) * LAMP + j] : 0.f;
-                        const float wp = fex2(lamp), iw = fex2(-lam);
-                        const float drs = gR[nt][x] * wp, dks = gK[nt][x] * iw;
-                        const float rr = rt * fex2(-lamp), kr = kt * fex2(lam);   // r_t, k_t
-                        const float gam_u = Gam[tt] * ue[h];
+                        const int tt = t0 + e, x = 2 * h + e;
+                        const float rt = e ? rt2.y : rt2.x, kt = e ? kt2.y : kt2.x, gm = e ? gam.y : gam.x;
+                        const float drs = gR[nt][x] * wp[e], dks = gK[nt][x] * iw[e + 1];
+                        const float rr = rt * iw[e], kr = kt * wp[e + 1];   // r_t, k_t
+                        const float gam_u = gm * ue[h];
                         const float rdr = rt * gR[nt][x];
                         ct[h][e] = rdr - kt * gK[nt][x];
                         gl[h][nt][e] = rdr;
-                        lw[h][nt][e] = (lam - lamp) * 0.6931471805599453f;   // log w_t
-                        gu_acc[h] = fmaf(Gam[tt], rr * kr, gu_acc[h]);
+                        lw[h][nt][e] = (lm[e + 1] - lm[e]) * 0.6931471805599453f;   // log w_t
+                        gu_acc[h] = fmaf(gm, rr * kr, gu_acc[h]);
                         stg[0][tt * 72 + j] = __float2bfloat16_rn(fmaf(gam_u, kr, drs));
                         stg[1][tt * 72 + j] = __float2bfloat16_rn(fmaf(gam_u, rr, dks));
                     }
+                }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {   // exclusive prefix over the tokens of this tile (token = 2*t + e over a quad)
                     const float pair = ct[h][0] + ct[h][1];
@@ -484,6 +496,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                 *reinterpret_cast<uint4*>(gk_ + o) = *reinterpret_cast<const uint4*>(stg[1] + tt * 72 + piece * 8);
             }
         }
+        stage_flush(Dv, gv_, tok0 + (i64)c * LC * C, C, tid, valid);
         if (!kStatic) {
             __syncthreads();
             const int tt = tid >> 3, piece = tid & 7;

@@ -61,6 +61,25 @@ __device__ __forceinline__ int sw(int row, int col, int half) {
 // the same for a [.][32] array (one half)
 __device__ __forceinline__ int sw32(int row, int col) { return row * 128 + ((((col >> 3) & 3) ^ (row & 3)) << 5) + (col & 7) * 4; }
 
+// Accumulator tiles give a lane of a quad the rows 2t and 2t + 1 (t = lane % 4) of an operand array at one column.
+// Taken in that order the four lanes meet in two of the four 32-byte pieces (row & 3 is 0, 2, 0, 2): every access
+// takes two passes.  Lanes 2 and 3 therefore take the odd row first (row & 3 is then 0, 2, 1, 3) and the words
+// change places in registers.  `row` is the even row, `flip` = t >> 1; the value is the one the tensor core used.
+__device__ __forceinline__ float2 tf32_pair(const unsigned char* arr, int row, int col, int half, int flip) {
+    const uint32_t a = *reinterpret_cast<const uint32_t*>(arr + sw(row + flip, col, half)) & 0xffffe000u;
+    const uint32_t b = *reinterpret_cast<const uint32_t*>(arr + sw(row + 1 - flip, col, half)) & 0xffffe000u;
+    return make_float2(__uint_as_float(flip ? b : a), __uint_as_float(flip ? a : b));
+}
+__device__ __forceinline__ float2 f32_pair(const unsigned char* arr, int row, int col, int half, int flip) {
+    const float a = *reinterpret_cast<const float*>(arr + sw(row + flip, col, half));
+    const float b = *reinterpret_cast<const float*>(arr + sw(row + 1 - flip, col, half));
+    return make_float2(flip ? b : a, flip ? a : b);
+}
+__device__ __forceinline__ void put_pair(unsigned char* arr, int row, int col, int half, int flip, float x0, float x1) {
+    *reinterpret_cast<float*>(arr + sw(row + flip, col, half)) = flip ? x1 : x0;
+    *reinterpret_cast<float*>(arr + sw(row + 1 - flip, col, half)) = flip ? x0 : x1;
+}
+
 __device__ __forceinline__ uint64_t desc_sw(uint32_t saddr, uint32_t lbo_bytes) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFF) >> 4);

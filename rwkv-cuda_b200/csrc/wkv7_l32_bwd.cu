@@ -89,9 +89,6 @@ __device__ __forceinline__ void scatter_u_half(const float (*u)[4], int quarter,
         }
 }
 
-__device__ __forceinline__ float tf32_seen(const unsigned char* p) {   // operand word -> the value the tensor core used
-    return __uint_as_float(*reinterpret_cast<const uint32_t*>(p) & 0xffffe000u);
-}
 
 __global__ void __launch_bounds__(BNT, 2)
 wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __restrict__ w_,
@@ -307,10 +304,8 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int i = row0 + g + ((e & 2) ? 8 : 0), tt = 16 * hs + nt * 8 + 2 * t + (e & 1);
-                    *reinterpret_cast<float*>(SV + sw(tt, i, HALF64)) = tf32rf(sa[nt][e]);
-                }
+                for (int h = 0; h < 2; ++h)
+                    put_pair(SV, 16 * hs + nt * 8 + 2 * t, row0 + g + 8 * h, HALF64, t >> 1, tf32rf(sa[nt][2 * h]), tf32rf(sa[nt][2 * h + 1]));
         }
         proxy_fence();
         tc_fence_before();
@@ -349,13 +344,16 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             tmem_ld_tiles<2>(dv, tmW1 + 32 + 16 * hs + lane_off);
             tmem_wait_ld();
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
+            for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    put_pair(EY, 16 * hs + nt * 8 + 2 * t, row0 + g + 8 * h, HALF64, t >> 1, tf32rf(ev[nt][2 * h]), tf32rf(ev[nt][2 * h + 1]));
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int i = row0 + g + ((e & 2) ? 8 : 0), tt = 16 * hs + nt * 8 + 2 * t + (e & 1);
-                    *reinterpret_cast<float*>(EY + sw(tt, i, HALF64)) = tf32rf(ev[nt][e]);
                     *reinterpret_cast<bf16*>(N1 + stage_off(tt, i)) = __float2bfloat16_rn(dv[nt][e]);   // N1 is dead: staged, sent with the others
                 }
+            }
         }
         proxy_fence();
         tc_fence_before();
@@ -426,13 +424,12 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             tmem_wait_ld();
             float acc0 = 0.f, acc1 = 0.f;
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int i = 32 * hs + nt * 8 + 2 * t + e;
-                    acc0 = fmaf(Td[nt][e], *reinterpret_cast<const float*>(S0 + sw(i, row0 + g, HALF64)), acc0);
-                    acc1 = fmaf(Td[nt][2 + e], *reinterpret_cast<const float*>(S0 + sw(i, row0 + g + 8, HALF64)), acc1);
-                }
+            for (int nt = 0; nt < 4; ++nt) {
+                const int i = 32 * hs + nt * 8 + 2 * t;
+                const float2 s0 = f32_pair(S0, i, row0 + g, HALF64, t >> 1), s1 = f32_pair(S0, i, row0 + g + 8, HALF64, t >> 1);
+                acc0 = fmaf(Td[nt][1], s0.y, fmaf(Td[nt][0], s0.x, acc0));
+                acc1 = fmaf(Td[nt][3], s1.y, fmaf(Td[nt][2], s1.x, acc1));
+            }
             acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1); acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
             acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1); acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
             if (t == 0) { A0p[hs * 64 + row0 + g] = acc0; A0p[hs * 64 + row0 + g + 8] = acc1; }
@@ -459,25 +456,30 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
                 float ct[2][2];
+                const int t0 = 16 * hs + nt * 8 + 2 * t;   // this lane's two tokens: t0, t0 + 1
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                for (int h = 0; h < 2; ++h) {
+                    const int j = row0 + g + 8 * h;
+                    const float2 at = tf32_pair(AR, t0, j, HALF64, t >> 1), rt = tf32_pair(AR, 32 + t0, j, HALF64, t >> 1);
+                    const float2 bt = tf32_pair(BK, t0, j, HALF64, t >> 1), kt = tf32_pair(BK, 32 + t0, j, HALF64, t >> 1);
+                    // cumulative log2 decays of tokens t0 - 1, t0, t0 + 1
+                    const float lm[3] = {t0 > 0 ? Lam[(t0 - 1) * LAMP + j] : 0.f, Lam[t0 * LAMP + j], Lam[(t0 + 1) * LAMP + j]};
+                    const float wt[3] = {fex2(lm[0]), fex2(lm[1]), fex2(lm[2])};
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const int j = row0 + g + 8 * h, tt = 16 * hs + nt * 8 + 2 * t + e, x = 2 * h + e;
-                        const float at = tf32_seen(AR + sw(tt, j, HALF64)), rt = tf32_seen(AR + sw(32 + tt, j, HALF64));
-                        const float bt = tf32_seen(BK + sw(tt, j, HALF64)), kt = tf32_seen(BK + sw(32 + tt, j, HALF64));
-                        const float ada = at * gA[nt][x];
-                        ct[h][e] = rt * gR[nt][x] + ada - bt * gB[nt][x] - kt * gK[nt][x];
+                        const int tt = t0 + e, x = 2 * h + e;
+                        const float ada = (e ? at.y : at.x) * gA[nt][x];
+                        ct[h][e] = (e ? rt.y : rt.x) * gR[nt][x] + ada - (e ? bt.y : bt.x) * gB[nt][x] - (e ? kt.y : kt.x) * gK[nt][x];
                         gl[h][nt][e] = ada;
-                        const float lam = Lam[tt * LAMP + j], lamp = tt > 0 ? Lam[(tt - 1) * LAMP + j] : 0.f;
-                        const float wt = fex2(lam), iw = fex2(-lam), wp = fex2(lamp);
-                        const float sg = (lam - lamp) * (1.f / kWScale2);
+                        const float iw = fex2(-lm[e + 1]);
+                        const float sg = (lm[e + 1] - lm[e]) * (1.f / kWScale2);
                         fw[h][nt][e] = kWScale * sg * (1.f - sg);
-                        stg[0][tt * 72 + j] = __float2bfloat16_rn(gR[nt][x] * wt);
-                        stg[1][tt * 72 + j] = __float2bfloat16_rn(gA[nt][x] * wp);
+                        stg[0][tt * 72 + j] = __float2bfloat16_rn(gR[nt][x] * wt[e + 1]);
+                        stg[1][tt * 72 + j] = __float2bfloat16_rn(gA[nt][x] * wt[e]);
                         stg[2][tt * 72 + j] = __float2bfloat16_rn(gK[nt][x] * iw);
                         stg[3][tt * 72 + j] = __float2bfloat16_rn(gB[nt][x] * iw);
                     }
+                }
                 // exclusive prefix over the tokens of this tile (token = 2*t + e across the four lanes of a quad)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
