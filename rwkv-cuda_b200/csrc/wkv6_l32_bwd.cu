@@ -226,14 +226,9 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
         tc_fence_before();
         if (__syncthreads_or(fail)) break;
         tc_fence_after();
-        {   // chunk-start state -> S0 (swizzled), 16-byte pieces
-            const float* s0g = ck + (i64)c * 64 * 64;
-#pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {
-                const int idx = q4 * BNT + tid, i = idx >> 4, col = (idx & 15) * 4;
-                cp_async16(S0 + sw(i, col, HALF64), s0g + i * 64 + col);
-            }
-            cp_async_commit();
+        if (tid == 224) {   // chunk-start state -> S0: the forward has left it in the array's layout
+            mbar_expect_bytes(bar + 5, ARR64);
+            bulk_load(S0, ck + (i64)c * 64 * 64, ARR64, bar + 5);
         }
         // ---- 1. operands: this thread has channels j0, j0+1 of tokens 4*warp .. 4*warp+3 ----------------
         if (staged) {
@@ -277,7 +272,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                 lp0 = base0 + cs0[q]; lp1 = base1 + cs1[q];
             }
         }
-        cp_async_wait<0>();
+        if (!mbar_wait(bar + 5, par)) fail = 7;   // the state
         proxy_fence();
         tc_fence_before();
         __syncthreads();

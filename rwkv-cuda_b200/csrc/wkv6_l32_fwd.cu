@@ -26,8 +26,9 @@
 //   chain warp, chunk c:      X = S^ R~^T, Y = X + V A, S^ += V K~, nothing but products;
 //   output warps, chunk c:    y out;
 //   state warps, chunk c+1:   the state at its start out (for a backward pass), S^ scaled where it has to be.
-// What bounded the form with one chain group that also wrote y and scaled the state (1248 us, B16 T4096 H64) was that
-// group: neither faster stores nor a second loader group changed it.
+// B16 T4096 H64, states saved: one chain group that also wrote y and scaled the state 1248 us (2700 cycles a chunk, whatever
+// the stores and loaders did); these roles with one loader group 1330, two loader groups 1140; the states through shared
+// memory and bulk copies 988 (16 stores of 8 bytes per thread were a third of the shared-memory pipe, which was 75 % busy).
 #include <cuda.h>
 
 #include "wkv7_l32.cuh"
@@ -43,12 +44,13 @@ constexpr int LTPW = 8;           // tokens of a loader warp
 constexpr int PNT = 5 * GNT + 32;
 constexpr int NA = 3;             // operand sets in flight
 constexpr int NU = 2;             // A matrices in flight
-constexpr int NS = 4;             // chunks of raw input rows in flight, two per loader group
-constexpr int kRawStage = 3 * 4096 + 8192;   // r, k, v tiles (bf16) and the decay tile (bf16 or fp32)
 constexpr float kMaxChunkLog2Decay = 80.f * 1.4426950408889634f;
 constexpr float kRenormLog2 = -60.f;
 
+template <int WMODE>
 struct Smem {
+    static constexpr int NS = WMODE == 0 ? 2 : 4;          // chunks of raw input rows in flight, half of them per loader group
+    static constexpr int kRawStage = 3 * 4096 + (WMODE == 0 ? 8192 : WMODE == 1 ? 4096 : 0);   // r, k, v tiles (bf16), the decay tile (bf16 or fp32)
     static constexpr int kASet = ARR32 + ARR64 + ARR32;   // R~ [32][64], K~ and K^ [64][64] in turns of 8 rows, V [32][64]
     static constexpr int kU = NA * kASet;                 // A matrices, swizzled [32][32]
     static constexpr int kWe = kU + NU * HALF32;          // per set: [64] S^ -> state, [64] what scales S^; then [64] of the end
@@ -56,10 +58,12 @@ struct Smem {
     static constexpr int kB = kHs + 4 * 1024;             // per group [64]: log2 D at the end of its chunk
     static constexpr int kY = kB + 512;                   // two staging tiles of y
     static constexpr int kRaw = (kY + 2 * 4096 + 127) / 128 * 128;
-    static constexpr int kBar = kRaw + NS * kRawStage;
+    static constexpr int kOut = (kRaw + NS * kRawStage + 1023) / 1024 * 1024;   // two images of the state on their way out
+    static constexpr int kBar = kOut + 2 * ARR64;
     static constexpr int kBytes = kBar + 512 + 1024;
 };
-static_assert(Smem::kASet % 1024 == 0 && Smem::kU % 1024 == 0 && Smem::kRaw % 128 == 0 && Smem::kBytes <= 232448, "layout");
+static_assert(Smem<0>::kASet % 1024 == 0 && Smem<0>::kU % 1024 == 0 && Smem<0>::kRaw % 128 == 0, "layout");
+static_assert(Smem<0>::kBytes <= 232448 && Smem<1>::kBytes <= 232448, "one block per SM");
 
 __device__ int g_v6q_error = 0;
 
@@ -85,7 +89,7 @@ struct Maps {
 
 // arrivals: kFullA one per loader warp; kEmptyA the matrix group, the state warps and the product S^ += V K~
 enum { kFullA = 0, kEmptyA = kFullA + NA, kFullU = kEmptyA + NA, kEmptyU = kFullU + NU, kFU = kEmptyU + NU, kBX, kBS, kState,
-       kD, kBY = kD + 2, kYTaken = kBY + 2, kRawFull = kYTaken + 2, kNBar = kRawFull + NS };
+       kD, kBY = kD + 2, kYTaken = kBY + 2, kRawFull = kYTaken + 2, kNBar = kRawFull + 4 };
 static_assert(8 * kNBar + 4 + 4 * (9 + NA) <= 512, "barrier space");
 
 // WMODE: 0 = fp32 log-decay (B,T,C), 1 = bf16 raw input (B,T,C) with log-decay = -exp(w), 2 = fp32 decay value (C),
@@ -95,6 +99,8 @@ __global__ void __launch_bounds__(PNT, 1)
 wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void* __restrict__ wstat_, const bf16* __restrict__ u_,
                      const void* __restrict__ s0_, int s0_kind, bf16* __restrict__ y_, float* __restrict__ sT_,
                      float* __restrict__ ck_, int* __restrict__ unsafe_, int flag_div) {
+    using Smem = v6q::Smem<WMODE>;
+    constexpr int NS = Smem::NS, kRawStage = Smem::kRawStage;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + Smem::kBar);
@@ -112,7 +118,7 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
     const i64 sbase = (i64)(bb * H + hh) * 64 * 64;
     const int nchunks = (T + LC - 1) / LC;
     constexpr bool kPerToken = WMODE < 2;
-    float* ck = ck_ ? ck_ + (i64)(bb * H + hh) * nchunks * 64 * 64 : nullptr;   // chunk-start states for a backward pass
+    float* ck = ck_ ? ck_ + (i64)(bb * H + hh) * nchunks * 64 * 64 : nullptr;   // chunk-start states for a backward pass, as images of its operand array
     const bool states_only = y_ == nullptr;                                  // no y: the pass that only saves the states
     constexpr int kWTile = WMODE == 0 ? 8192 : 4096;
 
@@ -358,13 +364,6 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
                 Sd[nt][0] *= x.x; Sd[nt][1] *= x.y; Sd[nt][2] *= x.x; Sd[nt][3] *= x.y;
             }
         };
-        auto send = [&](float* dst) {
-#pragma unroll
-            for (int nt = 0; nt < 8; ++nt) {
-                *reinterpret_cast<float2*>(dst + (row0 + g) * 64 + nt * 8 + 2 * t) = make_float2(Sd[nt][0], Sd[nt][1]);
-                *reinterpret_cast<float2*>(dst + (row0 + g + 8) * 64 + nt * 8 + 2 * t) = make_float2(Sd[nt][2], Sd[nt][3]);
-            }
-        };
         int sa = 0, ua = 0, c = 0;
         for (; c < nchunks; ++c) {   // the state at the start of chunk c
             if (c > 0 && !mbar_wait(bar + kBS, (c - 1) & 1)) fail = 43;
@@ -387,7 +386,7 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             if (lane == 0) mbar_arrive(bar + kState);   // the state may be read (scaled) and written (taken)
             if (ck != nullptr) {
                 if (!again) scale(Wc);
-                send(ck + (i64)c * 64 * 64);
+                send_rows(smem + Smem::kOut, c, reinterpret_cast<unsigned char*>(ck) + (i64)c * ARR64, Sd, row0, lane);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar + kEmptyA + sa);
@@ -400,9 +399,15 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
                 tmem_ld_tiles<8>(Sd, tmS + lane_off);
                 tmem_wait_ld();
                 scale(reinterpret_cast<const float*>(smem + Smem::kWe + NA * 512));
-                send(sT_ + sbase);
+                float* dst = sT_ + sbase;
+#pragma unroll
+                for (int nt = 0; nt < 8; ++nt) {
+                    *reinterpret_cast<float2*>(dst + (row0 + g) * 64 + nt * 8 + 2 * t) = make_float2(Sd[nt][0], Sd[nt][1]);
+                    *reinterpret_cast<float2*>(dst + (row0 + g + 8) * 64 + nt * 8 + 2 * t) = make_float2(Sd[nt][2], Sd[nt][3]);
+                }
             }
         }
+        sent_all(lane);
         if (fail) atomicMax(const_cast<int*>(abort_word), fail);
     } else {
         // ================================ chain warp =======================================================
@@ -514,9 +519,9 @@ int wkv6_l32_forward(int B, int T, int H, const void* r, const void* k, const vo
     dim3 grid(H, B);
 #define RWKV_GO(M)                                                                                                       \
     do {                                                                                                                 \
-        cudaError_t e = allow_smem<wkv6q_forward_kernel<M>>(Smem::kBytes); \
+        cudaError_t e = allow_smem<wkv6q_forward_kernel<M>>(Smem<M>::kBytes); \
         RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv6_forward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));  \
-        wkv6q_forward_kernel<M><<<grid, PNT, Smem::kBytes, st>>>(T, H, maps, w, (const bf16*)u, s0, s0_kind, (bf16*)y, sT, \
+        wkv6q_forward_kernel<M><<<grid, PNT, Smem<M>::kBytes, st>>>(T, H, maps, w, (const bf16*)u, s0, s0_kind, (bf16*)y, sT, \
                                                                 ck, unsafe, flag_div);                                       \
     } while (0)
     switch (w_mode) {

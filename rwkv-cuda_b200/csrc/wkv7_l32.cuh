@@ -186,6 +186,35 @@ __device__ __forceinline__ void stage_flush(const unsigned char* stage, bf16* ou
             *reinterpret_cast<const uint4*>(stage + tt * 128 + ((piece ^ (tt & 7)) << 4));
 }
 
+// A warp's 16 rows of a state (accumulator fragments) -> the n-th image that it sends, 16 KB in the swizzled layout of a [64][64]
+// operand array: 16 stores of 8 bytes per thread straight to device memory took longer than the products they ran beside, so
+// the rows go through shared memory (two buffers of 16 KB in turn) and leave as two bulk copies of 2 KB.
+__device__ __forceinline__ void send_rows(unsigned char* smem_out, int n, unsigned char* image, const float (&x)[8][4], int row0, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+    unsigned char* buf = smem_out + (n & 1) * ARR64;
+    if (n >= 2) {   // the copies that left this buffer before have read it
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+    }
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+        *reinterpret_cast<float2*>(buf + sw(row0 + g, nt * 8 + 2 * t, HALF64)) = make_float2(x[nt][0], x[nt][1]);
+        *reinterpret_cast<float2*>(buf + sw(row0 + g + 8, nt * 8 + 2 * t, HALF64)) = make_float2(x[nt][2], x[nt][3]);
+    }
+    proxy_fence();
+    __syncwarp();
+    if (lane == 0) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(__cvta_generic_to_global(image + h * HALF64 + row0 * 128)),
+                         "r"(smem_u32(buf + h * HALF64 + row0 * 128)), "r"(16 * 128) : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+}
+__device__ __forceinline__ void sent_all(int lane) {   // before the block ends
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 // ---- the part of a chunk that does not depend on the carried state ---------------------------------
 // Raw inputs of one chunk as loaded by a thread: channels (2*lane, 2*lane+1) of TPW consecutive tokens
 // (token index inside the chunk = TPW*warp + q).  NX tensors: r w k v a b [dy].
@@ -228,6 +257,12 @@ __device__ __forceinline__ void tma_tile_load(void* dst_smem, const CUtensorMap*
 }
 __device__ __forceinline__ void mbar_expect_bytes(uint64_t* bar, int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// contiguous bytes (a multiple of 16, both ends 16-byte aligned) -> shared memory by the copy engine, counted on the mbarrier
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
 }
 __device__ __forceinline__ void l2_prefetch_tile(const CUtensorMap* map, int x, int y) {
     asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y)

@@ -52,13 +52,6 @@ __device__ __forceinline__ void put_operand(uint32_t taddr, const float (&x)[8][
     tmem_st_tiles<8>(taddr, q);
     tmem_wait_st();
 }
-// whole record (a multiple of 16 bytes) -> shared memory by the copy engine, counted on the mbarrier
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, int bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-                 "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
 // ---- (1) the operators of a chunk ------------------------------------------------------------------------------
 // Blocks walk over the chunks of all units (two blocks per SM); the tiles of a block's next chunk are on their way while it
 // works on this one.
@@ -255,35 +248,6 @@ enum { kFull = 0, kEmpty = kFull + NSTG, kOper = kEmpty + NSTG, kState = kOper +
 __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
     __syncwarp();
     if (lane == 0) mbar_arrive(bar);
-}
-
-// A warp's 16 rows of S (or E) -> image `n` of a chunk in device memory, in the swizzled layout of an operand array: 16 stores of 8
-// bytes straight to device memory took longer than the products they ran beside, so the rows go through shared memory (two
-// buffers in turn) and leave as two bulk copies of 2 KB.
-__device__ __forceinline__ void send_rows(unsigned char* smem_out, int n, unsigned char* image, const float (&x)[8][4], int row0, int lane) {
-    const int g = lane >> 2, t = lane & 3;
-    unsigned char* buf = smem_out + (n & 1) * ARR64;
-    if (n >= 2) {   // the copies that left this buffer before have read it
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        __syncwarp();
-    }
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-        *reinterpret_cast<float2*>(buf + sw(row0 + g, nt * 8 + 2 * t, HALF64)) = make_float2(x[nt][0], x[nt][1]);
-        *reinterpret_cast<float2*>(buf + sw(row0 + g + 8, nt * 8 + 2 * t, HALF64)) = make_float2(x[nt][2], x[nt][3]);
-    }
-    proxy_fence();
-    __syncwarp();
-    if (lane == 0) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(__cvta_generic_to_global(image + h * HALF64 + row0 * 128)),
-                         "r"(smem_u32(buf + h * HALF64 + row0 * 128)), "r"(16 * 128) : "memory");
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    }
-}
-__device__ __forceinline__ void sent_all(int lane) {   // before the block ends
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // Forward: warps 0-3 carry S in fp32 registers (16 value rows each) and write the states and sT; warps 4-7 write y; warp 8 issues
