@@ -245,6 +245,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                 run0 += l0; run1 += l1; cs0[q] = run0; cs1[q] = run1;
             }
             *reinterpret_cast<float2*>(Hs + warp * 64 + j0) = make_float2(run0, run1);
+            if (staged) proxy_fence();   // (the words are still on their way to the registers: the copy engine must not be quicker)
             __syncthreads();
             if (staged && c > 0) { request(c - 1); pending = true; }   // every thread has taken its words: the stage is free
             float base0 = 0.f, base1 = 0.f, tot0 = 0.f, tot1 = 0.f;

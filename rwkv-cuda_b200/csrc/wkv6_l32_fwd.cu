@@ -215,6 +215,7 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             if (ua >= 1 && !mbar_wait(bar + kEmptyA + sa, (ua - 1) & 1)) fail = 30;
             if (fail) atomicMax(const_cast<int*>(abort_word), fail);
             if (wg == 0 && lane == 0) gabort[lg] = *abort_word;
+            proxy_fence();   // (the words are still on their way to the registers: the copy engine must not be quicker)
             group_sync(1 + lg, GNT);   // the warps' sums; every thread has taken its part of the rows, the stage may be refilled
             if (gabort[lg]) break;
             if (c + NS < nchunks) issue_raw(c + NS);

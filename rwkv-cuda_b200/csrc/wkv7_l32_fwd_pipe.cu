@@ -171,6 +171,7 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             PIPE_MARK(3);
             if (fail) atomicMax(const_cast<int*>(abort_word), fail);
             if (gtid == 0) gabort[0] = *abort_word;
+            proxy_fence();   // (the words are still on their way to the registers: the copy engine must not be quicker)
             group_sync(gbar, GNT);
             if (gtid == 0) mbar_arrive(bar + kTaken + st);   // every thread has taken its part of the rows: the stage may be refilled
             if (gabort[0]) break;
