@@ -59,7 +59,8 @@ struct PipeSmem {
     static constexpr int kUab = kHs + 1024;             // plain [32][UPITCH], scratch of the matrix group
     static constexpr int kY = kUab + 32 * UPITCH * 4;   // bf16 [32][72]
     static constexpr int kRaw = (kY + 32 * 72 * 2 + 127) / 128 * 128;   // raw input rows: [NS][6 tensors][32 tokens][64 bf16]
-    static constexpr int kBar = kRaw + NS * 6 * 32 * 128;         // mbarriers, tmem slot, abort words
+    static constexpr int kOut = (kRaw + NS * 6 * 32 * 128 + 1023) / 1024 * 1024;   // a quarter of the state on its way out (see send_state)
+    static constexpr int kBar = kOut + HALF32;                    // mbarriers, tmem slot, abort words
     static constexpr int kBytes = kBar + 256 + 1024;
 };
 static_assert(PipeSmem::kASet % 1024 == 0 && PipeSmem::kUSet % 1024 == 0 && PipeSmem::kBytes <= 232448, "layout");
@@ -81,7 +82,8 @@ __device__ __forceinline__ void tma_tile(void* dst_smem, const CUtensorMap* map,
                  : "memory");
 }
 struct InputMaps {
-    CUtensorMap m[6];   // r, w, k, v, a, b as (B*T, C) bf16, box 64 x 32
+    CUtensorMap m[6];    // r, w, k, v, a, b as (B*T, C) bf16, box 64 x 32
+    CUtensorMap state;   // the saved states as (B*H*T/16*64, 64) fp32 (see make_state_map)
 };
 __device__ __forceinline__ void mbar_init_count(uint64_t* bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
@@ -117,7 +119,7 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
 
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < kNBar; ++i) mbar_init_count(bar + i, (i >= kEmptyA && i < kEmptyA + NA) ? 2 : 1);
+        for (int i = 0; i < kNBar; ++i) mbar_init_count(bar + i, (i >= kEmptyA && i < kEmptyA + NA) ? 2 : (i >= kEmptyU && i < kEmptyU + NU) ? 4 : 1);
         *abort_word = 0; gabort[0] = 0; gabort[1] = 0; gabort[2] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -196,7 +198,6 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             unsigned char *Uak = U, *Ubr = U + HALF32, *Ukr = U + 2 * HALF32, *D0 = U + 3 * HALF32, *N1 = U + 4 * HALF32;
             PIPE_MARK(4);
             if (!mbar_wait(bar + kFullA + sa, ua & 1)) fail = 35;                              // operands of this chunk
-            if (c >= NU && !mbar_wait(bar + kEmptyU + su, ((c >> 1) - 1) & 1)) fail = 36;      // the chain group released this matrix set
             PIPE_MARK(0);
             if (fail) atomicMax(const_cast<int*>(abort_word), fail);
             if (gtid == 0) gabort[1] = *abort_word;
@@ -211,6 +212,7 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             if (!mbar_wait(bar + kFU, par)) fail = 37;
             tc_fence_after();
             if (gtid == 0) mbar_arrive(bar + kEmptyA + sa);   // this group is done with the operand set
+            if (c >= NU && !mbar_wait(bar + kEmptyU + su, ((c >> 1) - 1) & 1)) fail = 36;      // the chain group released this matrix set
             PIPE_MARK(1);
             {
                 float u[8][4];
@@ -270,6 +272,28 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             tmem_st_tiles<8>(tmS + lane_off, Sd);
             tmem_wait_st();
         }
+        // This warp's 16 rows of the state -> start state `row` / 64 of the saved ones.  16 stores of 8 bytes per thread straight
+        // to device memory kept the load/store data pipe, which all groups need, busy for 512 of 3700 cycles; so the rows go
+        // through shared memory and leave as two tiles of 2 KB.  There is no room for a buffer of 16 KB: U_ak, U_br
+        // and U_kr of this chunk are dead by now and take three quarters.  Their set is released when the copies have read it.
+        auto send_state = [&](const float (&x)[8][4], unsigned char* U, int row) {
+            unsigned char* half[2] = {U + row0 * 128, (wg < 2 ? U + 2 * HALF32 : smem + PipeSmem::kOut) + (row0 & 31) * 128};
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt) {
+                *reinterpret_cast<float2*>(half[nt >> 2] + sw32(g, (nt & 3) * 8 + 2 * t)) = make_float2(x[nt][0], x[nt][1]);
+                *reinterpret_cast<float2*>(half[nt >> 2] + sw32(g + 8, (nt & 3) * 8 + 2 * t)) = make_float2(x[nt][2], x[nt][3]);
+            }
+            proxy_fence();
+            __syncwarp();
+            if (lane == 0) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                                     reinterpret_cast<uint64_t>(&maps.state)),
+                                 "r"(32 * h), "r"(row + row0), "r"(smem_u32(half[h])) : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+        };
         ChainSync cs{bar + kBChain, 0, 0};
         int sa = 0;
         uint32_t par = 0;
@@ -290,6 +314,11 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             group_sync(gbar, GNT);
             tc_fence_after();
             if (gabort[2]) break;
+            if (c > 0 && lane == 0) {   // the matrix set of the chunk before: free once the state has left it
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                mbar_arrive(bar + kEmptyU + (su ^ 1));
+            }
+            __syncwarp();
             if (wg == 0) {
                 const uint32_t id64 = idesc64(64, 0, 0);
 #pragma unroll
@@ -346,7 +375,6 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             tc_fence_after();
             PIPE_MARK(2);
             {
-                float* dst = (c + 1 < nchunks) ? (ck ? ck + (i64)(c + 1) * 64 * 64 : nullptr) : (sT_ ? sT_ + sbase : nullptr);
                 float Sd[8][4];
                 tmem_ld_tiles<8>(Sd, tmS + lane_off);
                 tmem_wait_ld();
@@ -354,7 +382,13 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
                 for (int nt = 0; nt < 8; ++nt) {
                     const float2 we = *reinterpret_cast<const float2*>(We + nt * 8 + 2 * t);
                     Sd[nt][0] *= we.x; Sd[nt][1] *= we.y; Sd[nt][2] *= we.x; Sd[nt][3] *= we.y;
-                    if (dst != nullptr) {
+                }
+                if (c + 1 < nchunks) {
+                    if (ck != nullptr) send_state(Sd, U, ((bb * H + hh) * (T / 16) + c + 1) * 64);
+                } else if (sT_ != nullptr) {
+                    float* dst = sT_ + sbase;
+#pragma unroll
+                    for (int nt = 0; nt < 8; ++nt) {
                         *reinterpret_cast<float2*>(dst + (row0 + g) * 64 + nt * 8 + 2 * t) = make_float2(Sd[nt][0], Sd[nt][1]);
                         *reinterpret_cast<float2*>(dst + (row0 + g + 8) * 64 + nt * 8 + 2 * t) = make_float2(Sd[nt][2], Sd[nt][3]);
                     }
@@ -364,13 +398,11 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             }
             tc_fence_before();
             group_sync(gbar, GNT);
-            if (gtid == 0) {   // the other groups may refill the sets
-                mbar_arrive(bar + kEmptyA + sa);
-                mbar_arrive(bar + kEmptyU + su);
-            }
+            if (gtid == 0) mbar_arrive(bar + kEmptyA + sa);   // the other groups may refill the operand set
             PIPE_MARK(3);
             if (++sa == NA) sa = 0;
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // before the block ends
         if (fail) atomicMax(const_cast<int*>(abort_word), fail);
     }
 
@@ -418,6 +450,19 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols) {
     // (a thread that has made no runtime call yet has no context, which this driver call wants)
     return encode() || (cudaFree(nullptr) == cudaSuccess && encode());
 }
+// (rows, 64) fp32 states, box [16 rows][32 columns], the shared-memory side in the layout of the operand arrays
+bool make_state_map(CUtensorMap* m, const void* base, uint64_t rows) {
+    const cuuint64_t dims[2] = {64, rows};
+    const cuuint64_t strides[1] = {64 * 4};
+    const cuuint32_t box[2] = {32, 16};
+    const cuuint32_t elem[2] = {1, 1};
+    auto encode = [&] {
+        return encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, elem,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    return encode() || (cudaFree(nullptr) == cudaSuccess && encode());
+}
 }  // namespace
 
 bool wkv7_make_tile_map(void* map, const void* base, unsigned long long rows, unsigned long long cols) {
@@ -434,6 +479,8 @@ int wkv7_l32_forward_pipelined(int B, int T, int H, const float* s0, const void*
     const void* in[6] = {r, w, k, v, a, b};
     for (int x = 0; x < 6; ++x)
         if (!make_map(&maps.m[x], in[x], (uint64_t)B * T, (uint64_t)H * 64)) return 1;
+    maps.state = maps.m[0];
+    if (s != nullptr && !make_state_map(&maps.state, s, (uint64_t)B * H * (T / 16) * 64)) return 1;
     cudaError_t e = allow_smem<wkv7q_forward_kernel>(PipeSmem::kBytes);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv7_forward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     dim3 grid(H, B);
