@@ -18,6 +18,11 @@
 // (log w = -exp(w_raw): its derivative by w_raw is log w itself; wkv6_cuda_v1.cu:203 of the reference).  A static
 // decay (RWKV-5) has one gw per channel and batch row: the sum over the tokens.
 //
+// The products are issued in the order dV, dK' and dR', E and ET, and taken in that order: the first half of the epilogue runs
+// beside the updates of E and ET (waiting for them before it cost 730 of 9600 cycles a chunk); V and dY lie in the order that
+// gives the masking of A to four warps and that of G to the other four; gw of a chunk leaves after the next one's barrier.
+// B16 T4096 H64: 2368 -> 2344 us.
+//
 // One CTA of 8 warps per (batch, head), two CTAs per SM.  Tensor memory (256 columns): E | ET | W1 (G', then dV) |
 // U (the A product) | W2 (dK'^T | dR'^T).  The chunk-start states come from a pass of the forward kernel that
 // saves them every 32 tokens.
@@ -37,7 +42,7 @@ __device__ int g_v6b_error = 0;
 struct Smem {
     static constexpr int kRT = 0;                        // [32][64] r~_t
     static constexpr int kKK = kRT + ARR32;              // [64][64] rows 0-31 k~_s, rows 32-63 k^_s
-    static constexpr int kVY = kKK + ARR64;              // [64][64] rows 0-31 v_s, rows 32-63 gy_t (columns = value i)
+    static constexpr int kVY = kKK + ARR64;              // [64][64] rows 0-31 gy_t, rows 32-63 v_s (columns = value i)
     static constexpr int kS0 = kVY + ARR64;              // [i][j]
     static constexpr int kAm = kS0 + ARR64;              // [32][32] A[s][t]
     static constexpr int kGm = kAm + HALF32;             // [32][32] G[s][t], strict
@@ -221,11 +226,14 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     uint32_t par = 0;
     float gu_acc[2] = {0.f, 0.f}, gw_acc[2] = {0.f, 0.f};   // sums over this thread's tokens (gw only for a static decay)
 
+    auto flush_gw = [&](int c) { stage_flush(KK + 32 * 128, gw_, tok0 + (i64)c * LC * C, C, tid, min(LC, T - c * LC)); };
+
     for (int c = nchunks - 1; c >= 0; --c, par ^= 1) {
         const int valid = min(LC, T - c * LC);
         tc_fence_before();
         if (__syncthreads_or(fail)) break;
         tc_fence_after();
+        if (!kStatic && c + 1 < nchunks) flush_gw(c + 1);   // staged before this barrier; its rows are written again below
         if (tid == 224) {   // chunk-start state -> S0: the forward has left it in the array's layout
             mbar_expect_bytes(bar + 5, ARR64);
             bulk_load(S0, ck + (i64)c * 64 * 64, ARR64, bar + 5);
@@ -267,8 +275,8 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                 *reinterpret_cast<float2*>(RT + sw(tt, j0, HALF32)) = make_float2(tf32rf(r2.x * wp0), tf32rf(r2.y * wp1));
                 *reinterpret_cast<float2*>(KK + sw(tt, j0, HALF64)) = make_float2(tf32rf(k2.x * iw0), tf32rf(k2.y * iw1));
                 *reinterpret_cast<float2*>(KK + sw(32 + tt, j0, HALF64)) = make_float2(tf32rf(up0 * k2.x * ip0), tf32rf(up1 * k2.y * ip1));
-                *reinterpret_cast<float2*>(VY + sw(tt, j0, HALF64)) = bf16x2_to_f2(raw.x[2][q]);
-                *reinterpret_cast<float2*>(VY + sw(32 + tt, j0, HALF64)) = bf16x2_to_f2(raw.x[3][q]);
+                *reinterpret_cast<float2*>(VY + sw(32 + tt, j0, HALF64)) = bf16x2_to_f2(raw.x[2][q]);
+                *reinterpret_cast<float2*>(VY + sw(tt, j0, HALF64)) = bf16x2_to_f2(raw.x[3][q]);
                 *reinterpret_cast<float2*>(Lam + tt * LAMP + j0) = make_float2(l0, l1);
                 lp0 = base0 + cs0[q]; lp1 = base1 + cs1[q];
             }
@@ -284,8 +292,8 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             for (int ks = 0; ks < 8; ++ks)   // [K~;K^] R~^T
                 mma_ss(tmU, desc_k(kkA, 0, ks * 8, HALF64), desc_k(rtA, 0, ks * 8, HALF32), idesc64(32, 0, 0), ks > 0, lead);
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks)   // G' = [V;dY] dY^T (its rows 0-31 are V dY^T)
-                mma_ss(tmW1, desc_k(vyA, 0, ks * 8, HALF64), desc_k(vyA, 32, ks * 8, HALF64), idesc64(32, 0, 0), ks > 0, lead);
+            for (int ks = 0; ks < 8; ++ks)   // G' = [dY;V] dY^T (its rows 32-63 are V dY^T)
+                mma_ss(tmW1, desc_k(vyA, 0, ks * 8, HALF64), desc_k(vyA, 0, ks * 8, HALF64), idesc64(32, 0, 0), ks > 0, lead);
             mma_commit(bar, lead);
         }
         // meanwhile: Ew = E diag(We), ETw = diag(We) ET, and the request of the next chunk
@@ -324,20 +332,20 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                     const bool diag = nt == h && hs == (quarter & 1);         // the tile with the diagonal in it
                     const float a0 = ua[nt][2 * h], a1 = ua[nt][2 * h + 1], g0 = gg[nt][2 * h], g1 = gg[nt][2 * h + 1];
                     float* am = reinterpret_cast<float*>(Am + sw32(s, c0));
-                    if (quarter < 2) {   // rows k~_s / v_s; the diagonal of A comes from the rows k^_s
+                    if (quarter < 2) {   // rows k~_s: A but for its diagonal
                         const float2 as = make_float2(s < c0 ? tf32rf(a0) : 0.f, s < c0 + 1 ? tf32rf(a1) : 0.f);
                         if (!diag) {
                             *reinterpret_cast<float2*>(am) = as;
                         } else {
                             if (s != c0) am[0] = as.x;
                             if (s != c0 + 1) am[1] = as.y;
-                            if (s == c0) Gam[s] = g0;
-                            if (s == c0 + 1) Gam[s] = g1;
+                        }
+                    } else {             // rows k^_s: the diagonal of A; rows v_s: G and its diagonal
+                        if (diag) {
+                            if (s == c0) { am[0] = tf32rf(a0); Gam[s] = g0; }
+                            if (s == c0 + 1) { am[1] = tf32rf(a1); Gam[s] = g1; }
                         }
                         *reinterpret_cast<float2*>(Gm + sw32(s, c0)) = make_float2(s < c0 ? tf32rf(g0) : 0.f, s < c0 + 1 ? tf32rf(g1) : 0.f);
-                    } else if (diag) {
-                        if (s == c0) am[0] = tf32rf(a0);
-                        if (s == c0 + 1) am[1] = tf32rf(a1);
                     }
                 }
         }
@@ -352,27 +360,27 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                 mma_ts(tmW1, tmE + ks * 8, desc_k(kkA, 0, ks * 8, HALF64), idesc64(32, 0, 0), ks > 0, lead);
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)   //    + dY A^T
-                mma_ss(tmW1, desc_mn(vyA + 32 * 128, ks * 8, HALF64), desc_k(amA, 0, ks * 8, HALF32), idesc64(32, 1, 0), 1, lead);
+                mma_ss(tmW1, desc_mn(vyA, ks * 8, HALF64), desc_k(amA, 0, ks * 8, HALF32), idesc64(32, 1, 0), 1, lead);
             mma_commit(bar + 1, lead);
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)   // dK'^T = ETw V^T
-                mma_ts(tmW2, tmET + ks * 8, desc_k(vyA, 0, ks * 8, HALF64), idesc64(32, 0, 0), ks > 0, lead);
+                mma_ts(tmW2, tmET + ks * 8, desc_k(vyA, 32, ks * 8, HALF64), idesc64(32, 0, 0), ks > 0, lead);
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)   //       + R~^T G^T
                 mma_ss(tmW2, desc_mn(rtA, ks * 8, HALF32), desc_k(gmA, 0, ks * 8, HALF32), idesc64(32, 1, 0), 1, lead);
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)   // dR'^T = S0^T dY^T
-                mma_ss(tmW2 + 32, desc_mn(s0A, ks * 8, HALF64), desc_k(vyA, 32, ks * 8, HALF64), idesc64(32, 1, 0), ks > 0, lead);
+                mma_ss(tmW2 + 32, desc_mn(s0A, ks * 8, HALF64), desc_k(vyA, 0, ks * 8, HALF64), idesc64(32, 1, 0), ks > 0, lead);
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)   //       + K~^T G
                 mma_ss(tmW2 + 32, desc_mn(kkA, ks * 8, HALF64), desc_mn(gmA, ks * 8, HALF32), idesc64(32, 1, 1), 1, lead);
             mma_commit(bar + 2, lead);
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)   // E += dY (stacked over tokens) R~
-                mma_ss(tmE, desc_mn(vyA + 32 * 128, ks * 8, HALF64), desc_mn(rtA, ks * 8, HALF32), idesc64(64, 1, 1), 1, lead);
+                mma_ss(tmE, desc_mn(vyA, ks * 8, HALF64), desc_mn(rtA, ks * 8, HALF32), idesc64(64, 1, 1), 1, lead);
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)   // ET += R~^T dY
-                mma_ss(tmET, desc_mn(rtA, ks * 8, HALF32), desc_mn(vyA + 32 * 128, ks * 8, HALF64), idesc64(64, 1, 1), 1, lead);
+                mma_ss(tmET, desc_mn(rtA, ks * 8, HALF32), desc_mn(vyA, ks * 8, HALF64), idesc64(64, 1, 1), 1, lead);
             mma_commit(bar + 3, lead);
         }
         // ---- 5. dv: this warp's rows i, tokens 16*hs .. 16*hs+15 -----------------------------------------
@@ -390,32 +398,12 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                     *reinterpret_cast<bf16*>(Dv + stage_off(tt, i)) = __float2bfloat16_rn(dv[nt][e]);   // staged, sent with gr and gk
                 }
         }
-        // ---- 6. the anchor A0[j] = sum_i ET_new[j][i] S0[i][j]; this warp: value columns 32*hs .. 32*hs+31 -----
-        if (!mbar_wait(bar + 3, par)) fail = 4;
-        tc_fence_after();
-        {
-            float Td[4][4];
-            tmem_ld_tiles<4>(Td, tmET + 32 * hs + lane_off);
-            tmem_wait_ld();
-            float acc0 = 0.f, acc1 = 0.f;
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int i = 32 * hs + nt * 8 + 2 * t;
-                const float2 s0 = f32_pair(S0, i, row0 + g, HALF64, t >> 1), s1 = f32_pair(S0, i, row0 + g + 8, HALF64, t >> 1);
-                acc0 = fmaf(Td[nt][1], s0.y, fmaf(Td[nt][0], s0.x, acc0));
-                acc1 = fmaf(Td[nt][3], s1.y, fmaf(Td[nt][2], s1.x, acc1));
-            }
-            acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1); acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
-            acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1); acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
-            if (t == 0) { A0p[hs * 64 + row0 + g] = acc0; A0p[hs * 64 + row0 + g + 8] = acc1; }
-        }
         if (!mbar_wait(bar + 2, par)) fail = 3;
         tc_fence_after();
-        // ---- 7. epilogue: this warp has key rows row0+g / +8 and tokens 16*hs .. 16*hs+15 ---------------------
-        // staging rows ([32 tokens][72] bf16 each: gr, gk, gw) in the V / gy array, dead by now
-        bf16* stg[3];
-#pragma unroll
-        for (int o = 0; o < 3; ++o) stg[o] = reinterpret_cast<bf16*>(VY + o * (32 * 72 * 2));
+        // ---- 6. epilogue: this warp has key rows row0+g / +8 and tokens 16*hs .. 16*hs+15 ---------------------
+        // staging tiles of gr and gk in the rows of V, of gw in the rows of K^: nothing reads these any more, while the
+        // updates of E and ET may still be running (they read R~ and dY; they are waited for below, after this half)
+        unsigned char *sgR = VY + 32 * 128, *sgK = VY + HALF64 + 32 * 128, *sgW = KK + 32 * 128;
         float gl[2][2][2], lw[2][2][2];
         {
             float gK[2][4], gR[2][4];
@@ -448,8 +436,8 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                         gl[h][nt][e] = rdr;
                         lw[h][nt][e] = (lm[e + 1] - lm[e]) * 0.6931471805599453f;   // log w_t
                         gu_acc[h] = fmaf(gm, rr * kr, gu_acc[h]);
-                        stg[0][tt * 72 + j] = __float2bfloat16_rn(fmaf(gam_u, kr, drs));
-                        stg[1][tt * 72 + j] = __float2bfloat16_rn(fmaf(gam_u, rr, dks));
+                        *reinterpret_cast<bf16*>(sgR + stage_off(tt, j)) = __float2bfloat16_rn(fmaf(gam_u, kr, drs));
+                        *reinterpret_cast<bf16*>(sgK + stage_off(tt, j)) = __float2bfloat16_rn(fmaf(gam_u, rr, dks));
                     }
                 }
 #pragma unroll
@@ -469,6 +457,25 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             }
             if (hs == 0 && t == 0) { Carry[row0 + g] = run[0]; Carry[row0 + g + 8] = run[1]; }
         }
+        // ---- 7. the anchor A0[j] = sum_i ET_new[j][i] S0[i][j]; this warp: value columns 32*hs .. 32*hs+31 -----
+        if (!mbar_wait(bar + 3, par)) fail = 4;
+        tc_fence_after();
+        {
+            float Td[4][4];
+            tmem_ld_tiles<4>(Td, tmET + 32 * hs + lane_off);
+            tmem_wait_ld();
+            float acc0 = 0.f, acc1 = 0.f;
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const int i = 32 * hs + nt * 8 + 2 * t;
+                const float2 s0 = f32_pair(S0, i, row0 + g, HALF64, t >> 1), s1 = f32_pair(S0, i, row0 + g + 8, HALF64, t >> 1);
+                acc0 = fmaf(Td[nt][1], s0.y, fmaf(Td[nt][0], s0.x, acc0));
+                acc1 = fmaf(Td[nt][3], s1.y, fmaf(Td[nt][2], s1.x, acc1));
+            }
+            acc0 += __shfl_xor_sync(0xffffffffu, acc0, 1); acc0 += __shfl_xor_sync(0xffffffffu, acc0, 2);
+            acc1 += __shfl_xor_sync(0xffffffffu, acc1, 1); acc1 += __shfl_xor_sync(0xffffffffu, acc1, 2);
+            if (t == 0) { A0p[hs * 64 + row0 + g] = acc0; A0p[hs * 64 + row0 + g + 8] = acc1; }
+        }
         __syncthreads();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -481,24 +488,12 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                     const int tt = 16 * hs + nt * 8 + 2 * t + e;
                     const float gw = (a0 - gl[h][nt][e]) * lw[h][nt][e];
                     if (kStatic) gw_acc[h] += gw;
-                    else stg[2][tt * 72 + j] = __float2bfloat16_rn(gw);
+                    else *reinterpret_cast<bf16*>(sgW + stage_off(tt, j)) = __float2bfloat16_rn(gw);
                 }
         }
-        {   // gr, gk out: thread = (token, 16-byte piece)
-            const int tt = tid >> 3, piece = tid & 7;
-            if (tt < valid) {
-                const i64 o = tok0 + (i64)(c * LC + tt) * C + piece * 8;
-                *reinterpret_cast<uint4*>(gr_ + o) = *reinterpret_cast<const uint4*>(stg[0] + tt * 72 + piece * 8);
-                *reinterpret_cast<uint4*>(gk_ + o) = *reinterpret_cast<const uint4*>(stg[1] + tt * 72 + piece * 8);
-            }
-        }
+        stage_flush(sgR, gr_, tok0 + (i64)c * LC * C, C, tid, valid);
+        stage_flush(sgK, gk_, tok0 + (i64)c * LC * C, C, tid, valid);
         stage_flush(Dv, gv_, tok0 + (i64)c * LC * C, C, tid, valid);
-        if (!kStatic) {
-            __syncthreads();
-            const int tt = tid >> 3, piece = tid & 7;
-            if (tt < valid)
-                *reinterpret_cast<uint4*>(gw_ + tok0 + (i64)(c * LC + tt) * C + piece * 8) = *reinterpret_cast<const uint4*>(stg[2] + tt * 72 + piece * 8);
-        }
     }
 
     if (pending) mbar_wait(bar + 6, par);   // leaving early: the requested tiles must have landed before the block may end
@@ -509,6 +504,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (!kStatic) flush_gw(0);
     // gu (and gw of a static decay): sums over the four lanes of a quad and the two token halves
     {
 #pragma unroll
