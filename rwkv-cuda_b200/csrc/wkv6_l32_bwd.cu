@@ -167,7 +167,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             const bool in = t0 + q < T;
             win[q] = in;
             if (WMODE == 1) {
-                wraw[q] = in ? __ldg(reinterpret_cast<const unsigned int*>(reinterpret_cast<const bf16*>(w_) + tok0 + (i64)(t0 + q) * C + j0)) : 0u;
+                wraw[q] = in ? __ldg(reinterpret_cast<const unsigned int*>(reinterpret_cast<const bf16*>(w_) + tok0 + (i64)(t0 + q) * C + j0)) : 0xff80ff80u;
             } else if (WMODE == 0) {
                 wlog[q] = make_float2(0.f, 0.f);
                 if (in) wlog[q] = __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(w_) + tok0 + (i64)(t0 + q) * C + j0));
@@ -185,16 +185,24 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
         if (warp < 4 || (warp == 4 && WMODE <= 1)) tma_tile_load(Raw + warp * 4096, &maps.m[warp], hh * 64, bb * T + c * LC, bar + 6);
     };
     auto take = [&](int c) {
-        const int t0 = c * LC + BTPW * warp;
+        const int t0 = BTPW * warp, valid = min(LC, T - c * LC);
+        if (valid < LC) {   // the last chunk of a ragged T: neutral words in place of the rows beyond it (this thread's own)
+            for (int row = t0; row < t0 + BTPW; ++row) {
+                if (row < valid) continue;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) *reinterpret_cast<uint32_t*>(Raw + x * 4096 + row * 128 + lane * 4) = 0u;
+                if (WMODE == 1) *reinterpret_cast<uint32_t*>(Raw + 4 * 4096 + row * 128 + lane * 4) = 0xff80ff80u;   // -inf: no decay
+                if (WMODE == 0) *reinterpret_cast<float2*>(Raw + 4 * 4096 + row * 256 + lane * 8) = make_float2(0.f, 0.f);
+            }
+        }
 #pragma unroll
         for (int q = 0; q < BTPW; ++q) {
-            const bool in = t0 + q < T;
-            const int row = BTPW * warp + q;
-            win[q] = in;
+            const int row = t0 + q;
+            win[q] = WMODE < 2 || row < valid;
 #pragma unroll
-            for (int x = 0; x < 4; ++x) raw.x[x][q] = in ? *reinterpret_cast<const uint32_t*>(Raw + x * 4096 + row * 128 + lane * 4) : 0u;
-            if (WMODE == 1) wraw[q] = in ? *reinterpret_cast<const uint32_t*>(Raw + 4 * 4096 + row * 128 + lane * 4) : 0u;
-            if (WMODE == 0) wlog[q] = in ? *reinterpret_cast<const float2*>(Raw + 4 * 4096 + row * 256 + lane * 8) : make_float2(0.f, 0.f);
+            for (int x = 0; x < 4; ++x) raw.x[x][q] = *reinterpret_cast<const uint32_t*>(Raw + x * 4096 + row * 128 + lane * 4);
+            if (WMODE == 1) wraw[q] = *reinterpret_cast<const uint32_t*>(Raw + 4 * 4096 + row * 128 + lane * 4);
+            if (WMODE == 0) wlog[q] = *reinterpret_cast<const float2*>(Raw + 4 * 4096 + row * 256 + lane * 8);
         }
     };
     const bool staged = maps.valid != 0;
@@ -203,8 +211,8 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     auto decay_log2 = [&](int q, float& l0, float& l1) {
         if (WMODE == 1) {
             const float2 w2 = bf16x2_to_f2(wraw[q]);
-            l0 = win[q] ? -fexp(w2.x) * 1.4426950408889634f : 0.f;
-            l1 = win[q] ? -fexp(w2.y) * 1.4426950408889634f : 0.f;
+            l0 = -fexp(w2.x) * 1.4426950408889634f;
+            l1 = -fexp(w2.y) * 1.4426950408889634f;
         } else if (WMODE == 0) {
             l0 = wlog[q].x * 1.4426950408889634f;
             l1 = wlog[q].y * 1.4426950408889634f;

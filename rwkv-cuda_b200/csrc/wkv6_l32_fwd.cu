@@ -185,25 +185,33 @@ wkv6q_forward_kernel(int T, int H, const __grid_constant__ Maps maps, const void
             // this thread: channels j0, j0+1 of tokens 8*wg .. 8*wg+7
             uint32_t xr[LTPW], xk[LTPW], xv[LTPW];
             float ld0[LTPW], ld1[LTPW];   // log2 decay of the token
-            const unsigned char* rs = stg + st * kRawStage;
+            unsigned char* rs = stg + st * kRawStage;
+            if (valid < LC) {   // the last chunk of a ragged T: neutral words in place of the rows beyond it (this thread's own)
+                for (int tt = LTPW * wg; tt < LTPW * wg + LTPW; ++tt) {
+                    if (tt < valid) continue;
+#pragma unroll
+                    for (int x = 0; x < 3; ++x) *reinterpret_cast<uint32_t*>(rs + x * 4096 + tt * 128 + 4 * lane) = 0u;
+                    if (WMODE == 1) *reinterpret_cast<uint32_t*>(rs + 12288 + tt * 128 + 4 * lane) = 0xff80ff80u;   // -inf: no decay
+                    if (WMODE == 0) *reinterpret_cast<float2*>(rs + 12288 + tt * 256 + 8 * lane) = make_float2(0.f, 0.f);
+                }
+            }
 #pragma unroll
             for (int q = 0; q < LTPW; ++q) {
                 const int tt = LTPW * wg + q;
-                const bool in = tt < valid;
-                xr[q] = in ? *reinterpret_cast<const uint32_t*>(rs + tt * 128 + 4 * lane) : 0u;
-                xk[q] = in ? *reinterpret_cast<const uint32_t*>(rs + 4096 + tt * 128 + 4 * lane) : 0u;
-                xv[q] = in ? *reinterpret_cast<const uint32_t*>(rs + 8192 + tt * 128 + 4 * lane) : 0u;
+                xr[q] = *reinterpret_cast<const uint32_t*>(rs + tt * 128 + 4 * lane);
+                xk[q] = *reinterpret_cast<const uint32_t*>(rs + 4096 + tt * 128 + 4 * lane);
+                xv[q] = *reinterpret_cast<const uint32_t*>(rs + 8192 + tt * 128 + 4 * lane);
                 if (WMODE == 1) {
                     const float2 w2 = bf16x2_to_f2(*reinterpret_cast<const uint32_t*>(rs + 12288 + tt * 128 + 4 * lane));
-                    ld0[q] = in ? -fexp(w2.x) * 1.4426950408889634f : 0.f;
-                    ld1[q] = in ? -fexp(w2.y) * 1.4426950408889634f : 0.f;
+                    ld0[q] = -fexp(w2.x) * 1.4426950408889634f;
+                    ld1[q] = -fexp(w2.y) * 1.4426950408889634f;
                 } else if (WMODE == 0) {
                     const float2 w2 = *reinterpret_cast<const float2*>(rs + 12288 + tt * 256 + 8 * lane);
-                    ld0[q] = in ? w2.x * 1.4426950408889634f : 0.f;
-                    ld1[q] = in ? w2.y * 1.4426950408889634f : 0.f;
+                    ld0[q] = w2.x * 1.4426950408889634f;
+                    ld1[q] = w2.y * 1.4426950408889634f;
                 } else {
-                    ld0[q] = in ? ls0 : 0.f;
-                    ld1[q] = in ? ls1 : 0.f;
+                    ld0[q] = tt < valid ? ls0 : 0.f;
+                    ld1[q] = tt < valid ? ls1 : 0.f;
                 }
             }
             // cumulative log2 decays: within the warp's tokens, then across the warps
