@@ -223,8 +223,10 @@ struct RawChunk {
     uint32_t x[NX][TPW];
 };
 
-// Loads the thread's part of chunk c; tokens at or beyond T read as zeros (a zero raw decay input is
-// replaced by "no decay" in prepare_operands through the `valid` count).
+// A word of a token beyond the sequence: zeros, and -inf (no decay) as the raw decay input.
+__device__ __forceinline__ uint32_t neutral_word(int x) { return x == 1 ? 0xff80ff80u : 0u; }
+
+// Loads the thread's part of chunk c; tokens at or beyond T read as neutral words.
 template <int NX, int TPW>
 __device__ __forceinline__ void fetch_chunk(RawChunk<NX, TPW>& rc, const bf16* const* src, i64 tok0, int C, int c, int T,
                                             int warp, int lane) {
@@ -234,7 +236,23 @@ __device__ __forceinline__ void fetch_chunk(RawChunk<NX, TPW>& rc, const bf16* c
     for (int x = 0; x < NX; ++x)
 #pragma unroll
         for (int q = 0; q < TPW; ++q)
-            rc.x[x][q] = (t0 + q < T) ? __ldg(reinterpret_cast<const unsigned int*>(src[x] + off + (i64)q * C)) : 0u;
+            rc.x[x][q] = (t0 + q < T) ? __ldg(reinterpret_cast<const unsigned int*>(src[x] + off + (i64)q * C)) : neutral_word(x);
+}
+// The same out of tiles that the copy engine has staged (4 KB each, plain rows).  Rows at or beyond `valid` belong to something
+// else: the thread puts neutral words in their place first, so that a full chunk pays nothing for them (with a test at every
+// word, 8 % of the preparation's instructions).
+template <int NX, int TPW>
+__device__ __forceinline__ void take_chunk(RawChunk<NX, TPW>& rc, unsigned char* tiles, int valid, int warp, int lane) {
+    unsigned char* p = tiles + TPW * warp * 128 + lane * 4;
+    if (valid < LC) {
+        for (int q = max(0, valid - TPW * warp); q < TPW; ++q)
+#pragma unroll
+            for (int x = 0; x < NX; ++x) *reinterpret_cast<uint32_t*>(p + x * 4096 + q * 128) = neutral_word(x);
+    }
+#pragma unroll
+    for (int x = 0; x < NX; ++x)
+#pragma unroll
+        for (int q = 0; q < TPW; ++q) rc.x[x][q] = *reinterpret_cast<const uint32_t*>(p + x * 4096 + q * 128);
 }
 
 // Asks for the inputs of a chunk to be brought into L2 ahead of the loads above: one [32 tokens][64 channels] tile per
@@ -290,11 +308,11 @@ __device__ __forceinline__ void prefetch_chunk_l2(const TileMaps<NX>& maps, int 
 //   AR rows 0-31 = a~_t, rows 32-63 = r~_t        BK rows 0-31 = b~_t, rows 32-63 = k~_t      (columns = key channel)
 //   V rows = v_t (dst_v, a 32-row half-array pair at the given half stride), optionally dY the same way,
 //   We[j] = decay over the whole chunk, and optionally the cumulative log2-decays lam[t][j] (plain [32][LAMP]).
-// Tokens at or beyond `valid` (counted inside the chunk) are neutral: no decay, zero vectors.
+// Tokens beyond the sequence come as neutral words: no decay, zero vectors.
 // Hs is a [NW][64] exchange buffer.  Contains one barrier among the NW calling warps (the CTA, or the named
 // barrier `bar_id` of a warp group); the caller synchronises afterwards.
 template <int NX, int TPW, int NW>
-__device__ __forceinline__ void prepare_operands(const RawChunk<NX, TPW>& rc, int valid, unsigned char* AR, unsigned char* BK,
+__device__ __forceinline__ void prepare_operands(const RawChunk<NX, TPW>& rc, unsigned char* AR, unsigned char* BK,
                                                  unsigned char* dstV, int halfV, unsigned char* dstDY, int halfDY,
                                                  float* We, float* Hs, float* lam_out, int warp, int lane, int bar_id = 0) {
     const int j0 = 2 * lane, t0 = TPW * warp;
@@ -303,10 +321,8 @@ __device__ __forceinline__ void prepare_operands(const RawChunk<NX, TPW>& rc, in
 #pragma unroll
     for (int q = 0; q < TPW; ++q) {
         const float2 x = bf16x2_to_f2(rc.x[1][q]);
-        if (t0 + q < valid) {
-            run0 = fmaf(kWScale2, frcp(1.f + fexp(-x.x)), run0);
-            run1 = fmaf(kWScale2, frcp(1.f + fexp(-x.y)), run1);
-        }
+        run0 = fmaf(kWScale2, frcp(1.f + fexp(-x.x)), run0);
+        run1 = fmaf(kWScale2, frcp(1.f + fexp(-x.y)), run1);
         cs[q][0] = run0; cs[q][1] = run1;
     }
     *reinterpret_cast<float2*>(Hs + warp * 64 + j0) = make_float2(run0, run1);

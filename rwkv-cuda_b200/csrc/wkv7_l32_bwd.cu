@@ -193,14 +193,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             if ((reinterpret_cast<uintptr_t>(sp) & 15) == 0) l2_prefetch(sp, 64 * 64 * 4);
         }
     };
-    auto take = [&](int c) {
-        const int t0 = c * LC + BTPW * warp;
-#pragma unroll
-        for (int x = 0; x < 7; ++x)
-#pragma unroll
-            for (int q = 0; q < BTPW; ++q)
-                raw.x[x][q] = (t0 + q < T) ? *reinterpret_cast<const uint32_t*>(Raw + x * 4096 + (BTPW * warp + q) * 128 + lane * 4) : 0u;
-    };
+    auto take = [&](int c) { take_chunk<7, BTPW>(raw, Raw, min(LC, T - c * LC), warp, lane); };
     if (staged) { request(c_hi); pending = true; }
     else fetch_chunk<7, BTPW>(raw, src, tok0, C, c_hi, T, warp, lane);
     if (c_hi > c_lo) ask_l2(c_hi - 1);
@@ -231,7 +224,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             reinterpret_cast<float4*>(N1)[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         // ---- 1. operands ---------------------------------------------------------------------------
-        prepare_operands<7, BTPW, 8>(raw, valid, AR, BK, SV + 32 * 128, HALF64, EY + 32 * 128, HALF64, We, Hs, Lam, warp, lane);
+        prepare_operands<7, BTPW, 8>(raw, AR, BK, SV + 32 * 128, HALF64, EY + 32 * 128, HALF64, We, Hs, Lam, warp, lane);
         WKV7_PHASE(1);   // operand preparation
         cp_async_wait<0>();   // the chunk-start state
         proxy_fence();

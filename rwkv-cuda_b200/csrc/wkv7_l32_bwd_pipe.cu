@@ -245,12 +245,7 @@ wkv7p_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
             if (it >= 2) flush_outputs(base, c + 2);   // the set holds the staged outputs of the chunk that used it last: they leave from here
             if (staged) {
                 if (!mbar_wait(bar + kRaw + set, (it >> 1) & 1)) fail = 36;
-                const unsigned char* rawt = base + SetSmem::kEY;
-#pragma unroll
-                for (int x = 0; x < 7; ++x)
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        raw.x[x][q] = (c * LC + 4 * wg + q < T) ? *reinterpret_cast<const uint32_t*>(rawt + x * 4096 + (4 * wg + q) * 128 + lane * 4) : 0u;
+                take_chunk<7, 4>(raw, base + SetSmem::kEY, min(LC, T - c * LC), wg, lane);
                 if (gtid == 0) raw_got[set] = raw_got[set] + 1;
             }
             if (it >= 2 || staged) group_sync(gbar, GNT);   // before the set is written
@@ -270,7 +265,7 @@ wkv7p_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                 *reinterpret_cast<float*>(D0 + sw32(16 + s, cc)) = 0.f;
                 reinterpret_cast<float4*>(N1)[gtid] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            prepare_operands<7, 4, 8>(raw, valid, AR, BK, SV + 32 * 128, HALF64, EY + 32 * 128, HALF64, We, Hs, Lam, wg, lane, gbar);
+            prepare_operands<7, 4, 8>(raw, AR, BK, SV + 32 * 128, HALF64, EY + 32 * 128, HALF64, We, Hs, Lam, wg, lane, gbar);
             cp_async_wait<0>();
             proxy_fence();
             tc_fence_before();

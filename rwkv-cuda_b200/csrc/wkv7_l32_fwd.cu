@@ -130,7 +130,7 @@ wkv7x_forward_kernel(int T, int H, const float* __restrict__ s0_, const bf16* __
         tc_fence_after();
         WKV7_PHASE(0);   // top barrier
         // ---- 1. operands ---------------------------------------------------------------------------
-        prepare_operands<6, FTPW, 4>(raw, valid, AR, BK, Vs, HALF32, nullptr, 0, We, Hs, nullptr, warp, lane);
+        prepare_operands<6, FTPW, 4>(raw, AR, BK, Vs, HALF32, nullptr, 0, We, Hs, nullptr, warp, lane);
         WKV7_PHASE(1);   // operand preparation
         proxy_fence();
         WKV7_PHASE(11);  // proxy fence

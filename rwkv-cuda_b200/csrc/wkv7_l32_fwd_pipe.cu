@@ -163,13 +163,7 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             if (ua >= 1 && !mbar_wait(bar + kEmptyA + sa, (ua - 1) & 1)) fail = 30;       // both consumers released this set
             PIPE_MARK(0);
             RawChunk<6, 8> raw;
-#pragma unroll
-            for (int x = 0; x < 6; ++x)
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int tt = 8 * wg + q;
-                    raw.x[x][q] = tt < valid ? *reinterpret_cast<const uint32_t*>(stg + ((st * 6 + x) * 32 + tt) * 128 + 4 * lane) : 0u;
-                }
+            take_chunk<6, 8>(raw, stg + st * 6 * 32 * 128, valid, wg, lane);
             PIPE_MARK(3);
             if (fail) atomicMax(const_cast<int*>(abort_word), fail);
             if (gtid == 0) gabort[0] = *abort_word;
@@ -178,7 +172,7 @@ wkv7q_forward_kernel(int T, int H, const float* __restrict__ s0_, const __grid_c
             if (gtid == 0) mbar_arrive(bar + kTaken + st);   // every thread has taken its part of the rows: the stage may be refilled
             if (gabort[0]) break;
             PIPE_MARK(4);
-            prepare_operands<6, 8, 4>(raw, valid, A, A + ARR64, A + 2 * ARR64, HALF32, nullptr, 0, We, Hs, nullptr, wg, lane, gbar);
+            prepare_operands<6, 8, 4>(raw, A, A + ARR64, A + 2 * ARR64, HALF32, nullptr, 0, We, Hs, nullptr, wg, lane, gbar);
             proxy_fence();
             group_sync(gbar, GNT);
             if (gtid == 0) mbar_arrive(bar + kFullA + sa);

@@ -115,14 +115,8 @@ __global__ void __launch_bounds__(128, 2) wkv7_ops_kernel(int T, int H, int nch,
         if (!mbar_wait(bar, par)) fail = 1;
         pending = false;
         RawChunk<6, 8> raw;
-#pragma unroll
-        for (int x = 0; x < 6; ++x)
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int tt = 8 * warp + q;
-                raw.x[x][q] = tt < valid ? *reinterpret_cast<const uint32_t*>(Raw + x * 4096 + tt * 128 + 4 * lane) : 0u;
-            }
-        prepare_operands<6, 8, 4>(raw, valid, AR, BK, Vs, HALF32, nullptr, 0, We, Hs, nullptr, warp, lane);
+        take_chunk<6, 8>(raw, Raw, valid, warp, lane);
+        prepare_operands<6, 8, 4>(raw, AR, BK, Vs, HALF32, nullptr, 0, We, Hs, nullptr, warp, lane);
         proxy_fence();
         tc_fence_before();
         __syncthreads();
