@@ -160,7 +160,7 @@ wkv6b_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     float2 wlog[BTPW];        // WMODE 0: two fp32 log-decays
     bool win[BTPW];
     auto fetch = [&](int c) {
-        fetch_chunk<4, BTPW>(raw, src, tok0, C, c, T, warp, lane);
+        fetch_chunk<4, BTPW, -1>(raw, src, tok0, C, c, T, warp, lane);
         const int t0 = c * LC + BTPW * warp;
 #pragma unroll
         for (int q = 0; q < BTPW; ++q) {

@@ -224,10 +224,11 @@ struct RawChunk {
 };
 
 // A word of a token beyond the sequence: zeros, and -inf (no decay) as the raw decay input.
-__device__ __forceinline__ uint32_t neutral_word(int x) { return x == 1 ? 0xff80ff80u : 0u; }
+template <int XW>
+__device__ __forceinline__ uint32_t neutral_word(int x) { return x == XW ? 0xff80ff80u : 0u; }
 
-// Loads the thread's part of chunk c; tokens at or beyond T read as neutral words.
-template <int NX, int TPW>
+// Loads the thread's part of chunk c; tokens at or beyond T read as neutral words.  XW: which input is the raw decay (-1: none).
+template <int NX, int TPW, int XW = 1>
 __device__ __forceinline__ void fetch_chunk(RawChunk<NX, TPW>& rc, const bf16* const* src, i64 tok0, int C, int c, int T,
                                             int warp, int lane) {
     const int t0 = c * LC + TPW * warp;
@@ -236,7 +237,7 @@ __device__ __forceinline__ void fetch_chunk(RawChunk<NX, TPW>& rc, const bf16* c
     for (int x = 0; x < NX; ++x)
 #pragma unroll
         for (int q = 0; q < TPW; ++q)
-            rc.x[x][q] = (t0 + q < T) ? __ldg(reinterpret_cast<const unsigned int*>(src[x] + off + (i64)q * C)) : neutral_word(x);
+            rc.x[x][q] = (t0 + q < T) ? __ldg(reinterpret_cast<const unsigned int*>(src[x] + off + (i64)q * C)) : neutral_word<XW>(x);
 }
 // The same out of tiles that the copy engine has staged (4 KB each, plain rows).  Rows at or beyond `valid` belong to something
 // else: the thread puts neutral words in their place first, so that a full chunk pays nothing for them (with a test at every
@@ -247,7 +248,7 @@ __device__ __forceinline__ void take_chunk(RawChunk<NX, TPW>& rc, unsigned char*
     if (valid < LC) {
         for (int q = max(0, valid - TPW * warp); q < TPW; ++q)
 #pragma unroll
-            for (int x = 0; x < NX; ++x) *reinterpret_cast<uint32_t*>(p + x * 4096 + q * 128) = neutral_word(x);
+            for (int x = 0; x < NX; ++x) *reinterpret_cast<uint32_t*>(p + x * 4096 + q * 128) = neutral_word<1>(x);
     }
 #pragma unroll
     for (int x = 0; x < NX; ++x)
