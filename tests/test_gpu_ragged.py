@@ -51,3 +51,21 @@ def test_rwkv7_training_classes(use_s0):
     Hh.assert_close(y, want["y"], Hh.TOL_BF16, "y")
     for a, n in zip(g, names + ("s0",)):
         Hh.assert_close(a, want["d" + n], Hh.TOL_BF16, "d" + n)
+
+
+@pytest.mark.parametrize("T", [64, 300])
+@pytest.mark.parametrize("shift", [-5.0, -1.5, -0.5])
+def test_rwkv6_forward_scales_its_state(shift, T):
+    """Decays with which the forward scales the state in tensor memory never, every few chunks and before every chunk."""
+    import rwkv_cuda_b200 as R
+    g = Hh.gen(7)
+    B, H, N = 2, 2, 64
+    C = H * N
+    r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
+    w, u, s0 = Hh.randn(g, B, T, C) + shift, Hh.rand(g, H, N, lo=-1, hi=1), 0.1 * Hh.randn(g, B, H, N, N)
+    yo, sTo = O.wkv6(*(x.to(BF).double() for x in (r, k, v, w, u)), H, s0=s0.double(), return_state=True)
+    d = [x.to(BF).to("cuda").contiguous() for x in (r, k, v, w, u)]
+    y, sT = torch.full((B, T, C), float("nan"), dtype=BF, device="cuda"), torch.full((B, H, N, N), float("nan"), device="cuda")
+    R.ops.wkv6state_forward_ex(B, T, C, H, *d, s0.to("cuda"), y, sT)
+    Hh.assert_close(y, yo, Hh.TOL_BF16, "y")
+    Hh.assert_close(sT, sTo, Hh.TOL_BF16, "sT")
