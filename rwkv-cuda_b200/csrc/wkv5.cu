@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(NMAX) wkv5_backward_kernel(
 
 template <typename E>
 bool chunked_ok(int T, int N, std::initializer_list<const void*> ps) {
-    if (!std::is_same<E, bf16>::value || N != 64 || (T % 16 != 0 && !wkv6_ragged_ok(T))) return false;
+    if (!std::is_same<E, bf16>::value || N != 64 || T % 16 != 0) return false;
     for (const void* p : ps)
         if (p != nullptr && (reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
     return true;
@@ -247,9 +247,8 @@ int launch_fwd(int B, int T, int C, int H, const void* r, const void* k, const v
         int* flag = wkv6_chunked_flag(st);   // NULL: every slot is taken, the general-shape kernel runs alone
         if (flag != nullptr) {
             RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA, "wkv5_forward: clearing the device flag failed");
-            const int e = wkv6_chunked_forward(B, T, H, r, k, v, w1, 2, u1, nullptr, 0, y, nullptr, nullptr, flag, st);
-            if (e < 0) return e;
-            if (e == 0) only_if = flag;   // 1: no kernel for this T here, the general-shape kernel runs alone
+            if (int e = wkv6_chunked_forward(B, T, H, r, k, v, w1, 2, u1, nullptr, 0, y, nullptr, nullptr, flag, st)) return e;
+            only_if = flag;
         }
     }
 #define RWKV_GO(NM)                                                                                           \
@@ -271,17 +270,17 @@ int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const v
                void* scratch = nullptr, float* gw32 = nullptr, float* gu32 = nullptr) {
     const int N = C / H;
     const int* only_if = nullptr;
-    if (!DUAL && scratch != nullptr && (T % 16 == 0 || wkv6_states_fit(B, T, H)) && chunked_ok<E>(T, N, {r, k, v, u1, gy, gr, gk, gv, gw1, gu1, scratch})) {
+    if (!DUAL && scratch != nullptr && chunked_ok<E>(T, N, {r, k, v, u1, gy, gr, gk, gv, gw1, gu1, scratch})) {
         // chunked forward into the scratch buffer (chunk-start states), chunked reverse pass, then the
         // general-shape kernel only if the decay is too strong for the chunked form
         int* flag = wkv6_chunked_flag(st);   // NULL: every slot is taken, the general-shape kernel runs alone
         if (flag != nullptr) {
             RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA, "wkv5_backward: clearing the device flag failed");
             float* ck = static_cast<float*>(scratch);
-            const int e = wkv6_backward_with_states(B, T, H, r, k, v, ww1, 3, u1, nullptr, 0, gy, nullptr, ck, gr, gk, gv, gw1, gu1,
-                                                    nullptr, 0, flag, st, gw32, gu32);
-            if (e < 0) return e;
-            if (e == 0) only_if = flag;
+            if (int e = wkv6_backward_with_states(B, T, H, r, k, v, ww1, 3, u1, nullptr, 0, gy, nullptr, ck, gr, gk, gv, gw1, gu1,
+                                                  nullptr, 0, flag, st, gw32, gu32))
+                return e;
+            only_if = flag;
         }
     }
 #define RWKV_GO(NM)                                                                                              \
@@ -456,8 +455,8 @@ extern "C" int rwkvb200_wkv5_backward_saved(int dtype, int B, int T, int C, int 
 }
 
 // ---- training flow: the harness's pre- and post-operations inside the kernels -------------------------------------------
-// Path 0: bf16 / head size 64 on the tcgen05 kernels (as rwkvb200_wkv5_forward_saved); 1: other head sizes up to 64 and fp32 on
-// the segments of wkv5_seg.cu; 2: larger heads on the general-shape kernels.
+// Path 0: bf16 / head size 64 / T a multiple of 16 on the tcgen05 kernels (as rwkvb200_wkv5_forward_saved); 1: everything else up to
+// head size 64 in fp32 arithmetic on the segments of wkv5_seg.cu; 2: larger heads on the general-shape kernels.
 extern "C" size_t rwkvb200_wkv5_train_saved_bytes(int B, int T, int C, int H) {
     if (B <= 0 || T <= 0 || C <= 0 || H <= 0) return 0;
     return (size_t)B * H * (wkv5_seg_count(T) * (C / H) * (C / H) + 1) * sizeof(float);   // a state per 32 tokens and a flag per unit

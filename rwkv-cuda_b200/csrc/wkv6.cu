@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "wkv6_chunked.cuh"
 #include "wkv6_tsplit.cuh"
+#include "wkv6_seg.cuh"
 #include <initializer_list>
 #include <type_traits>
 
@@ -246,12 +247,9 @@ __global__ void __launch_bounds__(NMAX) wkv6_backward_kernel(
 
 static int g_wkv6_chunked_enabled = 1;
 
-// fp32_state_out: the call returns a state or its gradient in fp32.  Such a call with a ragged T stays on the fp32
-// general-shape kernels: TF32 operands would cost that output three digits (bf16 outputs are rounded more coarsely than that).
 template <typename E>
-bool chunked_ok(int T, int N, bool fp32_state_out, std::initializer_list<const void*> ps) {
-    if (!g_wkv6_chunked_enabled || !std::is_same<E, bf16>::value || N != 64) return false;
-    if (T % 16 != 0 && (fp32_state_out || !wkv6_ragged_ok(T))) return false;
+bool chunked_ok(int T, int N, std::initializer_list<const void*> ps) {
+    if (!g_wkv6_chunked_enabled || !std::is_same<E, bf16>::value || N != 64 || T % 16 != 0) return false;
     for (const void* p : ps)
         if (p != nullptr && (reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
     return true;
@@ -262,15 +260,14 @@ int launch_fwd(int B, int T, int C, int H, const void* r, const void* k, const v
                const void* u, const void* s0, int s0_kind, void* y, float* sT, cudaStream_t st, const char* what) {
     const int N = C / H;
     const int* only_if = nullptr;
-    if (chunked_ok<E>(T, N, sT != nullptr, {r, k, v, w, u, s0, y, sT})) {
+    if (chunked_ok<E>(T, N, {r, k, v, w, u, s0, y, sT})) {
         // tensor-core kernel first; the general-shape kernel below then only runs if that one found a
         // chunk whose decay is too strong for the chunked form
         int* flag = wkv6_chunked_flag(st);   // NULL: every slot is taken, the general-shape kernel runs alone
         if (flag != nullptr) {
             RWKV_REQUIRE(cudaMemsetAsync(flag, 0, sizeof(int) * kChunkedFlagUnits, st) == cudaSuccess, RWKVB200_ECUDA, "%s: clearing the device flag failed", what);
-            const int e = wkv6_chunked_forward(B, T, H, r, k, v, w, w_raw, u, s0, s0_kind, y, sT, nullptr, flag, st);
-            if (e < 0) return e;
-            if (e == 0) only_if = flag;   // 1: no kernel for this T here, the general-shape kernel runs alone
+            if (int e = wkv6_chunked_forward(B, T, H, r, k, v, w, w_raw, u, s0, s0_kind, y, sT, nullptr, flag, st)) return e;
+            only_if = flag;
         }
     }
 #define RWKV_GO(NM)                                                                                              \
@@ -292,7 +289,7 @@ int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const v
                const char* what, bool big_scratch = true, float* gu32 = nullptr) {
     const int N = C / H;
     const int* only_if = nullptr;
-    if (big_scratch && T % 16 == 0 && chunked_ok<E>(T, N, true, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, scratch})) {
+    if (big_scratch && chunked_ok<E>(T, N, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, scratch})) {
         // tensor-core kernels first: a forward pass that leaves the chunk-start states in the scratch
         // buffer, then the reverse pass; the general-shape kernel below then only runs if a chunk's decay
         // was too strong for the chunked form (it reuses the front of the same scratch buffer)
@@ -325,7 +322,7 @@ int launch_bwd(int B, int T, int C, int H, const void* r, const void* k, const v
 int tensor_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
                    const float* s0, void* y, float* sT, void* saved, cudaStream_t st, const char* what) {
     const int N = C / H, sk = s0 ? kF32 : kNone;
-    if (dtype != RWKVB200_BF16 || !wkv6_forward_choice() || !chunked_ok<bf16>(T, N, sT != nullptr, {r, k, v, w, u, s0, y, sT, saved})) return 1;
+    if (dtype != RWKVB200_BF16 || !wkv6_forward_choice() || !chunked_ok<bf16>(T, N, {r, k, v, w, u, s0, y, sT, saved})) return 1;
     int* flags = wkv6_saved_flags(saved, B, T, H);
     const int rc = wkv6_l32_forward(B, T, H, r, k, v, w, 1, u, s0, sk, y, sT, static_cast<float*>(saved), flags, st, 0);
     if (rc != 0) return rc;
@@ -506,7 +503,7 @@ extern "C" int rwkvb200_wkv6state_forward_tsplit(int dtype, int B, int T, int C,
     const int K = segments, N = C / H;
     RWKV_REQUIRE(K >= 1 && T % K == 0 && (T / K) % 16 == 0, RWKVB200_EINVAL,
                  "wkv6state_forward_tsplit: T = %d is not %d segments of a multiple of 16 tokens", T, K);
-    RWKV_REQUIRE(dtype == RWKVB200_BF16 && (T / K) % 16 == 0 && chunked_ok<bf16>(T / K, N, true, {r, k, v, w, u, s0, y, sT, work}), RWKVB200_EINVAL,
+    RWKV_REQUIRE(dtype == RWKVB200_BF16 && chunked_ok<bf16>(T / K, N, {r, k, v, w, u, s0, y, sT, work}), RWKVB200_EINVAL,
                  "wkv6state_forward_tsplit: needs bf16 tensors, head size 64, 16-byte alignment");
     cudaStream_t st = as_stream(stream);
     int* flag = wkv6_chunked_flag(st);
@@ -558,7 +555,7 @@ extern "C" int rwkvb200_wkv6state_backward_saved(int dtype, int B, int T, int C,
     RWKV_NOTNULL(gr); RWKV_NOTNULL(gk); RWKV_NOTNULL(gv); RWKV_NOTNULL(gw); RWKV_NOTNULL(gu); RWKV_NOTNULL(saved);
     const int sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
     cudaStream_t st = as_stream(stream);
-    if (saved_valid && dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, C / H, ds0 != nullptr, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, saved}))
+    if (saved_valid && dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, C / H, {r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, saved}))
         // (flagged units: the general-shape kernel uses the front of `saved` as its scratch, after the states have been read)
         return tensor_backward(B, T, C, H, r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, nullptr, saved, static_cast<float*>(saved), st, "wkv6state_backward_saved");
     return dtype == RWKVB200_F32
@@ -569,8 +566,10 @@ extern "C" int rwkvb200_wkv6state_backward_saved(int dtype, int B, int T, int C,
 // ---- training flow: gu summed over the batch inside the library, buffers of the size that the path needs -----------------
 // (the flagged units of the tcgen05 backward use the states in `saved` as scratch, as in rwkvb200_wkv6state_backward_saved:
 // they hold 2 floats per element and the scratch takes one)
+// Path 0: the tcgen05 kernels; 2: fp32 arithmetic split over time (wkv6_seg.cu); 1: everything else.
 extern "C" size_t rwkvb200_wkv6_train_saved_bytes(int dtype, int B, int T, int C, int H) {
     if (B <= 0 || T <= 0 || C <= 0 || H <= 0 || dtype != RWKVB200_BF16 || C / H != 64) return 16;
+    if (wkv6_seg_applies(dtype, T, C / H, false)) return wkv6_seg_saved(B, T, H) * sizeof(float);
     return (size_t)B * H * ((size_t)((T + 31) / 32) * 64 * 64 + 1) * sizeof(float);
 }
 
@@ -581,6 +580,10 @@ extern "C" int rwkvb200_wkv6_train_forward(int dtype, int B, int T, int C, int H
     cudaStream_t st = as_stream(stream);
     const int rc = tensor_forward(dtype, B, T, C, H, r, k, v, w, u, s0, y, sT, saved, st, "wkv6_train_forward");
     if (rc != 1) return rc;
+    if (wkv6_seg_applies(dtype, T, C / H, s0 != nullptr || sT != nullptr)) {
+        const int e = wkv6_seg_forward(B, T, H, r, k, v, w, u, y, static_cast<float*>(saved), st);
+        return e ? e : 2;
+    }
     const int sk = s0 ? kF32 : kNone;
     const int e = dtype == RWKVB200_F32 ? launch_fwd<float>(B, T, C, H, r, k, v, w, 1, u, s0, sk, y, sT, st, "wkv6_train_forward")
                                         : launch_fwd<bf16>(B, T, C, H, r, k, v, w, 1, u, s0, sk, y, sT, st, "wkv6_train_forward");
@@ -589,6 +592,7 @@ extern "C" int rwkvb200_wkv6_train_forward(int dtype, int B, int T, int C, int H
 
 extern "C" size_t rwkvb200_wkv6_train_work_bytes(int B, int T, int C, int path) {
     if (B <= 0 || T <= 0 || C <= 0) return 0;
+    if (path == 2) return (wkv6_seg_adjoints(B, T, C) + wkv6_seg_rows(B, T) * C) * sizeof(float);
     return (size_t)B * C * sizeof(float) + (path == 0 ? 0 : rwkvb200_wkv6_scratch_bytes(B, T, C));
 }
 
@@ -599,6 +603,12 @@ extern "C" int rwkvb200_wkv6_train_backward(int dtype, int B, int T, int C, int 
     RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w); RWKV_NOTNULL(u); RWKV_NOTNULL(gy);
     RWKV_NOTNULL(gr); RWKV_NOTNULL(gk); RWKV_NOTNULL(gv); RWKV_NOTNULL(gw); RWKV_NOTNULL(gu); RWKV_NOTNULL(saved); RWKV_NOTNULL(work);
     cudaStream_t st = as_stream(stream);
+    if (path == 2) {
+        RWKV_REQUIRE(wkv6_seg_applies(dtype, T, C / H, s0 != nullptr || dsT != nullptr || ds0 != nullptr), RWKVB200_EINVAL, "wkv6_train_backward: not a call of path 2");
+        float *adjoints = static_cast<float*>(work), *partial = adjoints + wkv6_seg_adjoints(B, T, C);
+        const int e = wkv6_seg_backward(B, T, H, r, k, v, w, u, gy, gr, gk, gv, gw, static_cast<const float*>(saved), adjoints, partial, st);
+        return e ? e : sum_rows(dtype, wkv6_seg_rows(B, T), C, partial, gu, st);
+    }
     const int sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
     float* scratch = static_cast<float*>(work);   // (path 1; the partials of gu come behind it)
     float* gu32 = path == 0 ? scratch : scratch + rwkvb200_wkv6_scratch_bytes(B, T, C) / sizeof(float);

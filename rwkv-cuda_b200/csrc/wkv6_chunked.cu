@@ -660,7 +660,6 @@ int wkv6_chunked_forward(int B, int T, int H, const void* r, const void* k, cons
         const int rc = wkv6_l32_forward(B, T, H, r, k, v, w, w_mode, u, s0, s0_kind, y, sT, nullptr, unsafe, st, flag_div);
         if (rc != 1) return rc;
     }
-    if (T % L != 0) return 1;
     RWKV_REQUIRE(w_mode >= 0 && w_mode <= 3, RWKVB200_EINVAL, "wkv6_forward(chunked): decay mode %d", w_mode);
     dim3 grid(H, B);
 #define RWKV_GO1(M, SO)                                                                                                \
@@ -701,7 +700,7 @@ int wkv6_backward_with_states(int B, int T, int H, const void* r, const void* k,
             return wkv6_l32_backward(B, T, H, r, k, v, w, w_mode, u, gy, dsT, ck, gr, gk, gv, gw, gu, ds0, ds0_kind, st, gw32, gu32);
         }
     }
-    if (int e = wkv6_chunked_forward(B, T, H, r, k, v, w, w_mode, u, s0, s0_kind, nullptr, nullptr, ck, unsafe, st)) return e;   // (1: see above)
+    if (int e = wkv6_chunked_forward(B, T, H, r, k, v, w, w_mode, u, s0, s0_kind, nullptr, nullptr, ck, unsafe, st)) return e;
     return wkv6_chunked_backward(B, T, H, r, k, v, w, w_mode, u, gy, dsT, ck, gr, gk, gv, gw, gu, ds0, ds0_kind, st, gw32, gu32);
 }
 

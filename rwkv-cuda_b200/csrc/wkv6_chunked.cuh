@@ -1,4 +1,4 @@
-// Launchers of the chunked (tensor-core) RWKV-6 kernels: bf16, head size 64, T a multiple of 16 (mma.sync) or any T (tcgen05).
+// Launchers of the chunked (tensor-core) RWKV-6 kernels: bf16, head size 64, T a multiple of 16.
 #pragma once
 #include "common.cuh"
 
@@ -44,13 +44,6 @@ int wkv6_backward_with_states(int B, int T, int H, const void* r, const void* k,
                               void* gk, void* gv, void* gw, void* gu, void* ds0, int ds0_kind, int* unsafe, cudaStream_t st,
                               float* gw32 = nullptr, float* gu32 = nullptr);
 int wkv6_forward_choice();
-// wkv6_chunked_forward and wkv6_backward_with_states return 1, with nothing enqueued, when T is not a multiple of 16 and
-// the tcgen05 kernels cannot run here.
-
-// T that is not a multiple of 16: only the tcgen05 kernels mask the tokens of a partial chunk.  A partial chunk costs as
-// much as a whole one, about 2 us, the time in which the general-shape forward takes two or three tokens: from one chunk on
-// they win.
-inline bool wkv6_ragged_ok(int T) { return T >= 32 && wkv6_forward_choice() && !tensor_maps_disabled(); }
 
 // the "decay too strong" flags of the calling stream: kChunkedFlagUnits ints, one per (batch, head) unit modulo that
 constexpr int kChunkedFlagUnits = 1024;

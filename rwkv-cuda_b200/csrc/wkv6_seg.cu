@@ -1,0 +1,310 @@
+// RWKV-6 training in fp32 arithmetic, bf16 activations, head size 64, no state in or out, split over time: the lengths that
+// are not whole tiles of the tensor-core kernels (wkv6_seg_applies).
+//
+// Per (batch, head), S indexed [key j][value i], d_t[j] = exp(-exp(w_t[j])) the decay of token t:
+//   y_t[i] = sum_j r_t[j] S_{t-1}[j,i] + v_t[i] sum_j r_t u k_t      S_t[j,i] = d_t[j] S_{t-1}[j,i] + k_t[j] v_t[i]
+// The steps are those of wkv5_seg.cu, with the products of the token decays in place of powers of one decay:
+//   local   the end state of every segment of 32 tokens from a zero start: sum_s (prod_{tau>s} d_tau) k_s v_s^T.  The products are
+//           put on k when it is staged; they are <= 1, so nothing can overflow, whatever the decays are;
+//   scan    start states of the segments, in place: S <- S diag(prod d) + local;
+//   y       every segment again, token by token from its start state.
+// Backward: the same two steps for the adjoint D = dL/dS (k, v -> r, gy, time reversed), then one block per segment: two warps
+// carry S forward (gr) while two carry D backward (gk, gv).  For the decay gradient they leave P_t = r_t sum_i gy_t S_{t-1} and
+// Q_t = k_t sum_i D_t v_t, and with A_t = sum_i D_{t-1}[j,i] S_{t-1}[j,i] (D_t: before token t is taken in, S_t: after it)
+//   dL/dlog d_t = A_{t+1} - Q_t       A_t = A_{t+1} - Q_t + P_t       (wkv6.cu)
+// walked over the segment's tokens only: A at its end is taken from the two states there.
+//
+// What bounds it: multiply-adds of the FP32 pipe, one per state element, token and product (9 of them forward + backward), and
+// the shared-memory reads of the token's vectors.  B8 T1000 H32, forward + backward on a B200: 4374 us on the general-shape
+// kernels, which walk the tokens with one block per unit; 1237 us here.  The tensor-core kernels take 258 us, but their operands
+// are TF32: outputs are then 2 to 4 % further from fp64 in norm than one rounding to bf16 (1.72e-3 instead of 1.66e-3; here
+// 1.66e-3), and gw 1.3e-2 instead of 3.9e-3 at its worst element.
+#include "wkv6_seg.cuh"
+#include "seg_tiles.cuh"
+
+namespace rwkvb200 {
+namespace {
+
+__device__ __forceinline__ float log_decay(const bf16* w_raw) { return -expf(to_f(*w_raw)); }
+
+// d of the segment's tokens as rows in the order of place(); 1 where there is no token.
+template <int NTH>
+__device__ __forceinline__ void stage_decay(float* dst, const bf16* __restrict__ w, int n, int C, int tid) {
+    stage<NTH>(dst, w, n, C, kN, tid);
+    // (each element is changed by the thread that reads it here, whichever thread has staged it)
+    __syncthreads();
+    for (int x = tid; x < kSeg * kN; x += NTH) dst[x] = x < n * kN ? expf(-expf(dst[x])) : 1.f;
+}
+
+// In place: local end states -> state before each segment (REV: adjoint after each segment).  One thread per state element.
+template <bool REV>
+__global__ void __launch_bounds__(256) seg6_scan_kernel(int nseg, const float* __restrict__ decays, float* __restrict__ states) {
+    const i64 unit = blockIdx.x / (kN * kN / 256);
+    const int e = blockIdx.x % (kN * kN / 256) * 256 + threadIdx.x;
+    const float* d = decays + unit * nseg * kN + place(e / kN);
+    float* p = states + unit * nseg * kN * kN + e;
+    constexpr int AHEAD = 16;
+    float cur = 0.f;
+    for (int k0 = 0; k0 < nseg; k0 += AHEAD) {   // the loads of AHEAD segments are in flight together
+        float x[AHEAD], f[AHEAD];
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q)
+            if (k0 + q < nseg) {
+                const i64 k = REV ? nseg - 1 - k0 - q : k0 + q;
+                x[q] = p[k * kN * kN];
+                f[q] = d[k * kN];
+            }
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q)
+            if (k0 + q < nseg) {
+                p[(i64)(REV ? nseg - 1 - k0 - q : k0 + q) * kN * kN] = cur;
+                cur = fmaf(cur, f[q], x[q]);
+            }
+    }
+}
+
+// One block per (unit, segment), 2 warps: a warp has the keys 32 warp .. of all values, a lane 8 keys x 8 values.
+// REV = false: a = k, b = v, and the product of the segment's decays goes to `decays`; REV = true: a = r, b = gy.
+template <bool REV>
+__global__ void __launch_bounds__(64) seg6_local_kernel(int T, int H, int nseg, const bf16* __restrict__ a_, const bf16* __restrict__ b_,
+                                                        const bf16* __restrict__ w_, float* __restrict__ states, float* __restrict__ decays) {
+    __shared__ __align__(16) float as[kSeg * kN], bs[kSeg * kN], ds[kSeg * kN];
+    const i64 unit = blockIdx.x / nseg;
+    const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, C = H * kN;
+    const int n = min(kSeg, T - seg * kSeg);
+    const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    stage<64>(as, a_ + base, n, C, kN, tid);
+    stage<64>(bs, b_ + base, n, C, kN, tid);
+    stage_decay<64>(ds, w_ + base, n, C, tid);
+    __syncthreads();
+    {   // a, times the decay between its token and the end (REV: the start) of the segment: a thread per channel
+        float f = 1.f;
+#pragma unroll 8
+        for (int q = 0; q < kSeg; ++q) {
+            const int t = REV ? q : kSeg - 1 - q;
+            as[t * kN + tid] *= f;
+            f *= ds[t * kN + tid];
+        }
+        if (!REV) decays[(i64)blockIdx.x * kN + tid] = f;
+    }
+    __syncthreads();
+    const int kg = 4 * (tid >> 5) + (lane & 3), vg = lane >> 2;
+    Tile s;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) s[i][p] = 0ull;
+#pragma unroll 2
+    for (int t = 0; t < n; ++t) {
+        f2 a[4], b[8];
+        pairs(load8(as + t * kN, kg), a);
+        twice(load8(bs + t * kN, vg), b);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int p = 0; p < 4; ++p) s[i][p] = fma2(a[p], b[i], s[i][p]);
+    }
+    store_tile(s, states + (i64)blockIdx.x * kN * kN, 8 * kg, 8 * vg, kN);
+}
+
+// One block per (unit, segment), 2 warps: a warp has the values 32 warp .. of all keys
+__global__ void __launch_bounds__(64) seg6_y_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
+                                                    const bf16* __restrict__ v_, const bf16* __restrict__ w_, const bf16* __restrict__ u_,
+                                                    const float* __restrict__ states, bf16* __restrict__ y_) {
+    __shared__ __align__(16) float rs[kSeg * kN], ks[kSeg * kN], vs[kSeg * kN], ds[kSeg * kN], us[kN], ruk[kSeg];
+    const i64 unit = blockIdx.x / nseg;
+    const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
+    const int n = min(kSeg, T - seg * kSeg);
+    const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    const int kg = lane >> 2, vg = 4 * warp + (lane & 3);
+    Tile s;
+    load_tile(s, states + (i64)blockIdx.x * kN * kN, 8 * kg, 8 * vg, kN);
+    stage<64>(rs, r_ + base, n, C, kN, tid);
+    stage<64>(ks, k_ + base, n, C, kN, tid);
+    stage<64>(vs, v_ + base, n, C, kN, tid);
+    us[place(tid)] = to_f(u_[h * kN + tid]);
+    stage_decay<64>(ds, w_ + base, n, C, tid);
+    __syncthreads();
+    for (int t = warp; t < n; t += 2) {   // the bonus of a token: one warp each
+        float x = fmaf(rs[t * kN + lane] * us[lane], ks[t * kN + lane], rs[t * kN + 32 + lane] * us[32 + lane] * ks[t * kN + 32 + lane]);
+#pragma unroll
+        for (int m = 16; m; m >>= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
+        if (lane == 0) ruk[t] = x;
+    }
+    __syncthreads();
+    const int i_out = 8 * vg + kg;   // the value whose sum this lane ends with
+    for (int t = 0; t < n; ++t) {
+        f2 r[4], k[4], d[4], v[8];
+        pairs(load8(rs + t * kN, kg), r);
+        pairs(load8(ks + t * kN, kg), k);
+        pairs(load8(ds + t * kN, kg), d);
+        twice(load8(vs + t * kN, vg), v);
+        float y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            f2 acc = mul2(s[i][0], r[0]);
+#pragma unroll
+            for (int p = 1; p < 4; ++p) acc = fma2(s[i][p], r[p], acc);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) s[i][p] = fma2(s[i][p], d[p], mul2(k[p], v[i]));
+            y[i] = sum2(acc);
+        }
+        const float yo = reduce8(y, lane);
+        y_[base + (i64)t * C + i_out] = from_f<bf16>(fmaf(vs[t * kN + place(i_out)], ruk[t], yo));
+    }
+}
+
+// One block per (unit, segment), 4 warps: warps 0, 1 carry S forward (gr, gu, P), warps 2, 3 carry D backward (gk, gv, Q); a warp
+// has 32 keys of all values.  gv sums over all keys: the two halves meet in shared memory at the end.
+struct Bwd6Smem {
+    float r[kSeg * kN], k[kSeg * kN], v[kSeg * kN], g[kSeg * kN], d[kSeg * kN], gv[2][kSeg * kN];
+    float P[kSeg * kN], Q[kSeg * kN], A[kN];   // [token][channel]
+    float u[kN], vg[kSeg], ruk[kSeg];
+};
+
+__global__ void __launch_bounds__(128, 3) seg6_backward_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
+                                                               const bf16* __restrict__ v_, const bf16* __restrict__ w_,
+                                                               const bf16* __restrict__ u_, const bf16* __restrict__ gy_,
+                                                               const float* __restrict__ S_, const float* __restrict__ D_, bf16* __restrict__ gr_,
+                                                               bf16* __restrict__ gk_, bf16* __restrict__ gv_, bf16* __restrict__ gw_,
+                                                               float* __restrict__ gu_) {
+    extern __shared__ __align__(16) unsigned char smem_seg6[];
+    Bwd6Smem& sm = *reinterpret_cast<Bwd6Smem*>(smem_seg6);
+    const i64 unit = blockIdx.x / nseg;
+    const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
+    const int n = min(kSeg, T - seg * kSeg);
+    const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    const float* D0 = D_ + (i64)blockIdx.x * kN * kN;
+    const int kg = 4 * (warp & 1) + (lane & 3), vg = lane >> 2, j_out = 8 * kg + vg;   // j_out: the key whose sums this lane ends with
+    Tile s;
+    load_tile(s, warp < 2 ? S_ + (i64)blockIdx.x * kN * kN : D0, 8 * kg, 8 * vg, kN);
+    stage<128>(sm.r, r_ + base, n, C, kN, tid);
+    stage<128>(sm.k, k_ + base, n, C, kN, tid);
+    stage<128>(sm.v, v_ + base, n, C, kN, tid);
+    stage<128>(sm.g, gy_ + base, n, C, kN, tid);
+    if (tid < kN) sm.u[place(tid)] = to_f(u_[h * kN + tid]);
+    stage_decay<128>(sm.d, w_ + base, n, C, tid);
+    __syncthreads();
+    for (int t = warp; t < n; t += 4) {   // sums of a token over its channels: one warp each
+        const float *r = sm.r + t * kN, *k = sm.k + t * kN, *v = sm.v + t * kN, *g = sm.g + t * kN;
+        float x = fmaf(r[lane] * sm.u[lane], k[lane], r[lane + 32] * sm.u[lane + 32] * k[lane + 32]);
+        float z = fmaf(v[lane], g[lane], v[lane + 32] * g[lane + 32]);
+#pragma unroll
+        for (int m = 16; m; m >>= 1) { x += __shfl_xor_sync(0xffffffffu, x, m); z += __shfl_xor_sync(0xffffffffu, z, m); }
+        if (lane == 0) { sm.ruk[t] = x; sm.vg[t] = z; }
+    }
+    __syncthreads();
+    const float uj = sm.u[place(j_out)];
+    if (warp < 2) {
+        float gu = 0.f;
+        for (int t = 0; t < n; ++t) {
+            f2 k[4], d[4], v[8], g[8], sg[4];
+            pairs(load8(sm.k + t * kN, kg), k);
+            pairs(load8(sm.d + t * kN, kg), d);
+            twice(load8(sm.v + t * kN, vg), v);
+            twice(load8(sm.g + t * kN, vg), g);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    sg[p] = i ? fma2(s[i][p], g[i], sg[p]) : mul2(s[i][p], g[i]);
+                    s[i][p] = fma2(s[i][p], d[p], mul2(k[p], v[i]));
+                }
+            float x[8];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) unpack2(sg[p], x[2 * p], x[2 * p + 1]);
+            const float sgj = reduce8(x, lane), rj = sm.r[t * kN + place(j_out)], kj = sm.k[t * kN + place(j_out)], vgt = sm.vg[t];
+            gr_[base + (i64)t * C + j_out] = from_f<bf16>(fmaf(uj * kj, vgt, sgj));
+            sm.P[t * kN + j_out] = rj * sgj;
+            gu = fmaf(rj * kj, vgt, gu);
+        }
+        f2 a2[4] = {0ull, 0ull, 0ull, 0ull};   // A at the end: sum over values of D_end S_end
+        float x[8];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            f2 e[8];
+            load_pair(e, p, D0, 8 * kg, 8 * vg, kN);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a2[p] = fma2(e[i], s[i][p], a2[p]);
+            unpack2(a2[p], x[2 * p], x[2 * p + 1]);
+        }
+        sm.A[j_out] = reduce8(x, lane);
+        gu_[(unit / H * nseg + seg) * C + h * kN + j_out] = gu;
+    } else {
+        for (int t = n - 1; t >= 0; --t) {
+            f2 r[4], k[4], d[4], v[8], g[8];
+            pairs(load8(sm.r + t * kN, kg), r);
+            pairs(load8(sm.k + t * kN, kg), k);
+            pairs(load8(sm.d + t * kN, kg), d);
+            twice(load8(sm.v + t * kN, vg), v);
+            twice(load8(sm.g + t * kN, vg), g);
+            f2 gk[4];
+            float x[8], y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                f2 acc = mul2(s[i][0], k[0]);
+#pragma unroll
+                for (int p = 1; p < 4; ++p) acc = fma2(s[i][p], k[p], acc);
+                y[i] = sum2(acc);
+#pragma unroll
+                for (int p = 0; p < 4; ++p) {
+                    gk[p] = i ? fma2(s[i][p], v[i], gk[p]) : mul2(s[i][p], v[i]);
+                    s[i][p] = fma2(s[i][p], d[p], mul2(r[p], g[i]));
+                }
+            }
+#pragma unroll
+            for (int p = 0; p < 4; ++p) unpack2(gk[p], x[2 * p], x[2 * p + 1]);
+            const float dv = reduce8(x, lane);
+            gk_[base + (i64)t * C + j_out] = from_f<bf16>(fmaf(uj * sm.r[t * kN + place(j_out)], sm.vg[t], dv));
+            sm.Q[t * kN + j_out] = sm.k[t * kN + place(j_out)] * dv;
+            reduce8_pairs(y, lane);
+            *reinterpret_cast<float2*>(sm.gv[warp - 2] + t * kN + 8 * vg + 2 * (lane & 3)) = make_float2(y[0], y[1]);
+        }
+    }
+    __syncthreads();
+    if (warp < 2) {   // the decay gradient: a thread per channel
+        float A = sm.A[tid];
+        for (int t = n - 1; t >= 0; --t) {
+            const i64 o = base + (i64)t * C + tid;
+            A -= sm.Q[t * kN + tid];
+            gw_[o] = from_f<bf16>(A * log_decay(w_ + o));   // d log d / d w_raw = log d
+            A += sm.P[t * kN + tid];
+        }
+    } else {
+        const int i = tid - 64;
+        for (int t = 0; t < n; ++t)
+            gv_[base + (i64)t * C + i] = from_f<bf16>(fmaf(sm.g[t * kN + place(i)], sm.ruk[t], sm.gv[0][t * kN + i] + sm.gv[1][t * kN + i]));
+    }
+}
+
+}  // namespace
+
+int wkv6_seg_forward(int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u, void* y, float* saved,
+                     cudaStream_t st) {
+    const int nseg = (T + kSeg - 1) / kSeg;
+    const i64 units = (i64)B * H;
+    RWKV_REQUIRE(units * nseg < (1ll << 31), RWKVB200_EINVAL, "wkv6_train_forward: too many segments");
+    float* decays = saved + units * nseg * kN * kN;
+    const unsigned grid = (unsigned)(units * nseg), scan = (unsigned)(units * (kN * kN / 256));
+    seg6_local_kernel<false><<<grid, 64, 0, st>>>(T, H, nseg, (const bf16*)k, (const bf16*)v, (const bf16*)w, saved, decays);
+    seg6_scan_kernel<false><<<scan, 256, 0, st>>>(nseg, decays, saved);
+    seg6_y_kernel<<<grid, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, saved, (bf16*)y);
+    return check_launch("wkv6_train_forward(segments)");
+}
+
+int wkv6_seg_backward(int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u, const void* gy, void* gr,
+                      void* gk, void* gv, void* gw, const float* saved, float* adjoints, float* gu_partial, cudaStream_t st) {
+    const int nseg = (T + kSeg - 1) / kSeg;
+    const i64 units = (i64)B * H;
+    const float* decays = saved + units * nseg * kN * kN;
+    const unsigned grid = (unsigned)(units * nseg), scan = (unsigned)(units * (kN * kN / 256));
+    const cudaError_t e = allow_smem<seg6_backward_kernel>(sizeof(Bwd6Smem));
+    RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv6_train_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    seg6_local_kernel<true><<<grid, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)gy, (const bf16*)w, adjoints, nullptr);
+    seg6_scan_kernel<true><<<scan, 256, 0, st>>>(nseg, decays, adjoints);
+    seg6_backward_kernel<<<grid, 128, sizeof(Bwd6Smem), st>>>(T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u,
+                                                              (const bf16*)gy, saved, adjoints, (bf16*)gr, (bf16*)gk, (bf16*)gv, (bf16*)gw, gu_partial);
+    return check_launch("wkv6_train_backward(segments)");
+}
+
+}  // namespace rwkvb200

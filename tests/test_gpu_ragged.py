@@ -1,5 +1,5 @@
-"""GPU parity at sequence lengths that are not whole chunks: the tensor-core kernels of RWKV-5 and RWKV-6 mask the tokens
-of a partial 32-token chunk.  Against the fp64 oracle, through the training classes."""
+"""GPU parity at sequence lengths that are not whole chunks, against the fp64 oracle, through the training classes.  RWKV-5 and
+RWKV-6 compute them in fp32, split over time into segments of 32 tokens."""
 import pytest
 import torch
 
@@ -34,6 +34,26 @@ def test_training_at_any_length(op, B, T, H):
     want = grads(lambda *xs: oracle(*xs, H), (r, k, v, w, u), gy)
     for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
         Hh.assert_close(a, b, Hh.TOL_BF16, f"{op} {name}")
+
+
+@pytest.mark.parametrize("op", ["wkv5", "wkv6"])
+@pytest.mark.parametrize("B,T,H", [(2, 33, 1), (1, 47, 3), (2, 191, 2), (1, 1000, 2)])
+def test_fp32_arithmetic_where_T_is_ragged(op, B, T, H):
+    """Every output is one rounding to bf16 away from fp64 (2^-8 of the value at most; TF32 operands add a few 2^-11 of the output's
+    size), and fp32 sums over at most 1000 tokens of 64 keys add less than 2^-15 of it."""
+    import rwkv_cuda_b200 as R
+    g = Hh.gen(T)
+    N, C = 64, H * 64
+    r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
+    u, gy = Hh.rand(g, H, N, lo=-1, hi=1), Hh.randn(g, B, T, C)
+    w = Hh.rand(g, H, N, lo=-6, hi=-1) if op == "wkv5" else Hh.randn(g, B, T, C) - 5.0
+    ours, oracle = (R.functions.WKV_5, O.wkv5) if op == "wkv5" else (R.functions.WKV_6, O.wkv6)
+    got = grads(lambda *xs: ours.apply(B, T, C, H, *xs), (r, k, v, w, u), gy, "cuda")
+    want = grads(lambda *xs: oracle(*xs, H), (r, k, v, w, u), gy)
+    for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
+        size = torch.maximum(b.abs(), b.square().mean().sqrt())
+        err = ((a.double().cpu().reshape(b.shape) - b).abs() / size).max().item()
+        assert err <= 2 ** -8 + 2 ** -15, f"{op} {name}: {err:.3e}"
 
 
 @pytest.mark.parametrize("use_s0", [False, True])
