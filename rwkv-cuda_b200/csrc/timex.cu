@@ -9,7 +9,7 @@
 //   forward: F = w[c] (shared by the batch), G = k[b,c]
 //   gw     : F = g[b,c] (one per batch),     G = k[b,c]
 //   gk     : F = w[c], G = g[b,c] read back to front, and the output written back to front.
-// so one kernel template serves them.  (Lengths of 65 to 1024 go through timex_fft.cu; the gradient per batch row and other
+// so one kernel template serves them.  (Lengths of 257 to 1024 go through timex_fft.cu; the gradient per batch row and other
 // lengths are done here.)
 //
 // Mapping: one CTA per (channel, group of BG batch rows).  The filter row(s) and the BG

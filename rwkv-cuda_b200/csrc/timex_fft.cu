@@ -8,7 +8,7 @@
 // k1 + i k2 is x1 + i x2.  For gw the rows of g are packed as g1 - i g2: (K1 + i K2)(G1 - i G2) has the spectrum of
 // k1*g1 + k2*g2 as its real sequence, so products are summed over the batch and transformed back once.
 //
-// A transform of N = 256 R points (R = 1, 2, 4, 8) is done by N/16 threads with 16 points each: radix 16, exchange through shared
+// A transform of N = 256 R points (R = 4, 8) is done by N/16 threads with 16 points each: radix 16, exchange through shared
 // memory, radix 16, exchange inside groups of R lanes, radix R.  Spectra stay in the order this leaves them in (thread and
 // register); the inverse takes the same steps backwards, so nothing is ever reordered.  The upper half of the input is zero
 // and the upper half of the output is not needed: the outer radix-16 steps do half of their work.  Row strides in shared
@@ -29,8 +29,6 @@ template <bool INV> __device__ __forceinline__ cf tw(cf a, cf b) { return INV ? 
 // a times -i (forward) or i (inverse)
 template <bool INV> __device__ __forceinline__ cf quarter(cf a) { return INV ? cf{-a.y, a.x} : cf{a.y, -a.x}; }
 
-template <bool INV>
-__device__ __forceinline__ void fft2(cf& a, cf& b) { const cf t = a - b; a = a + b; b = t; }
 // natural order in and out
 template <bool INV>
 __device__ __forceinline__ void fft4(cf& a, cf& b, cf& c, cf& d) {
@@ -134,11 +132,7 @@ struct Engine {
     }
     template <bool INV>
     static __device__ __forceinline__ void small(cf (&v)[16]) {   // the 16 / R transforms of length R
-        if constexpr (R == 1) {
-        } else if constexpr (R == 2) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) fft2<INV>(v[2 * e], v[2 * e + 1]);
-        } else if constexpr (R == 4) {
+        if constexpr (R == 4) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) fft4<INV>(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
         } else {
@@ -164,7 +158,6 @@ struct Engine {
 #pragma unroll
         for (int m = 0; m < 16; ++m) v[m] = b1[k1 * P::S1 + j1 + R * m];
         fft16<false, false>(v);
-        if (R == 1) return;   // (each thread has its points already)
         t2.apply<false>(v);
         __syncwarp();
 #pragma unroll
@@ -178,18 +171,16 @@ struct Engine {
     }
     // spectrum -> elements j + L m in v[m] (m < 8 are what the callers use), times N
     __device__ __forceinline__ void inverse(cf (&v)[16]) {
-        if (R > 1) {
-            small<true>(v);
-            __syncwarp();
+        small<true>(v);
+        __syncwarp();
 #pragma unroll
-            for (int e = 0; e < 16 / R; ++e)
+        for (int e = 0; e < 16 / R; ++e)
 #pragma unroll
-                for (int i = 0; i < R; ++i) b2[k1 * P::S2 + (j1 + R * e) * P::P2 + i] = v[e * R + i];
-            __syncwarp();
+            for (int i = 0; i < R; ++i) b2[k1 * P::S2 + (j1 + R * e) * P::P2 + i] = v[e * R + i];
+        __syncwarp();
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = b2[k1 * P::S2 + k * P::P2 + j1];
-            t2.apply<true>(v);
-        }
+        for (int k = 0; k < 16; ++k) v[k] = b2[k1 * P::S2 + k * P::P2 + j1];
+        t2.apply<true>(v);
         fft16<true, false>(v);
 #pragma unroll
         for (int m = 0; m < 16; ++m) b1[k1 * P::S1 + j1 + R * m] = v[m];
@@ -343,21 +334,17 @@ int backward(const float* w, const float* k, const float* g, float* gw, float* g
 
 }  // namespace
 
-// Below 65 tokens the direct form has less to do than a transform of 128 points; above 1024 the engine has no transform
-// long enough.  (B1 C768 T129 forward + backward: 15 + 21 us either way, launches; B8: 65 us direct, 34 us here.)
-bool timex_fft_applies(int T) { return T > 64 && T <= 1024; }
+// Up to 256 tokens the direct form is the more precise one: its error against fp64 is 1.48e-8 sqrt(T) of the norm, the
+// transforms' is 1.9e-7 (256 points) to 2.4e-7 (2048) and falls below it between 256 and 257 tokens, where the transforms
+// get longer (T = 256: 2.35e-7 direct, 2.43e-7 with 512 points; T = 257: 2.36e-7 direct, 2.14e-7 with 1024).  Above 1024 the
+// engine has no transform long enough.
+bool timex_fft_applies(int T) { return T > 256 && T <= 1024; }
 
 int timex_fft_forward(const float* w, const float* k, float* x, float eps, int B, int C, int T, cudaStream_t st) {
-    if (T <= 128) return forward<1>(w, k, x, eps, B, C, T, st);
-    if (T <= 256) return forward<2>(w, k, x, eps, B, C, T, st);
-    if (T <= 512) return forward<4>(w, k, x, eps, B, C, T, st);
-    return forward<8>(w, k, x, eps, B, C, T, st);
+    return T <= 512 ? forward<4>(w, k, x, eps, B, C, T, st) : forward<8>(w, k, x, eps, B, C, T, st);
 }
 int timex_fft_backward(const float* w, const float* k, const float* g, float* gw, float* gk, float* work, int B, int C, int T, cudaStream_t st) {
-    if (T <= 128) return backward<1>(w, k, g, gw, gk, work, kTimexSplits, B, C, T, st);
-    if (T <= 256) return backward<2>(w, k, g, gw, gk, work, kTimexSplits, B, C, T, st);
-    if (T <= 512) return backward<4>(w, k, g, gw, gk, work, kTimexSplits, B, C, T, st);
-    return backward<8>(w, k, g, gw, gk, work, kTimexSplits, B, C, T, st);
+    return T <= 512 ? backward<4>(w, k, g, gw, gk, work, kTimexSplits, B, C, T, st) : backward<8>(w, k, g, gw, gk, work, kTimexSplits, B, C, T, st);
 }
 
 }  // namespace rwkvb200
