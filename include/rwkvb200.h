@@ -81,6 +81,8 @@ int rwkvb200_wkv4_train_backward(int B, int T, int C, const float* w_raw, const 
  *   Any B and T (the reference requires T%4==0, T<=Tmax, B%BF==0).
  * rwkvb200_timex_backward_reduced writes gw already summed over the batch, shape (C,T); the sum is taken in a
  * fixed order (the per-row gradients pass through the gk buffer before gk is written).
+ * For 256 < T <= 1024 (forward, and the backward summed over the batch) rounding is relative to the norms of a batch row and
+ * of its filter, about 2.5e-7 of their product, at every token; other lengths round relative to the terms of each sum.
  */
 int rwkvb200_timex_forward(const float* w, const float* k, float* x, float eps, int B, int C,
                            int T, void* stream);
