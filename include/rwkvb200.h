@@ -256,7 +256,7 @@ int rwkvb200_wkv6_train_forward(int dtype, int B, int T, int C, int H, const voi
 int rwkvb200_wkv6_train_backward(int dtype, int B, int T, int C, int H, int path, const void* r, const void* k,
                                  const void* v, const void* w, const void* u, const float* s0, const void* gy,
                                  const float* dsT, void* gr, void* gk, void* gv, void* gw, void* gu, float* ds0,
-                                 void* saved, void* work, void* stream);
+                                 const void* saved, void* work, void* stream);
 
 /* Kernels of the bf16 / head-size-64 forward and backward of RWKV-5 and RWKV-6: 1 (default) = tcgen05 (32-token
  * chunks; the forward as three warp groups with inputs by TMA), 0 = mma.sync (16-token chunks).  Results agree to rounding.

@@ -333,10 +333,10 @@ int tensor_forward(int dtype, int B, int T, int C, int H, const void* r, const v
 
 // The backward that goes with it; scratch: (B,T,C) floats for the flagged units (may be `saved`).
 int tensor_backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, const float* s0,
-                    const void* gy, const float* dsT, void* gr, void* gk, void* gv, void* gw, void* gu, float* ds0, float* gu32, void* saved,
+                    const void* gy, const float* dsT, void* gr, void* gk, void* gv, void* gw, void* gu, float* ds0, float* gu32, const void* saved,
                     float* scratch, cudaStream_t st, const char* what) {
     const int N = C / H, sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
-    const int* flags = wkv6_saved_flags(saved, B, T, H);
+    const int* flags = wkv6_saved_flags(const_cast<void*>(saved), B, T, H);
     if (int e = wkv6_l32_backward(B, T, H, r, k, v, w, 1, u, gy, dsT, static_cast<const float*>(saved), gr, gk, gv, gw, gu, ds0, dk, st, nullptr,
                                   gu32, 0, flags))
         return e;
@@ -564,8 +564,8 @@ extern "C" int rwkvb200_wkv6state_backward_saved(int dtype, int B, int T, int C,
 }
 
 // ---- training flow: gu summed over the batch inside the library, buffers of the size that the path needs -----------------
-// (the flagged units of the tcgen05 backward use the states in `saved` as scratch, as in rwkvb200_wkv6state_backward_saved:
-// they hold 2 floats per element and the scratch takes one)
+// (the flagged units of the tcgen05 backward have a scratch in `work`: `saved` is read only, because a graph that is kept may
+// be walked again)
 // Path 0: the tcgen05 kernels; 2: fp32 arithmetic split over time (wkv6_seg.cu); 1: everything else.
 extern "C" size_t rwkvb200_wkv6_train_saved_bytes(int dtype, int B, int T, int C, int H) {
     if (B <= 0 || T <= 0 || C <= 0 || H <= 0 || dtype != RWKVB200_BF16 || C / H != 64) return 16;
@@ -593,12 +593,12 @@ extern "C" int rwkvb200_wkv6_train_forward(int dtype, int B, int T, int C, int H
 extern "C" size_t rwkvb200_wkv6_train_work_bytes(int B, int T, int C, int path) {
     if (B <= 0 || T <= 0 || C <= 0) return 0;
     if (path == 2) return (wkv6_seg_adjoints(B, T, C) + wkv6_seg_rows(B, T) * C) * sizeof(float);
-    return (size_t)B * C * sizeof(float) + (path == 0 ? 0 : rwkvb200_wkv6_scratch_bytes(B, T, C));
+    return (size_t)B * C * sizeof(float) + (path == 0 ? (size_t)B * T * C * sizeof(float) : rwkvb200_wkv6_scratch_bytes(B, T, C));
 }
 
 extern "C" int rwkvb200_wkv6_train_backward(int dtype, int B, int T, int C, int H, int path, const void* r, const void* k, const void* v,
                                             const void* w, const void* u, const float* s0, const void* gy, const float* dsT, void* gr,
-                                            void* gk, void* gv, void* gw, void* gu, float* ds0, void* saved, void* work, void* stream) {
+                                            void* gk, void* gv, void* gw, void* gu, float* ds0, const void* saved, void* work, void* stream) {
     if (int e = check_dims("wkv6_train_backward", dtype, B, T, C, H)) return e;
     RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w); RWKV_NOTNULL(u); RWKV_NOTNULL(gy);
     RWKV_NOTNULL(gr); RWKV_NOTNULL(gk); RWKV_NOTNULL(gv); RWKV_NOTNULL(gw); RWKV_NOTNULL(gu); RWKV_NOTNULL(saved); RWKV_NOTNULL(work);
@@ -610,14 +610,14 @@ extern "C" int rwkvb200_wkv6_train_backward(int dtype, int B, int T, int C, int 
         return e ? e : sum_rows(dtype, wkv6_seg_rows(B, T), C, partial, gu, st);
     }
     const int sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
-    float* scratch = static_cast<float*>(work);   // (path 1; the partials of gu come behind it)
-    float* gu32 = path == 0 ? scratch : scratch + rwkvb200_wkv6_scratch_bytes(B, T, C) / sizeof(float);
+    float* scratch = static_cast<float*>(work);   // (the partials of gu come behind it)
+    float* gu32 = scratch + (path == 0 ? (size_t)B * T * C : rwkvb200_wkv6_scratch_bytes(B, T, C) / sizeof(float));
     int e;
     if (path == 0) {
         RWKV_REQUIRE(dtype == RWKVB200_BF16 && C / H == 64, RWKVB200_EINVAL, "wkv6_train_backward: path 0 is bf16, head size 64");
         for (const void* p : std::initializer_list<const void*>{r, k, v, w, gy, dsT, gr, gk, gv, gw, ds0, saved})
             RWKV_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15) == 0, RWKVB200_EALIGN, "wkv6_train_backward: the bf16 N=64 path needs 16-byte aligned tensors");
-        e = tensor_backward(B, T, C, H, r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, nullptr, ds0, gu32, saved, static_cast<float*>(saved), st, "wkv6_train_backward");
+        e = tensor_backward(B, T, C, H, r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, nullptr, ds0, gu32, saved, scratch, st, "wkv6_train_backward");
     } else {
         e = dtype == RWKVB200_F32
                 ? launch_bwd<float>(B, T, C, H, r, k, v, w, 1, u, s0, sk, gy, dsT, gr, gk, gv, gw, nullptr, ds0, dk, scratch, st, "wkv6_train_backward", true, gu32)
