@@ -279,8 +279,8 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(i
                 const float xu = e[i] * eu, iden = 1.f / (s.q + xu);
                 bp[i] = s.p; bq[i] = s.q;
                 y[i] = fmaf(xu, v[i], s.p) * iden;
-                h[i] = g[i] * iden;                    // (g is zero where there is no token)
-                gu = fmaf(h[i] * xu, v[i] - y[i], gu);
+                h[i] = g[i] * iden;
+                if (i < n) gu = fmaf(h[i] * xu, v[i] - y[i], gu);   // (beyond the end k is 0, which may be far outside of the range)
                 s.p = fmaf(s.p, ew, e[i] * v[i]);
                 s.q = fmaf(s.q, ew, e[i]);
             }

@@ -545,3 +545,21 @@ def test_wkv4_exponents_on_both_sides_of_the_plain_form(R, spread, mix):
     for got, want, name in ((y, yo.detach(), "y"), (gw, xs[0].grad, "gw"), (gu, xs[1].grad, "gu"),
                             (gk, xs[2].grad, "gk"), (gv, xs[3].grad, "gv")):
         Hh.assert_close(got, want, 2e-5, f"wkv4 {name}")
+
+
+@pytest.mark.parametrize("shift", [-300.0, -100.0, 100.0])
+@pytest.mark.parametrize("T", [3, 8, 203])
+def test_wkv4_does_not_see_a_shift_of_all_exponents(R, T, shift):
+    """y and every gradient are the same for k and k + shift.  (k in steps of 1/64, which a shift keeps; sums of exponents of size 300
+    are rounded to 2^-16, T of them at most: 2e-5 each way and 1e-4 for the sum.)"""
+    g = Hh.gen(T)
+    B, C = 2, 40
+    w_raw, u = Hh.rand(g, C, lo=-4, hi=1), Hh.rand(g, C, lo=-2, hi=2)
+    k, v, gy = torch.round(64 * Hh.randn(g, B, T, C)) / 64, Hh.randn(g, B, T, C), Hh.randn(g, B, T, C)
+    xs = [x.double().requires_grad_(True) for x in (w_raw, u, k, v)]
+    yo = O.wkv4(*xs)
+    yo.backward(gy.double())
+    y, gw, gu, gk, gv = run_wkv4(R, w_raw, u, k + shift, v, gy)
+    for got, want, name in ((y, yo.detach(), "y"), (gw, xs[0].grad, "gw"), (gu, xs[1].grad, "gu"),
+                            (gk, xs[2].grad, "gk"), (gv, xs[3].grad, "gv")):
+        Hh.assert_close(got, want, 1e-4, f"wkv4 {name}")
