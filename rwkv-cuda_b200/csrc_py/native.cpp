@@ -96,30 +96,37 @@ struct Outputs {
 
 // ---- autograd -------------------------------------------------------------------------------------------------
 // One node type for all operators (a node of its own instead of torch::autograd::Function, whose context, argument unpacking
-// and dictionary cost as much as the launches): the inputs as saved variables, plain tensors that the forward made, a few
-// integers, and the operator's backward, which returns the gradients in the order of `inputs`.
+// and dictionary cost as much as the launches): the inputs and the buffer that the forward made as saved variables (so that
+// saved-tensor hooks, and with them checkpointing, see all that is kept), a few integers, and the operator's backward, which
+// returns the gradients in the order of `inputs`.
 struct Saved {
     std::array<Tensor, 8> in;       // contiguous inputs
-    std::array<Tensor, 2> own;      // buffers of the forward
+    Tensor own;                     // buffer of the forward
     std::array<int64_t, 6> dims{};
 };
+// A saved tensor as it comes back, possibly out of a hook's hands.
+Tensor unpacked(SavedVariable& x, at::ScalarType d, int64_t elements) {
+    const Tensor t = x.unpack();
+    TORCH_CHECK(t.defined() && t.is_cuda() && t.scalar_type() == d && t.numel() == elements,
+                "saved tensor: expected ", elements, " elements of ", d, " on a CUDA device");
+    return t.contiguous();
+}
 using BackwardFn = variable_list (*)(const Saved&, const variable_list& grads);
 
 struct OpNode : torch::autograd::Node {
     BackwardFn fn = nullptr;
     const char* op = "";
     int n = 0;
-    std::array<SavedVariable, 8> in;
-    std::array<Tensor, 8> copy;      // where a contiguous copy of the input had to be made
-    Saved own;
+    std::array<SavedVariable, 9> kept;   // the inputs, and behind them the forward's buffer
+    std::array<at::ScalarType, 9> types;
+    std::array<int64_t, 9> elements;
+    std::array<int64_t, 6> dims{};
     bool released = false;
 
     std::string name() const override { return op; }
     void release_variables() override {
         std::lock_guard<std::mutex> lock(mutex_);
-        for (auto& x : in) x.reset_data();
-        for (auto& x : copy) x.reset();
-        for (auto& x : own.own) x.reset();
+        for (auto& x : kept) x.reset_data();
         released = true;
     }
     variable_list apply(variable_list&& grads) override {
@@ -127,9 +134,9 @@ struct OpNode : torch::autograd::Node {
         {
             std::lock_guard<std::mutex> lock(mutex_);
             TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
-            for (int i = 0; i < n; ++i) s.in[i] = copy[i].defined() ? copy[i] : in[i].unpack();
-            s.own = own.own;
-            s.dims = own.dims;
+            for (int i = 0; i <= n; ++i)
+                if (elements[i] != 0) (i < n ? s.in[i] : s.own) = unpacked(kept[i], types[i], elements[i]);
+            s.dims = dims;
         }
         at::AutoDispatchBelowAutograd no_graph;
         for (size_t i = 0; i < grads.size(); ++i)
@@ -151,12 +158,14 @@ void record(const char* op, BackwardFn fn, at::ArrayRef<Tensor> inputs, Saved&& 
     node->fn = fn;
     node->op = op;
     node->n = inputs.size();
-    for (int i = 0; i < node->n; ++i) {
-        if (s.in[i].is_same(inputs[i])) node->in[i] = SavedVariable(inputs[i], false);
-        else node->copy[i] = s.in[i];
+    for (int i = 0; i <= node->n; ++i) {   // (s.in[i]: the input, or the contiguous copy that had to be made of it)
+        const Tensor& x = i < node->n ? s.in[i] : s.own;
+        node->elements[i] = x.defined() ? x.numel() : 0;
+        if (!x.defined()) continue;
+        node->types[i] = x.scalar_type();
+        node->kept[i] = SavedVariable(x, false);
     }
-    node->own.own = std::move(s.own);
-    node->own.dims = s.dims;
+    node->dims = s.dims;
     for (const Tensor& y : outputs) torch::autograd::set_history(y, node);
 }
 Tensor dense(const Tensor& x) {   // contiguous form, outside of the graph
@@ -192,7 +201,7 @@ static variable_list wkv4_backward(const Saved& s, const variable_list& g) {
     Tensor gk = o.next({B, T, C}, gy), gv = o.next({B, T, C}, gy), gwu = o.next({2, C}, gy);
     const Tensor partial = B > 1 ? o.next({B, 2, C}, gy) : Tensor();
     check_rc(rwkvb200_wkv4_train_backward(B, T, C, f32(s.in[0].data_ptr()), f32(s.in[1].data_ptr()), f32(s.in[2].data_ptr()),
-                                          f32(s.in[3].data_ptr()), f32(ptr(gy, "gy", f)), s.own[0].data_ptr(), f32(gwu.data_ptr()),
+                                          f32(s.in[3].data_ptr()), f32(ptr(gy, "gy", f)), s.own.data_ptr(), f32(gwu.data_ptr()),
                                           partial.defined() ? f32(partial.data_ptr()) : nullptr, f32(gk.data_ptr()), f32(gv.data_ptr()), stream()),
              "rwkvb200_wkv4_train_backward", true);
     return {part(gwu, 0, s.in[0]), part(gwu, C, s.in[1]), std::move(gk), std::move(gv)};
@@ -204,9 +213,9 @@ static Tensor wkv4(int64_t B, int64_t T, int64_t C, const Tensor& w, const Tenso
     Saved s{{dense(w), dense(u), dense(k), dense(v)}, {}, {B, T, C}};
     numel(w, C, "w"); numel(u, C, "u"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v");
     Tensor y = empty({B, T, C}, f, k);
-    s.own[0] = bytes(rwkvb200_wkv4_saved_bytes(B, T, C), k);
+    s.own = bytes(rwkvb200_wkv4_saved_bytes(B, T, C), k);
     check_rc(rwkvb200_wkv4_train_forward(B, T, C, f32(ptr(s.in[0], "w", f)), f32(ptr(s.in[1], "u", f)), f32(ptr(s.in[2], "k", f)),
-                                         f32(ptr(s.in[3], "v", f)), f32(y.data_ptr()), s.own[0].data_ptr(), stream()),
+                                         f32(ptr(s.in[3], "v", f)), f32(y.data_ptr()), s.own.data_ptr(), stream()),
              "rwkvb200_wkv4_train_forward");
     record("WKV", wkv4_backward, {w, u, k, v}, std::move(s), {y});
     return y;
@@ -253,7 +262,7 @@ static variable_list wkv5_backward(const Saved& s, const variable_list& g) {
     const Tensor work = bytes(rwkvb200_wkv5_train_work_bytes(B, T, C, H, path), gy);
     check_rc(rwkvb200_wkv5_train_backward(dt(s.in[0], "r"), B, T, C, H, path, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
                                           s.in[3].data_ptr(), s.in[4].data_ptr(), ptr(gy, "gy", d), gr.data_ptr(), gk.data_ptr(), gv.data_ptr(),
-                                          gwu.data_ptr(), s.own[0].data_ptr(), work.data_ptr(), stream()),
+                                          gwu.data_ptr(), s.own.data_ptr(), work.data_ptr(), stream()),
              "rwkvb200_wkv5_train_backward", true);
     return {std::move(gr), std::move(gk), std::move(gv), part(gwu, 0, s.in[3]), part(gwu, C, s.in[4])};
 }
@@ -266,9 +275,9 @@ static Tensor wkv5(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, 
     Saved s{{dense(r), dense(k), dense(v), dense(w), dense(u)}, {}, {B, T, C, H}};
     numel(r, B * T * C, "r"); numel(k, B * T * C, "k"); numel(v, B * T * C, "v"); numel(w, C, "w"); numel(u, C, "u");
     Tensor y = empty({B, T, C}, d, r);
-    s.own[0] = bytes(rwkvb200_wkv5_train_saved_bytes(B, T, C, H), r);
+    s.own = bytes(rwkvb200_wkv5_train_saved_bytes(B, T, C, H), r);
     const int path = rwkvb200_wkv5_train_forward(dtype, B, T, C, H, ptr(s.in[0], "r", d), ptr(s.in[1], "k", d), ptr(s.in[2], "v", d),
-                                                 ptr(s.in[3], "w", d), ptr(s.in[4], "u", d), y.data_ptr(), s.own[0].data_ptr(), stream());
+                                                 ptr(s.in[3], "w", d), ptr(s.in[4], "u", d), y.data_ptr(), s.own.data_ptr(), stream());
     check_rc(path, "rwkvb200_wkv5_train_forward");
     s.dims[4] = path;
     record("WKV_5", wkv5_backward, {r, k, v, w, u}, std::move(s), {y});
@@ -289,7 +298,7 @@ static variable_list wkv6_backward(const Saved& s, const variable_list& g) {
     check_rc(rwkvb200_wkv6_train_backward(dt(s.in[0], "r"), B, T, C, H, path, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
                                           s.in[3].data_ptr(), s.in[4].data_ptr(), state ? f32(s.in[5].data_ptr()) : nullptr, ptr(gy, "gy", d),
                                           state ? f32(ptr(g[1], "dsT", f)) : nullptr, gr.data_ptr(), gk.data_ptr(), gv.data_ptr(), gw.data_ptr(),
-                                          gu.data_ptr(), state ? f32(ds0.data_ptr()) : nullptr, s.own[0].data_ptr(), work.data_ptr(), stream()),
+                                          gu.data_ptr(), state ? f32(ds0.data_ptr()) : nullptr, s.own.data_ptr(), work.data_ptr(), stream()),
              "rwkvb200_wkv6_train_backward", true);
     variable_list out{std::move(gr), std::move(gk), std::move(gv), std::move(gw), std::move(gu)};
     if (state) out.push_back(std::move(ds0));
@@ -309,10 +318,10 @@ static std::tuple<Tensor, Tensor> wkv6_forward(int64_t B, int64_t T, int64_t C, 
         s.in[5] = dense(*s0);
         sT = same(*s0);
     }
-    s.own[0] = bytes(rwkvb200_wkv6_train_saved_bytes(dtype, B, T, C, H), r);
+    s.own = bytes(rwkvb200_wkv6_train_saved_bytes(dtype, B, T, C, H), r);
     const int path = rwkvb200_wkv6_train_forward(dtype, B, T, C, H, ptr(s.in[0], "r", d), ptr(s.in[1], "k", d), ptr(s.in[2], "v", d),
                                                  ptr(s.in[3], "w", d), ptr(s.in[4], "u", d), s0 ? f32(ptr(s.in[5], "s0", f)) : nullptr,
-                                                 y.data_ptr(), s0 ? f32(sT.data_ptr()) : nullptr, s.own[0].data_ptr(), stream());
+                                                 y.data_ptr(), s0 ? f32(sT.data_ptr()) : nullptr, s.own.data_ptr(), stream());
     check_rc(path, "rwkvb200_wkv6_train_forward");
     s.dims[4] = path;
     if (s0) record("WKV_6STATE_EX", wkv6_backward, {r, k, v, w, u, *s0}, std::move(s), {y, sT});
@@ -337,7 +346,7 @@ static variable_list wkv7_backward(const Saved& s, const variable_list& g) {
     const Tensor work = nwork ? bytes(nwork, g[0]) : Tensor();
     check_rc(rwkvb200_wkv7_train_backward(dt(s.in[0], "r"), B, T, H, N, path, s.in[0].data_ptr(), s.in[1].data_ptr(), s.in[2].data_ptr(),
                                           s.in[3].data_ptr(), s.in[4].data_ptr(), s.in[5].data_ptr(), ptr(g[0], "dy", d),
-                                          sT ? f32(ptr(g[1], "dsT", f)) : nullptr, s.own[0].data_ptr(), nwork ? work.data_ptr() : nullptr,
+                                          sT ? f32(ptr(g[1], "dsT", f)) : nullptr, s.own.data_ptr(), nwork ? work.data_ptr() : nullptr,
                                           s0 ? f32(ds0.data_ptr()) : nullptr, x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), x[3].data_ptr(),
                                           x[4].data_ptr(), x[5].data_ptr(), stream()),
              "rwkvb200_wkv7_train_backward", true);
@@ -358,12 +367,12 @@ static std::tuple<Tensor, Tensor> wkv7_forward(const Tensor* s0, const Tensor& r
     const int64_t B = r.size(0), T = r.size(1), H = r.size(2), N = r.size(3);
     const int path = rwkvb200_wkv7_train_path(dtype, B, T, H, N);
     Tensor y = passing ? empty({B, T, H * N}, d, r) : same(v), sT = passing ? same(*s0) : Tensor();
-    Saved s{{r, w, k, v, a, b}, {bytes(rwkvb200_wkv7_train_saved_bytes(B, T, H, N, path), r)}, {B, T, H, N, (s0 ? 1 : 0) + (passing ? 2 : 0), path}};
+    Saved s{{r, w, k, v, a, b}, bytes(rwkvb200_wkv7_train_saved_bytes(B, T, H, N, path), r), {B, T, H, N, (s0 ? 1 : 0) + (passing ? 2 : 0), path}};
     const size_t nwork = rwkvb200_wkv7_train_work_bytes(B, T, H, path, 0);
     const Tensor work = nwork ? bytes(nwork, r) : Tensor();
     check_rc(rwkvb200_wkv7_train_forward(dtype, B, T, H, N, path, s0 ? f32(ptr(*s0, "s0", f)) : nullptr, ptr(r, "r", d), ptr(w, "w", d),
                                          ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
-                                         passing ? f32(sT.data_ptr()) : nullptr, s.own[0].data_ptr(), nwork ? work.data_ptr() : nullptr, stream()),
+                                         passing ? f32(sT.data_ptr()) : nullptr, s.own.data_ptr(), nwork ? work.data_ptr() : nullptr, stream()),
              "rwkvb200_wkv7_train_forward");
     if (s0) s.in[6] = *s0;
     const char* op = passing ? "RWKV7_STATE_PASSING_CLAMPW_CUDA_OP" : s0 ? "RWKV7_STATE_CLAMPW_CUDA_OP" : "RWKV7_CLAMPW_CUDA_OP";
