@@ -374,7 +374,7 @@ static std::tuple<Tensor, Tensor> wkv7_forward(const Tensor* s0, const Tensor& r
                                          ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
                                          passing ? f32(sT.data_ptr()) : nullptr, s.own.data_ptr(), nwork ? work.data_ptr() : nullptr, stream()),
              "rwkvb200_wkv7_train_forward");
-    if (s0) s.in[6] = *s0;
+    // (the backward does not read s0: it is not kept, so that a program may carry its state in place)
     const char* op = passing ? "RWKV7_STATE_PASSING_CLAMPW_CUDA_OP" : s0 ? "RWKV7_STATE_CLAMPW_CUDA_OP" : "RWKV7_CLAMPW_CUDA_OP";
     if (passing) record(op, wkv7_backward, {r, w, k, v, a, b, *s0}, std::move(s), {y, sT});
     else if (s0) record(op, wkv7_backward, {r, w, k, v, a, b, *s0}, std::move(s), {y});

@@ -111,3 +111,15 @@ def test_checkpointing(name):
     got = gradients(lambda *x: torch.utils.checkpoint.checkpoint(call, *x, use_reentrant=False), xs)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", ["wkv7 state", "wkv7 state passing"])
+def test_rwkv7_state_carried_in_place(name):
+    """The initial state may be overwritten between forward and backward, as a program does that carries it in one buffer."""
+    xs, call = cases()[name]
+    xs = [x.cuda().requires_grad_(i > 0) for i, x in enumerate(xs)]
+    want = gradients(lambda *x: call(xs[0], *x), xs[1:])
+    ys = outputs(call(*xs))
+    xs[0].copy_(ys[1].detach() if len(ys) > 1 else torch.zeros_like(xs[0]))
+    for a, b in zip(torch.autograd.grad(ys, xs[1:], cotangents(ys)), want):
+        assert torch.equal(a, b)
