@@ -10,6 +10,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include "../../include/rwkvb200.h"
@@ -145,8 +146,28 @@ struct OpNode : torch::autograd::Node {
     }
 };
 
-// Ties `outputs` to a node that keeps `inputs` (as given) and what `s` holds; s.in are their contiguous forms.
-void record(const char* op, BackwardFn fn, at::ArrayRef<Tensor> inputs, Saved&& s, at::ArrayRef<Tensor> outputs) {
+// What a forward has made: the outputs, what is kept for the backward (s.in: contiguous forms of the inputs) and the backward.
+struct Made {
+    const char* op;
+    BackwardFn backward;
+    c10::SmallVector<Tensor, 2> outputs;
+    c10::SmallVector<Tensor, 8> inputs;   // the differentiable ones, as given
+    Saved s;
+};
+
+// Calls that are not for the node below: forward-mode derivatives, functorch's wrappers (grad, vmap, ...), tensors of classes
+// with a dispatch of their own (and jit tracing).  torch.autograd.Function knows what to do with them.
+bool ordinary(const Tensor& x) {
+    constexpr c10::DispatchKeySet special({c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::Python});
+    return !x.key_set().has_any(special) && !x._fw_grad(0).defined();
+}
+template <typename T>
+bool ordinary(const T&) { return true; }   // (a number)
+
+// Ties the outputs to a node that keeps what the forward has made.
+void record(Made& m) {
+    const auto& inputs = m.inputs;
+    const Saved& s = m.s;
     bool any = false;
     for (const Tensor& x : inputs) any |= x.requires_grad();
     if (!any || !at::GradMode::is_enabled()) return;
@@ -155,8 +176,8 @@ void record(const char* op, BackwardFn fn, at::ArrayRef<Tensor> inputs, Saved&& 
     edges.reserve(inputs.size());
     for (const Tensor& x : inputs) edges.push_back(torch::autograd::impl::gradient_edge(x));
     node->set_next_edges(std::move(edges));
-    node->fn = fn;
-    node->op = op;
+    node->fn = m.backward;
+    node->op = m.op;
     node->n = inputs.size();
     for (int i = 0; i <= node->n; ++i) {   // (s.in[i]: the input, or the contiguous copy that had to be made of it)
         const Tensor& x = i < node->n ? s.in[i] : s.own;
@@ -166,7 +187,7 @@ void record(const char* op, BackwardFn fn, at::ArrayRef<Tensor> inputs, Saved&& 
         node->kept[i] = SavedVariable(x, false);
     }
     node->dims = s.dims;
-    for (const Tensor& y : outputs) torch::autograd::set_history(y, node);
+    for (const Tensor& y : m.outputs) torch::autograd::set_history(y, node);
 }
 Tensor dense(const Tensor& x) {   // contiguous form, outside of the graph
     if (x.is_contiguous()) return x;
@@ -206,7 +227,7 @@ static variable_list wkv4_backward(const Saved& s, const variable_list& g) {
              "rwkvb200_wkv4_train_backward", true);
     return {part(gwu, 0, s.in[0]), part(gwu, C, s.in[1]), std::move(gk), std::move(gv)};
 }
-static Tensor wkv4(int64_t B, int64_t T, int64_t C, const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
+static Made wkv4(int64_t B, int64_t T, int64_t C, const Tensor& w, const Tensor& u, const Tensor& k, const Tensor& v) {
     on_device(k, "k");
     const c10::cuda::CUDAGuard guard(k.device());
     const auto f = at::kFloat;
@@ -217,8 +238,7 @@ static Tensor wkv4(int64_t B, int64_t T, int64_t C, const Tensor& w, const Tenso
     check_rc(rwkvb200_wkv4_train_forward(B, T, C, f32(ptr(s.in[0], "w", f)), f32(ptr(s.in[1], "u", f)), f32(ptr(s.in[2], "k", f)),
                                          f32(ptr(s.in[3], "v", f)), f32(y.data_ptr()), s.own.data_ptr(), stream()),
              "rwkvb200_wkv4_train_forward");
-    record("WKV", wkv4_backward, {w, u, k, v}, std::move(s), {y});
-    return y;
+    return {"WKVBackward", wkv4_backward, {y}, {w, u, k, v}, std::move(s)};
 }
 
 // ---- depthwise_conv1d -----------------------------------------------------------------------------------------
@@ -237,7 +257,7 @@ static variable_list timex_backward(const Saved& s, const variable_list& g) {
              "rwkvb200_timex_train_backward", true);
     return {std::move(gw), std::move(gk)};
 }
-static Tensor timex(const Tensor& w, const Tensor& k, int64_t B, int64_t C, int64_t T, double eps) {
+static Made timex(const Tensor& w, const Tensor& k, int64_t B, int64_t C, int64_t T, double eps) {
     on_device(k, "k");
     const c10::cuda::CUDAGuard guard(k.device());
     const auto f = at::kFloat;
@@ -246,8 +266,7 @@ static Tensor timex(const Tensor& w, const Tensor& k, int64_t B, int64_t C, int6
     Tensor x = empty({B, C, T}, f, k);
     check_rc(rwkvb200_timex_forward(f32(ptr(s.in[0], "w", f)), f32(ptr(s.in[1], "k", f)), f32(x.data_ptr()), (float)eps, B, C, T, stream()),
              "rwkvb200_timex_forward");
-    record("TimeX", timex_backward, {w, k}, std::move(s), {x});
-    return x;
+    return {"TimeXBackward", timex_backward, {x}, {w, k}, std::move(s)};
 }
 
 // ---- RWKV-5 ---------------------------------------------------------------------------------------------------
@@ -266,7 +285,7 @@ static variable_list wkv5_backward(const Saved& s, const variable_list& g) {
              "rwkvb200_wkv5_train_backward", true);
     return {std::move(gr), std::move(gk), std::move(gv), part(gwu, 0, s.in[3]), part(gwu, C, s.in[4])};
 }
-static Tensor wkv5(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
+static Made wkv5(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
     for (const Tensor* x : {&k, &v, &w, &u}) assert_py(x->scalar_type() == r.scalar_type(), "r, k, v, w, u must have one dtype");
     on_device(r, "r");
     const c10::cuda::CUDAGuard guard(r.device());
@@ -280,8 +299,7 @@ static Tensor wkv5(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, 
                                                  ptr(s.in[3], "w", d), ptr(s.in[4], "u", d), y.data_ptr(), s.own.data_ptr(), stream());
     check_rc(path, "rwkvb200_wkv5_train_forward");
     s.dims[4] = path;
-    record("WKV_5", wkv5_backward, {r, k, v, w, u}, std::move(s), {y});
-    return y;
+    return {"WKV_5Backward", wkv5_backward, {y}, {r, k, v, w, u}, std::move(s)};
 }
 
 // ---- RWKV-6, without a state or with an fp32 state in and out (s0, sT, dsT, ds0) ------------------------------------------
@@ -304,7 +322,7 @@ static variable_list wkv6_backward(const Saved& s, const variable_list& g) {
     if (state) out.push_back(std::move(ds0));
     return out;
 }
-static std::tuple<Tensor, Tensor> wkv6_forward(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v,
+static Made wkv6_forward(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v,
                                                const Tensor& w, const Tensor& u, const Tensor* s0) {
     on_device(r, "r");
     const c10::cuda::CUDAGuard guard(r.device());
@@ -324,9 +342,8 @@ static std::tuple<Tensor, Tensor> wkv6_forward(int64_t B, int64_t T, int64_t C, 
                                                  y.data_ptr(), s0 ? f32(sT.data_ptr()) : nullptr, s.own.data_ptr(), stream());
     check_rc(path, "rwkvb200_wkv6_train_forward");
     s.dims[4] = path;
-    if (s0) record("WKV_6STATE_EX", wkv6_backward, {r, k, v, w, u, *s0}, std::move(s), {y, sT});
-    else record("WKV_6", wkv6_backward, {r, k, v, w, u}, std::move(s), {y});
-    return {y, sT};
+    if (s0) return {"WKV_6STATE_EXBackward", wkv6_backward, {y, sT}, {r, k, v, w, u, *s0}, std::move(s)};
+    return {"WKV_6Backward", wkv6_backward, {y}, {r, k, v, w, u}, std::move(s)};
 }
 
 // ---- RWKV-7, the three operators: state in (s0) and out (sT) or not ---------------------------------------------
@@ -354,7 +371,7 @@ static variable_list wkv7_backward(const Saved& s, const variable_list& g) {
     if (s0) out.push_back(std::move(ds0));
     return out;
 }
-static std::tuple<Tensor, Tensor> wkv7_forward(const Tensor* s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v,
+static Made wkv7_forward(const Tensor* s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v,
                                                const Tensor& a, const Tensor& b, bool passing) {
     assert_py(r.dim() == 4 && r.size(1) % kChunkLen == 0, "T must be a multiple of 16");
     for (const Tensor* x : {&w, &k, &v, &a, &b}) assert_py(x->scalar_type() == r.scalar_type(), "r, w, k, v, a, b must have one dtype");
@@ -375,33 +392,69 @@ static std::tuple<Tensor, Tensor> wkv7_forward(const Tensor* s0, const Tensor& r
                                          passing ? f32(sT.data_ptr()) : nullptr, s.own.data_ptr(), nwork ? work.data_ptr() : nullptr, stream()),
              "rwkvb200_wkv7_train_forward");
     // (the backward does not read s0: it is not kept, so that a program may carry its state in place)
-    const char* op = passing ? "RWKV7_STATE_PASSING_CLAMPW_CUDA_OP" : s0 ? "RWKV7_STATE_CLAMPW_CUDA_OP" : "RWKV7_CLAMPW_CUDA_OP";
-    if (passing) record(op, wkv7_backward, {r, w, k, v, a, b, *s0}, std::move(s), {y, sT});
-    else if (s0) record(op, wkv7_backward, {r, w, k, v, a, b, *s0}, std::move(s), {y});
-    else record(op, wkv7_backward, {r, w, k, v, a, b}, std::move(s), {y});
-    return {y, sT};
+    if (passing) return {"RWKV7_STATE_PASSING_CLAMPW_CUDA_OPBackward", wkv7_backward, {y, sT}, {r, w, k, v, a, b, *s0}, std::move(s)};
+    if (s0) return {"RWKV7_STATE_CLAMPW_CUDA_OPBackward", wkv7_backward, {y}, {r, w, k, v, a, b, *s0}, std::move(s)};
+    return {"RWKV7_CLAMPW_CUDA_OPBackward", wkv7_backward, {y}, {r, w, k, v, a, b}, std::move(s)};
+}
+static Made wkv6(int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
+    return wkv6_forward(B, T, C, H, r, k, v, w, u, nullptr);
+}
+static Made wkv6_state(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u, const Tensor& s0) {
+    TORCH_CHECK_VALUE(r.dim() == 3, "r: expected (B,T,C), got ", r.sizes());
+    return wkv6_forward(r.size(0), r.size(1), r.size(2), u.size(0), r, k, v, w, u, &s0);
+}
+static Made wkv7(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
+    return wkv7_forward(nullptr, r, w, k, v, a, b, false);
+}
+static Made wkv7_state(const Tensor& s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
+    return wkv7_forward(&s0, r, w, k, v, a, b, false);
+}
+static Made wkv7_statepassing(const Tensor& s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
+    return wkv7_forward(&s0, r, w, k, v, a, b, true);
+}
+
+// ---- bindings -----------------------------------------------------------------------------------------------
+// name: the outputs with their graph, or None for a call that is not for the native node.
+// name_forward: the outputs, the tensors and integers that name_backward wants, and nothing recorded.
+template <typename... A>
+static void define(py::module_& m, const char* op_name, Made (*op)(A...), BackwardFn backward) {
+    const std::string name = op_name;
+    m.def(op_name, [op](A... args) -> py::object {
+        bool plain = !torch::jit::tracer::isTracing();
+        ((plain = plain && ordinary(args)), ...);
+        if (!plain) return py::none();
+        Made r = op(args...);
+        record(r);
+        return r.outputs.size() == 1 ? py::cast(r.outputs[0]) : py::object(py::make_tuple(r.outputs[0], r.outputs[1]));
+    });
+    m.def((name + "_forward").c_str(), [op](A... args) {
+        const Made r = op(args...);
+        std::vector<Tensor> kept;
+        for (size_t i = 0; i < r.s.in.size(); ++i)
+            if (r.s.in[i].defined()) kept.push_back(r.s.in[i]);
+        const size_t n = kept.size();
+        if (r.s.own.defined()) kept.push_back(r.s.own);
+        py::object y = r.outputs.size() == 1 ? py::cast(r.outputs[0]) : py::object(py::make_tuple(r.outputs[0], r.outputs[1]));
+        return py::make_tuple(y, py::tuple(py::cast(kept)), n, r.s.dims);
+    });
+    m.def((name + "_backward").c_str(), [backward](const std::vector<Tensor>& kept, size_t n, const std::array<int64_t, 6>& dims, variable_list grads) {
+        Saved s;
+        s.dims = dims;
+        for (size_t i = 0; i < kept.size(); ++i) (i < n ? s.in.at(i) : s.own) = kept[i].contiguous();
+        for (Tensor& g : grads) g = g.contiguous();
+        return backward(s, grads);
+    });
 }
 
 PYBIND11_MODULE(_native, m) {
     m.def("set_error_class", [](py::object cls) { g_error_class = cls.inc_ref().ptr(); });
     m.def("wkv7_state_update", &wkv7_state_update);
-    m.def("wkv4", &wkv4);
-    m.def("timex", &timex);
-    m.def("wkv5", &wkv5);
-    m.def("wkv6", [](int64_t B, int64_t T, int64_t C, int64_t H, const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u) {
-        return std::get<0>(wkv6_forward(B, T, C, H, r, k, v, w, u, nullptr));
-    });
-    m.def("wkv6_state", [](const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u, const Tensor& s0) {
-        TORCH_CHECK_VALUE(r.dim() == 3, "r: expected (B,T,C), got ", r.sizes());
-        return wkv6_forward(r.size(0), r.size(1), r.size(2), u.size(0), r, k, v, w, u, &s0);
-    });
-    m.def("wkv7", [](const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        return std::get<0>(wkv7_forward(nullptr, r, w, k, v, a, b, false));
-    });
-    m.def("wkv7_state", [](const Tensor& s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        return std::get<0>(wkv7_forward(&s0, r, w, k, v, a, b, false));
-    });
-    m.def("wkv7_statepassing", [](const Tensor& s0, const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b) {
-        return wkv7_forward(&s0, r, w, k, v, a, b, true);
-    });
+    define(m, "wkv4", &wkv4, wkv4_backward);
+    define(m, "timex", &timex, timex_backward);
+    define(m, "wkv5", &wkv5, wkv5_backward);
+    define(m, "wkv6", &wkv6, wkv6_backward);
+    define(m, "wkv6_state", &wkv6_state, wkv6_backward);
+    define(m, "wkv7", &wkv7, wkv7_backward);
+    define(m, "wkv7_state", &wkv7_state, wkv7_backward);
+    define(m, "wkv7_statepassing", &wkv7_statepassing, wkv7_backward);
 }

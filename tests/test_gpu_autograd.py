@@ -123,3 +123,99 @@ def test_rwkv7_state_carried_in_place(name):
     xs[0].copy_(ys[1].detach() if len(ys) > 1 else torch.zeros_like(xs[0]))
     for a, b in zip(torch.autograd.grad(ys, xs[1:], cotangents(ys)), want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_calls_that_only_an_autograd_function_can_take(name):
+    """jit tracing records the operator and not its result; forward-mode derivatives and functorch's transforms are refused and not
+    ignored; a subclass may replace forward and backward; and forward and backward give what the native node gives."""
+    import torch.autograd.forward_ad as fwAD
+    xs, call = cases()[name]
+    xs = [x.cuda() for x in xs]
+    first = lambda *x: outputs(call(*x))[0]
+    traced = torch.jit.trace(first, tuple(xs), check_trace=False)
+    other = [x.flip(0).contiguous() for x in xs]
+    assert torch.equal(traced(*other), first(*other))
+    with fwAD.dual_level(), pytest.raises((NotImplementedError, RuntimeError)):
+        call(*(fwAD.make_dual(x, torch.ones_like(x)) for x in xs))
+    for transform in (lambda: torch.func.grad(lambda *x: first(*x).float().sum())(*xs), lambda: torch.func.vjp(call, *xs),
+                      lambda: torch.vmap(call)(*(torch.stack([x, x]) for x in xs))):
+        with pytest.raises(RuntimeError, match="autograd.Function"):
+            transform()
+
+
+def test_forward_and_backward_of_the_classes():
+    import rwkv_cuda_b200 as R
+    F = R.functions
+    per_class = {"wkv4": F.WKV, "timex": F.TimeX, "wkv5": F.WKV_5, "wkv6": F.WKV_6, "wkv6 state": F.WKV_6STATE_EX,
+                 "wkv7": F.RWKV7_CLAMPW_CUDA_OP, "wkv7 state": F.RWKV7_STATE_CLAMPW_CUDA_OP,
+                 "wkv7 state passing": F.RWKV7_STATE_PASSING_CLAMPW_CUDA_OP}
+    for name, cls in per_class.items():
+        xs, call = cases()[name]
+        xs = [x.cuda().requires_grad_(True) for x in xs]
+        sub = type(cls.__name__ + "Sub", (cls,), {})
+        lead = dict(wkv4=(2, 24, 32), wkv5=(2, 64, 128, 2), wkv6=(2, 64, 128, 2)).get(name, ())
+        tail = (2, 8, 300, 0.1) if name == "timex" else ()
+        a, b = call(*xs), sub.apply(*lead, *xs, *tail)
+        assert outputs(b)[0].grad_fn.name() == sub.__name__ + "Backward" and outputs(a)[0].grad_fn.name() == cls.__name__ + "Backward"
+        for p, q in zip(outputs(a), outputs(b)):
+            assert torch.equal(p, q), name
+        for p, q in zip(gradients(call, xs), gradients(lambda *x: sub.apply(*lead, *x, *tail), xs)):
+            assert p.shape == q.shape and torch.equal(p, q), name
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_walks_unused_outputs_and_inputs_without_gradient(name):
+    xs, call = cases()[name]
+    xs = [x.cuda().requires_grad_(True) for x in xs]
+    want = gradients(call, xs)
+    ys = outputs(call(*xs))
+    for a, b in zip(torch.autograd.grad(ys, xs, cotangents(ys), retain_graph=True), want):
+        assert torch.equal(a, b)
+    # an expanded gradient; an output that nothing depends on counts as one with a gradient of zero
+    for y in ys:
+        one = torch.autograd.grad(y, xs, torch.ones((), device="cuda", dtype=y.dtype).expand(y.shape), retain_graph=True)
+        zero = [torch.ones_like(z) if z is y else torch.zeros_like(z) for z in ys]
+        for a, b in zip(one, torch.autograd.grad(ys, xs, zero, retain_graph=True)):
+            assert torch.equal(a, b)
+    torch.autograd.grad(ys, xs, cotangents(ys))
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(ys, xs, cotangents(ys))
+    some = [x.detach().requires_grad_(i % 2 == 0) for i, x in enumerate(xs)]
+    got = gradients_of(call, some, some[::2])
+    for a, b in zip(got, want[::2]):
+        assert torch.equal(a, b)
+    assert not outputs(call(*(x.detach() for x in xs)))[0].requires_grad
+    with torch.no_grad():
+        assert not outputs(call(*xs))[0].requires_grad
+
+
+def gradients_of(call, xs, wanted):
+    ys = outputs(call(*xs))
+    return torch.autograd.grad(ys, wanted, cotangents(ys))
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_two_streams_and_two_threads(name):
+    """The same call on two streams of two threads at once: every one gets the gradients of a call alone."""
+    import threading
+    xs, call = cases()[name]
+    xs = [x.cuda() for x in xs]
+    want = gradients(call, [x.clone().requires_grad_(True) for x in xs])
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work():
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                got = gradients(call, [x.clone().requires_grad_(True) for x in xs])
+                torch.cuda.current_stream().synchronize()
+                if not all(torch.equal(a, b) for a, b in zip(got, want)):
+                    wrong.append(name)
+
+    threads = [threading.Thread(target=work) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
