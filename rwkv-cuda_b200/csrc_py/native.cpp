@@ -165,7 +165,7 @@ template <typename T>
 bool ordinary(const T&) { return true; }   // (a number)
 
 // Ties the outputs to a node that keeps what the forward has made.
-void record(Made& m) {
+void record(const Made& m) {
     const auto& inputs = m.inputs;
     const Saved& s = m.s;
     bool any = false;
@@ -414,6 +414,13 @@ static Made wkv7_statepassing(const Tensor& s0, const Tensor& r, const Tensor& w
 }
 
 // ---- bindings -----------------------------------------------------------------------------------------------
+// A launch may wait for room in the GPU's queue: other Python threads run meanwhile.
+template <typename F>
+static auto unlocked(F f) {
+    py::gil_scoped_release no_gil;
+    return f();
+}
+
 // name: the outputs with their graph, or None for a call that is not for the native node.
 // name_forward: the outputs, the tensors and integers that name_backward wants, and nothing recorded.
 template <typename... A>
@@ -423,12 +430,15 @@ static void define(py::module_& m, const char* op_name, Made (*op)(A...), Backwa
         bool plain = !torch::jit::tracer::isTracing();
         ((plain = plain && ordinary(args)), ...);
         if (!plain) return py::none();
-        Made r = op(args...);
-        record(r);
+        const Made r = unlocked([&] {
+            Made made = op(args...);
+            record(made);
+            return made;
+        });
         return r.outputs.size() == 1 ? py::cast(r.outputs[0]) : py::object(py::make_tuple(r.outputs[0], r.outputs[1]));
     });
     m.def((name + "_forward").c_str(), [op](A... args) {
-        const Made r = op(args...);
+        const Made r = unlocked([&] { return op(args...); });
         std::vector<Tensor> kept;
         for (size_t i = 0; i < r.s.in.size(); ++i)
             if (r.s.in[i].defined()) kept.push_back(r.s.in[i]);
@@ -441,14 +451,16 @@ static void define(py::module_& m, const char* op_name, Made (*op)(A...), Backwa
         Saved s;
         s.dims = dims;
         for (size_t i = 0; i < kept.size(); ++i) (i < n ? s.in.at(i) : s.own) = kept[i].contiguous();
-        for (Tensor& g : grads) g = g.contiguous();
-        return backward(s, grads);
+        return unlocked([&] {
+            for (Tensor& g : grads) g = g.contiguous();
+            return backward(s, grads);
+        });
     });
 }
 
 PYBIND11_MODULE(_native, m) {
     m.def("set_error_class", [](py::object cls) { g_error_class = cls.inc_ref().ptr(); });
-    m.def("wkv7_state_update", &wkv7_state_update);
+    m.def("wkv7_state_update", &wkv7_state_update, py::call_guard<py::gil_scoped_release>());
     define(m, "wkv4", &wkv4, wkv4_backward);
     define(m, "timex", &timex, timex_backward);
     define(m, "wkv5", &wkv5, wkv5_backward);

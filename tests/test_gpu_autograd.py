@@ -219,3 +219,41 @@ def test_two_streams_and_two_threads(name):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("what", ["update", "training"])
+def test_other_threads_run_while_a_launch_waits(what):
+    """A launch waits when the GPU's queue is full (behind a kernel that takes half a second here); other Python threads go on."""
+    import threading
+    import time
+    import rwkv_cuda_b200 as R
+    if what == "training":
+        xs, fn = cases()["wkv4"]
+        xs = [x.cuda() for x in xs]
+        call = lambda: fn(*xs)
+    else:
+        xs = [x.cuda() for x in cases()["wkv7 state"][0]]
+        one = [x[:, :1].contiguous() for x in xs[1:]]
+        y = torch.empty_like(one[0])
+        call = lambda: R.ops.wkv7_state_update(xs[0], *one, y)
+    call()
+    torch.cuda.synchronize()
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.001)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    t0 = time.perf_counter()
+    torch.cuda._sleep(1_000_000_000)
+    for _ in range(3000):
+        call()
+    waited = time.perf_counter() - t0
+    stop.set()
+    thread.join()
+    torch.cuda.synchronize()
+    assert waited > 0.25, "the queue never filled up"
+    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.5 * waited
