@@ -507,12 +507,14 @@ extern "C" int rwkvb200_wkv5_train_backward(int dtype, int B, int T, int C, int 
     float* partial = static_cast<float*>(work);
     i64 rows = B;
     if (path == 0) {
-        RWKV_REQUIRE(dtype == RWKVB200_BF16 && chunked_ok<bf16>(T, C / H, {r, k, v, gy, gr, gk, gv, saved}), RWKVB200_EALIGN,
-                     "wkv5_train_backward: the bf16 N=64 path needs 16-byte aligned tensors");
-        const int* flags = wkv6_saved_flags(const_cast<void*>(saved), B, T, H);
-        if (int e = wkv6_l32_backward(B, T, H, r, k, v, w_raw, 4, u, gy, nullptr, static_cast<const float*>(saved), gr, gk, gv, nullptr, nullptr,
-                                      nullptr, 0, st, partial, partial + C, 2 * (i64)C, flags))
-            return e;
+        RWKV_REQUIRE(dtype == RWKVB200_BF16 && C / H == 64 && T % 16 == 0, RWKVB200_EINVAL, "wkv5_train_backward: not a call of path 0");
+        const int* flags = nullptr;   // a tensor that is not aligned (autograd may hand over any view as gy): all units on the general-shape kernel
+        if (chunked_ok<bf16>(T, C / H, {r, k, v, gy, gr, gk, gv, saved})) {
+            flags = wkv6_saved_flags(const_cast<void*>(saved), B, T, H);
+            if (int e = wkv6_l32_backward(B, T, H, r, k, v, w_raw, 4, u, gy, nullptr, static_cast<const float*>(saved), gr, gk, gv, nullptr, nullptr,
+                                          nullptr, 0, st, partial, partial + C, 2 * (i64)C, flags))
+                return e;
+        }
         wkv5_backward_kernel<bf16, 64, false><<<B * H, 64, 0, st>>>(
             T, C, H, C / H, (const bf16*)r, (const bf16*)k, (const bf16*)v, nullptr, nullptr, (const bf16*)u, nullptr, nullptr, nullptr, (const bf16*)gy,
             (bf16*)gr, (bf16*)gk, (bf16*)gv, nullptr, nullptr, nullptr, nullptr, flags, -1, (const bf16*)w_raw, partial, partial + C, 2 * (i64)C);

@@ -336,10 +336,13 @@ int tensor_backward(int B, int T, int C, int H, const void* r, const void* k, co
                     const void* gy, const float* dsT, void* gr, void* gk, void* gv, void* gw, void* gu, float* ds0, float* gu32, const void* saved,
                     float* scratch, cudaStream_t st, const char* what) {
     const int N = C / H, sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;
-    const int* flags = wkv6_saved_flags(const_cast<void*>(saved), B, T, H);
-    if (int e = wkv6_l32_backward(B, T, H, r, k, v, w, 1, u, gy, dsT, static_cast<const float*>(saved), gr, gk, gv, gw, gu, ds0, dk, st, nullptr,
-                                  gu32, 0, flags))
-        return e;
+    const int* flags = nullptr;   // a tensor that is not aligned (autograd may hand over any view as gy): all units on the general-shape kernel
+    if (chunked_ok<bf16>(T, N, {r, k, v, w, s0, gy, dsT, gr, gk, gv, gw, gu, ds0, saved})) {
+        flags = wkv6_saved_flags(const_cast<void*>(saved), B, T, H);
+        if (int e = wkv6_l32_backward(B, T, H, r, k, v, w, 1, u, gy, dsT, static_cast<const float*>(saved), gr, gk, gv, gw, gu, ds0, dk, st,
+                                      nullptr, gu32, 0, flags))
+            return e;
+    }
     wkv6_backward_kernel<bf16, 64><<<B * H, 64, 0, st>>>(T, C, H, N, (const bf16*)r, (const bf16*)k, (const bf16*)v, w, 1, (const bf16*)u, s0,
                                                         sk, (const bf16*)gy, dsT, (bf16*)gr, (bf16*)gk, (bf16*)gv, (bf16*)gw, (bf16*)gu,
                                                         ds0, dk, scratch, flags, -1, gu32);
@@ -614,9 +617,7 @@ extern "C" int rwkvb200_wkv6_train_backward(int dtype, int B, int T, int C, int 
     float* gu32 = scratch + (path == 0 ? (size_t)B * T * C : rwkvb200_wkv6_scratch_bytes(B, T, C) / sizeof(float));
     int e;
     if (path == 0) {
-        RWKV_REQUIRE(dtype == RWKVB200_BF16 && C / H == 64, RWKVB200_EINVAL, "wkv6_train_backward: path 0 is bf16, head size 64");
-        for (const void* p : std::initializer_list<const void*>{r, k, v, w, gy, dsT, gr, gk, gv, gw, ds0, saved})
-            RWKV_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15) == 0, RWKVB200_EALIGN, "wkv6_train_backward: the bf16 N=64 path needs 16-byte aligned tensors");
+        RWKV_REQUIRE(dtype == RWKVB200_BF16 && C / H == 64 && T % 16 == 0, RWKVB200_EINVAL, "wkv6_train_backward: not a call of path 0");
         e = tensor_backward(B, T, C, H, r, k, v, w, u, s0, gy, dsT, gr, gk, gv, gw, nullptr, ds0, gu32, saved, scratch, st, "wkv6_train_backward");
     } else {
         e = dtype == RWKVB200_F32

@@ -257,3 +257,26 @@ def test_other_threads_run_while_a_launch_waits(what):
     torch.cuda.synchronize()
     assert waited > 0.25, "the queue never filled up"
     assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.5 * waited
+
+
+@pytest.mark.parametrize("name", [n for n in NAMES if not n.startswith("wkv7")])   # (RWKV-7 refuses such tensors everywhere)
+def test_gradients_that_are_not_aligned(name):
+    """A contiguous gradient that starts anywhere in a larger one, as autograd hands it over when outputs are flattened and
+    concatenated.  Every class computes it; the aligned call differs by rounding."""
+    xs, call = cases()[name]
+    xs = [x.cuda().requires_grad_(True) for x in xs]
+    ys = outputs(call(*xs))
+    flat = torch.cat([torch.zeros(1, device="cuda")] + [y.float().flatten() for y in ys])
+    want = torch.autograd.grad(ys, xs, cotangents(ys), retain_graph=True)
+    odd = []
+    for c in cotangents(ys):
+        whole = torch.empty(c.numel() + 1, dtype=c.dtype, device="cuda")
+        whole[1:] = c.flatten()
+        odd.append(whole[1:].view(c.shape))
+        assert odd[-1].is_contiguous() and odd[-1].data_ptr() % 16
+    tol = Hh.TOL_BF16 if any(x.dtype == BF for x in xs) else Hh.TOL_FP32
+    for a, b in zip(torch.autograd.grad(ys, xs, odd, retain_graph=True), want):
+        Hh.assert_close(a, b.double().cpu(), tol, name)
+    whole = torch.autograd.grad(flat.square().sum(), xs, retain_graph=True)
+    for a, b in zip(whole, torch.autograd.grad(ys, xs, [2 * y.detach() for y in ys])):
+        Hh.assert_close(a, b.double().cpu(), tol, name)
