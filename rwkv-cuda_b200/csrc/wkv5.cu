@@ -465,7 +465,6 @@ extern "C" size_t rwkvb200_wkv5_train_saved_bytes(int B, int T, int C, int H) {
 extern "C" int rwkvb200_wkv5_train_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v,
                                            const void* w_raw, const void* u, void* y, void* saved, void* stream) {
     if (int e = check_dims("wkv5_train_forward", dtype, B, T, C, H)) return e;
-    RWKV_REQUIRE(B * (i64)H <= 65535, RWKVB200_EINVAL, "wkv5_train_forward: B*H=%lld exceeds 65535", B * (i64)H);
     RWKV_NOTNULL(r); RWKV_NOTNULL(k); RWKV_NOTNULL(v); RWKV_NOTNULL(w_raw); RWKV_NOTNULL(u); RWKV_NOTNULL(y); RWKV_NOTNULL(saved);
     cudaStream_t st = as_stream(stream);
     if (dtype == RWKVB200_BF16 && wkv6_forward_choice() && chunked_ok<bf16>(T, C / H, {r, k, v, y, saved})) {
@@ -479,6 +478,7 @@ extern "C" int rwkvb200_wkv5_train_forward(int dtype, int B, int T, int C, int H
         }
     }
     if (C / H <= 64) {
+        RWKV_REQUIRE(B * (i64)H * (i64)wkv5_seg_count(T) < (1ll << 31), RWKVB200_EINVAL, "wkv5_train_forward: too many segments");
         const int e = wkv5_seg_forward(dtype, B, T, C, H, r, k, v, w_raw, u, y, static_cast<float*>(saved), st);
         return e ? e : 1;
     }

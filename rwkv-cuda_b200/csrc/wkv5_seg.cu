@@ -35,7 +35,7 @@ __device__ __forceinline__ float power(float lw, int e) { return e == 0 ? 1.f : 
 // In place: local end states -> state before each segment (REV: adjoint after each segment).  One thread per state element.
 template <typename E, bool REV>
 __global__ void __launch_bounds__(256) seg_scan_kernel(int T, int H, int N, int nseg, const E* __restrict__ w_, float* __restrict__ states) {
-    const int e = blockIdx.x * 256 + threadIdx.x, unit = blockIdx.y;
+    const int parts = (N * N + 255) / 256, unit = blockIdx.x / parts, e = blockIdx.x % parts * 256 + threadIdx.x;
     if (e >= N * N) return;
     const float lw = log_decay(w_ + (unit % H) * N + e / N);
     const float full = expf(lw * kSeg), tail = expf(lw * (float)(T - (nseg - 1) * kSeg));
@@ -57,13 +57,13 @@ __global__ void __launch_bounds__(256) seg_scan_kernel(int T, int H, int N, int 
     }
 }
 
-// grid (segments, units), 2 warps: a warp has the keys 32 warp .. of all values, a lane 8 keys x 8 values.
+// One block per (unit, segment), 2 warps: a warp has the keys 32 warp .. of all values, a lane 8 keys x 8 values.
 // REV = false: a = k, b = v; REV = true: a = r, b = gy.
 template <typename E, bool REV>
-__global__ void __launch_bounds__(64, 8) seg_local_kernel(int T, int C, int H, int N, const E* __restrict__ a_, const E* __restrict__ b_,
+__global__ void __launch_bounds__(64, 8) seg_local_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ a_, const E* __restrict__ b_,
                                                           const E* __restrict__ w_, float* __restrict__ states) {
     __shared__ __align__(16) float as[kSeg * kN], bs[kSeg * kN], lw[kN];
-    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, tid = threadIdx.x, lane = tid & 31;
+    const int unit = blockIdx.x / nseg, seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
     lw[tid] = tid < N ? log_decay(w_ + h * N + tid) : 0.f;
@@ -88,21 +88,21 @@ __global__ void __launch_bounds__(64, 8) seg_local_kernel(int T, int C, int H, i
 #pragma unroll
             for (int p = 0; p < 4; ++p) s[i][p] = fma2(a[p], b[i], s[i][p]);
     }
-    store_tile(s, states + ((i64)unit * gridDim.x + seg) * N * N, 8 * kg, 8 * vg, N);
+    store_tile(s, states + (i64)blockIdx.x * N * N, 8 * kg, 8 * vg, N);
 }
 
-// grid (segments, units), 2 warps: a warp has the values 32 warp .. of all keys
+// One block per (unit, segment), 2 warps: a warp has the values 32 warp .. of all keys
 template <typename E>
-__global__ void __launch_bounds__(64, 8) seg_y_kernel(int T, int C, int H, int N, const E* __restrict__ r_, const E* __restrict__ k_,
+__global__ void __launch_bounds__(64, 8) seg_y_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
                                                       const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
                                                       const float* __restrict__ states, E* __restrict__ y_) {
     __shared__ __align__(16) float rs[kSeg * kN], ks[kSeg * kN], vs[kSeg * kN], ws[kN], us[kN], ruk[kSeg];
-    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int unit = blockIdx.x / nseg, seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
     const int kg = lane >> 2, vg = 4 * warp + (lane & 3);
     Tile s;
-    load_tile(s, states + ((i64)unit * gridDim.x + seg) * N * N, 8 * kg, 8 * vg, N);
+    load_tile(s, states + (i64)blockIdx.x * N * N, 8 * kg, 8 * vg, N);
     stage<64>(rs, r_ + base, n, C, N, tid);
     stage<64>(ks, k_ + base, n, C, N, tid);
     stage<64>(vs, v_ + base, n, C, N, tid);
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(64, 8) seg_y_kernel(int T, int C, int H, int N
     }
 }
 
-// grid (segments, units), 4 warps: warps 0, 1 carry S and Z forward (gr, gw, gu), warps 2, 3 carry D backward (gk, gv); a warp
+// One block per (unit, segment), 4 warps: warps 0, 1 carry S and Z forward (gr, gw, gu), warps 2, 3 carry D backward (gk, gv); a warp
 // has 32 keys of all values.  gv sums over all keys: the two halves meet in shared memory at the end.
 struct BwdSmem {
     float r[kSeg * kN], k[kSeg * kN], v[kSeg * kN], g[kSeg * kN], gv[2][kSeg * kN];
@@ -147,20 +147,20 @@ struct BwdSmem {
 };
 
 template <typename E>
-__global__ void __launch_bounds__(128, 2) seg_backward_kernel(int T, int C, int H, int N, const E* __restrict__ r_, const E* __restrict__ k_,
+__global__ void __launch_bounds__(128, 2) seg_backward_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
                                                               const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
                                                               const E* __restrict__ gy_, const float* __restrict__ S_, const float* __restrict__ D_,
                                                               E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_,
                                                               float* __restrict__ partial_) {
     extern __shared__ __align__(16) unsigned char smem_seg[];
     BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_seg);
-    const int seg = blockIdx.x, unit = blockIdx.y, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int unit = blockIdx.x / nseg, seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
-    const float* D0 = D_ + ((i64)unit * gridDim.x + seg) * N * N;
+    const float* D0 = D_ + (i64)blockIdx.x * N * N;
     const int kg = 4 * (warp & 1) + (lane & 3), vg = lane >> 2, j_out = 8 * kg + vg;   // j_out: the key whose sums this lane ends with
     Tile s;
-    load_tile(s, warp < 2 ? S_ + ((i64)unit * gridDim.x + seg) * N * N : D0, 8 * kg, 8 * vg, N);
+    load_tile(s, warp < 2 ? S_ + (i64)blockIdx.x * N * N : D0, 8 * kg, 8 * vg, N);
     stage<128>(sm.r, r_ + base, n, C, N, tid);
     stage<128>(sm.k, k_ + base, n, C, N, tid);
     stage<128>(sm.v, v_ + base, n, C, N, tid);
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(128, 2) seg_backward_kernel(int T, int C, int 
         }
         const float gw = reduce8(x, lane);
         if (j_out < N) {
-            float* p = partial_ + ((i64)(unit / H) * gridDim.x + seg) * 2 * C + h * N + j_out;
+            float* p = partial_ + ((i64)(unit / H) * nseg + seg) * 2 * C + h * N + j_out;
             p[0] = log_decay(w_ + h * N + j_out) * gw;   // d log w / d w_raw = log w
             p[C] = gu;
         }
@@ -272,10 +272,10 @@ template <typename E>
 int forward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, void* y, float* states,
             cudaStream_t st) {
     const int N = C / H, nseg = (T + kSeg - 1) / kSeg;
-    const dim3 grid(nseg, B * H), scan((N * N + 255) / 256, B * H);
-    seg_local_kernel<E, false><<<grid, 64, 0, st>>>(T, C, H, N, (const E*)k, (const E*)v, (const E*)w, states);
+    const unsigned grid = (unsigned)(B * (i64)H * nseg), scan = (unsigned)(B * (i64)H * ((N * N + 255) / 256));
+    seg_local_kernel<E, false><<<grid, 64, 0, st>>>(T, C, H, N, nseg, (const E*)k, (const E*)v, (const E*)w, states);
     seg_scan_kernel<E, false><<<scan, 256, 0, st>>>(T, H, N, nseg, (const E*)w, states);
-    seg_y_kernel<E><<<grid, 64, 0, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states, (E*)y);
+    seg_y_kernel<E><<<grid, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states, (E*)y);
     return check_launch("wkv5_train_forward(segments)");
 }
 
@@ -283,12 +283,12 @@ template <typename E>
 int backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, const void* gy, void* gr,
              void* gk, void* gv, const float* S, float* D, float* partial, cudaStream_t st) {
     const int N = C / H, nseg = (T + kSeg - 1) / kSeg, smem = sizeof(BwdSmem);
-    const dim3 grid(nseg, B * H), scan((N * N + 255) / 256, B * H);
+    const unsigned grid = (unsigned)(B * (i64)H * nseg), scan = (unsigned)(B * (i64)H * ((N * N + 255) / 256));
     const cudaError_t e = allow_smem<seg_backward_kernel<E>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv5_train_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    seg_local_kernel<E, true><<<grid, 64, 0, st>>>(T, C, H, N, (const E*)r, (const E*)gy, (const E*)w, D);
+    seg_local_kernel<E, true><<<grid, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)gy, (const E*)w, D);
     seg_scan_kernel<E, true><<<scan, 256, 0, st>>>(T, H, N, nseg, (const E*)w, D);
-    seg_backward_kernel<E><<<grid, 128, smem, st>>>(T, C, H, N, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, (const E*)gy, S,
+    seg_backward_kernel<E><<<grid, 128, smem, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, (const E*)gy, S,
                                                     D, (E*)gr, (E*)gk, (E*)gv, partial);
     return check_launch("wkv5_train_backward(segments)");
 }
