@@ -305,7 +305,8 @@ int rwkvb200_wkv7_backward(int dtype, int B, int T, int H, int N, int chunk_len,
 /* Training flow with buffers of the library's own: rwkvb200_wkv7_train_path picks the kernels for a shape (0: those of
  * rwkvb200_wkv7_forward / _backward; 1: the chunks of a sequence in parallel, for launches with few (batch, head) units) and
  * the other calls are told it; `saved` is kept from the forward to the backward, `work` (may be NULL when its size is 0) is
- * free after each call.  s0, sT, dsT, ds0 may be NULL as above. */
+ * free after each call.  The forward of path 1 returns RWKVB200_EUNSUPPORTED, with nothing enqueued, where the driver makes
+ * no tensor maps; path 0 takes every call.  s0, sT, dsT, ds0 may be NULL as above. */
 int rwkvb200_wkv7_train_path(int dtype, int B, int T, int H, int N);
 size_t rwkvb200_wkv7_train_saved_bytes(int B, int T, int H, int N, int path);
 size_t rwkvb200_wkv7_train_work_bytes(int B, int T, int H, int path, int backward);

@@ -219,9 +219,10 @@ extern "C" int rwkvb200_wkv7_state_update(int dtype, int B, int T, int H, int N,
 // Path 1: the chunks in parallel (wkv7_scan.cu), for tensor-core shapes with at most a unit per two SMs: beyond that the extra
 // products cost more than the short chain saves (T 2048, forward + backward: 32 units 408 -> 226 us, 64 units 410 -> 345 us,
 // 80 units 413 -> 399 us, 128 units 421 -> 586 us), and up to 64 tokens there is next to nothing to walk in parallel.
+// Its forward answers EUNSUPPORTED, with nothing enqueued, where the driver makes no tensor maps: the call is then one of path 0.
 // Path 0: rwkvb200_wkv7_forward / _backward, `saved` = s then sa.
 extern "C" int rwkvb200_wkv7_train_path(int dtype, int B, int T, int H, int N) {
-    const bool tensor = dtype == RWKVB200_BF16 && N == 64 && g_wkv7_path.load() != 1 && g_wkv7_bwd_form.load() == 0 && !g_no_tensor_maps.load();
+    const bool tensor = dtype == RWKVB200_BF16 && N == 64 && g_wkv7_path.load() != 1 && g_wkv7_bwd_form.load() == 0;
     return tensor && T > 64 && 2ll * B * H <= sm_count() ? 1 : 0;
 }
 extern "C" size_t rwkvb200_wkv7_train_saved_bytes(int B, int T, int H, int N, int path) {

@@ -382,15 +382,21 @@ static Made wkv7_forward(const Tensor* s0, const Tensor& r, const Tensor& w, con
     const auto d = r.scalar_type(), f = at::kFloat;
     const int dtype = dt(r, "r");
     const int64_t B = r.size(0), T = r.size(1), H = r.size(2), N = r.size(3);
-    const int path = rwkvb200_wkv7_train_path(dtype, B, T, H, N);
     Tensor y = passing ? empty({B, T, H * N}, d, r) : same(v), sT = passing ? same(*s0) : Tensor();
-    Saved s{{r, w, k, v, a, b}, bytes(rwkvb200_wkv7_train_saved_bytes(B, T, H, N, path), r), {B, T, H, N, (s0 ? 1 : 0) + (passing ? 2 : 0), path}};
-    const size_t nwork = rwkvb200_wkv7_train_work_bytes(B, T, H, path, 0);
-    const Tensor work = nwork ? bytes(nwork, r) : Tensor();
-    check_rc(rwkvb200_wkv7_train_forward(dtype, B, T, H, N, path, s0 ? f32(ptr(*s0, "s0", f)) : nullptr, ptr(r, "r", d), ptr(w, "w", d),
-                                         ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
-                                         passing ? f32(sT.data_ptr()) : nullptr, s.own.data_ptr(), nwork ? work.data_ptr() : nullptr, stream()),
-             "rwkvb200_wkv7_train_forward");
+    Saved s{{r, w, k, v, a, b}, {}, {B, T, H, N, (s0 ? 1 : 0) + (passing ? 2 : 0)}};
+    auto run = [&](int path) {
+        s.dims[5] = path;
+        s.own = bytes(rwkvb200_wkv7_train_saved_bytes(B, T, H, N, path), r);
+        const size_t nwork = rwkvb200_wkv7_train_work_bytes(B, T, H, path, 0);
+        const Tensor work = nwork ? bytes(nwork, r) : Tensor();
+        return rwkvb200_wkv7_train_forward(dtype, B, T, H, N, path, s0 ? f32(ptr(*s0, "s0", f)) : nullptr, ptr(r, "r", d), ptr(w, "w", d),
+                                           ptr(k, "k", d), ptr(v, "v", d), ptr(a, "a", d), ptr(b, "b", d), y.data_ptr(),
+                                           passing ? f32(sT.data_ptr()) : nullptr, s.own.data_ptr(), nwork ? work.data_ptr() : nullptr, stream());
+    };
+    const int path = rwkvb200_wkv7_train_path(dtype, B, T, H, N);
+    int rc = run(path);
+    if (rc == RWKVB200_EUNSUPPORTED && path != 0) rc = run(0);   // no tensor maps here: path 0 has kernels without
+    check_rc(rc, "rwkvb200_wkv7_train_forward");
     // (the backward does not read s0: it is not kept, so that a program may carry its state in place)
     if (passing) return {"RWKV7_STATE_PASSING_CLAMPW_CUDA_OPBackward", wkv7_backward, {y, sT}, {r, w, k, v, a, b, *s0}, std::move(s)};
     if (s0) return {"RWKV7_STATE_CLAMPW_CUDA_OPBackward", wkv7_backward, {y}, {r, w, k, v, a, b, *s0}, std::move(s)};

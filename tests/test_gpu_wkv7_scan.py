@@ -60,3 +60,22 @@ def test_agrees_with_the_chunk_by_chunk_kernels():
         L.rwkvb200_wkv7_select_form(0)
     for n, t in got.items():
         Hh.assert_close(t, want[n].double().cpu(), 1e-2, n)
+
+
+@pytest.mark.parametrize("form", ["plain", "state", "passing"])
+def test_without_tensor_maps(form):
+    """Where no tensor maps can be made the forward of the parallel form refuses with nothing enqueued, and the classes take the
+    kernels that do without."""
+    import rwkv_cuda_b200 as R
+    from rwkv_cuda_b200 import _lib
+    B, T, H = 2, 160, 2
+    inp = Hh.v7_inputs(B, T, H, 64, seed=8)
+    assert _lib.lib().rwkvb200_wkv7_train_path(1, B, T, H, 64) == 1
+    want = run(inp, B, T, H, form)
+    try:
+        _lib.call("rwkvb200_test_disable_tensor_maps", 1)
+        got = run(inp, B, T, H, form)
+    finally:
+        _lib.call("rwkvb200_test_disable_tensor_maps", 0)
+    for n, t in got.items():
+        Hh.assert_close(t, want[n].double().cpu(), 1e-2, n)
