@@ -53,7 +53,7 @@ static std::atomic<int> g_wkv7_path{0};
 static std::atomic<int> g_wkv7_test_expire{0};
 static std::atomic<int> g_wkv7_bwd_form{0};   // 0 automatic, 1 one-group kernels, 2 staged forward / two-stage backward
 
-static int sm_count() {
+int rwkvb200::sm_count() {
     constexpr int kMaxDevices = 64;
     static std::atomic<int> cache[kMaxDevices] = {};
     int dev = 0, n = 0;

@@ -69,6 +69,9 @@ inline cudaError_t allow_smem(int bytes) {
 // out[n] (fp32 or bf16) <- sums over the rows of partial[rows][n] (wkv5.cu)
 int sum_rows(int out_dtype, long long rows, int n, const float* partial, void* out, cudaStream_t st);
 
+// SMs of the current device (0 if that cannot be told), for the rules that split work over them.
+int sm_count();
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // test hook (rwkvb200_test_disable_tensor_maps): true makes every tensor-map maker report failure, so that the

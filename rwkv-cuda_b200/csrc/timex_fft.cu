@@ -420,8 +420,9 @@ __global__ void __launch_bounds__(kThreads, 3) timex_fft_backward_kernel(const f
 // spectrum of the filter is made once per block).
 int splits(int B, int C, int G, int most) {
     const int rounds = ((B + 1) / 2 + G - 1) / G;
+    const int sms = sm_count();
     int s = 1;
-    while (s < most && s * 2 <= rounds && (rounds / (s * 2) >= 4 || C * s < 592) && C * s < 2368) s *= 2;
+    while (s < most && s * 2 <= rounds && (rounds / (s * 2) >= 4 || C * s < 4 * sms) && C * s < 16 * sms) s *= 2;
     return s;
 }
 

@@ -359,7 +359,8 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(i
 // so that several blocks share an SM.  No more segments than the sequence has.
 int pick_segments(int B, int T, int C, int most) {
     const i64 groups = (i64)B * ((C + 31) / 32);
-    int S = groups <= 148 ? 32 : groups <= 296 ? 16 : 8;
+    const int sms = sm_count();
+    int S = groups <= sms ? 32 : groups <= 2 * sms ? 16 : 8;
     while (S > 8 && (S > most || (S / 2) * L >= T)) S /= 2;
     return S;
 }

@@ -23,6 +23,7 @@
 // (16 rows) and, where a region is split, on token half w/4.  Shared memory: six [64][64] operand
 // arrays (each read K-major and MN-major as needed), P reusing the space of the U matrices.
 // Tensor memory (256 columns): E | ET | W1 | W2, the two work regions reused along the chunk.
+#include <algorithm>
 #include "wkv7_l32.cuh"
 #include "wkv7_dispatch.cuh"
 
@@ -583,11 +584,12 @@ int wkv7_l32_backward_chunks(int B, int T, int H, const void* r, const void* w, 
     // Chunks per block: the fewest waves of blocks, two per SM, where starting a block costs about half a chunk (its first tiles
     // and the adjoint arrive with nothing to hide them).
     const int nch = (T + v7x::LC - 1) / v7x::LC;
+    const long long places = 2ll * std::max(1, sm_count());
     int group = 1;
     double best = 1e30;
     for (int g = 1; g <= nch; ++g) {
         const long long blocks = (long long)B * H * ((nch + g - 1) / g);
-        const double cost = (double)((blocks + 295) / 296) * (g + 0.5);
+        const double cost = (double)((blocks + places - 1) / places) * (g + 0.5);
         if (cost < best) { best = cost; group = g; }
     }
     return launch_l32_backward(B, T, H, group, r, w, k, v, a, b, dy, nullptr, adj, states, nullptr, dr, dw, dk, dv, da, db, st);

@@ -599,7 +599,7 @@ int wkv7_scan_forward(int B, int T, int H, const float* s0, const void* r, const
     unsigned char* recA = static_cast<unsigned char*>(saved) + (size_t)B * H * nch * 64 * 64 * sizeof(float);
     const long long total = (long long)B * H * nch;
     RWKV_REQUIRE(total < (1ll << 31), RWKVB200_EINVAL, "wkv7_train_forward: too many chunks");
-    wkv7_ops_kernel<<<(int)std::min<long long>(total, 2 * 148), 128, OpsSmem::kBytes, st>>>(T, H, nch, (int)total, maps, recA, static_cast<unsigned char*>(work));
+    wkv7_ops_kernel<<<(int)std::min<long long>(total, 2 * std::max(1, sm_count())), 128, OpsSmem::kBytes, st>>>(T, H, nch, (int)total, maps, recA, static_cast<unsigned char*>(work));
     wkv7_chain_forward_kernel<<<dim3(H, B), 320, ChainSmem::kBytes, st>>>(T, H, nch, s0, recA, static_cast<unsigned char*>(work), (bf16*)y, sT, states);
     return check_launch("wkv7_train_forward(chunks in parallel)");
 }
