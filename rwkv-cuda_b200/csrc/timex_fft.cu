@@ -13,15 +13,14 @@
 // the other.  A value that is not finite, or too large for the sums of a transform, would spoil the whole row, the tokens before
 // it too, and the row beside it: such a row, and all rows of a channel whose filter has such a value, are added up directly.
 // What remains is a bound by row: errors are about 4 2^-24 of (norm of the filter) x (norm of the row), at early tokens too.
-// (Looking at every pair costs a step of B32 C768 T768 320 -> 339 us.)
 //
 // A transform of N = 256 R points (R = 4, 8) is done by N/16 threads with 16 points each: radix 16, exchange through shared
 // memory, radix 16, exchange inside groups of R lanes, radix R.  Spectra stay in the order this leaves them in (thread and
 // register); the inverse takes the same steps backwards, so nothing is ever reordered.  The upper half of the input is zero
 // and the upper half of the output is not needed: the outer radix-16 steps do half of their work.  Row strides in shared
 // memory (L + R, and 16 (R+1) + R) make every exchange conflict free.  128 threads per block, 2048 / N transforms at a time.
-// B32 C768 T768 on a B200: forward 357 us direct, 100 us here; backward with its gw over the batch 1017 and 207 us.  Errors
-// against fp64 are 2.3e-7 of the norm (direct: 4.2e-7).
+// B32 C768 T768 on a B200: forward 357 us direct, 112 us here; backward with its gw over the batch 1017 and 236 us
+// (looking at the pairs is 19 us of these).  Errors against fp64 are 2.4e-7 of the norm (direct: 4.1e-7).
 #include "timex_fft.cuh"
 
 namespace rwkvb200 {
