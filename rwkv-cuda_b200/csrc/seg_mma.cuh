@@ -1,0 +1,864 @@
+// Matrix forms of the kernels that work on the time segments of a sequence at the same time (wkv5_seg.cu, wkv6_seg.cu): head
+// size 64, segments of 32 tokens, fp32 or bf16 activations, fp32 precision throughout.
+//
+// Inside a segment the recurrence is a set of small products (S: state before the segment, D: adjoint after it, both [key j]
+// [value i]; L_t: sum of log decays up to token t; m: the middle of the segment, where the scaled vectors are anchored so that
+// neither side of a product runs out of fp32's range):
+//   r~_t = r_t exp(L_{t-1} - L_m)    k~_s = k_s exp(L_m - L_s)    S' = exp(L_m) S    D' = exp(L_end - L_m) D
+//   A[s,t] = k~_s.r~_t (s < t), A[t,t] = sum_j r_t u k_t      G[s,t] = v_s.gy_t (s < t), gamma_t = v_t.gy_t
+//   y  = R~ S' + A^T V
+//   gv = K~ D' + A gY      dk~ = V D'^T + G R~      dr~ = gY S'^T + G^T K~
+//   gk_s = dk~_s exp(L_m - L_s) + gamma_s u r_s     gr_t = dr~_t exp(L_{t-1} - L_m) + gamma_t u k_t
+// and with P_t = r~_t dr~_t, Q_s = k~_s dk~_s (elementwise, without the u terms) and A_end = sum_i D S_end
+//   dL/dlog d_t = A_end - sum_{tau > t} (Q_tau - P_tau) - Q_t      A_end = sum_i D' S' + sum_s k~_s (V D'^T)_s
+//
+// Precision: the products run on mma.sync with bf16 operands, every fp32 operand as the sum of three bf16 numbers (24 bits: the
+// split is exact) and all partial products down to 2^-16 of the largest taken: 3 where the other side is a bf16 tensor as it
+// came, else 6.  What is left out is below 2^-25 of a product.
+// Why mma.sync and not tcgen05: these kernels are a block per segment with every accumulator and both states in registers,
+// four blocks per SM; the operands are split where they are used, and at 8 clocks per instruction and scheduler the tensor pipe
+// needs about as long as the arithmetic around it.
+// A segment whose decays leave the range (more than 2^-kRange between its middle and an end) or that holds values that are not
+// finite (a masked product would spread them over tokens before) is flagged and left to the token-by-token kernels.
+#pragma once
+#include "seg_tiles.cuh"
+
+namespace rwkvb200 {
+namespace {
+
+constexpr float kRange = 86.f;                 // log2; 60 in nats
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kImg = kSeg * 128;               // bytes of one bf16 image [32 tokens][64 channels]
+constexpr int kMld = 40;                       // floats of a row of a token x token matrix: 8-byte fragment reads hit every bank once
+
+// ---- bf16 images: rows of 128 bytes, their 16-byte pieces XOR-ed with the row ------------------------------------------------
+__device__ __forceinline__ uint32_t img_at(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// Fragments of mma.m16n8k16 by ldmatrix.  The place that a lane points at: (r0, c0) = first row, first 16-byte piece.
+//   frag_rows: A[m][k] from rows m, B[k][n] from rows k (transposed);  frag_cols: A from rows k (transposed), B from rows n
+// an x4 load is one A fragment, or the B fragments of two neighbouring n-tiles.
+__device__ __forceinline__ uint32_t frag_rows(int r0, int c0, int lane) { return img_at(r0 + (lane & 15), c0 + (lane >> 4)); }
+__device__ __forceinline__ uint32_t frag_cols(int r0, int c0, int lane) { return img_at(r0 + (lane & 7) + ((lane >> 4) << 3), c0 + ((lane >> 3) & 1)); }
+__device__ __forceinline__ void ldsm(uint32_t (&f)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_t(uint32_t (&f)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(addr) : "memory");
+}
+template <int NS>
+__device__ __forceinline__ void ldsm(uint32_t (&f)[NS][4], uint32_t addr) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) ldsm(f[s], addr + s * kImg);
+}
+template <int NS>
+__device__ __forceinline__ void ldsm_t(uint32_t (&f)[NS][4], uint32_t addr) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) ldsm_t(f[s], addr + s * kImg);
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// c[mt][nt] += a[mt] b[nt], split operands: the small partial products first
+template <int MT, int NA, int NB>
+__device__ __forceinline__ void mma_split(float (&c)[MT][2][4], const uint32_t (&a)[MT][NA][4], const uint32_t (&b)[NB][4]) {
+#pragma unroll
+    for (int order = (NA > 1 ? 2 : 0) + (NB > 1 ? 2 : 0); order >= 0; --order) {
+        if (order > 2) continue;
+#pragma unroll
+        for (int pa = 0; pa < NA; ++pa) {
+            const int pb = order - pa;
+            if (pb < 0 || pb >= NB) continue;
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                mma(c[mt][0], a[mt][pa], b[pb][0], b[pb][1]);
+                mma(c[mt][1], a[mt][pa], b[pb][2], b[pb][3]);
+            }
+        }
+    }
+}
+// x = sum of three bf16 numbers, two values at a time (the first in the low half)
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
+__device__ __forceinline__ float bf16_lo(uint32_t x) { return __uint_as_float(x << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t x) { return __uint_as_float(x & 0xffff0000u); }
+__device__ __forceinline__ void split3(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+    h = pack_bf16(x0, x1);
+    x0 -= bf16_lo(h); x1 -= bf16_hi(h);
+    m = pack_bf16(x0, x1);
+    x0 -= bf16_lo(m); x1 -= bf16_hi(m);
+    l = pack_bf16(x0, x1);
+}
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// ---- two neighbouring channels of a token, as loaded and decoded --------------------------------------------------------------
+template <typename E> struct PairOf;
+template <> struct PairOf<bf16> { using T = uint32_t; };
+template <> struct PairOf<float> { using T = float2; };
+template <typename E> using Pair = typename PairOf<E>::T;
+__device__ __forceinline__ uint32_t read_pair(const bf16* p, bool vec) {
+    if (vec) return __ldg(reinterpret_cast<const uint32_t*>(p));
+    const unsigned short* q = reinterpret_cast<const unsigned short*>(p);
+    return (uint32_t)__ldg(q) | (uint32_t)__ldg(q + 1) << 16;
+}
+__device__ __forceinline__ float2 read_pair(const float* p, bool vec) {
+    return vec ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(__ldg(p), __ldg(p + 1));
+}
+__device__ __forceinline__ float2 decode(uint32_t x) { return make_float2(bf16_lo(x), bf16_hi(x)); }
+__device__ __forceinline__ float2 decode(float2 x) { return x; }
+template <typename E> __device__ __forceinline__ Pair<E> no_pair();
+template <> __device__ __forceinline__ uint32_t no_pair<bf16>() { return 0u; }
+template <> __device__ __forceinline__ float2 no_pair<float>() { return make_float2(0.f, 0.f); }
+template <typename E> __device__ __forceinline__ bool vec_ok(const E* p, int elements) { return (reinterpret_cast<uintptr_t>(p) & (elements * sizeof(E) - 1)) == 0; }
+// rows t0 .. t0 + 7 of two channels
+template <typename E>
+__device__ __forceinline__ void read_rows(Pair<E> (&x)[8], const E* p, int t0, int n, int C, bool vec) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = t0 + i < n ? read_pair(p + (i64)(t0 + i) * C, vec) : no_pair<E>();
+}
+
+// images of a tensor as it came: bf16 one image, fp32 three
+template <typename E> constexpr int kParts = sizeof(E) == 2 ? 1 : 3;
+template <typename E>
+__device__ __forceinline__ void put_pair(unsigned char* img, int row, int lane, Pair<E> x);   // channels 2 lane, 2 lane + 1
+template <>
+__device__ __forceinline__ void put_pair<bf16>(unsigned char* img, int row, int lane, uint32_t x) {
+    *reinterpret_cast<uint32_t*>(img + img_at(row, lane >> 2) + (lane & 3) * 4) = x;
+}
+__device__ __forceinline__ void put_split(unsigned char* img, int row, int lane, float x, float y) {
+    uint32_t h, m, l;
+    split3(x, y, h, m, l);
+    unsigned char* p = img + img_at(row, lane >> 2) + (lane & 3) * 4;
+    *reinterpret_cast<uint32_t*>(p) = h;
+    *reinterpret_cast<uint32_t*>(p + kImg) = m;
+    *reinterpret_cast<uint32_t*>(p + 2 * kImg) = l;
+}
+template <>
+__device__ __forceinline__ void put_pair<float>(unsigned char* img, int row, int lane, float2 x) { put_split(img, row, lane, x.x, x.y); }
+
+// sums that are 0 unless one of the values is not finite
+__device__ __forceinline__ void check(float& bad, float2 x) { bad = fmaf(x.y, 0.f, fmaf(x.x, 0.f, bad)); }
+
+// log2 of the decays of two channels, from their raw inputs
+__device__ __forceinline__ float2 log2_decay(float2 w) { return make_float2(-kLog2e * ex2(kLog2e * w.x), -kLog2e * ex2(kLog2e * w.y)); }
+__device__ __forceinline__ float2 log2_decay_static(float2 w) { return make_float2(-kLog2e * expf(w.x), -kLog2e * expf(w.y)); }
+
+// ---- operands of a segment ---------------------------------------------------------------------------------------------------
+// 128 threads: channels 2 lane, 2 lane + 1 of the tokens 8 warp ..  Leaves the images of r~, k~, the bonus sums, S's and D's factors
+// and (ROWS) log2 of exp(L_{t-1} - L_m) as rows, row 32: the end.  True where the segment has to be left to the other kernels.
+struct Operands {
+    unsigned char R[3 * kImg], K[3 * kImg];
+    float tot[4 * kN], ruk[kSeg], em[kN], em2[kN];
+};
+template <typename E, bool STATIC, bool ROWS>
+__device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid, int n, int C, const E* __restrict__ r_, const E* __restrict__ k_,
+                                              const E* __restrict__ w_, const E* __restrict__ u_) {
+    const int lane = tid & 31, q = tid >> 5, c = 2 * lane, t0 = 8 * q;
+    Pair<E> rr[8], kk[8], ww[STATIC ? 1 : 8];
+    const bool vec = vec_ok(r_, 2) && vec_ok(k_, 2) && vec_ok(w_, 2);
+    read_rows<E>(rr, r_ + c, t0, n, C, vec);
+    read_rows<E>(kk, k_ + c, t0, n, C, vec);
+    if constexpr (!STATIC) read_rows<E>(ww, w_ + c, t0, n, C, vec);
+    else ww[0] = read_pair(w_ + c, vec);
+    const float2 u = decode(read_pair(u_ + c, vec_ok(u_, 2)));
+    float2 d[STATIC ? 1 : 8], pre, lm, le;   // log2 decays; L before the first of these tokens, L at the middle, L from there to the end
+    if constexpr (STATIC) {
+        d[0] = log2_decay_static(decode(ww[0]));
+        const float nm = (float)min(n, kSeg / 2), ne = (float)n - nm;
+        lm = make_float2(d[0].x * nm, d[0].y * nm);
+        le = make_float2(d[0].x * ne, d[0].y * ne);
+    } else {
+        float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            d[i] = t0 + i < n ? log2_decay(decode(ww[i])) : make_float2(0.f, 0.f);
+            s.x += d[i].x; s.y += d[i].y;
+        }
+        *reinterpret_cast<float2*>(o.tot + q * kN + c) = s;
+        __syncthreads();
+        float2 t[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) t[i] = *reinterpret_cast<const float2*>(o.tot + i * kN + c);
+        lm = make_float2(t[0].x + t[1].x, t[0].y + t[1].y);
+        le = make_float2(t[2].x + t[3].x, t[2].y + t[3].y);
+        pre = q == 0 ? make_float2(-lm.x, -lm.y) : q == 1 ? make_float2(-t[1].x, -t[1].y) : q == 2 ? make_float2(0.f, 0.f) : t[2];
+    }
+    float bad = 0.f, x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        float2 a, b;   // L before and after the token, from the middle
+        if constexpr (STATIC) {
+            const float ta = (float)(min(t0 + i, n) - min(n, kSeg / 2)), tb = (float)(min(t0 + i + 1, n) - min(n, kSeg / 2));
+            a = make_float2(d[0].x * ta, d[0].y * ta);
+            b = make_float2(d[0].x * tb, d[0].y * tb);
+        } else {
+            a = pre;
+            b = pre = make_float2(pre.x + d[i].x, pre.y + d[i].y);
+        }
+        if (ROWS) *reinterpret_cast<float2*>(rows + (t0 + i) * kN + c) = a;
+        const float2 r = decode(rr[i]), k = decode(kk[i]);
+        const float2 rs = make_float2(r.x * ex2(a.x), r.y * ex2(a.y)), ks = make_float2(k.x * ex2(-b.x), k.y * ex2(-b.y));
+        check(bad, rs); check(bad, ks);
+        put_split(o.R, t0 + i, lane, rs.x, rs.y);
+        put_split(o.K, t0 + i, lane, ks.x, ks.y);
+        x[i] = fmaf(r.x * u.x, k.x, r.y * u.y * k.y);
+        if (ROWS && q == 3 && i == 7) *reinterpret_cast<float2*>(rows + kSeg * kN + c) = b;
+    }
+    float s = reduce8(x, lane);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if ((lane & 3) == 0) o.ruk[t0 + (lane >> 2)] = s;
+    if (q == 0) {
+        *reinterpret_cast<float2*>(o.em + c) = make_float2(ex2(lm.x), ex2(lm.y));
+        *reinterpret_cast<float2*>(o.em2 + c) = make_float2(ex2(le.x), ex2(le.y));
+    }
+    check(bad, make_float2(s, 0.f));
+    const bool in = lm.x >= -kRange && lm.y >= -kRange && le.x >= -kRange && le.y >= -kRange;
+    return !(in && bad == 0.f);
+}
+// the images of a tensor as it came (pieces of 16 bytes where the alignment allows)
+template <typename E>
+__device__ __forceinline__ bool stage_images(unsigned char* img, int tid, int n, int C, const E* __restrict__ x_) {
+    float bad = 0.f;
+    const int lane = tid & 31, t0 = 8 * (tid >> 5);
+    if (sizeof(E) == 2 && vec_ok(x_, 8)) {
+        uint4 x[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int row = 16 * i + (tid >> 3);
+            x[i] = row < n ? __ldg(reinterpret_cast<const uint4*>(x_ + (i64)row * C + 8 * (tid & 7))) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            *reinterpret_cast<uint4*>(img + img_at(16 * i + (tid >> 3), tid & 7)) = x[i];
+            check(bad, decode(x[i].x)); check(bad, decode(x[i].y)); check(bad, decode(x[i].z)); check(bad, decode(x[i].w));
+        }
+    } else {
+        Pair<E> x[8];
+        read_rows<E>(x, x_ + 2 * lane, t0, n, C, vec_ok(x_, 2));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            check(bad, decode(x[i]));
+            put_pair<E>(img, t0 + i, lane, x[i]);
+        }
+    }
+    return bad != 0.f;
+}
+
+// Token x token products: c = rows 16 mt .. of one set of images times rows 16 nt .. of another, over the 64 channels
+template <int NA, int NB>
+__device__ __forceinline__ void gram(float (&c)[1][2][4], const unsigned char* a_img, const unsigned char* b_img, int mt, int nt, int lane) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[0][0][e] = c[0][1][e] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        uint32_t a[1][NA][4], b[NB][4];
+        ldsm<NA>(a[0], smem_addr(a_img) + frag_rows(16 * mt, 2 * kk, lane));
+        ldsm<NB>(b, smem_addr(b_img) + frag_cols(16 * nt, 2 * kk, lane));
+        mma_split<1, NA, NB>(c, a, b);
+    }
+}
+// An A fragment from a token x token matrix in shared memory, as stored or transposed
+template <bool TRANS>
+__device__ __forceinline__ void matrix_frag(uint32_t (&f)[3][4], const float* m, int m0, int k0, int lane) {
+    const int g = lane >> 2, q = lane & 3;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int row = m0 + g + 8 * (e & 1), col = k0 + 2 * q + 8 * (e >> 1);
+        float2 x;
+        if (TRANS) x = make_float2(m[col * kMld + row], m[(col + 1) * kMld + row]);
+        else x = *reinterpret_cast<const float2*>(m + row * kMld + col);
+        split3(x.x, x.y, f[0][e], f[1][e], f[2][e]);
+    }
+}
+
+// Rows of 16 channels out of two accumulator tiles: neighbouring lanes swap a pair, so that a lane stores four channels
+template <typename E>
+__device__ __forceinline__ void store_row(E* row, float x0, float x1, float z0, float z1, int lane, bool vec, bool in);
+template <>
+__device__ __forceinline__ void store_row<bf16>(bf16* row, float x0, float x1, float z0, float z1, int lane, bool vec, bool in) {
+    const uint32_t x = pack_bf16(x0, x1), z = pack_bf16(z0, z1);
+    const bool odd = lane & 1;
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? x : z, 1);
+    if (!in) return;
+    const uint2 v = odd ? make_uint2(got, z) : make_uint2(x, got);
+    bf16* p = row + (odd ? 8 + 2 * ((lane & 3) - 1) : 2 * (lane & 3));
+    if (vec) *reinterpret_cast<uint2*>(p) = v;
+    else {
+        unsigned short* s = reinterpret_cast<unsigned short*>(p);
+        s[0] = (unsigned short)v.x; s[1] = (unsigned short)(v.x >> 16); s[2] = (unsigned short)v.y; s[3] = (unsigned short)(v.y >> 16);
+    }
+}
+template <>
+__device__ __forceinline__ void store_row<float>(float* row, float x0, float x1, float z0, float z1, int lane, bool vec, bool in) {
+    const bool odd = lane & 1;
+    const float g0 = __shfl_xor_sync(0xffffffffu, odd ? x0 : z0, 1), g1 = __shfl_xor_sync(0xffffffffu, odd ? x1 : z1, 1);
+    if (!in) return;
+    const float4 v = odd ? make_float4(g0, g1, z0, z1) : make_float4(x0, x1, g0, g1);
+    float* p = row + (odd ? 8 + 2 * ((lane & 3) - 1) : 2 * (lane & 3));
+    if (vec) *reinterpret_cast<float4*>(p) = v;
+    else { p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w; }
+}
+
+// ---- kernels -----------------------------------------------------------------------------------------------------------------
+// y of a segment from its start state.  One block per (unit, segment), 4 warps; a warp has 16 values of all tokens.
+template <typename E>
+struct YSmem {
+    Operands o;
+    unsigned char V[kParts<E> * kImg];
+    float M[kSeg * kMld];   // A transposed: [t][s]
+};
+template <typename E, bool STATIC>
+__global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
+                                                           const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
+                                                           const float* __restrict__ states, E* __restrict__ y_, int* __restrict__ flags) {
+    extern __shared__ __align__(128) unsigned char smem_seg_y[];
+    YSmem<E>& sm = *reinterpret_cast<YSmem<E>*>(smem_seg_y);
+    constexpr int NV = kParts<E>;
+    const i64 unit = blockIdx.x / nseg;
+    const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
+    const int g = lane >> 2, q = lane & 3, n = min(kSeg, T - seg * kSeg);
+    const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    float S[4][2][4];   // [16 keys][8 values] as B fragments
+    {
+        const float* p = states + (i64)blockIdx.x * kN * kN + 16 * warp + g;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[kk][nt][e] = p[(16 * kk + 2 * q + (e & 1) + 8 * (e >> 1)) * kN + 8 * nt];
+    }
+    bool bad = make_operands<E, STATIC, false>(sm.o, nullptr, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN);
+    bad |= stage_images<E>(sm.V, tid, n, C, v_ + base);
+    if (__syncthreads_or(bad)) {
+        if (tid == 0) flags[blockIdx.x] = 1;
+        return;
+    }
+    if (tid == 0) flags[blockIdx.x] = 0;
+    // A: three of the warps a 16 x 16 tile each, and which three turns with the block (a warp's number is its scheduler)
+    const int job = (warp + blockIdx.x) & 3;
+    if (job < 3) {
+        const int mt = job > 0, nt = job > 1;
+        float c[1][2][4];
+        gram<3, 3>(c, sm.o.R, sm.o.K, mt, nt, lane);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int t = 16 * mt + g + 8 * (e >> 1), s = 16 * nt + 8 * j + 2 * q + (e & 1);
+                sm.M[t * kMld + s] = s < t ? c[0][j][e] : s == t ? sm.o.ruk[t] : 0.f;
+            }
+    }
+    float acc[2][2][4];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[mt][0][e] = acc[mt][1][e] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+        uint32_t a[2][3][4], b[3][4];
+        const float2 f0 = *reinterpret_cast<const float2*>(sm.o.em + 16 * kk + 2 * q), f1 = *reinterpret_cast<const float2*>(sm.o.em + 16 * kk + 8 + 2 * q);
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            split3(S[kk][nt][0] * f0.x, S[kk][nt][1] * f0.y, b[0][2 * nt], b[1][2 * nt], b[2][2 * nt]);
+            split3(S[kk][nt][2] * f1.x, S[kk][nt][3] * f1.y, b[0][2 * nt + 1], b[1][2 * nt + 1], b[2][2 * nt + 1]);
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) ldsm<3>(a[mt], smem_addr(sm.o.R) + frag_rows(16 * mt, 2 * kk, lane));
+        mma_split<2, 3, 3>(acc, a, b);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int kt = 0; kt < 2; ++kt) {
+        uint32_t b[NV][4];
+        ldsm_t<NV>(b, smem_addr(sm.V) + frag_rows(16 * kt, 2 * warp, lane));
+#pragma unroll
+        for (int mt = kt; mt < 2; ++mt) {
+            uint32_t a[1][3][4];
+            matrix_frag<false>(a[0], sm.M, 16 * mt, 16 * kt, lane);
+            float(&c)[1][2][4] = *reinterpret_cast<float(*)[1][2][4]>(&acc[mt]);
+            mma_split<1, 3, NV>(c, a, b);
+        }
+    }
+    const bool vec = vec_ok(y_, 4);
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int t = 16 * mt + g + 8 * e;
+            store_row<E>(y_ + base + (i64)t * C + 16 * warp, acc[mt][0][2 * e], acc[mt][0][2 * e + 1], acc[mt][1][2 * e], acc[mt][1][2 * e + 1], lane, vec, t < n);
+        }
+}
+
+// Gradients of a segment from its start state S and the adjoint D behind it.  One block per (unit, segment), 4 warps; a warp has
+// 16 keys (gr, gk, gw, gu) and 16 values (gv) of all tokens.  STATIC: out2 = partials (gw, gu) of the segment, rows of 2 C.
+template <typename E>
+struct BwdSmemM {
+    Operands o;
+    unsigned char V[kParts<E> * kImg], G[kParts<E> * kImg];
+    float A[kSeg * kMld], Gm[kSeg * kMld];
+    float rows[(kSeg + 1) * kN], gamma[kSeg], a0[kN];
+};
+template <typename E, bool STATIC>
+__global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
+    seg_mma_backward_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_, const E* __restrict__ v_,
+                            const E* __restrict__ w_, const E* __restrict__ u_, const E* __restrict__ gy_, const float* __restrict__ S_,
+                            const float* __restrict__ D_, E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_, E* __restrict__ gw_,
+                            float* __restrict__ partial_, int* __restrict__ flags) {
+    extern __shared__ __align__(128) unsigned char smem_seg_b[];
+    BwdSmemM<E>& sm = *reinterpret_cast<BwdSmemM<E>*>(smem_seg_b);
+    constexpr int NV = kParts<E>;
+    const i64 unit = blockIdx.x / nseg;
+    const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
+    const int g = lane >> 2, q = lane & 3, n = min(kSeg, T - seg * kSeg);
+    const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    bool bad = make_operands<E, STATIC, true>(sm.o, sm.rows, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN);
+    bad |= stage_images<E>(sm.V, tid, n, C, v_ + base);
+    bad |= stage_images<E>(sm.G, tid, n, C, gy_ + base);
+    if (__syncthreads_or(bad)) {
+        if (tid == 0) flags[blockIdx.x] = 1;
+        return;
+    }
+    if (tid == 0) flags[blockIdx.x] = 0;
+    const bool vec = vec_ok(gr_, 4) && vec_ok(gk_, 4) && vec_ok(gv_, 4) && (STATIC || vec_ok(gw_, 4));
+    // the two token x token matrices, 16 x 16 tiles (0,0), (0,1), (1,1): A six partial products each; G one (bf16) or six (fp32)
+    for (int job = (warp + blockIdx.x) & 3; job < 6; job = job >= 3 && NV == 1 ? job + 1 : NV == 1 ? 6 : job + 4) {
+        const int tile = job % 3, mt = tile > 1, nt = tile > 0;
+        float c[1][2][4];
+        if (job < 3) gram<3, 3>(c, sm.o.K, sm.o.R, mt, nt, lane);
+        else gram<NV, NV>(c, sm.V, sm.G, mt, nt, lane);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int s = 16 * mt + g + 8 * (e >> 1), t = 16 * nt + 8 * j + 2 * q + (e & 1);
+                const float x = c[0][j][e];
+                if (job < 3) sm.A[s * kMld + t] = s < t ? x : s == t ? sm.o.ruk[t] : 0.f;
+                else {
+                    sm.Gm[s * kMld + t] = s < t ? x : 0.f;
+                    if (s == t) sm.gamma[t] = x;
+                }
+            }
+    }
+    {   // gv = K~ D' + A gY
+        float acc[2][2][4];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[mt][0][e] = acc[mt][1][e] = 0.f;
+        const float* p = D_ + (i64)blockIdx.x * kN * kN + 16 * warp + g;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            uint32_t a[2][3][4], b[3][4];
+            const float2 f0 = *reinterpret_cast<const float2*>(sm.o.em2 + 16 * kk + 2 * q), f1 = *reinterpret_cast<const float2*>(sm.o.em2 + 16 * kk + 8 + 2 * q);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                float x[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[e] = p[(16 * kk + 2 * q + (e & 1) + 8 * (e >> 1)) * kN + 8 * nt];
+                split3(x[0] * f0.x, x[1] * f0.y, b[0][2 * nt], b[1][2 * nt], b[2][2 * nt]);
+                split3(x[2] * f1.x, x[3] * f1.y, b[0][2 * nt + 1], b[1][2 * nt + 1], b[2][2 * nt + 1]);
+            }
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) ldsm<3>(a[mt], smem_addr(sm.o.K) + frag_rows(16 * mt, 2 * kk, lane));
+            mma_split<2, 3, 3>(acc, a, b);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kt = 0; kt < 2; ++kt) {
+            uint32_t b[NV][4];
+            ldsm_t<NV>(b, smem_addr(sm.G) + frag_rows(16 * kt, 2 * warp, lane));
+#pragma unroll
+            for (int mt = 0; mt <= kt; ++mt) {
+                uint32_t a[1][3][4];
+                matrix_frag<false>(a[0], sm.A, 16 * mt, 16 * kt, lane);
+                float(&c)[1][2][4] = *reinterpret_cast<float(*)[1][2][4]>(&acc[mt]);
+                mma_split<1, 3, NV>(c, a, b);
+            }
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int t = 16 * mt + g + 8 * e;
+                store_row<E>(gv_ + base + (i64)t * C + 16 * warp, acc[mt][0][2 * e], acc[mt][0][2 * e + 1], acc[mt][1][2 * e], acc[mt][1][2 * e + 1], lane, vec, t < n);
+            }
+    }
+    // dk~ = V D'^T + G R~, dr~ = gY S'^T + G^T K~
+    float dk[2][2][4], dr[2][2][4], a0[2] = {0.f, 0.f};
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dk[mt][nt][e] = dr[mt][nt][e] = 0.f;
+    {
+        const i64 so = (i64)blockIdx.x * kN * kN + (16 * warp + g) * kN + 2 * q;
+        float fs[2], fd[2];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) { fs[nt] = sm.o.em[16 * warp + 8 * nt + g]; fd[nt] = sm.o.em2[16 * warp + 8 * nt + g]; }
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+            uint32_t bs[3][4], bd[3][4];
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float2 s = *reinterpret_cast<const float2*>(S_ + so + 8 * nt * kN + 16 * kk + 8 * e);
+                    float2 x = *reinterpret_cast<const float2*>(D_ + so + 8 * nt * kN + 16 * kk + 8 * e);
+                    s.x *= fs[nt]; s.y *= fs[nt]; x.x *= fd[nt]; x.y *= fd[nt];
+                    a0[nt] = fmaf(s.x, x.x, fmaf(s.y, x.y, a0[nt]));
+                    split3(s.x, s.y, bs[0][2 * nt + e], bs[1][2 * nt + e], bs[2][2 * nt + e]);
+                    split3(x.x, x.y, bd[0][2 * nt + e], bd[1][2 * nt + e], bd[2][2 * nt + e]);
+                }
+            uint32_t a[2][NV][4];
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) ldsm<NV>(a[mt], smem_addr(sm.V) + frag_rows(16 * mt, 2 * kk, lane));
+            mma_split<2, NV, 3>(dk, a, bd);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) ldsm<NV>(a[mt], smem_addr(sm.G) + frag_rows(16 * mt, 2 * kk, lane));
+            mma_split<2, NV, 3>(dr, a, bs);
+        }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {   // a0: sum over the values of a key, to the lanes that have its column below
+        a0[nt] += __shfl_xor_sync(0xffffffffu, a0[nt], 1);
+        a0[nt] += __shfl_xor_sync(0xffffffffu, a0[nt], 2);
+        if (q == 0) sm.a0[16 * warp + 8 * nt + g] = a0[nt];
+    }
+    __syncwarp();
+    Pair<E> rp[2][2][2], kp[2][2][2];   // [16 tokens][8 of them][tile]
+    {
+        const bool vin = vec_ok(r_, 2) && vec_ok(k_, 2);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    const int t = 16 * mt + 8 * e + g;
+                    const i64 o = base + (i64)t * C + 16 * warp + 8 * nt + 2 * q;
+                    rp[mt][e][nt] = t < n ? read_pair(r_ + o, vin) : no_pair<E>();
+                    kp[mt][e][nt] = t < n ? read_pair(k_ + o, vin) : no_pair<E>();
+                }
+    }
+    float2 aend[2];
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+        const int c = 16 * warp + 8 * nt + 2 * q;
+        float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float2 k = decode(kp[mt][e][nt]), l = *reinterpret_cast<const float2*>(sm.rows + (16 * mt + 8 * e + g + 1) * kN + c);
+                s.x = fmaf(k.x * ex2(-l.x), dk[mt][nt][2 * e], s.x);
+                s.y = fmaf(k.y * ex2(-l.y), dk[mt][nt][2 * e + 1], s.y);
+            }
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) {
+            s.x += __shfl_xor_sync(0xffffffffu, s.x, m);
+            s.y += __shfl_xor_sync(0xffffffffu, s.y, m);
+        }
+        aend[nt] = make_float2(s.x + sm.a0[c], s.y + sm.a0[c + 1]);
+    }
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+        float(&ck)[1][2][4] = *reinterpret_cast<float(*)[1][2][4]>(&dk[mt]);
+        float(&cr)[1][2][4] = *reinterpret_cast<float(*)[1][2][4]>(&dr[mt]);
+#pragma unroll
+        for (int kt = 0; kt < 2; ++kt) {
+            uint32_t a[1][3][4], b[3][4];
+            if (kt >= mt) {
+                matrix_frag<false>(a[0], sm.Gm, 16 * mt, 16 * kt, lane);
+                ldsm_t<3>(b, smem_addr(sm.o.R) + frag_rows(16 * kt, 2 * warp, lane));
+                mma_split<1, 3, 3>(ck, a, b);
+            }
+            if (kt <= mt) {
+                matrix_frag<true>(a[0], sm.Gm, 16 * mt, 16 * kt, lane);
+                ldsm_t<3>(b, smem_addr(sm.o.K) + frag_rows(16 * kt, 2 * warp, lane));
+                mma_split<1, 3, 3>(cr, a, b);
+            }
+        }
+    }
+    // per token and key: scales and bonus terms, then the decay gradient
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+        const int c = 16 * warp + 8 * nt + 2 * q;
+        const float2 u = decode(read_pair(u_ + h * kN + c, vec_ok(u_, 2)));
+        float2 x[4], Q[4], gu = make_float2(0.f, 0.f);   // x = Q - P
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int mt = b >> 1, e = b & 1, t = 8 * b + g;
+            const float2 r = decode(rp[mt][e][nt]), k = decode(kp[mt][e][nt]);
+            const float2 l0 = *reinterpret_cast<const float2*>(sm.rows + t * kN + c), l1 = *reinterpret_cast<const float2*>(sm.rows + (t + 1) * kN + c);
+            float &k0 = dk[mt][nt][2 * e], &k1 = dk[mt][nt][2 * e + 1], &r0 = dr[mt][nt][2 * e], &r1 = dr[mt][nt][2 * e + 1];
+            k0 *= ex2(-l1.x); k1 *= ex2(-l1.y); r0 *= ex2(l0.x); r1 *= ex2(l0.y);
+            Q[b] = make_float2(k.x * k0, k.y * k1);
+            x[b] = make_float2(fmaf(-r.x, r0, Q[b].x), fmaf(-r.y, r1, Q[b].y));
+            const float gm = sm.gamma[t];
+            gu.x = fmaf(gm, r.x * k.x, gu.x); gu.y = fmaf(gm, r.y * k.y, gu.y);
+            k0 = fmaf(gm * u.x, r.x, k0); k1 = fmaf(gm * u.y, r.y, k1);
+            r0 = fmaf(gm * u.x, k.x, r0); r1 = fmaf(gm * u.y, k.y, r1);
+        }
+        float2 after = make_float2(0.f, 0.f), gw = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int b = 3; b >= 0; --b) {   // sums over the tokens behind: over lanes inside eight tokens, then over the eights
+            float2 s = x[b];
+#pragma unroll
+            for (int m = 1; m < 8; m <<= 1) {
+                const float2 o = make_float2(__shfl_down_sync(0xffffffffu, s.x, 4 * m), __shfl_down_sync(0xffffffffu, s.y, 4 * m));
+                if (g + m < 8) { s.x += o.x; s.y += o.y; }
+            }
+            const float2 d = make_float2(aend[nt].x - (after.x + (s.x - x[b].x)) - Q[b].x, aend[nt].y - (after.y + (s.y - x[b].y)) - Q[b].y);
+            after.x += __shfl_sync(0xffffffffu, s.x, q);
+            after.y += __shfl_sync(0xffffffffu, s.y, q);
+            if (STATIC) { if (8 * b + g < n) { gw.x += d.x; gw.y += d.y; } }
+            else x[b] = d;
+        }
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) {
+            gu.x += __shfl_xor_sync(0xffffffffu, gu.x, m);
+            gu.y += __shfl_xor_sync(0xffffffffu, gu.y, m);
+            if (STATIC) { gw.x += __shfl_xor_sync(0xffffffffu, gw.x, m); gw.y += __shfl_xor_sync(0xffffffffu, gw.y, m); }
+        }
+        if (g == 0) {
+            float* p = partial_ + (unit / H * nseg + seg) * (STATIC ? 2 : 1) * C + h * kN + c;
+            if (STATIC) {
+                const float2 w = decode(read_pair(w_ + h * kN + c, vec_ok(w_, 2)));
+                p[0] = -expf(w.x) * gw.x; p[1] = -expf(w.y) * gw.y;   // d log d / d w_raw = log d
+                p += C;
+            }
+            p[0] = gu.x; p[1] = gu.y;
+        }
+        if (!STATIC) {
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int t = 8 * b + g;
+                const float2 w = t < n ? decode(read_pair(w_ + base + (i64)t * C + c, vec_ok(w_, 2))) : make_float2(0.f, 0.f);
+                // kept where Q and P of the tile were: dk and dr leave below with both tiles
+                x[b].x *= -ex2(kLog2e * w.x); x[b].y *= -ex2(kLog2e * w.y);
+                if (t < n) {
+                    E* p = gw_ + base + (i64)t * C + c;
+                    if (sizeof(E) == 2 && vec) *reinterpret_cast<uint32_t*>(p) = pack_bf16(x[b].x, x[b].y);
+                    else { p[0] = from_f<E>(x[b].x); p[1] = from_f<E>(x[b].y); }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int t = 16 * mt + g + 8 * e;
+            const i64 o = base + (i64)t * C + 16 * warp;
+            store_row<E>(gk_ + o, dk[mt][0][2 * e], dk[mt][0][2 * e + 1], dk[mt][1][2 * e], dk[mt][1][2 * e + 1], lane, vec, t < n);
+            store_row<E>(gr_ + o, dr[mt][0][2 * e], dr[mt][0][2 * e + 1], dr[mt][1][2 * e], dr[mt][1][2 * e + 1], lane, vec, t < n);
+        }
+}
+
+// States at the start of every segment (REV: adjoints at the end), one block per unit walking its segments: S <- S diag(f) + k'^T V
+// with k'_s = k_s exp(L_end - L_s) (REV: r'_t = r_t exp(L_{t-1}), gy): all factors are at most 1.  Warps 0 to 3 have the state in
+// registers, 16 keys each, warps 4 to 7 make the operands of the segments to come.
+template <typename E>
+struct ChainSmem {
+    unsigned char A[3 * kImg], B[kParts<E> * kImg];
+    float f[kN], tot[4 * kN];
+};
+template <int ID>
+__device__ __forceinline__ void bar_join(int odd) {
+    if (odd) asm volatile("bar.sync %0, 256;" ::"n"(ID + 1) : "memory");
+    else asm volatile("bar.sync %0, 256;" ::"n"(ID) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ void bar_tell(int odd) {
+    if (odd) asm volatile("bar.arrive %0, 256;" ::"n"(ID + 1) : "memory");
+    else asm volatile("bar.arrive %0, 256;" ::"n"(ID) : "memory");
+}
+template <typename E, bool STATIC, bool REV>
+__global__ void __launch_bounds__(256, 2) seg_mma_chain_kernel(int T, int H, int nseg, const E* __restrict__ a_, const E* __restrict__ b_,
+                                                               const E* __restrict__ w_, float* __restrict__ states) {
+    extern __shared__ __align__(128) unsigned char smem_seg_c[];
+    ChainSmem<E>* buf = reinterpret_cast<ChainSmem<E>*>(smem_seg_c);
+    constexpr int NV = kParts<E>;
+    const i64 unit = blockIdx.x;
+    const int h = unit % H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = H * kN;
+    const i64 base = unit / H * T * C + h * kN;
+    if (warp >= 4) {
+        // ---- operands: channels 2 lane, 2 lane + 1 of eight tokens ----------------------------------------------------------
+        const int p = warp - 4, t0 = 8 * p, c = 2 * lane, tid = threadIdx.x - 128;
+        const bool vec = vec_ok(a_, 2) && vec_ok(w_, 2), wide = sizeof(E) == 2 && vec_ok(b_, 8), vecb = vec_ok(b_, 2);
+        Pair<E> aa[8], ww[STATIC ? 1 : 8], bb[8];
+        uint4 bw[2];
+        auto fetch = [&](int it) {
+            const int seg = REV ? nseg - 1 - it : it, n = min(kSeg, T - seg * kSeg);
+            const i64 o = base + (i64)seg * kSeg * C;
+            read_rows<E>(aa, a_ + o + c, t0, n, C, vec);
+            if constexpr (!STATIC) read_rows<E>(ww, w_ + o + c, t0, n, C, vec);
+            if (wide) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int row = 16 * i + (tid >> 3);
+                    bw[i] = row < n ? __ldg(reinterpret_cast<const uint4*>(b_ + o + (i64)row * C + 8 * (tid & 7))) : make_uint4(0u, 0u, 0u, 0u);
+                }
+            } else read_rows<E>(bb, b_ + o + c, t0, n, C, vecb);
+        };
+        if constexpr (STATIC) ww[0] = read_pair(w_ + h * kN + c, vec);
+        if (nseg > 1) fetch(0);
+        for (int it = 0; it + 1 < nseg; ++it) {
+            const int seg = REV ? nseg - 1 - it : it, n = min(kSeg, T - seg * kSeg);
+            ChainSmem<E>& sm = buf[it & 1];
+            if (it >= 2) bar_join<3>(it & 1);
+            float2 d[STATIC ? 1 : 8], before, after;   // sums of log2 decays before and behind these tokens
+            if constexpr (STATIC) d[0] = log2_decay_static(decode(ww[0]));
+            else {
+                float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    d[i] = t0 + i < n ? log2_decay(decode(ww[i])) : make_float2(0.f, 0.f);
+                    s.x += d[i].x; s.y += d[i].y;
+                }
+                *reinterpret_cast<float2*>(sm.tot + p * kN + c) = s;
+                asm volatile("bar.sync 5, 128;" ::: "memory");
+                before = after = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 t = *reinterpret_cast<const float2*>(sm.tot + i * kN + c);
+                    if (i < p) { before.x += t.x; before.y += t.y; }
+                    if (i > p) { after.x += t.x; after.y += t.y; }
+                }
+                if (p == 0) *reinterpret_cast<float2*>(sm.f + c) = make_float2(ex2(s.x + after.x), ex2(s.y + after.y));
+            }
+            if (STATIC && p == 0) *reinterpret_cast<float2*>(sm.f + c) = make_float2(ex2(d[0].x * n), ex2(d[0].y * n));
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int i = REV ? j : 7 - j;   // towards the end that the products count from, starting there
+                const float2 a = decode(aa[i]);
+                float2 e;
+                if constexpr (STATIC) {
+                    const float x = (float)(REV ? t0 + i : max(n - 1 - (t0 + i), 0));
+                    e = make_float2(d[0].x * x, d[0].y * x);
+                } else {
+                    float2& s = REV ? before : after;
+                    e = s;
+                    s.x += d[i].x; s.y += d[i].y;
+                }
+                put_split(sm.A, t0 + i, lane, a.x * ex2(e.x), a.y * ex2(e.y));
+            }
+            if (wide) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(sm.B + img_at(16 * i + (tid >> 3), tid & 7)) = bw[i];
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) put_pair<E>(sm.B, t0 + i, lane, bb[i]);
+            }
+            if (it + 2 < nseg) fetch(it + 1);
+            bar_tell<1>(it & 1);
+        }
+        return;
+    }
+    // ---- the state: keys 16 warp + g, + 8 of all values -----------------------------------------------------------------------
+    const int g = lane >> 2, q = lane & 3;
+    float s[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[i][e] = 0.f;
+    for (int it = 0; it < nseg; ++it) {
+        float* p = states + (unit * nseg + (REV ? nseg - 1 - it : it)) * kN * kN + (16 * warp + g) * kN + 2 * q;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) *reinterpret_cast<float2*>(p + 8 * e * kN + 8 * i) = make_float2(s[i][2 * e], s[i][2 * e + 1]);
+        if (it + 1 == nseg) break;
+        bar_join<1>(it & 1);
+        const ChainSmem<E>& sm = buf[it & 1];
+        const float f0 = sm.f[16 * warp + g], f1 = sm.f[16 * warp + g + 8];
+        uint32_t a[2][1][3][4];
+#pragma unroll
+        for (int kt = 0; kt < 2; ++kt) ldsm_t<3>(a[kt][0], smem_addr(sm.A) + frag_cols(16 * kt, 2 * warp, lane));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float c[1][2][4];   // (summed apart from the state: the tensor core's sums are not rounded to nearest)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) c[0][0][e] = c[0][1][e] = 0.f;
+#pragma unroll
+            for (int kt = 0; kt < 2; ++kt) {
+                uint32_t b[NV][4];
+                ldsm_t<NV>(b, smem_addr(sm.B) + frag_rows(16 * kt, 2 * i, lane));
+                mma_split<1, 3, NV>(c, a[kt], b);
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[2 * i + j][e] = fmaf(s[2 * i + j][e], e < 2 ? f0 : f1, c[0][j][e]);
+        }
+        if (it + 3 < nseg) bar_tell<3>(it & 1);
+    }
+}
+
+// ---- the segments that the kernels above have left ----------------------------------------------------------------------------
+// Block b looks at the segments b, b + grid, ..: with none flagged that is one read per thread.
+template <typename F>
+__device__ __forceinline__ void for_flagged(const int* __restrict__ flags, i64 total, F body) {
+    for (i64 first = blockIdx.x; first < total; first += (i64)gridDim.x * blockDim.x) {
+        const i64 mine = first + (i64)threadIdx.x * gridDim.x;
+        if (!__syncthreads_or(mine < total && flags[mine])) continue;
+        for (int i = 0; i < (int)blockDim.x; ++i) {
+            const i64 block = first + (i64)i * gridDim.x;
+            if (block < total && flags[block]) {
+                body(block);
+                __syncthreads();
+            }
+        }
+    }
+}
+inline unsigned flagged_blocks(i64 total, int per_sm) {   // as many as are resident together
+    const i64 most = (i64)(sm_count() > 0 ? sm_count() : 148) * per_sm;
+    return (unsigned)(total < most ? total : most);
+}
+
+// ---- launches ----------------------------------------------------------------------------------------------------------------
+// One block per unit walks all segments, or (the other kernels) every segment on its own and a scan: with few units the walk is
+// as long as T, and the scan's passes over the states cost little.
+inline bool seg_chain_pays(i64 units) { return units * 2 > sm_count(); }
+
+template <typename E, bool STATIC, bool REV>
+int seg_chain(i64 units, int T, int H, int nseg, const void* a, const void* b, const void* w, float* states, cudaStream_t st) {
+    constexpr int smem = 2 * sizeof(ChainSmem<E>);
+    const cudaError_t e = allow_smem<seg_mma_chain_kernel<E, STATIC, REV>>(smem);
+    RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    seg_mma_chain_kernel<E, STATIC, REV><<<(unsigned)units, 256, smem, st>>>(T, H, nseg, (const E*)a, (const E*)b, (const E*)w, states);
+    return check_launch("training on segments: states");
+}
+template <typename E, bool STATIC>
+int seg_mma_y(i64 total, int T, int H, int nseg, const void* r, const void* k, const void* v, const void* w, const void* u, const float* states,
+              void* y, int* flags, cudaStream_t st) {
+    constexpr int smem = sizeof(YSmem<E>);
+    const cudaError_t e = allow_smem<seg_mma_y_kernel<E, STATIC>>(smem);
+    RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    seg_mma_y_kernel<E, STATIC><<<(unsigned)total, 128, smem, st>>>(T, H, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states,
+                                                                   (E*)y, flags);
+    return check_launch("training on segments: y");
+}
+template <typename E, bool STATIC>
+int seg_mma_backward(i64 total, int T, int H, int nseg, const void* r, const void* k, const void* v, const void* w, const void* u, const void* gy,
+                     const float* S, const float* D, void* gr, void* gk, void* gv, void* gw, float* partial, int* flags, cudaStream_t st) {
+    constexpr int smem = sizeof(BwdSmemM<E>);
+    const cudaError_t e = allow_smem<seg_mma_backward_kernel<E, STATIC>>(smem);
+    RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    seg_mma_backward_kernel<E, STATIC><<<(unsigned)total, 128, smem, st>>>(T, H, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u,
+                                                                          (const E*)gy, S, D, (E*)gr, (E*)gk, (E*)gv, (E*)gw, partial, flags);
+    return check_launch("training on segments: gradients");
+}
+
+}  // namespace
+}  // namespace rwkvb200

@@ -595,7 +595,7 @@ extern "C" int rwkvb200_wkv6_train_forward(int dtype, int B, int T, int C, int H
 
 extern "C" size_t rwkvb200_wkv6_train_work_bytes(int B, int T, int C, int path) {
     if (B <= 0 || T <= 0 || C <= 0) return 0;
-    if (path == 2) return (wkv6_seg_adjoints(B, T, C) + wkv6_seg_rows(B, T) * C) * sizeof(float);
+    if (path == 2) return (wkv6_seg_adjoints(B, T, C) + wkv6_seg_rows(B, T) * C + wkv6_seg_flags(B, T, C)) * sizeof(float);
     return (size_t)B * C * sizeof(float) + (path == 0 ? (size_t)B * T * C * sizeof(float) : rwkvb200_wkv6_scratch_bytes(B, T, C));
 }
 
@@ -609,7 +609,8 @@ extern "C" int rwkvb200_wkv6_train_backward(int dtype, int B, int T, int C, int 
     if (path == 2) {
         RWKV_REQUIRE(wkv6_seg_applies(dtype, T, C / H, s0 != nullptr || dsT != nullptr || ds0 != nullptr), RWKVB200_EINVAL, "wkv6_train_backward: not a call of path 2");
         float *adjoints = static_cast<float*>(work), *partial = adjoints + wkv6_seg_adjoints(B, T, C);
-        const int e = wkv6_seg_backward(B, T, H, r, k, v, w, u, gy, gr, gk, gv, gw, static_cast<const float*>(saved), adjoints, partial, st);
+        const int e = wkv6_seg_backward(B, T, H, r, k, v, w, u, gy, gr, gk, gv, gw, static_cast<const float*>(saved), adjoints, partial,
+                                        reinterpret_cast<int*>(partial + wkv6_seg_rows(B, T) * C), st);
         return e ? e : sum_rows(dtype, wkv6_seg_rows(B, T), C, partial, gu, st);
     }
     const int sk = s0 ? kF32 : kNone, dk = ds0 ? kF32 : kNone;

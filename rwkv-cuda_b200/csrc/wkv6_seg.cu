@@ -4,23 +4,23 @@
 // Per (batch, head), S indexed [key j][value i], d_t[j] = exp(-exp(w_t[j])) the decay of token t:
 //   y_t[i] = sum_j r_t[j] S_{t-1}[j,i] + v_t[i] sum_j r_t u k_t      S_t[j,i] = d_t[j] S_{t-1}[j,i] + k_t[j] v_t[i]
 // The steps are those of wkv5_seg.cu, with the products of the token decays in place of powers of one decay:
-//   local   the end state of every segment of 32 tokens from a zero start: sum_s (prod_{tau>s} d_tau) k_s v_s^T.  The products are
-//           put on k when it is staged; they are <= 1, so nothing can overflow, whatever the decays are;
-//   scan    start states of the segments, in place: S <- S diag(prod d) + local;
-//   y       every segment again, token by token from its start state.
-// Backward: the same two steps for the adjoint D = dL/dS (k, v -> r, gy, time reversed), then one block per segment: two warps
-// carry S forward (gr) while two carry D backward (gk, gv).  For the decay gradient they leave P_t = r_t sum_i gy_t S_{t-1} and
-// Q_t = k_t sum_i D_t v_t, and with A_t = sum_i D_{t-1}[j,i] S_{t-1}[j,i] (D_t: before token t is taken in, S_t: after it)
+//   states  at the start of every segment of 32 tokens (backward: the adjoint D = dL/dS behind it; k, v -> r, gy, time reversed):
+//           with many units by a walk along the segments (seg_mma_chain_kernel), with few by local end states from a zero start,
+//           sum_s (prod_{tau>s} d_tau) k_s v_s^T, and a scan over them in place, S <- S diag(prod d) + local.  The products of
+//           decays that are put on k are <= 1: nothing can overflow, whatever the decays are;
+//   y, gradients  of every segment at the same time from its states, by the products of seg_mma.cuh.  Segments that these leave
+//           (decays out of range, values that are not finite) are walked token by token by the kernels here: two warps carry S
+//           forward (gr) while two carry D backward (gk, gv).  For the decay gradient they leave P_t = r_t sum_i gy_t S_{t-1} and
+//           Q_t = k_t sum_i D_t v_t, and with A_t = sum_i D_{t-1}[j,i] S_{t-1}[j,i] (D_t: before token t is taken in, S_t: after it)
 //   dL/dlog d_t = A_{t+1} - Q_t       A_t = A_{t+1} - Q_t + P_t       (wkv6.cu)
 // walked over the segment's tokens only: A at its end is taken from the two states there.
 //
-// What bounds it: multiply-adds of the FP32 pipe, one per state element, token and product (9 of them forward + backward), and
-// the shared-memory reads of the token's vectors.  B8 T1000 H32, forward + backward on a B200: 4374 us on the general-shape
-// kernels, which walk the tokens with one block per unit; 1237 us here.  The tensor-core kernels take 258 us, but their operands
-// are TF32: outputs are then 2 to 4 % further from fp64 in norm than one rounding to bf16 (1.72e-3 instead of 1.66e-3; here
-// 1.66e-3), and gw 1.3e-2 instead of 3.9e-3 at its worst element.
+// B8 T1000 H32, forward + backward on a B200: 4374 us on the general-shape kernels, which walk the tokens with one block per unit;
+// 1237 us with the token-by-token kernels on all segments (multiply-adds at 46 % of the issue slots and the shared-memory reads of
+// the tokens' vectors); 606 us with products.  Errors against fp64 are the same to four digits (1.66e-3: one rounding to bf16).
+// The kernels for whole 32-token chunks take 258 us, but their operands are TF32: outputs are then 2 to 4 % further from fp64.
 #include "wkv6_seg.cuh"
-#include "seg_tiles.cuh"
+#include "seg_mma.cuh"
 
 namespace rwkvb200 {
 namespace {
@@ -107,18 +107,18 @@ __global__ void __launch_bounds__(64) seg6_local_kernel(int T, int H, int nseg, 
     store_tile(s, states + (i64)blockIdx.x * kN * kN, 8 * kg, 8 * vg, kN);
 }
 
-// One block per (unit, segment), 2 warps: a warp has the values 32 warp .. of all keys
-__global__ void __launch_bounds__(64) seg6_y_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
+// The segments that seg_mma_y_kernel has left.  2 warps: a warp has the values 32 warp .. of all keys
+__device__ __forceinline__ void seg6_y_segment(i64 block, int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
                                                     const bf16* __restrict__ v_, const bf16* __restrict__ w_, const bf16* __restrict__ u_,
                                                     const float* __restrict__ states, bf16* __restrict__ y_) {
     __shared__ __align__(16) float rs[kSeg * kN], ks[kSeg * kN], vs[kSeg * kN], ds[kSeg * kN], us[kN], ruk[kSeg];
-    const i64 unit = blockIdx.x / nseg;
-    const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
+    const i64 unit = block / nseg;
+    const int seg = block % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
     const int kg = lane >> 2, vg = 4 * warp + (lane & 3);
     Tile s;
-    load_tile(s, states + (i64)blockIdx.x * kN * kN, 8 * kg, 8 * vg, kN);
+    load_tile(s, states + block * kN * kN, 8 * kg, 8 * vg, kN);
     stage<64>(rs, r_ + base, n, C, kN, tid);
     stage<64>(ks, k_ + base, n, C, kN, tid);
     stage<64>(vs, v_ + base, n, C, kN, tid);
@@ -154,7 +154,13 @@ __global__ void __launch_bounds__(64) seg6_y_kernel(int T, int H, int nseg, cons
     }
 }
 
-// One block per (unit, segment), 4 warps: warps 0, 1 carry S forward (gr, gu, P), warps 2, 3 carry D backward (gk, gv, Q); a warp
+__global__ void __launch_bounds__(64) seg6_y_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
+                                                    const bf16* __restrict__ v_, const bf16* __restrict__ w_, const bf16* __restrict__ u_,
+                                                    const float* __restrict__ states, bf16* __restrict__ y_, const int* __restrict__ flags, i64 total) {
+    for_flagged(flags, total, [&](i64 block) { seg6_y_segment(block, T, H, nseg, r_, k_, v_, w_, u_, states, y_); });
+}
+
+// The segments that seg_mma_backward_kernel has left.  4 warps: warps 0, 1 carry S forward (gr, gu, P), warps 2, 3 carry D backward (gk, gv, Q); a warp
 // has 32 keys of all values.  gv sums over all keys: the two halves meet in shared memory at the end.
 struct Bwd6Smem {
     float r[kSeg * kN], k[kSeg * kN], v[kSeg * kN], g[kSeg * kN], d[kSeg * kN], gv[2][kSeg * kN];
@@ -162,22 +168,21 @@ struct Bwd6Smem {
     float u[kN], vg[kSeg], ruk[kSeg];
 };
 
-__global__ void __launch_bounds__(128, 3) seg6_backward_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
-                                                               const bf16* __restrict__ v_, const bf16* __restrict__ w_,
-                                                               const bf16* __restrict__ u_, const bf16* __restrict__ gy_,
-                                                               const float* __restrict__ S_, const float* __restrict__ D_, bf16* __restrict__ gr_,
-                                                               bf16* __restrict__ gk_, bf16* __restrict__ gv_, bf16* __restrict__ gw_,
-                                                               float* __restrict__ gu_) {
+__device__ __forceinline__ void seg6_backward_segment(i64 block, int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
+                                                      const bf16* __restrict__ v_, const bf16* __restrict__ w_, const bf16* __restrict__ u_,
+                                                      const bf16* __restrict__ gy_, const float* __restrict__ S_, const float* __restrict__ D_,
+                                                      bf16* __restrict__ gr_, bf16* __restrict__ gk_, bf16* __restrict__ gv_, bf16* __restrict__ gw_,
+                                                      float* __restrict__ gu_) {
     extern __shared__ __align__(16) unsigned char smem_seg6[];
     Bwd6Smem& sm = *reinterpret_cast<Bwd6Smem*>(smem_seg6);
-    const i64 unit = blockIdx.x / nseg;
-    const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
+    const i64 unit = block / nseg;
+    const int seg = block % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
-    const float* D0 = D_ + (i64)blockIdx.x * kN * kN;
+    const float* D0 = D_ + block * kN * kN;
     const int kg = 4 * (warp & 1) + (lane & 3), vg = lane >> 2, j_out = 8 * kg + vg;   // j_out: the key whose sums this lane ends with
     Tile s;
-    load_tile(s, warp < 2 ? S_ + (i64)blockIdx.x * kN * kN : D0, 8 * kg, 8 * vg, kN);
+    load_tile(s, warp < 2 ? S_ + block * kN * kN : D0, 8 * kg, 8 * vg, kN);
     stage<128>(sm.r, r_ + base, n, C, kN, tid);
     stage<128>(sm.k, k_ + base, n, C, kN, tid);
     stage<128>(sm.v, v_ + base, n, C, kN, tid);
@@ -277,33 +282,53 @@ __global__ void __launch_bounds__(128, 3) seg6_backward_kernel(int T, int H, int
     }
 }
 
+__global__ void __launch_bounds__(128, 3) seg6_backward_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
+                                                               const bf16* __restrict__ v_, const bf16* __restrict__ w_,
+                                                               const bf16* __restrict__ u_, const bf16* __restrict__ gy_,
+                                                               const float* __restrict__ S_, const float* __restrict__ D_, bf16* __restrict__ gr_,
+                                                               bf16* __restrict__ gk_, bf16* __restrict__ gv_, bf16* __restrict__ gw_,
+                                                               float* __restrict__ gu_, const int* __restrict__ flags, i64 total) {
+    for_flagged(flags, total, [&](i64 block) { seg6_backward_segment(block, T, H, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, gw_, gu_); });
+}
+
 }  // namespace
 
 int wkv6_seg_forward(int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u, void* y, float* saved,
                      cudaStream_t st) {
     const int nseg = (T + kSeg - 1) / kSeg;
-    const i64 units = (i64)B * H;
-    RWKV_REQUIRE(units * nseg < (1ll << 31), RWKVB200_EINVAL, "wkv6_train_forward: too many segments");
-    float* decays = saved + units * nseg * kN * kN;
-    const unsigned grid = (unsigned)(units * nseg), scan = (unsigned)(units * (kN * kN / 256));
-    seg6_local_kernel<false><<<grid, 64, 0, st>>>(T, H, nseg, (const bf16*)k, (const bf16*)v, (const bf16*)w, saved, decays);
-    seg6_scan_kernel<false><<<scan, 256, 0, st>>>(nseg, decays, saved);
-    seg6_y_kernel<<<grid, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, saved, (bf16*)y);
+    const i64 units = (i64)B * H, total = units * nseg;
+    RWKV_REQUIRE(total < (1ll << 31), RWKVB200_EINVAL, "wkv6_train_forward: too many segments");
+    float* decays = saved + total * kN * kN;
+    int* flags = reinterpret_cast<int*>(decays + total * kN);
+    if (seg_chain_pays(units)) {
+        if (const int e = seg_chain<bf16, false, false>(units, T, H, nseg, k, v, w, saved, st)) return e;
+    } else {
+        seg6_local_kernel<false><<<(unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)k, (const bf16*)v, (const bf16*)w, saved, decays);
+        seg6_scan_kernel<false><<<(unsigned)(units * (kN * kN / 256)), 256, 0, st>>>(nseg, decays, saved);
+    }
+    if (const int e = seg_mma_y<bf16, false>(total, T, H, nseg, r, k, v, w, u, saved, y, flags, st)) return e;
+    seg6_y_kernel<<<flagged_blocks(total, 8), 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, saved,
+                                                           (bf16*)y, flags, total);
     return check_launch("wkv6_train_forward(segments)");
 }
 
 int wkv6_seg_backward(int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u, const void* gy, void* gr,
-                      void* gk, void* gv, void* gw, const float* saved, float* adjoints, float* gu_partial, cudaStream_t st) {
+                      void* gk, void* gv, void* gw, const float* saved, float* adjoints, float* gu_partial, int* flags, cudaStream_t st) {
     const int nseg = (T + kSeg - 1) / kSeg;
-    const i64 units = (i64)B * H;
-    const float* decays = saved + units * nseg * kN * kN;
-    const unsigned grid = (unsigned)(units * nseg), scan = (unsigned)(units * (kN * kN / 256));
+    const i64 units = (i64)B * H, total = units * nseg;
+    const float* decays = saved + total * kN * kN;
     const cudaError_t e = allow_smem<seg6_backward_kernel>(sizeof(Bwd6Smem));
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv6_train_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    seg6_local_kernel<true><<<grid, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)gy, (const bf16*)w, adjoints, nullptr);
-    seg6_scan_kernel<true><<<scan, 256, 0, st>>>(nseg, decays, adjoints);
-    seg6_backward_kernel<<<grid, 128, sizeof(Bwd6Smem), st>>>(T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u,
-                                                              (const bf16*)gy, saved, adjoints, (bf16*)gr, (bf16*)gk, (bf16*)gv, (bf16*)gw, gu_partial);
+    if (seg_chain_pays(units)) {
+        if (const int e = seg_chain<bf16, false, true>(units, T, H, nseg, r, gy, w, adjoints, st)) return e;
+    } else {
+        seg6_local_kernel<true><<<(unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)gy, (const bf16*)w, adjoints, nullptr);
+        seg6_scan_kernel<true><<<(unsigned)(units * (kN * kN / 256)), 256, 0, st>>>(nseg, decays, adjoints);
+    }
+    if (const int e = seg_mma_backward<bf16, false>(total, T, H, nseg, r, k, v, w, u, gy, saved, adjoints, gr, gk, gv, gw, gu_partial, flags, st)) return e;
+    seg6_backward_kernel<<<flagged_blocks(total, 3), 128, sizeof(Bwd6Smem), st>>>(
+        T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, (const bf16*)gy, saved, adjoints, (bf16*)gr, (bf16*)gk,
+        (bf16*)gv, (bf16*)gw, gu_partial, flags, total);
     return check_launch("wkv6_train_backward(segments)");
 }
 

@@ -89,3 +89,46 @@ def test_rwkv6_forward_scales_its_state(shift, T):
     R.ops.wkv6state_forward_ex(B, T, C, H, *d, s0.to("cuda"), y, sT)
     Hh.assert_close(y, yo, Hh.TOL_BF16, "y")
     Hh.assert_close(sT, sTo, Hh.TOL_BF16, "sT")
+
+
+@pytest.mark.parametrize("B,T,H", [(1, 71, 2), (2, 333, 40)])   # states by a scan over the segments, and by a walk along them
+def test_rwkv6_segments_of_both_kinds(B, T, H):
+    """Segments with decays too strong for the matrix form (or for its anchor in the middle) beside others, every tensor one element off
+    its alignment: bounds as above."""
+    import rwkv_cuda_b200 as R
+    g = Hh.gen(T)
+    N, C = 64, H * 64
+    r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
+    u, gy, w = Hh.rand(g, H, N, lo=-1, hi=1), Hh.randn(g, B, T, C), Hh.randn(g, B, T, C) - 4.0
+    w[:, 40, 3] = 6.0             # one token of a segment, one channel
+    w[:, 64:, 2 * 64 - 1] = 1.5   # exp(1.5) * 16 > 60: from the third segment on
+    odd = lambda x: torch.cat([x.new_zeros(1), x.flatten()]).to(BF).cuda()[1:].view(x.shape)
+    xs = [odd(x).requires_grad_(True) for x in (r, k, v, w, u)]
+    y = R.functions.WKV_6.apply(B, T, C, H, *xs)
+    got = [y, *torch.autograd.grad(y, xs, odd(gy))]
+    xo = [x.to(BF).double().requires_grad_(True) for x in (r, k, v, w, u)]
+    yo = O.wkv6(*xo, H)
+    want = [yo, *torch.autograd.grad(yo, xo, gy.to(BF).double())]
+    for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
+        size = torch.maximum(b.abs(), b.square().mean().sqrt())
+        err = ((a.double().cpu().reshape(b.shape) - b).abs() / size).max().item()
+        assert err <= 2 ** -8 + 2 ** -15, f"{name}: {err:.3e}"
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("name", ["v", "k", "r"])
+def test_rwkv6_values_that_are_not_finite_stay_behind(name, value):
+    """Tokens before such a value are those of the call without it, inside its segment too."""
+    import rwkv_cuda_b200 as R
+    B, T, H, N, t = 1, 71, 1, 64, 45
+    g = Hh.gen(5)
+    C = H * N
+    x = {n: 0.5 * Hh.randn(g, B, T, C) for n in ("r", "k", "v")}
+    w, u = Hh.randn(g, B, T, C) - 4.0, Hh.rand(g, H, N, lo=-1, hi=1)
+    call = lambda: R.functions.WKV_6.apply(B, T, C, H, *(a.to(BF).cuda() for a in (x["r"], x["k"], x["v"], w, u)))
+    clean = call()
+    x[name][:, t, 7] = value
+    y = call()
+    size = clean.float().square().mean().sqrt()
+    assert ((y[:, :t].float() - clean[:, :t].float()).abs() / size).max().item() < 2 ** -6   # (other kernel: other rounding, in bf16)
+    assert not torch.isfinite(y[:, t]).all()
