@@ -18,7 +18,10 @@
 // Why mma.sync and not tcgen05: these kernels are a block per segment with every accumulator and both states in registers,
 // four blocks per SM; the operands are split where they are used, and at 8 clocks per instruction and scheduler the tensor pipe
 // needs about as long as the arithmetic around it.
-// A segment whose decays leave the range (more than 2^-kRange between its middle and an end) or that holds values that are not
+// B8 T1000 H32 bf16, backward kernel 285 us (314 with the rows of exponents 64 floats apart, the token matrices as fp32, a test of the
+// alignment per load and bf16 parts unpacked before they are subtracted), y 111 us; 4300 -> 3900 instructions a warp and 324 mma: issue slots
+// and the latency of 16 warps per SM (128 registers a thread) bound it, the tensor pipe is busy 27 % of the time.
+// A segment whose decays leave the range (more than kRange between its middle and an end) or that holds values that are not
 // finite (a masked product would spread them over tokens before) is flagged and left to the token-by-token kernels.
 #pragma once
 #include "seg_tiles.cuh"
@@ -26,10 +29,14 @@
 namespace rwkvb200 {
 namespace {
 
-constexpr float kRange = 86.f;                 // log2; 60 in nats
+// log2 of the largest decay between the middle of a segment and an end of it.  Per-token decays: 60 in nats.  A static decay: the
+// sum of its gradient over the tokens holds terms without a decay that cancel (T 47, factors up to 2.7 per token: error of gw 6.2e-7,
+// token by token 4.3e-7), so the limit is a factor of 2 per token.
+template <bool STATIC> constexpr float kRange = STATIC ? 16.f : 86.f;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kImg = kSeg * 128;               // bytes of one bf16 image [32 tokens][64 channels]
-constexpr int kMld = 40;                       // floats of a row of a token x token matrix: 8-byte fragment reads hit every bank once
+constexpr int kTiles = 3 * 512;                // bytes of one bf16 image of a triangular token x token matrix: its 16 x 16 tiles
+constexpr int kRld = 72;                       // floats of a row of 64 channels: 8-byte reads of eight rows hit every bank once
 
 // ---- bf16 images: rows of 128 bytes, their 16-byte pieces XOR-ed with the row ------------------------------------------------
 __device__ __forceinline__ uint32_t img_at(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
@@ -40,28 +47,38 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)
 __device__ __forceinline__ uint32_t frag_rows(int r0, int c0, int lane) { return img_at(r0 + (lane & 15), c0 + (lane >> 4)); }
 __device__ __forceinline__ uint32_t frag_cols(int r0, int c0, int lane) { return img_at(r0 + (lane & 7) + ((lane >> 4) << 3), c0 + ((lane >> 3) & 1)); }
 __device__ __forceinline__ void ldsm(uint32_t (&f)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(addr) : "memory");
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(addr));
 }
 __device__ __forceinline__ void ldsm_t(uint32_t (&f)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(addr) : "memory");
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(f[0]), "=r"(f[1]), "=r"(f[2]), "=r"(f[3]) : "r"(addr));
 }
-template <int NS>
+template <int NS, int STEP = kImg>
 __device__ __forceinline__ void ldsm(uint32_t (&f)[NS][4], uint32_t addr) {
 #pragma unroll
-    for (int s = 0; s < NS; ++s) ldsm(f[s], addr + s * kImg);
+    for (int s = 0; s < NS; ++s) ldsm(f[s], addr + s * STEP);
 }
-template <int NS>
+template <int NS, int STEP = kImg>
 __device__ __forceinline__ void ldsm_t(uint32_t (&f)[NS][4], uint32_t addr) {
 #pragma unroll
-    for (int s = 0; s < NS; ++s) ldsm_t(f[s], addr + s * kImg);
+    for (int s = 0; s < NS; ++s) ldsm_t(f[s], addr + s * STEP);
 }
 __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// c[mt][nt] += a[mt] b[nt], split operands: the small partial products first
-template <int MT, int NA, int NB>
+// c[mt][nt] += a[mt] b[nt], split operands: the small partial products first.  APART: summed from zero and then added, because the
+// tensor core's sums are not rounded to nearest (RWKV-5 fp32 B2 T333: error of y 5.9e-7 -> 1.6e-7
+// of the norm, 4.4e-7 token by token; bf16 results show no difference)
+template <bool APART, int MT, int NA, int NB>
 __device__ __forceinline__ void mma_split(float (&c)[MT][2][4], const uint32_t (&a)[MT][NA][4], const uint32_t (&b)[NB][4]) {
+    float x[MT][2][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            x[mt][0][e] = APART ? 0.f : c[mt][0][e];
+            x[mt][1][e] = APART ? 0.f : c[mt][1][e];
+        }
 #pragma unroll
     for (int order = (NA > 1 ? 2 : 0) + (NB > 1 ? 2 : 0); order >= 0; --order) {
         if (order > 2) continue;
@@ -71,11 +88,18 @@ __device__ __forceinline__ void mma_split(float (&c)[MT][2][4], const uint32_t (
             if (pb < 0 || pb >= NB) continue;
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
-                mma(c[mt][0], a[mt][pa], b[pb][0], b[pb][1]);
-                mma(c[mt][1], a[mt][pa], b[pb][2], b[pb][3]);
+                mma(x[mt][0], a[mt][pa], b[pb][0], b[pb][1]);
+                mma(x[mt][1], a[mt][pa], b[pb][2], b[pb][3]);
             }
         }
     }
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            c[mt][0][e] = APART ? c[mt][0][e] + x[mt][0][e] : x[mt][0][e];
+            c[mt][1][e] = APART ? c[mt][1][e] + x[mt][1][e] : x[mt][1][e];
+        }
 }
 // x = sum of three bf16 numbers, two values at a time (the first in the low half)
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -85,17 +109,25 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 __device__ __forceinline__ float bf16_lo(uint32_t x) { return __uint_as_float(x << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t x) { return __uint_as_float(x & 0xffff0000u); }
+// x - h with h as a bf16 operand of the multiply-add (exact; 14.7 clocks per split3 and scheduler, 19.1 with h unpacked first)
+__device__ __forceinline__ void less_bf16(float& x0, float& x1, uint32_t h) {
+    asm("{.reg .b16 a, b, c; mov.b32 {a, b}, %2; mov.b16 c, 0xBF80; fma.rn.f32.bf16 %0, a, c, %0; fma.rn.f32.bf16 %1, b, c, %1;}" : "+f"(x0), "+f"(x1) : "r"(h));
+}
 __device__ __forceinline__ void split3(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
     h = pack_bf16(x0, x1);
-    x0 -= bf16_lo(h); x1 -= bf16_hi(h);
+    less_bf16(x0, x1, h);
     m = pack_bf16(x0, x1);
-    x0 -= bf16_lo(m); x1 -= bf16_hi(m);
+    less_bf16(x0, x1, m);
     l = pack_bf16(x0, x1);
 }
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) {   // the line that holds *p
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p) & ~(size_t)127));
 }
 
 // ---- two neighbouring channels of a token, as loaded and decoded --------------------------------------------------------------
@@ -117,11 +149,29 @@ template <typename E> __device__ __forceinline__ Pair<E> no_pair();
 template <> __device__ __forceinline__ uint32_t no_pair<bf16>() { return 0u; }
 template <> __device__ __forceinline__ float2 no_pair<float>() { return make_float2(0.f, 0.f); }
 template <typename E> __device__ __forceinline__ bool vec_ok(const E* p, int elements) { return (reinterpret_cast<uintptr_t>(p) & (elements * sizeof(E) - 1)) == 0; }
-// rows t0 .. t0 + 7 of two channels
-template <typename E>
-__device__ __forceinline__ void read_rows(Pair<E> (&x)[8], const E* p, int t0, int n, int C, bool vec) {
+// rows t0 .. t0 + R - 1 of two channels (one test of the alignment for all of them)
+template <typename E, int R>
+__device__ __forceinline__ void read_rows(Pair<E> (&x)[R], const E* p, int t0, int n, int C, bool vec) {
+    p += (i64)t0 * C;
+    if (vec) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = t0 + i < n ? read_pair(p + (i64)(t0 + i) * C, vec) : no_pair<E>();
+        for (int i = 0; i < R; ++i) x[i] = t0 + i < n ? read_pair(p + i * C, true) : no_pair<E>();
+    } else {
+#pragma unroll
+        for (int i = 0; i < R; ++i) x[i] = t0 + i < n ? read_pair(p + i * C, false) : no_pair<E>();
+    }
+}
+// rows g, g + 8, g + 16, g + 24 of two channels
+template <typename E>
+__device__ __forceinline__ void read_eights(Pair<E> (&x)[4], const E* p, int g, int n, int C, bool vec) {
+    p += (i64)g * C;
+    if (vec) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) x[b] = g + 8 * b < n ? read_pair(p + 8 * b * C, true) : no_pair<E>();
+    } else {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) x[b] = g + 8 * b < n ? read_pair(p + 8 * b * C, false) : no_pair<E>();
+    }
 }
 
 // images of a tensor as it came: bf16 one image, fp32 three
@@ -163,9 +213,9 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
     const int lane = tid & 31, q = tid >> 5, c = 2 * lane, t0 = 8 * q;
     Pair<E> rr[8], kk[8], ww[STATIC ? 1 : 8];
     const bool vec = vec_ok(r_, 2) && vec_ok(k_, 2) && vec_ok(w_, 2);
-    read_rows<E>(rr, r_ + c, t0, n, C, vec);
-    read_rows<E>(kk, k_ + c, t0, n, C, vec);
-    if constexpr (!STATIC) read_rows<E>(ww, w_ + c, t0, n, C, vec);
+    read_rows<E, 8>(rr, r_ + c, t0, n, C, vec);
+    read_rows<E, 8>(kk, k_ + c, t0, n, C, vec);
+    if constexpr (!STATIC) read_rows<E, 8>(ww, w_ + c, t0, n, C, vec);
     else ww[0] = read_pair(w_ + c, vec);
     const float2 u = decode(read_pair(u_ + c, vec_ok(u_, 2)));
     float2 d[STATIC ? 1 : 8], pre, lm, le;   // log2 decays; L before the first of these tokens, L at the middle, L from there to the end
@@ -202,14 +252,14 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
             a = pre;
             b = pre = make_float2(pre.x + d[i].x, pre.y + d[i].y);
         }
-        if (ROWS) *reinterpret_cast<float2*>(rows + (t0 + i) * kN + c) = a;
+        if (ROWS) *reinterpret_cast<float2*>(rows + (t0 + i) * kRld + c) = a;
         const float2 r = decode(rr[i]), k = decode(kk[i]);
         const float2 rs = make_float2(r.x * ex2(a.x), r.y * ex2(a.y)), ks = make_float2(k.x * ex2(-b.x), k.y * ex2(-b.y));
         check(bad, rs); check(bad, ks);
         put_split(o.R, t0 + i, lane, rs.x, rs.y);
         put_split(o.K, t0 + i, lane, ks.x, ks.y);
         x[i] = fmaf(r.x * u.x, k.x, r.y * u.y * k.y);
-        if (ROWS && q == 3 && i == 7) *reinterpret_cast<float2*>(rows + kSeg * kN + c) = b;
+        if (ROWS && q == 3 && i == 7) *reinterpret_cast<float2*>(rows + kSeg * kRld + c) = b;
     }
     float s = reduce8(x, lane);
     s += __shfl_xor_sync(0xffffffffu, s, 1);
@@ -220,7 +270,7 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
         *reinterpret_cast<float2*>(o.em2 + c) = make_float2(ex2(le.x), ex2(le.y));
     }
     check(bad, make_float2(s, 0.f));
-    const bool in = lm.x >= -kRange && lm.y >= -kRange && le.x >= -kRange && le.y >= -kRange;
+    const bool in = lm.x >= -kRange<STATIC> && lm.y >= -kRange<STATIC> && le.x >= -kRange<STATIC> && le.y >= -kRange<STATIC>;
     return !(in && bad == 0.f);
 }
 // the images of a tensor as it came (pieces of 16 bytes where the alignment allows)
@@ -242,7 +292,7 @@ __device__ __forceinline__ bool stage_images(unsigned char* img, int tid, int n,
         }
     } else {
         Pair<E> x[8];
-        read_rows<E>(x, x_ + 2 * lane, t0, n, C, vec_ok(x_, 2));
+        read_rows<E, 8>(x, x_ + 2 * lane, t0, n, C, vec_ok(x_, 2));
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             check(bad, decode(x[i]));
@@ -252,31 +302,42 @@ __device__ __forceinline__ bool stage_images(unsigned char* img, int tid, int n,
     return bad != 0.f;
 }
 
-// Token x token products: c = rows 16 mt .. of one set of images times rows 16 nt .. of another, over the 64 channels
-template <int NA, int NB>
+// Token x token products: c = rows 16 mt .. of one set of images times rows 16 nt .. of another, over the 64 channels (two sums side
+// by side: the products of one sum wait for one another)
+template <bool APART, int NA, int NB>
 __device__ __forceinline__ void gram(float (&c)[1][2][4], const unsigned char* a_img, const unsigned char* b_img, int mt, int nt, int lane) {
+    float c2[1][2][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) c[0][0][e] = c[0][1][e] = 0.f;
+    for (int e = 0; e < 4; ++e) c[0][0][e] = c[0][1][e] = c2[0][0][e] = c2[0][1][e] = 0.f;
 #pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-        uint32_t a[1][NA][4], b[NB][4];
+    for (int kk = 0; kk < 4; kk += 2) {
+        uint32_t a[1][NA][4], b[NB][4], a2[1][NA][4], b2[NB][4];
         ldsm<NA>(a[0], smem_addr(a_img) + frag_rows(16 * mt, 2 * kk, lane));
         ldsm<NB>(b, smem_addr(b_img) + frag_cols(16 * nt, 2 * kk, lane));
-        mma_split<1, NA, NB>(c, a, b);
+        ldsm<NA>(a2[0], smem_addr(a_img) + frag_rows(16 * mt, 2 * kk + 2, lane));
+        ldsm<NB>(b2, smem_addr(b_img) + frag_cols(16 * nt, 2 * kk + 2, lane));
+        mma_split<APART, 1, NA, NB>(c, a, b);
+        mma_split<APART, 1, NA, NB>(c2, a2, b2);
     }
-}
-// An A fragment from a token x token matrix in shared memory, as stored or transposed
-template <bool TRANS>
-__device__ __forceinline__ void matrix_frag(uint32_t (&f)[3][4], const float* m, int m0, int k0, int lane) {
-    const int g = lane >> 2, q = lane & 3;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int row = m0 + g + 8 * (e & 1), col = k0 + 2 * q + 8 * (e >> 1);
-        float2 x;
-        if (TRANS) x = make_float2(m[col * kMld + row], m[(col + 1) * kMld + row]);
-        else x = *reinterpret_cast<const float2*>(m + row * kMld + col);
-        split3(x.x, x.y, f[0][e], f[1][e], f[2][e]);
-    }
+    for (int e = 0; e < 4; ++e) { c[0][0][e] += c2[0][0][e]; c[0][1][e] += c2[0][1][e]; }
+}
+
+// Triangular token x token matrices: three images of the tiles (0,0), (0,1) or (1,0), (1,1) at mt + nt, rows of two 16-byte pieces
+__device__ __forceinline__ uint32_t tile_at(int tile, int row, int piece) { return tile * 512 + row * 32 + ((piece ^ ((row >> 2) & 1)) << 4); }
+// a pair of row `row`, columns 8 j + 2 q, + 1 of a tile
+__device__ __forceinline__ void put_tile(unsigned char* img, int tile, int row, int j, int q, float x, float y) {
+    uint32_t h, m, l;
+    split3(x, y, h, m, l);
+    unsigned char* p = img + tile_at(tile, row, j) + 4 * q;
+    *reinterpret_cast<uint32_t*>(p) = h;
+    *reinterpret_cast<uint32_t*>(p + kTiles) = m;
+    *reinterpret_cast<uint32_t*>(p + 2 * kTiles) = l;
+}
+template <bool TRANS>   // a tile as A fragments, as stored or transposed
+__device__ __forceinline__ void tile_frag(uint32_t (&f)[3][4], const unsigned char* img, int tile, int lane) {
+    if (TRANS) ldsm_t<3, kTiles>(f, smem_addr(img) + tile_at(tile, (lane & 7) + ((lane >> 4) << 3), (lane >> 3) & 1));
+    else ldsm<3, kTiles>(f, smem_addr(img) + tile_at(tile, lane & 15, lane >> 4));
 }
 
 // Rows of 16 channels out of two accumulator tiles: neighbouring lanes swap a pair, so that a lane stores four channels
@@ -307,18 +368,27 @@ __device__ __forceinline__ void store_row<float>(float* row, float x0, float x1,
     else { p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w; }
 }
 
+// Asks L2 for what the block `ahead` places further on will read first: rows of up to five tensors, a state or two (128 lines each)
+template <typename E>
+__device__ __forceinline__ void prefetch_rows(const E* x, i64 base, int n, int C, int row) {
+    if (row < n) {
+        prefetch_l2(x + base + (i64)row * C);
+        if (sizeof(E) == 4) prefetch_l2(x + base + (i64)row * C + 32);
+    }
+}
+
 // ---- kernels -----------------------------------------------------------------------------------------------------------------
 // y of a segment from its start state.  One block per (unit, segment), 4 warps; a warp has 16 values of all tokens.
 template <typename E>
 struct YSmem {
     Operands o;
     unsigned char V[kParts<E> * kImg];
-    float M[kSeg * kMld];   // A transposed: [t][s]
+    unsigned char M[3 * kTiles];   // A transposed: [t][s]
 };
 template <typename E, bool STATIC>
 __global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
                                                            const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
-                                                           const float* __restrict__ states, E* __restrict__ y_, int* __restrict__ flags) {
+                                                           const float* __restrict__ states, E* __restrict__ y_, int* __restrict__ flags, int ahead) {
     extern __shared__ __align__(128) unsigned char smem_seg_y[];
     YSmem<E>& sm = *reinterpret_cast<YSmem<E>*>(smem_seg_y);
     constexpr int NV = kParts<E>;
@@ -326,6 +396,14 @@ __global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nse
     const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
     const int g = lane >> 2, q = lane & 3, n = min(kSeg, T - seg * kSeg);
     const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    if (blockIdx.x + ahead < gridDim.x) {
+        const i64 next = blockIdx.x + ahead;
+        const int seg1 = next % nseg, h1 = next / nseg % H, n1 = min(kSeg, T - seg1 * kSeg);
+        const i64 base1 = (next / nseg / H * T + (i64)seg1 * kSeg) * C + h1 * kN;
+        const E* x = warp == 0 ? r_ : warp == 1 ? k_ : warp == 2 ? v_ : w_;
+        if (!STATIC || warp < 3) prefetch_rows(x, base1, n1, C, lane);
+        prefetch_l2(states + next * kN * kN + tid * 32);
+    }
     float S[4][2][4];   // [16 keys][8 values] as B fragments
     {
         const float* p = states + (i64)blockIdx.x * kN * kN + 16 * warp + g;
@@ -348,13 +426,14 @@ __global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nse
     if (job < 3) {
         const int mt = job > 0, nt = job > 1;
         float c[1][2][4];
-        gram<3, 3>(c, sm.o.R, sm.o.K, mt, nt, lane);
+        gram<sizeof(E) == 4, 3, 3>(c, sm.o.R, sm.o.K, mt, nt, lane);
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int t = 16 * mt + g + 8 * (e >> 1), s = 16 * nt + 8 * j + 2 * q + (e & 1);
-                sm.M[t * kMld + s] = s < t ? c[0][j][e] : s == t ? sm.o.ruk[t] : 0.f;
+            for (int e = 0; e < 2; ++e) {
+                const int t = 16 * mt + g + 8 * e, s = 16 * nt + 8 * j + 2 * q;
+                const float x = s < t ? c[0][j][2 * e] : s == t ? sm.o.ruk[t] : 0.f, z = s + 1 < t ? c[0][j][2 * e + 1] : s + 1 == t ? sm.o.ruk[t] : 0.f;
+                put_tile(sm.M, mt + nt, g + 8 * e, j, q, x, z);
             }
     }
     float acc[2][2][4];
@@ -373,7 +452,7 @@ __global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nse
         }
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) ldsm<3>(a[mt], smem_addr(sm.o.R) + frag_rows(16 * mt, 2 * kk, lane));
-        mma_split<2, 3, 3>(acc, a, b);
+        mma_split<sizeof(E) == 4, 2, 3, 3>(acc, a, b);
     }
     __syncthreads();
 #pragma unroll
@@ -383,9 +462,9 @@ __global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nse
 #pragma unroll
         for (int mt = kt; mt < 2; ++mt) {
             uint32_t a[1][3][4];
-            matrix_frag<false>(a[0], sm.M, 16 * mt, 16 * kt, lane);
+            tile_frag<false>(a[0], sm.M, mt + kt, lane);
             float(&c)[1][2][4] = *reinterpret_cast<float(*)[1][2][4]>(&acc[mt]);
-            mma_split<1, 3, NV>(c, a, b);
+            mma_split<sizeof(E) == 4, 1, 3, NV>(c, a, b);
         }
     }
     const bool vec = vec_ok(y_, 4);
@@ -404,15 +483,15 @@ template <typename E>
 struct BwdSmemM {
     Operands o;
     unsigned char V[kParts<E> * kImg], G[kParts<E> * kImg];
-    float A[kSeg * kMld], Gm[kSeg * kMld];
-    float rows[(kSeg + 1) * kN], gamma[kSeg], a0[kN];
+    unsigned char A[3 * kTiles], Gm[3 * kTiles];
+    float rows[(kSeg + 1) * kRld], gamma[kSeg], a0[kN];
 };
 template <typename E, bool STATIC>
 __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     seg_mma_backward_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_, const E* __restrict__ v_,
                             const E* __restrict__ w_, const E* __restrict__ u_, const E* __restrict__ gy_, const float* __restrict__ S_,
                             const float* __restrict__ D_, E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_, E* __restrict__ gw_,
-                            float* __restrict__ partial_, int* __restrict__ flags) {
+                            float* __restrict__ partial_, int* __restrict__ flags, int ahead) {
     extern __shared__ __align__(128) unsigned char smem_seg_b[];
     BwdSmemM<E>& sm = *reinterpret_cast<BwdSmemM<E>*>(smem_seg_b);
     constexpr int NV = kParts<E>;
@@ -420,6 +499,26 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
     const int g = lane >> 2, q = lane & 3, n = min(kSeg, T - seg * kSeg);
     const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    if (blockIdx.x + ahead < gridDim.x) {
+        const i64 next = blockIdx.x + ahead;
+        const int seg1 = next % nseg, h1 = next / nseg % H, n1 = min(kSeg, T - seg1 * kSeg);
+        const i64 base1 = (next / nseg / H * T + (i64)seg1 * kSeg) * C + h1 * kN;
+        const E* x = warp == 0 ? r_ : warp == 1 ? k_ : warp == 2 ? v_ : gy_;
+        prefetch_rows(x, base1, n1, C, lane);
+        if (!STATIC && warp == 0) prefetch_rows(w_, base1, n1, C, lane);
+        prefetch_l2(S_ + next * kN * kN + tid * 32);
+        prefetch_l2(D_ + next * kN * kN + tid * 32);
+    }
+    float D[4][2][4];   // [16 keys][8 values] as B fragments
+    {
+        const float* p = D_ + (i64)blockIdx.x * kN * kN + 16 * warp + g;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) D[kk][nt][e] = p[(16 * kk + 2 * q + (e & 1) + 8 * (e >> 1)) * kN + 8 * nt];
+    }
     bool bad = make_operands<E, STATIC, true>(sm.o, sm.rows, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN);
     bad |= stage_images<E>(sm.V, tid, n, C, v_ + base);
     bad |= stage_images<E>(sm.G, tid, n, C, gy_ + base);
@@ -433,19 +532,19 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     for (int job = (warp + blockIdx.x) & 3; job < 6; job = job >= 3 && NV == 1 ? job + 1 : NV == 1 ? 6 : job + 4) {
         const int tile = job % 3, mt = tile > 1, nt = tile > 0;
         float c[1][2][4];
-        if (job < 3) gram<3, 3>(c, sm.o.K, sm.o.R, mt, nt, lane);
-        else gram<NV, NV>(c, sm.V, sm.G, mt, nt, lane);
+        if (job < 3) gram<sizeof(E) == 4, 3, 3>(c, sm.o.K, sm.o.R, mt, nt, lane);
+        else gram<sizeof(E) == 4, NV, NV>(c, sm.V, sm.G, mt, nt, lane);
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int s = 16 * mt + g + 8 * (e >> 1), t = 16 * nt + 8 * j + 2 * q + (e & 1);
-                const float x = c[0][j][e];
-                if (job < 3) sm.A[s * kMld + t] = s < t ? x : s == t ? sm.o.ruk[t] : 0.f;
-                else {
-                    sm.Gm[s * kMld + t] = s < t ? x : 0.f;
-                    if (s == t) sm.gamma[t] = x;
-                }
+            for (int e = 0; e < 2; ++e) {
+                const int s = 16 * mt + g + 8 * e, t = 16 * nt + 8 * j + 2 * q;
+                const float x = c[0][j][2 * e], z = c[0][j][2 * e + 1];
+                const bool diag = job < 3;
+                if (!diag && s == t) sm.gamma[s] = x;
+                if (!diag && s == t + 1) sm.gamma[s] = z;
+                put_tile(diag ? sm.A : sm.Gm, mt + nt, g + 8 * e, j, q, s < t ? x : diag && s == t ? sm.o.ruk[s] : 0.f,
+                         s < t + 1 ? z : diag && s == t + 1 ? sm.o.ruk[s] : 0.f);
             }
     }
     {   // gv = K~ D' + A gY
@@ -454,22 +553,18 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[mt][0][e] = acc[mt][1][e] = 0.f;
-        const float* p = D_ + (i64)blockIdx.x * kN * kN + 16 * warp + g;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             uint32_t a[2][3][4], b[3][4];
             const float2 f0 = *reinterpret_cast<const float2*>(sm.o.em2 + 16 * kk + 2 * q), f1 = *reinterpret_cast<const float2*>(sm.o.em2 + 16 * kk + 8 + 2 * q);
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                float x[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) x[e] = p[(16 * kk + 2 * q + (e & 1) + 8 * (e >> 1)) * kN + 8 * nt];
-                split3(x[0] * f0.x, x[1] * f0.y, b[0][2 * nt], b[1][2 * nt], b[2][2 * nt]);
-                split3(x[2] * f1.x, x[3] * f1.y, b[0][2 * nt + 1], b[1][2 * nt + 1], b[2][2 * nt + 1]);
+                split3(D[kk][nt][0] * f0.x, D[kk][nt][1] * f0.y, b[0][2 * nt], b[1][2 * nt], b[2][2 * nt]);
+                split3(D[kk][nt][2] * f1.x, D[kk][nt][3] * f1.y, b[0][2 * nt + 1], b[1][2 * nt + 1], b[2][2 * nt + 1]);
             }
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt) ldsm<3>(a[mt], smem_addr(sm.o.K) + frag_rows(16 * mt, 2 * kk, lane));
-            mma_split<2, 3, 3>(acc, a, b);
+            mma_split<sizeof(E) == 4, 2, 3, 3>(acc, a, b);
         }
         __syncthreads();
 #pragma unroll
@@ -479,9 +574,9 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
             for (int mt = 0; mt <= kt; ++mt) {
                 uint32_t a[1][3][4];
-                matrix_frag<false>(a[0], sm.A, 16 * mt, 16 * kt, lane);
+                tile_frag<false>(a[0], sm.A, mt + kt, lane);
                 float(&c)[1][2][4] = *reinterpret_cast<float(*)[1][2][4]>(&acc[mt]);
-                mma_split<1, 3, NV>(c, a, b);
+                mma_split<sizeof(E) == 4, 1, 3, NV>(c, a, b);
             }
         }
 #pragma unroll
@@ -522,10 +617,10 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             uint32_t a[2][NV][4];
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt) ldsm<NV>(a[mt], smem_addr(sm.V) + frag_rows(16 * mt, 2 * kk, lane));
-            mma_split<2, NV, 3>(dk, a, bd);
+            mma_split<sizeof(E) == 4, 2, NV, 3>(dk, a, bd);
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt) ldsm<NV>(a[mt], smem_addr(sm.G) + frag_rows(16 * mt, 2 * kk, lane));
-            mma_split<2, NV, 3>(dr, a, bs);
+            mma_split<sizeof(E) == 4, 2, NV, 3>(dr, a, bs);
         }
     }
 #pragma unroll
@@ -535,20 +630,15 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         if (q == 0) sm.a0[16 * warp + 8 * nt + g] = a0[nt];
     }
     __syncwarp();
-    Pair<E> rp[2][2][2], kp[2][2][2];   // [16 tokens][8 of them][tile]
+    Pair<E> rp[2][4], kp[2][4];   // [tile][eight tokens]
     {
         const bool vin = vec_ok(r_, 2) && vec_ok(k_, 2);
+        const i64 o = base + 16 * warp + 2 * q;
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    const int t = 16 * mt + 8 * e + g;
-                    const i64 o = base + (i64)t * C + 16 * warp + 8 * nt + 2 * q;
-                    rp[mt][e][nt] = t < n ? read_pair(r_ + o, vin) : no_pair<E>();
-                    kp[mt][e][nt] = t < n ? read_pair(k_ + o, vin) : no_pair<E>();
-                }
+        for (int nt = 0; nt < 2; ++nt) {
+            read_eights<E>(rp[nt], r_ + o + 8 * nt, g, n, C, vin);
+            read_eights<E>(kp[nt], k_ + o + 8 * nt, g, n, C, vin);
+        }
     }
     float2 aend[2];
 #pragma unroll
@@ -559,7 +649,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const float2 k = decode(kp[mt][e][nt]), l = *reinterpret_cast<const float2*>(sm.rows + (16 * mt + 8 * e + g + 1) * kN + c);
+                const float2 k = decode(kp[nt][2 * mt + e]), l = *reinterpret_cast<const float2*>(sm.rows + (16 * mt + 8 * e + g + 1) * kRld + c);
                 s.x = fmaf(k.x * ex2(-l.x), dk[mt][nt][2 * e], s.x);
                 s.y = fmaf(k.y * ex2(-l.y), dk[mt][nt][2 * e + 1], s.y);
             }
@@ -578,14 +668,14 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         for (int kt = 0; kt < 2; ++kt) {
             uint32_t a[1][3][4], b[3][4];
             if (kt >= mt) {
-                matrix_frag<false>(a[0], sm.Gm, 16 * mt, 16 * kt, lane);
+                tile_frag<false>(a[0], sm.Gm, mt + kt, lane);
                 ldsm_t<3>(b, smem_addr(sm.o.R) + frag_rows(16 * kt, 2 * warp, lane));
-                mma_split<1, 3, 3>(ck, a, b);
+                mma_split<sizeof(E) == 4, 1, 3, 3>(ck, a, b);
             }
             if (kt <= mt) {
-                matrix_frag<true>(a[0], sm.Gm, 16 * mt, 16 * kt, lane);
+                tile_frag<true>(a[0], sm.Gm, mt + kt, lane);
                 ldsm_t<3>(b, smem_addr(sm.o.K) + frag_rows(16 * kt, 2 * warp, lane));
-                mma_split<1, 3, 3>(cr, a, b);
+                mma_split<sizeof(E) == 4, 1, 3, 3>(cr, a, b);
             }
         }
     }
@@ -598,8 +688,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const int mt = b >> 1, e = b & 1, t = 8 * b + g;
-            const float2 r = decode(rp[mt][e][nt]), k = decode(kp[mt][e][nt]);
-            const float2 l0 = *reinterpret_cast<const float2*>(sm.rows + t * kN + c), l1 = *reinterpret_cast<const float2*>(sm.rows + (t + 1) * kN + c);
+            const float2 r = decode(rp[nt][b]), k = decode(kp[nt][b]);
+            const float2 l0 = *reinterpret_cast<const float2*>(sm.rows + t * kRld + c), l1 = *reinterpret_cast<const float2*>(sm.rows + (t + 1) * kRld + c);
             float &k0 = dk[mt][nt][2 * e], &k1 = dk[mt][nt][2 * e + 1], &r0 = dr[mt][nt][2 * e], &r1 = dr[mt][nt][2 * e + 1];
             k0 *= ex2(-l1.x); k1 *= ex2(-l1.y); r0 *= ex2(l0.x); r1 *= ex2(l0.y);
             Q[b] = make_float2(k.x * k0, k.y * k1);
@@ -640,16 +730,16 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             p[0] = gu.x; p[1] = gu.y;
         }
         if (!STATIC) {
+            Pair<E> wp[4];
+            read_eights<E>(wp, w_ + base + c, g, n, C, vec_ok(w_, 2));
+            E* p = gw_ + base + (i64)g * C + c;
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                const int t = 8 * b + g;
-                const float2 w = t < n ? decode(read_pair(w_ + base + (i64)t * C + c, vec_ok(w_, 2))) : make_float2(0.f, 0.f);
-                // kept where Q and P of the tile were: dk and dr leave below with both tiles
+                const float2 w = decode(wp[b]);
                 x[b].x *= -ex2(kLog2e * w.x); x[b].y *= -ex2(kLog2e * w.y);
-                if (t < n) {
-                    E* p = gw_ + base + (i64)t * C + c;
-                    if (sizeof(E) == 2 && vec) *reinterpret_cast<uint32_t*>(p) = pack_bf16(x[b].x, x[b].y);
-                    else { p[0] = from_f<E>(x[b].x); p[1] = from_f<E>(x[b].y); }
+                if (8 * b + g < n) {
+                    if (sizeof(E) == 2 && vec) *reinterpret_cast<uint32_t*>(p + 8 * b * C) = pack_bf16(x[b].x, x[b].y);
+                    else { p[8 * b * C] = from_f<E>(x[b].x); p[8 * b * C + 1] = from_f<E>(x[b].y); }
                 }
             }
         }
@@ -667,24 +757,25 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 
 // States at the start of every segment (REV: adjoints at the end), one block per unit walking its segments: S <- S diag(f) + k'^T V
 // with k'_s = k_s exp(L_end - L_s) (REV: r'_t = r_t exp(L_{t-1}), gy): all factors are at most 1.  Warps 0 to 3 have the state in
-// registers, 16 keys each, warps 4 to 7 make the operands of the segments to come.
+// registers, 16 keys each, warps 4 to 11 make the operands of the segments to come (B8 T1000 H32 bf16: 80 us with four of them, 72 with
+// eight and rows asked for in L2 six segments ahead: 1.8 TB/s; the walk waits for instructions of the operands and for barriers).
 template <typename E>
 struct ChainSmem {
     unsigned char A[3 * kImg], B[kParts<E> * kImg];
-    float f[kN], tot[4 * kN];
+    float f[kN], tot[8 * kN];
 };
 template <int ID>
 __device__ __forceinline__ void bar_join(int odd) {
-    if (odd) asm volatile("bar.sync %0, 256;" ::"n"(ID + 1) : "memory");
-    else asm volatile("bar.sync %0, 256;" ::"n"(ID) : "memory");
+    if (odd) asm volatile("bar.sync %0, 384;" ::"n"(ID + 1) : "memory");
+    else asm volatile("bar.sync %0, 384;" ::"n"(ID) : "memory");
 }
 template <int ID>
 __device__ __forceinline__ void bar_tell(int odd) {
-    if (odd) asm volatile("bar.arrive %0, 256;" ::"n"(ID + 1) : "memory");
-    else asm volatile("bar.arrive %0, 256;" ::"n"(ID) : "memory");
+    if (odd) asm volatile("bar.arrive %0, 384;" ::"n"(ID + 1) : "memory");
+    else asm volatile("bar.arrive %0, 384;" ::"n"(ID) : "memory");
 }
 template <typename E, bool STATIC, bool REV>
-__global__ void __launch_bounds__(256, 2) seg_mma_chain_kernel(int T, int H, int nseg, const E* __restrict__ a_, const E* __restrict__ b_,
+__global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_kernel(int T, int H, int nseg, const E* __restrict__ a_, const E* __restrict__ b_,
                                                                const E* __restrict__ w_, float* __restrict__ states) {
     extern __shared__ __align__(128) unsigned char smem_seg_c[];
     ChainSmem<E>* buf = reinterpret_cast<ChainSmem<E>*>(smem_seg_c);
@@ -693,59 +784,68 @@ __global__ void __launch_bounds__(256, 2) seg_mma_chain_kernel(int T, int H, int
     const int h = unit % H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = H * kN;
     const i64 base = unit / H * T * C + h * kN;
     if (warp >= 4) {
-        // ---- operands: channels 2 lane, 2 lane + 1 of eight tokens ----------------------------------------------------------
-        const int p = warp - 4, t0 = 8 * p, c = 2 * lane, tid = threadIdx.x - 128;
+        // ---- operands: channels 2 lane, 2 lane + 1 of four tokens ----------------------------------------------------------
+        constexpr int R = 4;
+        const int p = warp - 4, t0 = R * p, c = 2 * lane, tid = threadIdx.x - 128;
         const bool vec = vec_ok(a_, 2) && vec_ok(w_, 2), wide = sizeof(E) == 2 && vec_ok(b_, 8), vecb = vec_ok(b_, 2);
-        Pair<E> aa[8], ww[STATIC ? 1 : 8], bb[8];
-        uint4 bw[2];
-        auto fetch = [&](int it) {
+        struct Raw {   // of two segments: what is asked for in one step of the loop below is read two steps later
+            Pair<E> aa[R], ww[STATIC ? 1 : R], bb[R];
+            uint4 bw;
+        } raw[2];
+        auto fetch = [&](Raw& x, int it) {
             const int seg = REV ? nseg - 1 - it : it, n = min(kSeg, T - seg * kSeg);
             const i64 o = base + (i64)seg * kSeg * C;
-            read_rows<E>(aa, a_ + o + c, t0, n, C, vec);
-            if constexpr (!STATIC) read_rows<E>(ww, w_ + o + c, t0, n, C, vec);
+            read_rows<E, R>(x.aa, a_ + o + c, t0, n, C, vec);
+            if constexpr (!STATIC) read_rows<E, R>(x.ww, w_ + o + c, t0, n, C, vec);
             if (wide) {
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int row = 16 * i + (tid >> 3);
-                    bw[i] = row < n ? __ldg(reinterpret_cast<const uint4*>(b_ + o + (i64)row * C + 8 * (tid & 7))) : make_uint4(0u, 0u, 0u, 0u);
-                }
-            } else read_rows<E>(bb, b_ + o + c, t0, n, C, vecb);
+                const int row = tid >> 3;
+                x.bw = row < n ? __ldg(reinterpret_cast<const uint4*>(b_ + o + (i64)row * C + 8 * (tid & 7))) : make_uint4(0u, 0u, 0u, 0u);
+            } else read_rows<E, R>(x.bb, b_ + o + c, t0, n, C, vecb);
+            const int far = REV ? seg - 6 : seg + 6;   // (two steps are not long enough for HBM)
+            if (far >= 0 && far < nseg && tid < (STATIC ? 64 : 96)) {
+                const E* y = tid < 32 ? a_ : tid < 64 ? b_ : w_;
+                prefetch_rows(y, base + (i64)far * kSeg * C, min(kSeg, T - far * kSeg), C, lane);
+            }
         };
-        if constexpr (STATIC) ww[0] = read_pair(w_ + h * kN + c, vec);
-        if (nseg > 1) fetch(0);
-        for (int it = 0; it + 1 < nseg; ++it) {
+        if constexpr (STATIC) raw[0].ww[0] = raw[1].ww[0] = read_pair(w_ + h * kN + c, vec);
+        if (nseg > 1) fetch(raw[0], 0);
+        if (nseg > 2) fetch(raw[1], 1);
+        auto make = [&](Raw& x, int it) {
             const int seg = REV ? nseg - 1 - it : it, n = min(kSeg, T - seg * kSeg);
             ChainSmem<E>& sm = buf[it & 1];
             if (it >= 2) bar_join<3>(it & 1);
-            float2 d[STATIC ? 1 : 8], before, after;   // sums of log2 decays before and behind these tokens
-            if constexpr (STATIC) d[0] = log2_decay_static(decode(ww[0]));
+            float2 d[STATIC ? 1 : R], before, after;   // sums of log2 decays before and behind these tokens
+            if constexpr (STATIC) d[0] = log2_decay_static(decode(x.ww[0]));
             else {
                 float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    d[i] = t0 + i < n ? log2_decay(decode(ww[i])) : make_float2(0.f, 0.f);
+                for (int i = 0; i < R; ++i) {
+                    d[i] = t0 + i < n ? log2_decay(decode(x.ww[i])) : make_float2(0.f, 0.f);
                     s.x += d[i].x; s.y += d[i].y;
                 }
                 *reinterpret_cast<float2*>(sm.tot + p * kN + c) = s;
-                asm volatile("bar.sync 5, 128;" ::: "memory");
+                asm volatile("bar.sync 5, 256;" ::: "memory");
                 before = after = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < kSeg / R; ++i) {
                     const float2 t = *reinterpret_cast<const float2*>(sm.tot + i * kN + c);
                     if (i < p) { before.x += t.x; before.y += t.y; }
                     if (i > p) { after.x += t.x; after.y += t.y; }
                 }
                 if (p == 0) *reinterpret_cast<float2*>(sm.f + c) = make_float2(ex2(s.x + after.x), ex2(s.y + after.y));
             }
-            if (STATIC && p == 0) *reinterpret_cast<float2*>(sm.f + c) = make_float2(ex2(d[0].x * n), ex2(d[0].y * n));
+            if (STATIC && p == 0) {   // (exact to a rounding: the same factor acts once per segment)
+                const float2 w = decode(x.ww[0]);
+                *reinterpret_cast<float2*>(sm.f + c) = make_float2(expf(-expf(w.x) * n), expf(-expf(w.y) * n));
+            }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int i = REV ? j : 7 - j;   // towards the end that the products count from, starting there
-                const float2 a = decode(aa[i]);
+            for (int j = 0; j < R; ++j) {
+                const int i = REV ? j : R - 1 - j;   // towards the end that the products count from, starting there
+                const float2 a = decode(x.aa[i]);
                 float2 e;
                 if constexpr (STATIC) {
-                    const float x = (float)(REV ? t0 + i : max(n - 1 - (t0 + i), 0));
-                    e = make_float2(d[0].x * x, d[0].y * x);
+                    const float m = (float)(REV ? t0 + i : max(n - 1 - (t0 + i), 0));
+                    e = make_float2(d[0].x * m, d[0].y * m);
                 } else {
                     float2& s = REV ? before : after;
                     e = s;
@@ -754,14 +854,17 @@ __global__ void __launch_bounds__(256, 2) seg_mma_chain_kernel(int T, int H, int
                 put_split(sm.A, t0 + i, lane, a.x * ex2(e.x), a.y * ex2(e.y));
             }
             if (wide) {
-#pragma unroll
-                for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(sm.B + img_at(16 * i + (tid >> 3), tid & 7)) = bw[i];
+                *reinterpret_cast<uint4*>(sm.B + img_at(tid >> 3, tid & 7)) = x.bw;
             } else {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) put_pair<E>(sm.B, t0 + i, lane, bb[i]);
+                for (int i = 0; i < R; ++i) put_pair<E>(sm.B, t0 + i, lane, x.bb[i]);
             }
-            if (it + 2 < nseg) fetch(it + 1);
+            if (it + 3 < nseg) fetch(x, it + 2);
             bar_tell<1>(it & 1);
+        };
+        for (int it = 0; it + 1 < nseg; it += 2) {
+            make(raw[0], it);
+            if (it + 2 < nseg) make(raw[1], it + 1);
         }
         return;
     }
@@ -794,7 +897,7 @@ __global__ void __launch_bounds__(256, 2) seg_mma_chain_kernel(int T, int H, int
             for (int kt = 0; kt < 2; ++kt) {
                 uint32_t b[NV][4];
                 ldsm_t<NV>(b, smem_addr(sm.B) + frag_rows(16 * kt, 2 * i, lane));
-                mma_split<1, 3, NV>(c, a[kt], b);
+                mma_split<sizeof(E) == 4, 1, 3, NV>(c, a[kt], b);
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j)
@@ -830,13 +933,16 @@ inline unsigned flagged_blocks(i64 total, int per_sm) {   // as many as are resi
 // One block per unit walks all segments, or (the other kernels) every segment on its own and a scan: with few units the walk is
 // as long as T, and the scan's passes over the states cost little.
 inline bool seg_chain_pays(i64 units) { return units * 2 > sm_count(); }
+// Up to four segments per SM the token-by-token kernels take all of them: a launch less each way, and nothing to win (RWKV-6 T1000
+// H8 B1, 256 segments: 110 us, 114 by products; B2 T1000 H32, 2048 segments: 324 and 225 us).
+inline bool seg_mma_pays(i64 total) { return total > 4ll * sm_count(); }
 
 template <typename E, bool STATIC, bool REV>
 int seg_chain(i64 units, int T, int H, int nseg, const void* a, const void* b, const void* w, float* states, cudaStream_t st) {
     constexpr int smem = 2 * sizeof(ChainSmem<E>);
     const cudaError_t e = allow_smem<seg_mma_chain_kernel<E, STATIC, REV>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    seg_mma_chain_kernel<E, STATIC, REV><<<(unsigned)units, 256, smem, st>>>(T, H, nseg, (const E*)a, (const E*)b, (const E*)w, states);
+    seg_mma_chain_kernel<E, STATIC, REV><<<(unsigned)units, 384, smem, st>>>(T, H, nseg, (const E*)a, (const E*)b, (const E*)w, states);
     return check_launch("training on segments: states");
 }
 template <typename E, bool STATIC>
@@ -846,7 +952,7 @@ int seg_mma_y(i64 total, int T, int H, int nseg, const void* r, const void* k, c
     const cudaError_t e = allow_smem<seg_mma_y_kernel<E, STATIC>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     seg_mma_y_kernel<E, STATIC><<<(unsigned)total, 128, smem, st>>>(T, H, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states,
-                                                                   (E*)y, flags);
+                                                                   (E*)y, flags, 4 * sm_count());
     return check_launch("training on segments: y");
 }
 template <typename E, bool STATIC>
@@ -856,7 +962,8 @@ int seg_mma_backward(i64 total, int T, int H, int nseg, const void* r, const voi
     const cudaError_t e = allow_smem<seg_mma_backward_kernel<E, STATIC>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     seg_mma_backward_kernel<E, STATIC><<<(unsigned)total, 128, smem, st>>>(T, H, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u,
-                                                                          (const E*)gy, S, D, (E*)gr, (E*)gk, (E*)gv, (E*)gw, partial, flags);
+                                                                          (const E*)gy, S, D, (E*)gr, (E*)gk, (E*)gv, (E*)gw, partial, flags,
+                                                                          4 * sm_count());
     return check_launch("training on segments: gradients");
 }
 

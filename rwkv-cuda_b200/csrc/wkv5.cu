@@ -459,7 +459,7 @@ extern "C" int rwkvb200_wkv5_backward_saved(int dtype, int B, int T, int C, int 
 // head size 64 in fp32 arithmetic on the segments of wkv5_seg.cu; 2: larger heads on the general-shape kernels.
 extern "C" size_t rwkvb200_wkv5_train_saved_bytes(int B, int T, int C, int H) {
     if (B <= 0 || T <= 0 || C <= 0 || H <= 0) return 0;
-    return (size_t)B * H * (wkv5_seg_count(T) * (C / H) * (C / H) + 1) * sizeof(float);   // a state per 32 tokens and a flag per unit
+    return (size_t)B * H * wkv5_seg_count(T) * ((C / H) * (C / H) + 1) * sizeof(float);   // a state and a flag per 32 tokens (path 0: a flag per unit)
 }
 
 extern "C" int rwkvb200_wkv5_train_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v,
@@ -479,7 +479,8 @@ extern "C" int rwkvb200_wkv5_train_forward(int dtype, int B, int T, int C, int H
     }
     if (C / H <= 64) {
         RWKV_REQUIRE(B * (i64)H * (i64)wkv5_seg_count(T) < (1ll << 31), RWKVB200_EINVAL, "wkv5_train_forward: too many segments");
-        const int e = wkv5_seg_forward(dtype, B, T, C, H, r, k, v, w_raw, u, y, static_cast<float*>(saved), st);
+        const int e = wkv5_seg_forward(dtype, B, T, C, H, r, k, v, w_raw, u, y, static_cast<float*>(saved),
+                                       static_cast<int*>(saved) + (size_t)B * H * wkv5_seg_count(T) * (C / H) * (C / H), st);
         return e ? e : 1;
     }
 #define RWKV_GO(E)                                                                                                                   \
@@ -494,7 +495,7 @@ extern "C" int rwkvb200_wkv5_train_forward(int dtype, int B, int T, int C, int H
 extern "C" size_t rwkvb200_wkv5_train_work_bytes(int B, int T, int C, int H, int path) {
     if (B <= 0 || T <= 0 || C <= 0 || H <= 0) return 0;
     if (path != 1) return (size_t)B * 2 * C * sizeof(float);
-    return wkv5_seg_count(T) * ((size_t)B * H * (C / H) * (C / H) + (size_t)B * 2 * C) * sizeof(float);
+    return wkv5_seg_count(T) * ((size_t)B * H * ((C / H) * (C / H) + 1) + (size_t)B * 2 * C) * sizeof(float);
 }
 
 extern "C" int rwkvb200_wkv5_train_backward(int dtype, int B, int T, int C, int H, int path, const void* r, const void* k, const void* v,
@@ -529,7 +530,8 @@ extern "C" int rwkvb200_wkv5_train_backward(int dtype, int B, int T, int C, int 
         if (int e = check_launch("wkv5_train_backward")) return e;
     } else {
         float* D = partial + (size_t)B * wkv5_seg_count(T) * 2 * C;
-        if (int e = wkv5_seg_backward(dtype, B, T, C, H, r, k, v, w_raw, u, gy, gr, gk, gv, static_cast<const float*>(saved), D, partial, st)) return e;
+        if (int e = wkv5_seg_backward(dtype, B, T, C, H, r, k, v, w_raw, u, gy, gr, gk, gv, static_cast<const float*>(saved), D, partial,
+                                      reinterpret_cast<int*>(D + (size_t)B * H * wkv5_seg_count(T) * (C / H) * (C / H)), st)) return e;
         rows = (i64)B * wkv5_seg_count(T);
     }
     return sum_rows(dtype, rows, 2 * C, partial, gwu, st);

@@ -14,14 +14,18 @@
 // The decays of a segment act on its own outputs and on its end state: with Z = dS/dlog w counted from the segment's start
 // (Z_0 = 0, Z <- w (Z + S)), the segment's part of dL/dlog w is sum_t r_t sum_i gy_t Z_t + sum_i D_end Z_end.  (The sum over
 // states and gradients that needs no Z cancels for fast decays: 10 % error in gw at w = exp(-exp(3)).)
-// Inputs are staged in shared memory once per segment, so the token loops have no barrier; multiply-adds are packed in pairs.
+// With head size 64 the states come from one block per unit that walks its segments where there are many units, and y and the
+// gradients from products of split operands (seg_mma.cuh); the kernels here then take the segments that those leave, and all of them
+// for smaller heads and in small launches.
+// Their inputs are staged in shared memory once per segment, so the token loops have no barrier; multiply-adds are packed in pairs.
 // Shared memory delivers 4 bytes per lane and clock even when all lanes read the same word, so with one state line per thread
 // the reads of the token's vectors bound everything (512 bytes per 96 packed multiply-adds); a lane therefore owns a tile of
 // 8 keys x 8 values, and the sums over lanes are taken for eight elements at a time (7 shuffles).
-// fp32, B8 T512 H16 N64, forward + backward on a B200: 1285 us with wkv5.cu, 635 us with a line per thread, 320 us here
-// (without register spills in the backward, which two blocks per SM allow and three do not: 212 -> 167 us for that kernel).
+// fp32, B8 T512 H16 N64, forward + backward on a B200: 1285 us with wkv5.cu, 309 us token by token on all segments (without register
+// spills in the backward, which two blocks per SM allow and three do not: 212 -> 167 us for that kernel), 192 us by products, whose errors
+// against fp64 are a third of that (T 1000: y 5.3e-7 -> 1.8e-7 of the norm, gw 8.8e-7 -> 3.1e-7).
 #include "wkv5_seg.cuh"
-#include "seg_tiles.cuh"
+#include "seg_mma.cuh"
 
 namespace rwkvb200 {
 namespace {
@@ -91,18 +95,18 @@ __global__ void __launch_bounds__(64, 8) seg_local_kernel(int T, int C, int H, i
     store_tile(s, states + (i64)blockIdx.x * N * N, 8 * kg, 8 * vg, N);
 }
 
-// One block per (unit, segment), 2 warps: a warp has the values 32 warp .. of all keys
+// A segment token by token.  2 warps: a warp has the values 32 warp .. of all keys
 template <typename E>
-__global__ void __launch_bounds__(64, 8) seg_y_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
-                                                      const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
-                                                      const float* __restrict__ states, E* __restrict__ y_) {
+__device__ __forceinline__ void y_segment(i64 block, int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
+                                          const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
+                                          const float* __restrict__ states, E* __restrict__ y_) {
     __shared__ __align__(16) float rs[kSeg * kN], ks[kSeg * kN], vs[kSeg * kN], ws[kN], us[kN], ruk[kSeg];
-    const int unit = blockIdx.x / nseg, seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int unit = block / nseg, seg = block % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
     const int kg = lane >> 2, vg = 4 * warp + (lane & 3);
     Tile s;
-    load_tile(s, states + (i64)blockIdx.x * N * N, 8 * kg, 8 * vg, N);
+    load_tile(s, states + block * N * N, 8 * kg, 8 * vg, N);
     stage<64>(rs, r_ + base, n, C, N, tid);
     stage<64>(ks, k_ + base, n, C, N, tid);
     stage<64>(vs, v_ + base, n, C, N, tid);
@@ -139,7 +143,16 @@ __global__ void __launch_bounds__(64, 8) seg_y_kernel(int T, int C, int H, int N
     }
 }
 
-// One block per (unit, segment), 4 warps: warps 0, 1 carry S and Z forward (gr, gw, gu), warps 2, 3 carry D backward (gk, gv); a warp
+// every segment, or (flags) those that the kernels by products have left
+template <typename E>
+__global__ void __launch_bounds__(64, 8) seg_y_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
+                                                      const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
+                                                      const float* __restrict__ states, E* __restrict__ y_, const int* __restrict__ flags, i64 total) {
+    if (flags == nullptr) y_segment(blockIdx.x, T, C, H, N, nseg, r_, k_, v_, w_, u_, states, y_);
+    else for_flagged(flags, total, [&](i64 block) { y_segment(block, T, C, H, N, nseg, r_, k_, v_, w_, u_, states, y_); });
+}
+
+// A segment token by token.  4 warps: warps 0, 1 carry S and Z forward (gr, gw, gu), warps 2, 3 carry D backward (gk, gv); a warp
 // has 32 keys of all values.  gv sums over all keys: the two halves meet in shared memory at the end.
 struct BwdSmem {
     float r[kSeg * kN], k[kSeg * kN], v[kSeg * kN], g[kSeg * kN], gv[2][kSeg * kN];
@@ -147,20 +160,19 @@ struct BwdSmem {
 };
 
 template <typename E>
-__global__ void __launch_bounds__(128, 2) seg_backward_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
-                                                              const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
-                                                              const E* __restrict__ gy_, const float* __restrict__ S_, const float* __restrict__ D_,
-                                                              E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_,
-                                                              float* __restrict__ partial_) {
+__device__ __forceinline__ void backward_segment(i64 block, int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
+                                                 const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
+                                                 const E* __restrict__ gy_, const float* __restrict__ S_, const float* __restrict__ D_,
+                                                 E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_, float* __restrict__ partial_) {
     extern __shared__ __align__(16) unsigned char smem_seg[];
     BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_seg);
-    const int unit = blockIdx.x / nseg, seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int unit = block / nseg, seg = block % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
-    const float* D0 = D_ + (i64)blockIdx.x * N * N;
+    const float* D0 = D_ + block * N * N;
     const int kg = 4 * (warp & 1) + (lane & 3), vg = lane >> 2, j_out = 8 * kg + vg;   // j_out: the key whose sums this lane ends with
     Tile s;
-    load_tile(s, warp < 2 ? S_ + (i64)blockIdx.x * N * N : D0, 8 * kg, 8 * vg, N);
+    load_tile(s, warp < 2 ? S_ + block * N * N : D0, 8 * kg, 8 * vg, N);
     stage<128>(sm.r, r_ + base, n, C, N, tid);
     stage<128>(sm.k, k_ + base, n, C, N, tid);
     stage<128>(sm.v, v_ + base, n, C, N, tid);
@@ -269,40 +281,73 @@ __global__ void __launch_bounds__(128, 2) seg_backward_kernel(int T, int C, int 
 }
 
 template <typename E>
+__global__ void __launch_bounds__(128, 2) seg_backward_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
+                                                              const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
+                                                              const E* __restrict__ gy_, const float* __restrict__ S_, const float* __restrict__ D_,
+                                                              E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_,
+                                                              float* __restrict__ partial_, const int* __restrict__ flags, i64 total) {
+    if (flags == nullptr) backward_segment(blockIdx.x, T, C, H, N, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, partial_);
+    else for_flagged(flags, total, [&](i64 block) { backward_segment(block, T, C, H, N, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, partial_); });
+}
+
+// Head size 64: y and gradients by products (seg_mma.cuh), the kernels here only for the segments that those leave (flags).
+template <typename E>
 int forward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, void* y, float* states,
-            cudaStream_t st) {
+            int* flags, cudaStream_t st) {
     const int N = C / H, nseg = (T + kSeg - 1) / kSeg;
-    const unsigned grid = (unsigned)(B * (i64)H * nseg), scan = (unsigned)(B * (i64)H * ((N * N + 255) / 256));
-    seg_local_kernel<E, false><<<grid, 64, 0, st>>>(T, C, H, N, nseg, (const E*)k, (const E*)v, (const E*)w, states);
-    seg_scan_kernel<E, false><<<scan, 256, 0, st>>>(T, H, N, nseg, (const E*)w, states);
-    seg_y_kernel<E><<<grid, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states, (E*)y);
+    const i64 units = B * (i64)H, total = units * nseg;
+    if (N == kN && seg_chain_pays(units)) {
+        if (const int e = seg_chain<E, true, false>(units, T, H, nseg, k, v, w, states, st)) return e;
+    } else {
+        seg_local_kernel<E, false><<<(unsigned)total, 64, 0, st>>>(T, C, H, N, nseg, (const E*)k, (const E*)v, (const E*)w, states);
+        seg_scan_kernel<E, false><<<(unsigned)(units * ((N * N + 255) / 256)), 256, 0, st>>>(T, H, N, nseg, (const E*)w, states);
+    }
+    unsigned grid = (unsigned)total;
+    if (N != kN || !seg_mma_pays(total)) flags = nullptr;
+    if (flags != nullptr) {
+        if (const int e = seg_mma_y<E, true>(total, T, H, nseg, r, k, v, w, u, states, y, flags, st)) return e;
+        grid = flagged_blocks(total, 8);
+    }
+    seg_y_kernel<E><<<grid, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states, (E*)y,
+                                         flags, total);
     return check_launch("wkv5_train_forward(segments)");
 }
 
 template <typename E>
 int backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, const void* gy, void* gr,
-             void* gk, void* gv, const float* S, float* D, float* partial, cudaStream_t st) {
+             void* gk, void* gv, const float* S, float* D, float* partial, int* flags, cudaStream_t st) {
     const int N = C / H, nseg = (T + kSeg - 1) / kSeg, smem = sizeof(BwdSmem);
-    const unsigned grid = (unsigned)(B * (i64)H * nseg), scan = (unsigned)(B * (i64)H * ((N * N + 255) / 256));
+    const i64 units = B * (i64)H, total = units * nseg;
     const cudaError_t e = allow_smem<seg_backward_kernel<E>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv5_train_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    seg_local_kernel<E, true><<<grid, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)gy, (const E*)w, D);
-    seg_scan_kernel<E, true><<<scan, 256, 0, st>>>(T, H, N, nseg, (const E*)w, D);
+    if (N == kN && seg_chain_pays(units)) {
+        if (const int e = seg_chain<E, true, true>(units, T, H, nseg, r, gy, w, D, st)) return e;
+    } else {
+        seg_local_kernel<E, true><<<(unsigned)total, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)gy, (const E*)w, D);
+        seg_scan_kernel<E, true><<<(unsigned)(units * ((N * N + 255) / 256)), 256, 0, st>>>(T, H, N, nseg, (const E*)w, D);
+    }
+    unsigned grid = (unsigned)total;
+    if (N != kN || !seg_mma_pays(total)) flags = nullptr;
+    if (flags != nullptr) {
+        if (const int e = seg_mma_backward<E, true>(total, T, H, nseg, r, k, v, w, u, gy, S, D, gr, gk, gv, nullptr, partial, flags, st)) return e;
+        grid = flagged_blocks(total, 2);
+    }
     seg_backward_kernel<E><<<grid, 128, smem, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, (const E*)gy, S,
-                                                    D, (E*)gr, (E*)gk, (E*)gv, partial);
+                                                    D, (E*)gr, (E*)gk, (E*)gv, partial, flags, total);
     return check_launch("wkv5_train_backward(segments)");
 }
 
 }  // namespace
 
 int wkv5_seg_forward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, void* y,
-                     float* states, cudaStream_t st) {
-    return dtype == RWKVB200_F32 ? forward<float>(B, T, C, H, r, k, v, w, u, y, states, st) : forward<bf16>(B, T, C, H, r, k, v, w, u, y, states, st);
+                     float* states, int* flags, cudaStream_t st) {
+    return dtype == RWKVB200_F32 ? forward<float>(B, T, C, H, r, k, v, w, u, y, states, flags, st)
+                                 : forward<bf16>(B, T, C, H, r, k, v, w, u, y, states, flags, st);
 }
 int wkv5_seg_backward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
-                      const void* gy, void* gr, void* gk, void* gv, const float* S, float* D, float* partial, cudaStream_t st) {
-    return dtype == RWKVB200_F32 ? backward<float>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, st)
-                                 : backward<bf16>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, st);
+                      const void* gy, void* gr, void* gk, void* gv, const float* S, float* D, float* partial, int* flags, cudaStream_t st) {
+    return dtype == RWKVB200_F32 ? backward<float>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, flags, st)
+                                 : backward<bf16>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, flags, st);
 }
 
 }  // namespace rwkvb200

@@ -17,7 +17,7 @@
 //
 // B8 T1000 H32, forward + backward on a B200: 4374 us on the general-shape kernels, which walk the tokens with one block per unit;
 // 1237 us with the token-by-token kernels on all segments (multiply-adds at 46 % of the issue slots and the shared-memory reads of
-// the tokens' vectors); 606 us with products.  Errors against fp64 are the same to four digits (1.66e-3: one rounding to bf16).
+// the tokens' vectors); 552 us with products.  Errors against fp64 are the same to four digits (1.66e-3: one rounding to bf16).
 // The kernels for whole 32-token chunks take 258 us, but their operands are TF32: outputs are then 2 to 4 % further from fp64.
 #include "wkv6_seg.cuh"
 #include "seg_mma.cuh"
@@ -157,7 +157,8 @@ __device__ __forceinline__ void seg6_y_segment(i64 block, int T, int H, int nseg
 __global__ void __launch_bounds__(64) seg6_y_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
                                                     const bf16* __restrict__ v_, const bf16* __restrict__ w_, const bf16* __restrict__ u_,
                                                     const float* __restrict__ states, bf16* __restrict__ y_, const int* __restrict__ flags, i64 total) {
-    for_flagged(flags, total, [&](i64 block) { seg6_y_segment(block, T, H, nseg, r_, k_, v_, w_, u_, states, y_); });
+    if (flags == nullptr) seg6_y_segment(blockIdx.x, T, H, nseg, r_, k_, v_, w_, u_, states, y_);   // all segments
+    else for_flagged(flags, total, [&](i64 block) { seg6_y_segment(block, T, H, nseg, r_, k_, v_, w_, u_, states, y_); });
 }
 
 // The segments that seg_mma_backward_kernel has left.  4 warps: warps 0, 1 carry S forward (gr, gu, P), warps 2, 3 carry D backward (gk, gv, Q); a warp
@@ -288,7 +289,8 @@ __global__ void __launch_bounds__(128, 3) seg6_backward_kernel(int T, int H, int
                                                                const float* __restrict__ S_, const float* __restrict__ D_, bf16* __restrict__ gr_,
                                                                bf16* __restrict__ gk_, bf16* __restrict__ gv_, bf16* __restrict__ gw_,
                                                                float* __restrict__ gu_, const int* __restrict__ flags, i64 total) {
-    for_flagged(flags, total, [&](i64 block) { seg6_backward_segment(block, T, H, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, gw_, gu_); });
+    if (flags == nullptr) seg6_backward_segment(blockIdx.x, T, H, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, gw_, gu_);   // all segments
+    else for_flagged(flags, total, [&](i64 block) { seg6_backward_segment(block, T, H, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, gw_, gu_); });
 }
 
 }  // namespace
@@ -299,15 +301,16 @@ int wkv6_seg_forward(int B, int T, int H, const void* r, const void* k, const vo
     const i64 units = (i64)B * H, total = units * nseg;
     RWKV_REQUIRE(total < (1ll << 31), RWKVB200_EINVAL, "wkv6_train_forward: too many segments");
     float* decays = saved + total * kN * kN;
-    int* flags = reinterpret_cast<int*>(decays + total * kN);
+    int* flags = seg_mma_pays(total) ? reinterpret_cast<int*>(decays + total * kN) : nullptr;
     if (seg_chain_pays(units)) {
         if (const int e = seg_chain<bf16, false, false>(units, T, H, nseg, k, v, w, saved, st)) return e;
     } else {
         seg6_local_kernel<false><<<(unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)k, (const bf16*)v, (const bf16*)w, saved, decays);
         seg6_scan_kernel<false><<<(unsigned)(units * (kN * kN / 256)), 256, 0, st>>>(nseg, decays, saved);
     }
-    if (const int e = seg_mma_y<bf16, false>(total, T, H, nseg, r, k, v, w, u, saved, y, flags, st)) return e;
-    seg6_y_kernel<<<flagged_blocks(total, 8), 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, saved,
+    if (flags != nullptr)
+        if (const int e = seg_mma_y<bf16, false>(total, T, H, nseg, r, k, v, w, u, saved, y, flags, st)) return e;
+    seg6_y_kernel<<<flags != nullptr ? flagged_blocks(total, 8) : (unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, saved,
                                                            (bf16*)y, flags, total);
     return check_launch("wkv6_train_forward(segments)");
 }
@@ -325,8 +328,9 @@ int wkv6_seg_backward(int B, int T, int H, const void* r, const void* k, const v
         seg6_local_kernel<true><<<(unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)gy, (const bf16*)w, adjoints, nullptr);
         seg6_scan_kernel<true><<<(unsigned)(units * (kN * kN / 256)), 256, 0, st>>>(nseg, decays, adjoints);
     }
-    if (const int e = seg_mma_backward<bf16, false>(total, T, H, nseg, r, k, v, w, u, gy, saved, adjoints, gr, gk, gv, gw, gu_partial, flags, st)) return e;
-    seg6_backward_kernel<<<flagged_blocks(total, 3), 128, sizeof(Bwd6Smem), st>>>(
+    if (!seg_mma_pays(total)) flags = nullptr;
+    else if (const int e = seg_mma_backward<bf16, false>(total, T, H, nseg, r, k, v, w, u, gy, saved, adjoints, gr, gk, gv, gw, gu_partial, flags, st)) return e;
+    seg6_backward_kernel<<<flags != nullptr ? flagged_blocks(total, 3) : (unsigned)total, 128, sizeof(Bwd6Smem), st>>>(
         T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, (const bf16*)gy, saved, adjoints, (bf16*)gr, (bf16*)gk,
         (bf16*)gv, (bf16*)gw, gu_partial, flags, total);
     return check_launch("wkv6_train_backward(segments)");

@@ -91,7 +91,8 @@ def test_rwkv6_forward_scales_its_state(shift, T):
     Hh.assert_close(sT, sTo, Hh.TOL_BF16, "sT")
 
 
-@pytest.mark.parametrize("B,T,H", [(1, 71, 2), (2, 333, 40)])   # states by a scan over the segments, and by a walk along them
+# few segments; enough of them for the products, with states by a walk along the segments and (32 units) by a scan over them
+@pytest.mark.parametrize("B,T,H", [(1, 71, 2), (5, 33, 64), (3, 47, 110), (2, 333, 40), (1, 1000, 32)])
 def test_rwkv6_segments_of_both_kinds(B, T, H):
     """Segments with decays too strong for the matrix form (or for its anchor in the middle) beside others, every tensor one element off
     its alignment: bounds as above."""
@@ -100,7 +101,7 @@ def test_rwkv6_segments_of_both_kinds(B, T, H):
     N, C = 64, H * 64
     r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
     u, gy, w = Hh.rand(g, H, N, lo=-1, hi=1), Hh.randn(g, B, T, C), Hh.randn(g, B, T, C) - 4.0
-    w[:, 40, 3] = 6.0             # one token of a segment, one channel
+    w[:, -7, 3] = 6.0             # one token of a segment, one channel
     w[:, 64:, 2 * 64 - 1] = 1.5   # exp(1.5) * 16 > 60: from the third segment on
     odd = lambda x: torch.cat([x.new_zeros(1), x.flatten()]).to(BF).cuda()[1:].view(x.shape)
     xs = [odd(x).requires_grad_(True) for x in (r, k, v, w, u)]
@@ -120,7 +121,7 @@ def test_rwkv6_segments_of_both_kinds(B, T, H):
 def test_rwkv6_values_that_are_not_finite_stay_behind(name, value):
     """Tokens before such a value are those of the call without it, inside its segment too."""
     import rwkv_cuda_b200 as R
-    B, T, H, N, t = 1, 71, 1, 64, 45
+    B, T, H, N, t = 1, 71, 220, 64, 45   # (more than four segments per SM: by products)
     g = Hh.gen(5)
     C = H * N
     x = {n: 0.5 * Hh.randn(g, B, T, C) for n in ("r", "k", "v")}
@@ -132,3 +133,26 @@ def test_rwkv6_values_that_are_not_finite_stay_behind(name, value):
     size = clean.float().square().mean().sqrt()
     assert ((y[:, :t].float() - clean[:, :t].float()).abs() / size).max().item() < 2 ** -6   # (other kernel: other rounding, in bf16)
     assert not torch.isfinite(y[:, t]).all()
+
+
+@pytest.mark.parametrize("B,T,H", [(5, 40, 64), (2, 333, 40), (1, 1000, 32)])
+def test_rwkv5_fp32_by_products(B, T, H):
+    """fp32 through the products of split operands, heads with decays too strong for them among the others, tensors off their alignment.
+    Bounds: a sum of n products has an error of about sqrt(n) 2^-24 of their size; n is at most 64 keys x some 32 tokens, and gw
+    weights its terms by their distance in time (test of the operator: 1e-4)."""
+    import rwkv_cuda_b200 as R
+    g = Hh.gen(T)
+    N, C = 64, H * 64
+    r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
+    u, gy, w = Hh.rand(g, H, N, lo=-1, hi=1), Hh.randn(g, B, T, C), Hh.rand(g, H, N, lo=-6, hi=-1)
+    w[1, 5], w[2] = 2.0, 1.0
+    odd = lambda x: torch.cat([x.new_zeros(1), x.flatten()]).float().cuda()[1:].view(x.shape)
+    xs = [odd(x).requires_grad_(True) for x in (r, k, v, w, u)]
+    y = R.functions.WKV_5.apply(B, T, C, H, *xs)
+    got = [y, *torch.autograd.grad(y, xs, odd(gy))]
+    xo = [x.float().double().requires_grad_(True) for x in (r, k, v, w, u)]
+    yo = O.wkv5(*xo, H)
+    want = [yo, *torch.autograd.grad(yo, xo, gy.float().double())]
+    for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
+        err = ((a.double().cpu().reshape(b.shape) - b).norm() / b.norm()).item()
+        assert err <= 1e-6, f"{name}: {err:.3e}"
