@@ -103,3 +103,10 @@ def test_values_a_transform_cannot_take(T, bad):
     for got, ref, clean, name in zip((x, gw, gk), want, (clean_x, clean_gw, clean_gk), ("x", "gw", "gk")):
         Hh.assert_close(got[clean], ref[clean], Hh.TOL_FP32_STRICT, name)
         assert (~(got[~clean].abs() < 1e30)).float().mean() > 0.9, name
+
+
+@pytest.mark.parametrize("T", [383, 384, 385, 640, 767, 768, 769])   # the ends of the lengths 768 and 1536, which are not powers of two
+@pytest.mark.parametrize("B,C", [(1, 2), (3, 2), (33, 2)])
+def test_lengths_that_are_three_times_a_power_of_two(B, C, T):
+    test_conv1d_training_class(B, C, T)
+    test_errors_of_a_running_sum(T)
