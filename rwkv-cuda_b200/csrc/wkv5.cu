@@ -585,10 +585,28 @@ __global__ void __launch_bounds__(256) sum_rows_kernel(i64 rows, int n, const E*
         out[j] = from_f<O>(acc);
     }
 }
+// The same sums (in the same order) for up to 8 rows of four columns per thread: there is one row for each of the 8 threads
+// above, and most of the time goes into starting blocks (4 rows of 590 k columns: 18 us, and a
+// depthwise_conv1d training step of B32 C768 T768 takes 297 instead of 309 us).
+__global__ void __launch_bounds__(256) sum_few_rows_kernel(int rows, int n, const float* __restrict__ partial, float* __restrict__ out) {
+    const int j = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (j >= n) return;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int b = 0; b < rows; ++b) {
+        const float4 x = *reinterpret_cast<const float4*>(partial + (i64)b * n + j);
+        acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+    }
+    *reinterpret_cast<float4*>(out + j) = acc;
+}
 }  // namespace
 
 int sum_rows(int out_dtype, long long rows, int n, const float* partial, void* out, cudaStream_t st) {
     const dim3 block(32, 8);
+    if (out_dtype == RWKVB200_F32 && rows <= 8 && n >= 65536 && n % 4 == 0 && ((reinterpret_cast<uintptr_t>(partial) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
+        sum_few_rows_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, st>>>((int)rows, n, partial, static_cast<float*>(out));
+        return check_launch("sum_rows");
+    }
     if (out_dtype == RWKVB200_F32) sum_rows_kernel<float, float><<<(n + 31) / 32, block, 0, st>>>(rows, n, partial, (float*)out);
     else sum_rows_kernel<float, bf16><<<(n + 31) / 32, block, 0, st>>>(rows, n, partial, (bf16*)out);
     return check_launch("sum_rows");
