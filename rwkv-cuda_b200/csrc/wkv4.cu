@@ -154,11 +154,13 @@ __global__ void __launch_bounds__(32 * S) wkv4_forward_kernel(int T, int C, cons
     if (warp == 0) { buf.w[lane] = w; buf.carry[0][lane] = 0.f; buf.carry[1][lane] = 0.f; buf.carry[2][lane] = kNegInf; }
     float kn[L], vn[L];
     auto fetch = [&](int t0) {
+        const i64 o = off + (i64)t0 * C;
+        const float *kp = k_ + o, *vp = v_ + o;
 #pragma unroll
         for (int i = 0; i < L; ++i) {
             const bool in = t0 + i < T;
-            kn[i] = in ? k_[off + (i64)(t0 + i) * C] : 0.f;
-            vn[i] = in ? v_[off + (i64)(t0 + i) * C] : 0.f;
+            kn[i] = in ? kp[i * C] : 0.f;
+            vn[i] = in ? vp[i * C] : 0.f;
         }
     };
     fetch(warp * L);
@@ -168,15 +170,21 @@ __global__ void __launch_bounds__(32 * S) wkv4_forward_kernel(int T, int C, cons
         for (int i = 0; i < L; ++i) { k[i] = kn[i]; v[i] = vn[i]; }
         fetch(t0 + S * L);   // the next tile's loads are in flight during this tile's math
         const int n = T - t0;
-        Range rg = range_of(k, n);
+        const bool full = n >= L;   // whole segments have their own loops: no test per token
+        Range rg = full ? range_of(k, L) : range_of(k, n);
         Sum s = {0.f, 0.f, kNegInf};
         float e[L], base = rg.hi;
         const bool plain = __all_sync(0xffffffffu, bonus_ok && rg.hi - rg.lo <= kSpan);
         if (plain) {
 #pragma unroll
-            for (int i = 0; i < L; ++i) {
-                e[i] = expf(k[i] - rg.hi);
-                if (i < n) { s.p = fmaf(s.p, ew, e[i] * v[i]); s.q = fmaf(s.q, ew, e[i]); }
+            for (int i = 0; i < L; ++i) e[i] = expf(k[i] - rg.hi);
+            if (full) {
+#pragma unroll
+                for (int i = 0; i < L; ++i) { s.p = fmaf(s.p, ew, e[i] * v[i]); s.q = fmaf(s.q, ew, e[i]); }
+            } else {
+#pragma unroll
+                for (int i = 0; i < L; ++i)
+                    if (i < n) { s.p = fmaf(s.p, ew, e[i] * v[i]); s.q = fmaf(s.q, ew, e[i]); }
             }
             if (n > 0) s.o = rg.hi;
         } else {
@@ -190,14 +198,21 @@ __global__ void __launch_bounds__(32 * S) wkv4_forward_kernel(int T, int C, cons
         if (Y && plain && __all_sync(0xffffffffu, join(rg, s))) {
             const float fs = s.q != 0.f ? expf(s.o - rg.hi) : 0.f, fk = expf(base - rg.hi);
             float p = s.p * fs, q = s.q * fs;
+            float* yp = y_ + off + (i64)t0 * C;
+            auto token = [&](int i) {
+                const float x = e[i] * fk, xu = x * eu;
+                if (at.live) yp[i * C] = fmaf(xu, v[i], p) / (q + xu);
+                p = fmaf(p, ew, x * v[i]);
+                q = fmaf(q, ew, x);
+            };
+            if (full) {
 #pragma unroll
-            for (int i = 0; i < L; ++i)
-                if (i < n) {
-                    const float x = e[i] * fk, xu = x * eu;
-                    if (at.live) y_[off + (i64)(t0 + i) * C] = fmaf(xu, v[i], p) / (q + xu);
-                    p = fmaf(p, ew, x * v[i]);
-                    q = fmaf(q, ew, x);
-                }
+                for (int i = 0; i < L; ++i) token(i);
+            } else {
+#pragma unroll
+                for (int i = 0; i < L; ++i)
+                    if (i < n) token(i);
+            }
         } else if (Y && at.live) {
             forward_running_max(s, min(n, L), w, u, k_ + off + (i64)t0 * C, v_ + off + (i64)t0 * C, y_ + off + (i64)t0 * C, C);
         }
@@ -251,12 +266,16 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(i
     float gw = 0.f, gw_plain = 0.f, gu = 0.f;   // gw_plain: without the factor e^w
     for (int t0 = (T - 1) / (S * L) * (S * L) + warp * L; t0 >= 0; t0 -= S * L) {
         const int n = T - t0;
+        const bool full = n >= L;
+        const i64 o0 = off + (i64)t0 * C;
         float k[L], v[L], g[L];
+        {
+            const float *kp = k_ + o0, *vp = v_ + o0, *gp = gy_ + o0;
 #pragma unroll
-        for (int i = 0; i < L; ++i) {
-            const bool in = i < n;
-            const i64 o = off + (i64)(t0 + i) * C;
-            k[i] = in ? k_[o] : 0.f; v[i] = in ? v_[o] : 0.f; g[i] = in ? gy_[o] : 0.f;
+            for (int i = 0; i < L; ++i) {
+                const bool in = i < n;
+                k[i] = in ? kp[i * C] : 0.f; v[i] = in ? vp[i * C] : 0.f; g[i] = in ? gp[i * C] : 0.f;
+            }
         }
         Sum s = {0.f, 0.f, kNegInf};
         if (t0 > 0 && n > 0) {
@@ -264,7 +283,7 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(i
             s = Sum{p[0], p[C], p[2 * (i64)C]};
         }
         const Sum start = s;
-        Range rg = range_of(k, n);
+        Range rg = full ? range_of(k, L) : range_of(k, n);
         const bool plain = __all_sync(0xffffffffu, bonus_ok && join(rg, s));
         // forward inside the segment: the running sums before each token, y, and the token's term h (1, -y) of the adjoint (all in
         // units of the largest weight); then the adjoint that the segment adds by itself
@@ -284,9 +303,14 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(i
                 s.p = fmaf(s.p, ew, e[i] * v[i]);
                 s.q = fmaf(s.q, ew, e[i]);
             }
+            if (full) {
 #pragma unroll
-            for (int i = L - 1; i >= 0; --i)
-                if (i < n) { G.p = fmaf(G.p, ew, h[i]); G.q = fmaf(G.q, ew, -h[i] * y[i]); }
+                for (int i = L - 1; i >= 0; --i) { G.p = fmaf(G.p, ew, h[i]); G.q = fmaf(G.q, ew, -h[i] * y[i]); }
+            } else {
+#pragma unroll
+                for (int i = L - 1; i >= 0; --i)
+                    if (i < n) { G.p = fmaf(G.p, ew, h[i]); G.q = fmaf(G.q, ew, -h[i] * y[i]); }
+            }
             if (n > 0) G.o = -rg.hi;
         } else {
             // running-maximum form; y and log den are rebuilt by the reverse walk
@@ -308,19 +332,25 @@ __global__ void __launch_bounds__(32 * S, S == 8 ? 3 : 1) wkv4_backward_kernel(i
         if (plain && __all_sync(0xffffffffu, empty || fabsf(G.o + rg.hi) <= kSpan)) {
             const float f = empty ? 0.f : expf(G.o + rg.hi);
             float gp = G.p * f, gq = G.q * f;
-#pragma unroll
-            for (int i = L - 1; i >= 0; --i)
-                if (i < n) {
-                    const float A = h[i] * e[i] * eu;
-                    gw_plain = fmaf(gp, bp[i], fmaf(gq, bq[i], gw_plain));
-                    if (at.live) {
-                        const i64 o = off + (i64)(t0 + i) * C;
-                        gk_[o] = fmaf(A, v[i] - y[i], e[i] * fmaf(gp, v[i], gq));
-                        gv_[o] = fmaf(e[i], gp, A);
-                    }
-                    gp = fmaf(gp, ew, h[i]);
-                    gq = fmaf(gq, ew, -h[i] * y[i]);
+            float *gkp = gk_ + o0, *gvp = gv_ + o0;
+            auto token = [&](int i) {
+                const float A = h[i] * e[i] * eu;
+                gw_plain = fmaf(gp, bp[i], fmaf(gq, bq[i], gw_plain));
+                if (at.live) {
+                    gkp[i * C] = fmaf(A, v[i] - y[i], e[i] * fmaf(gp, v[i], gq));
+                    gvp[i * C] = fmaf(e[i], gp, A);
                 }
+                gp = fmaf(gp, ew, h[i]);
+                gq = fmaf(gq, ew, -h[i] * y[i]);
+            };
+            if (full) {
+#pragma unroll
+                for (int i = L - 1; i >= 0; --i) token(i);
+            } else {
+#pragma unroll
+                for (int i = L - 1; i >= 0; --i)
+                    if (i < n) token(i);
+            }
         } else {
             gw += reverse_running_max(start, G, min(n, L), w, u, k_ + off + (i64)t0 * C, v_ + off + (i64)t0 * C, gy_ + off + (i64)t0 * C,
                                       gk_ + off + (i64)t0 * C, gv_ + off + (i64)t0 * C, C, at.live);
