@@ -179,13 +179,17 @@ extern "C" int rwkvb200_wkv7_backward(int dtype, int B, int T, int H, int N, int
     if (tensor) {
         RWKV_REQUIRE(aligned16({r, w, k, v, a, b, dy, dsT, s, sa, ds0, dr, dw, dk, dv, da, db}), RWKVB200_EALIGN,
                      "wkv7_backward: the bf16 N=64 path needs 16-byte aligned tensors");
-        // at most one unit per SM: the time is one unit's chain of chunks, which the two-stage form (one thread
-        // block per SM, two warp groups on consecutive chunks) nearly halves; with more units per SM two
-        // independent one-group blocks per SM give more throughput
-        const int form = g_wkv7_bwd_form.load();
-        if (form == 2 || (form == 0 && (long long)B * H <= sm_count()))
-            return wkv7_l32_backward_pipelined(B, T, H, r, w, k, v, a, b, dy, dsT, s, ds0, dr, dw, dk, dv, da, db, as_stream(stream));
-        return wkv7_l32_backward(B, T, H, r, w, k, v, a, b, dy, dsT, s, ds0, dr, dw, dk, dv, da, db, as_stream(stream));
+        // Two independent one-group blocks per SM give the most throughput while every place has a unit (8.6 k cycles per chunk
+        // and SM); units that have an SM to themselves take the two-stage form (one block per SM, two warp groups on consecutive
+        // chunks: 8.8 k cycles per chunk against 13.3 k).  So the whole rounds of the one, then what is left over in the other
+        // where that is at most a unit per SM (B16 T4096 H64: 888 units and 136, 5650 -> 5516 us forward + backward; B8 H40, 296 and 24,
+        // 2566 -> 2403 us).  Short sequences have less to gain than a launch and the wait between the two cost (B16 T128: 239 -> 250 us).
+        const int form = g_wkv7_bwd_form.load(), units = B * H, sms = sm_count();
+        const int rest = form == 1 ? 0 : form == 2 ? units : units <= sms ? units : sms > 0 && T >= 512 && units % (2 * sms) <= sms ? units % (2 * sms) : 0;
+        if (units > rest)
+            if (int e = wkv7_l32_backward(B, T, H, 0, units - rest, r, w, k, v, a, b, dy, dsT, s, ds0, dr, dw, dk, dv, da, db, as_stream(stream))) return e;
+        if (rest == 0) return RWKVB200_OK;
+        return wkv7_l32_backward_pipelined(B, T, H, units - rest, rest, r, w, k, v, a, b, dy, dsT, s, ds0, dr, dw, dk, dv, da, db, as_stream(stream));
     }
     return wkv7_generic_backward(dtype, B, T, H, N, chunk_len, r, w, k, v, a, b, dy, dsT, s, sa, ds0, dr, dw, dk, dv,
                                  da, db, as_stream(stream));

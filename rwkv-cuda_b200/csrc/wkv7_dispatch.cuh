@@ -23,7 +23,8 @@ int wkv7_update64(int dtype, int B, int T, int H, float* state, const void* r, c
 // in flight: the product it waits for is not issued), to exercise the bounded-wait path.
 int wkv7_l32_forward(int B, int T, int H, const float* s0, const void* r, const void* w, const void* k, const void* v,
                      const void* a, const void* b, void* y, float* sT, float* s, int test_expire, cudaStream_t st);
-int wkv7_l32_backward(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
+// (backward: `units` of the B H (batch, head) units, from `first` on)
+int wkv7_l32_backward(int B, int T, int H, int first, int units, const void* r, const void* w, const void* k, const void* v, const void* a,
                       const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
                       void* dk, void* dv, void* da, void* db, cudaStream_t st);
 // The same kernel with a block per few chunks: adj = the adjoint at the end, states = the state at the start of every chunk,
@@ -42,8 +43,8 @@ int wkv7_scan_backward(int B, int T, int H, const void* r, const void* w, const 
                        void* da, void* db, cudaStream_t st);
 int wkv7_scan_error(int clear);
 // The backward as two warp groups working on consecutive chunks (one thread block per SM; same
-// products, results equal to rounding); for launches with at most one unit per SM.  Error word: read (clear = 0) or reset (clear = 1).
-int wkv7_l32_backward_pipelined(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
+// products, results equal to rounding); for the units that have an SM each.  Error word: read (clear = 0) or reset (clear = 1).
+int wkv7_l32_backward_pipelined(int B, int T, int H, int first, int units, const void* r, const void* w, const void* k, const void* v, const void* a,
                                 const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
                                 void* dk, void* dv, void* da, void* db, cudaStream_t st);
 int wkv7_l32_bwdp_error(int clear);

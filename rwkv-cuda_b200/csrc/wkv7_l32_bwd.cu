@@ -97,7 +97,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                       const bf16* __restrict__ b_, const bf16* __restrict__ dy_, const float* __restrict__ dsT_,
                       const float* __restrict__ ck_, float* __restrict__ ds0_, bf16* __restrict__ dr_,
                       bf16* __restrict__ dw_, bf16* __restrict__ dk_, bf16* __restrict__ dv_, bf16* __restrict__ da_,
-                      bf16* __restrict__ db_, const float* __restrict__ adj_, int group, const __grid_constant__ TileMaps<7> maps) {
+                      bf16* __restrict__ db_, const float* __restrict__ adj_, int group, int first, const __grid_constant__ TileMaps<7> maps) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);   // the swizzle acts on address bits
     unsigned char *AR = smem + BwdSmemX::kAR, *BK = smem + BwdSmemX::kBK, *SV = smem + BwdSmemX::kSV, *EY = smem + BwdSmemX::kEY;
@@ -113,7 +113,7 @@ wkv7x_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 8);
     unsigned char* Raw = smem + BwdSmemX::kRaw;
 
-    const int hh = blockIdx.x, bb = blockIdx.y;
+    const int hh = (first + blockIdx.x) % H, bb = (first + blockIdx.x) / H;
     const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int quarter = warp & 3, hs = warp >> 2;
@@ -555,7 +555,7 @@ WKV7_PHASE_READER(rwkvb200_phase_clocks_l32_bwd)
 
 }  // namespace v7x
 
-static int launch_l32_backward(int B, int T, int H, int group, const void* r, const void* w, const void* k, const void* v, const void* a,
+static int launch_l32_backward(int B, int T, int H, int group, int first, int units, const void* r, const void* w, const void* k, const void* v, const void* a,
                                const void* b, const void* dy, const float* dsT, const float* adj, const float* s, float* ds0, void* dr,
                                void* dw, void* dk, void* dv, void* da, void* db, cudaStream_t st) {
     using namespace v7x;
@@ -565,17 +565,17 @@ static int launch_l32_backward(int B, int T, int H, int group, const void* r, co
     const void* in[7] = {r, w, k, v, a, b, dy};
     make_tile_maps<7>(maps, in, B, T, H);
     const int groups = ((T + LC - 1) / LC + group - 1) / group;
-    wkv7x_backward_kernel<<<dim3(H, B, groups), BNT, BwdSmemX::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)w, (const bf16*)k,
+    wkv7x_backward_kernel<<<dim3(units, 1, groups), BNT, BwdSmemX::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)w, (const bf16*)k,
                                                                              (const bf16*)v, (const bf16*)a, (const bf16*)b,
                                                                              (const bf16*)dy, dsT, s, ds0, (bf16*)dr, (bf16*)dw, (bf16*)dk,
-                                                                             (bf16*)dv, (bf16*)da, (bf16*)db, adj, group, maps);
+                                                                             (bf16*)dv, (bf16*)da, (bf16*)db, adj, group, first, maps);
     return check_launch("wkv7_backward(tcgen05, 32-token chunks)");
 }
 
-int wkv7_l32_backward(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
+int wkv7_l32_backward(int B, int T, int H, int first, int units, const void* r, const void* w, const void* k, const void* v, const void* a,
                       const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
                       void* dk, void* dv, void* da, void* db, cudaStream_t st) {
-    return launch_l32_backward(B, T, H, (T + v7x::LC - 1) / v7x::LC, r, w, k, v, a, b, dy, dsT, nullptr, s, ds0, dr, dw, dk, dv, da, db, st);
+    return launch_l32_backward(B, T, H, (T + v7x::LC - 1) / v7x::LC, first, units, r, w, k, v, a, b, dy, dsT, nullptr, s, ds0, dr, dw, dk, dv, da, db, st);
 }
 
 int wkv7_l32_backward_chunks(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
@@ -592,7 +592,7 @@ int wkv7_l32_backward_chunks(int B, int T, int H, const void* r, const void* w, 
         const double cost = (double)((blocks + places - 1) / places) * (g + 0.5);
         if (cost < best) { best = cost; group = g; }
     }
-    return launch_l32_backward(B, T, H, group, r, w, k, v, a, b, dy, nullptr, adj, states, nullptr, dr, dw, dk, dv, da, db, st);
+    return launch_l32_backward(B, T, H, group, 0, B * H, r, w, k, v, a, b, dy, nullptr, adj, states, nullptr, dr, dw, dk, dv, da, db, st);
 }
 
 int wkv7_l32_bwd_error_clear() {

@@ -124,7 +124,7 @@ wkv7p_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
                       const bf16* __restrict__ b_, const bf16* __restrict__ dy_, const float* __restrict__ dsT_,
                       const float* __restrict__ ck_, float* __restrict__ ds0_, bf16* __restrict__ dr_,
                       bf16* __restrict__ dw_, bf16* __restrict__ dk_, bf16* __restrict__ dv_, bf16* __restrict__ da_,
-                      bf16* __restrict__ db_, const __grid_constant__ TileMaps<7> maps) {
+                      bf16* __restrict__ db_, int first, const __grid_constant__ TileMaps<7> maps) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     float* A0p = reinterpret_cast<float*>(smem + PipeSmem::kA0);
@@ -136,7 +136,7 @@ wkv7p_backward_kernel(int T, int H, const bf16* __restrict__ r_, const bf16* __r
     volatile int* raw_req = gabort + 2;      // [2]: tile requests issued per set;  raw_got = raw_req + 2: [2] requests whose tiles were taken
     volatile int* raw_got = raw_req + 2;
 
-    const int hh = blockIdx.x, bb = blockIdx.y;
+    const int hh = (first + blockIdx.x) % H, bb = (first + blockIdx.x) / H;
     const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int grp = warp >> 3, wg = warp & 7, gtid = tid & (GNT - 1);   // group, warp and thread inside the group
@@ -636,7 +636,7 @@ WKV7_PHASE_READER(rwkvb200_phase_clocks_l32_bwdp)
 
 }  // namespace v7p
 
-int wkv7_l32_backward_pipelined(int B, int T, int H, const void* r, const void* w, const void* k, const void* v, const void* a,
+int wkv7_l32_backward_pipelined(int B, int T, int H, int first, int units, const void* r, const void* w, const void* k, const void* v, const void* a,
                                 const void* b, const void* dy, const float* dsT, const float* s, float* ds0, void* dr, void* dw,
                                 void* dk, void* dv, void* da, void* db, cudaStream_t st) {
     using namespace v7p;
@@ -645,11 +645,10 @@ int wkv7_l32_backward_pipelined(int B, int T, int H, const void* r, const void* 
     TileMaps<7> maps;
     const void* in[7] = {r, w, k, v, a, b, dy};
     make_tile_maps<7>(maps, in, B, T, H);
-    dim3 grid(H, B);
-    wkv7p_backward_kernel<<<grid, PNT, PipeSmem::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)w, (const bf16*)k,
+    wkv7p_backward_kernel<<<units, PNT, PipeSmem::kBytes, st>>>(T, H, (const bf16*)r, (const bf16*)w, (const bf16*)k,
                                                                (const bf16*)v, (const bf16*)a, (const bf16*)b, (const bf16*)dy,
                                                                dsT, s, ds0, (bf16*)dr, (bf16*)dw, (bf16*)dk, (bf16*)dv,
-                                                               (bf16*)da, (bf16*)db, maps);
+                                                               (bf16*)da, (bf16*)db, first, maps);
     return check_launch("wkv7_backward(tcgen05, 32-token chunks, two stages)");
 }
 
