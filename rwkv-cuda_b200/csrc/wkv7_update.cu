@@ -9,16 +9,20 @@
 // wkv7_rows_kernel, T > 1 (prompts of any length).  The recurrence of one value row
 //     sa_t = S_{t-1}.a_t      S_t = S_{t-1} d_t + sa_t b_t + v_t k_t      y_t = S_t.r_t
 // needs nothing of the other 63 rows, so a unit is spread over 1 to 4 blocks; what bounds a launch with few units is the
-// chain from one token's sa to the next (a dot product over 64 keys and its reduction over lanes) and, with many rows on
-// an SM, the shared-memory reads of the token's vectors (2 / RPT wavefronts per row and vector whatever the lane split).
-// Against the chain: 8 or 16 lanes own a row, and the dot product runs one token ahead of sa: with
-// G_t = S_{t-1} d_t + v_t k_t (no sa_t in it) and beta_t = b_t.a_{t+1} (one scalar per token),
-//     sa_{t+1} = G_t.a_{t+1} + sa_t beta_t          S_t = G_t + sa_t b_t
-// so the reduction of token t+1 overlaps the update of token t.  Against the reads: RPT rows per thread.
-// NCW warps compute, four stage the next 16 tokens in shared memory (fp32: d, b, k, r, v of token t and a of token t+1)
-// behind named barriers.  Multiply-adds are packed in pairs (fma.rn.f32x2), y is reduced for eight tokens at a time.
-// One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 212 us here (106 ns per token); 256 units
-// 2045 -> 870 us.
+// chain from one dot product over 64 keys, with its reduction over lanes, to the next, and, with many rows on an SM, the
+// shared-memory reads of the tokens' vectors (2 / RPT wavefronts per row and vector whatever the lane split).
+// So four tokens are one step.  With W_t = d_0 .. d_t inside the step (t = 0 .. 3)
+//     a~_t = a_t W_{t-1}    r~_t = r_t W_t    b^_s = b_s d_{s+1} .. d_3    k^_s = k_s d_{s+1} .. d_3
+//     sa_t = S.a~_t + sum_{s<t} sa_s Ub[s,t] + v_s Uk[s,t]         Ub[s,t] = b_s.(a_t d_{s+1} .. d_{t-1}), Uk with k_s
+//     y_t  = S.r~_t + sum_{s<=t} sa_s Rb[s,t] + v_s Rk[s,t]        Rb[s,t] = b_s.(r_t d_{s+1} .. d_t), Rk with k_s
+//     S   <- S W_3 + sum_s sa_s b^_s + v_s k^_s
+// the eight dot products of a row are reduced together (8 shuffles, not 4 per token), 17 vectors are read instead of 20, and the
+// chain has one reduction per four tokens.  NCW warps compute; NSW warps stage, a step each: they make the scaled vectors (products of
+// decays are carried as sums of two numbers: a vector is rounded once) and the 32 scalars of a step, which all rows share.
+// One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 213 us with a token as a step, 201 us here; 128 units
+// 427 -> 375 us, 256 units 852 -> 660 us.  A step takes 790 clocks where a unit has four SMs: 350 of the shared-memory reads, the
+// rest the latency of 260 instructions of one warp per scheduler; eight staging warps instead of four change nothing there.
+// Errors of the state against fp64 9.1e-8 of the norm (a token as a step 8.3e-8: the same fp32 sums in another order), y as before.
 #include "common.cuh"
 #include "packed.cuh"
 #include "wkv7_dispatch.cuh"
@@ -88,7 +92,6 @@ __global__ void __launch_bounds__(128) wkv7_decode_kernel(float* __restrict__ st
 // ---- prompts ----------------------------------------------------------------------------------------------
 // The 64 / LG keys of lane x of a row (LG = 8 or 16 lanes).  In shared memory the first four of every eight keys come
 // first, then the other four, so that eight lanes read and write 128 consecutive bytes: staged_at(key) is the place.
-__device__ __forceinline__ int staged_at(int ch) { return ((ch & 4) << 3) + ((ch >> 3) << 2) + (ch & 3); }
 template <int LG>
 __device__ __forceinline__ int first_key(int x) { return LG == 8 ? 8 * x : 8 * (x & 7) + ((x & 8) >> 1); }
 template <int LG>
@@ -110,46 +113,36 @@ __device__ __forceinline__ float dot_keys(const f2 (&s)[32 / LG], const Keys<LG>
     for (int e = 1; e < 32 / LG; ++e) acc = fma2(s[e], a.x[e], acc);
     return sum2(acc);
 }
-template <int LG>
-__device__ __forceinline__ float row_sum(float x) {
-#pragma unroll
-    for (int m = 1; m < LG; m <<= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
-    return x;
-}
+constexpr int kQ = 4;   // tokens of a step
+// The scaled vectors of a step, the products of its decays (w), its values, and the scalars of the steps inside it: b, k of token s
+// against a of token t (s < t) at ((t - 1) t / 2 + s) * 2, then against r of token t (s <= t, zero above) at 12 + 8 t + 2 s.
+struct __align__(16) Step { float a[kQ][kN], r[kQ][kN], b[kQ][kN], k[kQ][kN], w[kN], v[kQ][kN], u[12 + 8 * kQ]; };
+template <int NSW>
+struct __align__(16) Staged { Step s[NSW]; };   // a step per staging warp
 
-constexpr int kCh = 16;                              // tokens staged at a time
-struct __align__(16) Token { float d[kN], b[kN], k[kN], r[kN], an[kN], v[kN]; };
-struct __align__(16) Staged { Token t[kCh]; float beta[kCh]; };
-constexpr int kRowsSmem = 2 * sizeof(Staged);
-
-// 8 consecutive elements as loaded, and decoded
+// Two neighbouring elements, as loaded and decoded
+template <typename E> struct Pair2;
+template <> struct Pair2<bf16> { uint32_t x; };
+template <> struct Pair2<float> { float2 x; };
 template <typename E>
-struct Raw8 { uint4 q[sizeof(E) / 2]; };
-template <typename E>
-__device__ __forceinline__ Raw8<E> load8(const E* p, bool in) {
-    Raw8<E> x;
-#pragma unroll
-    for (int i = 0; i < (int)sizeof(E) / 2; ++i) x.q[i] = in ? __ldg(reinterpret_cast<const uint4*>(p) + i) : make_uint4(0u, 0u, 0u, 0u);
-    return x;
+__device__ __forceinline__ Pair2<E> load2(const E* p, bool in) {
+    Pair2<E> r;
+    if constexpr (sizeof(E) == 2) r.x = in ? __ldg(reinterpret_cast<const uint32_t*>(p)) : 0u;
+    else r.x = in ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(0.f, 0.f);
+    return r;
 }
-__device__ __forceinline__ void decode8(const Raw8<float>& p, float (&x)[8]) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        x[4 * i] = __uint_as_float(p.q[i].x); x[4 * i + 1] = __uint_as_float(p.q[i].y);
-        x[4 * i + 2] = __uint_as_float(p.q[i].z); x[4 * i + 3] = __uint_as_float(p.q[i].w);
-    }
+__device__ __forceinline__ float2 decode2(Pair2<bf16> p) { return make_float2(__uint_as_float(p.x << 16), __uint_as_float(p.x & 0xffff0000u)); }
+__device__ __forceinline__ float2 decode2(Pair2<float> p) { return p.x; }
+__device__ __forceinline__ float2 times(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
+struct Exact2 { float2 hi, lo; };   // hi + lo, for two keys
+__device__ __forceinline__ float2 times(float2 a, Exact2 b) { return make_float2(fmaf(a.x, b.hi.x, a.x * b.lo.x), fmaf(a.y, b.hi.y, a.y * b.lo.y)); }
+__device__ __forceinline__ Exact2 times(Exact2 a, float2 b) {
+    const float2 h = times(a.hi, b);
+    return Exact2{h, make_float2(fmaf(a.lo.x, b.x, fmaf(a.hi.x, b.x, -h.x)), fmaf(a.lo.y, b.y, fmaf(a.hi.y, b.y, -h.y)))};
 }
-__device__ __forceinline__ void decode8(const Raw8<bf16>& p, float (&x)[8]) {
-    const uint32_t u[4] = {p.q[0].x, p.q[0].y, p.q[0].z, p.q[0].w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { x[2 * i] = __uint_as_float(u[i] << 16); x[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u); }
-}
+__device__ __forceinline__ float dot2(float2 a, float2 b) { return fmaf(a.y, b.y, a.x * b.x); }
 __device__ __forceinline__ void prefetch_l2(const void* p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p)));
-}
-__device__ __forceinline__ void store8(float* row, int l8, const float (&x)[8]) {
-    *reinterpret_cast<float4*>(row + 4 * l8) = make_float4(x[0], x[1], x[2], x[3]);
-    *reinterpret_cast<float4*>(row + 32 + 4 * l8) = make_float4(x[4], x[5], x[6], x[7]);
 }
 // named barriers ID + odd (constants: a barrier number in a register makes the block reserve all sixteen)
 template <int ID, int NTH>
@@ -162,128 +155,235 @@ __device__ __forceinline__ void bar_arrive(int odd) {
     if (odd) asm volatile("bar.arrive %0, %1;" ::"n"(ID + 1), "n"(NTH) : "memory");
     else asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(NTH) : "memory");
 }
+// Sums of v[0..7] over LG lanes: lane x ends with the sum of v[x >> 1] (16 lanes) or v[x] (8 lanes).
+template <int LG>
+__device__ __forceinline__ float reduce8_over(float (&v)[8], int x) {
+#pragma unroll
+    for (int m = LG / 2, n = 4; n >= 1; m >>= 1, n >>= 1) {
+        const bool up = (x & m) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+        }
+    }
+    return LG == 16 ? v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1) : v[0];
+}
+// RPT neighbouring outputs
+template <typename E, int RPT>
+__device__ __forceinline__ void store_rows(E* p, const float (&y)[RPT]) {
+    if constexpr (sizeof(E) == 2) {
+        uint32_t w[RPT / 2];
+#pragma unroll
+        for (int i = 0; i < RPT / 2; ++i) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(y[2 * i], y[2 * i + 1]);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        if constexpr (RPT == 2) *reinterpret_cast<uint32_t*>(p) = w[0];
+        else *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+    } else {
+        if constexpr (RPT == 2) *reinterpret_cast<float2*>(p) = make_float2(y[0], y[1]);
+        else *reinterpret_cast<float4*>(p) = make_float4(y[0], y[1], y[2], y[3]);
+    }
+}
 
-// grid (units, 64 / (16 RPT)); 4 compute warps (a warp: 4 groups of 8 lanes, RPT rows each) and 4 staging warps
-template <typename E, int LG, int NCW, int RPT>
-__global__ void __launch_bounds__(32 * (NCW + 4)) wkv7_rows_kernel(int T, int H, float* __restrict__ state, const E* __restrict__ r_,
+// grid (units, 64 LG / (32 NCW RPT)); NCW warps compute (a warp: 32 / LG groups of LG lanes, RPT rows each), NSW warps stage
+template <typename E, int LG, int NCW, int RPT, int NSW>
+__global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int H, float* __restrict__ state, const E* __restrict__ r_,
                                                         const E* __restrict__ w_, const E* __restrict__ k_, const E* __restrict__ v_,
                                                         const E* __restrict__ a_, const E* __restrict__ b_, E* __restrict__ y_) {
     extern __shared__ __align__(16) unsigned char smem_rows[];
-    Staged* buf = reinterpret_cast<Staged*>(smem_rows);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l8 = lane & 7;
+    constexpr int kCh = NSW * kQ, NTH = 32 * (NCW + NSW);   // tokens staged at a time
+    Staged<NSW>* buf = reinterpret_cast<Staged<NSW>*>(smem_rows);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int unit = blockIdx.x, C = H * kN;
     const i64 base = (i64)(unit / H) * T * C + (unit % H) * kN;
     const int nch = (T + kCh - 1) / kCh;
-    constexpr int NTH = 32 * (NCW + 4);
 
     if (warp >= NCW) {
-        // ---- staging: this lane has keys 8 l8 .. of token 4 (warp - NCW) + lane / 8 of every chunk --------------
-        // (in registers one chunk ahead of the stores, asked for in L2 four chunks ahead)
-        const int q = 4 * (warp - NCW) + (lane >> 3);
-        const E* src[6] = {w_, b_, k_, r_, v_, a_ + C};   // a: of the token after
-        const i64 o0 = base + (i64)q * C + 8 * l8;
-        Raw8<E> raw[6];
+        // ---- staging: a step of every chunk per warp, two keys per lane (those of the places 2 lane, 2 lane + 1 of a staged row) ----
+        // (in registers one chunk ahead of the stores, asked for in L2 64 tokens ahead)
+        const int q = warp - NCW, key = lane < 16 ? 8 * (lane >> 1) + 2 * (lane & 1) : 8 * ((lane - 16) >> 1) + 4 + 2 * (lane & 1);
+        const E* src[6] = {w_, a_, b_, k_, r_, v_};
+        const i64 o0 = base + (i64)q * kQ * C;
+        Pair2<E> raw[6][kQ];
         auto fetch = [&](int c) {
-            const int t = c * kCh + q;
-            const i64 o = o0 + (i64)c * kCh * C;
+            const int t = c * kCh + q * kQ;
+            const i64 o = o0 + (i64)c * kCh * C + key;
 #pragma unroll
-            for (int x = 0; x < 6; ++x) raw[x] = load8(src[x] + o, t + (x == 5) < T);
-            if (t + 4 * kCh + 1 < T && (l8 & (64 / sizeof(E) / 8 * 2 - 1)) == 0)   // one lane per 128-byte line
+            for (int x = 0; x < 6; ++x)
 #pragma unroll
-                for (int x = 0; x < 6; ++x) prefetch_l2(src[x] + o + (i64)4 * kCh * C);
+                for (int i = 0; i < kQ; ++i) raw[x][i] = load2(src[x] + o + (i64)i * C, t + i < T);
+            if (lane < 24 && t + 64 + (lane & 3) < T) {   // one row per lane: 128 or 256 bytes
+                const E* p = lane < 4 ? w_ : lane < 8 ? a_ : lane < 12 ? b_ : lane < 16 ? k_ : lane < 20 ? r_ : v_;
+                p += o0 + (i64)(c * kCh + 64 + (lane & 3)) * C;
+                prefetch_l2(p);
+                if (sizeof(E) == 4) prefetch_l2(p + 32);
+            }
         };
+        if (lane < 12) {   // the scalars above the diagonal: zero, and never written again
+            const int t = lane < 6 ? 0 : lane < 10 ? 1 : 2, x = lane - (lane < 6 ? 0 : lane < 10 ? 6 : 10);
+            buf[0].s[q].u[12 + 8 * t + 2 * (t + 1) + x] = buf[1].s[q].u[12 + 8 * t + 2 * (t + 1) + x] = 0.f;
+        }
+        const int yt = lane >= 24 ? 3 : lane >= 18 ? 2 : lane >= 14 ? 1 : 0, slot = lane < 12 ? lane : 12 + 8 * yt + lane - (yt == 3 ? 24 : yt == 2 ? 18 : yt == 1 ? 14 : 12);
         fetch(0);
         for (int c = 0; c < nch; ++c) {
-            const bool in = c * kCh + q < T;
-            float w[8], b[8], k[8], r[8], v[8], an[8];
-            decode8(raw[0], w); decode8(raw[1], b); decode8(raw[2], k); decode8(raw[3], r); decode8(raw[4], v); decode8(raw[5], an);
+            const int t0 = c * kCh + q * kQ;
+            float2 d[kQ], a[kQ], b[kQ], k[kQ], r[kQ], v[kQ];
+#pragma unroll
+            for (int i = 0; i < kQ; ++i) {
+                const float2 w = decode2(raw[0][i]);
+                d[i] = t0 + i < T ? make_float2(decay7(w.x), decay7(w.y)) : make_float2(1.f, 1.f);
+                a[i] = decode2(raw[1][i]); b[i] = decode2(raw[2][i]); k[i] = decode2(raw[3][i]); r[i] = decode2(raw[4][i]); v[i] = decode2(raw[5][i]);
+            }
             if (c + 1 < nch) fetch(c + 1);
-            float beta = 0.f;
+            // every pair of tokens: b_s, k_s times the decays between s and t, against a_t (without token t's) and r_t (with it)
+            float u[32];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) { w[i] = in ? decay7(w[i]) : 1.f; beta = fmaf(b[i], an[i], beta); }
+            for (int s = 0; s < kQ; ++s) {
+                float2 p = b[s], z = k[s];
+                constexpr int first[kQ] = {12, 14, 18, 24};
+                u[first[s] + 2 * s] = dot2(p, r[s]);
+                u[first[s] + 2 * s + 1] = dot2(z, r[s]);
 #pragma unroll
-            for (int m = 1; m < 8; m <<= 1) beta += __shfl_xor_sync(0xffffffffu, beta, m);
+                for (int t = s + 1; t < kQ; ++t) {
+                    u[(t - 1) * t + 2 * s] = dot2(p, a[t]);
+                    u[(t - 1) * t + 2 * s + 1] = dot2(z, a[t]);
+                    p = times(p, d[t]);
+                    z = times(z, d[t]);
+                    u[first[t] + 2 * s] = dot2(p, r[t]);
+                    u[first[t] + 2 * s + 1] = dot2(z, r[t]);
+                }
+            }
+            // the vectors of the step, with the decays of the tokens before them (a, r) and behind them (b, k): products of decays as
+            // sums of two numbers, so that a vector is rounded once
+            Exact2 w{d[0], make_float2(0.f, 0.f)}, e{d[kQ - 1], make_float2(0.f, 0.f)};
+            r[0] = times(r[0], d[0]);
+#pragma unroll
+            for (int t = 1; t < kQ; ++t) {
+                a[t] = times(a[t], w);
+                w = times(w, d[t]);
+                r[t] = times(r[t], w);
+            }
+#pragma unroll
+            for (int s = kQ - 2; s >= 0; --s) {
+                b[s] = times(b[s], e);
+                k[s] = times(k[s], e);
+                if (s > 0) e = times(e, d[s]);
+            }
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1) {   // sums over the lanes: lane x ends with u[x]
+                const bool up = (lane & m) != 0;
+#pragma unroll
+                for (int i = 0; i < m; ++i) {
+                    const float send = up ? u[i] : u[i + m], keep = up ? u[i + m] : u[i];
+                    u[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+                }
+            }
             if (c >= 2) bar_sync<3, NTH>(c & 1);   // the compute warps are done with the chunk before last
-            Staged& s = buf[c & 1];
-            Token& d = s.t[q];
-            store8(d.d, l8, w); store8(d.b, l8, b); store8(d.k, l8, k);
-            store8(d.r, l8, r); store8(d.an, l8, an); store8(d.v, l8, v);
-            if (l8 == 0) s.beta[q] = beta;
+            Step& st = buf[c & 1].s[q];
+#pragma unroll
+            for (int i = 0; i < kQ; ++i) {
+                *reinterpret_cast<float2*>(st.a[i] + 2 * lane) = a[i];
+                *reinterpret_cast<float2*>(st.r[i] + 2 * lane) = r[i];
+                *reinterpret_cast<float2*>(st.b[i] + 2 * lane) = b[i];
+                *reinterpret_cast<float2*>(st.k[i] + 2 * lane) = k[i];
+                *reinterpret_cast<float2*>(st.v[i] + key) = v[i];
+            }
+            *reinterpret_cast<float2*>(st.w + 2 * lane) = make_float2(w.hi.x + w.lo.x, w.hi.y + w.lo.y);
+            st.u[slot] = u[0];
             bar_arrive<1, NTH>(c & 1);
         }
         return;
     }
 
-    // ---- the recurrence: RPT rows per group of LG lanes -----------------------------------------------------------
-    constexpr int GPW = 32 / LG, KP = 32 / LG;   // groups of a warp; pairs of keys of a lane
+    // ---- the recurrence: RPT rows per group of LG lanes, four tokens per step -------------------------------------------------------
+    constexpr int GPW = 32 / LG, KP = 32 / LG, TS = LG / 8;   // groups of a warp; pairs of keys of a lane; lanes per sum
     const int x = lane & (LG - 1), row0 = ((blockIdx.y * NCW + warp) * GPW + lane / LG) * RPT;
     float* st = state + (i64)unit * kN * kN + row0 * kN + first_key<LG>(x);
     f2 S[RPT][KP];
-    float sa[RPT];
-    {
-        Keys<LG> a;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
 #pragma unroll
         for (int h = 0; h < KP / 2; ++h) {
-            const float4 q = load4(a_ + base + first_key<LG>(x) + 4 * h);
-            a.x[2 * h] = pack2(q.x, q.y); a.x[2 * h + 1] = pack2(q.z, q.w);
+            const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(st + i * kN + 4 * h);
+            S[i][2 * h] = p.x; S[i][2 * h + 1] = p.y;
         }
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-#pragma unroll
-            for (int h = 0; h < KP / 2; ++h) {
-                const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(st + i * kN + 4 * h);
-                S[i][2 * h] = p.x; S[i][2 * h + 1] = p.y;
-            }
-            sa[i] = row_sum<LG>(dot_keys<LG>(S[i], a));
-        }
-    }
     for (int c = 0; c < nch; ++c) {
         bar_sync<1, NTH>(c & 1);
-        const Staged& s = buf[c & 1];
 #pragma unroll 1
-        for (int half = 0; half < 2; ++half) {
-            float yp[RPT][8];
+        for (int q = 0; q < kCh / kQ; ++q) {
+            const Step& s = buf[c & 1].s[q];
+            float p[RPT][8];   // S.r~_t, S.a~_t: parts of this lane
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const Token& tk = s.t[8 * half + q];
-                const float beta = s.beta[8 * half + q];
-                const Keys<LG> d = load_keys<LG>(tk.d, x), k = load_keys<LG>(tk.k, x), an = load_keys<LG>(tk.an, x), b = load_keys<LG>(tk.b, x),
-                               r = load_keys<LG>(tk.r, x);
-                float z[RPT];
+            for (int t = 0; t < kQ; ++t) {
+                const Keys<LG> a = load_keys<LG>(s.a[t], x), r = load_keys<LG>(s.r[t], x);
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) { p[i][4 + t] = dot_keys<LG>(S[i], a); p[i][t] = dot_keys<LG>(S[i], r); }
+            }
+            float own[RPT];
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) own[i] = reduce8_over<LG>(p[i], x);
+            // while these are under way: S <- S w + sum v_s k^_s
+            float v[kQ][RPT];
+            {
+                const Keys<LG> w = load_keys<LG>(s.w, x);
+#pragma unroll
+                for (int i = 0; i < RPT; ++i)
+#pragma unroll
+                    for (int e = 0; e < KP; ++e) S[i][e] = mul2(S[i][e], w.x[e]);
+            }
+#pragma unroll
+            for (int t = 0; t < kQ; ++t) {
+                const Keys<LG> k = load_keys<LG>(s.k[t], x);
 #pragma unroll
                 for (int i = 0; i < RPT; ++i) {
-                    const float v = tk.v[staged_at(row0 + i)];
-                    const f2 vv = pack2(v, v);
+                    v[t][i] = s.v[t][row0 + i];
+                    const f2 vv = pack2(v[t][i], v[t][i]);
 #pragma unroll
-                    for (int e = 0; e < KP; ++e) S[i][e] = fma2(S[i][e], d.x[e], mul2(k.x[e], vv));   // G_t
-                    z[i] = dot_keys<LG>(S[i], an);
-                }
-#pragma unroll
-                for (int i = 0; i < RPT; ++i) {
-                    const f2 sv = pack2(sa[i], sa[i]);
-#pragma unroll
-                    for (int e = 0; e < KP; ++e) S[i][e] = fma2(sv, b.x[e], S[i][e]);                 // S_t
-                    yp[i][q] = dot_keys<LG>(S[i], r);
-                    sa[i] = fmaf(sa[i], beta, row_sum<LG>(z[i]));                                     // sa_{t+1}
+                    for (int e = 0; e < KP; ++e) S[i][e] = fma2(k.x[e], vv, S[i][e]);
                 }
             }
-            // sums over the lanes of a row for 8 tokens: every lane of a row ends with one token (pairs of lanes when LG = 16)
-            constexpr int TS = LG / 8;
-            const int t = c * kCh + 8 * half + x / TS;
+            float u[12], g[8];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) *reinterpret_cast<float4*>(u + 4 * i) = *reinterpret_cast<const float4*>(s.u + 4 * i);
+            const int ty = (x / TS) & 3;   // the token whose y this lane makes (lanes with an S.a~ repeat one)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) *reinterpret_cast<float4*>(g + 4 * i) = *reinterpret_cast<const float4*>(s.u + 12 + 8 * ty + 4 * i);
+            float sa[kQ][RPT];
 #pragma unroll
             for (int i = 0; i < RPT; ++i) {
+                float z[kQ];
 #pragma unroll
-                for (int m = 4; m >= 1; m >>= 1) {
-                    const bool up = (x & (m * TS)) != 0;
+                for (int t = 0; t < kQ; ++t) z[t] = __shfl_sync(0xffffffffu, own[i], (4 + t) * TS, LG);
 #pragma unroll
-                    for (int e = 0; e < m; ++e) {
-                        const float send = up ? yp[i][e] : yp[i][e + m], keep = up ? yp[i][e + m] : yp[i][e];
-                        yp[i][e] = keep + __shfl_xor_sync(0xffffffffu, send, m * TS);
-                    }
+                for (int t = 0; t < kQ; ++t) {
+#pragma unroll
+                    for (int e = 0; e < t; ++e) z[t] = fmaf(v[e][i], u[(t - 1) * t + 2 * e + 1], z[t]);
+#pragma unroll
+                    for (int e = 0; e < t; ++e) z[t] = fmaf(sa[e][i], u[(t - 1) * t + 2 * e], z[t]);
+                    sa[t][i] = z[t];
                 }
-                if (LG == 16) yp[i][0] += __shfl_xor_sync(0xffffffffu, yp[i][0], 1);
-                if (t < T && x % TS == 0) y_[base + (i64)t * C + row0 + i] = from_f<E>(yp[i][0]);
             }
+#pragma unroll
+            for (int t = 0; t < kQ; ++t) {
+                const Keys<LG> b = load_keys<LG>(s.b[t], x);
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) {
+                    const f2 sv = pack2(sa[t][i], sa[t][i]);
+#pragma unroll
+                    for (int e = 0; e < KP; ++e) S[i][e] = fma2(b.x[e], sv, S[i][e]);
+                }
+            }
+            float y[RPT];
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) {
+                y[i] = own[i];
+#pragma unroll
+                for (int e = 0; e < kQ; ++e) y[i] = fmaf(sa[e][i], g[2 * e], fmaf(v[e][i], g[2 * e + 1], y[i]));
+            }
+            const int t = c * kCh + kQ * q + ty;
+            if (x < 4 * TS && x % TS == 0 && t < T) store_rows<E, RPT>(y_ + base + (i64)t * C + row0, y);
         }
         if (c + 2 < nch) bar_arrive<3, NTH>(c & 1);
     }
@@ -293,12 +393,13 @@ __global__ void __launch_bounds__(32 * (NCW + 4)) wkv7_rows_kernel(int T, int H,
         for (int h = 0; h < KP / 2; ++h) *reinterpret_cast<ulonglong2*>(st + i * kN + 4 * h) = make_ulonglong2(S[i][2 * h], S[i][2 * h + 1]);
 }
 
-template <typename E, int LG, int NCW, int RPT>
+template <typename E, int LG, int NCW, int RPT, int NSW>
 int launch_rows(int B, int T, int H, float* state, const void* r, const void* w, const void* k, const void* v, const void* a,
                 const void* b, void* y, cudaStream_t st) {
-    const cudaError_t e = allow_smem<wkv7_rows_kernel<E, LG, NCW, RPT>>(kRowsSmem);
+    constexpr int smem = 2 * sizeof(Staged<NSW>);
+    const cudaError_t e = allow_smem<wkv7_rows_kernel<E, LG, NCW, RPT, NSW>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv7_state_update: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    wkv7_rows_kernel<E, LG, NCW, RPT><<<dim3(B * H, kN * LG / (32 * NCW * RPT)), 32 * (NCW + 4), kRowsSmem, st>>>(
+    wkv7_rows_kernel<E, LG, NCW, RPT, NSW><<<dim3(B * H, kN * LG / (32 * NCW * RPT)), 32 * (NCW + NSW), smem, st>>>(
         T, H, state, (const E*)r, (const E*)w, (const E*)k, (const E*)v, (const E*)a, (const E*)b, (E*)y);
     return check_launch("wkv7_state_update(rows)");
 }
@@ -311,12 +412,12 @@ int update(int B, int T, int H, float* state, const void* r, const void* w, cons
         return check_launch("wkv7_state_update(decode)");
     }
     // The fewest rows per block that still give every block an SM of its own (blocks that share one share its shared-memory
-    // bandwidth: 64 units in blocks of 16 rows take 356 us, in blocks of 32 rows 284 us); with more units than SMs / 2 the
-    // most rows per thread, which read every staged vector for four rows (T = 1999: 128 units 480 us, 256 units 870 us).
+    // bandwidth: with a token as a step 64 units took 356 us in blocks of 16 rows and 284 us in blocks of 32); with more units than
+    // SMs / 2 the most rows per thread, which read every staged vector for four rows.
     const int units = B * H;
-    if (units * 4 <= sms) return launch_rows<E, 16, 4, 2>(B, T, H, state, r, w, k, v, a, b, y, st);
-    if (units * 2 <= sms) return launch_rows<E, 8, 4, 2>(B, T, H, state, r, w, k, v, a, b, y, st);
-    return launch_rows<E, 8, 4, 4>(B, T, H, state, r, w, k, v, a, b, y, st);
+    if (units * 4 <= sms) return launch_rows<E, 16, 4, 2, 4>(B, T, H, state, r, w, k, v, a, b, y, st);
+    if (units * 2 <= sms) return launch_rows<E, 8, 4, 2, 4>(B, T, H, state, r, w, k, v, a, b, y, st);
+    return launch_rows<E, 8, 4, 4, 4>(B, T, H, state, r, w, k, v, a, b, y, st);
 }
 
 }  // namespace
