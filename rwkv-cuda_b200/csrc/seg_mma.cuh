@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 
 // States at the start of every segment (REV: adjoints at the end), one block per unit walking its segments: S <- S diag(f) + k'^T V
 // with k'_s = k_s exp(L_end - L_s) (REV: r'_t = r_t exp(L_{t-1}), gy): all factors are at most 1.  Warps 0 to 3 have the state in
-// registers, 16 keys each, warps 4 to 11 make the operands of the segments to come (B8 T1000 H32 bf16: 80 us with four of them, 72 with
+// registers, 16 keys each, warps 4 to 11 make the operands of the segments to come (B8 T1000 H32 bf16: 80 us with four of them, 68 with
 // eight and rows asked for in L2 six segments ahead: 1.8 TB/s; the walk waits for instructions of the operands and for barriers).
 template <typename E>
 struct ChainSmem {
@@ -885,25 +885,35 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
         bar_join<1>(it & 1);
         const ChainSmem<E>& sm = buf[it & 1];
         const float f0 = sm.f[16 * warp + g], f1 = sm.f[16 * warp + g + 8];
-        uint32_t a[2][1][3][4];
+        // bf16: straight onto the state, eight sums side by side; fp32: products apart (see mma_split)
+        float c[4][1][2][4];
 #pragma unroll
-        for (int kt = 0; kt < 2; ++kt) ldsm_t<3>(a[kt][0], smem_addr(sm.A) + frag_cols(16 * kt, 2 * warp, lane));
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float c[1][2][4];   // (summed apart from the state: the tensor core's sums are not rounded to nearest)
+            for (int e = 0; e < 4; ++e) c[i / 2][0][i & 1][e] = sizeof(E) == 4 ? 0.f : s[i][e] * (e < 2 ? f0 : f1);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) c[0][0][e] = c[0][1][e] = 0.f;
+        for (int kt = 0; kt < 2; ++kt) {
+            uint32_t a[1][3][4], b[4][NV][4];
+            ldsm_t<3>(a[0], smem_addr(sm.A) + frag_cols(16 * kt, 2 * warp, lane));
 #pragma unroll
-            for (int kt = 0; kt < 2; ++kt) {
-                uint32_t b[NV][4];
-                ldsm_t<NV>(b, smem_addr(sm.B) + frag_rows(16 * kt, 2 * i, lane));
-                mma_split<sizeof(E) == 4, 1, 3, NV>(c, a[kt], b);
+            for (int i = 0; i < 4; ++i) ldsm_t<NV>(b[i], smem_addr(sm.B) + frag_rows(16 * kt, 2 * i, lane));
+            if constexpr (NV == 1) {
+#pragma unroll
+                for (int pa = 2; pa >= 0; --pa)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        mma(c[i][0][0], a[0][pa], b[i][0][0], b[i][0][1]);
+                        mma(c[i][0][1], a[0][pa], b[i][0][2], b[i][0][3]);
+                    }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mma_split<true, 1, 3, NV>(c[i], a, b[i]);
             }
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[2 * i + j][e] = fmaf(s[2 * i + j][e], e < 2 ? f0 : f1, c[0][j][e]);
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[i][e] = sizeof(E) == 4 ? fmaf(s[i][e], e < 2 ? f0 : f1, c[i / 2][0][i & 1][e]) : c[i / 2][0][i & 1][e];
         if (it + 3 < nseg) bar_tell<3>(it & 1);
     }
 }
