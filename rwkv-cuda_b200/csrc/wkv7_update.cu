@@ -21,7 +21,8 @@
 // decays are carried as sums of two numbers: a vector is rounded once) and the 32 scalars of a step, which all rows share.
 // One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 213 us with a token as a step, 201 us here; 128 units
 // 427 -> 375 us, 256 units 852 -> 660 us.  A step takes 790 clocks where a unit has four SMs: 350 of the shared-memory reads, the
-// rest the latency of 260 instructions of one warp per scheduler; eight staging warps instead of four change nothing there.
+// rest 430 instructions per scheduler, of one warp that computes and one or two that stage (four staging warps 209 us, eight 201; with
+// more rows per block eight were slower: 128 units 411 us).
 // Errors of the state against fp64 9.1e-8 of the norm (a token as a step 8.3e-8: the same fp32 sums in another order), y as before.
 #include "common.cuh"
 #include "packed.cuh"
@@ -415,7 +416,7 @@ int update(int B, int T, int H, float* state, const void* r, const void* w, cons
     // bandwidth: with a token as a step 64 units took 356 us in blocks of 16 rows and 284 us in blocks of 32); with more units than
     // SMs / 2 the most rows per thread, which read every staged vector for four rows.
     const int units = B * H;
-    if (units * 4 <= sms) return launch_rows<E, 16, 4, 2, 4>(B, T, H, state, r, w, k, v, a, b, y, st);
+    if (units * 4 <= sms) return launch_rows<E, 16, 4, 2, 8>(B, T, H, state, r, w, k, v, a, b, y, st);
     if (units * 2 <= sms) return launch_rows<E, 8, 4, 2, 4>(B, T, H, state, r, w, k, v, a, b, y, st);
     return launch_rows<E, 8, 4, 4, 4>(B, T, H, state, r, w, k, v, a, b, y, st);
 }
