@@ -18,9 +18,10 @@
 // Why mma.sync and not tcgen05: these kernels are a block per segment with every accumulator and both states in registers,
 // four blocks per SM; the operands are split where they are used, and at 8 clocks per instruction and scheduler the tensor pipe
 // needs about as long as the arithmetic around it.
-// B8 T1000 H32 bf16, backward kernel 285 us (314 with the rows of exponents 64 floats apart, the token matrices as fp32, a test of the
-// alignment per load and bf16 parts unpacked before they are subtracted), y 111 us; 4300 -> 3900 instructions a warp and 324 mma: issue slots
-// and the latency of 16 warps per SM (128 registers a thread) bound it, the tensor pipe is busy 27 % of the time.
+// B8 T1000 H32 bf16: backward kernel 257 us (314 with a channel order in which a lane has two neighbours and not four, rows of
+// exponents 64 floats apart, the token matrices as fp32, a test of the alignment per load and bf16 parts unpacked before they are
+// subtracted), y 109 us.  3700 instructions a warp, 324 of them mma: issue slots and the latency of 16 warps per SM (128 registers a
+// thread) bound it, the tensor pipe is busy 30 % of the time.
 // A segment whose decays leave the range (more than kRange between its middle and an end) or that holds values that are not
 // finite (a masked product would spread them over tokens before) is flagged and left to the token-by-token kernels.
 #pragma once
@@ -36,9 +37,15 @@ template <bool STATIC> constexpr float kRange = STATIC ? 16.f : 86.f;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kImg = kSeg * 128;               // bytes of one bf16 image [32 tokens][64 channels]
 constexpr int kTiles = 3 * 512;                // bytes of one bf16 image of a triangular token x token matrix: its 16 x 16 tiles
-constexpr int kRld = 72;                       // floats of a row of 64 channels: 8-byte reads of eight rows hit every bank once
+constexpr int kRld = 80;                       // floats of a row of 64 channels: 16-byte reads of two rows hit every bank once
 
 // ---- bf16 images: rows of 128 bytes, their 16-byte pieces XOR-ed with the row ------------------------------------------------
+// The channels of each group of 16 stand in the order 0 1 4 5 8 9 12 13 2 3 6 7 10 11 14 15.  A lane's four k of a product over channels
+// and the four columns that it gets in two tiles are then neighbours, channels 4 q .. 4 q + 3: states, inputs and outputs move in
+// pieces of four (in the plain order of two: the backward kernel's load/store pipe was busy 70 % of the time with lines
+// that were touched twice, and B8 T1000 H32 took 544 us forward + backward instead of 510).
+// Row (or column) g of a tile is channel at16(g), of the tile beside it at16(g) + 2.
+__device__ __forceinline__ int at16(int g) { return 4 * (g >> 1) + (g & 1); }
 __device__ __forceinline__ uint32_t img_at(int row, int piece) { return row * 128 + ((piece ^ (row & 7)) << 4); }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // Fragments of mma.m16n8k16 by ldmatrix.  The place that a lane points at: (r0, c0) = first row, first 16-byte piece.
@@ -161,31 +168,49 @@ __device__ __forceinline__ void read_rows(Pair<E> (&x)[R], const E* p, int t0, i
         for (int i = 0; i < R; ++i) x[i] = t0 + i < n ? read_pair(p + i * C, false) : no_pair<E>();
     }
 }
-// rows g, g + 8, g + 16, g + 24 of two channels
+// rows g, g + 8, g + 16, g + 24 of four channels
+__device__ __forceinline__ void read_four(uint32_t& lo, uint32_t& hi, const bf16* p) {
+    const uint2 x = __ldg(reinterpret_cast<const uint2*>(p));
+    lo = x.x; hi = x.y;
+}
+__device__ __forceinline__ void read_four(float2& lo, float2& hi, const float* p) {
+    const float4 x = __ldg(reinterpret_cast<const float4*>(p));
+    lo = make_float2(x.x, x.y); hi = make_float2(x.z, x.w);
+}
 template <typename E>
-__device__ __forceinline__ void read_eights(Pair<E> (&x)[4], const E* p, int g, int n, int C, bool vec) {
+__device__ __forceinline__ void read_eights(Pair<E> (&x)[2][4], const E* p, int g, int n, int C, bool vec) {
     p += (i64)g * C;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) x[0][b] = x[1][b] = no_pair<E>();
     if (vec) {
 #pragma unroll
-        for (int b = 0; b < 4; ++b) x[b] = g + 8 * b < n ? read_pair(p + 8 * b * C, true) : no_pair<E>();
+        for (int b = 0; b < 4; ++b)
+            if (g + 8 * b < n) read_four(x[0][b], x[1][b], p + 8 * b * C);
     } else {
 #pragma unroll
-        for (int b = 0; b < 4; ++b) x[b] = g + 8 * b < n ? read_pair(p + 8 * b * C, false) : no_pair<E>();
+        for (int b = 0; b < 4; ++b)
+            if (g + 8 * b < n) { x[0][b] = read_pair(p + 8 * b * C, false); x[1][b] = read_pair(p + 8 * b * C + 2, false); }
     }
 }
 
+__device__ __forceinline__ uint32_t pair_at(int row, int pair) { return img_at(row, 2 * (pair >> 3) + (pair & 1)) + ((pair >> 1) & 3) * 4; }
+// eight channels as loaded
+__device__ __forceinline__ void put_eight(unsigned char* img, int row, int eight, uint4 x) {
+    *reinterpret_cast<uint2*>(img + img_at(row, eight & ~1) + 8 * (eight & 1)) = make_uint2(x.x, x.z);
+    *reinterpret_cast<uint2*>(img + img_at(row, eight | 1) + 8 * (eight & 1)) = make_uint2(x.y, x.w);
+}
 // images of a tensor as it came: bf16 one image, fp32 three
 template <typename E> constexpr int kParts = sizeof(E) == 2 ? 1 : 3;
 template <typename E>
 __device__ __forceinline__ void put_pair(unsigned char* img, int row, int lane, Pair<E> x);   // channels 2 lane, 2 lane + 1
 template <>
 __device__ __forceinline__ void put_pair<bf16>(unsigned char* img, int row, int lane, uint32_t x) {
-    *reinterpret_cast<uint32_t*>(img + img_at(row, lane >> 2) + (lane & 3) * 4) = x;
+    *reinterpret_cast<uint32_t*>(img + pair_at(row, lane)) = x;
 }
 __device__ __forceinline__ void put_split(unsigned char* img, int row, int lane, float x, float y) {
     uint32_t h, m, l;
     split3(x, y, h, m, l);
-    unsigned char* p = img + img_at(row, lane >> 2) + (lane & 3) * 4;
+    unsigned char* p = img + pair_at(row, lane);
     *reinterpret_cast<uint32_t*>(p) = h;
     *reinterpret_cast<uint32_t*>(p + kImg) = m;
     *reinterpret_cast<uint32_t*>(p + 2 * kImg) = l;
@@ -287,7 +312,7 @@ __device__ __forceinline__ bool stage_images(unsigned char* img, int tid, int n,
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            *reinterpret_cast<uint4*>(img + img_at(16 * i + (tid >> 3), tid & 7)) = x[i];
+            put_eight(img, 16 * i + (tid >> 3), tid & 7, x[i]);
             check(bad, decode(x[i].x)); check(bad, decode(x[i].y)); check(bad, decode(x[i].z)); check(bad, decode(x[i].w));
         }
     } else {
@@ -340,32 +365,18 @@ __device__ __forceinline__ void tile_frag(uint32_t (&f)[3][4], const unsigned ch
     else ldsm<3, kTiles>(f, smem_addr(img) + tile_at(tile, lane & 15, lane >> 4));
 }
 
-// Rows of 16 channels out of two accumulator tiles: neighbouring lanes swap a pair, so that a lane stores four channels
-template <typename E>
-__device__ __forceinline__ void store_row(E* row, float x0, float x1, float z0, float z1, int lane, bool vec, bool in);
-template <>
-__device__ __forceinline__ void store_row<bf16>(bf16* row, float x0, float x1, float z0, float z1, int lane, bool vec, bool in) {
-    const uint32_t x = pack_bf16(x0, x1), z = pack_bf16(z0, z1);
-    const bool odd = lane & 1;
-    const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? x : z, 1);
-    if (!in) return;
-    const uint2 v = odd ? make_uint2(got, z) : make_uint2(x, got);
-    bf16* p = row + (odd ? 8 + 2 * ((lane & 3) - 1) : 2 * (lane & 3));
+// four neighbouring channels out of two accumulator tiles
+__device__ __forceinline__ void store_four(bf16* p, float x0, float x1, float x2, float x3, bool vec) {
+    const uint2 v = make_uint2(pack_bf16(x0, x1), pack_bf16(x2, x3));
     if (vec) *reinterpret_cast<uint2*>(p) = v;
     else {
         unsigned short* s = reinterpret_cast<unsigned short*>(p);
         s[0] = (unsigned short)v.x; s[1] = (unsigned short)(v.x >> 16); s[2] = (unsigned short)v.y; s[3] = (unsigned short)(v.y >> 16);
     }
 }
-template <>
-__device__ __forceinline__ void store_row<float>(float* row, float x0, float x1, float z0, float z1, int lane, bool vec, bool in) {
-    const bool odd = lane & 1;
-    const float g0 = __shfl_xor_sync(0xffffffffu, odd ? x0 : z0, 1), g1 = __shfl_xor_sync(0xffffffffu, odd ? x1 : z1, 1);
-    if (!in) return;
-    const float4 v = odd ? make_float4(g0, g1, z0, z1) : make_float4(x0, x1, g0, g1);
-    float* p = row + (odd ? 8 + 2 * ((lane & 3) - 1) : 2 * (lane & 3));
-    if (vec) *reinterpret_cast<float4*>(p) = v;
-    else { p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w; }
+__device__ __forceinline__ void store_four(float* p, float x0, float x1, float x2, float x3, bool vec) {
+    if (vec) *reinterpret_cast<float4*>(p) = make_float4(x0, x1, x2, x3);
+    else { p[0] = x0; p[1] = x1; p[2] = x2; p[3] = x3; }
 }
 
 // Asks L2 for what the block `ahead` places further on will read first: rows of up to five tensors, a state or two (128 lines each)
@@ -406,13 +417,13 @@ __global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nse
     }
     float S[4][2][4];   // [16 keys][8 values] as B fragments
     {
-        const float* p = states + (i64)blockIdx.x * kN * kN + 16 * warp + g;
+        const float* p = states + (i64)blockIdx.x * kN * kN + 16 * warp + at16(g);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) S[kk][nt][e] = p[(16 * kk + 2 * q + (e & 1) + 8 * (e >> 1)) * kN + 8 * nt];
+                for (int e = 0; e < 4; ++e) S[kk][nt][e] = p[(16 * kk + 4 * q + e) * kN + 2 * nt];
     }
     bool bad = make_operands<E, STATIC, false>(sm.o, nullptr, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN);
     bad |= stage_images<E>(sm.V, tid, n, C, v_ + base);
@@ -444,11 +455,11 @@ __global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nse
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
         uint32_t a[2][3][4], b[3][4];
-        const float2 f0 = *reinterpret_cast<const float2*>(sm.o.em + 16 * kk + 2 * q), f1 = *reinterpret_cast<const float2*>(sm.o.em + 16 * kk + 8 + 2 * q);
+        const float4 f = *reinterpret_cast<const float4*>(sm.o.em + 16 * kk + 4 * q);
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-            split3(S[kk][nt][0] * f0.x, S[kk][nt][1] * f0.y, b[0][2 * nt], b[1][2 * nt], b[2][2 * nt]);
-            split3(S[kk][nt][2] * f1.x, S[kk][nt][3] * f1.y, b[0][2 * nt + 1], b[1][2 * nt + 1], b[2][2 * nt + 1]);
+            split3(S[kk][nt][0] * f.x, S[kk][nt][1] * f.y, b[0][2 * nt], b[1][2 * nt], b[2][2 * nt]);
+            split3(S[kk][nt][2] * f.z, S[kk][nt][3] * f.w, b[0][2 * nt + 1], b[1][2 * nt + 1], b[2][2 * nt + 1]);
         }
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt) ldsm<3>(a[mt], smem_addr(sm.o.R) + frag_rows(16 * mt, 2 * kk, lane));
@@ -473,7 +484,7 @@ __global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nse
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int t = 16 * mt + g + 8 * e;
-            store_row<E>(y_ + base + (i64)t * C + 16 * warp, acc[mt][0][2 * e], acc[mt][0][2 * e + 1], acc[mt][1][2 * e], acc[mt][1][2 * e + 1], lane, vec, t < n);
+            if (t < n) store_four(y_ + base + (i64)t * C + 16 * warp + 4 * q, acc[mt][0][2 * e], acc[mt][0][2 * e + 1], acc[mt][1][2 * e], acc[mt][1][2 * e + 1], vec);
         }
 }
 
@@ -511,13 +522,13 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     }
     float D[4][2][4];   // [16 keys][8 values] as B fragments
     {
-        const float* p = D_ + (i64)blockIdx.x * kN * kN + 16 * warp + g;
+        const float* p = D_ + (i64)blockIdx.x * kN * kN + 16 * warp + at16(g);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) D[kk][nt][e] = p[(16 * kk + 2 * q + (e & 1) + 8 * (e >> 1)) * kN + 8 * nt];
+                for (int e = 0; e < 4; ++e) D[kk][nt][e] = p[(16 * kk + 4 * q + e) * kN + 2 * nt];
     }
     bool bad = make_operands<E, STATIC, true>(sm.o, sm.rows, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN);
     bad |= stage_images<E>(sm.V, tid, n, C, v_ + base);
@@ -556,11 +567,11 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             uint32_t a[2][3][4], b[3][4];
-            const float2 f0 = *reinterpret_cast<const float2*>(sm.o.em2 + 16 * kk + 2 * q), f1 = *reinterpret_cast<const float2*>(sm.o.em2 + 16 * kk + 8 + 2 * q);
+            const float4 f = *reinterpret_cast<const float4*>(sm.o.em2 + 16 * kk + 4 * q);
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                split3(D[kk][nt][0] * f0.x, D[kk][nt][1] * f0.y, b[0][2 * nt], b[1][2 * nt], b[2][2 * nt]);
-                split3(D[kk][nt][2] * f1.x, D[kk][nt][3] * f1.y, b[0][2 * nt + 1], b[1][2 * nt + 1], b[2][2 * nt + 1]);
+                split3(D[kk][nt][0] * f.x, D[kk][nt][1] * f.y, b[0][2 * nt], b[1][2 * nt], b[2][2 * nt]);
+                split3(D[kk][nt][2] * f.z, D[kk][nt][3] * f.w, b[0][2 * nt + 1], b[1][2 * nt + 1], b[2][2 * nt + 1]);
             }
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt) ldsm<3>(a[mt], smem_addr(sm.o.K) + frag_rows(16 * mt, 2 * kk, lane));
@@ -584,7 +595,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int t = 16 * mt + g + 8 * e;
-                store_row<E>(gv_ + base + (i64)t * C + 16 * warp, acc[mt][0][2 * e], acc[mt][0][2 * e + 1], acc[mt][1][2 * e], acc[mt][1][2 * e + 1], lane, vec, t < n);
+                if (t < n) store_four(gv_ + base + (i64)t * C + 16 * warp + 4 * q, acc[mt][0][2 * e], acc[mt][0][2 * e + 1], acc[mt][1][2 * e], acc[mt][1][2 * e + 1], vec);
             }
     }
     // dk~ = V D'^T + G R~, dr~ = gY S'^T + G^T K~
@@ -596,24 +607,25 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
             for (int e = 0; e < 4; ++e) dk[mt][nt][e] = dr[mt][nt][e] = 0.f;
     {
-        const i64 so = (i64)blockIdx.x * kN * kN + (16 * warp + g) * kN + 2 * q;
+        const i64 so = (i64)blockIdx.x * kN * kN + (16 * warp + at16(g)) * kN + 4 * q;
         float fs[2], fd[2];
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) { fs[nt] = sm.o.em[16 * warp + 8 * nt + g]; fd[nt] = sm.o.em2[16 * warp + 8 * nt + g]; }
+        for (int nt = 0; nt < 2; ++nt) { fs[nt] = sm.o.em[16 * warp + at16(g) + 2 * nt]; fd[nt] = sm.o.em2[16 * warp + at16(g) + 2 * nt]; }
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             uint32_t bs[3][4], bd[3][4];
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    float2 s = *reinterpret_cast<const float2*>(S_ + so + 8 * nt * kN + 16 * kk + 8 * e);
-                    float2 x = *reinterpret_cast<const float2*>(D_ + so + 8 * nt * kN + 16 * kk + 8 * e);
-                    s.x *= fs[nt]; s.y *= fs[nt]; x.x *= fd[nt]; x.y *= fd[nt];
-                    a0[nt] = fmaf(s.x, x.x, fmaf(s.y, x.y, a0[nt]));
-                    split3(s.x, s.y, bs[0][2 * nt + e], bs[1][2 * nt + e], bs[2][2 * nt + e]);
-                    split3(x.x, x.y, bd[0][2 * nt + e], bd[1][2 * nt + e], bd[2][2 * nt + e]);
-                }
+            for (int nt = 0; nt < 2; ++nt) {
+                float4 s = *reinterpret_cast<const float4*>(S_ + so + 2 * nt * kN + 16 * kk);
+                float4 x = *reinterpret_cast<const float4*>(D_ + so + 2 * nt * kN + 16 * kk);
+                s.x *= fs[nt]; s.y *= fs[nt]; s.z *= fs[nt]; s.w *= fs[nt];
+                x.x *= fd[nt]; x.y *= fd[nt]; x.z *= fd[nt]; x.w *= fd[nt];
+                a0[nt] = fmaf(s.x, x.x, fmaf(s.y, x.y, fmaf(s.z, x.z, fmaf(s.w, x.w, a0[nt]))));
+                split3(s.x, s.y, bs[0][2 * nt], bs[1][2 * nt], bs[2][2 * nt]);
+                split3(s.z, s.w, bs[0][2 * nt + 1], bs[1][2 * nt + 1], bs[2][2 * nt + 1]);
+                split3(x.x, x.y, bd[0][2 * nt], bd[1][2 * nt], bd[2][2 * nt]);
+                split3(x.z, x.w, bd[0][2 * nt + 1], bd[1][2 * nt + 1], bd[2][2 * nt + 1]);
+            }
             uint32_t a[2][NV][4];
 #pragma unroll
             for (int mt = 0; mt < 2; ++mt) ldsm<NV>(a[mt], smem_addr(sm.V) + frag_rows(16 * mt, 2 * kk, lane));
@@ -627,38 +639,28 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     for (int nt = 0; nt < 2; ++nt) {   // a0: sum over the values of a key, to the lanes that have its column below
         a0[nt] += __shfl_xor_sync(0xffffffffu, a0[nt], 1);
         a0[nt] += __shfl_xor_sync(0xffffffffu, a0[nt], 2);
-        if (q == 0) sm.a0[16 * warp + 8 * nt + g] = a0[nt];
+        if (q == 0) sm.a0[16 * warp + at16(g) + 2 * nt] = a0[nt];
     }
     __syncwarp();
-    Pair<E> rp[2][4], kp[2][4];   // [tile][eight tokens]
-    {
-        const bool vin = vec_ok(r_, 2) && vec_ok(k_, 2);
-        const i64 o = base + 16 * warp + 2 * q;
+    const int c = 16 * warp + 4 * q;   // this lane's four keys: two of each tile
+    Pair<E> rp[2][4], kp[2][4];        // [two keys][eight tokens]
+    read_eights<E>(rp, r_ + base + c, g, n, C, vec_ok(r_, 4));
+    read_eights<E>(kp, k_ + base + c, g, n, C, vec_ok(k_, 4));
+    float aend[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-            read_eights<E>(rp[nt], r_ + o + 8 * nt, g, n, C, vin);
-            read_eights<E>(kp[nt], k_ + o + 8 * nt, g, n, C, vin);
-        }
+    for (int b = 0; b < 4; ++b) {
+        const float4 l = *reinterpret_cast<const float4*>(sm.rows + (8 * b + g + 1) * kRld + c);
+        const float2 k0 = decode(kp[0][b]), k1 = decode(kp[1][b]);
+        aend[0] = fmaf(k0.x * ex2(-l.x), dk[b >> 1][0][2 * (b & 1)], aend[0]);
+        aend[1] = fmaf(k0.y * ex2(-l.y), dk[b >> 1][0][2 * (b & 1) + 1], aend[1]);
+        aend[2] = fmaf(k1.x * ex2(-l.z), dk[b >> 1][1][2 * (b & 1)], aend[2]);
+        aend[3] = fmaf(k1.y * ex2(-l.w), dk[b >> 1][1][2 * (b & 1) + 1], aend[3]);
     }
-    float2 aend[2];
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-        const int c = 16 * warp + 8 * nt + 2 * q;
-        float2 s = make_float2(0.f, 0.f);
+    for (int i = 0; i < 4; ++i) {
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const float2 k = decode(kp[nt][2 * mt + e]), l = *reinterpret_cast<const float2*>(sm.rows + (16 * mt + 8 * e + g + 1) * kRld + c);
-                s.x = fmaf(k.x * ex2(-l.x), dk[mt][nt][2 * e], s.x);
-                s.y = fmaf(k.y * ex2(-l.y), dk[mt][nt][2 * e + 1], s.y);
-            }
-#pragma unroll
-        for (int m = 4; m < 32; m <<= 1) {
-            s.x += __shfl_xor_sync(0xffffffffu, s.x, m);
-            s.y += __shfl_xor_sync(0xffffffffu, s.y, m);
-        }
-        aend[nt] = make_float2(s.x + sm.a0[c], s.y + sm.a0[c + 1]);
+        for (int m = 4; m < 32; m <<= 1) aend[i] += __shfl_xor_sync(0xffffffffu, aend[i], m);
+        aend[i] += sm.a0[c + i];
     }
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
@@ -680,68 +682,29 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         }
     }
     // per token and key: scales and bonus terms, then the decay gradient
+    float P[4][4], x[4][4], gu[4] = {0.f, 0.f, 0.f, 0.f}, u[4];   // [eight tokens][key]; x = Q - P
+    {
+        const bool vu = vec_ok(u_, 2);
+        const float2 u0 = decode(read_pair(u_ + h * kN + c, vu)), u1 = decode(read_pair(u_ + h * kN + c + 2, vu));
+        u[0] = u0.x; u[1] = u0.y; u[2] = u1.x; u[3] = u1.y;
+    }
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-        const int c = 16 * warp + 8 * nt + 2 * q;
-        const float2 u = decode(read_pair(u_ + h * kN + c, vec_ok(u_, 2)));
-        float2 x[4], Q[4], gu = make_float2(0.f, 0.f);   // x = Q - P
+    for (int b = 0; b < 4; ++b) {
+        const int mt = b >> 1, e = b & 1, t = 8 * b + g;
+        const float4 l0 = *reinterpret_cast<const float4*>(sm.rows + t * kRld + c), l1 = *reinterpret_cast<const float4*>(sm.rows + (t + 1) * kRld + c);
+        const float before[4] = {l0.x, l0.y, l0.z, l0.w}, behind[4] = {l1.x, l1.y, l1.z, l1.w}, gm = sm.gamma[t];
+        const float2 r0 = decode(rp[0][b]), r1 = decode(rp[1][b]), k0 = decode(kp[0][b]), k1 = decode(kp[1][b]);
+        const float r[4] = {r0.x, r0.y, r1.x, r1.y}, k[4] = {k0.x, k0.y, k1.x, k1.y};
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int mt = b >> 1, e = b & 1, t = 8 * b + g;
-            const float2 r = decode(rp[nt][b]), k = decode(kp[nt][b]);
-            const float2 l0 = *reinterpret_cast<const float2*>(sm.rows + t * kRld + c), l1 = *reinterpret_cast<const float2*>(sm.rows + (t + 1) * kRld + c);
-            float &k0 = dk[mt][nt][2 * e], &k1 = dk[mt][nt][2 * e + 1], &r0 = dr[mt][nt][2 * e], &r1 = dr[mt][nt][2 * e + 1];
-            k0 *= ex2(-l1.x); k1 *= ex2(-l1.y); r0 *= ex2(l0.x); r1 *= ex2(l0.y);
-            Q[b] = make_float2(k.x * k0, k.y * k1);
-            x[b] = make_float2(fmaf(-r.x, r0, Q[b].x), fmaf(-r.y, r1, Q[b].y));
-            const float gm = sm.gamma[t];
-            gu.x = fmaf(gm, r.x * k.x, gu.x); gu.y = fmaf(gm, r.y * k.y, gu.y);
-            k0 = fmaf(gm * u.x, r.x, k0); k1 = fmaf(gm * u.y, r.y, k1);
-            r0 = fmaf(gm * u.x, k.x, r0); r1 = fmaf(gm * u.y, k.y, r1);
-        }
-        float2 after = make_float2(0.f, 0.f), gw = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int b = 3; b >= 0; --b) {   // sums over the tokens behind: over lanes inside eight tokens, then over the eights
-            float2 s = x[b];
-#pragma unroll
-            for (int m = 1; m < 8; m <<= 1) {
-                const float2 o = make_float2(__shfl_down_sync(0xffffffffu, s.x, 4 * m), __shfl_down_sync(0xffffffffu, s.y, 4 * m));
-                if (g + m < 8) { s.x += o.x; s.y += o.y; }
-            }
-            const float2 d = make_float2(aend[nt].x - (after.x + (s.x - x[b].x)) - Q[b].x, aend[nt].y - (after.y + (s.y - x[b].y)) - Q[b].y);
-            after.x += __shfl_sync(0xffffffffu, s.x, q);
-            after.y += __shfl_sync(0xffffffffu, s.y, q);
-            if (STATIC) { if (8 * b + g < n) { gw.x += d.x; gw.y += d.y; } }
-            else x[b] = d;
-        }
-#pragma unroll
-        for (int m = 4; m < 32; m <<= 1) {
-            gu.x += __shfl_xor_sync(0xffffffffu, gu.x, m);
-            gu.y += __shfl_xor_sync(0xffffffffu, gu.y, m);
-            if (STATIC) { gw.x += __shfl_xor_sync(0xffffffffu, gw.x, m); gw.y += __shfl_xor_sync(0xffffffffu, gw.y, m); }
-        }
-        if (g == 0) {
-            float* p = partial_ + (unit / H * nseg + seg) * (STATIC ? 2 : 1) * C + h * kN + c;
-            if (STATIC) {
-                const float2 w = decode(read_pair(w_ + h * kN + c, vec_ok(w_, 2)));
-                p[0] = -expf(w.x) * gw.x; p[1] = -expf(w.y) * gw.y;   // d log d / d w_raw = log d
-                p += C;
-            }
-            p[0] = gu.x; p[1] = gu.y;
-        }
-        if (!STATIC) {
-            Pair<E> wp[4];
-            read_eights<E>(wp, w_ + base + c, g, n, C, vec_ok(w_, 2));
-            E* p = gw_ + base + (i64)g * C + c;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const float2 w = decode(wp[b]);
-                x[b].x *= -ex2(kLog2e * w.x); x[b].y *= -ex2(kLog2e * w.y);
-                if (8 * b + g < n) {
-                    if (sizeof(E) == 2 && vec) *reinterpret_cast<uint32_t*>(p + 8 * b * C) = pack_bf16(x[b].x, x[b].y);
-                    else { p[8 * b * C] = from_f<E>(x[b].x); p[8 * b * C + 1] = from_f<E>(x[b].y); }
-                }
-            }
+        for (int i = 0; i < 4; ++i) {
+            float &yk = dk[mt][i >> 1][2 * e + (i & 1)], &yr = dr[mt][i >> 1][2 * e + (i & 1)];
+            yk *= ex2(-behind[i]);
+            yr *= ex2(before[i]);
+            P[b][i] = r[i] * yr;
+            x[b][i] = fmaf(k[i], yk, -P[b][i]);
+            gu[i] = fmaf(gm, r[i] * k[i], gu[i]);
+            yk = fmaf(gm * u[i], r[i], yk);
+            yr = fmaf(gm * u[i], k[i], yr);
         }
     }
 #pragma unroll
@@ -749,16 +712,63 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int t = 16 * mt + g + 8 * e;
-            const i64 o = base + (i64)t * C + 16 * warp;
-            store_row<E>(gk_ + o, dk[mt][0][2 * e], dk[mt][0][2 * e + 1], dk[mt][1][2 * e], dk[mt][1][2 * e + 1], lane, vec, t < n);
-            store_row<E>(gr_ + o, dr[mt][0][2 * e], dr[mt][0][2 * e + 1], dr[mt][1][2 * e], dr[mt][1][2 * e + 1], lane, vec, t < n);
+            const i64 o = base + (i64)t * C + c;
+            if (t < n) {
+                store_four(gk_ + o, dk[mt][0][2 * e], dk[mt][0][2 * e + 1], dk[mt][1][2 * e], dk[mt][1][2 * e + 1], vec);
+                store_four(gr_ + o, dr[mt][0][2 * e], dr[mt][0][2 * e + 1], dr[mt][1][2 * e], dr[mt][1][2 * e + 1], vec);
+            }
         }
+    float gw[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float after = 0.f;
+        gw[i] = 0.f;
+#pragma unroll
+        for (int b = 3; b >= 0; --b) {   // sums over the tokens from here on: over lanes inside eight tokens, then over the eights
+            float s = x[b][i];
+#pragma unroll
+            for (int m = 1; m < 8; m <<= 1) {
+                const float o = __shfl_down_sync(0xffffffffu, s, 4 * m);
+                if (g + m < 8) s += o;
+            }
+            // A_end - sum_{tau > t} (Q - P) - Q_t = A_end - sum_{tau >= t} (Q - P) - P_t
+            x[b][i] = aend[i] - (after + s) - P[b][i];
+            after += __shfl_sync(0xffffffffu, s, q);
+            if (STATIC && 8 * b + g < n) gw[i] += x[b][i];
+        }
+#pragma unroll
+        for (int m = 4; m < 32; m <<= 1) {
+            gu[i] += __shfl_xor_sync(0xffffffffu, gu[i], m);
+            if (STATIC) gw[i] += __shfl_xor_sync(0xffffffffu, gw[i], m);
+        }
+    }
+    if (g == 0) {
+        float* p = partial_ + (unit / H * nseg + seg) * (STATIC ? 2 : 1) * C + h * kN + c;
+        if (STATIC) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) p[i] = -expf(to_f(w_[h * kN + c + i])) * gw[i];   // d log d / d w_raw = log d
+            p += C;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = gu[i];
+    }
+    if constexpr (!STATIC) {
+        Pair<E> wp[2][4];
+        read_eights<E>(wp, w_ + base + c, g, n, C, vec_ok(w_, 4));
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float2 w0 = decode(wp[0][b]), w1 = decode(wp[1][b]);
+            if (8 * b + g < n)
+                store_four(gw_ + base + (i64)(8 * b + g) * C + c, -ex2(kLog2e * w0.x) * x[b][0], -ex2(kLog2e * w0.y) * x[b][1], -ex2(kLog2e * w1.x) * x[b][2],
+                           -ex2(kLog2e * w1.y) * x[b][3], vec);
+        }
+    }
 }
 
 // States at the start of every segment (REV: adjoints at the end), one block per unit walking its segments: S <- S diag(f) + k'^T V
 // with k'_s = k_s exp(L_end - L_s) (REV: r'_t = r_t exp(L_{t-1}), gy): all factors are at most 1.  Warps 0 to 3 have the state in
-// registers, 16 keys each, warps 4 to 11 make the operands of the segments to come (B8 T1000 H32 bf16: 80 us with four of them, 68 with
-// eight and rows asked for in L2 six segments ahead: 1.8 TB/s; the walk waits for instructions of the operands and for barriers).
+// registers, 16 keys each, warps 4 to 11 make the operands of the segments to come (B8 T1000 H32 bf16: 80 us with four of them, two
+// sums of products at a time and states stored in pieces of 8 bytes, 63 us now: 3.7 TB/s).
 template <typename E>
 struct ChainSmem {
     unsigned char A[3 * kImg], B[kParts<E> * kImg];
@@ -854,7 +864,7 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
                 put_split(sm.A, t0 + i, lane, a.x * ex2(e.x), a.y * ex2(e.y));
             }
             if (wide) {
-                *reinterpret_cast<uint4*>(sm.B + img_at(tid >> 3, tid & 7)) = x.bw;
+                put_eight(sm.B, tid >> 3, tid & 7, x.bw);
             } else {
 #pragma unroll
                 for (int i = 0; i < R; ++i) put_pair<E>(sm.B, t0 + i, lane, x.bb[i]);
@@ -868,7 +878,7 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
         }
         return;
     }
-    // ---- the state: keys 16 warp + g, + 8 of all values -----------------------------------------------------------------------
+    // ---- the state: keys 16 warp + at16(g), + 2 of all values -----------------------------------------------------------------------
     const int g = lane >> 2, q = lane & 3;
     float s[8][4];
 #pragma unroll
@@ -876,15 +886,16 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[i][e] = 0.f;
     for (int it = 0; it < nseg; ++it) {
-        float* p = states + (unit * nseg + (REV ? nseg - 1 - it : it)) * kN * kN + (16 * warp + g) * kN + 2 * q;
+        float* p = states + (unit * nseg + (REV ? nseg - 1 - it : it)) * kN * kN + (16 * warp + at16(g)) * kN + 4 * q;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) *reinterpret_cast<float2*>(p + 8 * e * kN + 8 * i) = make_float2(s[i][2 * e], s[i][2 * e + 1]);
+            for (int e = 0; e < 2; ++e)
+                *reinterpret_cast<float4*>(p + 2 * e * kN + 16 * i) = make_float4(s[2 * i][2 * e], s[2 * i][2 * e + 1], s[2 * i + 1][2 * e], s[2 * i + 1][2 * e + 1]);
         if (it + 1 == nseg) break;
         bar_join<1>(it & 1);
         const ChainSmem<E>& sm = buf[it & 1];
-        const float f0 = sm.f[16 * warp + g], f1 = sm.f[16 * warp + g + 8];
+        const float f0 = sm.f[16 * warp + at16(g)], f1 = sm.f[16 * warp + at16(g) + 2];
         // bf16: straight onto the state, eight sums side by side; fp32: products apart (see mma_split)
         float c[4][1][2][4];
 #pragma unroll
