@@ -19,8 +19,8 @@
 // the eight dot products of a row are reduced together (8 shuffles, not 4 per token), 17 vectors are read instead of 20, and the
 // chain has one reduction per four tokens.  NCW warps compute; NSW warps stage, a step each: they make the scaled vectors (products of
 // decays are carried as sums of two numbers: a vector is rounded once) and the 32 scalars of a step, which all rows share.
-// One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 213 us with a token as a step, 201 us here; 128 units
-// 427 -> 375 us, 256 units 852 -> 660 us.  A step takes 790 clocks where a unit has four SMs: 350 of the shared-memory reads, the
+// One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 213 us with a token as a step, 205 us here; 128 units
+// 427 -> 380 us, 256 units 852 -> 670 us.  A step takes 790 clocks where a unit has four SMs: 350 of the shared-memory reads, the
 // rest 430 instructions per scheduler, of one warp that computes and one or two that stage (four staging warps 209 us, eight 201; with
 // more rows per block eight were slower: 128 units 411 us).
 // Errors of the state against fp64 9.1e-8 of the norm (a token as a step 8.3e-8: the same fp32 sums in another order), y as before.
@@ -381,7 +381,8 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
             for (int i = 0; i < RPT; ++i) {
                 y[i] = own[i];
 #pragma unroll
-                for (int e = 0; e < kQ; ++e) y[i] = fmaf(sa[e][i], g[2 * e], fmaf(v[e][i], g[2 * e + 1], y[i]));
+                for (int e = 0; e < kQ; ++e)
+                    if (e <= ty) y[i] = fmaf(sa[e][i], g[2 * e], fmaf(v[e][i], g[2 * e + 1], y[i]));   // (a later token's may not be finite)
             }
             const int t = c * kCh + kQ * q + ty;
             if (x < 4 * TS && x % TS == 0 && t < T) store_rows<E, RPT>(y_ + base + (i64)t * C + row0, y);

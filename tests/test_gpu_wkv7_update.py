@@ -21,3 +21,26 @@ def test_state_update(dtype, B, T, H):
     R.ops.wkv7_state_update(state, *(inp[n].to(dtype).cuda().view(B, T, H, N).contiguous() for n in names), y)
     Hh.assert_close(y.view(B, T, H * N), y64, Hh.tol_for(dtype), "y")
     Hh.assert_close(state, sT64, 1e-5, "state")   # fp32 whatever the activations are
+
+
+@pytest.mark.parametrize("name", ["r", "w", "k", "v", "a", "b"])
+@pytest.mark.parametrize("t", [4, 6, 7])   # first, third and last token of a step of four
+def test_values_that_are_not_finite_stay_behind(t, name):
+    """Tokens before such a value, in its own step too, and the rows of other units are those of the call without it."""
+    import rwkv_cuda_b200 as R
+    B, T, H, N = 1, 17, 2, 64
+    inp = Hh.v7_inputs(B, T, H, N, seed=2)
+
+    def call(x):
+        state = x["s0"].cuda()
+        y = torch.empty(B, T, H, N, device="cuda")
+        R.ops.wkv7_state_update(state, *(x[n].float().cuda().view(B, T, H, N).contiguous() for n in ("r", "w", "k", "v", "a", "b")), y)
+        return y, state
+
+    y0, s0 = call(inp)
+    bad = dict(inp)
+    bad[name] = inp[name].clone().reshape(B, T, H, N)
+    bad[name][0, t, 0, 5] = float("nan")
+    y, s = call(bad)
+    assert torch.equal(y[:, :t], y0[:, :t]) and torch.equal(y[:, :, 1], y0[:, :, 1]) and torch.equal(s[:, 1], s0[:, 1])
+    assert torch.isnan(y[:, t:, 0]).any()
