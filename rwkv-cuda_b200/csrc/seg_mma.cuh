@@ -20,7 +20,7 @@
 // needs about as long as the arithmetic around it.
 // B8 T1000 H32 bf16: backward kernel 257 us (314 with a channel order in which a lane has two neighbours and not four, rows of
 // exponents 64 floats apart, the token matrices as fp32, a test of the alignment per load and bf16 parts unpacked before they are
-// subtracted), y 109 us.  3700 instructions a warp, 324 of them mma: issue slots and the latency of 16 warps per SM (128 registers a
+// subtracted), y 104 us (110 with four blocks per SM and 125 registers a thread instead of five and 96).  3700 instructions a warp, 324 of them mma: issue slots and the latency of 16 warps per SM (128 registers a
 // thread) bound it, the tensor pipe is busy 30 % of the time.
 // A segment whose decays leave the range (more than kRange between its middle and an end) or that holds values that are not
 // finite (a masked product would spread them over tokens before) is flagged and left to the token-by-token kernels.
@@ -397,7 +397,7 @@ struct YSmem {
     unsigned char M[3 * kTiles];   // A transposed: [t][s]
 };
 template <typename E, bool STATIC>
-__global__ void __launch_bounds__(128, 4) seg_mma_y_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
+__global__ void __launch_bounds__(128, sizeof(E) == 2 ? 5 : 4) seg_mma_y_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
                                                            const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
                                                            const float* __restrict__ states, E* __restrict__ y_, int* __restrict__ flags, int ahead) {
     extern __shared__ __align__(128) unsigned char smem_seg_y[];
