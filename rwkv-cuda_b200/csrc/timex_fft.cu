@@ -20,8 +20,9 @@
 // register); the inverse takes the same steps backwards, so nothing is ever reordered.  The upper half of the input is zero
 // and the upper half of the output is not needed: the outer radix-16 steps do half of their work.  Row strides in shared
 // memory (L + R, and 16 (R+1) + R) make every exchange conflict free.  128 threads per block, 2048 / N transforms at a time.
-// B32 C768 T768 on a B200: forward 357 us direct, 112 us here; backward with its gw over the batch 1017 and 236 us
-// (looking at the pairs is 19 us of these).  Errors against fp64 are 2.4e-7 of the norm (direct: 4.1e-7).
+// B32 C768 T768 on a B200: forward 357 us direct, 112 us with 2048 points, 104 us with 1536; backward with its gw over the batch 1017,
+// 236 and 189 us (three blocks of 96 threads per SM; four, which spill registers, 6 us more; looking at the pairs is 19 us of these).
+// Errors against fp64 are 2.4e-7 of the norm (direct: 4.1e-7).
 #include "timex_fft.cuh"
 
 namespace rwkvb200 {
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(Plan<R>::kThreads, R % 3 ? 4 : 5) timex_fft_fo
 
 // gk, and the filter gradient summed over the batch rows of the block: gw[blockIdx.y][c][t]
 template <int R>
-__global__ void __launch_bounds__(Plan<R>::kThreads, R % 3 ? 3 : 4) timex_fft_backward_kernel(const float* __restrict__ w, const float* __restrict__ k_,
+__global__ void __launch_bounds__(Plan<R>::kThreads, 3) timex_fft_backward_kernel(const float* __restrict__ w, const float* __restrict__ k_,
                                                                          const float* __restrict__ g_, float* __restrict__ gw_,
                                                                          float* __restrict__ gk_, int B, int C, int T) {
     using P = Plan<R>;
