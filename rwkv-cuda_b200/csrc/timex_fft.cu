@@ -20,8 +20,9 @@
 // register); the inverse takes the same steps backwards, so nothing is ever reordered.  The upper half of the input is zero
 // and the upper half of the output is not needed: the outer radix-16 steps do half of their work.  Row strides in shared
 // memory (L + R, and 16 (R+1) + R) make every exchange conflict free.  128 threads per block, 2048 / N transforms at a time.
-// B32 C768 T768 on a B200: forward 357 us direct, 112 us with 2048 points, 104 us with 1536; backward with its gw over the batch 1017,
-// 236 and 189 us (three blocks of 96 threads per SM; four, which spill registers, 6 us more; looking at the pairs is 19 us of these).
+// B32 C768 T768 on a B200: forward 357 us direct, 112 us with 2048 points, 102 us with 1536; backward with its gw over the batch 1017,
+// 218 and 182 us (compiled for three blocks of 96 threads per SM; for four 191; looking at the pairs is 19 us of these), and 5 us to
+// sum its parts.
 // Errors against fp64 are 2.4e-7 of the norm (direct: 4.1e-7).
 #include "timex_fft.cuh"
 
