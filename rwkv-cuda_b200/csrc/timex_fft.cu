@@ -21,7 +21,8 @@
 // and the upper half of the output is not needed: the outer radix-16 steps do half of their work.  Row strides in shared
 // memory (L + R, and 16 (R+1) + R) make every exchange conflict free.  128 threads per block, 2048 / N transforms at a time.
 // B32 C768 T768 on a B200: forward 357 us direct, 112 us with 2048 points, 102 us with 1536; backward with its gw over the batch 1017,
-// 218 and 182 us (compiled for three blocks of 96 threads per SM; for four 191; looking at the pairs is 19 us of these), and 5 us to
+// 218 and 182 us (compiled for three blocks of 96 threads per SM; for four 191; looking at the pairs took 19 us of these with a
+// barrier of its own, 2 or 3 less with the vote at the first barrier of a transform), and 5 us to
 // sum its parts.
 // Errors against fp64 are 2.4e-7 of the norm (direct: 4.1e-7).
 #include "timex_fft.cuh"
@@ -176,12 +177,15 @@ struct Engine {
     }
     // v[m] = element j + L m (m < 8) -> spectrum.  A forward right after another forward needs a __syncthreads before it (the
     // other threads may still read the first exchange); between forward and inverse every thread writes what only it has read.
-    __device__ __forceinline__ void forward(cf (&v)[V]) {
+    // VOTE: the block's first barrier also asks whether any thread is against it; if so, nothing more is done and the answer is true.
+    template <bool VOTE>
+    __device__ __forceinline__ bool forward(cf (&v)[V], bool against) {
         fft16<false, true>(v);
         t1.apply<false>(v);
 #pragma unroll
         for (int k = 0; k < 16; ++k) b1[k * P::S1 + j] = v[k];
-        __syncthreads();
+        if (VOTE) { if (__syncthreads_or(against)) return true; }
+        else __syncthreads();
 #pragma unroll
         for (int m = 0; m < 16; ++m) v[m] = b1[k1 * P::S1 + j1 + R * m];
         fft16<false, false>(v);
@@ -195,7 +199,9 @@ struct Engine {
 #pragma unroll
             for (int i = 0; i < R; ++i) v[e * R + i] = 16 % R == 0 || j1 + R * e < 16 ? b2[k1 * P::S2 + (j1 + R * e) * P::P2 + i] : cf{0.f, 0.f};
         small<false>(v);
+        return false;
     }
+    __device__ __forceinline__ void forward(cf (&v)[V]) { forward<false>(v, false); }
     // spectrum -> elements j + L m in v[m] (m < 8 are what the callers use), times N
     __device__ __forceinline__ void inverse(cf (&v)[V]) {
         small<true>(v);
@@ -313,12 +319,9 @@ __global__ void __launch_bounds__(Plan<R>::kThreads, R % 3 ? 4 : 5) timex_fft_fo
             const int t = fft.j + P::L * m;
             v[m] = cf{t < n0 ? k_[r0 + t] : 0.f, t < n1 ? k_[r1 + t] : 0.f};
         }
-        if (pass == kTogether) {
-            if (__syncthreads_or(apart<P::kRatio>(v, n1 != 0, threadIdx.x & 31) || bad_filter)) { pass = kFirst; continue; }
-        } else if (bad_filter || unfit(v)) {
-            bad[2 * g + (pass == kSecond)] = 1;
-        }
-        fft.forward(v);
+        const bool together = pass == kTogether;
+        if (!together && (bad_filter || unfit(v))) bad[2 * g + (pass == kSecond)] = 1;
+        if (fft.template forward<true>(v, together && (apart<P::kRatio>(v, n1 != 0, threadIdx.x & 31) || bad_filter))) { pass = kFirst; continue; }
 #pragma unroll
         for (int k = 0; k < P::V; ++k) v[k] = mul(v[k], Wh[k * P::L + fft.j]);
         fft.inverse(v);
@@ -375,13 +378,14 @@ __global__ void __launch_bounds__(Plan<R>::kThreads, 3) timex_fft_backward_kerne
             z[m] = cf{t < n0 ? k_[r0 + t] : 0.f, t < n1 ? k_[r1 + t] : 0.f};
             v[m] = cf{t < n0 ? g_[r0 + T - 1 - t] : 0.f, t < n1 ? -g_[r1 + T - 1 - t] : 0.f};
         }
+        bool against = false;
         if (pass == kTogether) {
             const bool za = apart<P::kRatio>(z, n1 != 0, threadIdx.x & 31), va = apart<P::kRatio>(v, n1 != 0, threadIdx.x & 31);
-            if (__syncthreads_or(za || va || bad_filter)) { pass = kFirst; continue; }
+            against = za || va || bad_filter;
         } else if (unfit(z) || unfit(v)) {
             bad[2 * g + (pass == kSecond)] = 1;
         }
-        fft.forward(z);
+        if (fft.template forward<true>(z, against)) { pass = kFirst; continue; }
         __syncthreads();
         const bool skip = pass != kTogether && bad[2 * g + (pass == kSecond)];
         fft.forward(v);
