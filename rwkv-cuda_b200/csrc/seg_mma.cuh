@@ -18,10 +18,11 @@
 // Why mma.sync and not tcgen05: these kernels are a block per segment with every accumulator and both states in registers,
 // four blocks per SM; the operands are split where they are used, and at 8 clocks per instruction and scheduler the tensor pipe
 // needs about as long as the arithmetic around it.
-// B8 T1000 H32 bf16: backward kernel 257 us (314 with a channel order in which a lane has two neighbours and not four, rows of
-// exponents 64 floats apart, the token matrices as fp32, a test of the alignment per load and bf16 parts unpacked before they are
-// subtracted), y 104 us (110 with four blocks per SM and 125 registers a thread instead of five and 96).  3700 instructions a warp, 324 of them mma: issue slots and the latency of 16 warps per SM (128 registers a
-// thread) bound it, the tensor pipe is busy 30 % of the time.
+// B8 T1000 H32 bf16: backward kernel 249 us (314 with a channel order in which a lane has two neighbours and not four, rows of
+// exponents 64 floats apart, the token matrices as fp32, a test of the alignment per load, bf16 parts unpacked before they are
+// subtracted and states read where they are used), y 103 us (110 with four blocks per SM and 125 registers a thread instead of five
+// and 96).  3700 instructions a warp, 324 of them mma: issue slots and the latency of 16 warps per SM (128 registers a thread) bound
+// it, the tensor pipe is busy 30 % of the time.
 // A segment whose decays leave the range (more than kRange between its middle and an end) or that holds values that are not
 // finite (a masked product would spread them over tokens before) is flagged and left to the token-by-token kernels.
 #pragma once
@@ -388,6 +389,13 @@ __device__ __forceinline__ void prefetch_rows(const E* x, i64 base, int n, int C
     }
 }
 
+// A read that stays where it is written: the states are asked for a step before they are used, which the compiler would undo
+__device__ __forceinline__ float4 read_now(const float* p) {
+    float4 x;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w) : "l"(p));
+    return x;
+}
+
 // ---- kernels -----------------------------------------------------------------------------------------------------------------
 // y of a segment from its start state.  One block per (unit, segment), 4 warps; a warp has 16 values of all tokens.
 template <typename E>
@@ -397,7 +405,7 @@ struct YSmem {
     unsigned char M[3 * kTiles];   // A transposed: [t][s]
 };
 template <typename E, bool STATIC>
-__global__ void __launch_bounds__(128, sizeof(E) == 2 ? 5 : 4) seg_mma_y_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
+__global__ void __launch_bounds__(128, 5) seg_mma_y_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
                                                            const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
                                                            const float* __restrict__ states, E* __restrict__ y_, int* __restrict__ flags, int ahead) {
     extern __shared__ __align__(128) unsigned char smem_seg_y[];
@@ -558,6 +566,15 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
                          s < t + 1 ? z : diag && s == t + 1 ? sm.o.ruk[s] : 0.f);
             }
     }
+    const i64 so = (i64)blockIdx.x * kN * kN + (16 * warp + at16(g)) * kN + 4 * q;
+    float4 s4[2][2], x4[2][2];   // S and D of 16 values: of this step and of the next, [tile]
+    auto read_states = [&](int kk) {
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            s4[kk & 1][nt] = read_now(S_ + so + 2 * nt * kN + 16 * kk);
+            x4[kk & 1][nt] = read_now(D_ + so + 2 * nt * kN + 16 * kk);
+        }
+    };
     {   // gv = K~ D' + A gY
         float acc[2][2][4];
 #pragma unroll
@@ -577,6 +594,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             for (int mt = 0; mt < 2; ++mt) ldsm<3>(a[mt], smem_addr(sm.o.K) + frag_rows(16 * mt, 2 * kk, lane));
             mma_split<sizeof(E) == 4, 2, 3, 3>(acc, a, b);
         }
+        read_states(0);
         __syncthreads();
 #pragma unroll
         for (int kt = 0; kt < 2; ++kt) {
@@ -599,6 +617,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             }
     }
     // dk~ = V D'^T + G R~, dr~ = gY S'^T + G^T K~
+    const int c = 16 * warp + 4 * q;   // this lane's four keys: two of each tile
+    Pair<E> rp[2][4], kp[2][4];        // [two keys][eight tokens]
     float dk[2][2][4], dr[2][2][4], a0[2] = {0.f, 0.f};
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
@@ -607,17 +627,20 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
             for (int e = 0; e < 4; ++e) dk[mt][nt][e] = dr[mt][nt][e] = 0.f;
     {
-        const i64 so = (i64)blockIdx.x * kN * kN + (16 * warp + at16(g)) * kN + 4 * q;
         float fs[2], fd[2];
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) { fs[nt] = sm.o.em[16 * warp + at16(g) + 2 * nt]; fd[nt] = sm.o.em2[16 * warp + at16(g) + 2 * nt]; }
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
             uint32_t bs[3][4], bd[3][4];
+            if (kk < 3) read_states(kk + 1);
+            else {
+                read_eights<E>(rp, r_ + base + c, g, n, C, vec_ok(r_, 4));
+                read_eights<E>(kp, k_ + base + c, g, n, C, vec_ok(k_, 4));
+            }
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                float4 s = *reinterpret_cast<const float4*>(S_ + so + 2 * nt * kN + 16 * kk);
-                float4 x = *reinterpret_cast<const float4*>(D_ + so + 2 * nt * kN + 16 * kk);
+                float4 s = s4[kk & 1][nt], x = x4[kk & 1][nt];
                 s.x *= fs[nt]; s.y *= fs[nt]; s.z *= fs[nt]; s.w *= fs[nt];
                 x.x *= fd[nt]; x.y *= fd[nt]; x.z *= fd[nt]; x.w *= fd[nt];
                 a0[nt] = fmaf(s.x, x.x, fmaf(s.y, x.y, fmaf(s.z, x.z, fmaf(s.w, x.w, a0[nt]))));
@@ -642,10 +665,6 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         if (q == 0) sm.a0[16 * warp + at16(g) + 2 * nt] = a0[nt];
     }
     __syncwarp();
-    const int c = 16 * warp + 4 * q;   // this lane's four keys: two of each tile
-    Pair<E> rp[2][4], kp[2][4];        // [two keys][eight tokens]
-    read_eights<E>(rp, r_ + base + c, g, n, C, vec_ok(r_, 4));
-    read_eights<E>(kp, k_ + base + c, g, n, C, vec_ok(k_, 4));
     float aend[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
@@ -718,6 +737,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
                 store_four(gr_ + o, dr[mt][0][2 * e], dr[mt][0][2 * e + 1], dr[mt][1][2 * e], dr[mt][1][2 * e + 1], vec);
             }
         }
+    Pair<E> wp[2][4];
+    if constexpr (!STATIC) read_eights<E>(wp, w_ + base + c, g, n, C, vec_ok(w_, 4));
     float gw[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -753,8 +774,6 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         for (int i = 0; i < 4; ++i) p[i] = gu[i];
     }
     if constexpr (!STATIC) {
-        Pair<E> wp[2][4];
-        read_eights<E>(wp, w_ + base + c, g, n, C, vec_ok(w_, 4));
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const float2 w0 = decode(wp[0][b]), w1 = decode(wp[1][b]);

@@ -22,7 +22,7 @@
 // the reads of the token's vectors bound everything (512 bytes per 96 packed multiply-adds); a lane therefore owns a tile of
 // 8 keys x 8 values, and the sums over lanes are taken for eight elements at a time (7 shuffles).
 // fp32, B8 T512 H16 N64, forward + backward on a B200: 1285 us with wkv5.cu, 309 us token by token on all segments (without register
-// spills in the backward, which two blocks per SM allow and three do not: 212 -> 167 us for that kernel), 181 us by products, whose errors
+// spills in the backward, which two blocks per SM allow and three do not: 212 -> 167 us for that kernel), 178 us by products, whose errors
 // against fp64 are a third of that (T 1000: y 5.3e-7 -> 1.8e-7 of the norm, gw 8.8e-7 -> 3.1e-7).
 #include "wkv5_seg.cuh"
 #include "seg_mma.cuh"
