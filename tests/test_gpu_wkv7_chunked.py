@@ -178,3 +178,35 @@ def test_paths_without_tensor_maps_agree(form, B, T, H):
     # the forward differs in form (staged with maps, one group without when form != 1): equal up to rounding
     for n in ("y", "sT"):
         assert (with_maps[n].float() - without[n].float()).abs().max() <= 2e-2 * with_maps[n].float().abs().max(), n
+
+
+@pytest.mark.parametrize("T,extra", [(512, 1), (512, 20), (528, 148), (496, 20), (512, 149)])
+def test_units_left_over_from_whole_rounds(T, extra):
+    """2 x SMs units and `extra` more: the automatic choice, which gives up to a unit per SM of what is left to the two-stage kernel
+    (from 512 tokens on), against the one-group kernel alone.  Same products: a few elements of dw by one unit of the last place."""
+    import rwkv_cuda_b200 as R
+    from rwkv_cuda_b200 import _lib
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B, H, N = 1, 2 * sms + (extra if extra < 148 else sms + extra - 148), 64
+    g = torch.Generator(device=DEV).manual_seed(extra)
+    rn = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    kk = torch.nn.functional.normalize(rn(B, T, H, N), dim=-1)
+    r, w, k, v = ((c * rn(B, T, H, N)).bfloat16() for c in (0.5, 1.0, 0.5, 0.5))
+    x = (r, w, k, v, (-kk).bfloat16(), (kk * torch.sigmoid(rn(B, T, H, N))).bfloat16())
+    s0, dy, dsT = 0.1 * rn(B, H, N, N), rn(B, T, H, N).bfloat16(), rn(B, H, N, N)
+    y, sT, s, sa = torch.empty_like(r), torch.empty_like(s0), torch.empty(B, H, T // 16, N, N, device=DEV), torch.empty(B, T, H, N, device=DEV)
+    R.ops.wkv7_forward(s0, *x, y, sT, s, sa)
+    got = []
+    for form in (0, 1):
+        _lib.call("rwkvb200_wkv7_select_form", form)
+        try:
+            out = [torch.full_like(s0, float("nan")), *(torch.full_like(r, float("nan")) for _ in range(6))]
+            R.ops.wkv7_backward(*x, dy, dsT, s, sa, *out)
+            got.append(out)
+        finally:
+            _lib.call("rwkvb200_wkv7_select_form", 0)
+    for a, b in zip(*got):
+        assert torch.isfinite(a).all()
+        assert ((a.double() - b.double()).abs() <= 2 ** -7 * b.double().abs() + 1e-6 * b.double().abs().max()).all()
+        assert (a != b).double().mean().item() < 1e-3
+    assert _lib.lib().rwkvb200_device_status() == 0
