@@ -787,7 +787,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 // States at the start of every segment (REV: adjoints at the end), one block per unit walking its segments: S <- S diag(f) + k'^T V
 // with k'_s = k_s exp(L_end - L_s) (REV: r'_t = r_t exp(L_{t-1}), gy): all factors are at most 1.  Warps 0 to 3 have the state in
 // registers, 16 keys each, warps 4 to 11 make the operands of the segments to come (B8 T1000 H32 bf16: 80 us with four of them, two
-// sums of products at a time and states stored in pieces of 8 bytes, 63 us now: 3.7 TB/s).
+// sums of products at a time and states stored in pieces of 8 bytes, 62 us now: 3.7 TB/s; a third buffer of
+// operands changed nothing).
 template <typename E>
 struct ChainSmem {
     unsigned char A[3 * kImg], B[kParts<E> * kImg];
