@@ -874,8 +874,8 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
                 const float2 a = decode(x.aa[i]);
                 float2 e;
                 if constexpr (STATIC) {
-                    const float m = (float)(REV ? t0 + i : max(n - 1 - (t0 + i), 0));
-                    e = make_float2(d[0].x * m, d[0].y * m);
+                    const int m = REV ? t0 + i : max(n - 1 - (t0 + i), 0);
+                    e = m == 0 ? make_float2(0.f, 0.f) : make_float2(d[0].x * m, d[0].y * m);   // (also for a decay of 0, whose logarithm is -inf)
                 } else {
                     float2& s = REV ? before : after;
                     e = s;

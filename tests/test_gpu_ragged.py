@@ -156,3 +156,33 @@ def test_rwkv5_fp32_by_products(B, T, H):
     for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
         err = ((a.double().cpu().reshape(b.shape) - b).norm() / b.norm()).item()
         assert err <= 1e-6, f"{name}: {err:.3e}"
+
+
+# states by a walk along the segments (more than a unit per two SMs) and by a scan over them; products and (1, 40, 3) token by token
+@pytest.mark.parametrize("B,T,H,dtype", [(5, 40, 64, torch.float32), (2, 333, 40, BF), (1, 1000, 32, torch.float32), (1, 40, 3, torch.float32)])
+@pytest.mark.parametrize("w0", [95.0, 88.5, 20.0])
+def test_rwkv5_decay_of_zero(w0, B, T, H, dtype):
+    """exp(-exp(w0)) is 0 and (above 88.3) its logarithm -inf: a token reaches the next one only.  Bounds as above; dL/dw of such a
+    channel is -inf * 0 in fp32 and is left out."""
+    import rwkv_cuda_b200 as R
+    g = Hh.gen(T)
+    N, C = 64, H * 64
+    r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
+    u, gy, w = Hh.rand(g, H, N, lo=-1, hi=1), Hh.randn(g, B, T, C), Hh.rand(g, H, N, lo=-6, hi=-1)
+    w[1, 5] = w[2, 63] = w0
+    xs = [x.to(dtype).cuda().requires_grad_(True) for x in (r, k, v, w, u)]
+    y = R.functions.WKV_5.apply(B, T, C, H, *xs)
+    got = [y, *torch.autograd.grad(y, xs, gy.to(dtype).cuda())]
+    xo = [x.to(dtype).double().requires_grad_(True) for x in (r, k, v, w, u)]
+    yo = O.wkv5(*xo, H)
+    want = [yo, *torch.autograd.grad(yo, xo, gy.to(dtype).double())]
+    for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
+        a = a.detach().double().cpu().reshape(b.shape)
+        if name == "gw":
+            a, b = (torch.where(w == w0, torch.zeros_like(x), x) for x in (a, b))
+        if dtype == BF:
+            err = ((a - b).abs() / torch.maximum(b.abs(), b.square().mean().sqrt())).max().item()
+            assert err <= 2 ** -8 + 2 ** -15, f"{name}: {err:.3e}"
+        else:
+            err = ((a - b).norm() / b.norm()).item()
+            assert err <= 2e-6, f"{name}: {err:.3e}"
