@@ -23,8 +23,9 @@
 // subtracted and states read where they are used), y 103 us (110 with four blocks per SM and 125 registers a thread instead of five
 // and 96).  3700 instructions a warp, 324 of them mma: issue slots and the latency of 16 warps per SM (128 registers a thread) bound
 // it, the tensor pipe is busy 30 % of the time.
-// A segment whose decays leave the range (more than kRange between its middle and an end) or that holds values that are not
-// finite (a masked product would spread them over tokens before) is flagged and left to the token-by-token kernels.
+// A segment whose decays leave the range (more than kRange between its middle and an end), that holds values that are not
+// finite (a masked product would spread them over tokens before) or whose results are not (a state that is not finite; scaled operands
+// whose product overflows although the result would not) is flagged and left to the token-by-token kernels.
 #pragma once
 #include "seg_tiles.cuh"
 
@@ -439,7 +440,6 @@ __global__ void __launch_bounds__(128, 5) seg_mma_y_kernel(int T, int H, int nse
         if (tid == 0) flags[blockIdx.x] = 1;
         return;
     }
-    if (tid == 0) flags[blockIdx.x] = 0;
     // A: three of the warps a 16 x 16 tile each, and which three turns with the block (a warp's number is its scheduler)
     const int job = (warp + blockIdx.x) & 3;
     if (job < 3) {
@@ -494,6 +494,13 @@ __global__ void __launch_bounds__(128, 5) seg_mma_y_kernel(int T, int H, int nse
             const int t = 16 * mt + g + 8 * e;
             if (t < n) store_four(y_ + base + (i64)t * C + 16 * warp + 4 * q, acc[mt][0][2 * e], acc[mt][0][2 * e + 1], acc[mt][1][2 * e], acc[mt][1][2 * e + 1], vec);
         }
+    float wrong = 0.f;
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) check(wrong, make_float2(acc[mt][0][e], acc[mt][1][e]));
+    bad = __syncthreads_or(wrong != 0.f);   // a state that is not finite, or a product that left the range of fp32
+    if (tid == 0) flags[blockIdx.x] = bad;
 }
 
 // Gradients of a segment from its start state S and the adjoint D behind it.  One block per (unit, segment), 4 warps; a warp has
@@ -545,7 +552,6 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         if (tid == 0) flags[blockIdx.x] = 1;
         return;
     }
-    if (tid == 0) flags[blockIdx.x] = 0;
     const bool vec = vec_ok(gr_, 4) && vec_ok(gk_, 4) && vec_ok(gv_, 4) && (STATIC || vec_ok(gw_, 4));
     // the two token x token matrices, 16 x 16 tiles (0,0), (0,1), (1,1): A six partial products each; G one (bf16) or six (fp32)
     for (int job = (warp + blockIdx.x) & 3; job < 6; job = job >= 3 && NV == 1 ? job + 1 : NV == 1 ? 6 : job + 4) {
@@ -566,6 +572,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
                          s < t + 1 ? z : diag && s == t + 1 ? sm.o.ruk[s] : 0.f);
             }
     }
+    float wrong = 0.f;
     const i64 so = (i64)blockIdx.x * kN * kN + (16 * warp + at16(g)) * kN + 4 * q;
     float4 s4[2][2], x4[2][2];   // S and D of 16 values: of this step and of the next, [tile]
     auto read_states = [&](int kk) {
@@ -614,6 +621,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             for (int e = 0; e < 2; ++e) {
                 const int t = 16 * mt + g + 8 * e;
                 if (t < n) store_four(gv_ + base + (i64)t * C + 16 * warp + 4 * q, acc[mt][0][2 * e], acc[mt][0][2 * e + 1], acc[mt][1][2 * e], acc[mt][1][2 * e + 1], vec);
+                check(wrong, make_float2(acc[mt][0][2 * e], acc[mt][0][2 * e + 1]));
+                check(wrong, make_float2(acc[mt][1][2 * e], acc[mt][1][2 * e + 1]));
             }
     }
     // dk~ = V D'^T + G R~, dr~ = gY S'^T + G^T K~
@@ -722,8 +731,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             P[b][i] = r[i] * yr;
             x[b][i] = fmaf(k[i], yk, -P[b][i]);
             gu[i] = fmaf(gm, r[i] * k[i], gu[i]);
-            yk = fmaf(gm * u[i], r[i], yk);
-            yr = fmaf(gm * u[i], k[i], yr);
+            yk = fmaf(u[i] * r[i], gm, yk);   // (in the order of the token-by-token kernels, which cannot overflow where the result does not)
+            yr = fmaf(u[i] * k[i], gm, yr);
         }
     }
 #pragma unroll
@@ -762,6 +771,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             gu[i] += __shfl_xor_sync(0xffffffffu, gu[i], m);
             if (STATIC) gw[i] += __shfl_xor_sync(0xffffffffu, gw[i], m);
         }
+        // (the sum over all tokens in the first one's: every P and Q of the key is in it, and so every gr and gk)
+        check(wrong, make_float2(STATIC ? gw[i] : x[0][i], gu[i]));
     }
     if (g == 0) {
         float* p = partial_ + (unit / H * nseg + seg) * (STATIC ? 2 : 1) * C + h * kN + c;
@@ -782,6 +793,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
                            -ex2(kLog2e * w1.y) * x[b][3], vec);
         }
     }
+    bad = __syncthreads_or(wrong != 0.f);
+    if (tid == 0) flags[blockIdx.x] = bad;
 }
 
 // States at the start of every segment (REV: adjoints at the end), one block per unit walking its segments: S <- S diag(f) + k'^T V

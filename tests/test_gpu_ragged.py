@@ -186,3 +186,27 @@ def test_rwkv5_decay_of_zero(w0, B, T, H, dtype):
         else:
             err = ((a - b).norm() / b.norm()).item()
             assert err <= 2e-6, f"{name}: {err:.3e}"
+
+
+@pytest.mark.parametrize("name", ["gy", "k", "r"])
+def test_rwkv6_products_that_overflow(name):
+    """Decays just inside the range of the matrix form and a tensor of 1e20: scaled operands times it leave fp32's range, the results do
+    not.  Bounds as above."""
+    import rwkv_cuda_b200 as R
+    B, T, H, N = 2, 333, 40, 64
+    g = Hh.gen(1)
+    C = H * N
+    x = {n: 0.5 * Hh.randn(g, B, T, C) for n in ("r", "k", "v", "gy")}
+    x[name] *= 1e20
+    w, u = Hh.randn(g, B, T, C) - 5.0, Hh.rand(g, H, N, lo=-1, hi=1)
+    w.view(B, T, H, N)[..., 9] = 1.2   # 16 exp(1.2) log2(e) = 77
+    xs = [a.to(BF).cuda().requires_grad_(True) for a in (x["r"], x["k"], x["v"], w, u)]
+    y = R.functions.WKV_6.apply(B, T, C, H, *xs)
+    got = [y, *torch.autograd.grad(y, xs, x["gy"].to(BF).cuda())]
+    xo = [a.to(BF).double().requires_grad_(True) for a in (x["r"], x["k"], x["v"], w, u)]
+    yo = O.wkv6(*xo, H)
+    want = [yo, *torch.autograd.grad(yo, xo, x["gy"].to(BF).double())]
+    for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
+        size = torch.maximum(b.abs(), b.square().mean().sqrt())
+        err = ((a.double().cpu().reshape(b.shape) - b).abs() / size).max().item()
+        assert err <= 2 ** -8 + 2 ** -15, f"{name}: {err:.3e}"
