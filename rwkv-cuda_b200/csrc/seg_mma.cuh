@@ -913,6 +913,7 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
     }
     // ---- the state: keys 16 warp + at16(g), + 2 of all values -----------------------------------------------------------------------
     const int g = lane >> 2, q = lane & 3;
+    const uint32_t fa = frag_cols(0, 2 * warp, lane), fb = frag_rows(0, 0, lane);   // (an even piece further on: XOR, see img_at)
     float s[8][4];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
@@ -929,35 +930,52 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
         bar_join<1>(it & 1);
         const ChainSmem<E>& sm = buf[it & 1];
         const float f0 = sm.f[16 * warp + at16(g)], f1 = sm.f[16 * warp + at16(g) + 2];
-        // bf16: straight onto the state, eight sums side by side; fp32: products apart (see mma_split)
-        float c[4][1][2][4];
+        // The segment's own sums from zero, four side by side, then one rounded multiply-add per state element: the tensor core's sums are
+        // cut off, not rounded, and with the state itself as the accumulator that adds up along the sequence.  Errors of the states in norm
+        // (B2 T1000 H40; local sums and a scan in fp32 / state as accumulator / this): decay inputs around -10 6.4e-6 (there the rounding of
+        // the decays themselves) / 2.3e-6 / 2.1e-7, -5 3.1e-7 / 3.9e-7 / 1.2e-7, -1 5.7e-8 / 6.5e-8 / 6.7e-8, 1 3.0e-8 / 5.0e-8 / 5.0e-8
+        // (one cut of the newest tokens' sum).  B8 T1000 H32 497 -> 501 us.
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int half = 0; half < 2; ++half) {
+            float c[2][1][2][4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) c[i / 2][0][i & 1][e] = sizeof(E) == 4 ? 0.f : s[i][e] * (e < 2 ? f0 : f1);
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int kt = 0; kt < 2; ++kt) {
-            uint32_t a[1][3][4], b[4][NV][4];
-            ldsm_t<3>(a[0], smem_addr(sm.A) + frag_cols(16 * kt, 2 * warp, lane));
-#pragma unroll
-            for (int i = 0; i < 4; ++i) ldsm_t<NV>(b[i], smem_addr(sm.B) + frag_rows(16 * kt, 2 * i, lane));
+                for (int e = 0; e < 4; ++e) c[i / 2][0][i & 1][e] = 0.f;
             if constexpr (NV == 1) {
+                uint32_t b[2][2][4];
 #pragma unroll
-                for (int pa = 2; pa >= 0; --pa)
+                for (int kt = 0; kt < 2; ++kt)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        mma(c[i][0][0], a[0][pa], b[i][0][0], b[i][0][1]);
-                        mma(c[i][0][1], a[0][pa], b[i][0][2], b[i][0][3]);
+                    for (int i = 0; i < 2; ++i) ldsm_t(b[kt][i], smem_addr(sm.B) + 16 * kt * 128 + (fb ^ (4 * half + 2 * i) << 4));
+#pragma unroll
+                for (int pa = 2; pa >= 0; --pa)   // the small parts of all tokens first: what is cut off behind them is small too
+#pragma unroll
+                    for (int kt = 0; kt < 2; ++kt) {
+                        uint32_t a[4];
+                        ldsm_t(a, smem_addr(sm.A) + pa * kImg + 16 * kt * 128 + fa);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            mma(c[i][0][0], a, b[kt][i][0], b[kt][i][1]);
+                            mma(c[i][0][1], a, b[kt][i][2], b[kt][i][3]);
+                        }
                     }
             } else {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) mma_split<true, 1, 3, NV>(c[i], a, b[i]);
+                for (int kt = 0; kt < 2; ++kt) {
+                    uint32_t a[1][3][4], b[2][NV][4];
+                    ldsm_t<3>(a[0], smem_addr(sm.A) + 16 * kt * 128 + fa);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) ldsm_t<NV>(b[i], smem_addr(sm.B) + 16 * kt * 128 + (fb ^ (4 * half + 2 * i) << 4));
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) mma_split<true, 1, 3, NV>(c[i], a, b[i]);
+                }
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[4 * half + i][e] = fmaf(s[4 * half + i][e], e < 2 ? f0 : f1, c[i / 2][0][i & 1][e]);
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) s[i][e] = sizeof(E) == 4 ? fmaf(s[i][e], e < 2 ? f0 : f1, c[i / 2][0][i & 1][e]) : c[i / 2][0][i & 1][e];
         if (it + 3 < nseg) bar_tell<3>(it & 1);
     }
 }

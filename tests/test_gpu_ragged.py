@@ -210,3 +210,30 @@ def test_rwkv6_products_that_overflow(name):
         size = torch.maximum(b.abs(), b.square().mean().sqrt())
         err = ((a.double().cpu().reshape(b.shape) - b).abs() / size).max().item()
         assert err <= 2 ** -8 + 2 ** -15, f"{name}: {err:.3e}"
+
+
+@pytest.mark.parametrize("shift", [-10.0, -5.0])
+def test_rwkv6_states_of_the_walk(shift):
+    """fp32 states at the start of every segment (left for the backward), with slow decays: sums over the whole sequence.  Bound: one rounding
+    per segment at the size of the state, 32 of them at random, and four at the size of a segment's own sum, all 2^-24."""
+    import rwkv_cuda_b200 as R
+    B, T, H, N = 2, 1000, 40, 64   # (more than a unit per two SMs: by the walk)
+    g = Hh.gen(3)
+    C, nseg = H * N, (T + 31) // 32
+    r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
+    w, u = Hh.randn(g, B, T, C) + shift, Hh.rand(g, H, N, lo=-1, hi=1)
+    d = [x.to(BF).cuda() for x in (r, k, v, w, u)]
+    y = torch.empty_like(d[0])
+    saved = torch.empty(R._lib.lib().rwkvb200_wkv6_train_saved_bytes(R._lib.BF16, B, T, C, H) // 4 + 1, device="cuda")
+    rc = R._lib.lib().rwkvb200_wkv6_train_forward(R._lib.BF16, B, T, C, H, *(x.data_ptr() for x in d), None, y.data_ptr(), None, saved.data_ptr(),
+                                                  torch.cuda.current_stream().cuda_stream)
+    assert rc == 2, rc
+    got = saved[:B * H * nseg * N * N].view(B, H, nseg, N, N).double()
+    kk, vv, dd = (x.double().view(B, T, H, N) for x in (d[1], d[2], torch.exp(-torch.exp(d[3].double()))))
+    S = torch.zeros(B, H, N, N, dtype=torch.float64, device="cuda")
+    err = size = 0.0
+    for t in range(T):
+        if t % 32 == 0:
+            err, size = err + (got[:, :, t // 32] - S).square().sum().item(), size + S.square().sum().item()
+        S = S * dd[:, t, :, :, None] + kk[:, t, :, :, None] * vv[:, t, :, None, :]
+    assert (err / size) ** 0.5 <= (32 ** 0.5 + 4) * 2 ** -24, (err / size) ** 0.5
