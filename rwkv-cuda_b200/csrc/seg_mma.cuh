@@ -817,6 +817,35 @@ __device__ __forceinline__ void bar_tell(int odd) {
     if (odd) asm volatile("bar.arrive %0, 384;" ::"n"(ID + 1) : "memory");
     else asm volatile("bar.arrive %0, 384;" ::"n"(ID) : "memory");
 }
+// The same walk once more, where a state has come out not finite: as the local sums and the scan do it, in fp32 with one multiply-add
+// per token.  (By products the parts of an infinity, and an infinity against a part that is 0, make NaN where these have an infinity.)
+template <typename E, bool STATIC, bool REV>
+__device__ __noinline__ void walk_again(int T, int nseg, int C, const E* a_, const E* b_, const E* w_, float* states) {
+    const int j = threadIdx.x >> 2, i0 = 16 * (threadIdx.x & 3);   // a key, 16 values
+    if (j >= kN) return;
+    float S[16], c[16], lw = 0.f, f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) S[i] = 0.f;
+    if (STATIC) lw = -expf(to_f(w_[j]));
+    for (int it = 0; it < nseg; ++it) {
+        const int seg = REV ? nseg - 1 - it : it, n = min(kSeg, T - seg * kSeg);
+        float* p = states + (i64)seg * kN * kN + j * kN + i0;
+        f = 1.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { p[i] = S[i]; c[i] = 0.f; }
+        for (int q = 0; q < n; ++q) {
+            const i64 o = ((i64)seg * kSeg + (REV ? q : n - 1 - q)) * C;
+            if (STATIC) f = q == 0 ? 1.f : expf(lw * (float)q);
+            const float a = to_f(a_[o + j]) * f;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) c[i] = fmaf(a, to_f(b_[o + i0 + i]), c[i]);
+            if (!STATIC) f *= expf(-expf(to_f(w_[o + j])));
+        }
+        if (STATIC) f = expf(lw * (float)n);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) S[i] = fmaf(S[i], f, c[i]);
+    }
+}
 template <typename E, bool STATIC, bool REV>
 __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_kernel(int T, int H, int nseg, const E* __restrict__ a_, const E* __restrict__ b_,
                                                                const E* __restrict__ w_, float* __restrict__ states) {
@@ -826,6 +855,7 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
     const i64 unit = blockIdx.x;
     const int h = unit % H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, C = H * kN;
     const i64 base = unit / H * T * C + h * kN;
+    float wrong = 0.f;
     if (warp >= 4) {
         // ---- operands: channels 2 lane, 2 lane + 1 of four tokens ----------------------------------------------------------
         constexpr int R = 4;
@@ -909,75 +939,81 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
             make(raw[0], it);
             if (it + 2 < nseg) make(raw[1], it + 1);
         }
-        return;
-    }
-    // ---- the state: keys 16 warp + at16(g), + 2 of all values -----------------------------------------------------------------------
-    const int g = lane >> 2, q = lane & 3;
-    const uint32_t fa = frag_cols(0, 2 * warp, lane), fb = frag_rows(0, 0, lane);   // (an even piece further on: XOR, see img_at)
-    float s[8][4];
+    } else {
+        // ---- the state: keys 16 warp + at16(g), + 2 of all values -----------------------------------------------------------------------
+        const int g = lane >> 2, q = lane & 3;
+        const uint32_t fa = frag_cols(0, 2 * warp, lane), fb = frag_rows(0, 0, lane);   // (an even piece further on: XOR, see img_at)
+        float s[8][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[i][e] = 0.f;
-    for (int it = 0; it < nseg; ++it) {
-        float* p = states + (unit * nseg + (REV ? nseg - 1 - it : it)) * kN * kN + (16 * warp + at16(g)) * kN + 4 * q;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int e = 0; e < 2; ++e)
-                *reinterpret_cast<float4*>(p + 2 * e * kN + 16 * i) = make_float4(s[2 * i][2 * e], s[2 * i][2 * e + 1], s[2 * i + 1][2 * e], s[2 * i + 1][2 * e + 1]);
-        if (it + 1 == nseg) break;
-        bar_join<1>(it & 1);
-        const ChainSmem<E>& sm = buf[it & 1];
-        const float f0 = sm.f[16 * warp + at16(g)], f1 = sm.f[16 * warp + at16(g) + 2];
-        // The segment's own sums from zero, four side by side, then one rounded multiply-add per state element: the tensor core's sums are
-        // cut off, not rounded, and with the state itself as the accumulator that adds up along the sequence.  Errors of the states in norm
-        // (B2 T1000 H40; local sums and a scan in fp32 / state as accumulator / this): decay inputs around -10 6.4e-6 (there the rounding of
-        // the decays themselves) / 2.3e-6 / 2.1e-7, -5 3.1e-7 / 3.9e-7 / 1.2e-7, -1 5.7e-8 / 6.5e-8 / 6.7e-8, 1 3.0e-8 / 5.0e-8 / 5.0e-8
-        // (one cut of the newest tokens' sum).  B8 T1000 H32 497 -> 501 us.
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float c[2][1][2][4];
+            for (int e = 0; e < 4; ++e) s[i][e] = 0.f;
+        for (int it = 0; it < nseg; ++it) {
+            float* p = states + (unit * nseg + (REV ? nseg - 1 - it : it)) * kN * kN + (16 * warp + at16(g)) * kN + 4 * q;
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) c[i / 2][0][i & 1][e] = 0.f;
-            if constexpr (NV == 1) {
-                uint32_t b[2][2][4];
+                for (int e = 0; e < 2; ++e)
+                    *reinterpret_cast<float4*>(p + 2 * e * kN + 16 * i) = make_float4(s[2 * i][2 * e], s[2 * i][2 * e + 1], s[2 * i + 1][2 * e], s[2 * i + 1][2 * e + 1]);
+            if (it + 1 == nseg) break;
+            bar_join<1>(it & 1);
+            const ChainSmem<E>& sm = buf[it & 1];
+            const float f0 = sm.f[16 * warp + at16(g)], f1 = sm.f[16 * warp + at16(g) + 2];
+            // The segment's own sums from zero, four side by side, then one rounded multiply-add per state element: the tensor core's sums are
+            // cut off, not rounded, and with the state itself as the accumulator that adds up along the sequence.  Errors of the states in norm
+            // (B2 T1000 H40; local sums and a scan in fp32 / state as accumulator / this): decay inputs around -10 6.4e-6 (there the rounding of
+            // the decays themselves) / 2.3e-6 / 2.1e-7, -5 3.1e-7 / 3.9e-7 / 1.2e-7, -1 5.7e-8 / 6.5e-8 / 6.7e-8, 1 3.0e-8 / 5.0e-8 / 5.0e-8
+            // (one cut of the newest tokens' sum).  B8 T1000 H32 497 -> 501 us.
 #pragma unroll
-                for (int kt = 0; kt < 2; ++kt)
+            for (int half = 0; half < 2; ++half) {
+                float c[2][1][2][4];
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) ldsm_t(b[kt][i], smem_addr(sm.B) + 16 * kt * 128 + (fb ^ (4 * half + 2 * i) << 4));
+                for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int pa = 2; pa >= 0; --pa)   // the small parts of all tokens first: what is cut off behind them is small too
+                    for (int e = 0; e < 4; ++e) c[i / 2][0][i & 1][e] = 0.f;
+                if constexpr (NV == 1) {
+                    uint32_t b[2][2][4];
+#pragma unroll
+                    for (int kt = 0; kt < 2; ++kt)
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) ldsm_t(b[kt][i], smem_addr(sm.B) + 16 * kt * 128 + (fb ^ (4 * half + 2 * i) << 4));
+#pragma unroll
+                    for (int pa = 2; pa >= 0; --pa)   // the small parts of all tokens first: what is cut off behind them is small too
+#pragma unroll
+                        for (int kt = 0; kt < 2; ++kt) {
+                            uint32_t a[4];
+                            ldsm_t(a, smem_addr(sm.A) + pa * kImg + 16 * kt * 128 + fa);
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                mma(c[i][0][0], a, b[kt][i][0], b[kt][i][1]);
+                                mma(c[i][0][1], a, b[kt][i][2], b[kt][i][3]);
+                            }
+                        }
+                } else {
 #pragma unroll
                     for (int kt = 0; kt < 2; ++kt) {
-                        uint32_t a[4];
-                        ldsm_t(a, smem_addr(sm.A) + pa * kImg + 16 * kt * 128 + fa);
+                        uint32_t a[1][3][4], b[2][NV][4];
+                        ldsm_t<3>(a[0], smem_addr(sm.A) + 16 * kt * 128 + fa);
 #pragma unroll
-                        for (int i = 0; i < 2; ++i) {
-                            mma(c[i][0][0], a, b[kt][i][0], b[kt][i][1]);
-                            mma(c[i][0][1], a, b[kt][i][2], b[kt][i][3]);
-                        }
+                        for (int i = 0; i < 2; ++i) ldsm_t<NV>(b[i], smem_addr(sm.B) + 16 * kt * 128 + (fb ^ (4 * half + 2 * i) << 4));
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) mma_split<true, 1, 3, NV>(c[i], a, b[i]);
                     }
-            } else {
-#pragma unroll
-                for (int kt = 0; kt < 2; ++kt) {
-                    uint32_t a[1][3][4], b[2][NV][4];
-                    ldsm_t<3>(a[0], smem_addr(sm.A) + 16 * kt * 128 + fa);
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) ldsm_t<NV>(b[i], smem_addr(sm.B) + 16 * kt * 128 + (fb ^ (4 * half + 2 * i) << 4));
-#pragma unroll
-                    for (int i = 0; i < 2; ++i) mma_split<true, 1, 3, NV>(c[i], a, b[i]);
                 }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[4 * half + i][e] = fmaf(s[4 * half + i][e], e < 2 ? f0 : f1, c[i / 2][0][i & 1][e]);
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[4 * half + i][e] = fmaf(s[4 * half + i][e], e < 2 ? f0 : f1, c[i / 2][0][i & 1][e]);
+            if (it + 3 < nseg) bar_tell<3>(it & 1);
         }
-        if (it + 3 < nseg) bar_tell<3>(it & 1);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {   // (what is not finite stays so: the last state tells)
+            check(wrong, make_float2(s[i][0], s[i][1]));
+            check(wrong, make_float2(s[i][2], s[i][3]));
+        }
     }
+    if (__syncthreads_or(wrong != 0.f)) walk_again<E, STATIC, REV>(T, nseg, C, a_ + base, b_ + base, w_ + (STATIC ? h * kN : base), states + unit * nseg * kN * kN);
 }
 
 // ---- the segments that the kernels above have left ----------------------------------------------------------------------------

@@ -237,3 +237,31 @@ def test_rwkv6_states_of_the_walk(shift):
             err, size = err + (got[:, :, t // 32] - S).square().sum().item(), size + S.square().sum().item()
         S = S * dd[:, t, :, :, None] + kk[:, t, :, :, None] * vv[:, t, :, None, :]
     assert (err / size) ** 0.5 <= (32 ** 0.5 + 4) * 2 ** -24, (err / size) ** 0.5
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("name", ["r", "k", "v", "gy"])
+@pytest.mark.parametrize("op", ["wkv6", "wkv5 fp32"])
+def test_values_that_are_not_finite_as_token_by_token(op, name, value):
+    """y and gradients of two heads in a call with many heads (states by the walk, the rest by products) and in one with these two only
+    (token by token): infinities, NaN and numbers in the same places."""
+    import rwkv_cuda_b200 as R
+    B, T, N, t, H = 1, 103, 64, 45, 160
+    dtype, F = (BF, R.functions.WKV_6) if op == "wkv6" else (torch.float32, R.functions.WKV_5)
+    g = Hh.gen(5)
+    x = {n: 0.5 * Hh.randn(g, B, T, H, N) for n in ("r", "k", "v", "gy")}
+    x["w"] = Hh.randn(g, B, T, H, N) - 4.0 if op == "wkv6" else Hh.rand(g, H, N, lo=-6, hi=-1)
+    x["u"] = Hh.rand(g, H, N, lo=-1, hi=1)
+    x[name][:, t, 0, 7] = value
+
+    def call(H):
+        xs = [(x[n][:, :, :H].reshape(B, T, H * N) if x[n].dim() == 4 else x[n][:H]).to(dtype).cuda().contiguous().requires_grad_(n != "gy")
+              for n in ("r", "k", "v", "w", "u", "gy")]
+        y = F.apply(B, T, H * N, H, *xs[:5])
+        out = [y, *torch.autograd.grad(y, xs[:5], xs[5])]
+        return [(z.view(B, T, H, N)[:, :, :2] if z.dim() == 3 else z.view(H, N)[:2]).float() for z in out]
+
+    for a, b, out in zip(call(H), call(2), ("y", "gr", "gk", "gv", "gw", "gu")):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isposinf(), b.isposinf()) and torch.equal(a.isneginf(), b.isneginf()), out
+        a, b = (torch.where(z.isfinite(), z, torch.zeros_like(z)) for z in (a, b))
+        assert ((a - b).abs() / torch.maximum(b.abs(), b.square().mean().sqrt())).max().item() <= (2 ** -7 if dtype == BF else 2e-5), out
