@@ -19,11 +19,13 @@
 // the eight dot products of a row are reduced together (8 shuffles, not 4 per token), 17 vectors are read instead of 20, and the
 // chain has one reduction per four tokens.  NCW warps compute; NSW warps stage, a step each: they make the scaled vectors (products of
 // decays are carried as sums of two numbers: a vector is rounded once) and the 32 scalars of a step, which all rows share.
-// One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 213 us with a token as a step, 205 us here; 128 units
+// One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 213 us with a token as a step, 203 us here; 128 units
 // 427 -> 380 us, 256 units 852 -> 670 us.  A step takes 790 clocks where a unit has four SMs: 350 of the shared-memory reads, the
 // rest 430 instructions per scheduler, of one warp that computes and one or two that stage (four staging warps 209 us, eight 201; with
 // more rows per block eight were slower: 128 units 411 us).
-// Errors of the state against fp64 9.1e-8 of the norm (a token as a step 8.3e-8: the same fp32 sums in another order), y as before.
+// Errors against fp64 (T 1999, H 8, of the norm): state 8.3e-8, y 1.11e-7; a token as a step 8.7e-8 and 1.12e-7.  Most of the state is of the last
+// few tokens, and where all eight terms of a step went onto it one by one, each was rounded at its full size (9.3e-8, 1.14e-7); so
+// the four of sa are summed first.
 #include "common.cuh"
 #include "packed.cuh"
 #include "wkv7_dispatch.cuh"
@@ -366,6 +368,8 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
                     sa[t][i] = z[t];
                 }
             }
+            // sum sa_s b^_s by itself, then onto the state (one rounding at the size of the state, not four)
+            f2 sb[RPT][KP];
 #pragma unroll
             for (int t = 0; t < kQ; ++t) {
                 const Keys<LG> b = load_keys<LG>(s.b[t], x);
@@ -373,9 +377,13 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
                 for (int i = 0; i < RPT; ++i) {
                     const f2 sv = pack2(sa[t][i], sa[t][i]);
 #pragma unroll
-                    for (int e = 0; e < KP; ++e) S[i][e] = fma2(b.x[e], sv, S[i][e]);
+                    for (int e = 0; e < KP; ++e) sb[i][e] = t ? fma2(b.x[e], sv, sb[i][e]) : mul2(b.x[e], sv);
                 }
             }
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+#pragma unroll
+                for (int e = 0; e < KP; ++e) S[i][e] = add2(S[i][e], sb[i][e]);
             float y[RPT];
 #pragma unroll
             for (int i = 0; i < RPT; ++i) {
