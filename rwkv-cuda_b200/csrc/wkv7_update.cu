@@ -119,7 +119,7 @@ __device__ __forceinline__ float dot_keys(const f2 (&s)[32 / LG], const Keys<LG>
 constexpr int kQ = 4;   // tokens of a step
 // The scaled vectors of a step, the products of its decays (w), its values, and the scalars of the steps inside it: b, k of token s
 // against a of token t (s < t) at ((t - 1) t / 2 + s) * 2, then against r of token t (s <= t, zero above) at 12 + 8 t + 2 s.
-struct __align__(16) Step { float a[kQ][kN], r[kQ][kN], b[kQ][kN], k[kQ][kN], w[kN], v[kQ][kN], u[12 + 8 * kQ]; };
+struct __align__(16) Step { float a[kQ][kN], r[kQ][kN], b[kQ][kN], k[kQ][kN], w[kN], v[kQ][kN], u[12 + 8 * kQ]; int odd; };
 template <int NSW>
 struct __align__(16) Staged { Step s[NSW]; };   // a step per staging warp
 
@@ -190,6 +190,65 @@ __device__ __forceinline__ void store_rows(E* p, const float (&y)[RPT]) {
     }
 }
 
+// sums that are 0 unless one of the values is not finite
+__device__ __forceinline__ void check(float& bad, float x) { bad = fmaf(x, 0.f, bad); }
+
+// The rows of a warp once more, token by token from the state in memory: with values that are not finite the sums over four tokens are
+// others than token by token (infinities of both signs meet, parts of a product are infinity times 0), and NaN would stand where the
+// recurrence gives an infinity.  S_t = G_t + sa_t b_t with G_t = S_{t-1} d_t + v_t k_t, and sa_{t+1} = G_t.a_{t+1} + sa_t (b_t.a_{t+1}).
+// What is a number in both forms stays as it is (other: the state by steps of four): in what order it was summed does not depend on
+// a value beyond its reach.
+template <typename E, int LG, int RPT>
+__device__ __noinline__ void rows_again(int T, int C, i64 base, int row0, int x, float* st, const E* r_, const E* w_, const E* k_, const E* v_,
+                                        const E* a_, const E* b_, E* y_, const float (&other)[RPT][64 / LG]) {
+    constexpr int K = 64 / LG;
+    auto sum = [](float p) {
+#pragma unroll
+        for (int m = 1; m < LG; m <<= 1) p += __shfl_xor_sync(0xffffffffu, p, m);
+        return p;
+    };
+    const i64 key = base + first_key<LG>(x);
+    float S[RPT][K], sa[RPT];
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        float p = 0.f;
+#pragma unroll
+        for (int j = 0; j < K; ++j) { S[i][j] = st[i * kN + j]; p = fmaf(S[i][j], to_f(a_[key + j]), p); }
+        sa[i] = sum(p);
+    }
+    for (int t = 0; t < T; ++t) {
+        const i64 o = (i64)t * C;
+        float d[K], k[K], b[K], r[K], an[K], beta = 0.f;
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            d[j] = decay7(to_f(w_[o + key + j])); k[j] = to_f(k_[o + key + j]); b[j] = to_f(b_[o + key + j]); r[j] = to_f(r_[o + key + j]);
+            an[j] = t + 1 < T ? to_f(a_[o + C + key + j]) : 0.f;
+            beta = fmaf(b[j], an[j], beta);
+        }
+        beta = sum(beta);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const float v = to_f(v_[o + base + row0 + i]);
+            float z = 0.f, y = 0.f;
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+                S[i][j] = fmaf(S[i][j], d[j], k[j] * v);
+                z = fmaf(S[i][j], an[j], z);
+                S[i][j] = fmaf(sa[i], b[j], S[i][j]);
+                y = fmaf(S[i][j], r[j], y);
+            }
+            y = sum(y);
+            sa[i] = fmaf(sa[i], beta, sum(z));
+            E* p = y_ + o + base + row0 + i;
+            if (x == 0 && !(isfinite(y) && isfinite(to_f(*p)))) *p = from_f<E>(y);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
+#pragma unroll
+        for (int j = 0; j < K; ++j) st[i * kN + j] = isfinite(S[i][j]) && isfinite(other[i][j]) ? other[i][j] : S[i][j];
+}
+
 // grid (units, 64 LG / (32 NCW RPT)); NCW warps compute (a warp: 32 / LG groups of LG lanes, RPT rows each), NSW warps stage
 template <typename E, int LG, int NCW, int RPT, int NSW>
 __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int H, float* __restrict__ state, const E* __restrict__ r_,
@@ -229,6 +288,7 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
             buf[0].s[q].u[12 + 8 * t + 2 * (t + 1) + x] = buf[1].s[q].u[12 + 8 * t + 2 * (t + 1) + x] = 0.f;
         }
         const int yt = lane >= 24 ? 3 : lane >= 18 ? 2 : lane >= 14 ? 1 : 0, slot = lane < 12 ? lane : 12 + 8 * yt + lane - (yt == 3 ? 24 : yt == 2 ? 18 : yt == 1 ? 14 : 12);
+        float odd = 0.f;
         fetch(0);
         for (int c = 0; c < nch; ++c) {
             const int t0 = c * kCh + q * kQ;
@@ -295,6 +355,8 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
             }
             *reinterpret_cast<float2*>(st.w + 2 * lane) = make_float2(w.hi.x + w.lo.x, w.hi.y + w.lo.y);
             st.u[slot] = u[0];
+            check(odd, u[0]);   // every r is in one of these sums; all other values reach the state
+            if (c + 1 == nch) st.odd = __any_sync(0xffffffffu, odd != 0.f);
             bar_arrive<1, NTH>(c & 1);
         }
         return;
@@ -396,6 +458,22 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
             if (x < 4 * TS && x % TS == 0 && t < T) store_rows<E, RPT>(y_ + base + (i64)t * C + row0, y);
         }
         if (c + 2 < nch) bar_arrive<3, NTH>(c & 1);
+    }
+    float bad = 0.f;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
+#pragma unroll
+        for (int e = 0; e < KP; ++e) check(bad, sum2(S[i][e]));
+    for (int q = 0; q < NSW; ++q)
+        if (buf[(nch - 1) & 1].s[q].odd) bad = 1.f;
+    if (__any_sync(0xffffffffu, bad != 0.f)) {   // (an infinity never leaves a state: d > 0.5; r does not enter it)
+        float other[RPT][2 * KP];
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+#pragma unroll
+            for (int e = 0; e < KP; ++e) unpack2(S[i][e], other[i][2 * e], other[i][2 * e + 1]);
+        rows_again<E, LG, RPT>(T, C, base, row0, x, st, r_, w_, k_, v_, a_, b_, y_, other);
+        return;
     }
 #pragma unroll
     for (int i = 0; i < RPT; ++i)

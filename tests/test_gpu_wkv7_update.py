@@ -71,3 +71,37 @@ def test_errors_of_a_prompt():
             sa = fl(sa * fl((b[t] * a[t + 1]).sum(1))[:, None] + fl((G * a[t + 1][:, None]).sum(2)))
     error = lambda z: ((z - exact).norm() / exact.norm()).item()
     assert error(state[0].double().cpu()) <= 1.02 * error(S), (error(state[0].double().cpu()), error(S))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("name", ["r", "k", "v", "a", "b", "s0"])
+@pytest.mark.parametrize("H", [2, 40, 80])   # four, two blocks and one per unit
+def test_infinities_of_the_recurrence(H, name, value, dtype):
+    """Infinities, NaN and numbers stand where the recurrence has them token by token (S_t = G_t + sa_t b_t with G_t = S_{t-1} d_t + v_t k_t,
+    sa_{t+1} = G_t.a_{t+1} + sa_t (b_t.a_{t+1})): in what order a sum over keys is taken does not change that."""
+    import rwkv_cuda_b200 as R
+    B, T, N, t, names = 1, 11, 64, 6, ("r", "w", "k", "v", "a", "b")
+    inp = {n: x.clone().reshape(B, T, H, N) if x.dim() == 3 else x.clone() for n, x in Hh.v7_inputs(B, T, H, N, seed=4).items()}
+    if name == "s0":
+        inp["s0"][0, 0, 3, 5] = value
+    else:
+        inp[name][0, t, 0, 5] = value
+    x = [inp[n].to(dtype).cuda().contiguous() for n in names]
+    state, y = inp["s0"].cuda(), torch.empty(B, T, H, N, dtype=dtype, device="cuda")
+    R.ops.wkv7_state_update(state, *x, y)
+
+    r, w, k, v, a, b = (inp[n][0, :, 0].to(dtype).double() for n in names)
+    d, S, rows = torch.exp(-0.6065306597126334 * torch.sigmoid(w)), inp["s0"][0, 0].double(), []
+    sa = (S * a[0]).sum(1)
+    for i in range(T):
+        G = S * d[i] + v[i][:, None] * k[i]
+        S = G + sa[:, None] * b[i]
+        rows.append((S * r[i]).sum(1))
+        if i + 1 < T:
+            sa = (G * a[i + 1]).sum(1) + sa * (b[i] * a[i + 1]).sum()
+    for got, want in ((y[0, :, 0], torch.stack(rows)), (state[0, 0], S)):
+        got = got.double().cpu()
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+        ok = want.isfinite()
+        assert not ok.any() or (got[ok] - want[ok]).abs().max() <= Hh.tol_for(dtype) * want[ok].abs().max()
