@@ -11,6 +11,10 @@
 //   gk_s = dk~_s exp(L_m - L_s) + gamma_s u r_s     gr_t = dr~_t exp(L_{t-1} - L_m) + gamma_t u k_t
 // and with P_t = r~_t dr~_t, Q_s = k~_s dk~_s (elementwise, without the u terms) and A_end = sum_i D S_end
 //   dL/dlog d_t = A_end - sum_{tau > t} (Q_tau - P_tau) - Q_t      A_end = sum_i D' S' + sum_s k~_s (V D'^T)_s
+// A static decay has the sum of these over the tokens, where terms that no decay acts on stand many times and cancel (error of gw at
+// decays of 0.7 per token 1.0e-6 of its norm, token by token 2.9e-7); so in fp32 every term times the number of decays in it
+// (n: tokens of the segment, t from 0), 2.0e-7:
+//   dL/dlog d = n sum_i D' S' + sum_s (n-1-s) k~_s (V D'^T)_s + sum_t t r~_t (gY S'^T)_t + sum_t r~_t sum_{s<t} (t-1-s) G[s,t] k~_s
 //
 // Precision: the products run on mma.sync with bf16 operands, every fp32 operand as the sum of three bf16 numbers (24 bits: the
 // split is exact) and all partial products down to 2^-16 of the largest taken: 3 where the other side is a bf16 tensor as it
@@ -361,6 +365,15 @@ __device__ __forceinline__ void put_tile(unsigned char* img, int tile, int row, 
     *reinterpret_cast<uint32_t*>(p + kTiles) = m;
     *reinterpret_cast<uint32_t*>(p + 2 * kTiles) = l;
 }
+// Fragments of a transposed tile (rows t0 + .., columns s0 + ..), each element times t - 1 - s
+__device__ __forceinline__ void weigh_by_distance(uint32_t (&w)[3][4], const uint32_t (&f)[3][4], int t0, int s0, int lane) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float d = (float)(t0 + (lane >> 2) + 8 * (i & 1) - 1 - (s0 + 2 * (lane & 3) + 8 * (i >> 1)));
+        const float x = bf16_lo(f[0][i]) + (bf16_lo(f[1][i]) + bf16_lo(f[2][i])), z = bf16_hi(f[0][i]) + (bf16_hi(f[1][i]) + bf16_hi(f[2][i]));
+        split3(x * d, z * (d - 1.f), w[0][i], w[1][i], w[2][i]);
+    }
+}
 template <bool TRANS>   // a tile as A fragments, as stored or transposed
 __device__ __forceinline__ void tile_frag(uint32_t (&f)[3][4], const unsigned char* img, int tile, int lane) {
     if (TRANS) ldsm_t<3, kTiles>(f, smem_addr(img) + tile_at(tile, (lane & 7) + ((lane >> 4) << 3), (lane >> 3) & 1));
@@ -521,6 +534,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     extern __shared__ __align__(128) unsigned char smem_seg_b[];
     BwdSmemM<E>& sm = *reinterpret_cast<BwdSmemM<E>*>(smem_seg_b);
     constexpr int NV = kParts<E>;
+    constexpr bool WEIGHTS = STATIC && sizeof(E) == 4;   // see dL/dlog d above (bf16: its rounding is a thousand times what cancels)
     const i64 unit = blockIdx.x / nseg;
     const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
     const int g = lane >> 2, q = lane & 3, n = min(kSeg, T - seg * kSeg);
@@ -678,7 +692,17 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
         const float4 l = *reinterpret_cast<const float4*>(sm.rows + (8 * b + g + 1) * kRld + c);
-        const float2 k0 = decode(kp[0][b]), k1 = decode(kp[1][b]);
+        float2 k0 = decode(kp[0][b]), k1 = decode(kp[1][b]);
+        if constexpr (WEIGHTS) {   // the distances to the segment's end, and to its start
+            const float4 l0 = *reinterpret_cast<const float4*>(sm.rows + (8 * b + g) * kRld + c);
+            const float2 r0 = decode(rp[0][b]), r1 = decode(rp[1][b]);
+            const float t = (float)(8 * b + g), d = (float)(n - 1) - t;
+            k0.x *= d; k0.y *= d; k1.x *= d; k1.y *= d;
+            aend[0] = fmaf(t * r0.x * ex2(l0.x), dr[b >> 1][0][2 * (b & 1)], aend[0]);
+            aend[1] = fmaf(t * r0.y * ex2(l0.y), dr[b >> 1][0][2 * (b & 1) + 1], aend[1]);
+            aend[2] = fmaf(t * r1.x * ex2(l0.z), dr[b >> 1][1][2 * (b & 1)], aend[2]);
+            aend[3] = fmaf(t * r1.y * ex2(l0.w), dr[b >> 1][1][2 * (b & 1) + 1], aend[3]);
+        }
         aend[0] = fmaf(k0.x * ex2(-l.x), dk[b >> 1][0][2 * (b & 1)], aend[0]);
         aend[1] = fmaf(k0.y * ex2(-l.y), dk[b >> 1][0][2 * (b & 1) + 1], aend[1]);
         aend[2] = fmaf(k1.x * ex2(-l.z), dk[b >> 1][1][2 * (b & 1)], aend[2]);
@@ -688,7 +712,14 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     for (int i = 0; i < 4; ++i) {
 #pragma unroll
         for (int m = 4; m < 32; m <<= 1) aend[i] += __shfl_xor_sync(0xffffffffu, aend[i], m);
-        aend[i] += sm.a0[c + i];
+        aend[i] = WEIGHTS ? fmaf((float)n, sm.a0[c + i], aend[i]) : aend[i] + sm.a0[c + i];
+    }
+    float dw[WEIGHTS ? 2 : 1][2][4];   // sum_s (t - 1 - s) G[s,t] k~_s
+    if constexpr (WEIGHTS) {
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dw[mt][0][e] = dw[mt][1][e] = 0.f;
     }
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
@@ -706,11 +737,17 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
                 tile_frag<true>(a[0], sm.Gm, mt + kt, lane);
                 ldsm_t<3>(b, smem_addr(sm.o.K) + frag_rows(16 * kt, 2 * warp, lane));
                 mma_split<sizeof(E) == 4, 1, 3, 3>(cr, a, b);
+                if constexpr (WEIGHTS) {
+                    uint32_t d[1][3][4];
+                    float(&cw)[1][2][4] = *reinterpret_cast<float(*)[1][2][4]>(&dw[mt]);
+                    weigh_by_distance(d[0], a[0], 16 * mt, 16 * kt, lane);
+                    mma_split<sizeof(E) == 4, 1, 3, 3>(cw, d, b);
+                }
             }
         }
     }
     // per token and key: scales and bonus terms, then the decay gradient
-    float P[4][4], x[4][4], gu[4] = {0.f, 0.f, 0.f, 0.f}, u[4];   // [eight tokens][key]; x = Q - P
+    float P[4][4], x[4][4], gu[4] = {0.f, 0.f, 0.f, 0.f}, gw[4] = {0.f, 0.f, 0.f, 0.f}, u[4];   // [eight tokens][key]; x = Q - P
     {
         const bool vu = vec_ok(u_, 2);
         const float2 u0 = decode(read_pair(u_ + h * kN + c, vu)), u1 = decode(read_pair(u_ + h * kN + c + 2, vu));
@@ -727,9 +764,16 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         for (int i = 0; i < 4; ++i) {
             float &yk = dk[mt][i >> 1][2 * e + (i & 1)], &yr = dr[mt][i >> 1][2 * e + (i & 1)];
             yk *= ex2(-behind[i]);
-            yr *= ex2(before[i]);
-            P[b][i] = r[i] * yr;
-            x[b][i] = fmaf(k[i], yk, -P[b][i]);
+            if constexpr (WEIGHTS) {
+                const float f = ex2(before[i]);
+                gw[i] = fmaf(r[i] * f, dw[mt][i >> 1][2 * e + (i & 1)], gw[i]);
+                yr *= f;
+                check(wrong, make_float2(yk, yr));
+            } else {
+                yr *= ex2(before[i]);
+                P[b][i] = r[i] * yr;
+                x[b][i] = fmaf(k[i], yk, -P[b][i]);
+            }
             gu[i] = fmaf(gm, r[i] * k[i], gu[i]);
             yk = fmaf(u[i] * r[i], gm, yk);   // (in the order of the token-by-token kernels, which cannot overflow where the result does not)
             yr = fmaf(u[i] * k[i], gm, yr);
@@ -748,13 +792,11 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
         }
     Pair<E> wp[2][4];
     if constexpr (!STATIC) read_eights<E>(wp, w_ + base + c, g, n, C, vec_ok(w_, 4));
-    float gw[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         float after = 0.f;
-        gw[i] = 0.f;
 #pragma unroll
-        for (int b = 3; b >= 0; --b) {   // sums over the tokens from here on: over lanes inside eight tokens, then over the eights
+        for (int b = 3; b >= 0 && !WEIGHTS; --b) {   // sums over the tokens from here on: over lanes inside eight tokens, then over the eights
             float s = x[b][i];
 #pragma unroll
             for (int m = 1; m < 8; m <<= 1) {
@@ -771,7 +813,8 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             gu[i] += __shfl_xor_sync(0xffffffffu, gu[i], m);
             if (STATIC) gw[i] += __shfl_xor_sync(0xffffffffu, gw[i], m);
         }
-        // (the sum over all tokens in the first one's: every P and Q of the key is in it, and so every gr and gk)
+        if (WEIGHTS) gw[i] += aend[i];
+        // (per-token decays: the sum over all tokens in the first one's; every P and Q of the key is in it, and so every gr and gk)
         check(wrong, make_float2(STATIC ? gw[i] : x[0][i], gu[i]));
     }
     if (g == 0) {
