@@ -36,10 +36,11 @@
 namespace rwkvb200 {
 namespace {
 
-// log2 of the largest decay between the middle of a segment and an end of it.  Per-token decays: 60 in nats.  A static decay: the
-// sum of its gradient over the tokens holds terms without a decay that cancel (T 47, factors up to 2.7 per token: error of gw 6.2e-7,
-// token by token 4.3e-7), so the limit is a factor of 2 per token.
-template <bool STATIC> constexpr float kRange = STATIC ? 16.f : 86.f;
+// log2 of the largest decay between the middle of a segment and an end of it: 60 in nats.
+constexpr float kRange = 86.f;
+// log2 of the largest decay of one token that is the same for all tokens: a factor of 2.  (Of a token and not up to the middle, which
+// let a short last segment have more: at T 34 a factor of 256.)
+constexpr float kStaticRange = 1.f;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kImg = kSeg * 128;               // bytes of one bf16 image [32 tokens][64 channels]
 constexpr int kTiles = 3 * 512;                // bytes of one bf16 image of a triangular token x token matrix: its 16 x 16 tiles
@@ -301,7 +302,9 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
         *reinterpret_cast<float2*>(o.em2 + c) = make_float2(ex2(le.x), ex2(le.y));
     }
     check(bad, make_float2(s, 0.f));
-    const bool in = lm.x >= -kRange<STATIC> && lm.y >= -kRange<STATIC> && le.x >= -kRange<STATIC> && le.y >= -kRange<STATIC>;
+    bool in;
+    if constexpr (STATIC) in = d[0].x >= -kStaticRange && d[0].y >= -kStaticRange;
+    else in = lm.x >= -kRange && lm.y >= -kRange && le.x >= -kRange && le.y >= -kRange;
     return !(in && bad == 0.f);
 }
 // the images of a tensor as it came (pieces of 16 bytes where the alignment allows)

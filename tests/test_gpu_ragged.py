@@ -285,3 +285,26 @@ def test_rwkv5_fp32_decay_gradient(lo, hi, B, T, H):
     for a, b, name in zip(got, want, ("gr", "gk", "gv", "gw", "gu")):
         err = ((a.double().cpu().reshape(b.shape) - b).norm() / b.norm()).item()
         assert err <= 10 * 2 ** -24, f"{name}: {err:.3e}"
+
+
+@pytest.mark.parametrize("T", [34, 48, 64, 65])
+def test_rwkv5_segments_left_to_the_other_kernel(T):
+    """A head with a channel that decays by more than a factor of 2 per token is left to the token-by-token kernels, its last segment too however
+    short, and no other head."""
+    import rwkv_cuda_b200 as R
+    B, H, N = 5, 64, 64
+    g = Hh.gen(T)
+    C, nseg = H * N, (T + 31) // 32
+    d = [(0.5 * Hh.randn(g, B, T, C)).cuda() for _ in range(3)]
+    w, u = Hh.rand(g, H, N, lo=-6, hi=-0.4), Hh.rand(g, H, N, lo=-1, hi=1)
+    w[3, 5], w[60, 63] = 1.0, -0.3
+    y = torch.empty_like(d[0])
+    lib, n = R._lib.lib(), B * H * nseg
+    saved = torch.empty(lib.rwkvb200_wkv5_train_saved_bytes(B, T, C, H) // 4, dtype=torch.int32, device="cuda")
+    rc = lib.rwkvb200_wkv5_train_forward(R._lib.F32, B, T, C, H, *(x.data_ptr() for x in (*d, w.cuda(), u.cuda(), y)), saved.data_ptr(),
+                                         torch.cuda.current_stream().cuda_stream)
+    assert rc == 1, rc
+    flags = saved[n * N * N:n * N * N + n].view(B, H, nseg).bool().cpu()
+    want = torch.zeros_like(flags)
+    want[:, [3, 60]] = True
+    assert torch.equal(flags, want)
