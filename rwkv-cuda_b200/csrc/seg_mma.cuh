@@ -232,9 +232,24 @@ __device__ __forceinline__ void check(float& bad, float2 x) { bad = fmaf(x.y, 0.
 __device__ __forceinline__ float2 log2_decay(float2 w) { return make_float2(-kLog2e * ex2(kLog2e * w.x), -kLog2e * ex2(kLog2e * w.y)); }
 __device__ __forceinline__ float2 log2_decay_static(float2 w) { return make_float2(-kLog2e * expf(w.x), -kLog2e * expf(w.y)); }
 
+// fp32: a static decay to a power, exp(-e)^m, m of either sign.  The rounding of e m is put back, which the exponential would make large
+// (error of y at decays of 0.55 to 0.65 per token 1.5e-7 of its norm, 1.1e-7 with it, token by token 9e-8; inputs w of -6 to -1: 1.9e-7 -> 1.8e-7, 5.2e-7)
+__device__ __forceinline__ float decay_power(float e, int m) {
+    const float x = (float)m, p = e * x, f = expf(-p);
+    return fmaf(f, -fmaf(e, x, -p), f);
+}
+__device__ __forceinline__ float reciprocal(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// From `rows` (make_operands): what a token's r is scaled by, and k of the token before it
+template <bool POWERS> __device__ __forceinline__ float scale_r(float x) { return POWERS ? x : ex2(x); }
+template <bool POWERS> __device__ __forceinline__ float scale_k(float x) { return POWERS ? reciprocal(x) : ex2(-x); }
+
 // ---- operands of a segment ---------------------------------------------------------------------------------------------------
 // 128 threads: channels 2 lane, 2 lane + 1 of the tokens 8 warp ..  Leaves the images of r~, k~, the bonus sums, S's and D's factors
-// and (ROWS) log2 of exp(L_{t-1} - L_m) as rows, row 32: the end.  True where the segment has to be left to the other kernels.
+// and (ROWS) exp(L_{t-1} - L_m) as rows (POWERS; else its log2), row 32: the end.  True where the segment has to be left to the other kernels.
 struct Operands {
     unsigned char R[3 * kImg], K[3 * kImg];
     float tot[4 * kN], ruk[kSeg], em[kN], em2[kN];
@@ -250,12 +265,17 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
     if constexpr (!STATIC) read_rows<E, 8>(ww, w_ + c, t0, n, C, vec);
     else ww[0] = read_pair(w_ + c, vec);
     const float2 u = decode(read_pair(u_ + c, vec_ok(u_, 2)));
-    float2 d[STATIC ? 1 : 8], pre, lm, le;   // log2 decays; L before the first of these tokens, L at the middle, L from there to the end
+    constexpr bool POWERS = STATIC && sizeof(E) == 4;
+    const int mid = min(n, kSeg / 2);
+    float2 d[STATIC ? 1 : 8], pre, rate, lm, le;   // log2 decays; L before the first of these tokens, L at the middle, L from there to the end
     if constexpr (STATIC) {
         d[0] = log2_decay_static(decode(ww[0]));
-        const float nm = (float)min(n, kSeg / 2), ne = (float)n - nm;
+        const float nm = (float)mid, ne = (float)(n - mid);
         lm = make_float2(d[0].x * nm, d[0].y * nm);
         le = make_float2(d[0].x * ne, d[0].y * ne);
+        const float2 w = decode(ww[0]);
+        rate = make_float2(expf(w.x), expf(w.y));
+        if (POWERS) pre = make_float2(decay_power(rate.x, min(t0, n) - mid), decay_power(rate.y, min(t0, n) - mid));
     } else {
         float2 s = make_float2(0.f, 0.f);
 #pragma unroll
@@ -275,9 +295,13 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
     float bad = 0.f, x[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        float2 a, b;   // L before and after the token, from the middle
-        if constexpr (STATIC) {
-            const float ta = (float)(min(t0 + i, n) - min(n, kSeg / 2)), tb = (float)(min(t0 + i + 1, n) - min(n, kSeg / 2));
+        float2 a, b;   // L before and after the token, from the middle; the decay there (POWERS)
+        if constexpr (POWERS) {
+            const int behind = min(t0 + i + 1, n) - mid;
+            a = pre;
+            b = pre = make_float2(decay_power(rate.x, behind), decay_power(rate.y, behind));
+        } else if constexpr (STATIC) {
+            const float ta = (float)(min(t0 + i, n) - mid), tb = (float)(min(t0 + i + 1, n) - mid);
             a = make_float2(d[0].x * ta, d[0].y * ta);
             b = make_float2(d[0].x * tb, d[0].y * tb);
         } else {
@@ -286,7 +310,7 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
         }
         if (ROWS) *reinterpret_cast<float2*>(rows + (t0 + i) * kRld + c) = a;
         const float2 r = decode(rr[i]), k = decode(kk[i]);
-        const float2 rs = make_float2(r.x * ex2(a.x), r.y * ex2(a.y)), ks = make_float2(k.x * ex2(-b.x), k.y * ex2(-b.y));
+        const float2 rs = make_float2(r.x * scale_r<POWERS>(a.x), r.y * scale_r<POWERS>(a.y)), ks = make_float2(k.x * scale_k<POWERS>(b.x), k.y * scale_k<POWERS>(b.y));
         check(bad, rs); check(bad, ks);
         put_split(o.R, t0 + i, lane, rs.x, rs.y);
         put_split(o.K, t0 + i, lane, ks.x, ks.y);
@@ -298,8 +322,13 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     if ((lane & 3) == 0) o.ruk[t0 + (lane >> 2)] = s;
     if (q == 0) {
-        *reinterpret_cast<float2*>(o.em + c) = make_float2(ex2(lm.x), ex2(lm.y));
-        *reinterpret_cast<float2*>(o.em2 + c) = make_float2(ex2(le.x), ex2(le.y));
+        if constexpr (POWERS) {
+            *reinterpret_cast<float2*>(o.em + c) = make_float2(decay_power(rate.x, mid), decay_power(rate.y, mid));
+            *reinterpret_cast<float2*>(o.em2 + c) = make_float2(decay_power(rate.x, n - mid), decay_power(rate.y, n - mid));
+        } else {
+            *reinterpret_cast<float2*>(o.em + c) = make_float2(ex2(lm.x), ex2(lm.y));
+            *reinterpret_cast<float2*>(o.em2 + c) = make_float2(ex2(le.x), ex2(le.y));
+        }
     }
     check(bad, make_float2(s, 0.f));
     bool in;
@@ -537,7 +566,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     extern __shared__ __align__(128) unsigned char smem_seg_b[];
     BwdSmemM<E>& sm = *reinterpret_cast<BwdSmemM<E>*>(smem_seg_b);
     constexpr int NV = kParts<E>;
-    constexpr bool WEIGHTS = STATIC && sizeof(E) == 4;   // see dL/dlog d above (bf16: its rounding is a thousand times what cancels)
+    constexpr bool WEIGHTS = STATIC && sizeof(E) == 4, POWERS = WEIGHTS;   // see dL/dlog d above (bf16: its rounding is a thousand times what cancels)
     const i64 unit = blockIdx.x / nseg;
     const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
     const int g = lane >> 2, q = lane & 3, n = min(kSeg, T - seg * kSeg);
@@ -701,15 +730,15 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
             const float2 r0 = decode(rp[0][b]), r1 = decode(rp[1][b]);
             const float t = (float)(8 * b + g), d = (float)(n - 1) - t;
             k0.x *= d; k0.y *= d; k1.x *= d; k1.y *= d;
-            aend[0] = fmaf(t * r0.x * ex2(l0.x), dr[b >> 1][0][2 * (b & 1)], aend[0]);
-            aend[1] = fmaf(t * r0.y * ex2(l0.y), dr[b >> 1][0][2 * (b & 1) + 1], aend[1]);
-            aend[2] = fmaf(t * r1.x * ex2(l0.z), dr[b >> 1][1][2 * (b & 1)], aend[2]);
-            aend[3] = fmaf(t * r1.y * ex2(l0.w), dr[b >> 1][1][2 * (b & 1) + 1], aend[3]);
+            aend[0] = fmaf(t * r0.x * l0.x, dr[b >> 1][0][2 * (b & 1)], aend[0]);
+            aend[1] = fmaf(t * r0.y * l0.y, dr[b >> 1][0][2 * (b & 1) + 1], aend[1]);
+            aend[2] = fmaf(t * r1.x * l0.z, dr[b >> 1][1][2 * (b & 1)], aend[2]);
+            aend[3] = fmaf(t * r1.y * l0.w, dr[b >> 1][1][2 * (b & 1) + 1], aend[3]);
         }
-        aend[0] = fmaf(k0.x * ex2(-l.x), dk[b >> 1][0][2 * (b & 1)], aend[0]);
-        aend[1] = fmaf(k0.y * ex2(-l.y), dk[b >> 1][0][2 * (b & 1) + 1], aend[1]);
-        aend[2] = fmaf(k1.x * ex2(-l.z), dk[b >> 1][1][2 * (b & 1)], aend[2]);
-        aend[3] = fmaf(k1.y * ex2(-l.w), dk[b >> 1][1][2 * (b & 1) + 1], aend[3]);
+        aend[0] = fmaf(k0.x * scale_k<POWERS>(l.x), dk[b >> 1][0][2 * (b & 1)], aend[0]);
+        aend[1] = fmaf(k0.y * scale_k<POWERS>(l.y), dk[b >> 1][0][2 * (b & 1) + 1], aend[1]);
+        aend[2] = fmaf(k1.x * scale_k<POWERS>(l.z), dk[b >> 1][1][2 * (b & 1)], aend[2]);
+        aend[3] = fmaf(k1.y * scale_k<POWERS>(l.w), dk[b >> 1][1][2 * (b & 1) + 1], aend[3]);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -766,14 +795,14 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             float &yk = dk[mt][i >> 1][2 * e + (i & 1)], &yr = dr[mt][i >> 1][2 * e + (i & 1)];
-            yk *= ex2(-behind[i]);
+            yk *= scale_k<POWERS>(behind[i]);
             if constexpr (WEIGHTS) {
-                const float f = ex2(before[i]);
+                const float f = scale_r<POWERS>(before[i]);
                 gw[i] = fmaf(r[i] * f, dw[mt][i >> 1][2 * e + (i & 1)], gw[i]);
                 yr *= f;
                 check(wrong, make_float2(yk, yr));
             } else {
-                yr *= ex2(before[i]);
+                yr *= scale_r<POWERS>(before[i]);
                 P[b][i] = r[i] * yr;
                 x[b][i] = fmaf(k[i], yk, -P[b][i]);
             }

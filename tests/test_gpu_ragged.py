@@ -287,6 +287,27 @@ def test_rwkv5_fp32_decay_gradient(lo, hi, B, T, H):
         assert err <= 10 * 2 ** -24, f"{name}: {err:.3e}"
 
 
+@pytest.mark.parametrize("lo,hi", [(-6.0, -1.0), (-3.0, -2.5), (-0.6, -0.4)])
+def test_rwkv5_fp32_errors(lo, hi):
+    """y and gradients by products, a few 2^-24 of their norm (-0.6 to -0.4, just inside the limit of these kernels: token by token 1.5 2^-24;
+    powers of a decay as exponentials of a rounded product 2.5).  -6 to -1: sums over the slow channels' long memory, token by token 8.7."""
+    import rwkv_cuda_b200 as R
+    B, T, H, N = 2, 333, 40, 64
+    g = Hh.gen(T)
+    C = H * N
+    r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
+    u, gy, w = Hh.rand(g, H, N, lo=-1, hi=1), Hh.randn(g, B, T, C), Hh.rand(g, H, N, lo=lo, hi=hi)
+    xs = [x.cuda().requires_grad_(True) for x in (r, k, v, w, u)]
+    y = R.functions.WKV_5.apply(B, T, C, H, *xs)
+    got = [y, *torch.autograd.grad(y, xs, gy.cuda())]
+    xo = [x.double().requires_grad_(True) for x in (r, k, v, w, u)]
+    yo = O.wkv5(*xo, H)
+    want = [yo, *torch.autograd.grad(yo, xo, gy.double())]
+    for a, b, name in list(zip(got, want, ("y", "gr", "gk", "gv")))[:4]:
+        err = ((a.double().cpu().reshape(b.shape) - b).norm() / b.norm()).item()
+        assert err <= (2.2 if hi > -1 else 3) * 2 ** -24, f"{name}: {err:.3e}"
+
+
 @pytest.mark.parametrize("T", [34, 48, 64, 65])
 def test_rwkv5_segments_left_to_the_other_kernel(T):
     """A head with a channel that decays by more than a factor of 2 per token is left to the token-by-token kernels, its last segment too however
