@@ -566,7 +566,7 @@ extern "C" int rwkvb200_wkv5a_backward(int dtype, int B, int T, int C, int H, co
 namespace rwkvb200 {
 namespace {
 // out[j] = sum over rows of partial[row][j], in fp32 and in an order that depends on the shape only: NY threads take every
-// NY-th row of a column, their sums are added in order.  A row is read as 32 consecutive columns per warp.  (From 64 rows on 32
+// NY-th row of a column, their sums are added in order (8) or in pairs (32: one after the other, 64 rows were 10 % less exact than with 8).  A row is read as 32 consecutive columns per warp.  (From 64 rows on 32
 // threads: there are few blocks, and a thread's loads wait for one another; 256 rows of 2048 columns 4.3 us, 7.4 us with 8.)
 template <typename E, typename O, int NY>
 __global__ void __launch_bounds__(32 * NY) sum_rows_kernel(i64 rows, int n, const E* __restrict__ partial, O* __restrict__ out) {
@@ -580,10 +580,19 @@ __global__ void __launch_bounds__(32 * NY) sum_rows_kernel(i64 rows, int n, cons
     part[threadIdx.y][threadIdx.x] = acc;
     __syncthreads();
     if (threadIdx.y == 0 && j < n) {
-        acc = 0.f;
+        float x[NY];
 #pragma unroll
-        for (int q = 0; q < NY; ++q) acc += part[q][threadIdx.x];
-        out[j] = from_f<O>(acc);
+        for (int q = 0; q < NY; ++q) x[q] = part[q][threadIdx.x];
+        if (NY > 8) {
+#pragma unroll
+            for (int m = NY / 2; m >= 1; m >>= 1)
+#pragma unroll
+                for (int q = 0; q < m; ++q) x[q] += x[q + m];
+        } else {
+#pragma unroll
+            for (int q = 1; q < NY; ++q) x[0] += x[q];
+        }
+        out[j] = from_f<O>(x[0]);
     }
 }
 // The same sums (in the same order) for up to 8 rows of four columns per thread: there is one row for each of the 8 threads
