@@ -598,8 +598,8 @@ __global__ void __launch_bounds__(32 * NY) sum_rows_kernel(i64 rows, int n, cons
 // The same sums (in the same order) for up to 8 rows of four columns per thread: there is one row for each of the 8 threads
 // above, and most of the time goes into starting blocks (4 rows of 590 k columns: 18 -> 5 us).
 __global__ void __launch_bounds__(256) sum_few_rows_kernel(int rows, int n, const float* __restrict__ partial, float* __restrict__ out) {
-    const unsigned j = (blockIdx.x * 256 + threadIdx.x) * 4;   // (a last block may reach beyond 2^31)
-    if (j >= (unsigned)n) return;
+    const int j = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (j >= n) return;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
     for (int b = 0; b < rows; ++b) {

@@ -39,15 +39,3 @@ def test_errors_of_a_sum_over_many_rows(rows):
         eight += s
     want = x.double().sum(0)
     assert (out.cpu().double() - want).norm() <= 1.02 * (eight.double() - want).norm()
-
-
-def test_as_many_columns_as_an_int_holds():
-    """A last block of threads reaches beyond 2^31 columns."""
-    import rwkv_cuda_b200 as R
-    n = 2 ** 31 - 64
-    x = torch.full((1, n), 2.0, device="cuda")
-    x[0, :5] = 3.0
-    x[0, -5:] = 4.0
-    out = torch.zeros(n, device="cuda")
-    R.ops.reduce_batch_partials(x, out)
-    assert torch.equal(out, x[0])
