@@ -36,8 +36,11 @@
 namespace rwkvb200 {
 namespace {
 
-// log2 of the largest decay between the middle of a segment and an end of it: 60 in nats.
-constexpr float kRange = 86.f;
+// log2 of the largest decay between the middle of a segment and an end of it.  A value scaled by 2^-48 and split in three keeps its 24 bits
+// down to 2^-133, so from 4e-19 on, and 12 of them from 9e-23 on; the logarithms' rounding makes 2e-6.  (With 86 gradients of 1e-14
+// kept three bits and the decay gradient of a channel just inside had an error of 4.6e-3 at its worst element, 3.9e-3 being its rounding
+// to bf16; with 60 it was 3.97e-3.  With 32, inputs of w around -1 +- 1 flag so many segments that B8 T1000 H32 takes 1140 us, 580 with 48.)
+constexpr float kRange = 48.f;
 // log2 of the largest decay of one token that is the same for all tokens: a factor of 2.  (Of a token and not up to the middle, which
 // let a short last segment have more: at T 34 a factor of 256.)
 constexpr float kStaticRange = 1.f;
@@ -228,6 +231,9 @@ __device__ __forceinline__ void put_pair<float>(unsigned char* img, int row, int
 // sums that are 0 unless one of the values is not finite
 __device__ __forceinline__ void check(float& bad, float2 x) { bad = fmaf(x.y, 0.f, fmaf(x.x, 0.f, bad)); }
 
+// are the logarithms of two decays beyond a limit, or no numbers?
+__device__ __forceinline__ bool beyond(float2 l, float limit) { return !(l.x >= -limit && l.y >= -limit); }
+
 // log2 of the decays of two channels, from their raw inputs
 __device__ __forceinline__ float2 log2_decay(float2 w) { return make_float2(-kLog2e * ex2(kLog2e * w.x), -kLog2e * ex2(kLog2e * w.y)); }
 __device__ __forceinline__ float2 log2_decay_static(float2 w) { return make_float2(-kLog2e * expf(w.x), -kLog2e * expf(w.y)); }
@@ -249,14 +255,15 @@ template <bool POWERS> __device__ __forceinline__ float scale_k(float x) { retur
 
 // ---- operands of a segment ---------------------------------------------------------------------------------------------------
 // 128 threads: channels 2 lane, 2 lane + 1 of the tokens 8 warp ..  Leaves the images of r~, k~, the bonus sums, S's and D's factors
-// and (ROWS) exp(L_{t-1} - L_m) as rows (POWERS; else its log2), row 32: the end.  True where the segment has to be left to the other kernels.
+// and (ROWS) exp(L_{t-1} - L_m) as rows (POWERS; else its log2), row 32: the end.  False (for all
+// threads): decays out of range, nothing left.  odd: this thread has seen something else that leaves the segment to the other kernels.
 struct Operands {
     unsigned char R[3 * kImg], K[3 * kImg];
     float tot[4 * kN], ruk[kSeg], em[kN], em2[kN];
 };
 template <typename E, bool STATIC, bool ROWS>
 __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid, int n, int C, const E* __restrict__ r_, const E* __restrict__ k_,
-                                              const E* __restrict__ w_, const E* __restrict__ u_) {
+                                              const E* __restrict__ w_, const E* __restrict__ u_, bool& odd) {
     const int lane = tid & 31, q = tid >> 5, c = 2 * lane, t0 = 8 * q;
     Pair<E> rr[8], kk[8], ww[STATIC ? 1 : 8];
     const bool vec = vec_ok(r_, 2) && vec_ok(k_, 2) && vec_ok(w_, 2);
@@ -284,7 +291,7 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
             s.x += d[i].x; s.y += d[i].y;
         }
         *reinterpret_cast<float2*>(o.tot + q * kN + c) = s;
-        __syncthreads();
+        if (__syncthreads_or(beyond(s, kRange))) return false;   // (eight tokens alone are too much)
         float2 t[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) t[i] = *reinterpret_cast<const float2*>(o.tot + i * kN + c);
@@ -331,10 +338,8 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
         }
     }
     check(bad, make_float2(s, 0.f));
-    bool in;
-    if constexpr (STATIC) in = d[0].x >= -kStaticRange && d[0].y >= -kStaticRange;
-    else in = lm.x >= -kRange && lm.y >= -kRange && le.x >= -kRange && le.y >= -kRange;
-    return !(in && bad == 0.f);
+    odd = bad != 0.f || (STATIC ? beyond(d[0], kStaticRange) : beyond(lm, kRange) || beyond(le, kRange));
+    return true;
 }
 // the images of a tensor as it came (pieces of 16 bytes where the alignment allows)
 template <typename E>
@@ -479,7 +484,11 @@ __global__ void __launch_bounds__(128, 5) seg_mma_y_kernel(int T, int H, int nse
 #pragma unroll
                 for (int e = 0; e < 4; ++e) S[kk][nt][e] = p[(16 * kk + 4 * q + e) * kN + 2 * nt];
     }
-    bool bad = make_operands<E, STATIC, false>(sm.o, nullptr, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN);
+    bool bad;
+    if (!make_operands<E, STATIC, false>(sm.o, nullptr, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN, bad)) {
+        if (tid == 0) flags[blockIdx.x] = 1;
+        return;
+    }
     bad |= stage_images<E>(sm.V, tid, n, C, v_ + base);
     if (__syncthreads_or(bad)) {
         if (tid == 0) flags[blockIdx.x] = 1;
@@ -591,7 +600,11 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) D[kk][nt][e] = p[(16 * kk + 4 * q + e) * kN + 2 * nt];
     }
-    bool bad = make_operands<E, STATIC, true>(sm.o, sm.rows, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN);
+    bool bad;
+    if (!make_operands<E, STATIC, true>(sm.o, sm.rows, tid, n, C, r_ + base, k_ + base, w_ + (STATIC ? h * kN : base), u_ + h * kN, bad)) {
+        if (tid == 0) flags[blockIdx.x] = 1;
+        return;
+    }
     bad |= stage_images<E>(sm.V, tid, n, C, v_ + base);
     bad |= stage_images<E>(sm.G, tid, n, C, gy_ + base);
     if (__syncthreads_or(bad)) {

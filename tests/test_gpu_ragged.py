@@ -329,3 +329,29 @@ def test_rwkv5_segments_left_to_the_other_kernel(T):
     want = torch.zeros_like(flags)
     want[:, [3, 60]] = True
     assert torch.equal(flags, want)
+
+
+@pytest.mark.parametrize("w0", [0.72, 0.74, 1.3, 1.4])   # inside and outside of 48 bits up to the middle of a segment, and of 86
+@pytest.mark.parametrize("scale", [1e-14, 1e-8, 1e12])
+def test_rwkv6_gradients_of_any_size(scale, w0):
+    """One channel with a strong decay beside others, gradients that a loss scale made large or small; the gradients of that channel by
+    themselves.  Bounds as above."""
+    import rwkv_cuda_b200 as R
+    B, T, H, N = 2, 333, 40, 64
+    g = Hh.gen(1)
+    C = H * N
+    r, k, v = (0.5 * Hh.randn(g, B, T, C) for _ in range(3))
+    gy, w, u = scale * Hh.randn(g, B, T, C), Hh.randn(g, B, T, C) - 5.0, Hh.rand(g, H, N, lo=-1, hi=1)
+    w.view(B, T, H, N)[..., 9] = w0
+    xs = [a.to(BF).cuda().requires_grad_(True) for a in (r, k, v, w, u)]
+    y = R.functions.WKV_6.apply(B, T, C, H, *xs)
+    got = [y, *torch.autograd.grad(y, xs, gy.to(BF).cuda())]
+    xo = [a.to(BF).double().requires_grad_(True) for a in (r, k, v, w, u)]
+    yo = O.wkv6(*xo, H)
+    want = [yo, *torch.autograd.grad(yo, xo, gy.to(BF).double())]
+    for a, b, name in zip(got, want, ("y", "gr", "gk", "gv", "gw", "gu")):
+        a, b = (z.detach().double().cpu().reshape(-1, N) for z in (a, b))
+        for part in (slice(0, N), slice(9, 10)):
+            size = torch.maximum(b[:, part].abs(), b[:, part].square().mean().sqrt())
+            err = ((a[:, part] - b[:, part]).abs() / size).max().item()
+            assert err <= 2 ** -8 + 2 ** -15, f"{name} {part}: {err:.3e}"
