@@ -29,7 +29,8 @@
 // it, the tensor pipe is busy 30 % of the time.
 // A segment whose decays leave the range (more than kRange between its middle and an end), that holds values that are not
 // finite (a masked product would spread them over tokens before) or whose results are not (a state that is not finite; scaled operands
-// whose product overflows although the result would not) is flagged and left to the token-by-token kernels.
+// whose product overflows although the result would not) is flagged and left to the token-by-token kernels.  Static decays are looked at where
+// the states are made, decays per token there too with few units (the walk took 64 -> 72 us with it), else at the first barrier here.
 #pragma once
 #include "seg_tiles.cuh"
 
@@ -39,7 +40,7 @@ namespace {
 // log2 of the largest decay between the middle of a segment and an end of it.  A value scaled by 2^-48 and split in three keeps its 24 bits
 // down to 2^-133, so from 4e-19 on, and 12 of them from 9e-23 on; the logarithms' rounding makes 2e-6.  (With 86 gradients of 1e-14
 // kept three bits and the decay gradient of a channel just inside had an error of 4.6e-3 at its worst element, 3.9e-3 being its rounding
-// to bf16; with 60 it was 3.97e-3.  With 32, inputs of w around -1 +- 1 flag so many segments that B8 T1000 H32 takes 1140 us, 580 with 48.)
+// to bf16; with 60 it was 3.97e-3.  With 32, inputs of w around -1 +- 1 flag so many segments that B8 T1000 H32 takes 1140 us, 620 with 48.)
 constexpr float kRange = 48.f;
 // log2 of the largest decay of one token that is the same for all tokens: a factor of 2.  (Of a token and not up to the middle, which
 // let a short last segment have more: at T 34 a factor of 256.)
@@ -338,7 +339,7 @@ __device__ __forceinline__ bool make_operands(Operands& o, float* rows, int tid,
         }
     }
     check(bad, make_float2(s, 0.f));
-    odd = bad != 0.f || (STATIC ? beyond(d[0], kStaticRange) : beyond(lm, kRange) || beyond(le, kRange));
+    odd = bad != 0.f || (!STATIC && (beyond(lm, kRange) || beyond(le, kRange)));
     return true;
 }
 // the images of a tensor as it came (pieces of 16 bytes where the alignment allows)
@@ -458,7 +459,7 @@ struct YSmem {
 template <typename E, bool STATIC>
 __global__ void __launch_bounds__(128, 5) seg_mma_y_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
                                                            const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
-                                                           const float* __restrict__ states, E* __restrict__ y_, int* __restrict__ flags, int ahead) {
+                                                           const float* __restrict__ states, E* __restrict__ y_, int* __restrict__ flags, bool known, int ahead) {
     extern __shared__ __align__(128) unsigned char smem_seg_y[];
     YSmem<E>& sm = *reinterpret_cast<YSmem<E>*>(smem_seg_y);
     constexpr int NV = kParts<E>;
@@ -466,6 +467,7 @@ __global__ void __launch_bounds__(128, 5) seg_mma_y_kernel(int T, int H, int nse
     const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
     const int g = lane >> 2, q = lane & 3, n = min(kSeg, T - seg * kSeg);
     const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    if (known && flags[blockIdx.x]) return;
     if (blockIdx.x + ahead < gridDim.x) {
         const i64 next = blockIdx.x + ahead;
         const int seg1 = next % nseg, h1 = next / nseg % H, n1 = min(kSeg, T - seg1 * kSeg);
@@ -571,7 +573,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     seg_mma_backward_kernel(int T, int H, int nseg, const E* __restrict__ r_, const E* __restrict__ k_, const E* __restrict__ v_,
                             const E* __restrict__ w_, const E* __restrict__ u_, const E* __restrict__ gy_, const float* __restrict__ S_,
                             const float* __restrict__ D_, E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_, E* __restrict__ gw_,
-                            float* __restrict__ partial_, int* __restrict__ flags, int ahead) {
+                            float* __restrict__ partial_, const int* __restrict__ left, int* __restrict__ flags, int ahead) {
     extern __shared__ __align__(128) unsigned char smem_seg_b[];
     BwdSmemM<E>& sm = *reinterpret_cast<BwdSmemM<E>*>(smem_seg_b);
     constexpr int NV = kParts<E>;
@@ -580,6 +582,10 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
     const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = H * kN;
     const int g = lane >> 2, q = lane & 3, n = min(kSeg, T - seg * kSeg);
     const i64 base = (unit / H * T + (i64)seg * kSeg) * C + h * kN;
+    if (left != nullptr && left[blockIdx.x]) {
+        if (tid == 0) flags[blockIdx.x] = 1;
+        return;
+    }
     if (blockIdx.x + ahead < gridDim.x) {
         const i64 next = blockIdx.x + ahead;
         const int seg1 = next % nseg, h1 = next / nseg % H, n1 = min(kSeg, T - seg1 * kSeg);
@@ -936,7 +942,7 @@ __device__ __noinline__ void walk_again(int T, int nseg, int C, const E* a_, con
 }
 template <typename E, bool STATIC, bool REV>
 __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_kernel(int T, int H, int nseg, const E* __restrict__ a_, const E* __restrict__ b_,
-                                                               const E* __restrict__ w_, float* __restrict__ states) {
+                                                               const E* __restrict__ w_, float* __restrict__ states, int* __restrict__ flags) {
     extern __shared__ __align__(128) unsigned char smem_seg_c[];
     ChainSmem<E>* buf = reinterpret_cast<ChainSmem<E>*>(smem_seg_c);
     constexpr int NV = kParts<E>;
@@ -968,7 +974,13 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
                 prefetch_rows(y, base + (i64)far * kSeg * C, min(kSeg, T - far * kSeg), C, lane);
             }
         };
-        if constexpr (STATIC) raw[0].ww[0] = raw[1].ww[0] = read_pair(w_ + h * kN + c, vec);
+        if constexpr (STATIC) {
+            raw[0].ww[0] = raw[1].ww[0] = read_pair(w_ + h * kN + c, vec);
+            if (!REV && p == 7 && flags != nullptr) {
+                const bool out = __any_sync(0xffffffffu, beyond(log2_decay_static(decode(raw[0].ww[0])), kStaticRange));
+                for (int i = lane; i < nseg; i += 32) flags[unit * nseg + i] = out;
+            }
+        }
         if (nseg > 1) fetch(raw[0], 0);
         if (nseg > 2) fetch(raw[1], 1);
         auto make = [&](Raw& x, int it) {
@@ -1105,25 +1117,34 @@ __global__ void __launch_bounds__(384, sizeof(E) == 2 ? 2 : 1) seg_mma_chain_ker
 }
 
 // ---- the segments that the kernels above have left ----------------------------------------------------------------------------
-// Block b looks at the segments b, b + grid, ..: with none flagged that is one read per thread.
-template <typename F>
+// ONE: a block per segment (flags: none, or whether it is one of those).  Else block b looks at the segments b, b + grid, .. together: with
+// none flagged, starting the blocks is all that the launch costs.
+template <bool ONE, typename F>
 __device__ __forceinline__ void for_flagged(const int* __restrict__ flags, i64 total, F body) {
-    for (i64 first = blockIdx.x; first < total; first += (i64)gridDim.x * blockDim.x) {
-        const i64 mine = first + (i64)threadIdx.x * gridDim.x;
-        if (!__syncthreads_or(mine < total && flags[mine])) continue;
-        for (int i = 0; i < (int)blockDim.x; ++i) {
-            const i64 block = first + (i64)i * gridDim.x;
-            if (block < total && flags[block]) {
-                body(block);
-                __syncthreads();
-            }
+    if constexpr (ONE) {
+        if (flags == nullptr || flags[blockIdx.x]) body((i64)blockIdx.x);
+    } else {
+        __shared__ unsigned found[4];   // a bit per thread of up to 128
+        for (i64 first = blockIdx.x; first < total; first += (i64)gridDim.x * blockDim.x) {
+            const i64 mine = first + (i64)threadIdx.x * gridDim.x;
+            const bool flag = mine < total && flags[mine];
+            const unsigned bits = __ballot_sync(0xffffffffu, flag);
+            if ((threadIdx.x & 31) == 0) found[threadIdx.x >> 5] = bits;
+            if (!__syncthreads_or(flag)) continue;
+            for (int w = 0; w < (int)blockDim.x / 32; ++w)
+                for (unsigned left = found[w]; left != 0; left &= left - 1) {
+                    body(first + (i64)(32 * w + __ffs(left) - 1) * gridDim.x);
+                    __syncthreads();
+                }
+            __syncthreads();
         }
     }
 }
-inline unsigned flagged_blocks(i64 total, int per_sm) {   // as many as are resident together
-    const i64 most = (i64)(sm_count() > 0 ? sm_count() : 148) * per_sm;
-    return (unsigned)(total < most ? total : most);
-}
+// A block per segment up to eight rounds of resident blocks: nothing is faster where all are flagged.  Above, four rounds of blocks, because with
+// none flagged it is the rounds that cost.  B8 T1000 H32, 8192 segments, y and gradients, none flagged / all: a block each 8 + 14 / 223 + 627 us,
+// eight rounds 9 + 11 / 279 + 659, four 6 + 7 / 270 + 680, one 4.5 + 4.3 / 301 + 694.
+inline i64 resident_blocks(int per_sm) { return (i64)(sm_count() > 0 ? sm_count() : 148) * per_sm; }
+inline bool block_per_segment(i64 total, int per_sm) { return total <= 8 * resident_blocks(per_sm); }
 
 // ---- launches ----------------------------------------------------------------------------------------------------------------
 // One block per unit walks all segments, or (the other kernels) every segment on its own and a scan: with few units the walk is
@@ -1134,31 +1155,31 @@ inline bool seg_chain_pays(i64 units) { return units * 2 > sm_count(); }
 inline bool seg_mma_pays(i64 total) { return total > 4ll * sm_count(); }
 
 template <typename E, bool STATIC, bool REV>
-int seg_chain(i64 units, int T, int H, int nseg, const void* a, const void* b, const void* w, float* states, cudaStream_t st) {
+int seg_chain(i64 units, int T, int H, int nseg, const void* a, const void* b, const void* w, float* states, int* flags, cudaStream_t st) {
     constexpr int smem = 2 * sizeof(ChainSmem<E>);
     const cudaError_t e = allow_smem<seg_mma_chain_kernel<E, STATIC, REV>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    seg_mma_chain_kernel<E, STATIC, REV><<<(unsigned)units, 384, smem, st>>>(T, H, nseg, (const E*)a, (const E*)b, (const E*)w, states);
+    seg_mma_chain_kernel<E, STATIC, REV><<<(unsigned)units, 384, smem, st>>>(T, H, nseg, (const E*)a, (const E*)b, (const E*)w, states, flags);
     return check_launch("training on segments: states");
 }
 template <typename E, bool STATIC>
 int seg_mma_y(i64 total, int T, int H, int nseg, const void* r, const void* k, const void* v, const void* w, const void* u, const float* states,
-              void* y, int* flags, cudaStream_t st) {
+              void* y, int* flags, bool known, cudaStream_t st) {
     constexpr int smem = sizeof(YSmem<E>);
     const cudaError_t e = allow_smem<seg_mma_y_kernel<E, STATIC>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     seg_mma_y_kernel<E, STATIC><<<(unsigned)total, 128, smem, st>>>(T, H, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states,
-                                                                   (E*)y, flags, 4 * sm_count());
+                                                                   (E*)y, flags, known, 4 * sm_count());
     return check_launch("training on segments: y");
 }
 template <typename E, bool STATIC>
 int seg_mma_backward(i64 total, int T, int H, int nseg, const void* r, const void* k, const void* v, const void* w, const void* u, const void* gy,
-                     const float* S, const float* D, void* gr, void* gk, void* gv, void* gw, float* partial, int* flags, cudaStream_t st) {
+                     const float* S, const float* D, void* gr, void* gk, void* gv, void* gw, float* partial, const int* left, int* flags, cudaStream_t st) {
     constexpr int smem = sizeof(BwdSmemM<E>);
     const cudaError_t e = allow_smem<seg_mma_backward_kernel<E, STATIC>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "training on segments: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     seg_mma_backward_kernel<E, STATIC><<<(unsigned)total, 128, smem, st>>>(T, H, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u,
-                                                                          (const E*)gy, S, D, (E*)gr, (E*)gk, (E*)gv, (E*)gw, partial, flags,
+                                                                          (const E*)gy, S, D, (E*)gr, (E*)gk, (E*)gv, (E*)gw, partial, left, flags,
                                                                           4 * sm_count());
     return check_launch("training on segments: gradients");
 }

@@ -531,6 +531,7 @@ extern "C" int rwkvb200_wkv5_train_backward(int dtype, int B, int T, int C, int 
     } else {
         float* D = partial + (size_t)B * wkv5_seg_count(T) * 2 * C;
         if (int e = wkv5_seg_backward(dtype, B, T, C, H, r, k, v, w_raw, u, gy, gr, gk, gv, static_cast<const float*>(saved), D, partial,
+                                      static_cast<const int*>(saved) + (size_t)B * H * wkv5_seg_count(T) * (C / H) * (C / H),
                                       reinterpret_cast<int*>(D + (size_t)B * H * wkv5_seg_count(T) * (C / H) * (C / H)), st)) return e;
         rows = (i64)B * wkv5_seg_count(T);
     }

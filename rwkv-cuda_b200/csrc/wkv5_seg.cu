@@ -65,14 +65,15 @@ __global__ void __launch_bounds__(256) seg_scan_kernel(int T, int H, int N, int 
 // REV = false: a = k, b = v; REV = true: a = r, b = gy.
 template <typename E, bool REV>
 __global__ void __launch_bounds__(64, 8) seg_local_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ a_, const E* __restrict__ b_,
-                                                          const E* __restrict__ w_, float* __restrict__ states) {
+                                                          const E* __restrict__ w_, float* __restrict__ states, int* __restrict__ flags) {
     __shared__ __align__(16) float as[kSeg * kN], bs[kSeg * kN], lw[kN];
     const int unit = blockIdx.x / nseg, seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31;
     const int n = min(kSeg, T - seg * kSeg);
     const i64 base = ((i64)(unit / H) * T + seg * kSeg) * C + h * N;
     lw[tid] = tid < N ? log_decay(w_ + h * N + tid) : 0.f;
     stage<64>(bs, b_ + base, n, C, N, tid);
-    __syncthreads();
+    const bool out = __syncthreads_or(beyond(make_float2(kLog2e * lw[tid], 0.f), kStaticRange));
+    if (!REV && flags != nullptr && tid == 0) flags[blockIdx.x] = out;
     // a, times the decay between its token and the end (REV: the start) of the segment
     stage<64>(as, a_ + base, n, C, N, tid, [&](int t, int j) { return t < n ? power(lw[j], REV ? t : n - 1 - t) : 0.f; });
     __syncthreads();
@@ -144,12 +145,11 @@ __device__ __forceinline__ void y_segment(i64 block, int T, int C, int H, int N,
 }
 
 // every segment, or (flags) those that the kernels by products have left
-template <typename E>
+template <typename E, bool ONE>
 __global__ void __launch_bounds__(64, 8) seg_y_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
                                                       const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
                                                       const float* __restrict__ states, E* __restrict__ y_, const int* __restrict__ flags, i64 total) {
-    if (flags == nullptr) y_segment(blockIdx.x, T, C, H, N, nseg, r_, k_, v_, w_, u_, states, y_);
-    else for_flagged(flags, total, [&](i64 block) { y_segment(block, T, C, H, N, nseg, r_, k_, v_, w_, u_, states, y_); });
+    for_flagged<ONE>(flags, total, [&](i64 block) { y_segment(block, T, C, H, N, nseg, r_, k_, v_, w_, u_, states, y_); });
 }
 
 // A segment token by token.  4 warps: warps 0, 1 carry S and Z forward (gr, gw, gu), warps 2, 3 carry D backward (gk, gv); a warp
@@ -280,14 +280,13 @@ __device__ __forceinline__ void backward_segment(i64 block, int T, int C, int H,
     }
 }
 
-template <typename E>
+template <typename E, bool ONE>
 __global__ void __launch_bounds__(128, 2) seg_backward_kernel(int T, int C, int H, int N, int nseg, const E* __restrict__ r_, const E* __restrict__ k_,
                                                               const E* __restrict__ v_, const E* __restrict__ w_, const E* __restrict__ u_,
                                                               const E* __restrict__ gy_, const float* __restrict__ S_, const float* __restrict__ D_,
                                                               E* __restrict__ gr_, E* __restrict__ gk_, E* __restrict__ gv_,
                                                               float* __restrict__ partial_, const int* __restrict__ flags, i64 total) {
-    if (flags == nullptr) backward_segment(blockIdx.x, T, C, H, N, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, partial_);
-    else for_flagged(flags, total, [&](i64 block) { backward_segment(block, T, C, H, N, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, partial_); });
+    for_flagged<ONE>(flags, total, [&](i64 block) { backward_segment(block, T, C, H, N, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, partial_); });
 }
 
 // Head size 64: y and gradients by products (seg_mma.cuh), the kernels here only for the segments that those leave (flags).
@@ -296,43 +295,40 @@ int forward(int B, int T, int C, int H, const void* r, const void* k, const void
             int* flags, cudaStream_t st) {
     const int N = C / H, nseg = (T + kSeg - 1) / kSeg;
     const i64 units = B * (i64)H, total = units * nseg;
+    if (N != kN || !seg_mma_pays(total)) flags = nullptr;
     if (N == kN && seg_chain_pays(units)) {
-        if (const int e = seg_chain<E, true, false>(units, T, H, nseg, k, v, w, states, st)) return e;
+        if (const int e = seg_chain<E, true, false>(units, T, H, nseg, k, v, w, states, flags, st)) return e;
     } else {
-        seg_local_kernel<E, false><<<(unsigned)total, 64, 0, st>>>(T, C, H, N, nseg, (const E*)k, (const E*)v, (const E*)w, states);
+        seg_local_kernel<E, false><<<(unsigned)total, 64, 0, st>>>(T, C, H, N, nseg, (const E*)k, (const E*)v, (const E*)w, states, flags);
         seg_scan_kernel<E, false><<<(unsigned)(units * ((N * N + 255) / 256)), 256, 0, st>>>(T, H, N, nseg, (const E*)w, states);
     }
-    unsigned grid = (unsigned)total;
-    if (N != kN || !seg_mma_pays(total)) flags = nullptr;
-    if (flags != nullptr) {
-        if (const int e = seg_mma_y<E, true>(total, T, H, nseg, r, k, v, w, u, states, y, flags, st)) return e;
-        grid = flagged_blocks(total, 8);
-    }
-    seg_y_kernel<E><<<grid, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states, (E*)y,
+    if (flags != nullptr)
+        if (const int e = seg_mma_y<E, true>(total, T, H, nseg, r, k, v, w, u, states, y, flags, true, st)) return e;
+    const bool one = flags == nullptr || block_per_segment(total, 8);
+    (one ? seg_y_kernel<E, true> : seg_y_kernel<E, false>)<<<(unsigned)(one ? total : 4 * resident_blocks(8)), 64, 0, st>>>(
+        T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, states, (E*)y,
                                          flags, total);
     return check_launch("wkv5_train_forward(segments)");
 }
 
 template <typename E>
 int backward(int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u, const void* gy, void* gr,
-             void* gk, void* gv, const float* S, float* D, float* partial, int* flags, cudaStream_t st) {
+             void* gk, void* gv, const float* S, float* D, float* partial, const int* left, int* flags, cudaStream_t st) {
     const int N = C / H, nseg = (T + kSeg - 1) / kSeg, smem = sizeof(BwdSmem);
     const i64 units = B * (i64)H, total = units * nseg;
-    const cudaError_t e = allow_smem<seg_backward_kernel<E>>(smem);
+    const bool one = N != kN || !seg_mma_pays(total) || block_per_segment(total, 2);
+    const cudaError_t e = one ? allow_smem<seg_backward_kernel<E, true>>(smem) : allow_smem<seg_backward_kernel<E, false>>(smem);
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv5_train_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     if (N == kN && seg_chain_pays(units)) {
-        if (const int e = seg_chain<E, true, true>(units, T, H, nseg, r, gy, w, D, st)) return e;
+        if (const int e = seg_chain<E, true, true>(units, T, H, nseg, r, gy, w, D, nullptr, st)) return e;
     } else {
-        seg_local_kernel<E, true><<<(unsigned)total, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)gy, (const E*)w, D);
+        seg_local_kernel<E, true><<<(unsigned)total, 64, 0, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)gy, (const E*)w, D, nullptr);
         seg_scan_kernel<E, true><<<(unsigned)(units * ((N * N + 255) / 256)), 256, 0, st>>>(T, H, N, nseg, (const E*)w, D);
     }
-    unsigned grid = (unsigned)total;
     if (N != kN || !seg_mma_pays(total)) flags = nullptr;
-    if (flags != nullptr) {
-        if (const int e = seg_mma_backward<E, true>(total, T, H, nseg, r, k, v, w, u, gy, S, D, gr, gk, gv, nullptr, partial, flags, st)) return e;
-        grid = flagged_blocks(total, 2);
-    }
-    seg_backward_kernel<E><<<grid, 128, smem, st>>>(T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, (const E*)gy, S,
+    else if (const int e = seg_mma_backward<E, true>(total, T, H, nseg, r, k, v, w, u, gy, S, D, gr, gk, gv, nullptr, partial, left, flags, st)) return e;
+    (one ? seg_backward_kernel<E, true> : seg_backward_kernel<E, false>)<<<(unsigned)(one ? total : 4 * resident_blocks(2)), 128, smem, st>>>(
+        T, C, H, N, nseg, (const E*)r, (const E*)k, (const E*)v, (const E*)w, (const E*)u, (const E*)gy, S,
                                                     D, (E*)gr, (E*)gk, (E*)gv, partial, flags, total);
     return check_launch("wkv5_train_backward(segments)");
 }
@@ -345,9 +341,9 @@ int wkv5_seg_forward(int dtype, int B, int T, int C, int H, const void* r, const
                                  : forward<bf16>(B, T, C, H, r, k, v, w, u, y, states, flags, st);
 }
 int wkv5_seg_backward(int dtype, int B, int T, int C, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
-                      const void* gy, void* gr, void* gk, void* gv, const float* S, float* D, float* partial, int* flags, cudaStream_t st) {
-    return dtype == RWKVB200_F32 ? backward<float>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, flags, st)
-                                 : backward<bf16>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, flags, st);
+                      const void* gy, void* gr, void* gk, void* gv, const float* S, float* D, float* partial, const int* left, int* flags, cudaStream_t st) {
+    return dtype == RWKVB200_F32 ? backward<float>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, left, flags, st)
+                                 : backward<bf16>(B, T, C, H, r, k, v, w, u, gy, gr, gk, gv, S, D, partial, left, flags, st);
 }
 
 }  // namespace rwkvb200

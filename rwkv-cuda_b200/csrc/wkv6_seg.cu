@@ -25,6 +25,7 @@
 namespace rwkvb200 {
 namespace {
 
+constexpr float kLeast = 1.f / (1ll << (int)kRange);
 __device__ __forceinline__ float log_decay(const bf16* w_raw) { return -expf(to_f(*w_raw)); }
 
 // d of the segment's tokens as rows in the order of place(); 1 where there is no token.
@@ -67,7 +68,8 @@ __global__ void __launch_bounds__(256) seg6_scan_kernel(int nseg, const float* _
 // REV = false: a = k, b = v, and the product of the segment's decays goes to `decays`; REV = true: a = r, b = gy.
 template <bool REV>
 __global__ void __launch_bounds__(64) seg6_local_kernel(int T, int H, int nseg, const bf16* __restrict__ a_, const bf16* __restrict__ b_,
-                                                        const bf16* __restrict__ w_, float* __restrict__ states, float* __restrict__ decays) {
+                                                        const bf16* __restrict__ w_, float* __restrict__ states, float* __restrict__ decays,
+                                                        int* __restrict__ flags) {
     __shared__ __align__(16) float as[kSeg * kN], bs[kSeg * kN], ds[kSeg * kN];
     const i64 unit = blockIdx.x / nseg;
     const int seg = blockIdx.x % nseg, h = unit % H, tid = threadIdx.x, lane = tid & 31, C = H * kN;
@@ -79,15 +81,24 @@ __global__ void __launch_bounds__(64) seg6_local_kernel(int T, int H, int nseg, 
     __syncthreads();
     {   // a, times the decay between its token and the end (REV: the start) of the segment: a thread per channel
         float f = 1.f;
+        bool out = false;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            float g = 1.f;
 #pragma unroll 8
-        for (int q = 0; q < kSeg; ++q) {
-            const int t = REV ? q : kSeg - 1 - q;
-            as[t * kN + tid] *= f;
-            f *= ds[t * kN + tid];
+            for (int q = 0; q < kSeg / 2; ++q) {
+                const int t = REV ? half * (kSeg / 2) + q : kSeg - 1 - half * (kSeg / 2) - q;
+                const float d = ds[t * kN + tid];
+                as[t * kN + tid] *= f;
+                f *= d;
+                if (!REV) g *= d;
+            }
+            out |= !(g >= kLeast);
         }
         if (!REV) decays[(i64)blockIdx.x * kN + tid] = f;
+        out = __syncthreads_or(out);
+        if (!REV && flags != nullptr && tid == 0) flags[blockIdx.x] = out;   // (as the products would find it, at less cost)
     }
-    __syncthreads();
     const int kg = 4 * (tid >> 5) + (lane & 3), vg = lane >> 2;
     Tile s;
 #pragma unroll
@@ -154,11 +165,11 @@ __device__ __forceinline__ void seg6_y_segment(i64 block, int T, int H, int nseg
     }
 }
 
-__global__ void __launch_bounds__(64) seg6_y_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
+template <bool ONE>
+__global__ void __launch_bounds__(64, ONE ? 1 : 6) seg6_y_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
                                                     const bf16* __restrict__ v_, const bf16* __restrict__ w_, const bf16* __restrict__ u_,
                                                     const float* __restrict__ states, bf16* __restrict__ y_, const int* __restrict__ flags, i64 total) {
-    if (flags == nullptr) seg6_y_segment(blockIdx.x, T, H, nseg, r_, k_, v_, w_, u_, states, y_);   // all segments
-    else for_flagged(flags, total, [&](i64 block) { seg6_y_segment(block, T, H, nseg, r_, k_, v_, w_, u_, states, y_); });
+    for_flagged<ONE>(flags, total, [&](i64 block) { seg6_y_segment(block, T, H, nseg, r_, k_, v_, w_, u_, states, y_); });
 }
 
 // The segments that seg_mma_backward_kernel has left.  4 warps: warps 0, 1 carry S forward (gr, gu, P), warps 2, 3 carry D backward (gk, gv, Q); a warp
@@ -283,14 +294,14 @@ __device__ __forceinline__ void seg6_backward_segment(i64 block, int T, int H, i
     }
 }
 
+template <bool ONE>
 __global__ void __launch_bounds__(128, 3) seg6_backward_kernel(int T, int H, int nseg, const bf16* __restrict__ r_, const bf16* __restrict__ k_,
                                                                const bf16* __restrict__ v_, const bf16* __restrict__ w_,
                                                                const bf16* __restrict__ u_, const bf16* __restrict__ gy_,
                                                                const float* __restrict__ S_, const float* __restrict__ D_, bf16* __restrict__ gr_,
                                                                bf16* __restrict__ gk_, bf16* __restrict__ gv_, bf16* __restrict__ gw_,
                                                                float* __restrict__ gu_, const int* __restrict__ flags, i64 total) {
-    if (flags == nullptr) seg6_backward_segment(blockIdx.x, T, H, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, gw_, gu_);   // all segments
-    else for_flagged(flags, total, [&](i64 block) { seg6_backward_segment(block, T, H, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, gw_, gu_); });
+    for_flagged<ONE>(flags, total, [&](i64 block) { seg6_backward_segment(block, T, H, nseg, r_, k_, v_, w_, u_, gy_, S_, D_, gr_, gk_, gv_, gw_, gu_); });
 }
 
 }  // namespace
@@ -303,15 +314,16 @@ int wkv6_seg_forward(int B, int T, int H, const void* r, const void* k, const vo
     float* decays = saved + total * kN * kN;
     int* flags = seg_mma_pays(total) ? reinterpret_cast<int*>(decays + total * kN) : nullptr;
     if (seg_chain_pays(units)) {
-        if (const int e = seg_chain<bf16, false, false>(units, T, H, nseg, k, v, w, saved, st)) return e;
+        if (const int e = seg_chain<bf16, false, false>(units, T, H, nseg, k, v, w, saved, nullptr, st)) return e;
     } else {
-        seg6_local_kernel<false><<<(unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)k, (const bf16*)v, (const bf16*)w, saved, decays);
+        seg6_local_kernel<false><<<(unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)k, (const bf16*)v, (const bf16*)w, saved, decays, flags);
         seg6_scan_kernel<false><<<(unsigned)(units * (kN * kN / 256)), 256, 0, st>>>(nseg, decays, saved);
     }
     if (flags != nullptr)
-        if (const int e = seg_mma_y<bf16, false>(total, T, H, nseg, r, k, v, w, u, saved, y, flags, st)) return e;
-    seg6_y_kernel<<<flags != nullptr ? flagged_blocks(total, 8) : (unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, saved,
-                                                           (bf16*)y, flags, total);
+        if (const int e = seg_mma_y<bf16, false>(total, T, H, nseg, r, k, v, w, u, saved, y, flags, !seg_chain_pays(units), st)) return e;
+    const bool one = flags == nullptr || block_per_segment(total, 6);
+    (one ? seg6_y_kernel<true> : seg6_y_kernel<false>)<<<(unsigned)(one ? total : 4 * resident_blocks(6)), 64, 0, st>>>(
+        T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, saved, (bf16*)y, flags, total);
     return check_launch("wkv6_train_forward(segments)");
 }
 
@@ -320,17 +332,19 @@ int wkv6_seg_backward(int B, int T, int H, const void* r, const void* k, const v
     const int nseg = (T + kSeg - 1) / kSeg;
     const i64 units = (i64)B * H, total = units * nseg;
     const float* decays = saved + total * kN * kN;
-    const cudaError_t e = allow_smem<seg6_backward_kernel>(sizeof(Bwd6Smem));
+    const int* left = seg_chain_pays(units) ? nullptr : reinterpret_cast<const int*>(decays + total * kN);   // known from the forward
+    const bool one = !seg_mma_pays(total) || block_per_segment(total, 3);
+    const cudaError_t e = one ? allow_smem<seg6_backward_kernel<true>>(sizeof(Bwd6Smem)) : allow_smem<seg6_backward_kernel<false>>(sizeof(Bwd6Smem));
     RWKV_REQUIRE(e == cudaSuccess, RWKVB200_ECUDA, "wkv6_train_backward: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     if (seg_chain_pays(units)) {
-        if (const int e = seg_chain<bf16, false, true>(units, T, H, nseg, r, gy, w, adjoints, st)) return e;
+        if (const int e = seg_chain<bf16, false, true>(units, T, H, nseg, r, gy, w, adjoints, nullptr, st)) return e;
     } else {
-        seg6_local_kernel<true><<<(unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)gy, (const bf16*)w, adjoints, nullptr);
+        seg6_local_kernel<true><<<(unsigned)total, 64, 0, st>>>(T, H, nseg, (const bf16*)r, (const bf16*)gy, (const bf16*)w, adjoints, nullptr, nullptr);
         seg6_scan_kernel<true><<<(unsigned)(units * (kN * kN / 256)), 256, 0, st>>>(nseg, decays, adjoints);
     }
     if (!seg_mma_pays(total)) flags = nullptr;
-    else if (const int e = seg_mma_backward<bf16, false>(total, T, H, nseg, r, k, v, w, u, gy, saved, adjoints, gr, gk, gv, gw, gu_partial, flags, st)) return e;
-    seg6_backward_kernel<<<flags != nullptr ? flagged_blocks(total, 3) : (unsigned)total, 128, sizeof(Bwd6Smem), st>>>(
+    else if (const int e = seg_mma_backward<bf16, false>(total, T, H, nseg, r, k, v, w, u, gy, saved, adjoints, gr, gk, gv, gw, gu_partial, left, flags, st)) return e;
+    (one ? seg6_backward_kernel<true> : seg6_backward_kernel<false>)<<<(unsigned)(one ? total : 4 * resident_blocks(3)), 128, sizeof(Bwd6Smem), st>>>(
         T, H, nseg, (const bf16*)r, (const bf16*)k, (const bf16*)v, (const bf16*)w, (const bf16*)u, (const bf16*)gy, saved, adjoints, (bf16*)gr, (bf16*)gk,
         (bf16*)gv, (bf16*)gw, gu_partial, flags, total);
     return check_launch("wkv6_train_backward(segments)");

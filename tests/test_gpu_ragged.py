@@ -355,3 +355,34 @@ def test_rwkv6_gradients_of_any_size(scale, w0):
             size = torch.maximum(b[:, part].abs(), b[:, part].square().mean().sqrt())
             err = ((a[:, part] - b[:, part]).abs() / size).max().item()
             assert err <= 2 ** -8 + 2 ** -15, f"{name} {part}: {err:.3e}"
+
+
+@pytest.mark.parametrize("op,H", [("wkv6", 512), ("wkv5 fp32", 640)])
+def test_many_segments_some_left_to_the_other_kernels(op, H):
+    """So many segments (7680 and 9600) that a block of the token-by-token kernels looks at several: heads with strong decays, throughout or in a few
+    segments, and their neighbours against a call with these heads only (few segments: token by token)."""
+    import rwkv_cuda_b200 as R
+    B, T, N, picks = 1, 463, 64, [0, 7, 8, 200, 201, H - 1]
+    dtype, F = (BF, R.functions.WKV_6) if op == "wkv6" else (torch.float32, R.functions.WKV_5)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rn = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x = {n: 0.5 * rn(B, T, H, N) for n in ("r", "k", "v", "gy")}
+    x["u"] = rn(H, N)
+    if op == "wkv6":
+        x["w"] = rn(B, T, H, N) - 4.0
+        x["w"][:, :, 7, 3] = x["w"][:, 40:100, 200, 5] = x["w"][:, -1, H - 1, 0] = 4.0
+    else:
+        x["w"] = torch.rand(H, N, device="cuda", generator=g) * 5.0 - 6.0
+        x["w"][7, 3] = x["w"][200, 5] = x["w"][H - 1, 0] = 2.0
+
+    def call(heads):
+        xs = [(x[n][:, :, heads].reshape(B, T, -1) if x[n].dim() == 4 else x[n][heads]).to(dtype).contiguous().requires_grad_(n != "gy")
+              for n in ("r", "k", "v", "w", "u", "gy")]
+        y = F.apply(B, T, len(heads) * N, len(heads), *xs[:5])
+        out = [y, *torch.autograd.grad(y, xs[:5], xs[5])]
+        return [z.view(B, T, len(heads), N) if z.dim() == 3 else z.view(len(heads), N) for z in out]
+
+    for a, b, name in zip(call(list(range(H))), call(picks), ("y", "gr", "gk", "gv", "gw", "gu")):
+        a = (a[:, :, picks] if a.dim() == 4 else a[picks]).float()
+        err = ((a - b.float()).abs() / torch.maximum(b.float().abs(), b.float().square().mean().sqrt())).max().item()
+        assert err <= (2 ** -7 if dtype == BF else 2e-5), f"{name}: {err:.3e}"
