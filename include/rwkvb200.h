@@ -338,8 +338,9 @@ int rwkvb200_wkv7_state_update(int dtype, int B, int T, int H, int N, float* sta
 int rwkvb200_wkv7_select_path(int path);
 /* Form of the tensor-core RWKV-7 kernels: 0 = automatic (forward: the staged kernel, three warp groups on
  * consecutive chunks with inputs by TMA; backward: the two-stage kernel for launches with at most one
- * (batch, head) unit per SM, or for what is left over from whole rounds of two per SM; the one-group kernel otherwise), 1 = one-group kernels, 2 = staged / two-stage
- * kernels.  All run the same products; results agree to the last bf16 digit (a few dw elements differ by one ulp).
+ * (batch, head) unit per SM, or for what is left over from one or two whole rounds of two per SM in long sequences; the one-group kernel otherwise), 1 = one-group kernels, 2 = staged / two-stage
+ * kernels.  All run the same products; results agree to the last bf16 digit (a few dw elements differ by one ulp): with 1 or 2
+ * they do not depend on how many units a call has.
  * Process-wide; no counterpart in the reference. */
 int rwkvb200_wkv7_select_form(int form);
 /* Synchronous read of the current device's sticky status word: 0, or 10 + n / 20 + n when the n-th

@@ -181,11 +181,14 @@ extern "C" int rwkvb200_wkv7_backward(int dtype, int B, int T, int H, int N, int
                      "wkv7_backward: the bf16 N=64 path needs 16-byte aligned tensors");
         // Two independent one-group blocks per SM give the most throughput while every place has a unit (8.6 k cycles per chunk
         // and SM); units that have an SM to themselves take the two-stage form (one block per SM, two warp groups on consecutive
-        // chunks: 8.8 k cycles per chunk against 13.3 k).  So the whole rounds of the one, then what is left over in the other
-        // where that is at most a unit per SM (B16 T4096 H64: 888 units and 136, 5650 -> 5516 us forward + backward; B8 H40, 296 and 24,
-        // 2566 -> 2403 us).  Short sequences have less to gain than a launch and the wait between the two cost (B16 T128: 239 -> 250 us).
-        const int form = g_wkv7_bwd_form.load(), units = B * H, sms = sm_count();
-        const int rest = form == 1 ? 0 : form == 2 ? units : units <= sms ? units : sms > 0 && T >= 512 && units % (2 * sms) <= sms ? units % (2 * sms) : 0;
+        // chunks: 8.8 k cycles per chunk against 13.3 k).  So after one or two whole rounds of the one what is left over goes to the other,
+        // where that is at most a unit per SM.  Forward + backward, us, one-group blocks only / this: one round and 24 to 148 units T512 345 to
+        // 360 / 340 to 351, T1024 659 to 679 / 637 to 653, T4096 (B8 H40) 2533 / 2388; T256 187 / 190.  Two rounds T512 545 / 548, T1024 1043 / 1039,
+        // T2048 2043 / 2020.  After three rounds the SMs are apart by so much that blocks of the last one start beside others: T512 744 / 757,
+        // T1024 1428 / 1439, T2048 2797 / 2800, B16 T4096 H64 5592 / 5577 (two runs differ by 0.2 %; other boxes by 3 %).
+        const int form = g_wkv7_bwd_form.load(), units = B * H, sms = sm_count(), places = 2 * sms, rounds = places > 0 ? units / places : 0;
+        const bool tail = rounds >= 1 && rounds <= 2 && T >= 512 * rounds && units % places <= sms;
+        const int rest = form == 1 ? 0 : form == 2 || units <= sms ? units : tail ? units % places : 0;
         if (units > rest)
             if (int e = wkv7_l32_backward(B, T, H, 0, units - rest, r, w, k, v, a, b, dy, dsT, s, ds0, dr, dw, dk, dv, da, db, as_stream(stream))) return e;
         if (rest == 0) return RWKVB200_OK;

@@ -210,3 +210,28 @@ def test_units_left_over_from_whole_rounds(T, extra):
         assert ((a.double() - b.double()).abs() <= 2 ** -7 * b.double().abs() + 1e-6 * b.double().abs().max()).all()
         assert (a != b).double().mean().item() < 1e-3
     assert _lib.lib().rwkvb200_device_status() == 0
+
+
+@pytest.mark.parametrize("T,rounds,same", [(512, 1, False), (512, 2, True), (512, 3, True), (1024, 2, False), (1024, 3, True)])
+def test_where_left_over_units_take_the_other_kernel(T, rounds, same):
+    """24 units more than whole rounds of two per SM: the two-stage kernel takes them after one round from 512 tokens on and after two from 1024 on;
+    elsewhere the automatic choice is the one-group kernel for all, bit for bit."""
+    import rwkv_cuda_b200 as R
+    from rwkv_cuda_b200 import _lib
+    B, H, N = 1, 2 * rounds * torch.cuda.get_device_properties(0).multi_processor_count + 24, 64
+    g = torch.Generator(device=DEV).manual_seed(rounds)
+    rn = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    kk = torch.nn.functional.normalize(rn(B, T, H, N), dim=-1)
+    x = [z.bfloat16() for z in (0.5 * rn(B, T, H, N), rn(B, T, H, N), 0.5 * rn(B, T, H, N), 0.5 * rn(B, T, H, N), -kk, kk * torch.sigmoid(rn(B, T, H, N)))]
+    s0, dy, dsT = 0.1 * rn(B, H, N, N), rn(B, T, H, N).bfloat16(), rn(B, H, N, N)
+    y, sT, s, sa = torch.empty_like(x[0]), torch.empty_like(s0), torch.empty(B, H, T // 16, N, N, device=DEV), torch.empty(B, T, H, N, device=DEV)
+    R.ops.wkv7_forward(s0, *x, y, sT, s, sa)
+    got = []
+    for form in (0, 1):
+        _lib.call("rwkvb200_wkv7_select_form", form)
+        try:
+            got.append([torch.empty_like(s0), *(torch.empty_like(y) for _ in range(6))])
+            R.ops.wkv7_backward(*x, dy, dsT, s, sa, *got[-1])
+        finally:
+            _lib.call("rwkvb200_wkv7_select_form", 0)
+    assert all(torch.equal(a, b) for a, b in zip(*got)) == same
