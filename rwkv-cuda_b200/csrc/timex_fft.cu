@@ -275,7 +275,7 @@ __device__ __noinline__ void direct(const float* f, const float* s, float* out, 
     }
 }
 
-// spectrum of w' / N into shared memory, in the engine's order (16 per thread of a transform); true if a value is unfit for it
+// spectrum of w' / N into shared memory, in the engine's order (Plan::V per thread of a transform); true if a value is unfit for it
 template <int R>
 __device__ __forceinline__ bool filter_spectrum(Engine<R>& fft, cf* Wh, const float* __restrict__ w, int T) {
     using P = Plan<R>;
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(Plan<R>::kThreads, 3) timex_fft_backward_kerne
         }
         p0 += gridDim.y * P::G;
     }
-    // the spectra of the block's transforms are added up (each thread's 16 points meet their likes at the same j), then one inverse
+    // the spectra of the block's transforms are added up (each thread's points meet their likes at the same j), then one inverse
     __syncthreads();
     if (P::G > 1) {
         cf* sum = smem_fft;   // [G][V][L]

@@ -118,7 +118,7 @@ __device__ __forceinline__ float dot_keys(const f2 (&s)[32 / LG], const Keys<LG>
 }
 constexpr int kQ = 4;   // tokens of a step
 // The scaled vectors of a step, the products of its decays (w), its values, and the scalars of the steps inside it: b, k of token s
-// against a of token t (s < t) at ((t - 1) t / 2 + s) * 2, then against r of token t (s <= t, zero above) at 12 + 8 t + 2 s.
+// against a of token t (s < t) at ((t - 1) t / 2 + s) * 2, then against r of token t (s <= t, nothing above) at 12 + 8 t + 2 s.
 struct __align__(16) Step { float a[kQ][kN], r[kQ][kN], b[kQ][kN], k[kQ][kN], w[kN], v[kQ][kN], u[12 + 8 * kQ]; int odd; };
 template <int NSW>
 struct __align__(16) Staged { Step s[NSW]; };   // a step per staging warp
@@ -283,10 +283,6 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
                 if (sizeof(E) == 4) prefetch_l2(p + 32);
             }
         };
-        if (lane < 12) {   // the scalars above the diagonal: zero, and never written again
-            const int t = lane < 6 ? 0 : lane < 10 ? 1 : 2, x = lane - (lane < 6 ? 0 : lane < 10 ? 6 : 10);
-            buf[0].s[q].u[12 + 8 * t + 2 * (t + 1) + x] = buf[1].s[q].u[12 + 8 * t + 2 * (t + 1) + x] = 0.f;
-        }
         const int yt = lane >= 24 ? 3 : lane >= 18 ? 2 : lane >= 14 ? 1 : 0, slot = lane < 12 ? lane : 12 + 8 * yt + lane - (yt == 3 ? 24 : yt == 2 ? 18 : yt == 1 ? 14 : 12);
         float odd = 0.f;
         fetch(0);
@@ -452,7 +448,7 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
                 y[i] = own[i];
 #pragma unroll
                 for (int e = 0; e < kQ; ++e)
-                    if (e <= ty) y[i] = fmaf(sa[e][i], g[2 * e], fmaf(v[e][i], g[2 * e + 1], y[i]));   // (a later token's may not be finite)
+                    if (e <= ty) y[i] = fmaf(sa[e][i], g[2 * e], fmaf(v[e][i], g[2 * e + 1], y[i]));   // (g is not set for later tokens)
             }
             const int t = c * kCh + kQ * q + ty;
             if (x < 4 * TS && x % TS == 0 && t < T) store_rows<E, RPT>(y_ + base + (i64)t * C + row0, y);

@@ -105,7 +105,7 @@ def test_values_a_transform_cannot_take(T, bad):
         assert (~(got[~clean].abs() < 1e30)).float().mean() > 0.9, name
 
 
-@pytest.mark.parametrize("T", [383, 384, 385, 640, 767, 768, 769])   # the ends of the lengths 768 and 1536, which are not powers of two
+@pytest.mark.parametrize("T", [511, 512, 513, 514, 640, 767, 768, 769])   # both ends of the transforms of 1536 points (513 to 768 tokens)
 @pytest.mark.parametrize("B,C", [(1, 2), (3, 2), (33, 2)])
 def test_lengths_that_are_three_times_a_power_of_two(B, C, T):
     test_conv1d_training_class(B, C, T)

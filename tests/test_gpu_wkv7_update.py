@@ -1,5 +1,6 @@
 """GPU parity of the RWKV-7 inference kernels (head size 64, fp32 arithmetic) against the fp64 oracle at the lengths and
-unit counts where their forms change: one token, parts of a 16-token stage, and 1, 2 or 4 blocks per unit."""
+unit counts where their forms change: one token, parts of a step of four tokens, 1, 2 or 4 blocks per unit (16, 16 and 32 tokens staged at
+a time), and five stages and more, in which both buffers are handed back."""
 import pytest
 import torch
 
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("B,T,H", [(3, 1, 5), (1, 2, 3), (2, 15, 3), (1, 17, 38), (2, 33, 2), (3, 47, 37)])
+@pytest.mark.parametrize("B,T,H", [(3, 1, 5), (1, 2, 3), (2, 15, 3), (1, 17, 38), (2, 33, 2), (3, 47, 37), (1, 173, 3), (1, 87, 40), (3, 87, 37)])
 def test_state_update(dtype, B, T, H):
     import rwkv_cuda_b200 as R
     N, names = 64, ("r", "w", "k", "v", "a", "b")
