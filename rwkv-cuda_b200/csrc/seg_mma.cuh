@@ -1,5 +1,5 @@
 // Matrix forms of the kernels that work on the time segments of a sequence at the same time (wkv5_seg.cu, wkv6_seg.cu): head
-// size 64, segments of 32 tokens, fp32 or bf16 activations, fp32 precision throughout.
+// size 64, segments of 32 tokens, fp32 or bf16 activations, products of 24-bit operands and fp32 states.
 //
 // Inside a segment the recurrence is a set of small products (S: state before the segment, D: adjoint after it, both [key j]
 // [value i]; L_t: sum of log decays up to token t; m: the middle of the segment, where the scaled vectors are anchored so that
@@ -18,13 +18,17 @@
 //
 // Precision: the products run on mma.sync with bf16 operands, every fp32 operand as the sum of three bf16 numbers (24 bits: the
 // split is exact) and all partial products down to 2^-16 of the largest taken: 3 where the other side is a bf16 tensor as it
-// came, else 6.  What is left out is below 2^-25 of a product.
+// came, else 6.  What is left out is below 2^-25 of a product.  The split keeps its 24 bits as long as the last part is not below 2^-133: values
+// from 2^-109 on, times what scales them (kRange, kStaticRange).  The tensor core cuts its sums off instead of rounding them.  Where a
+// result is fp32 every group of products is summed from zero and added with rounding, and so is a segment's part of a state; y and
+// gradients in bf16 accumulate on the tensor core over one segment (5.9e-7 of the norm against 4.4e-7, where the rounding to bf16 makes 1.66e-3:
+// results equal to four digits at all decays, and 497 us instead of 526 for B8 T1000 H32).
 // Why mma.sync and not tcgen05: these kernels are a block per segment with every accumulator and both states in registers,
-// four blocks per SM; the operands are split where they are used, and at 8 clocks per instruction and scheduler the tensor pipe
+// three to five blocks per SM; the operands are split where they are used, and at 8 clocks per instruction and scheduler the tensor pipe
 // needs about as long as the arithmetic around it.
-// B8 T1000 H32 bf16: backward kernel 249 us (314 with a channel order in which a lane has two neighbours and not four, rows of
+// B8 T1000 H32 bf16: backward kernel 251 us (314 with a channel order in which a lane has two neighbours and not four, rows of
 // exponents 64 floats apart, the token matrices as fp32, a test of the alignment per load, bf16 parts unpacked before they are
-// subtracted and states read where they are used), y 103 us (110 with four blocks per SM and 125 registers a thread instead of five
+// subtracted and states read where they are used), y 105 us (110 with four blocks per SM and 125 registers a thread instead of five
 // and 96).  3700 instructions a warp, 324 of them mma: issue slots and the latency of 16 warps per SM (128 registers a thread) bound
 // it, the tensor pipe is busy 30 % of the time.
 // A segment whose decays leave the range (more than kRange between its middle and an end), that holds values that are not
@@ -43,7 +47,8 @@ namespace {
 // to bf16; with 60 it was 3.97e-3.  With 32, inputs of w around -1 +- 1 flag so many segments that B8 T1000 H32 takes 1140 us, 620 with 48.)
 constexpr float kRange = 48.f;
 // log2 of the largest decay of one token that is the same for all tokens: a factor of 2.  (Of a token and not up to the middle, which
-// let a short last segment have more: at T 34 a factor of 256.)
+// let a short last segment have more: at T 34 a factor of 256.)  Errors of y in fp32, products / token by token, of the norm: w from -6 to -1
+// 1.8e-7 / 5.2e-7, -1.2 to -1 1.15e-7 / 1.11e-7, -1 to -0.4 1.12e-7 / 9.4e-8 where all channels of a head are that fast; slower ones decide beside them.
 constexpr float kStaticRange = 1.f;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kImg = kSeg * 128;               // bytes of one bf16 image [32 tokens][64 channels]
@@ -894,7 +899,7 @@ __global__ void __launch_bounds__(128, sizeof(E) == 2 ? 4 : 3)
 // States at the start of every segment (REV: adjoints at the end), one block per unit walking its segments: S <- S diag(f) + k'^T V
 // with k'_s = k_s exp(L_end - L_s) (REV: r'_t = r_t exp(L_{t-1}), gy): all factors are at most 1.  Warps 0 to 3 have the state in
 // registers, 16 keys each, warps 4 to 11 make the operands of the segments to come (B8 T1000 H32 bf16: 80 us with four of them, two
-// sums of products at a time and states stored in pieces of 8 bytes, 62 us now: 3.7 TB/s; a third buffer of
+// sums of products at a time and states stored in pieces of 8 bytes, 65 us now: 3.5 TB/s; a third buffer of
 // operands changed nothing).
 template <typename E>
 struct ChainSmem {
@@ -1142,16 +1147,18 @@ __device__ __forceinline__ void for_flagged(const int* __restrict__ flags, i64 t
 }
 // A block per segment up to eight rounds of resident blocks: nothing is faster where all are flagged.  Above, four rounds of blocks, because with
 // none flagged it is the rounds that cost.  B8 T1000 H32, 8192 segments, y and gradients, none flagged / all: a block each 8 + 14 / 223 + 627 us,
-// eight rounds 9 + 11 / 279 + 659, four 6 + 7 / 270 + 680, one 4.5 + 4.3 / 301 + 694.
+// four rounds 6 + 6 / 277 + 684, one 4.5 + 4.3 / 301 + 694.
 inline i64 resident_blocks(int per_sm) { return (i64)(sm_count() > 0 ? sm_count() : 148) * per_sm; }
 inline bool block_per_segment(i64 total, int per_sm) { return total <= 8 * resident_blocks(per_sm); }
 
 // ---- launches ----------------------------------------------------------------------------------------------------------------
 // One block per unit walks all segments, or (the other kernels) every segment on its own and a scan: with few units the walk is
-// as long as T, and the scan's passes over the states cost little.
+// as long as T, and the scan's passes over the states cost little.  Forward + backward, us, scan / walk: RWKV-6 T999 48 units 166 / 176, 64 units
+// 205 / 204 (T4095 812 / 700), 80 units 255 / 227; RWKV-5 fp32 183 / 190, 226 / 221 (896 / 767), 275 / 253.
 inline bool seg_chain_pays(i64 units) { return units * 2 > sm_count(); }
-// Up to four segments per SM the token-by-token kernels take all of them: a launch less each way, and nothing to win (RWKV-6 T1000
-// H8 B1, 256 segments: 110 us, 114 by products; B2 T1000 H32, 2048 segments: 324 and 225 us).
+// Up to four segments per SM the token-by-token kernels take all of them: a launch less each way, and little to win.  Us, those / by
+// products, RWKV-6 and RWKV-5 fp32: 256 segments 95 / 101 and 91 / 96, 384 102 / 100 and 99 / 96, 512 121 / 100 and 108 / 97 (one sequence), 90 / 93
+// and 88 / 94 (eight of 100 tokens: 592 is where none is slower), 608 137 / 100 and 124 / 98, 768 149 / 103 and 138 / 108.  (About 90 us are the host's.)
 inline bool seg_mma_pays(i64 total) { return total > 4ll * sm_count(); }
 
 template <typename E, bool STATIC, bool REV>

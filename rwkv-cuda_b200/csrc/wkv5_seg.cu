@@ -22,8 +22,9 @@
 // the reads of the token's vectors bound everything (512 bytes per 96 packed multiply-adds); a lane therefore owns a tile of
 // 8 keys x 8 values, and the sums over lanes are taken for eight elements at a time (7 shuffles).
 // fp32, B8 T512 H16 N64, forward + backward on a B200: 1285 us with wkv5.cu, 309 us token by token on all segments (without register
-// spills in the backward, which two blocks per SM allow and three do not: 212 -> 167 us for that kernel), 178 us by products, whose errors
-// against fp64 are a third of that (T 1000: y 5.3e-7 -> 1.8e-7 of the norm, gw 8.8e-7 -> 3.1e-7).
+// spills in the backward, which two blocks per SM allow and three do not: 212 -> 167 us for that kernel), 190 us by products, whose errors
+// against fp64 are a third of that (T 1000, w from -6 to -1: y 5.2e-7 -> 1.8e-7 of the norm, gw 9.2e-7 -> 2.9e-7), 278 us where every head is
+// left to the kernels here.
 #include "wkv5_seg.cuh"
 #include "seg_mma.cuh"
 

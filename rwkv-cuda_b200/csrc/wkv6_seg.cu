@@ -17,7 +17,9 @@
 //
 // B8 T1000 H32, forward + backward on a B200: 4374 us on the general-shape kernels, which walk the tokens with one block per unit;
 // 1237 us with the token-by-token kernels on all segments (multiply-adds at 46 % of the issue slots and the shared-memory reads of
-// the tokens' vectors); 492 us with products.  Errors against fp64 are the same to four digits (1.66e-3: one rounding to bf16).
+// the tokens' vectors); 499 us with products, 1205 us where every segment has
+// a decay too strong for them.  Errors of bf16 results against fp64 are the same to four digits (1.66e-3: one rounding; B2 T1000 H40, decay inputs
+// around -5 to 1).
 // The kernels for whole 32-token chunks take 258 us, but their operands are TF32: outputs are then 2 to 4 % further from fp64.
 #include "wkv6_seg.cuh"
 #include "seg_mma.cuh"

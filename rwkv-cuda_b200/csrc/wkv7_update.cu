@@ -19,13 +19,13 @@
 // the eight dot products of a row are reduced together (8 shuffles, not 4 per token), 17 vectors are read instead of 20, and the
 // chain has one reduction per four tokens.  NCW warps compute; NSW warps stage, a step each: they make the scaled vectors (products of
 // decays are carried as sums of two numbers: a vector is rounded once) and the 32 scalars of a step, which all rows share.
-// One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 213 us with a token as a step, 203 us here; 128 units
-// 427 -> 380 us, 256 units 852 -> 670 us.  A step takes 790 clocks where a unit has four SMs: 350 of the shared-memory reads, the
+// One sequence of 1999 tokens, 32 heads: 2010 us for the general-shape kernel, 213 us with a token as a step, 209 us here; 128 units
+// 428 -> 394 us, 256 units 852 -> 700 us.  A step takes 790 clocks where a unit has four SMs: 350 of the shared-memory reads, the
 // rest 430 instructions per scheduler, of one warp that computes and one or two that stage (four staging warps 209 us, eight 201; with
 // more rows per block eight were slower: 128 units 411 us).
 // Errors against fp64 (T 1999, H 8, of the norm): state 8.3e-8, y 1.11e-7; a token as a step 8.7e-8 and 1.12e-7.  Most of the state is of the last
 // few tokens, and where all eight terms of a step went onto it one by one, each was rounded at its full size (9.3e-8, 1.14e-7); so
-// the four of sa are summed first.
+// the four of sa are summed first (one more instruction per pair: 256 units 670 -> 690).  What is not finite goes token by token: rows_again.
 #include "common.cuh"
 #include "packed.cuh"
 #include "wkv7_dispatch.cuh"
