@@ -468,6 +468,7 @@ __global__ void __launch_bounds__(32 * (NCW + NSW)) wkv7_rows_kernel(int T, int 
         for (int i = 0; i < RPT; ++i)
 #pragma unroll
             for (int e = 0; e < KP; ++e) unpack2(S[i][e], other[i][2 * e], other[i][2 * e + 1]);
+        __syncwarp();   // (other lanes of the warp have written the y that it looks at)
         rows_again<E, LG, RPT>(T, C, base, row0, x, st, r_, w_, k_, v_, a_, b_, y_, other);
         return;
     }
